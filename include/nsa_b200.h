@@ -98,12 +98,12 @@ int nsa_selection_bwd(const void* q, const void* k, const void* v, const int32_t
                       const float* row_scale, const float* row_dot,
                       void* workspace, size_t workspace_bytes, int impl, void* stream);
 
-/* The tcgen05 selection kernels walk the block list block by block: CSR (nsa_fsa.py:14-64), the
- * (query, slot) -> pair map and a work list, which nsa_selection_fwd and nsa_selection_bwd each
- * build inside their workspace.  A caller that runs both on one block list (every training step)
+/* The tcgen05 selection kernels walk the block list block by block: the queries of each block (what
+ * nsa_fsa.py:14-64 builds), the (query, slot) -> pair map and a work list, which nsa_selection_fwd
+ * and nsa_selection_bwd each build inside their workspace.  A caller that runs both on one block list (every training step)
  * can build them once into a buffer of nsa_selection_plan_bytes bytes (0: shape not served by the
- * tcgen05 kernels) and hand it to the *_planned forms, which copy it into place instead of
- * building.  The reference builds its CSR once per forward and once per backward
+ * tcgen05 kernels) and hand it to the *_planned forms, which read it instead of building
+ * their own.  The reference builds its CSR once per forward and once per backward
  * (nsa_selection_kernel.py:199-201, nsa_selection_backward.py:356-358); no counterpart for the
  * reuse. */
 size_t nsa_selection_plan_bytes(const NsaDims* dims, int S, int block_size);
@@ -147,6 +147,44 @@ int nsa_range_attn_bwd_acc(const void* q, const void* k, const void* v, const vo
                            void* workspace, size_t workspace_bytes, void* stream);
 int nsa_dq_finish(const NsaDims* dims, int S, int block_size, const float* dq_acc, const void* ws_slc,
                   void* dq, void* stream);
+
+/* ---- the whole op ------------------------------------------------------------------------------
+ * pooling -> compression attention -> block scoring and top-n -> selection attention, window
+ * attention -> gate blend (nsa_model.py:306-370 without the projections; nsa_fused_kernel.py:560-573
+ * when the lists are given and the pooling is the mean) in one call, and its backward in one call.
+ * The results are those of the entry points of the parts.  nsa_attention_fwd keeps in `saved` what
+ * nsa_attention_bwd needs (summaries, branch outputs, softmax statistics, selection plan; with
+ * need_grad = 0 it is only scratch); sizes come from nsa_attention_sizes.  Small problems run the
+ * branches on side streams of the library (one set per host thread and device), forked off `stream`
+ * and joined to it inside the call, so to the caller everything happens on `stream`. */
+typedef struct NsaAttentionDesc {
+  NsaDims dims;
+  int32_t block_size, n_sel, window;
+  int32_t n_init, n_local;            /* forced blocks, see nsa_topn_blocks_forced */
+  int32_t cmp_len, cmp_stride;        /* both block_size for the reference's grid */
+  int32_t learned;                    /* 1: learned pooling (comp[] given), 0: mean pooling */
+  int32_t given_lists;                /* 1: block_idx is an input, 0: the scorer writes it */
+  int32_t need_grad;
+  int32_t dq_accumulator;             /* window and compression dQ through one fp32 accumulator */
+  int32_t impl;                       /* NSA_IMPL_* */
+} NsaAttentionDesc;
+
+typedef struct NsaAttentionTensors {
+  const void *q, *kc, *vc, *ks, *vs, *kw, *vw, *gate;
+  const float* comp[6];               /* K side intra_pos, pool_logits, proj; V side the same */
+  int32_t* block_idx;
+  void* out;
+  const void* d_out;                  /* from here on: backward only */
+  void *dq, *dkc, *dvc, *dks, *dvs, *dkw, *dvw, *d_gate;
+  float* d_comp[6];
+} NsaAttentionTensors;
+
+int nsa_attention_sizes(const NsaAttentionDesc* desc, size_t* saved_bytes, size_t* fwd_workspace_bytes,
+                        size_t* bwd_workspace_bytes);
+int nsa_attention_fwd(const NsaAttentionDesc* desc, const NsaAttentionTensors* t, void* saved, void* workspace,
+                      size_t workspace_bytes, void* stream);
+int nsa_attention_bwd(const NsaAttentionDesc* desc, const NsaAttentionTensors* t, const void* saved,
+                      void* workspace, size_t workspace_bytes, void* stream);
 
 /* ---- block -> query CSR ---------------------------------------------------------------------
  * Replaces build_block_to_query_csr (nsa_fsa.py:14-64): pairs (query i, block j) with j >= 0

@@ -19,6 +19,12 @@ class NsaDims(ctypes.Structure):
     _fields_ = [(n, ctypes.c_int32) for n in ("B", "Hq", "Hkv", "T", "D", "dtype")]
 
 
+class NsaAttentionDesc(ctypes.Structure):
+    _fields_ = [("dims", NsaDims)] + [(n, ctypes.c_int32) for n in (
+        "block_size", "n_sel", "window", "n_init", "n_local", "cmp_len", "cmp_stride", "learned", "given_lists",
+        "need_grad", "dq_accumulator", "impl")]
+
+
 class NsaError(RuntimeError):
     pass
 
@@ -26,6 +32,10 @@ class NsaError(RuntimeError):
 _lib = None
 _vp, _i, _sz, _f = ctypes.c_void_p, ctypes.c_int, ctypes.c_size_t, ctypes.c_float
 _dp = ctypes.POINTER(NsaDims)
+_ap = ctypes.POINTER(NsaAttentionDesc)
+_sp = ctypes.POINTER(ctypes.c_size_t)
+# NsaAttentionTensors is a run of pointers: q..gate, comp[6], block_idx, out, d_out, dq..d_gate, d_comp[6]
+OP_TENSORS = ctypes.c_void_p * 31
 
 # every symbol the header declares, with its signature
 SIGNATURES = {
@@ -72,6 +82,9 @@ SIGNATURES = {
     "nsa_range_attn_bwd_acc_workspace_bytes": (_sz, [_dp, _i, _i, _i]),
     "nsa_range_attn_bwd_acc": (_i, [_vp] * 9 + [_dp, _i, _i, _i, _i, _vp, _vp, _vp, _sz, _vp]),
     "nsa_dq_finish": (_i, [_dp, _i, _i, _vp, _vp, _vp, _vp]),
+    "nsa_attention_sizes": (_i, [_ap, _sp, _sp, _sp]),
+    "nsa_attention_fwd": (_i, [_ap, _vp, _vp, _vp, _sz, _vp]),
+    "nsa_attention_bwd": (_i, [_ap, _vp, _vp, _vp, _sz, _vp]),
     "nsa_fused_projection_width": (_i, [_i, _i, _i]),
     "nsa_split_heads": (_i, [_vp] * 4 + [_i] * 6 + [_vp]),
     "nsa_merge_heads": (_i, [_vp] * 4 + [_i] * 6 + [_vp]),
@@ -122,6 +135,11 @@ def ptr(t):
 
 def stream():
     return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+
+def raw_stream(device):
+    """The current stream of `device` as the integer the C ABI takes."""
+    return torch._C._cuda_getCurrentRawStream(device.index)
 
 
 def dims(B, Hq, Hkv, T, D, dtype):

@@ -3,11 +3,12 @@ import hashlib
 import os
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(CSRC, "libnsa_b200.so")
-SOURCES = ["api.cu", "simt.cu", "aux.cu", "tc.cu", "tc_bwd.cu", "tc_score.cu", "tc_fwdpair.cu", "tc_fwdpair_kernel.cu", "optim.cu"]
+SOURCES = ["api.cu", "simt.cu", "aux.cu", "pool.cu", "sel_plan.cu", "tc.cu", "tc_bwd.cu", "tc_score.cu", "tc_fwdpair.cu", "tc_fwdpair_kernel.cu", "op.cu", "optim.cu"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "-DNSA_B200",
               "-Xptxas", "-v"]
@@ -38,17 +39,19 @@ def build_library(force=False, verbose=False):
     if (not force and os.path.exists(LIB) and os.path.exists(stamp_file)
             and open(stamp_file).read() == stamp):
         return LIB
-    objs = []
-    log = []
-    for src in SOURCES:
-        obj = os.path.join(CSRC, src[:-3] + ".o")
+    objs = [os.path.join(CSRC, src[:-3] + ".o") for src in SOURCES]
+
+    def compile_one(src, obj):
         cmd = [_nvcc()] + NVCC_FLAGS + ["-c", os.path.join(CSRC, src), "-o", obj]
-        r = subprocess.run(cmd, capture_output=True, text=True)
-        log.append(r.stderr)
+        return subprocess.run(cmd, capture_output=True, text=True)
+
+    with ThreadPoolExecutor(max_workers=min(len(SOURCES), os.cpu_count() or 1)) as pool:
+        results = list(pool.map(compile_one, SOURCES, objs))
+    log = [r.stderr for r in results]
+    for src, r in zip(SOURCES, results):
         if r.returncode != 0:
             sys.stderr.write(r.stdout + r.stderr)
             raise RuntimeError("nvcc failed on " + src)
-        objs.append(obj)
     r = subprocess.run([_nvcc(), "-shared", "-o", LIB] + objs + ["-lcudart"], capture_output=True, text=True)
     if r.returncode != 0:
         sys.stderr.write(r.stdout + r.stderr)

@@ -8,7 +8,7 @@
 #include <string>
 #include <vector>
 
-#include "common.cuh"
+#include "op.cuh"
 
 namespace nsa {
 
@@ -24,10 +24,54 @@ void set_error(const char* fmt, ...) {
 // One status word per device, raised (atomicOr) by kernels whose bounded waits run out.
 __device__ int g_device_status = 0;
 
+// What launches need to know of a device, looked up once per device: every lookup returns the same
+// value whichever thread makes it, so racing first calls are harmless.
+constexpr int kMaxDevices = 64;
+static int current_device() {
+  int dev = -1;
+  return cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < kMaxDevices ? dev : -1;
+}
+
 int* device_status_ptr() {
-  int* p = nullptr;
-  if (cudaGetSymbolAddress((void**)&p, g_device_status) != cudaSuccess) return nullptr;
+  static std::atomic<int*> known[kMaxDevices];
+  const int dev = current_device();
+  if (dev < 0) return nullptr;
+  int* p = known[dev].load(std::memory_order_acquire);
+  if (!p) {
+    if (cudaGetSymbolAddress((void**)&p, g_device_status) != cudaSuccess) return nullptr;
+    known[dev].store(p, std::memory_order_release);
+  }
   return p;
+}
+
+int sm_count() {
+  static std::atomic<int> known[kMaxDevices];
+  const int dev = current_device();
+  if (dev < 0) return 1;
+  int n = known[dev].load(std::memory_order_relaxed);
+  if (n == 0) {
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) n = 1;
+    known[dev].store(n, std::memory_order_relaxed);
+  }
+  return n;
+}
+
+cudaError_t func_smem(const void* kernel, size_t bytes) {
+  struct Entry { const void* kernel; int dev; size_t bytes; };
+  static std::mutex mu;
+  static std::vector<Entry> known;            // a few dozen kernels
+  const int dev = current_device();
+  std::lock_guard<std::mutex> lk(mu);
+  for (Entry& e : known)
+    if (e.kernel == kernel && e.dev == dev) {
+      if (e.bytes >= bytes) return cudaSuccess;
+      const cudaError_t rc = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+      if (rc == cudaSuccess) e.bytes = bytes;
+      return rc;
+    }
+  const cudaError_t rc = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (rc == cudaSuccess) known.push_back({kernel, dev, bytes});
+  return rc;
 }
 
 // ---- kernel accounting ---------------------------------------------------------------------
@@ -37,6 +81,8 @@ struct ProfRec { std::string name; cudaEvent_t e0, e1; };
 static std::mutex g_prof_mu;
 static std::vector<ProfRec> g_prof;
 static thread_local cudaEvent_t t_open_e1 = nullptr;
+
+bool profiling() { return g_profile.load(std::memory_order_relaxed) != 0; }
 
 void kernel_begin(const char* name, cudaStream_t st) {
   g_launches.fetch_add(1, std::memory_order_relaxed);
@@ -65,7 +111,7 @@ int get_option_merged_boxes() { return g_opt_merged.load(); }
 static std::atomic<int> g_opt_starve{0};
 int get_option_debug_starve_load() { return g_opt_starve.load(); }
 
-static int check_dims(const NsaDims* d) {
+int check_dims(const NsaDims* d) {
   NSA_CHECK_ARG(d != nullptr, "dims is null");
   NSA_CHECK_ARG(d->B >= 0 && d->T >= 0 && d->Hq > 0 && d->Hkv > 0, "bad B/T/Hq/Hkv");
   NSA_CHECK_ARG(d->Hq % d->Hkv == 0, "Hq=%d is not a multiple of Hkv=%d", d->Hq, d->Hkv);
@@ -77,7 +123,7 @@ static int check_dims(const NsaDims* d) {
 
 static size_t elem_size(int dtype) { return dtype == NSA_DTYPE_BF16 ? 2 : 4; }
 
-static AttnArgs base_args(const NsaDims* d, int Lk) {
+AttnArgs base_args(const NsaDims* d, int Lk) {
   AttnArgs a;
   memset(&a, 0, sizeof(a));
   a.B = d->B; a.Hq = d->Hq; a.Hkv = d->Hkv; a.T = d->T; a.D = d->D; a.Lk = Lk;
@@ -85,7 +131,7 @@ static AttnArgs base_args(const NsaDims* d, int Lk) {
   return a;
 }
 
-static bool use_tc(const NsaDims* d, int block_size, int impl, int* err) {
+bool use_tc(const NsaDims* d, int block_size, int impl, int* err) {
   *err = NSA_OK;
   if (impl == NSA_IMPL_SIMT) return false;
   const bool ok = tc_shape_ok(*d, block_size);
@@ -495,7 +541,7 @@ extern "C" int nsa_dq_reduce3(const NsaDims* dims, int Lk_cmp, int cmp_len, int 
   NSA_CHECK_ARG(!ws_win || window >= 1, "bad window");
   const AttnArgs a = base_args(dims, dims->T);
   return tc_dq_reduce3(a, Lk_cmp, cmp_len, cmp_stride, S, block_size, window, ws_cmp, ws_slc, ws_win,
-                       nullptr, dq, (cudaStream_t)stream);
+                       nullptr, nullptr, dq, (cudaStream_t)stream);
 }
 
 extern "C" int nsa_dq_finish(const NsaDims* dims, int S, int block_size, const float* dq_acc,
@@ -506,5 +552,5 @@ extern "C" int nsa_dq_finish(const NsaDims* dims, int S, int block_size, const f
   NSA_CHECK_ARG(use_tc(dims, block_size, NSA_IMPL_AUTO, &rc), "nsa_dq_finish needs a shape the tcgen05 kernels serve");
   NSA_CHECK_ARG(!ws_slc || S > 0, "bad S");
   const AttnArgs a = base_args(dims, dims->T);
-  return tc_dq_reduce3(a, 0, 0, 0, S, block_size, 1, nullptr, ws_slc, nullptr, dq_acc, dq, (cudaStream_t)stream);
+  return tc_dq_reduce3(a, 0, 0, 0, S, block_size, 1, nullptr, ws_slc, nullptr, nullptr, dq_acc, dq, (cudaStream_t)stream);
 }

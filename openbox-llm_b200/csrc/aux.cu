@@ -2,7 +2,7 @@
 // top-n, block->query CSR inversion and the sigmoid gate combine.
 #include <atomic>
 
-#include "common.cuh"
+#include "pool.cuh"
 
 namespace nsa {
 namespace {
@@ -127,219 +127,12 @@ __global__ void compress_bwd_block_kernel(const T* __restrict__ x, const float* 
   }
 }
 
-// ------------------------------------------------------------------------------------------
-// bf16 fast path of the learned pooling for D in {16,32,64,128}: one CTA of 256 threads takes
-// kCompRows consecutive blocks, streams their tokens with 16-byte loads (D/8 threads per token
-// row, 256/(D/8) token rows at a time) and keeps the projection matrix in shared memory
-// ------------------------------------------------------------------------------------------
-constexpr int kCompRows = 8;
-constexpr int kCompThreads = 256;
-
-__device__ __forceinline__ void unpack8(const uint4& u, float* f) {
-  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
-#pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    const float2 t = __bfloat1622float2(h[e]);
-    f[2 * e] = t.x; f[2 * e + 1] = t.y;
-  }
-}
-__device__ __forceinline__ uint32_t pack2(float a, float b) {
-  __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-  return *reinterpret_cast<uint32_t*>(&h);
-}
-
 __device__ __forceinline__ void pool_weights(const float* __restrict__ logits, float* w, int bs) {
   float mx = -INFINITY;
   for (int r = 0; r < bs; ++r) mx = fmaxf(mx, logits[r]);
   float den = 0.f;
   for (int r = 0; r < bs; ++r) den += expf(logits[r] - mx);
   for (int r = threadIdx.x; r < bs; r += blockDim.x) w[r] = expf(logits[r] - mx) / den;
-}
-
-// shared memory: w[bs] | cvec[D] | pooled[kCompRows][D] | part[kCompRows][8][D] | projT[D][D+1]
-__global__ void __launch_bounds__(kCompThreads)
-compress_fast_fwd_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ intra,
-                         const float* __restrict__ logits, const float* __restrict__ proj,
-                         __nv_bfloat16* __restrict__ out, float* __restrict__ pooled_out, int T_, int D,
-                         int bs, int stride, int n_blk, size_t rows) {
-  extern __shared__ float sm[];
-  float* w = sm;
-  float* cvec = w + bs;
-  float* pooled = cvec + D;
-  float* part = pooled + kCompRows * D;
-  float* projT = part + kCompRows * 8 * D;
-  const int tid = threadIdx.x, warp = tid >> 5;
-  const int VL = D >> 3, RG = kCompThreads / VL;
-  const int vl = tid % VL, rg = tid / VL;
-  const size_t row0 = (size_t)blockIdx.x * kCompRows;
-  if (out)
-    for (int idx = tid; idx < D * D; idx += kCompThreads) projT[(idx % D) * (D + 1) + idx / D] = proj[idx];
-  pool_weights(logits, w, bs);
-  __syncthreads();
-  // the block-independent part: sum_r w[r] * intra[r][:]
-  {
-    float a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    for (int r = rg; r < bs; r += RG) {
-      const float4 lo = *reinterpret_cast<const float4*>(intra + (size_t)r * D + vl * 8);
-      const float4 hi = *reinterpret_cast<const float4*>(intra + (size_t)r * D + vl * 8 + 4);
-      const float wr = w[r];
-      a[0] = fmaf(wr, lo.x, a[0]); a[1] = fmaf(wr, lo.y, a[1]); a[2] = fmaf(wr, lo.z, a[2]); a[3] = fmaf(wr, lo.w, a[3]);
-      a[4] = fmaf(wr, hi.x, a[4]); a[5] = fmaf(wr, hi.y, a[5]); a[6] = fmaf(wr, hi.z, a[6]); a[7] = fmaf(wr, hi.w, a[7]);
-    }
-    // threads of a warp that hold the same columns (VL apart) meet by shuffles
-    for (int o = 16; o >= VL; o >>= 1)
-#pragma unroll
-      for (int e = 0; e < 8; ++e) a[e] += __shfl_xor_sync(0xffffffffu, a[e], o);
-    if ((tid & 31) < VL)
-#pragma unroll
-      for (int e = 0; e < 8; ++e) part[warp * D + vl * 8 + e] = a[e];
-  }
-  __syncthreads();
-  if (tid < D) {
-    float c = 0.f;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) c += part[k * D + tid];
-    cvec[tid] = c;
-  }
-  __syncthreads();
-#pragma unroll
-  for (int b = 0; b < kCompRows; ++b) {
-    const size_t row = row0 + b;
-    float a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    if (row < rows) {
-      const size_t bh = row / n_blk;
-      const int j = (int)(row % n_blk);
-      const __nv_bfloat16* xb = x + (bh * T_ + (size_t)j * stride) * D + vl * 8;
-      for (int r = rg; r < bs; r += RG) {
-        const uint4 u = __ldg(reinterpret_cast<const uint4*>(xb + (size_t)r * D));
-        float f[8];
-        unpack8(u, f);
-        const float wr = w[r];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) a[e] = fmaf(wr, f[e], a[e]);
-      }
-    }
-    for (int o = 16; o >= VL; o >>= 1)
-#pragma unroll
-      for (int e = 0; e < 8; ++e) a[e] += __shfl_xor_sync(0xffffffffu, a[e], o);
-    if ((tid & 31) < VL)
-#pragma unroll
-      for (int e = 0; e < 8; ++e) part[(b * 8 + warp) * D + vl * 8 + e] = a[e];
-  }
-  __syncthreads();
-  for (int idx = tid; idx < kCompRows * D; idx += kCompThreads) {
-    const int b = idx / D, d = idx % D;
-    float s = cvec[d];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) s += part[(b * 8 + k) * D + d];
-    pooled[idx] = s;
-    if (pooled_out && row0 + b < rows) pooled_out[(row0 + b) * D + d] = s;
-  }
-  if (!out) return;
-  __syncthreads();
-  // out[row][o] = sum_i proj[o][i] * pooled[row][i], four rows per thread
-  for (int idx = tid; idx < (kCompRows / 4) * D; idx += kCompThreads) {
-    const int b0 = (idx / D) * 4, o = idx % D;
-    float acc[4] = {0.f, 0.f, 0.f, 0.f};
-    for (int i = 0; i < D; ++i) {
-      const float pv = projT[i * (D + 1) + o];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) acc[k] = fmaf(pv, pooled[(b0 + k) * D + i], acc[k]);
-    }
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-      if (row0 + b0 + k < rows) out[(row0 + b0 + k) * D + o] = __float2bfloat16(acc[k]);
-  }
-}
-
-// backward of the same: d_pooled = d_out @ W, dx = w[pos] * d_pooled, sum_dpooled += d_pooled,
-// d_w[pos] += sum_d d_pooled[d] * x[pos][d] (the intra_pos share of d_w is added by the final
-// kernel from sum_dpooled).  shared memory: w[bs] | dw[bs] | go[rows][D] | dp[rows][D] | proj[D][D]
-__global__ void __launch_bounds__(kCompThreads)
-compress_fast_bwd_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ logits,
-                         const float* __restrict__ proj, const __nv_bfloat16* __restrict__ d_out,
-                         __nv_bfloat16* __restrict__ dx, float* __restrict__ d_pooled_out,
-                         float* __restrict__ sum_dpooled, float* __restrict__ d_w, int T_, int D, int bs,
-                         int stride, int n_blk, size_t rows) {
-  extern __shared__ float sm[];
-  float* w = sm;
-  float* dw = w + bs;
-  float* go = dw + bs;
-  float* dp = go + kCompRows * D;
-  float* pj = dp + kCompRows * D;
-  const int tid = threadIdx.x;
-  const int VL = D >> 3, RG = kCompThreads / VL;
-  const int vl = tid % VL, rg = tid / VL;
-  const size_t row0 = (size_t)blockIdx.x * kCompRows;
-  for (int idx = tid; idx < D * D; idx += kCompThreads) pj[idx] = proj[idx];
-  for (int idx = tid; idx < kCompRows * D; idx += kCompThreads)
-    go[idx] = row0 + idx / D < rows ? __bfloat162float(d_out[row0 * D + idx]) : 0.f;
-  for (int r = tid; r < bs; r += kCompThreads) dw[r] = 0.f;
-  pool_weights(logits, w, bs);
-  __syncthreads();
-  for (int idx = tid; idx < (kCompRows / 4) * D; idx += kCompThreads) {
-    const int b0 = (idx / D) * 4, d = idx % D;
-    float acc[4] = {0.f, 0.f, 0.f, 0.f};
-    for (int o = 0; o < D; ++o) {
-      const float pv = pj[o * D + d];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) acc[k] = fmaf(go[(b0 + k) * D + o], pv, acc[k]);
-    }
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      dp[(b0 + k) * D + d] = acc[k];
-      if (row0 + b0 + k < rows) d_pooled_out[(row0 + b0 + k) * D + d] = acc[k];
-    }
-  }
-  __syncthreads();
-  if (tid < D) {
-    float s = 0.f;
-#pragma unroll
-    for (int b = 0; b < kCompRows; ++b) s += dp[b * D + tid];   // rows past the end hold zeros
-    atomicAdd(sum_dpooled + tid, s);
-  }
-#pragma unroll 2
-  for (int b = 0; b < kCompRows; ++b) {
-    const size_t row = row0 + b;
-    if (row >= rows) break;
-    const size_t bh = row / n_blk;
-    const int j = (int)(row % n_blk);
-    const size_t base = (bh * T_ + (size_t)j * stride) * D + vl * 8;
-    const bool write_dx = stride == bs;               // overlapping windows: compress_dx_kernel
-    float g[8];
-#pragma unroll
-    for (int e = 0; e < 8; ++e) g[e] = dp[b * D + vl * 8 + e];
-    for (int r0 = 0; r0 < bs; r0 += RG) {
-      const int r = r0 + rg;
-      float dot = 0.f;
-      if (r < bs) {
-        const uint4 u = __ldg(reinterpret_cast<const uint4*>(x + base + (size_t)r * D));
-        float f[8];
-        unpack8(u, f);
-        const float wr = w[r];
-        uint4 o;
-        o.x = pack2(wr * g[0], wr * g[1]); o.y = pack2(wr * g[2], wr * g[3]);
-        o.z = pack2(wr * g[4], wr * g[5]); o.w = pack2(wr * g[6], wr * g[7]);
-        if (write_dx) *reinterpret_cast<uint4*>(dx + base + (size_t)r * D) = o;
-#pragma unroll
-        for (int e = 0; e < 8; ++e) dot = fmaf(g[e], f[e], dot);
-      }
-      for (int o = VL >> 1; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
-      if (vl == 0 && r < bs) atomicAdd(dw + r, dot);
-    }
-  }
-  __syncthreads();
-  for (int r = tid; r < bs; r += kCompThreads) atomicAdd(d_w + r, dw[r]);
-}
-
-bool compress_fast_ok(int D, int bs, int dtype) {
-  return dtype == NSA_DTYPE_BF16 && (D == 16 || D == 32 || D == 64 || D == 128) && bs >= 1 && bs <= 1024;
-}
-size_t compress_fast_fwd_smem(int D, int bs, bool with_proj) {
-  return ((size_t)bs + D + kCompRows * D + kCompRows * 8 * D + (with_proj ? (size_t)D * (D + 1) : 0)) * sizeof(float);
-}
-size_t compress_fast_bwd_smem(int D, int bs) {
-  return (2 * (size_t)bs + 2 * kCompRows * D + (size_t)D * D) * sizeof(float);
 }
 
 // dx for overlapping windows (stride < length): token pos of (b, hkv) collects
@@ -361,34 +154,6 @@ __global__ void compress_dx_kernel(const float* __restrict__ d_pooled, const flo
   float acc = 0.f;
   for (int j = j_lo; j <= j_hi; ++j) acc = fmaf(w[pos - j * stride], d_pooled[(bh * n_blk + j) * D + d], acc);
   dx[i] = from_float<T>(acc);
-}
-
-// the same for bf16 rows of D = 8 * k elements: one thread per 8 columns, 16-byte stores
-__global__ void compress_dx_vec_kernel(const float* __restrict__ d_pooled, const float* __restrict__ logits,
-                                       __nv_bfloat16* __restrict__ dx, int T_, int D, int bs, int stride,
-                                       int n_blk, size_t n_vec) {
-  extern __shared__ float w[];
-  pool_weights(logits, w, bs);
-  __syncthreads();
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n_vec) return;
-  const int VL = D >> 3;
-  const int vl = (int)(i % VL);
-  const int pos = (int)((i / VL) % T_);
-  const size_t bh = i / ((size_t)VL * T_);
-  const int j_hi = min(n_blk - 1, pos / stride);
-  const int j_lo = max(0, (pos - bs + stride) / stride);
-  float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  for (int j = j_lo; j <= j_hi; ++j) {
-    const float wj = w[pos - j * stride];
-    const float4 lo = *reinterpret_cast<const float4*>(d_pooled + (bh * n_blk + j) * D + vl * 8);
-    const float4 hi = *reinterpret_cast<const float4*>(d_pooled + (bh * n_blk + j) * D + vl * 8 + 4);
-    acc[0] = fmaf(wj, lo.x, acc[0]); acc[1] = fmaf(wj, lo.y, acc[1]); acc[2] = fmaf(wj, lo.z, acc[2]); acc[3] = fmaf(wj, lo.w, acc[3]);
-    acc[4] = fmaf(wj, hi.x, acc[4]); acc[5] = fmaf(wj, hi.y, acc[5]); acc[6] = fmaf(wj, hi.z, acc[6]); acc[7] = fmaf(wj, hi.w, acc[7]);
-  }
-  uint4 o;
-  o.x = pack2(acc[0], acc[1]); o.y = pack2(acc[2], acc[3]); o.z = pack2(acc[4], acc[5]); o.w = pack2(acc[6], acc[7]);
-  *reinterpret_cast<uint4*>(dx + i * 8) = o;
 }
 
 // tail tokens past the last complete block get zero gradient
@@ -418,18 +183,9 @@ __global__ void compress_bwd_proj_kernel(const T* __restrict__ d_out, const floa
 // stage C: d_intra[pos][d] = w[pos] * sum_dpooled[d]; d_logits = w * (d_w - sum(d_w * w))
 __global__ void compress_bwd_final_kernel(const float* __restrict__ logits,
                                           const float* __restrict__ sum_dpooled,
-                                          float* __restrict__ d_w, const float* __restrict__ intra,
-                                          float* __restrict__ d_intra,
+                                          const float* __restrict__ d_w, float* __restrict__ d_intra,
                                           float* __restrict__ d_logits, int D, int bs) {
   extern __shared__ float w[];
-  if (intra) {   // the streaming kernel left out sum_d sum_dpooled[d] * intra_pos[pos][d]
-    for (int r = threadIdx.x; r < bs; r += blockDim.x) {
-      float s = 0.f;
-      for (int d = 0; d < D; ++d) s = fmaf(sum_dpooled[d], intra[(size_t)r * D + d], s);
-      d_w[r] += s;
-    }
-    __syncthreads();
-  }
   float mx = -INFINITY;
   for (int r = 0; r < bs; ++r) mx = fmaxf(mx, logits[r]);
   float den = 0.f;
@@ -825,6 +581,12 @@ __global__ void gate_bwd_rows_kernel(const T* __restrict__ oc, const T* __restri
   }
 }
 
+// rows of whole, aligned 16-byte vectors: the kernels of pool.cu
+inline bool pool_vec_ok(int D, int dtype, const void* a, const void* b) {
+  const int per = dtype == NSA_DTYPE_BF16 ? 8 : 4;
+  return D % per == 0 && (((uintptr_t)a | (uintptr_t)b) & 15) == 0;
+}
+
 inline unsigned blocks_for(size_t n, int per) { return (unsigned)((n + per - 1) / per); }
 
 }  // namespace
@@ -839,6 +601,11 @@ extern "C" int nsa_block_mean_pool_fwd(const void* x, void* out, int B, int Hkv,
   const size_t n = (size_t)B * Hkv * n_blk * D;
   if (n == 0) return NSA_OK;
   cudaStream_t st = (cudaStream_t)stream;
+  if (pool_vec_ok(D, dtype, x, out)) {
+    PoolSides p = {};
+    p.n = 1; p.x[0] = x; p.out[0] = out;
+    return pool_mean_fwd(p, B, Hkv, T, D, block_size, dtype, st);
+  }
   if (dtype == NSA_DTYPE_BF16)
     { KernelScope ks("mean_pool_fwd_kernel", st); mean_pool_fwd_kernel<<<blocks_for(n, 256), 256, 0, st>>>((const __nv_bfloat16*)x, (__nv_bfloat16*)out, T, D, block_size, n_blk, n); }
   else
@@ -854,6 +621,11 @@ extern "C" int nsa_block_mean_pool_bwd(const void* d_out, void* dx, int B, int H
   const size_t n = (size_t)B * Hkv * T * D;
   if (n == 0) return NSA_OK;
   cudaStream_t st = (cudaStream_t)stream;
+  if (pool_vec_ok(D, dtype, d_out, dx)) {
+    PoolSides p = {};
+    p.n = 1; p.d_out[0] = d_out; p.dx[0] = dx;
+    return pool_mean_bwd(p, B, Hkv, T, D, block_size, dtype, st);
+  }
   if (dtype == NSA_DTYPE_BF16)
     { KernelScope ks("mean_pool_bwd_kernel", st); mean_pool_bwd_kernel<<<blocks_for(n, 256), 256, 0, st>>>((const __nv_bfloat16*)d_out, (__nv_bfloat16*)dx, T, D, block_size, n_blk, n); }
   else
@@ -882,13 +654,10 @@ extern "C" int nsa_block_compress_strided_fwd(const void* x, const float* intra_
   if (ctas == 0) return NSA_OK;
   cudaStream_t st = (cudaStream_t)stream;
   const size_t sm = (size_t)(block_size + D) * sizeof(float);
-  if (compress_fast_ok(D, block_size, dtype)) {
-    const size_t fsm = compress_fast_fwd_smem(D, block_size, true);
-    NSA_CUDA_OK(cudaFuncSetAttribute(compress_fast_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fsm));
-    KernelScope ks("compress_fast_fwd_kernel", st);
-    compress_fast_fwd_kernel<<<(unsigned)((ctas + kCompRows - 1) / kCompRows), kCompThreads, fsm, st>>>(
-        (const __nv_bfloat16*)x, intra_pos, pool_logits, proj_w, (__nv_bfloat16*)out, (float*)nullptr, T, D,
-        block_size, stride, n_blk, ctas);
+  if (pool_learned_ok(D, block_size, dtype)) {
+    PoolSides p = {};
+    p.n = 1; p.x[0] = x; p.intra[0] = intra_pos; p.logits[0] = pool_logits; p.proj[0] = proj_w; p.out[0] = out;
+    return pool_learned_fwd(p, B, Hkv, T, D, block_size, stride, st);
   } else if (dtype == NSA_DTYPE_BF16)
     { KernelScope ks("compress_fwd_kernel", st); compress_fwd_kernel<<<(unsigned)ctas, (D + 31) / 32 * 32, sm, st>>>((const __nv_bfloat16*)x, intra_pos, pool_logits, proj_w, (__nv_bfloat16*)out, (float*)nullptr, T, D, block_size, stride, n_blk); }
   else
@@ -904,8 +673,8 @@ extern "C" size_t nsa_block_compress_bwd_workspace_bytes(int B, int Hkv, int T, 
 extern "C" size_t nsa_block_compress_strided_bwd_workspace_bytes(int B, int Hkv, int T, int D,
                                                                  int block_size, int stride) {
   const size_t rows = (size_t)B * Hkv * (block_size > 0 && stride > 0 ? n_windows(T, block_size, stride) : 0);
-  // pooled[rows,D] + d_pooled[rows,D] + sum_dpooled[D] + d_w[block_size]
-  return align_up((2 * rows * D + D + block_size) * sizeof(float), 256);
+  // pooled[rows,D] + d_pooled[rows,D] + the accumulators of the parameter gradients
+  return align_up((2 * rows * D + pool_acc_floats(D, block_size)) * sizeof(float), 256);
 }
 
 extern "C" int nsa_block_compress_bwd(const void* x, const float* intra_pos, const float* pool_logits,
@@ -937,6 +706,15 @@ extern "C" int nsa_block_compress_strided_bwd(const void* x, const float* intra_
   float* d_pooled = pooled + rows * D;
   float* sum_dp = d_pooled + rows * D;
   float* d_w = sum_dp + D;
+  if (pool_learned_ok(D, block_size, dtype)) {
+    PoolSides p = {};
+    p.n = 1; p.x[0] = x; p.intra[0] = intra_pos; p.logits[0] = pool_logits; p.proj[0] = proj_w; p.pooled[0] = pooled;
+    p.d_out[0] = d_out; p.dx[0] = dx; p.d_pooled[0] = d_pooled; p.acc[0] = sum_dp;
+    p.d_intra[0] = d_intra_pos; p.d_logits[0] = d_pool_logits; p.d_proj[0] = d_proj_w;
+    NSA_CUDA_OK(cudaMemsetAsync(sum_dp, 0, pool_acc_floats(D, block_size) * sizeof(float), st));
+    int rc = pool_learned_fwd(p, B, Hkv, T, D, block_size, stride, st);
+    return rc == NSA_OK ? pool_learned_bwd(p, B, Hkv, T, D, block_size, stride, st) : rc;
+  }
   NSA_CUDA_OK(cudaMemsetAsync(sum_dp, 0, (size_t)(D + block_size) * sizeof(float), st));
   const size_t sm_f = (size_t)(block_size + D) * sizeof(float);
   const size_t sm_b = (size_t)(block_size + D + 32) * sizeof(float);
@@ -944,23 +722,8 @@ extern "C" int nsa_block_compress_strided_bwd(const void* x, const float* intra_
   const size_t tail = overlap ? 0 : (size_t)(T - n_blk * block_size) * D * B * Hkv;
   NSA_CUDA_OK(cudaMemsetAsync(d_proj_w, 0, (size_t)D * D * sizeof(float), st));
   const dim3 pgrid(D, (unsigned)(rows >= 4096 ? 64 : (rows >= 64 ? rows / 64 : 1)));
-  const bool fast = compress_fast_ok(D, block_size, dtype);
   if (rows > 0) {
-    if (fast) {
-      const size_t fsm = compress_fast_fwd_smem(D, block_size, false), bsm = compress_fast_bwd_smem(D, block_size);
-      NSA_CUDA_OK(cudaFuncSetAttribute(compress_fast_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)compress_fast_fwd_smem(D, block_size, true)));
-      NSA_CUDA_OK(cudaFuncSetAttribute(compress_fast_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bsm));
-      const unsigned grid = (unsigned)((rows + kCompRows - 1) / kCompRows);
-      { KernelScope ks("compress_fast_fwd_kernel", st);
-        compress_fast_fwd_kernel<<<grid, kCompThreads, fsm, st>>>((const __nv_bfloat16*)x, intra_pos, pool_logits, proj_w,
-                                                                 (__nv_bfloat16*)nullptr, pooled, T, D, block_size, stride, n_blk, rows); }
-      { KernelScope ks("compress_fast_bwd_kernel", st);
-        compress_fast_bwd_kernel<<<grid, kCompThreads, bsm, st>>>((const __nv_bfloat16*)x, pool_logits, proj_w,
-                                                                 (const __nv_bfloat16*)d_out, (__nv_bfloat16*)dx, d_pooled,
-                                                                 sum_dp, d_w, T, D, block_size, stride, n_blk, rows); }
-      { KernelScope ks("compress_bwd_proj_kernel", st); compress_bwd_proj_kernel<<<pgrid, (D + 31) / 32 * 32, 0, st>>>((const __nv_bfloat16*)d_out, pooled, d_proj_w, rows, D); }
-    } else if (dtype == NSA_DTYPE_BF16) {
+    if (dtype == NSA_DTYPE_BF16) {
       { KernelScope ks("compress_fwd_kernel", st); compress_fwd_kernel<<<(unsigned)rows, (D + 31) / 32 * 32, sm_f, st>>>((const __nv_bfloat16*)x, intra_pos, pool_logits, proj_w, (__nv_bfloat16*)nullptr, pooled, T, D, block_size, stride, n_blk); }
       { KernelScope ks("compress_bwd_block_kernel", st); compress_bwd_block_kernel<<<(unsigned)rows, (D + 31) / 32 * 32, sm_b, st>>>((const __nv_bfloat16*)x, intra_pos, pool_logits, proj_w, (const __nv_bfloat16*)d_out, (__nv_bfloat16*)dx, d_pooled, sum_dp, d_w, T, D, block_size, stride, n_blk); }
       { KernelScope ks("compress_bwd_proj_kernel", st); compress_bwd_proj_kernel<<<pgrid, (D + 31) / 32 * 32, 0, st>>>((const __nv_bfloat16*)d_out, pooled, d_proj_w, rows, D); }
@@ -976,9 +739,7 @@ extern "C" int nsa_block_compress_strided_bwd(const void* x, const float* intra_
     if (n && rows == 0) NSA_CUDA_OK(cudaMemsetAsync(dx, 0, n * (dtype == NSA_DTYPE_BF16 ? 2 : 4), st));
     if (n && rows) {
       KernelScope ks("compress_dx_kernel", st);
-      if (dtype == NSA_DTYPE_BF16 && D % 8 == 0)
-        compress_dx_vec_kernel<<<blocks_for(n / 8, 256), 256, block_size * sizeof(float), st>>>(d_pooled, pool_logits, (__nv_bfloat16*)dx, T, D, block_size, stride, n_blk, n / 8);
-      else if (dtype == NSA_DTYPE_BF16)
+      if (dtype == NSA_DTYPE_BF16)
         compress_dx_kernel<<<blocks_for(n, 256), 256, block_size * sizeof(float), st>>>(d_pooled, pool_logits, (__nv_bfloat16*)dx, T, D, block_size, stride, n_blk, n);
       else
         compress_dx_kernel<<<blocks_for(n, 256), 256, block_size * sizeof(float), st>>>(d_pooled, pool_logits, (float*)dx, T, D, block_size, stride, n_blk, n);
@@ -992,7 +753,7 @@ extern "C" int nsa_block_compress_strided_bwd(const void* x, const float* intra_
       { KernelScope ks("zero_tail_kernel", st); zero_tail_kernel<<<blocks_for(tail, 256), 256, 0, st>>>((float*)dx, T, D, n_blk * block_size, (size_t)B * Hkv); }
     NSA_LAUNCH_OK("zero_tail_kernel");
   }
-  { KernelScope ks("compress_bwd_final_kernel", st); compress_bwd_final_kernel<<<1, 256, block_size * sizeof(float), st>>>(pool_logits, sum_dp, d_w, fast && rows > 0 ? intra_pos : nullptr, d_intra_pos, d_pool_logits, D, block_size); }
+  { KernelScope ks("compress_bwd_final_kernel", st); compress_bwd_final_kernel<<<1, 256, block_size * sizeof(float), st>>>(pool_logits, sum_dp, d_w, d_intra_pos, d_pool_logits, D, block_size); }
   NSA_LAUNCH_OK("compress_bwd_final_kernel");
   return NSA_OK;
 }

@@ -78,6 +78,10 @@ __device__ __forceinline__ float warp_max(float x) {
 
 // error word raised by kernels whose bounded waits run out; defined in api.cu
 int* device_status_ptr();
+int sm_count();                                          // multiprocessors of the current device
+// lets `kernel` use `bytes` of dynamic shared memory on the current device (a driver call the
+// first time only)
+cudaError_t func_smem(const void* kernel, size_t bytes);
 
 // Per-kernel accounting (api.cu): every kernel launch of the library sits inside a KernelScope,
 // which counts it and, when profiling is on, brackets it with CUDA events on its stream.
@@ -99,7 +103,8 @@ struct AttnArgs {
   const void* d_o; void* dq; float* dk_acc; float* dv_acc;   // backward
   const float* row_scale; const float* row_dot;   // backward of a gated branch (may be null)
   float* dq_acc;     // tcgen05 window / compression backward: fp32 accumulator [B*Hkv][T][G][D] that takes dQ (or null)
-  const void* sel_plan;   // tcgen05 selection: CSR + pair map + work list built earlier (tc_sel_plan_build), or null
+  const void* sel_plan;   // tcgen05 selection: plan built earlier (tc_sel_plan_build), or null
+  bool plan_kept;         // the plan outlives the dQ reduction: the backward need not copy its pair map
   int B, Hq, Hkv, T, Lk, D, S;
   int kind;          // 0 window, 1 compress, 2 selection
   int window, block_size;
@@ -116,10 +121,11 @@ size_t tc_sel_fwd_workspace(const AttnArgs& a);
 int tc_sel_fwd(const AttnArgs& a, void* ws, size_t ws_bytes, cudaStream_t st);
 size_t tc_sel_plan_bytes(const AttnArgs& a);
 int tc_sel_plan_build(const AttnArgs& a, void* plan, size_t plan_bytes, cudaStream_t st);
+const int32_t* sel_plan_pair_map(const AttnArgs& a, int S, int block_size, const void* plan);
 size_t tc_attn_bwd_workspace(const AttnArgs& a);
 int tc_attn_bwd(const AttnArgs& a, void* ws, size_t ws_bytes, cudaStream_t st);
 int tc_dq_reduce3(const AttnArgs& base, int Lk_cmp, int cmp_len, int cmp_stride, int S, int block_size,
                   int window, const void* ws_cmp, const void* ws_slc, const void* ws_win,
-                  const float* dq_acc, void* dq, cudaStream_t st);
+                  const int32_t* pos, const float* dq_acc, void* dq, cudaStream_t st);
 
 }  // namespace nsa

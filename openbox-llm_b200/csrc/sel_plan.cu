@@ -1,0 +1,306 @@
+// Builds the index structures of sel_plan.cuh in three launches whatever the size: count, scan,
+// fill.  A CTA of the first and the last takes a chunk of consecutive queries of one unit and
+// marks its list entries in a bitmap [key tile][query] in shared memory, from which ranks are
+// population counts; nothing but the counts and the results touches global memory.  At 16 units of
+// 32768 queries x 16 slots: 0.17 ms, against 0.30 ms and eight launches with the bitmap in global
+// memory (bound by the scattered 4-byte stores of the pairs); at 4 units of 1024 queries 16 us,
+// bound by latency.
+#include "sel_plan.cuh"
+
+namespace nsa {
+namespace {
+
+constexpr int kKeysPerTile = 64;
+constexpr int kThreads = 256;
+constexpr int kScanThreads = 1024;
+
+// key tile of a list entry of query t, -1 when the entry is empty or lies after t
+__device__ __forceinline__ int tile_of(int blk, int t, int block_size) {
+  if (blk < 0 || (long long)blk * block_size > t) return -1;
+  return (blk * block_size) / kKeysPerTile;
+}
+
+// Bitmap words are laid out [word][tile]: the entries a warp marks together name different tiles of
+// one or two queries, so they fall into different banks.
+__device__ __forceinline__ void mark_chunk(const int32_t* __restrict__ idx, uint32_t* bm, int t0, int n_q, int S,
+                                           int block_size, int n_kt, int cw) {
+  for (int i = threadIdx.x; i < n_kt * cw; i += kThreads) bm[i] = 0u;
+  __syncthreads();
+#pragma unroll 4
+  for (int e = threadIdx.x; e < n_q * S; e += kThreads) {
+    const int ql = e / S;
+    const int j = tile_of(__ldg(idx + e), t0 + ql, block_size);
+    if (j >= 0) atomicOr(&bm[(ql >> 5) * n_kt + j], 1u << (ql & 31));
+  }
+  __syncthreads();
+}
+
+// counts[unit][chunk][tile] and, per CTA, the distinct (query tile, key tile) pairs
+__global__ void __launch_bounds__(kThreads)
+plan_count_kernel(const int32_t* __restrict__ block_idx, int32_t* __restrict__ counts, int32_t* __restrict__ unions,
+                  SelPlanHeader* __restrict__ hdr, int T, int S, int block_size, int n_kt, int cw, int n_chunks,
+                  int nq_union) {
+  extern __shared__ uint32_t bm[];
+  const int chunk = blockIdx.x, unit = blockIdx.y;
+  if (chunk == 0 && unit == 0 && threadIdx.x == 0) { hdr->union_tiles = 0ull; hdr->pairs = 0ull; }
+  const int t0 = chunk * cw * 32, n_q = min(T - t0, cw * 32);
+  mark_chunk(block_idx + ((size_t)unit * T + t0) * S, bm, t0, n_q, S, block_size, n_kt, cw);
+  int uni = 0;
+  const int per = nq_union < 32 ? nq_union : 32;        // a query tile is a part of a word or whole words
+  const int tw = nq_union > 32 ? nq_union / 32 : 1;
+  const uint32_t mask = per == 32 ? 0xffffffffu : (1u << per) - 1u;
+  for (int j = threadIdx.x; j < n_kt; j += kThreads) {
+    int c = 0;
+    uint32_t run = 0u;
+    for (int w = 0; w < cw; ++w) {
+      const uint32_t b = bm[w * n_kt + j];
+      c += __popc(b);
+      if (per < 32) {
+        for (int k = 0; k < 32; k += per) uni += ((b >> k) & mask) != 0u;
+      } else {
+        run |= b;
+        if ((w + 1) % tw == 0 || w + 1 == cw) { uni += run != 0u; run = 0u; }
+      }
+    }
+    counts[((size_t)unit * n_chunks + chunk) * n_kt + j] = c;
+  }
+  __shared__ int s_uni;
+  if (threadIdx.x == 0) s_uni = 0;
+  __syncthreads();
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) uni += __shfl_xor_sync(0xffffffffu, uni, o);
+  if ((threadIdx.x & 31) == 0 && uni) atomicAdd(&s_uni, uni);
+  __syncthreads();
+  if (threadIdx.x == 0) unions[unit * n_chunks + chunk] = s_uni;
+}
+
+// exclusive scan of v over the CTA; *total gets the sum
+__device__ __forceinline__ int block_scan(int v, int* warp_sums, int* total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int incl = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += u;
+  }
+  if (lane == 31) warp_sums[warp] = incl;
+  __syncthreads();
+  if (warp == 0) {
+    int w = lane < kScanThreads / 32 ? warp_sums[lane] : 0;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, w, o);
+      if (lane >= o) w += u;
+    }
+    warp_sums[lane] = w;
+  }
+  __syncthreads();
+  const int before = warp ? warp_sums[warp - 1] : 0;
+  *total = warp_sums[kScanThreads / 32 - 1];
+  __syncthreads();
+  return before + incl - v;
+}
+
+// One CTA per unit: offsets of the key tiles, the start of every (chunk, tile) run in place of its
+// count, and the work items in (tile, chunk) order.  Up to 1024 tiles a pass; with fewer tiles the
+// chunks are dealt out over groups of threads, so the column sums are not one long chain of loads.
+__global__ void __launch_bounds__(kScanThreads)
+plan_scan_kernel(int32_t* __restrict__ counts, const int32_t* __restrict__ unions, SelPlan p, int T, int S,
+                 int n_kt, int n_chunks, int nq) {
+  constexpr int kBatch = 16;                  // loads in flight per thread
+  __shared__ int warp_sums[32];
+  __shared__ int part_sum[kScanThreads];
+  const int unit = blockIdx.x, tid = threadIdx.x;
+  int32_t* cnt = counts + (size_t)unit * n_chunks * n_kt;
+  int pair_carry = unit * T * S, item_carry = 0;
+  int32_t* off = p.offsets + (size_t)unit * (n_kt + 1);
+  int4* items = p.items + (size_t)unit * p.max_items;
+  int width = 32;                             // tiles per pass, a power of two
+  while (width < kScanThreads && width < n_kt) width <<= 1;
+  const int parts = kScanThreads / width, part = tid / width;
+  const int per = (n_chunks + parts - 1) / parts;
+  const int c0 = min(n_chunks, part * per), c1 = min(n_chunks, c0 + per);
+  for (int j0 = 0; j0 < n_kt; j0 += width) {
+    const int j = j0 + (tid & (width - 1));
+    int n = 0;
+    if (j < n_kt) {
+#pragma unroll 16
+      for (int c = c0; c < c1; ++c) n += cnt[(size_t)c * n_kt + j];
+    }
+    part_sum[tid] = n;
+    __syncthreads();
+    int before = 0, all = 0;                  // pairs of tile j in earlier groups of chunks / in all
+    for (int q = 0; q < parts; ++q) {
+      const int v = part_sum[q * width + (tid & (width - 1))];
+      if (q < part) before += v;
+      all += v;
+    }
+    const bool first_part = part == 0 && j < n_kt;
+    const int n_rt = (all + nq - 1) / nq;
+    // at least one item, so that a tile nobody lists still gets its zero gradients
+    const int n_it = first_part ? max(1, (n_rt + kSelChunkTiles - 1) / kSelChunkTiles) : 0;
+    int total, total_it;
+    const int start = pair_carry + block_scan(first_part ? all : 0, warp_sums, &total);
+    const int first = item_carry + block_scan(n_it, warp_sums, &total_it);
+    if (first_part) {
+      off[j] = start;
+      for (int k = 0; k < n_it && first + k < p.max_items; ++k)
+        items[first + k] = make_int4(unit, j, k * kSelChunkTiles, n_it);
+      part_sum[tid] = start;
+    }
+    __syncthreads();
+    if (j < n_kt) {
+      int run = part_sum[tid & (width - 1)] + before;
+      for (int c = c0; c < c1; c += kBatch) {
+        int v[kBatch];
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k) v[k] = c + k < c1 ? cnt[(size_t)(c + k) * n_kt + j] : 0;
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k) {
+          if (c + k < c1) cnt[(size_t)(c + k) * n_kt + j] = run;
+          run += v[k];
+        }
+      }
+    }
+    __syncthreads();
+    pair_carry += total;
+    item_carry += total_it;
+  }
+  int uni = 0;
+  for (int c = tid; c < n_chunks; c += kScanThreads) uni += unions[unit * n_chunks + c];
+  int uni_total;
+  block_scan(uni, warp_sums, &uni_total);
+  if (tid == 0) {
+    off[n_kt] = pair_carry;
+    p.n_items[unit] = min(item_carry, p.max_items);
+    atomicAdd(&p.hdr->union_tiles, (unsigned long long)uni_total);
+    atomicAdd(&p.hdr->pairs, (unsigned long long)(pair_carry - unit * T * S));
+  }
+}
+
+// Every entry's pair: the start of its (chunk, tile) run plus the rank of its query in the bitmap.
+// kMatch: a query's S entries sit in one warp (S divides 32), so the entries of one query that
+// name the same tile find one another by a warp match instead of reading the list again.
+template <bool kMatch>
+__global__ void __launch_bounds__(kThreads)
+plan_fill_kernel(const int32_t* __restrict__ block_idx, const int32_t* __restrict__ starts,
+                 int32_t* __restrict__ pairs, int32_t* __restrict__ pair_of_slot, int T, int S, int block_size,
+                 int n_kt, int cw, int n_chunks) {
+  extern __shared__ uint32_t bm[];
+  uint16_t* before = reinterpret_cast<uint16_t*>(bm + n_kt * cw);   // [word][tile]: queries in earlier words
+  const int chunk = blockIdx.x, unit = blockIdx.y;
+  const int t0 = chunk * cw * 32, n_q = min(T - t0, cw * 32);
+  const int32_t* idx = block_idx + ((size_t)unit * T + t0) * S;
+  mark_chunk(idx, bm, t0, n_q, S, block_size, n_kt, cw);
+  for (int j = threadIdx.x; j < n_kt; j += kThreads) {
+    int run = 0;
+    for (int w = 0; w < cw; ++w) {
+      before[w * n_kt + j] = (uint16_t)run;
+      run += __popc(bm[w * n_kt + j]);
+    }
+  }
+  __syncthreads();
+  const int32_t* st = starts + ((size_t)unit * n_chunks + chunk) * n_kt;
+  int32_t* pos = pair_of_slot + ((size_t)unit * T + t0) * S;
+  const uint32_t one = (1u << (block_size >> 4)) - 1u;              // column groups of one block
+  const int n_e = n_q * S;
+  for (int e0 = 0; e0 < n_e; e0 += kThreads) {
+    const int e = e0 + threadIdx.x;
+    const bool in = e < n_e;
+    const int ql = in ? e / S : 0, t = t0 + ql, slot = e - ql * S;
+    const int blk = in ? __ldg(idx + e) : -1;
+    const int j = tile_of(blk, t, block_size);
+    uint32_t groups = j < 0 ? 0u : one << ((blk * block_size - j * kKeysPerTile) >> 4);
+    bool dup = false;
+    if (kMatch) {
+      const uint32_t peers = __match_any_sync(0xffffffffu, j < 0 ? -1 - (int)threadIdx.x : (ql << 16) | j);
+      dup = (peers & ((1u << (threadIdx.x & 31)) - 1u)) != 0u;
+      if (block_size < kKeysPerTile) groups = __reduce_or_sync(peers, groups);
+    } else if (j >= 0) {
+      const int32_t* row = idx + ql * S;
+      for (int s = 0; s < S; ++s) {
+        const int b2 = __ldg(row + s);
+        if (tile_of(b2, t, block_size) != j) continue;
+        dup |= s < slot;
+        groups |= one << ((b2 * block_size - j * kKeysPerTile) >> 4);
+      }
+    }
+    int r = -1;
+    if (j >= 0 && !dup) {
+      const int at = (ql >> 5) * n_kt + j;
+      r = __ldg(st + j) + before[at] + __popc(bm[at] & ((1u << (ql & 31)) - 1u));
+      pairs[r] = (int32_t)((uint32_t)t | (groups << kPairPosBits));
+    }
+    if (in) pos[e] = r;
+  }
+}
+
+}  // namespace
+
+SelPlanLayout sel_plan_layout(int units, int T, int S, int nq) {
+  SelPlanLayout l;
+  l.n_ktiles = (T + kKeysPerTile - 1) / kKeysPerTile;
+  // sum over tiles of max(1, ceil(ceil(n_q / nq) / chunk)) <= tiles * (1 + 1/chunk) + pairs / (chunk * nq)
+  l.max_items = (int)((size_t)l.n_ktiles + l.n_ktiles / kSelChunkTiles + (size_t)T * S / ((size_t)kSelChunkTiles * nq) + 2);
+  // queries per chunk: a long chunk keeps the scan short, a short one keeps the SMs busy and the
+  // bitmap inside 64 KB
+  int cw = 16;
+  while (cw > 1 && ((size_t)l.n_ktiles * cw * 4 > 64 * 1024 || (cw > 2 && (long long)units * ((T + 32 * cw - 1) / (32 * cw)) < 148))) cw >>= 1;
+  l.chunk_words = cw;
+  l.n_chunks = (T + 32 * cw - 1) / (32 * cw);
+  const size_t cap = (size_t)units * T * S;
+  size_t off = 0;
+  auto take = [&](size_t bytes) { const size_t at = off; off += align_up(bytes, 256); return at; };
+  l.hdr = take(sizeof(SelPlanHeader));
+  l.n_items = take((size_t)units * 4);
+  l.items = take((size_t)units * l.max_items * sizeof(int4));
+  l.offsets = take((size_t)units * (l.n_ktiles + 1) * 4);
+  l.pairs = take(cap * 4);
+  l.pos = take(cap * 4);
+  l.scratch = take(((size_t)units * l.n_chunks * l.n_ktiles + (size_t)units * l.n_chunks) * 4);
+  l.total = off;
+  return l;
+}
+
+SelPlan sel_plan_at(const void* base, const SelPlanLayout& l) {
+  char* b = (char*)base;
+  SelPlan p;
+  p.hdr = (SelPlanHeader*)(b + l.hdr);
+  p.n_items = (int32_t*)(b + l.n_items);
+  p.items = (int4*)(b + l.items);
+  p.offsets = (int32_t*)(b + l.offsets);
+  p.pairs = (int32_t*)(b + l.pairs);
+  p.pair_of_slot = (int32_t*)(b + l.pos);
+  p.max_items = l.max_items;
+  return p;
+}
+
+int sel_plan_build(const int32_t* block_idx, void* base, const SelPlanLayout& l, int units, int T, int S,
+                   int block_size, int nq, int nq_union, cudaStream_t st) {
+  if (units == 0 || T == 0) return NSA_OK;
+  const SelPlan p = sel_plan_at(base, l);
+  int32_t* counts = (int32_t*)((char*)base + l.scratch);
+  int32_t* unions = counts + (size_t)units * l.n_chunks * l.n_ktiles;
+  const size_t smem = (size_t)l.n_ktiles * l.chunk_words * 4;
+  const dim3 grid(l.n_chunks, units);
+  const bool match = S <= 32 && 32 % S == 0 && l.n_ktiles < (1 << 16);
+  NSA_CUDA_OK(func_smem((const void*)plan_count_kernel, smem));
+  NSA_CUDA_OK(match ? func_smem((const void*)plan_fill_kernel<true>, smem + smem / 2)
+                    : func_smem((const void*)plan_fill_kernel<false>, smem + smem / 2));
+  { KernelScope ks("plan_count_kernel", st);
+    plan_count_kernel<<<grid, kThreads, smem, st>>>(block_idx, counts, unions, p.hdr, T, S, block_size, l.n_ktiles,
+                                                    l.chunk_words, l.n_chunks, nq_union); }
+  { KernelScope ks("plan_scan_kernel", st);
+    plan_scan_kernel<<<units, kScanThreads, 0, st>>>(counts, unions, p, T, S, l.n_ktiles, l.n_chunks, nq); }
+  { KernelScope ks("plan_fill_kernel", st);
+    if (match)
+      plan_fill_kernel<true><<<grid, kThreads, smem + smem / 2, st>>>(block_idx, counts, p.pairs, p.pair_of_slot, T, S,
+                                                                      block_size, l.n_ktiles, l.chunk_words, l.n_chunks);
+    else
+      plan_fill_kernel<false><<<grid, kThreads, smem + smem / 2, st>>>(block_idx, counts, p.pairs, p.pair_of_slot, T, S,
+                                                                       block_size, l.n_ktiles, l.chunk_words, l.n_chunks); }
+  NSA_LAUNCH_OK("selection plan kernels");
+  return NSA_OK;
+}
+
+}  // namespace nsa

@@ -29,8 +29,7 @@ struct FwdArgs {
   int* status;
   int B, Hq, Hkv, T, Lk, S, G, Gp, nq;
   int kind, window, block_size;
-  const unsigned long long* stats;   // selection: statistics for the variant choice (may be null)
-  const int32_t* offsets;            // selection: CSR offsets (pair count at the end)
+  const SelPlanHeader* plan;         // selection: statistics for the variant choice (null: this kernel serves the call)
   int force;
   int debug_starve;          // test only: the V load of the second key tile is never sent
   int n_qtiles, nb_sel;      // nb_sel = ceil(T / 64) blocks a selection list may name
@@ -97,8 +96,7 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   uint32_t* s_member = (uint32_t*)(s_scan + 132);   // [nb_sel * nw]   (selection only)
   uint16_t* s_tiles = (uint16_t*)(s_member + (p.kind == 2 ? p.nb_sel * p.nw : 0));
 
-  if (p.kind == 2 && p.stats != nullptr &&
-      prefer_pairs(p.stats, p.offsets, p.B * p.Hkv, p.nb_sel, p.nq, p.force))
+  if (p.kind == 2 && p.plan != nullptr && prefer_pairs(p.plan, p.nq, p.force))
     return;   // the block-outer variant serves this call: leave before anything is set up
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int qtile = p.n_qtiles - 1 - (int)blockIdx.x;   // long rows first
@@ -829,11 +827,10 @@ bool tc_shape_ok(const NsaDims& d, int block_size) {
 
 int get_option_debug_starve_load();   // api.cu
 
-static int launch_fwd(const AttnArgs& a, const unsigned long long* stats, const int32_t* offsets,
-                      int force, cudaStream_t st) {
+static int launch_fwd(const AttnArgs& a, const SelPlanHeader* plan, int force, cudaStream_t st) {
   using namespace tc;
   FwdArgs p;
-  p.stats = stats; p.offsets = offsets; p.force = force;
+  p.plan = plan; p.force = force;
   p.debug_starve = get_option_debug_starve_load();
   p.block_idx = a.block_idx;
   p.o = (__nv_bfloat16*)a.o;
@@ -857,18 +854,16 @@ static int launch_fwd(const AttnArgs& a, const unsigned long long* stats, const 
   const size_t smem = fwd_smem_bytes(a.D, p.nb_sel, p.nw, a.kind);
   if (a.kind != 2) {
     // window / compression: persistent CTAs, two per SM, each walking its share of the row tiles
-    int dev = 0, sms = 0;
-    NSA_CUDA_OK(cudaGetDevice(&dev));
-    NSA_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    const int sms = sm_count();
     const long long n_work = (long long)p.n_qtiles * a.B * a.Hkv;
     if (n_work == 0) return NSA_OK;
     const unsigned g1 = (unsigned)(n_work < 2LL * sms ? n_work : 2LL * sms);
     KernelScope ks(branch_name(kFwdNames, a.kind), st);
     if (a.D == 128) {
-      NSA_CUDA_OK(cudaFuncSetAttribute(tc_fwd_range_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      NSA_CUDA_OK(func_smem((const void*)tc_fwd_range_kernel<128>, smem));
       tc_fwd_range_kernel<128><<<g1, kFwdThreads, smem, st>>>(tm_q, tm_k, tm_v, p);
     } else {
-      NSA_CUDA_OK(cudaFuncSetAttribute(tc_fwd_range_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      NSA_CUDA_OK(func_smem((const void*)tc_fwd_range_kernel<64>, smem));
       tc_fwd_range_kernel<64><<<g1, kFwdThreads, smem, st>>>(tm_q, tm_k, tm_v, p);
     }
     NSA_LAUNCH_OK("tc_fwd_range_kernel");
@@ -876,21 +871,20 @@ static int launch_fwd(const AttnArgs& a, const unsigned long long* stats, const 
   }
   dim3 grid(p.n_qtiles, a.B * a.Hkv);
   if (a.D == 128) {
-    NSA_CUDA_OK(cudaFuncSetAttribute(tc_fwd_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    NSA_CUDA_OK(func_smem((const void*)tc_fwd_kernel<128>, smem));
     { KernelScope ks(branch_name(kFwdNames, a.kind), st); tc_fwd_kernel<128><<<grid, kFwdThreads, smem, st>>>(tm_q, tm_k, tm_v, p); }
   } else {
-    NSA_CUDA_OK(cudaFuncSetAttribute(tc_fwd_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    NSA_CUDA_OK(func_smem((const void*)tc_fwd_kernel<64>, smem));
     { KernelScope ks(branch_name(kFwdNames, a.kind), st); tc_fwd_kernel<64><<<grid, kFwdThreads, smem, st>>>(tm_q, tm_k, tm_v, p); }
   }
   NSA_LAUNCH_OK("tc_fwd_kernel");
   return NSA_OK;
 }
 
-int tc_attn_fwd(const AttnArgs& a, cudaStream_t st) { return launch_fwd(a, nullptr, nullptr, 0, st); }
+int tc_attn_fwd(const AttnArgs& a, cudaStream_t st) { return launch_fwd(a, nullptr, 0, st); }
 
-int tc_fwd_union_launch(const AttnArgs& a, const unsigned long long* stats, const int32_t* offsets,
-                        int force, cudaStream_t st) {
-  return launch_fwd(a, stats, offsets, force, st);
+int tc_fwd_union_launch(const AttnArgs& a, const SelPlanHeader* plan, int force, cudaStream_t st) {
+  return launch_fwd(a, plan, force, st);
 }
 
 }  // namespace nsa

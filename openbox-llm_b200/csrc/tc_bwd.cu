@@ -38,14 +38,12 @@ struct BwdArgs {
   const float* lse;
   const float* delta;          // sum_d dO * O per row (unscaled)
   const float* row_scale;      // gate value per row of a gated branch, or null
-  const int32_t* q_of_block;
-  const int32_t* offsets;      // [B*Hkv, n_ktiles + 1] global pair offsets (selection)
+  SelPlan plan;                // selection
   __nv_bfloat16* dk;
   __nv_bfloat16* dv;
   __nv_bfloat16* dq_part;
   float* dk_acc;               // fp32 accumulators, used when the row tiles of a key tile are split
   float* dv_acc;
-  const SelWorkHeader* work;   // selection: work items {bh, block, first row tile, chunks of the block}
   int* status;
   int split_chunk;             // row tiles per CTA when split
   int B, Hq, Hkv, T, Lk, G, nq;
@@ -108,7 +106,6 @@ __device__ __forceinline__ bool named_or_b(int id, int threads, int pred) {
 template <int D>
 __global__ void __launch_bounds__(512, 1)
 tc_bwd_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
-              const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
               const __grid_constant__ CUtensorMap tm_q_run, const __grid_constant__ CUtensorMap tm_do_run,
               const __grid_constant__ CUtensorMap tm_dq, const __grid_constant__ CUtensorMap tm_dqacc,
               const BwdArgs p) {
@@ -148,13 +145,8 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
   int* s_rowt = s_rowt_all + grp * 2 * kMaxNq;
   uint32_t* s_prow = s_prow_all + grp * 128;
 
-  int4 item = make_int4((int)blockIdx.y, (int)blockIdx.x, 0, 1);
-  if (p.kind == 2) {                                 // selection: one work item per CTA
-    if ((int)blockIdx.x >= p.work->n_items) return;
-    item = reinterpret_cast<const int4*>(p.work + 1)[blockIdx.x];
-  }
-  const int j = item.y;                              // key tile
-  const int bh = item.x;
+  const int j = blockIdx.x;                          // key tile
+  const int bh = blockIdx.y;
   const int b = bh / p.Hkv, hkv = bh % p.Hkv;
   const int key0 = j * kKeys;
   const int ql = row / p.G, g = row % p.G;
@@ -162,24 +154,21 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
   const bool row_slot_ok = ql < p.nq;
 
   // ---- the queries that attend this key tile ---------------------------------------------
-  int t_lo = 0, n_q = 0, pair_base = 0;
+  int t_lo = 0, n_q = 0;
   if (p.kind == 0) {
     t_lo = key0;
     n_q = min(p.T - 1, key0 + kKeys - 1 + p.window - 1) - t_lo + 1;
-  } else if (p.kind == 1) {
+  } else {
     t_lo = key0 * p.window + p.block_size - 1;       // first query that sees summary key0 (window: the stride)
     n_q = p.T - t_lo;
-  } else {
-    pair_base = __ldg(p.offsets + (size_t)bh * (p.n_ktiles + 1) + j);
-    n_q = __ldg(p.offsets + (size_t)bh * (p.n_ktiles + 1) + j + 1) - pair_base;
   }
   n_q = max(n_q, 0);
   const int n_rt_all = (n_q + p.nq - 1) / p.nq;
   // gridDim.z > 1: the row tiles are split in chunks and dK / dV go through fp32 atomics
-  const int chunk = p.kind == 2 ? kSelChunkTiles : ((int)gridDim.z > 1 ? p.split_chunk : n_rt_all);
-  const int rt_begin = p.kind == 2 ? item.z : (int)blockIdx.z * chunk;
+  const int chunk = (int)gridDim.z > 1 ? p.split_chunk : n_rt_all;
+  const int rt_begin = (int)blockIdx.z * chunk;
   const int rt_end = min(n_rt_all, rt_begin + chunk);
-  const bool split = p.kind == 2 ? item.w > 1 : gridDim.z > 1;
+  const bool split = gridDim.z > 1;
 
   if (rt_end <= rt_begin) {
     if (!split && n_rt_all == 0) {   // nobody attends these keys: their gradients are zero
@@ -208,7 +197,7 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
     mbar_init(bars + 7, 1); mbar_init(bars + 9, 1);   // per group: an aborted CTA waits here for its last MMAs
     fence_barrier_init();
     prefetch_tensormap(&tm_k); prefetch_tensormap(&tm_v);
-    prefetch_tensormap(&tm_q); prefetch_tensormap(&tm_do);
+    prefetch_tensormap(&tm_q_run); prefetch_tensormap(&tm_do_run);
     prefetch_tensormap(p.dq_acc_mode ? &tm_dqacc : &tm_dq);
   }
   __syncthreads();
@@ -231,9 +220,8 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
   const uint32_t tmem = *s_tmem;
   const uint32_t lane_base = tmem + ((uint32_t)(quad * 32) << 16);
   const uint32_t colS = grp * 128, colDP = grp * 128 + 64, colDQ = grp * 128;
-  // Q / dO tiles: slab-major (8-row groups 1024 bytes apart, slabs kRows * 128 apart) or, with merged
-  // boxes, the two slabs of an 8-row group side by side (groups 2048 bytes apart)
-  const uint32_t q_slab = p.merged ? 1024u : (uint32_t)(kRows * 128), q_sbo = p.merged ? 2048u : 1024u;
+  // Q / dO tiles: slab-major (8-row groups 1024 bytes apart, slabs kRows * 128 apart)
+  constexpr uint32_t q_slab = kRows * 128, q_sbo = 1024u;
 
   if (tid == 0) {
     mbar_expect_tx(bar_kv, 2 * kKVBytes);
@@ -261,52 +249,21 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
   auto row_query = [&](int i) -> int {
     const int qi = i * p.nq + ql;
     if (!row_slot_ok || qi >= n_q) return -1;
-    if (p.kind == 2) return ldg_s32_now(p.q_of_block + pair_base + qi);
     return t_lo + qi;
   };
   auto row_index = [&](int t) -> size_t { return (size_t)(b * p.Hq + head) * p.T + t; };
-  // one TMA box per query and slab for Q and for dO; a missing query reads past T: zeros
   const uint32_t gather_bytes = (uint32_t)(p.nq * p.G * 128 * kSlabs * 2);
-  // part (window / compression only): 0 = Q and dO, 1 = Q now (the byte count of both is
+  // part: 0 = Q and dO, 1 = Q now (the byte count of both is
   // announced), 2 = dO, issued later because its tile served as staging meanwhile
   auto gather = [&](const int* rowt, int part = 0) {
-    if (p.kind != 2) {
-      // window / compression: the tile's queries are consecutive tokens, one box per slab
-      if (lt == 0) {
-        if (part != 2) mbar_expect_tx(bar_g, gather_bytes);
-        const int tq = rowt[0] >= 0 ? rowt[0] : p.T;
+    // the tile's queries are consecutive tokens, one box per slab
+    if (lt == 0) {
+      if (part != 2) mbar_expect_tx(bar_g, gather_bytes);
+      const int tq = rowt[0] >= 0 ? rowt[0] : p.T;
 #pragma unroll
-        for (int s = 0; s < kSlabs; ++s) {
-          if (part != 2) tma_load_3d(sQ + s * (kRows * 128), &tm_q_run, bar_g, s * 64, b * p.Hq + hkv * p.G, tq);
-          if (part != 1) tma_load_3d(sDO + s * (kRows * 128), &tm_do_run, bar_g, s * 64, b * p.Hq + hkv * p.G, tq);
-        }
-      }
-    } else {
-      // selection: one box per (query, slab, tensor); the boxes are dealt out over the eight
-      // warps of the group (a few lanes each) because one warp issues them one after another
-      if (lt == 0) mbar_expect_tx(bar_g, gather_bytes);
-      const int op = lane * 8 + wg;                       // op id -> (query, slab, Q or dO)
-      if (p.merged) {
-        // a box costs the TMA unit a fixed time whatever its size, and the boxes of a tile are what
-        // bounds the kernel: one box per (query, tensor) brings both slabs, laid out side by side
-        for (int o = op; o < p.nq * 2; o += kGroupThreads) {
-          const int qq = o >> 1;
-          const int tq = rowt[qq] >= 0 ? rowt[qq] : p.T;
-          tma_load_5d(((o & 1) ? sDO : sQ) + qq * (p.G / 8) * 2048, (o & 1) ? &tm_do : &tm_q, bar_g, 0, 0, 0, tq,
-                      (b * p.Hq + hkv * p.G) >> 3);
-        }
-      }
-      const int n_ops = p.merged ? 0 : p.nq * kSlabs * 2;
-      for (int o = op; o < n_ops; o += kGroupThreads) {
-        const int qq = o / (kSlabs * 2), k = o % (kSlabs * 2);
-        const int s = k >> 1;
-        const int tq = rowt[qq] >= 0 ? rowt[qq] : p.T;   // a missing query reads past T: zeros
-        if (k & 1)
-          tma_load_3d(sDO + s * (kRows * 128) + qq * p.G * 128, &tm_do, bar_g, s * 64,
-                      b * p.Hq + hkv * p.G, tq);
-        else
-          tma_load_3d(sQ + s * (kRows * 128) + qq * p.G * 128, &tm_q, bar_g, s * 64,
-                      b * p.Hq + hkv * p.G, tq);
+      for (int s = 0; s < kSlabs; ++s) {
+        if (part != 2) tma_load_3d(sQ + s * (kRows * 128), &tm_q_run, bar_g, s * 64, b * p.Hq + hkv * p.G, tq);
+        if (part != 1) tma_load_3d(sDO + s * (kRows * 128), &tm_do_run, bar_g, s * 64, b * p.Hq + hkv * p.G, tq);
       }
     }
   };
@@ -371,10 +328,8 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
       if (p.kind == 0) {
         lo = max(0, t_cur - p.window + 1 - key0);
         hi = min(kKeys - 1, t_cur - key0);
-      } else if (p.kind == 1) {
-        hi = min(kKeys - 1, cmp_visible(t_cur, p.block_size, p.window, p.Lk) - 1 - key0);
       } else {
-        hi = min(kKeys - 1, min(t_cur, p.T - 1) - key0);
+        hi = min(kKeys - 1, cmp_visible(t_cur, p.block_size, p.window, p.Lk) - 1 - key0);
       }
     }
     const float lse2_cur = lse_cur * kLog2e;
@@ -435,12 +390,8 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
     if (half == 0) {
       uint32_t prow = 0xffffffffu;
       if (t_cur >= 0) {
-        if (p.kind == 2) {
-          prow = (uint32_t)((size_t)(pair_base + i * p.nq + ql) * p.G + g);
-        } else {
-          const int slot = p.kind == 0 ? j % p.n_slots : j;
-          prow = (uint32_t)((((size_t)bh * p.T + t_cur) * p.n_slots + slot) * p.G + g);
-        }
+        const int slot = p.kind == 0 ? j % p.n_slots : j;
+        prow = (uint32_t)((((size_t)bh * p.T + t_cur) * p.n_slots + slot) * p.G + g);
       }
       s_prow[row] = prow;
     }
@@ -515,9 +466,8 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
       if ((i + 1) * p.nq <= n_q) {
         // a full tile: its rows are consecutive in the partial buffer, one TMA store per slab
         if (lt == 0) {
-          const int slot = p.kind == 2 ? 0 : (p.kind == 0 ? j % p.n_slots : j);
-          const int mid = p.kind == 2 ? pair_base + i * p.nq : t_lo + i * p.nq;
-          const int outer = p.kind == 2 ? 0 : bh;
+          const int slot = p.kind == 0 ? j % p.n_slots : j;
+          const int mid = t_lo + i * p.nq, outer = bh;
 #pragma unroll
           for (int sl = 0; sl < kSlabs; ++sl)
             tma_store_5d(&tm_dq, sP + sl * (kRows * 128), sl * 64, 0, slot, mid, outer);
@@ -636,8 +586,8 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
 
   int4 item = make_int4((int)blockIdx.y, (int)blockIdx.x, 0, 1);
   if (p.kind == 2) {                                 // selection: one work item per CTA
-    if ((int)blockIdx.x >= p.work->n_items) return;
-    item = reinterpret_cast<const int4*>(p.work + 1)[blockIdx.x];
+    if ((int)(blockIdx.x % p.plan.max_items) >= p.plan.n_items[blockIdx.x / p.plan.max_items]) return;
+    item = p.plan.items[blockIdx.x];
   }
   const int j = item.y;                              // key tile
   const int bh = item.x;
@@ -653,8 +603,8 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
     t_lo = key0 * p.window + p.block_size - 1;       // first query that sees summary key0 (window: the stride)
     n_q = p.T - t_lo;
   } else {
-    pair_base = __ldg(p.offsets + (size_t)bh * (p.n_ktiles + 1) + j);
-    n_q = __ldg(p.offsets + (size_t)bh * (p.n_ktiles + 1) + j + 1) - pair_base;
+    pair_base = __ldg(p.plan.offsets + (size_t)bh * (p.n_ktiles + 1) + j);
+    n_q = __ldg(p.plan.offsets + (size_t)bh * (p.n_ktiles + 1) + j + 1) - pair_base;
   }
   n_q = max(n_q, 0);
   const int n_rt_all = (n_q + p.nq - 1) / p.nq;
@@ -746,7 +696,7 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
     auto box_of = [&](int r) -> int { return (r * 32 + lane) * kB2Producers + pw; };
     auto tq_of = [&](int k, int o) -> int {          // query position of box o of tile k (none: past T, zeros)
       const int qi = (rt_begin + k) * p.nq + o / per_q;
-      return (o < n_ops && qi < n_q) ? ldg_s32_now(p.q_of_block + pair_base + qi) : p.T;
+      return (o < n_ops && qi < n_q) ? (int)(ldg_s32_now(p.plan.pairs + pair_base + qi) & kPairPosMask) : p.T;
     };
     int tq[kRounds];
     if (p.kind == 2) {
@@ -893,13 +843,15 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
     uint8_t* sDS = sP + kPBytes;
     uint32_t* s_prow_g = s_prow + sb * 128;
     const uint32_t lane_base = tmem + ((uint32_t)(quad * 32) << 16) + sb * 128;
+    // query of this thread's row in tile k (selection: with the tile's column groups it attends in
+    // the bits above the position), -1: no row
     auto row_query = [&](int k) -> int {
       const int qi = (rt_begin + k) * p.nq + ql;
       if (!row_slot_ok || qi >= n_q) return -1;
-      if (p.kind == 2) return ldg_s32_now(p.q_of_block + pair_base + qi);
+      if (p.kind == 2) return ldg_s32_now(p.plan.pairs + pair_base + qi);
       return t_lo + qi;
     };
-    auto row_index = [&](int t) -> size_t { return (size_t)(b * p.Hq + head) * p.T + t; };
+    auto row_index = [&](int t) -> size_t { return (size_t)(b * p.Hq + head) * p.T + (t & (int)kPairPosMask); };
     int t_cur = sb < n_tiles ? row_query(sb) : -1;
     int t_nxt = sb + 2 < n_tiles ? row_query(sb + 2) : -1;
     float lse_cur = 0.f, delta_cur = 0.f, gate_cur = 1.f;
@@ -925,7 +877,7 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
         } else if (p.kind == 1) {
           hi = min(kKeys - 1, cmp_visible(t_cur, p.block_size, p.window, p.Lk) - 1 - key0);
         } else {
-          hi = min(kKeys - 1, min(t_cur, p.T - 1) - key0);
+          hi = min(kKeys - 1, (t_cur & (int)kPairPosMask) - key0);
         }
       }
       // gate * p = 2^(s * scale * log2e - lse * log2e + log2(gate)): the branch's dO is gate * dO, so dV takes
@@ -1282,16 +1234,9 @@ struct BwdPlan {
   int n_ktiles, n_slots, nq, n_splits, split_chunk;
   size_t off_acc;
   size_t cap_pairs;          // selection: pairs the CSR may hold
-  size_t off_delta, off_part, off_csr_ws, off_qob, off_off, off_pbh, off_pos, off_work, total;
-  size_t sel_region_bytes;   // selection: bytes from off_qob to the end of the work list
+  SelPlanLayout layout;      // selection
+  size_t off_delta, off_part, off_plan, total;
 };
-
-struct SelRegion { size_t qob, pbh, off, pos, work, total; };                     // tc_fwdpair.cu
-SelRegion sel_region(size_t units, int n_ktiles, size_t cap_pairs, int nq);
-size_t sel_work_max_items(size_t units, int n_ktiles, size_t cap_pairs, int nq);
-size_t sel_work_bytes(size_t units, int n_ktiles, size_t cap_pairs, int nq);
-int sel_build_worklist(const int32_t* offsets, int n_ktiles, size_t units, size_t cap_pairs, int nq,
-                       void* work, cudaStream_t st);
 
 }  // namespace tc
 int get_option_merged_boxes();   // api.cu
@@ -1317,14 +1262,10 @@ static BwdPlan plan_bwd(const AttnArgs& a) {
   size_t off = 0;
   pl.off_delta = off; off += align_up((size_t)a.B * a.Hq * a.T * sizeof(float), 256);
   pl.off_part = off; off += align_up(part_rows * G * a.D * 2, 256);
-  pl.off_csr_ws = pl.off_qob = pl.off_off = pl.off_pbh = pl.off_pos = off;
+  pl.off_plan = off;
   if (a.kind == 2) {
-    pl.off_csr_ws = off; off += align_up(nsa_csr_workspace_bytes(a.B, a.Hkv, pl.n_ktiles * kKeys, a.S, kKeys), 256);
-    const SelRegion r = sel_region(units, pl.n_ktiles, pl.cap_pairs, pl.nq);   // same layout as the forward's
-    pl.off_qob = off + r.qob; pl.off_pbh = off + r.pbh; pl.off_off = off + r.off;
-    pl.off_pos = off + r.pos; pl.off_work = off + r.work;
-    pl.sel_region_bytes = r.total;
-    off += r.total;
+    pl.layout = sel_plan_layout((int)units, a.T, a.S, pl.nq);
+    off += pl.layout.total;
   }
   // compression: a few key tiles are attended by (almost) every query; split their row tiles
   pl.n_splits = 1;
@@ -1345,10 +1286,7 @@ static BwdPlan plan_bwd(const AttnArgs& a) {
 
 }  // namespace tc
 
-// defined in aux.cu: CSR with an explicit block count and the (query, slot) -> pair map
-int build_csr_internal(const int32_t* block_idx, int B, int Hkv, int T, int S, int block_size,
-                       int n_blk, int32_t* q_of_block, int32_t* block_offsets, int32_t* pair_bh,
-                       int32_t* pair_of_slot, void* workspace, size_t workspace_bytes, cudaStream_t st);
+int tc_sel_plan_build(const AttnArgs& a, void* plan, size_t plan_bytes, cudaStream_t st);   // tc_fwdpair.cu
 
 size_t tc_attn_bwd_workspace(const AttnArgs& a) { return tc::plan_bwd(a).total; }
 
@@ -1367,12 +1305,10 @@ int tc_attn_bwd(const AttnArgs& a, void* ws, size_t ws_bytes, cudaStream_t st) {
   p.lse = a.lse;
   p.delta = a.row_dot ? a.row_dot : (float*)(base + pl.off_delta);
   p.row_scale = a.row_scale;
-  p.q_of_block = (const int32_t*)(base + pl.off_qob);
-  p.offsets = (const int32_t*)(base + pl.off_off);
   p.dk = (__nv_bfloat16*)a.dk_acc;     // the API passes the dk / dv outputs through these fields
   p.dv = (__nv_bfloat16*)a.dv_acc;
   p.dq_part = (__nv_bfloat16*)(base + pl.off_part);
-  p.work = nullptr;
+  p.plan = SelPlan{};
   p.status = device_status_ptr();
   if (!p.status) { set_error("device status word unavailable"); return NSA_ERR_CUDA; }
   p.B = a.B; p.Hq = a.Hq; p.Hkv = a.Hkv; p.T = a.T; p.Lk = a.Lk; p.G = G; p.nq = pl.nq;
@@ -1396,22 +1332,19 @@ int tc_attn_bwd(const AttnArgs& a, void* ws, size_t ws_bytes, cudaStream_t st) {
                                                              (float*)(base + pl.off_delta), rows, a.D);
   }
   NSA_LAUNCH_OK("delta_kernel");
-  int32_t* pair_of_slot = (int32_t*)(base + pl.off_pos);
   if (a.kind == 2) {
-    if (a.sel_plan) {      // built earlier for this block list: one copy instead of the build
-      NSA_CUDA_OK(cudaMemcpyAsync(base + pl.off_qob, a.sel_plan, pl.sel_region_bytes, cudaMemcpyDeviceToDevice, st));
-    } else {
-      int rc = build_csr_internal(a.block_idx, a.B, a.Hkv, a.T, a.S, kKeys, pl.n_ktiles,
-                                  (int32_t*)(base + pl.off_qob), (int32_t*)(base + pl.off_off),
-                                  (int32_t*)(base + pl.off_pbh), pair_of_slot, base + pl.off_csr_ws,
-                                  pl.off_qob - pl.off_csr_ws, st);
+    const void* plan_mem = a.sel_plan;
+    if (!plan_mem) {
+      plan_mem = base + pl.off_plan;
+      int rc = tc_sel_plan_build(a, base + pl.off_plan, pl.layout.total, st);
       if (rc != NSA_OK) return rc;
-      rc = sel_build_worklist(p.offsets, pl.n_ktiles, (size_t)a.B * a.Hkv, pl.cap_pairs, pl.nq, base + pl.off_work, st);
-      if (rc != NSA_OK) return rc;
+    } else if (!a.dq && !a.plan_kept) {      // nsa_dq_reduce3 looks the pair map up in the workspace
+      NSA_CUDA_OK(cudaMemcpyAsync(base + pl.off_plan + pl.layout.pos, (const char*)plan_mem + pl.layout.pos,
+                                  pl.cap_pairs * sizeof(int32_t), cudaMemcpyDeviceToDevice, st));
     }
-    p.work = (const SelWorkHeader*)(base + pl.off_work);
+    p.plan = sel_plan_at(plan_mem, pl.layout);
     KernelScope ks("sel_split_blocks_kernel", st);
-    sel_split_blocks_kernel<<<dim3(pl.n_ktiles, a.B * a.Hkv), 256, 0, st>>>(p.offsets, p.dk_acc, p.dv_acc, p.dk, p.dv,
+    sel_split_blocks_kernel<<<dim3(pl.n_ktiles, a.B * a.Hkv), 256, 0, st>>>(p.plan.offsets, p.dk_acc, p.dv_acc, p.dk, p.dv,
                                                                         pl.n_ktiles, pl.nq, a.Lk, a.D, 0);
   }
   CUtensorMap tm_k, tm_v, tm_q, tm_do;
@@ -1437,29 +1370,29 @@ int tc_attn_bwd(const AttnArgs& a, void* ws, size_t ws_bytes, cudaStream_t st) {
   const size_t smem = bwd_smem_bytes(a.D);
   dim3 grid(pl.n_ktiles, a.B * a.Hkv, pl.n_splits);
   if (a.kind == 2)
-    grid = dim3((unsigned)sel_work_max_items((size_t)a.B * a.Hkv, pl.n_ktiles, pl.cap_pairs, pl.nq));
-  if (get_option_bwd_kernel() == 1 && !p.dq_acc_mode) {       // compute groups relieved of the issuing
+    grid = dim3((unsigned)((size_t)a.B * a.Hkv * pl.layout.max_items));
+  if ((get_option_bwd_kernel() == 1 || a.kind == 2) && !p.dq_acc_mode) {   // compute groups relieved of the issuing
     KernelScope ks(branch_name(kBwdNames, a.kind), st);
     if (a.D == 128) {
-      NSA_CUDA_OK(cudaFuncSetAttribute(tc_bwd2_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      NSA_CUDA_OK(func_smem((const void*)tc_bwd2_kernel<128>, smem));
       tc_bwd2_kernel<128><<<grid, kB2Threads, smem, st>>>(tm_k, tm_v, tm_q, tm_do, tm_q_run, tm_do_run, tm_dq, p);
     } else {
-      NSA_CUDA_OK(cudaFuncSetAttribute(tc_bwd2_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      NSA_CUDA_OK(func_smem((const void*)tc_bwd2_kernel<64>, smem));
       tc_bwd2_kernel<64><<<grid, kB2Threads, smem, st>>>(tm_k, tm_v, tm_q, tm_do, tm_q_run, tm_do_run, tm_dq, p);
     }
   } else if (a.D == 128) {
-    NSA_CUDA_OK(cudaFuncSetAttribute(tc_bwd_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    NSA_CUDA_OK(func_smem((const void*)tc_bwd_kernel<128>, smem));
     KernelScope ks(branch_name(kBwdNames, a.kind), st);
-    tc_bwd_kernel<128><<<grid, 512, smem, st>>>(tm_k, tm_v, tm_q, tm_do, tm_q_run, tm_do_run, tm_dq, tm_dqacc, p);
+    tc_bwd_kernel<128><<<grid, 512, smem, st>>>(tm_k, tm_v, tm_q_run, tm_do_run, tm_dq, tm_dqacc, p);
   } else {
-    NSA_CUDA_OK(cudaFuncSetAttribute(tc_bwd_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    NSA_CUDA_OK(func_smem((const void*)tc_bwd_kernel<64>, smem));
     KernelScope ks(branch_name(kBwdNames, a.kind), st);
-    tc_bwd_kernel<64><<<grid, 512, smem, st>>>(tm_k, tm_v, tm_q, tm_do, tm_q_run, tm_do_run, tm_dq, tm_dqacc, p);
+    tc_bwd_kernel<64><<<grid, 512, smem, st>>>(tm_k, tm_v, tm_q_run, tm_do_run, tm_dq, tm_dqacc, p);
   }
   NSA_LAUNCH_OK("tc_bwd_kernel");
   if (a.kind == 2) {
     KernelScope ks("sel_split_blocks_kernel", st);
-    sel_split_blocks_kernel<<<dim3(pl.n_ktiles, a.B * a.Hkv), 256, 0, st>>>(p.offsets, p.dk_acc, p.dv_acc, p.dk, p.dv,
+    sel_split_blocks_kernel<<<dim3(pl.n_ktiles, a.B * a.Hkv), 256, 0, st>>>(p.plan.offsets, p.dk_acc, p.dv_acc, p.dk, p.dv,
                                                                         pl.n_ktiles, pl.nq, a.Lk, a.D, 1);
     NSA_LAUNCH_OK("sel_split_blocks_kernel");
   }
@@ -1474,11 +1407,11 @@ int tc_attn_bwd(const AttnArgs& a, void* ws, size_t ws_bytes, cudaStream_t st) {
   {
     KernelScope ks(branch_name(kRedNames, a.kind), st);
     if (a.D == 128)
-      dq_reduce_kernel<128><<<rgrid, 256, 0, st>>>(p.dq_part, pair_of_slot, (__nv_bfloat16*)a.dq, a.B, a.Hq,
+      dq_reduce_kernel<128><<<rgrid, 256, 0, st>>>(p.dq_part, p.plan.pair_of_slot, (__nv_bfloat16*)a.dq, a.B, a.Hq,
                                                   a.Hkv, a.T, G, a.kind, a.window, a.block_size, a.Lk,
                                                   pl.n_slots, a.S);
     else
-      dq_reduce_kernel<64><<<rgrid, 256, 0, st>>>(p.dq_part, pair_of_slot, (__nv_bfloat16*)a.dq, a.B, a.Hq,
+      dq_reduce_kernel<64><<<rgrid, 256, 0, st>>>(p.dq_part, p.plan.pair_of_slot, (__nv_bfloat16*)a.dq, a.B, a.Hq,
                                                  a.Hkv, a.T, G, a.kind, a.window, a.block_size, a.Lk,
                                                  pl.n_slots, a.S);
   }
@@ -1489,10 +1422,11 @@ int tc_attn_bwd(const AttnArgs& a, void* ws, size_t ws_bytes, cudaStream_t st) {
 
 // dq of the whole op from the three branch workspaces (each written by tc_attn_bwd with a null
 // dq) and / or the fp32 accumulator: `base` carries B, Hq, Hkv, T, D; a null workspace means the
-// branch is absent (or sits in the accumulator).
+// branch is absent (or sits in the accumulator).  pos: the pair map of the selection branch where it
+// is not the one inside ws_slc.
 int tc_dq_reduce3(const AttnArgs& base, int Lk_cmp, int cmp_len, int cmp_stride, int S, int block_size,
                   int window, const void* ws_cmp, const void* ws_slc, const void* ws_win,
-                  const float* dq_acc, void* dq, cudaStream_t st) {
+                  const int32_t* pos, const float* dq_acc, void* dq, cudaStream_t st) {
   using namespace tc;
   Reduce3Args r;
   r.acc = dq_acc;
@@ -1512,7 +1446,7 @@ int tc_dq_reduce3(const AttnArgs& base, int Lk_cmp, int cmp_len, int cmp_stride,
     AttnArgs a = base; a.kind = 2; a.Lk = base.T; a.S = S; a.block_size = block_size;
     const BwdPlan pl = plan_bwd(a);
     r.part_slc = (const __nv_bfloat16*)((const char*)ws_slc + pl.off_part);
-    r.pair_of_slot = (const int32_t*)((const char*)ws_slc + pl.off_pos);
+    r.pair_of_slot = pos ? pos : sel_plan_at((const char*)ws_slc + pl.off_plan, pl.layout).pair_of_slot;
   }
   if (ws_win) {
     AttnArgs a = base; a.kind = 0; a.Lk = base.T; a.window = window;

@@ -5,7 +5,7 @@
 
 #include <cuda.h>   // CUtensorMap (types only; the encode entry point is fetched at run time)
 
-#include "common.cuh"
+#include "sel_plan.cuh"
 
 namespace nsa {
 namespace tc {
@@ -82,14 +82,6 @@ __device__ __forceinline__ bool mbar_wait_drain(uint64_t* bar, uint32_t parity) 
     if (clock64() - start > kDrainLimitCycles) return false;
   return true;
 }
-
-// ---- selection work list -----------------------------------------------------------------------
-// The block-outer selection kernels take one work item per CTA: a 64-token block of one
-// (batch, kv head) and a chunk of at most kSelChunkTiles of its row tiles.  A block that many
-// queries list (an attention-sink block, a forced initial block) becomes several items, so no
-// single CTA walks its whole query list.
-constexpr int kSelChunkTiles = 128;
-struct SelWorkHeader { int n_items; int pad[63]; };   // 256 bytes in front of the int4 items
 
 // ---- TMA -------------------------------------------------------------------------------------
 __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* tm, uint64_t* bar, int c0,
@@ -320,15 +312,12 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 }
 
 // ---- which selection-forward variant does the work ------------------------------------------
-// stats[0] = number of (query tile, distinct block) pairs of the query-outer kernel.
-// The query-outer kernel runs one 64-key tile per such pair; this kernel runs one row tile per
-// nq (query, block) pairs, at about three times the cost of a query-outer tile.
-__device__ __forceinline__ bool prefer_pairs(const unsigned long long* stats, const int32_t* offsets,
-                                             int units, int n_ktiles, int nq, int force) {
+// The query-outer kernel runs one 64-key tile per (query tile, distinct key tile) pair; the
+// block-outer kernel runs one row tile per nq (query, key tile) pairs, at about three times the
+// cost of a query-outer tile.
+__device__ __forceinline__ bool prefer_pairs(const SelPlanHeader* hdr, int nq, int force) {
   if (force) return force == 2;
-  const unsigned long long union_tiles = stats[0];
-  const unsigned long long pairs = (unsigned long long)__ldg(offsets + (size_t)units * (n_ktiles + 1) - 1);
-  return union_tiles * (unsigned long long)nq > 3ull * pairs;
+  return __ldg(&hdr->union_tiles) * (unsigned long long)nq > 3ull * __ldg(&hdr->pairs);
 }
 
 // byte offset of element (row, col) inside a 128B-swizzled slab sequence; col in elements

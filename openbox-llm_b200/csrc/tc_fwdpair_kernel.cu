@@ -22,12 +22,9 @@ namespace nsa {
 namespace tc {
 
 struct PairArgs {
-  const int32_t* q_of_block;
-  const int32_t* offsets;        // [B*Hkv, n_ktiles + 1]
+  SelPlan plan;
   __nv_bfloat16* o_part;         // [pairs, G, D]
   float* ml;                     // [pairs, G, 2]: the row maximum m and the sum of p
-  const unsigned long long* stats;
-  const SelWorkHeader* work;     // n_items, then int4 items {bh, block, first row tile, chunks of the block}
   int* status;
   int force;                     // 0: device-side choice, 1: query-outer kernel, 2: this kernel
   int B, Hq, Hkv, T, G, nq, n_ktiles, nq_union;
@@ -95,14 +92,14 @@ tc_fwdpair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
   volatile int* s_issued = (volatile int*)(s_tmem + 2);   // row tiles whose gather has been issued
   uint32_t* s_prow = (uint32_t*)(s_tmem + 4);             // [128] partial row of each tile row (ragged tile)
 
-  if (!prefer_pairs(p.stats, p.offsets, p.B * p.Hkv, p.n_ktiles, p.nq_union, p.force)) return;
-  if ((int)blockIdx.x >= p.work->n_items) return;
-  const int4 item = reinterpret_cast<const int4*>(p.work + 1)[blockIdx.x];
+  if (!prefer_pairs(p.plan.hdr, p.nq_union, p.force)) return;
+  if ((int)(blockIdx.x % p.plan.max_items) >= p.plan.n_items[blockIdx.x / p.plan.max_items]) return;
+  const int4 item = p.plan.items[blockIdx.x];
   const int bh = item.x, j = item.y;
   const int b = bh / p.Hkv, hkv = bh % p.Hkv;
   const int key0 = j * kKeys;
-  const int pair_base = __ldg(p.offsets + (size_t)bh * (p.n_ktiles + 1) + j);
-  const int n_q = __ldg(p.offsets + (size_t)bh * (p.n_ktiles + 1) + j + 1) - pair_base;
+  const int pair_base = __ldg(p.plan.offsets + (size_t)bh * (p.n_ktiles + 1) + j);
+  const int n_q = __ldg(p.plan.offsets + (size_t)bh * (p.n_ktiles + 1) + j + 1) - pair_base;
   const int rt_end = min((n_q + p.nq - 1) / p.nq, item.z + kSelChunkTiles);
   const int n_tiles = rt_end - item.z;              // row tiles of this work item
   if (n_tiles <= 0) return;
@@ -163,7 +160,7 @@ tc_fwdpair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
     // query position of one of this lane's boxes in tile k (a missing query reads past T: zeros)
     auto tq_of = [&](int k, int o) -> int {
       const int qi = (item.z + k) * p.nq + o / per_q;
-      return (o < n_ops && qi < n_q) ? ldg_s32_now(p.q_of_block + pair_base + qi) : p.T;
+      return (o < n_ops && qi < n_q) ? (int)(ldg_s32_now(p.plan.pairs + pair_base + qi) & kPairPosMask) : p.T;
     };
     int tq0 = tq_of(0, o0), tq1 = tq_of(0, o1);
     for (int k = 0; k < n_tiles; ++k) {
@@ -248,7 +245,7 @@ tc_fwdpair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
     auto row_query = [&](int k) -> int {
       const int qi = (item.z + k) * p.nq + ql;
       if (!row_slot_ok || qi >= n_q) return -1;
-      return ldg_s32_now(p.q_of_block + pair_base + qi);
+      return (int)(ldg_s32_now(p.plan.pairs + pair_base + qi) & kPairPosMask);
     };
     int t_cur = sb < n_tiles ? row_query(sb) : -1;
     for (int k = sb; k < n_tiles; k += 2) {
@@ -386,15 +383,13 @@ tc_fwdpair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
 int get_option_merged_boxes();   // api.cu
 
 // launched by tc_sel_fwd (tc_fwdpair.cu)
-int tc_fwdpair_launch(const AttnArgs& a, const int32_t* q_of_block, const int32_t* offsets, void* o_part,
-                       float* ml, const unsigned long long* stats, const void* work, int force, int nq,
-                       int n_ktiles, int nq_union, size_t cap_pairs, unsigned grid, cudaStream_t st) {
+int tc_fwdpair_launch(const AttnArgs& a, const SelPlan& plan, void* o_part, float* ml, int force, int nq,
+                      int n_ktiles, int nq_union, size_t cap_pairs, unsigned grid, cudaStream_t st) {
   using namespace tc;
   const int G = a.Hq / a.Hkv;
   PairArgs p;
-  p.q_of_block = q_of_block; p.offsets = offsets;
-  p.o_part = (__nv_bfloat16*)o_part; p.ml = ml; p.stats = stats;
-  p.work = (const SelWorkHeader*)work;
+  p.plan = plan;
+  p.o_part = (__nv_bfloat16*)o_part; p.ml = ml;
   p.status = device_status_ptr();
   if (!p.status) { set_error("device status word unavailable"); return NSA_ERR_CUDA; }
   p.force = force;
@@ -412,10 +407,10 @@ int tc_fwdpair_launch(const AttnArgs& a, const int32_t* q_of_block, const int32_
   const size_t smem = pair_smem_bytes(a.D);
   KernelScope ks("tc_fwd_slc_pairs", st);
   if (a.D == 128) {
-    NSA_CUDA_OK(cudaFuncSetAttribute(tc_fwdpair_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    NSA_CUDA_OK(func_smem((const void*)tc_fwdpair_kernel<128>, smem));
     tc_fwdpair_kernel<128><<<grid, kPairThreads, smem, st>>>(tm_k, tm_v, tm_q, tm_o, p);
   } else {
-    NSA_CUDA_OK(cudaFuncSetAttribute(tc_fwdpair_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    NSA_CUDA_OK(func_smem((const void*)tc_fwdpair_kernel<64>, smem));
     tc_fwdpair_kernel<64><<<grid, kPairThreads, smem, st>>>(tm_k, tm_v, tm_q, tm_o, p);
   }
   NSA_LAUNCH_OK("tc_fwdpair_kernel");

@@ -543,10 +543,10 @@ static int launch_score_lanes(const void* q, const void* k_cmp, const NsaDims& d
   const size_t smem = score_lanes_smem_bytes(d.D);
   KernelScope ks("tc_score_topn", st);
   if (p.r == 1 && p.overlap == 0) {
-    NSA_CUDA_OK(cudaFuncSetAttribute(tc_score_lanes_kernel<D, GP, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    NSA_CUDA_OK(func_smem((const void*)tc_score_lanes_kernel<D, GP, true>, smem));
     tc_score_lanes_kernel<D, GP, true><<<dim3(p.n_qtiles, d.B * d.Hkv), 128, smem, st>>>(tm_q, tm_k, p);
   } else {
-    NSA_CUDA_OK(cudaFuncSetAttribute(tc_score_lanes_kernel<D, GP, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    NSA_CUDA_OK(func_smem((const void*)tc_score_lanes_kernel<D, GP, false>, smem));
     tc_score_lanes_kernel<D, GP, false><<<dim3(p.n_qtiles, d.B * d.Hkv), 128, smem, st>>>(tm_q, tm_k, p);
   }
   return NSA_OK;
@@ -602,11 +602,11 @@ int tc_topn(const void* q, const void* k_cmp, const float* lse, int32_t* block_i
   const size_t smem = score_smem_bytes(d.D, p.nq);
   dim3 grid(p.n_qtiles, d.B * d.Hkv);
   if (d.D == 128) {
-    NSA_CUDA_OK(cudaFuncSetAttribute(tc_score_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    NSA_CUDA_OK(func_smem((const void*)tc_score_kernel<128>, smem));
     KernelScope ks("tc_score_topn", st);
     tc_score_kernel<128><<<grid, 128, smem, st>>>(tm_q, tm_k, p);
   } else {
-    NSA_CUDA_OK(cudaFuncSetAttribute(tc_score_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    NSA_CUDA_OK(func_smem((const void*)tc_score_kernel<64>, smem));
     KernelScope ks("tc_score_topn", st);
     tc_score_kernel<64><<<grid, 128, smem, st>>>(tm_q, tm_k, p);
   }

@@ -11,6 +11,9 @@ Names, argument meaning and error behaviour follow the reference modules they re
 `nsa_attention` is the one addition: the whole op (pooling, compression attention, block
 scoring + top-n, selection, window, gate) behind one autograd.Function.
 """
+import ctypes
+import functools
+
 import torch
 
 from . import _lib as L
@@ -53,6 +56,7 @@ def get_dq_accumulator() -> bool:
 def set_option(name: str, value: int):
     """Library tuning switch (see nsa_set_option in include/nsa_b200.h)."""
     L.check(L.lib().nsa_set_option(name.encode(), int(value)))
+    _op_desc.cache_clear()            # workspace sizes depend on the switches
 
 
 def tc_supported(B, Hq, Hkv, T, D, dtype, block_size=64) -> bool:
@@ -536,12 +540,71 @@ def heads_to_tokens(x):
 
 def nsa_fused_forward(q, kc, vc, ks, vs, kw, vw, gate_logits, block_idx, block_size, window):
     """nsa_fused_kernel.py:560-573: the three branches with a given block_idx, mean pooling."""
-    k_cmp = block_mean_pool(kc, block_size)
-    v_cmp = block_mean_pool(vc, block_size)
-    o_cmp = compression_attn_triton(q, k_cmp, v_cmp, block_size)
-    o_slc = selection_attn_triton(q, ks, vs, block_idx, block_size)
-    o_win = window_attn_triton(q, kw, vw, window)
-    return gate_combine(o_cmp, o_slc, o_win, gate_logits)
+    bs = int(block_size)
+    return _op(q, (kc, vc, ks, vs, kw, vw), gate_logits, block_idx, bs, 0, window, (0, 0, bs, bs), None)[0]
+
+
+@functools.lru_cache(maxsize=512)
+def _op_desc(B, Hq, Hkv, T, D, dtype, block_size, n_sel, window, n_init, n_local, cmp_len, cmp_stride, learned,
+             given_lists, need_grad, dq_accumulator, impl):
+    """Descriptor of a whole-op call and the bytes it keeps and needs (saved, forward, backward)."""
+    d = L.NsaAttentionDesc(L.dims(B, Hq, Hkv, T, D, dtype), block_size, n_sel, window, n_init, n_local, cmp_len,
+                           cmp_stride, int(learned), int(given_lists), int(need_grad), int(dq_accumulator), impl)
+    sizes = [ctypes.c_size_t() for _ in range(3)]
+    L.check(L.lib().nsa_attention_sizes(d, *sizes))
+    return (d, *(x.value for x in sizes))
+
+
+def _op_forward(q, kv, gate_logits, block_idx, block_size, n_sel, window, forced, comp, need_grad):
+    """Forward of the whole op: (out, block_idx, what backward needs).  forced = (n_init, n_local,
+    summary length, summary stride); comp: the six compressor parameters, or None for mean pooling."""
+    B, Hq, T, D = q.shape
+    Hkv = kv[0].shape[1]
+    dtype = L.dtype_code(q)
+    assert q.is_cuda, "libnsa_b200 needs CUDA tensors; there is no CPU path"
+    assert Hq % Hkv == 0, "GQA needs Hq divisible by Hkv"
+    assert D in (16, 32, 64, 128), "head dim must be a power of two <= 128"
+    assert block_size >= 16, "block_size must be >= 16 (tl.dot inner dim)"
+    shape, dev = (B, Hkv, T, D), q.device
+    tensors = [q]
+    for t in kv:
+        assert t.shape == shape and t.dtype == q.dtype
+        tensors.append(t)
+    gate = gate_logits if gate_logits.dtype == q.dtype else gate_logits.to(q.dtype)
+    tensors.append(gate)
+    given = block_idx is not None
+    if given:
+        assert block_idx.shape[:3] == (B, Hkv, T)
+        n_sel = block_idx.shape[3]
+        block_idx = block_idx.to(torch.int32).contiguous()
+        tensors.append(block_idx)
+    cp = [] if comp is None else [t.detach().float().contiguous() for t in comp]
+    for t in (*tensors, *cp):
+        if t.device != dev:
+            raise L.NsaError(f"libnsa_b200: tensors on different devices ({dev} and {t.device})")
+    if comp is None:
+        assert forced[2] == forced[3] == block_size, "mean pooling is defined on the aligned grid only"
+    if torch.cuda.current_device() != dev.index:
+        with torch.cuda.device(dev):
+            return _op_forward(q, kv, gate_logits, block_idx, block_size, n_sel, window, forced, comp, need_grad)
+    tensors = [t if t.is_contiguous() else t.contiguous() for t in tensors[:8]]
+    if not given:
+        block_idx = torch.empty(B, Hkv, T, n_sel, device=dev, dtype=torch.int32)
+    desc, saved_bytes, fwd_bytes, bwd_bytes = _op_desc(
+        B, Hq, Hkv, T, D, dtype, int(block_size), int(n_sel), int(window), *forced, comp is not None, given, need_grad,
+        _dq_accumulator, L.IMPL[_impl])
+    out = torch.empty(B, Hq, T, D, device=dev, dtype=q.dtype)
+    saved = torch.empty(saved_bytes + (0 if need_grad else fwd_bytes) + 1, device=dev, dtype=torch.uint8)
+    ws, ws_ptr = None, saved.data_ptr() + saved_bytes
+    if need_grad and fwd_bytes:
+        ws = L.workspace(fwd_bytes, dev)
+        ws_ptr = ws.data_ptr()
+    ptrs = L.OP_TENSORS(*[t.data_ptr() for t in tensors], *([t.data_ptr() for t in cp] or (None,) * 6),
+                        block_idx.data_ptr(), out.data_ptr())
+    L.check(L.lib().nsa_attention_fwd(desc, ptrs, saved.data_ptr(), ws_ptr, fwd_bytes, L.raw_stream(dev)))
+    if L.CHECK_STATUS_EVERY_CALL:
+        L.check_device_status()
+    return out, block_idx, (tensors, cp, saved, desc, bwd_bytes)
 
 
 class _NSAAttention(torch.autograd.Function):
@@ -549,118 +612,50 @@ class _NSAAttention(torch.autograd.Function):
     top-n -> selection attention -> window attention -> gate combine.  Saves q once."""
 
     @staticmethod
-    @L.on_device
-    def forward(ctx, q, kc, vc, ks, vs, kw, vw, gate_logits, block_size, n_sel, window,
-                block_idx, forced, k_intra, k_logits, k_proj, v_intra, v_logits, v_proj):
-        learned = k_intra is not None
-        n_init, n_local, cl, cs = forced          # cl, cs: length and stride of the summaries
-        if learned:
-            cp = [t.detach().float().contiguous() for t in
-                  (k_intra, k_logits, k_proj, v_intra, v_logits, v_proj)]
-            k_cmp = _compress_fwd(kc, cp[0], cp[1], cp[2], cl, cs)
-            v_cmp = _compress_fwd(vc, cp[3], cp[4], cp[5], cl, cs)
-        else:
-            assert cl == cs == block_size, "mean pooling is defined on the aligned grid only"
-            cp = []
-            k_cmp = _mean_pool_fwd(kc, block_size)
-            v_cmp = _mean_pool_fwd(vc, block_size)
-        # the three branches' outputs and softmax statistics live in one tensor each
-        q = q.contiguous()
-        o3 = torch.empty((3,) + tuple(q.shape), device=q.device, dtype=q.dtype)
-        lse3 = torch.empty((3,) + tuple(q.shape[:3]), device=q.device, dtype=torch.float32)
-        o_cmp, lse_cmp = range_attn_forward(q, k_cmp, v_cmp, MODE_COMPRESS_STRIDED, cs, cl, out=(o3[0], lse3[0]))
-        if block_idx is None:
-            block_idx = topn_blocks(q, k_cmp, lse_cmp, block_size, n_sel, n_init_blocks=n_init,
-                                    n_local_blocks=n_local, cmp_len=cl, cmp_stride=cs)
-        else:
-            block_idx = block_idx.to(torch.int32).contiguous()
-        # CSR, pair map and work list of the block list: built once, used by forward and backward
-        plan = selection_plan(q, ks, block_idx, block_size) if q.dtype == torch.bfloat16 else None
-        o_slc, _ = selection_forward_triton(q, ks, vs, block_idx, block_size, return_lse=True,
-                                            out=(o3[1], lse3[1]), plan=plan)
-        o_win, _ = range_attn_forward(q, kw, vw, MODE_WINDOW, window, 0, out=(o3[2], lse3[2]))
-        gate = gate_logits.to(q.dtype).contiguous()
-        out = _gate_fwd(o_cmp, o_slc, o_win, gate)
-        ctx.save_for_backward(q, kc, vc, ks, vs, kw, vw, gate, k_cmp, v_cmp, o3, lse3, block_idx, *cp)
-        ctx.sel_plan = plan          # (an opaque byte buffer: kept on the context, not a differentiable input)
-        ctx.cfg = (block_size, window, learned, gate_logits.dtype,
-                   tuple(t.dtype for t in (k_intra, k_logits, k_proj, v_intra, v_logits, v_proj))
-                   if learned else None, cl, cs)
+    def forward(ctx, q, kc, vc, ks, vs, kw, vw, gate_logits, block_size, n_sel, window, block_idx, forced, *comp):
+        out, block_idx, (tensors, cp, saved, desc, bwd_bytes) = _op_forward(
+            q, (kc, vc, ks, vs, kw, vw), gate_logits, block_idx, block_size, n_sel, window, forced, comp or None, True)
+        ctx.save_for_backward(*tensors, block_idx, saved, *cp)
+        ctx.cfg = (desc, bwd_bytes, gate_logits.dtype, tuple(t.dtype for t in comp))
         ctx.mark_non_differentiable(block_idx)
-        if L.CHECK_STATUS_EVERY_CALL:
-            L.check_device_status()
+        ctx.set_materialize_grads(False)
         return out, block_idx
 
     @staticmethod
-    @L.on_device
     def backward(ctx, d_out, _d_idx):
-        (q, kc, vc, ks, vs, kw, vw, gate, k_cmp, v_cmp, o3, lse3, block_idx, *cp) = ctx.saved_tensors
-        (o_cmp, o_slc, o_win), (lse_cmp, lse_slc, lse_win) = o3, lse3
-        block_size, window, learned, gate_dtype, pdt, cl, cs = ctx.cfg
-        T = q.shape[2]
-        # gate backward as per-row statistics; the branch kernels apply the gate factor themselves
-        B, Hq = q.shape[0], q.shape[1]
+        desc, bwd_bytes, gate_dtype, comp_dtypes = ctx.cfg
+        if d_out is None:
+            return (None,) * (13 + len(comp_dtypes))
+        kept = ctx.saved_tensors
+        tensors, block_idx, saved, cp = kept[:8], kept[8], kept[9], kept[10:]
+        dev = saved.device
+        if torch.cuda.current_device() != dev.index:
+            with torch.cuda.device(dev):
+                return _NSAAttention.backward(ctx, d_out, _d_idx)
+        if d_out.device != dev:
+            raise L.NsaError(f"libnsa_b200: tensors on different devices ({dev} and {d_out.device})")
+        assert d_out.dtype == tensors[0].dtype
         d_out = d_out.contiguous()
-        rs = torch.empty(3, B, Hq, T, device=q.device, dtype=torch.float32)
-        rd = torch.empty(3, B, Hq, T, device=q.device, dtype=torch.float32)
-        d_gate = torch.empty_like(gate)
-        L.check(L.lib().nsa_gate_combine_bwd_rows(
-            L.ptr(o_cmp), L.ptr(o_slc), L.ptr(o_win), L.ptr(gate), L.ptr(d_out), L.ptr(rs), L.ptr(rd),
-            L.ptr(d_gate), L.dims(B, Hq, 1, T, q.shape[3], L.dtype_code(q)), L.stream()))
-        S = block_idx.shape[-1]
-        # tcgen05 shapes: the three branches leave their dQ partials in their workspaces and one
-        # kernel adds them all; otherwise three dq tensors and a sum
-        fused = (_impl != "simt" and S > 0 and q.dtype == torch.bfloat16 and
-                 tc_supported(B, Hq, ks.shape[1], T, q.shape[3], q.dtype, block_size))
-        dq_sum = torch.empty_like(q)
-        dm = L.dims(B, Hq, ks.shape[1], T, q.shape[3], L.dtype_code(q))
-        n_cmp = k_cmp.shape[2]
-        if fused and _dq_accumulator:
-            # window and compression add their dQ into one fp32 accumulator; only the selection
-            # branch keeps partials (its rows are gathered, the adds would miss L2)
-            G = Hq // ks.shape[1]
-            dq_acc = torch.zeros(B * ks.shape[1], T, G, q.shape[3], device=q.device, dtype=torch.float32)
-            if n_cmp > 0:
-                dk_cmp, dv_cmp = range_attn_backward_acc(q, k_cmp, v_cmp, o_cmp, lse_cmp, d_out,
-                                                         MODE_COMPRESS_STRIDED, cs, cl, rs[0], rd[0], dq_acc)
-            else:
-                dk_cmp, dv_cmp = torch.zeros_like(k_cmp), torch.zeros_like(v_cmp)
-            dkw, dvw = range_attn_backward_acc(q, kw, vw, o_win, lse_win, d_out, MODE_WINDOW, window, 0,
-                                               rs[2], rd[2], dq_acc)
-            ws2, dks, dvs = _selection_backward(q, ks, vs, block_idx, block_size, d_out, o_slc, lse_slc,
-                                                rs[1], rd[1], defer_dq=True, plan=ctx.sel_plan)
-            L.check(L.lib().nsa_dq_finish(dm, S, int(block_size), L.ptr(dq_acc), L.ptr(ws2), L.ptr(dq_sum),
-                                          L.stream()))
-            del ws2, dq_acc
-        else:
-            dq, dk_cmp, dv_cmp = range_attn_backward(q, k_cmp, v_cmp, o_cmp, lse_cmp, d_out,
-                                                     MODE_COMPRESS_STRIDED, cs, cl, rs[0], rd[0],
-                                                     defer_dq=fused)
-            dq2, dks, dvs = _selection_backward(q, ks, vs, block_idx, block_size, d_out, o_slc, lse_slc,
-                                                rs[1], rd[1], defer_dq=fused, plan=ctx.sel_plan)
-            dq3, dkw, dvw = range_attn_backward(q, kw, vw, o_win, lse_win, d_out, MODE_WINDOW, window, 0,
-                                                rs[2], rd[2], defer_dq=fused)
-            if fused:
-                L.check(L.lib().nsa_dq_reduce3(dm, n_cmp, int(cl), int(cs), S, int(block_size), int(window),
-                                               L.ptr(dq) if n_cmp > 0 else None, L.ptr(dq2), L.ptr(dq3),
-                                               L.ptr(dq_sum), L.stream()))
-            else:
-                L.check(L.lib().nsa_sum3(L.ptr(dq), L.ptr(dq2), L.ptr(dq3), L.ptr(dq_sum), dq.numel(),
-                                         L.dtype_code(dq), L.stream()))
-            del dq, dq2, dq3
-        dq = dq_sum
-        pgrads = [None] * 6
-        if learned:
-            dkc, a, b, c = _compress_bwd(kc, cp[0], cp[1], cp[2], dk_cmp, cl, cs)
-            dvc, d, e, f = _compress_bwd(vc, cp[3], cp[4], cp[5], dv_cmp, cl, cs)
-            pgrads = [g.to(t) for g, t in zip((a, b, c, d, e, f), pdt)]
-        else:
-            dkc = _mean_pool_bwd(dk_cmp, T, block_size)
-            dvc = _mean_pool_bwd(dv_cmp, T, block_size)
+        grads = [torch.empty_like(t) for t in tensors]
+        d_cp = [torch.empty_like(t) for t in cp]
+        ws = L.workspace(bwd_bytes, dev)
+        ptrs = L.OP_TENSORS(*[t.data_ptr() for t in tensors], *([t.data_ptr() for t in cp] or (None,) * 6),
+                            block_idx.data_ptr(), None, d_out.data_ptr(), *[t.data_ptr() for t in grads],
+                            *[t.data_ptr() for t in d_cp])
+        L.check(L.lib().nsa_attention_bwd(desc, ptrs, saved.data_ptr(), ws.data_ptr(), bwd_bytes, L.raw_stream(dev)))
         if L.CHECK_STATUS_EVERY_CALL:
             L.check_device_status()
-        return (dq, dkc, dvc, dks, dvs, dkw, dvw, d_gate.to(gate_dtype), None, None, None, None, None,
-                *pgrads)
+        if gate_dtype != d_out.dtype:
+            grads[7] = grads[7].to(gate_dtype)
+        d_cp = [g if g.dtype == t else g.to(t) for g, t in zip(d_cp, comp_dtypes)]
+        return (*grads, None, None, None, None, None, *d_cp)
+
+
+def _op(q, kv, gate_logits, block_idx, block_size, n_sel, window, forced, comp):
+    """The whole op, through autograd only where a gradient is asked for."""
+    if torch.is_grad_enabled() and any(t.requires_grad for t in (q, *kv, gate_logits, *(comp or ()))):
+        return _NSAAttention.apply(q, *kv, gate_logits, block_size, n_sel, window, block_idx, forced, *(comp or ()))
+    return _op_forward(q, kv, gate_logits, block_idx, block_size, n_sel, window, forced, comp, False)[:2]
 
 
 @torch.no_grad()
@@ -702,11 +697,11 @@ def nsa_attention(q, kc, vc, ks, vs, kw, vw, gate_logits, block_size, n_sel, win
     selection blocks; the compressor parameters then have cmp_len positions.
     With NSA_B200_CHECK_STATUS=1 in the environment the device status word is read (one stream
     synchronisation) after every forward and backward and a give-up raises NsaError."""
-    cp = [None] * 6
+    cp = None
     if compressor is not None:
-        cp = [compressor[n] for n in ("k_intra", "k_logits", "k_proj", "v_intra", "v_logits", "v_proj")]
+        cp = tuple(compressor[n] for n in ("k_intra", "k_logits", "k_proj", "v_intra", "v_logits", "v_proj"))
     cl = int(block_size if cmp_len is None else cmp_len)
     cs = int(cl if cmp_stride is None else cmp_stride)
-    out, idx = _NSAAttention.apply(q, kc, vc, ks, vs, kw, vw, gate_logits, block_size, n_sel,
-                                   window, block_idx, (int(n_init_blocks), int(n_local_blocks), cl, cs), *cp)
+    out, idx = _op(q, (kc, vc, ks, vs, kw, vw), gate_logits, block_idx, block_size, n_sel, window,
+                   (int(n_init_blocks), int(n_local_blocks), cl, cs), cp)
     return (out, idx) if return_block_idx else out
