@@ -136,7 +136,7 @@ bool use_tc(const NsaDims* d, int block_size, int impl, int* err) {
   if (impl == NSA_IMPL_SIMT) return false;
   const bool ok = tc_shape_ok(*d, block_size);
   if (impl == NSA_IMPL_TC && !ok) {
-    set_error("shape not served by the tcgen05 kernels (bf16, D in {64,128}, 64-token blocks, 2 to 128 query heads per kv head)");
+    set_error("shape not served by the tcgen05 kernels (bf16, D in {64,128}, blocks of 16, 32 or 64 tokens, 2 to 128 query heads per kv head)");
     *err = NSA_ERR_UNSUPPORTED;
   }
   return ok;

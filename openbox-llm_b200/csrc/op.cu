@@ -272,9 +272,12 @@ extern "C" int nsa_attention_fwd(const NsaAttentionDesc* d, const NsaAttentionTe
   NSA_TRY(nsa_range_attn_fwd(t->q, k_cmp, v_cmp, o[0], lse[0], &m, p.n_cmp, NSA_MODE_COMPRESS_STRIDED, d->cmp_stride,
                              d->cmp_len, d->impl, stream));
   if (!d->given_lists) {
+    // impl chooses the attention kernels; lists longer than the tensor-core scorer keeps (16) are scored
+    // on the CUDA cores even where it names the former
     if (p.S > 0)
       NSA_TRY(nsa_topn_blocks_general(t->q, k_cmp, lse[0], t->block_idx, nullptr, &m, p.n_cmp, d->cmp_len, d->cmp_stride,
-                                      d->block_size, p.S, d->n_init, d->n_local, d->impl, stream));
+                                      d->block_size, p.S, d->n_init, d->n_local,
+                                      d->impl == NSA_IMPL_TC ? NSA_IMPL_AUTO : d->impl, stream));
     if (plan && !p.fwd_ws) {      // only the backward reads the plan: it is built beside the forward kernel
       NSA_TRY(fork.begin());
       NSA_TRY(nsa_selection_plan_build(t->block_idx, &m, p.S, d->block_size, plan, p.plan_bytes, fork.stream(1)));

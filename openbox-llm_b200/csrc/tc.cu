@@ -5,8 +5,8 @@
 // share every K/V tile.  The CTA walks a list of 64-key tiles:
 //   window      the tiles covering [t_first - W + 1, t_last]
 //   compression the tiles covering summaries [0, (t_last + 1) / Bsz - 1]
-//   selection   the union of the 64-token blocks listed for the tile's nq queries, built in
-//               shared memory, with a per-(query, block) membership bit
+//   selection   the 64-key tiles holding blocks (of 16, 32 or 64 tokens) listed for the tile's nq
+//               queries, found in shared memory, with a membership bit per (query, block)
 // Per tile: a TMA warp brings K and V (128B-swizzled boxes) into a 2-stage ring; an MMA warp
 // issues S = Q K^T (tcgen05.mma, Q held in TMEM as the A operand, accumulator in TMEM); each of
 // the 128 softmax threads owns one row of S (tcgen05.ld, lane = row), masks it, runs the online
@@ -32,8 +32,9 @@ struct FwdArgs {
   const SelPlanHeader* plan;         // selection: statistics for the variant choice (null: this kernel serves the call)
   int force;
   int debug_starve;          // test only: the V load of the second key tile is never sent
-  int n_qtiles, nb_sel;      // nb_sel = ceil(T / 64) blocks a selection list may name
+  int n_qtiles, nb_sel;      // nb_sel = ceil(T / 64) key tiles a selection list may name
   int nw;                    // 32-bit membership words per block = max(1, nq / 32)
+  int n_sub;                 // selection: list blocks per 64-key tile (64 / block_size)
   float scale_log2;
 };
 
@@ -44,10 +45,10 @@ template <int D> struct FwdSmem {
   static constexpr int kFixed = kQBytes + 4 * kKVBytes;   // Q + 2 K stages + 2 V stages
 };
 
-__host__ __device__ inline size_t fwd_smem_bytes(int D, int nb_sel, int nw, int kind) {
+__host__ __device__ inline size_t fwd_smem_bytes(int D, int nb_sel, int nw, int n_sub, int kind) {
   size_t fixed = (size_t)(kRows * 128 + 4 * kKeys * 128) * (D / 64);
   size_t extra = 256 /*barriers etc*/ + 132 * 4 /*scan*/;
-  if (kind == 2) extra += (size_t)nb_sel * nw * 4 + (size_t)nb_sel * 2 + 16;
+  if (kind == 2) extra += (size_t)nb_sel * n_sub * nw * 4 + (size_t)nb_sel * 2 + 16;
   return fixed + extra + 1024 /*alignment slack*/;
 }
 
@@ -93,8 +94,9 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   volatile int* s_abort = (volatile int*)(s_tmem + 1);
   int* s_ntiles = (int*)(s_tmem + 2);
   int* s_scan = (int*)(s_tmem + 4);                 // [129]
-  uint32_t* s_member = (uint32_t*)(s_scan + 132);   // [nb_sel * nw]   (selection only)
-  uint16_t* s_tiles = (uint16_t*)(s_member + (p.kind == 2 ? p.nb_sel * p.nw : 0));
+  uint32_t* s_member = (uint32_t*)(s_scan + 132);   // [nb_sel][n_sub][nw]   (selection only)
+  const int tile_words = p.n_sub * p.nw;
+  uint16_t* s_tiles = (uint16_t*)(s_member + (p.kind == 2 ? p.nb_sel * tile_words : 0));
 
   if (p.kind == 2 && p.plan != nullptr && prefer_pairs(p.plan, p.nq, p.force))
     return;   // the block-outer variant serves this call: leave before anything is set up
@@ -135,7 +137,7 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     const int hi_last = cmp_visible(t_last, p.block_size, p.window, p.Lk) - 1;   // window: the stride
     n_tiles = hi_last < 0 ? 0 : hi_last / kKeys + 1;
   } else {
-    const int nmem = p.nb_sel * p.nw;
+    const int nmem = p.nb_sel * tile_words;
     for (int i = tid; i < nmem; i += kFwdThreads) s_member[i] = 0u;
     __syncthreads();
     const int32_t* idx = p.block_idx + ((size_t)bh * p.T + t0) * p.S;
@@ -143,7 +145,8 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     for (int e = tid; e < n_entries; e += kFwdThreads) {
       const int q_local = e / p.S;
       const int blk = __ldg(idx + e);
-      if (blk >= 0 && blk < p.nb_sel && blk * kKeys <= t0 + q_local)
+      // list block blk = part blk % n_sub of key tile blk / n_sub
+      if (blk >= 0 && (long long)blk * p.block_size <= t0 + q_local)
         atomicOr(&s_member[blk * p.nw + (q_local >> 5)], 1u << (q_local & 31));
     }
     __syncthreads();
@@ -152,7 +155,7 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     int cnt = 0;
     for (int j = j0; j < j1; ++j) {
       uint32_t any = 0;
-      for (int w = 0; w < p.nw; ++w) any |= s_member[j * p.nw + w];
+      for (int w = 0; w < tile_words; ++w) any |= s_member[j * tile_words + w];
       cnt += any != 0;
     }
     if (tid < 128) s_scan[tid + 1] = cnt;
@@ -166,7 +169,7 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     int pos = tid < 128 ? s_scan[tid] : 0;
     for (int j = j0; j < j1; ++j) {
       uint32_t any = 0;
-      for (int w = 0; w < p.nw; ++w) any |= s_member[j * p.nw + w];
+      for (int w = 0; w < tile_words; ++w) any |= s_member[j * tile_words + w];
       if (any) s_tiles[pos++] = (uint16_t)j;
     }
     __syncthreads();
@@ -312,6 +315,7 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
 
       // valid columns of this row in this tile form one range [lo, hi]
       int lo = 0, hi = -1;
+      uint32_t groups = 0xfu;              // 16-column groups of the tile the row attends
       if (row_ok) {
         if (p.kind == 0) {
           lo = max(0, t - p.window + 1 - key0);
@@ -319,13 +323,20 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         } else if (p.kind == 1) {
           hi = min(kKeys - 1, cmp_visible(t, p.block_size, p.window, p.Lk) - 1 - key0);
         } else {
-          const uint32_t w = s_member[(key0 / kKeys) * p.nw + (ql >> 5)];
-          if ((w >> (ql & 31)) & 1u) hi = min(kKeys - 1, t - key0);
+          hi = min(kKeys - 1, t - key0);
+          const uint32_t* mem = s_member + (key0 / kKeys) * tile_words + (ql >> 5);
+          if (p.n_sub == 1) {
+            if (!((mem[0] >> (ql & 31)) & 1u)) hi = -1;
+          } else {
+            groups = 0u;
+            for (int k = 0; k < p.n_sub; ++k)
+              if ((mem[k * p.nw] >> (ql & 31)) & 1u) groups |= ((1u << (p.block_size >> 4)) - 1u) << (k * (p.block_size >> 4));
+          }
         }
       }
       float x[64];
       float tmax = -INFINITY;
-      if (lo <= 0 && hi >= kKeys - 1) {
+      if (lo <= 0 && hi >= kKeys - 1 && groups == 0xfu) {
 #pragma unroll
         for (int c = 0; c < 64; ++c) {
           x[c] = __uint_as_float(r[c]) * p.scale_log2;
@@ -334,7 +345,7 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       } else {
 #pragma unroll
         for (int c = 0; c < 64; ++c) {
-          x[c] = (c >= lo && c <= hi) ? __uint_as_float(r[c]) * p.scale_log2 : -INFINITY;
+          x[c] = (c >= lo && c <= hi && ((groups >> (c >> 4)) & 1u)) ? __uint_as_float(r[c]) * p.scale_log2 : -INFINITY;
           tmax = fmaxf(tmax, x[c]);
         }
       }
@@ -814,14 +825,14 @@ static const char* const kFwdNames[3] = {"tc_fwd_win", "tc_fwd_cmp", "tc_fwd_slc
 bool tc_shape_ok(const NsaDims& d, int block_size) {
   if (d.dtype != NSA_DTYPE_BF16) return false;
   if (d.D != 64 && d.D != 128) return false;
-  if (block_size != tc::kKeys) return false;
+  if (block_size != 16 && block_size != 32 && block_size != tc::kKeys) return false;   // whole 16-column groups of a key tile
   const int G = d.Hq / d.Hkv;
   if (G < 2 || G > 128) return false;   // the backward tiles hold at most 64 queries
   if (d.T < 1) return false;
   const int nq = tc::kRows / tc::group_pad(G);
   const int nb = (d.T + tc::kKeys - 1) / tc::kKeys;
   if (nb > 65535) return false;
-  if (tc::fwd_smem_bytes(d.D, nb, nq >= 32 ? nq / 32 : 1, 2) > 112 * 1024) return false;
+  if (tc::fwd_smem_bytes(d.D, nb, nq >= 32 ? nq / 32 : 1, tc::kKeys / block_size, 2) > 112 * 1024) return false;
   return true;
 }
 
@@ -845,13 +856,14 @@ static int launch_fwd(const AttnArgs& a, const SelPlanHeader* plan, int force, c
   p.n_qtiles = (a.T + p.nq - 1) / p.nq;
   p.nb_sel = (a.T + kKeys - 1) / kKeys;
   p.nw = p.nq >= 32 ? p.nq / 32 : 1;
+  p.n_sub = a.kind == 2 ? kKeys / a.block_size : 1;
   p.scale_log2 = a.scale * kLog2e;
   CUtensorMap tm_q, tm_k, tm_v;
   int rc = make_map(&tm_q, a.q, a.D, a.T, a.B * a.Hq, p.nq, p.Gp);
   if (rc == NSA_OK) rc = make_map(&tm_k, a.k, a.D, a.Lk, a.B * a.Hkv, kKeys, 1);
   if (rc == NSA_OK) rc = make_map(&tm_v, a.v, a.D, a.Lk, a.B * a.Hkv, kKeys, 1);
   if (rc != NSA_OK) return rc;
-  const size_t smem = fwd_smem_bytes(a.D, p.nb_sel, p.nw, a.kind);
+  const size_t smem = fwd_smem_bytes(a.D, p.nb_sel, p.nw, p.n_sub, a.kind);
   if (a.kind != 2) {
     // window / compression: persistent CTAs, two per SM, each walking its share of the row tiles
     const int sms = sm_count();

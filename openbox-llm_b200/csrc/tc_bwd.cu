@@ -870,6 +870,7 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
         if (p.row_scale) gate_nxt = ldg_f32_now(p.row_scale + row_index(t_nxt));
       }
       int lo = 0, hi = -1;                           // valid key columns of this row: one range [lo, hi]
+      uint32_t groups = 0x3u;                        // and, for selection, the 16-column groups of this thread's half
       if (t_cur >= 0) {
         if (p.kind == 0) {
           lo = max(0, t_cur - p.window + 1 - key0);
@@ -878,6 +879,7 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
           hi = min(kKeys - 1, cmp_visible(t_cur, p.block_size, p.window, p.Lk) - 1 - key0);
         } else {
           hi = min(kKeys - 1, (t_cur & (int)kPairPosMask) - key0);
+          groups = ((uint32_t)t_cur >> (kPairPosBits + 2 * half)) & 0x3u;
         }
       }
       // gate * p = 2^(s * scale * log2e - lse * log2e + log2(gate)): the branch's dO is gate * dO, so dV takes
@@ -885,7 +887,7 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
       const float lse2 = lse_cur * kLog2e - __log2f(gate_cur);
       const float dscale = p.scale, ddelta = delta_cur * p.scale;
       // every column of this thread's half is attended (the usual case away from the diagonal)?
-      const bool all_cols = lo <= half * 32 && hi >= half * 32 + 31;
+      const bool all_cols = lo <= half * 32 && hi >= half * 32 + 31 && groups == 0x3u;
       mbar_wait(sp_full + sb, u & 1, p.status, s_abort, 64);
       // the P / dS tiles double as the dQ staging tile: this group's store of tile k-2 has read it
       if (lt == 0) bulk_wait_read();
@@ -913,7 +915,7 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
               const int c = half * 32 + c2 * 2 + e;
-              const bool ok = (c >= lo) && (c <= hi);
+              const bool ok = (c >= lo) && (c <= hi) && ((groups >> (c2 >> 3)) & 1u);
               const float pr = ok ? ex2(fmaf(__uint_as_float(rs[c2 * 2 + e]), p.scale_log2, -lse2)) : 0.f;
               pv[e] = pr;
               dv[e] = pr * fmaf(__uint_as_float(rp[c2 * 2 + e]), dscale, -ddelta);

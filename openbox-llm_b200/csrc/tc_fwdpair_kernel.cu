@@ -245,13 +245,14 @@ tc_fwdpair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
     auto row_query = [&](int k) -> int {
       const int qi = (item.z + k) * p.nq + ql;
       if (!row_slot_ok || qi >= n_q) return -1;
-      return (int)(ldg_s32_now(p.plan.pairs + pair_base + qi) & kPairPosMask);
+      return ldg_s32_now(p.plan.pairs + pair_base + qi);
     };
     int t_cur = sb < n_tiles ? row_query(sb) : -1;
     for (int k = sb; k < n_tiles; k += 2) {
       if (*s_abort) break;
       const int t_nxt = k + 2 < n_tiles ? row_query(k + 2) : -1;
-      const int hi = t_cur >= 0 ? min(kKeys - 1, min(t_cur, p.T - 1) - key0) : -1;
+      const int hi = t_cur >= 0 ? min(kKeys - 1, (int)(t_cur & kPairPosMask) - key0) : -1;
+      const uint32_t groups = (uint32_t)t_cur >> kPairPosBits;      // 16-column groups the row attends
       mbar_wait(s_full + sb, (k >> 1) & 1, p.status, s_abort, 64);
       if (*s_abort) break;
       tc_fence_after();
@@ -260,7 +261,7 @@ tc_fwdpair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
       tmem_ld32(lane_base + 32, r + 32);
       tmem_wait_ld();
       float mx = -INFINITY;
-      if (hi >= kKeys - 1) {
+      if (hi >= kKeys - 1 && groups == 0xfu) {
 #pragma unroll
         for (int c = 0; c < 64; ++c) {
           const float x = __uint_as_float(r[c]) * p.scale_log2;
@@ -270,7 +271,7 @@ tc_fwdpair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
       } else {
 #pragma unroll
         for (int c = 0; c < 64; ++c) {
-          const float x = c <= hi ? __uint_as_float(r[c]) * p.scale_log2 : -INFINITY;
+          const float x = (c <= hi && ((groups >> (c >> 4)) & 1u)) ? __uint_as_float(r[c]) * p.scale_log2 : -INFINITY;
           r[c] = __float_as_uint(x);
           mx = fmaxf(mx, x);
         }
