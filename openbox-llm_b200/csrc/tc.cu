@@ -7,15 +7,15 @@
 //   compression the tiles covering summaries [0, (t_last + 1) / Bsz - 1]
 //   selection   the 64-key tiles holding blocks (of 16, 32 or 64 tokens) listed for the tile's nq
 //               queries, found in shared memory, with a membership bit per (query, block)
-// Per tile: a TMA warp brings K and V (128B-swizzled boxes) into a 2-stage ring; an MMA warp
-// issues S = Q K^T (tcgen05.mma, Q held in TMEM as the A operand, accumulator in TMEM); each of
-// the 128 softmax threads owns one row of S (tcgen05.ld, lane = row), masks it, runs the online
-// softmax in the log2 domain without any cross-thread traffic and writes P as packed bf16 over S
-// in TMEM (tcgen05.st); the MMA warp then issues O += P V with P as the TMEM A operand and V as
-// an MN-major shared-memory B operand.  The running maximum is only raised when it grows by more
-// than 8 (log2 units), so the O accumulator in TMEM is rescaled rarely.
-// tc_fwd_kernel takes one row tile per CTA (query-outer selection); tc_fwd_range_kernel is the
-// persistent form for window and compression.
+// Per tile: a TMA warp brings K and V (128B-swizzled boxes) into a ring; an MMA warp issues
+// S = Q K^T (tcgen05.mma, accumulator in one of two TMEM buffers); each of the 128 softmax threads
+// owns one row of S (tcgen05.ld, lane = row), masks it, runs the online softmax in the log2 domain
+// without any cross-thread traffic and writes P as packed bf16 over S in TMEM (tcgen05.st); the MMA
+// warp then issues O += P V with P as the TMEM A operand and V as an MN-major shared-memory B
+// operand.  The running maximum is only raised when it grows by more than 8 (log2 units), so the O
+// accumulator in TMEM is rescaled rarely.
+#include <algorithm>
+
 #include "tc_common.cuh"
 #include "tc_host.cuh"
 
@@ -38,39 +38,72 @@ struct FwdArgs {
   float scale_log2;
 };
 
+// D = 128: Q 32 KB + two stages of K and V = 96 KB, two CTAs per SM.  D = 64: four stages in 80 KB.
 template <int D> struct FwdSmem {
   static constexpr int kSlabs = D / 64;
+  static constexpr int kStages = D == 64 ? 4 : 2;
   static constexpr int kQBytes = kRows * 128 * kSlabs;
   static constexpr int kKVBytes = kKeys * 128 * kSlabs;
-  static constexpr int kFixed = kQBytes + 4 * kKVBytes;   // Q + 2 K stages + 2 V stages
+  static constexpr int kFixed = kQBytes + 2 * kStages * kKVBytes;
+  static constexpr int kBars = 9 + 4 * kStages;
 };
 
 __host__ __device__ inline size_t fwd_smem_bytes(int D, int nb_sel, int nw, int n_sub, int kind) {
-  size_t fixed = (size_t)(kRows * 128 + 4 * kKeys * 128) * (D / 64);
   size_t extra = 256 /*barriers etc*/ + 132 * 4 /*scan*/;
   if (kind == 2) extra += (size_t)nb_sel * n_sub * nw * 4 + (size_t)nb_sel * 2 + 16;
-  return fixed + extra + 1024 /*alignment slack*/;
+  return (D == 64 ? FwdSmem<64>::kFixed : FwdSmem<128>::kFixed) + extra + 1024 /*alignment slack*/;
 }
 
-// 192 threads in roles.  Warps 0-3 (thread = row = TMEM lane) own the softmax; warp 4 sends the
-// TMA loads; warp 5 issues the MMAs.  With the issuing on a softmax warp, as an earlier version
-// had it, every tile waited for that warp to get its TMA boxes and a dozen MMAs out between its
-// own exponentials.  The Q tile is copied into tensor memory once per CTA, so S = Q K^T takes its
-// A operand from there (an MMA of 128 x 64 x 16 that fetches both operands from shared memory is
-// bound by that fetch, not by its arithmetic).  Two CTAs per SM.
 constexpr int kFwdThreads = 192;
 constexpr int kFwdSoftmax = 128;
 
-template <int D>
+// Packed pairs of fp32: one instruction for two lanes' worth of the softmax arithmetic.
+__device__ __forceinline__ uint64_t pack_f32x2(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpack_f32x2(uint64_t v, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
+// One kernel for the three branches (kSel: selection).  192 threads in roles: warps 0-3 (thread = row
+// = TMEM lane) own the softmax, warp 4 sends the TMA loads, warp 5 issues the MMAs; two CTAs per SM,
+// each walking many row tiles (tile w, w + gridDim.x, ...), long rows first.
+//
+// What bounds it: one row tile is a chain S -> exponentials -> P V per key tile, and with a single S
+// buffer the hand-overs of that chain (two barrier hops, two MMA latencies) took twice the
+// arithmetic: 1.34 k cycles per key tile and SM with two chains running, where the exponentials
+// need 512 (16 MUFU results per clock), the MMAs as much, and shared memory 768 (operands and
+// incoming tiles, D = 128).  Two S buffers take the MMA latency out of the chain: S of the next key
+// tile is computed while the softmax works on this one.  They fill the tensor memory that Q
+// occupied before (O 128 + 2 x 64 columns per CTA), so S takes both operands from shared memory.
+// The producer runs ahead into the next row tile, whose first S is computed while the threads write
+// this tile's output.  Every barrier's phase follows a running count (of row tiles, or of key tiles
+// over all row tiles) that each role keeps itself.
+//
+// Selection builds the list of a row tile's key tiles first, all threads together, and so works row
+// tile by row tile.
+template <int D, bool kSel>
 __global__ void __launch_bounds__(kFwdThreads, 2)
 tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
               const __grid_constant__ CUtensorMap tm_v, const FwdArgs p) {
   using L = FwdSmem<D>;
-  constexpr int kSlabs = L::kSlabs;
+  constexpr int kSlabs = L::kSlabs, kStages = L::kStages;
   constexpr uint32_t kTmemCols = 256;
-  // O in columns 0-127, S in 128-191 (P, bf16, is written over its first 32 columns by the thread
-  // that read the row), the Q tile (bf16, D / 2 columns) in 192-255
-  constexpr uint32_t kColO = 0, kColS = 128, kColQ = 192;
+  // O in columns 0-127, two buffers of S (P, bf16, is written over the first 32 columns of its S by the
+  // thread that read the row)
+  constexpr uint32_t kColO = 0, kColS = 128;
   constexpr uint32_t kIdescQK = idesc_bf16(128, kKeys, 0, 0);
   constexpr uint32_t kIdescPV = idesc_bf16(128, D, 0, 1);
 
@@ -78,423 +111,37 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);   // pointer arithmetic keeps the shared address space
   uint8_t* sQ = smem;
   uint8_t* sK = sQ + L::kQBytes;
-  uint8_t* sV = sK + 2 * L::kKVBytes;
-  uint64_t* bars = (uint64_t*)(sV + 2 * L::kKVBytes);
-  uint64_t* bar_q = bars + 0;        // Q tile landed (TMA bytes)
-  uint64_t* bar_k = bars + 1;        // [2] K stage landed
-  uint64_t* bar_v = bars + 3;        // [2] V stage landed
-  uint64_t* k_free = bars + 5;       // [2] the S MMA that read the stage is done
-  uint64_t* v_free = bars + 7;       // [2] the PV MMA that read the stage is done
-  uint64_t* bar_s = bars + 9;        // S of a tile is in tensor memory
-  uint64_t* bar_p = bars + 10;       // the 128 rows of P are written (and S is read)
-  uint64_t* bar_o = bars + 11;       // PV of a tile is done
-  uint64_t* bar_qt = bars + 12;      // the 128 rows of Q are in tensor memory
-  uint64_t* bar_drain = bars + 13;   // an aborted CTA waits here for its last MMAs
-  uint32_t* s_tmem = (uint32_t*)(bars + 14);
+  uint8_t* sV = sK + kStages * L::kKVBytes;
+  uint64_t* bars = (uint64_t*)(sV + kStages * L::kKVBytes);
+  uint64_t* bar_q = bars + 0;        // Q tile landed (TMA bytes); phase = row tile count
+  uint64_t* q_free = bars + 1;       // the last S MMA of a row tile has read Q
+  uint64_t* bar_s = bars + 2;        // [2] S of a key tile is in tensor memory; phase = (key tile count) >> 1
+  uint64_t* bar_p = bars + 4;        // [2] the 128 rows of P are written (and S is read)
+  uint64_t* bar_o = bars + 6;        // [2] PV of a key tile is done; phase = (key tile count) >> 1 (two in turn: the
+                                     //     PVs of two tiles may be under way when a thread waits for the later)
+  uint64_t* bar_drain = bars + 8;    // an aborted CTA waits here for its last MMAs
+  uint64_t* bar_k = bars + 9;                  // [kStages] K stage landed; phase = (key tile count) / kStages
+  uint64_t* bar_v = bar_k + kStages;           // [kStages] V stage landed
+  uint64_t* k_free = bar_v + kStages;          // [kStages] the S MMA that read the stage is done
+  uint64_t* v_free = k_free + kStages;         // [kStages] the PV MMA that read the stage is done
+  uint32_t* s_tmem = (uint32_t*)(bars + L::kBars);
   volatile int* s_abort = (volatile int*)(s_tmem + 1);
   int* s_ntiles = (int*)(s_tmem + 2);
   int* s_scan = (int*)(s_tmem + 4);                 // [129]
   uint32_t* s_member = (uint32_t*)(s_scan + 132);   // [nb_sel][n_sub][nw]   (selection only)
   const int tile_words = p.n_sub * p.nw;
-  uint16_t* s_tiles = (uint16_t*)(s_member + (p.kind == 2 ? p.nb_sel * tile_words : 0));
+  uint16_t* s_tiles = (uint16_t*)(s_member + (kSel ? p.nb_sel * tile_words : 0));
 
-  if (p.kind == 2 && p.plan != nullptr && prefer_pairs(p.plan, p.nq, p.force))
+  if (kSel && p.plan != nullptr && prefer_pairs(p.plan, p.nq, p.force))
     return;   // the block-outer variant serves this call: leave before anything is set up
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int qtile = p.n_qtiles - 1 - (int)blockIdx.x;   // long rows first
-  const int bh = blockIdx.y;
-  const int b = bh / p.Hkv, hkv = bh % p.Hkv;
-  const int t0 = qtile * p.nq;
-  const int t_last = min(p.T - 1, t0 + p.nq - 1);
-  // softmax threads: row of the tile = thread index
-  const int row = tid & (kFwdSoftmax - 1);
-  const int g = row / p.nq, ql = row % p.nq;
-  const int t = t0 + ql;
-  const bool row_ok = tid < kFwdSoftmax && (g < p.G) && (t < p.T);
-  const int head = hkv * p.G + g;
-
   if (tid == 0) {
     *s_abort = (*(volatile int*)p.status != 0) ? 1 : 0;
     mbar_init(bar_q, 1);
-    for (int k = 1; k <= 8; ++k) mbar_init(bars + k, 1);
-    mbar_init(bar_s, 1);
-    mbar_init(bar_p, kFwdSoftmax);
-    mbar_init(bar_o, 1);
-    mbar_init(bar_qt, kFwdSoftmax);
+    mbar_init(q_free, 1);
+    for (int k = 0; k < 2; ++k) { mbar_init(bar_s + k, 1); mbar_init(bar_p + k, kFwdSoftmax); mbar_init(bar_o + k, 1); }
     mbar_init(bar_drain, 1);
-    fence_barrier_init();
-    prefetch_tensormap(&tm_q); prefetch_tensormap(&tm_k); prefetch_tensormap(&tm_v);
-  }
-  __syncthreads();
-  if (*s_abort) return;
-
-  // ---- tile list ------------------------------------------------------------------------
-  int n_tiles = 0, first_key = 0;
-  if (p.kind == 0) {
-    first_key = max(0, t0 - p.window + 1) & ~(kKeys - 1);
-    n_tiles = (min(t_last, p.Lk - 1) - first_key) / kKeys + 1;
-  } else if (p.kind == 1) {
-    const int hi_last = cmp_visible(t_last, p.block_size, p.window, p.Lk) - 1;   // window: the stride
-    n_tiles = hi_last < 0 ? 0 : hi_last / kKeys + 1;
-  } else {
-    const int nmem = p.nb_sel * tile_words;
-    for (int i = tid; i < nmem; i += kFwdThreads) s_member[i] = 0u;
-    __syncthreads();
-    const int32_t* idx = p.block_idx + ((size_t)bh * p.T + t0) * p.S;
-    const int n_entries = (t_last - t0 + 1) * p.S;
-    for (int e = tid; e < n_entries; e += kFwdThreads) {
-      const int q_local = e / p.S;
-      const int blk = __ldg(idx + e);
-      // list block blk = part blk % n_sub of key tile blk / n_sub
-      if (blk >= 0 && (long long)blk * p.block_size <= t0 + q_local)
-        atomicOr(&s_member[blk * p.nw + (q_local >> 5)], 1u << (q_local & 31));
-    }
-    __syncthreads();
-    const int per = (p.nb_sel + 127) / 128;       // the first 128 threads scan `per` blocks each
-    const int j0 = tid < 128 ? tid * per : p.nb_sel, j1 = min(p.nb_sel, j0 + per);
-    int cnt = 0;
-    for (int j = j0; j < j1; ++j) {
-      uint32_t any = 0;
-      for (int w = 0; w < tile_words; ++w) any |= s_member[j * tile_words + w];
-      cnt += any != 0;
-    }
-    if (tid < 128) s_scan[tid + 1] = cnt;
-    __syncthreads();
-    if (tid == 0) {
-      s_scan[0] = 0;
-      for (int i = 1; i <= 128; ++i) s_scan[i] += s_scan[i - 1];
-      *s_ntiles = s_scan[128];
-    }
-    __syncthreads();
-    int pos = tid < 128 ? s_scan[tid] : 0;
-    for (int j = j0; j < j1; ++j) {
-      uint32_t any = 0;
-      for (int w = 0; w < tile_words; ++w) any |= s_member[j * tile_words + w];
-      if (any) s_tiles[pos++] = (uint16_t)j;
-    }
-    __syncthreads();
-    n_tiles = *s_ntiles;
-  }
-
-  float m_used = -INFINITY, l_sum = 0.f;
-  __nv_bfloat16* orow = p.o + ((size_t)(b * p.Hq + head) * p.T + t) * D;
-  if (n_tiles == 0) {                       // (uniform over the CTA) rows without a key: zeros
-    if (row_ok) {
-      uint4* dst = reinterpret_cast<uint4*>(orow);
-#pragma unroll
-      for (int v4 = 0; v4 < D / 8; ++v4) dst[v4] = make_uint4(0, 0, 0, 0);
-      p.lse[(size_t)(b * p.Hq + head) * p.T + t] = kLseEmpty;
-    }
-    return;
-  }
-
-  // ---- TMEM ---------------------------------------------------------------------------
-  if (warp == 0) {
-    tmem_alloc(s_tmem, kTmemCols);
-    tmem_relinquish();
-  }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = *s_tmem;
-  const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) * 32) << 16);
-  auto key0_of = [&](int i) -> int {
-    if (p.kind == 2) return (int)s_tiles[i] * kKeys;
-    return first_key + i * kKeys;
-  };
-  int last_k[2] = {-1, -1}, last_v[2] = {-1, -1};   // producer: last tile sent into each stage
-
-  if (warp == 4) {
-    // ---- producer -------------------------------------------------------------------------
-    if (lane == 0) {
-      auto load_k = [&](int i) {
-        uint64_t* bar = bar_k + (i & 1);
-        mbar_expect_tx(bar, L::kKVBytes);
-#pragma unroll
-        for (int s = 0; s < kSlabs; ++s)
-          tma_load_3d(sK + (i & 1) * L::kKVBytes + s * (kKeys * 128), &tm_k, bar, s * 64, key0_of(i), bh);
-        last_k[i & 1] = i;
-      };
-      auto load_v = [&](int i) {
-        uint64_t* bar = bar_v + (i & 1);
-        if (p.debug_starve && i == 1) return;   // test only: this tile's wait has to run out
-        mbar_expect_tx(bar, L::kKVBytes);
-#pragma unroll
-        for (int s = 0; s < kSlabs; ++s)
-          tma_load_3d(sV + (i & 1) * L::kKVBytes + s * (kKeys * 128), &tm_v, bar, s * 64, key0_of(i), bh);
-        last_v[i & 1] = i;
-      };
-      mbar_expect_tx(bar_q, L::kQBytes);
-#pragma unroll
-      for (int s = 0; s < kSlabs; ++s)
-        tma_load_3d(sQ + s * (kRows * 128), &tm_q, bar_q, s * 64, t0, b * p.Hq + hkv * p.G);
-      load_k(0);
-      load_v(0);
-      if (n_tiles > 1) { load_k(1); load_v(1); }
-      for (int i = 0; i + 2 < n_tiles; ++i) {
-        // stage i & 1 is free once the MMAs of tile i that read it are done (a barrier per stage:
-        // its next completion needs the very load that waits here, so no phase can be missed)
-        if (!mbar_wait(k_free + (i & 1), (i >> 1) & 1, p.status, s_abort, 0x4000)) break;
-        load_k(i + 2);
-        if (!mbar_wait(v_free + (i & 1), (i >> 1) & 1, p.status, s_abort, 0x4000)) break;
-        load_v(i + 2);
-      }
-    }
-  } else if (warp == 5) {
-    // ---- MMA issuer ------------------------------------------------------------------------
-    if (lane == 0) {
-      auto issue_s = [&](int i) {   // S = Q K^T for tile i, Q from tensor memory
-        const uint32_t ka = desc_lo_kmajor(smem_u32(sK + (i & 1) * L::kKVBytes));
-#pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) {
-          const uint32_t slab = kk >> 2, in = (kk & 3) * 32;
-          mma_ts(tmem + kColS, tmem + kColQ + kk * 8, desc_at(ka, slab * (kKeys * 128) + in), kIdescQK, kk > 0);
-        }
-        tc_commit(bar_s);
-        tc_commit(k_free + (i & 1));
-      };
-      auto issue_pv = [&](int i) {  // O (+)= P V for tile i
-        const uint32_t va = desc_lo_mnmajor(smem_u32(sV + (i & 1) * L::kKVBytes), kKeys * 128);
-#pragma unroll
-        for (int kk = 0; kk < kKeys / 16; ++kk)
-          mma_ts(tmem + kColO, tmem + kColS + kk * 8, desc_at(va, kk * 2048), kIdescPV, (i > 0) || (kk > 0));
-        tc_commit(bar_o);
-        tc_commit(v_free + (i & 1));
-      };
-      bool ok = mbar_wait(bar_qt, 0, p.status, s_abort, 0x8000) &&
-                mbar_wait(bar_k, 0, p.status, s_abort, 2);
-      if (ok) {
-        tc_fence_after();
-        issue_s(0);
-      }
-      for (int i = 0; ok && i < n_tiles; ++i) {
-        ok = mbar_wait(bar_p, i & 1, p.status, s_abort, 0x2000) &&
-             mbar_wait(bar_v + (i & 1), (i >> 1) & 1, p.status, s_abort, 16);
-        if (!ok) break;
-        tc_fence_after();
-        issue_pv(i);
-        if (i + 1 < n_tiles) {
-          // S of the next tile overwrites P of this one: the tensor pipe keeps the order
-          ok = mbar_wait(bar_k + ((i + 1) & 1), ((i + 1) >> 1) & 1, p.status, s_abort, 2);
-          if (ok) issue_s(i + 1);
-        }
-      }
-      // the tensor pipe is idle before tensor memory is read for the output and given back
-      tc_commit(bar_drain);
-      if (!mbar_wait(bar_drain, 0, p.status, s_abort, 0x1000)) mbar_wait_drain(bar_drain, 0);
-    }
-  } else {
-    // ---- softmax: thread = row ---------------------------------------------------------------
-    // Q: shared memory -> tensor memory, every thread its row
-    bool ok = mbar_wait(bar_q, 0, p.status, s_abort, 1);
-    {
-#pragma unroll
-      for (int sl = 0; sl < kSlabs; ++sl) {
-        const uint8_t* src = sQ + sl * (kRows * 128) + row * 128;
-        uint32_t qv[32];
-#pragma unroll
-        for (int c = 0; c < 8; ++c) {
-          const uint4 u = *reinterpret_cast<const uint4*>(src + ((c ^ (row & 7)) << 4));
-          qv[4 * c + 0] = u.x; qv[4 * c + 1] = u.y; qv[4 * c + 2] = u.z; qv[4 * c + 3] = u.w;
-        }
-        tmem_st32(lane_base + kColQ + sl * 32, qv);
-      }
-      tmem_wait_st();
-      tc_fence_before();
-      mbar_arrive(bar_qt);
-    }
-    for (int i = 0; i < n_tiles; ++i) {
-      const int key0 = key0_of(i);
-      ok = mbar_wait(bar_s, i & 1, p.status, s_abort, 4) && ok;
-      if (!__all_sync(0xffffffffu, ok)) break;              // the whole warp leaves together
-      tc_fence_after();
-      uint32_t r[64];
-      tmem_ld32(lane_base + kColS, r);
-      tmem_ld32(lane_base + kColS + 32, r + 32);
-      tmem_wait_ld();
-
-      // valid columns of this row in this tile form one range [lo, hi]
-      int lo = 0, hi = -1;
-      uint32_t groups = 0xfu;              // 16-column groups of the tile the row attends
-      if (row_ok) {
-        if (p.kind == 0) {
-          lo = max(0, t - p.window + 1 - key0);
-          hi = min(kKeys - 1, t - key0);
-        } else if (p.kind == 1) {
-          hi = min(kKeys - 1, cmp_visible(t, p.block_size, p.window, p.Lk) - 1 - key0);
-        } else {
-          hi = min(kKeys - 1, t - key0);
-          const uint32_t* mem = s_member + (key0 / kKeys) * tile_words + (ql >> 5);
-          if (p.n_sub == 1) {
-            if (!((mem[0] >> (ql & 31)) & 1u)) hi = -1;
-          } else {
-            groups = 0u;
-            for (int k = 0; k < p.n_sub; ++k)
-              if ((mem[k * p.nw] >> (ql & 31)) & 1u) groups |= ((1u << (p.block_size >> 4)) - 1u) << (k * (p.block_size >> 4));
-          }
-        }
-      }
-      float x[64];
-      float tmax = -INFINITY;
-      if (lo <= 0 && hi >= kKeys - 1 && groups == 0xfu) {
-#pragma unroll
-        for (int c = 0; c < 64; ++c) {
-          x[c] = __uint_as_float(r[c]) * p.scale_log2;
-          tmax = fmaxf(tmax, x[c]);
-        }
-      } else {
-#pragma unroll
-        for (int c = 0; c < 64; ++c) {
-          x[c] = (c >= lo && c <= hi && ((groups >> (c >> 4)) & 1u)) ? __uint_as_float(r[c]) * p.scale_log2 : -INFINITY;
-          tmax = fmaxf(tmax, x[c]);
-        }
-      }
-      float alpha = 1.f;
-      bool rescale = false;
-      if (tmax > m_used + 8.f) {              // also the first finite maximum (m_used = -inf)
-        if (m_used != -INFINITY) {
-          alpha = ex2(m_used - tmax);
-          rescale = true;
-          l_sum *= alpha;
-        }
-        m_used = tmax;
-      }
-      const float msub = (m_used == -INFINITY) ? 0.f : m_used;
-      float psum = 0.f;
-      uint32_t pk[32];
-#pragma unroll
-      for (int c = 0; c < 32; ++c) {
-        const float p0 = ex2(x[2 * c] - msub), p1 = ex2(x[2 * c + 1] - msub);
-        psum += p0 + p1;
-        pk[c] = pack_bf16(p0, p1);
-      }
-      l_sum += psum;
-
-      // O may be touched once PV of tile i-1 is done; only a warp that has to rescale waits for it
-      if (i > 0 && __any_sync(0xffffffffu, rescale)) {
-        ok = mbar_wait(bar_o, (i - 1) & 1, p.status, s_abort, 8);
-        if (!__all_sync(0xffffffffu, ok)) break;
-        tc_fence_after();
-#pragma unroll
-        for (int cc = 0; cc < D / 32; ++cc) {
-          uint32_t o32[32];
-          tmem_ld32(lane_base + kColO + cc * 32, o32);
-          tmem_wait_ld();
-#pragma unroll
-          for (int c = 0; c < 32; ++c) o32[c] = __float_as_uint(__uint_as_float(o32[c]) * alpha);
-          tmem_st32(lane_base + kColO + cc * 32, o32);
-        }
-      }
-      tmem_st32(lane_base + kColS, pk);        // over the S columns this thread has just read
-      tmem_wait_st();
-      tc_fence_before();
-      mbar_arrive(bar_p);
-    }
-    // the last PV
-    if (__all_sync(0xffffffffu, ok)) mbar_wait(bar_o, (n_tiles - 1) & 1, p.status, s_abort, 8);
-  }
-
-  // ---- teardown -------------------------------------------------------------------------------
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  if (*s_abort) {
-    // Give-up path: no output is written.  The producer waits (bounded) for the loads still on
-    // their way into this CTA's shared memory; the MMA thread has waited for the tensor pipe
-    // above; then the tensor memory goes back.
-    if (warp == 4 && lane == 0) {
-      mbar_wait_drain(bar_q, 0);
-#pragma unroll
-      for (int st = 0; st < 2; ++st) {
-        if (last_k[st] >= 0) mbar_wait_drain(bar_k + st, (last_k[st] >> 1) & 1);
-        if (last_v[st] >= 0) mbar_wait_drain(bar_v + st, (last_v[st] >> 1) & 1);
-      }
-    }
-    if (warp == 5 && lane == 0) mbar_wait_drain(bar_drain, 0);
-    __syncthreads();
-    if (warp == 0) tmem_dealloc(tmem, kTmemCols);
-    return;
-  }
-
-  // ---- epilogue ---------------------------------------------------------------------------
-  if (tid < kFwdSoftmax) {
-    const float inv = l_sum > 0.f ? 1.f / l_sum : 0.f;
-#pragma unroll
-    for (int cc = 0; cc < D / 32; ++cc) {
-      uint32_t o32[32];
-      tmem_ld32(lane_base + kColO + cc * 32, o32);
-      tmem_wait_ld();
-      if (row_ok) {
-        uint4* dst = reinterpret_cast<uint4*>(orow + cc * 32);
-#pragma unroll
-        for (int v4 = 0; v4 < 4; ++v4) {
-          uint4 u;
-          u.x = pack_bf16(__uint_as_float(o32[v4 * 8 + 0]) * inv, __uint_as_float(o32[v4 * 8 + 1]) * inv);
-          u.y = pack_bf16(__uint_as_float(o32[v4 * 8 + 2]) * inv, __uint_as_float(o32[v4 * 8 + 3]) * inv);
-          u.z = pack_bf16(__uint_as_float(o32[v4 * 8 + 4]) * inv, __uint_as_float(o32[v4 * 8 + 5]) * inv);
-          u.w = pack_bf16(__uint_as_float(o32[v4 * 8 + 6]) * inv, __uint_as_float(o32[v4 * 8 + 7]) * inv);
-          if (l_sum > 0.f) dst[v4] = u; else dst[v4] = make_uint4(0, 0, 0, 0);
-        }
-      }
-    }
-    if (row_ok)
-      p.lse[(size_t)(b * p.Hq + head) * p.T + t] =
-          l_sum > 0.f ? (m_used + log2f(l_sum)) * kLn2 : kLseEmpty;
-  }
-  tc_fence_before();
-  __syncthreads();
-  if (warp == 0) tmem_dealloc(tmem, kTmemCols);
-}
-
-// ---- window / compression forward as a persistent kernel ---------------------------------------
-// The same roles and tensor-memory layout as tc_fwd_kernel, but a CTA walks many row tiles (tile
-// w, w + gridDim.x, ...), so what a CTA per row tile pays between tiles -- barrier set-up, the
-// tensor-memory allocation, the latency of the first Q / K / V loads, the tail of the epilogue --
-// is paid once or hidden: the producer runs ahead into the next row tile (its Q lands in shared
-// memory while this tile is worked on; the K / V ring never drains), a softmax thread moves its
-// row of the next Q into tensor memory right after its last P of this tile, and the next tile's
-// first S is computed while the threads write this tile's output.  Every barrier's phase follows
-// a running count (of row tiles, or of key tiles over all row tiles) that each role keeps itself.
-template <int D>
-__global__ void __launch_bounds__(kFwdThreads, 2)
-tc_fwd_range_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-                    const __grid_constant__ CUtensorMap tm_v, const FwdArgs p) {
-  using L = FwdSmem<D>;
-  constexpr int kSlabs = L::kSlabs;
-  constexpr uint32_t kTmemCols = 256;
-  constexpr uint32_t kColO = 0, kColS = 128, kColQ = 192;   // as in tc_fwd_kernel
-  constexpr uint32_t kIdescQK = idesc_bf16(128, kKeys, 0, 0);
-  constexpr uint32_t kIdescPV = idesc_bf16(128, D, 0, 1);
-
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-  uint8_t* sQ = smem;
-  uint8_t* sK = sQ + L::kQBytes;
-  uint8_t* sV = sK + 2 * L::kKVBytes;
-  uint64_t* bars = (uint64_t*)(sV + 2 * L::kKVBytes);
-  uint64_t* bar_q = bars + 0;        // Q tile landed (TMA bytes); phase = row tile count
-  uint64_t* bar_k = bars + 1;        // [2] K stage landed; phase = (key tile count) >> 1
-  uint64_t* bar_v = bars + 3;        // [2] V stage landed
-  uint64_t* k_free = bars + 5;       // [2] the S MMA that read the stage is done
-  uint64_t* v_free = bars + 7;       // [2] the PV MMA that read the stage is done
-  uint64_t* bar_s = bars + 9;        // S of a key tile is in tensor memory; phase = key tile count
-  uint64_t* bar_p = bars + 10;       // the 128 rows of P are written (and S is read)
-  uint64_t* bar_o = bars + 11;       // PV of a key tile is done
-  uint64_t* bar_qt = bars + 12;      // the 128 rows of Q are in tensor memory (and its shared-memory tile is free)
-  uint64_t* bar_drain = bars + 13;
-  uint32_t* s_tmem = (uint32_t*)(bars + 14);
-  volatile int* s_abort = (volatile int*)(s_tmem + 1);
-
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (tid == 0) {
-    *s_abort = (*(volatile int*)p.status != 0) ? 1 : 0;
-    mbar_init(bar_q, 1);
-    for (int k = 1; k <= 8; ++k) mbar_init(bars + k, 1);
-    mbar_init(bar_s, 1);
-    mbar_init(bar_p, kFwdSoftmax);
-    mbar_init(bar_o, 1);
-    mbar_init(bar_qt, kFwdSoftmax);
-    mbar_init(bar_drain, 1);
+    for (int k = 0; k < 4 * kStages; ++k) mbar_init(bar_k + k, 1);
     fence_barrier_init();
     prefetch_tensormap(&tm_q); prefetch_tensormap(&tm_k); prefetch_tensormap(&tm_v);
   }
@@ -519,257 +166,275 @@ tc_fwd_range_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     const int qtile = p.n_qtiles - 1 - w / units;
     x.t0 = qtile * p.nq;
     x.t_last = min(p.T - 1, x.t0 + p.nq - 1);
-    if (p.kind == 0) {
+    x.first_key = 0;
+    if (kSel) {
+      x.n_tiles = *s_ntiles;
+    } else if (p.kind == 0) {
       x.first_key = max(0, x.t0 - p.window + 1) & ~(kKeys - 1);
       x.n_tiles = (min(x.t_last, p.Lk - 1) - x.first_key) / kKeys + 1;
     } else {
-      x.first_key = 0;
       const int hi_last = cmp_visible(x.t_last, p.block_size, p.window, p.Lk) - 1;   // window: the stride
       x.n_tiles = hi_last < 0 ? 0 : hi_last / kKeys + 1;
     }
     return x;
   };
-  int last_k[2] = {-1, -1}, last_v[2] = {-1, -1};   // producer: running index of the last tile sent into each stage
-  int q_sent = 0;                                   // producer: row tiles whose Q was sent
-
-  if (warp == 4) {
-    // ---- producer -------------------------------------------------------------------------
-    if (lane == 0) {
-      int c = 0, it = 0;                              // running key tile / live row tile counts
-      bool ok = true;
-      for (int w = blockIdx.x; ok && w < n_work; w += gridDim.x) {
-        const Tile x = tile_of(w);
-        if (x.n_tiles == 0) continue;
-        const int b = x.bh / p.Hkv, hkv = x.bh % p.Hkv;
-        // the Q tile in shared memory is free once every row of the previous one is in tensor memory
-        if (it > 0) ok = mbar_wait(bar_qt, (it - 1) & 1, p.status, s_abort, 0x8000);
-        if (!ok) break;
-        mbar_expect_tx(bar_q, L::kQBytes);
+  auto key0_of = [&](const Tile& x, int i) -> int { return kSel ? (int)s_tiles[i] * kKeys : x.first_key + i * kKeys; };
+  // the key tiles that hold a block listed by one of the row tile's queries, with a membership bit per
+  // (query, list block)
+  auto build_list = [&](int w) {
+    const int bh = w % units, t0 = (p.n_qtiles - 1 - w / units) * p.nq, t_last = min(p.T - 1, t0 + p.nq - 1);
+    const int n_vis = t_last / kKeys + 1;              // key tiles that start at or before the last query
+    for (int i = tid; i < n_vis * tile_words; i += kFwdThreads) s_member[i] = 0u;
+    __syncthreads();
+    const int32_t* idx = p.block_idx + ((size_t)bh * p.T + t0) * p.S;
+    const int n_entries = (t_last - t0 + 1) * p.S;
+    for (int e = tid; e < n_entries; e += kFwdThreads) {
+      const int q_local = e / p.S;
+      const int blk = __ldg(idx + e);
+      // list block blk = part blk % n_sub of key tile blk / n_sub
+      if (blk >= 0 && (long long)blk * p.block_size <= t0 + q_local)
+        atomicOr(&s_member[blk * p.nw + (q_local >> 5)], 1u << (q_local & 31));
+    }
+    __syncthreads();
+    const int per = (n_vis + 127) / 128;               // the first 128 threads scan `per` tiles each
+    const int j0 = tid < 128 ? min(n_vis, tid * per) : n_vis, j1 = min(n_vis, j0 + per);
+    int cnt = 0;
+    for (int j = j0; j < j1; ++j) {
+      uint32_t any = 0;
+      for (int k = 0; k < tile_words; ++k) any |= s_member[j * tile_words + k];
+      cnt += any != 0;
+    }
+    int incl = cnt;
 #pragma unroll
-        for (int s = 0; s < kSlabs; ++s)
-          tma_load_3d(sQ + s * (kRows * 128), &tm_q, bar_q, s * 64, x.t0, b * p.Hq + hkv * p.G);
-        q_sent = it + 1;
-        for (int i = 0; i < x.n_tiles; ++i, ++c) {
-          const int st = c & 1;
-          // a stage is free once the MMAs of the tile two back, which read it, are done
-          if (c >= 2) {
-            ok = mbar_wait(k_free + st, ((c >> 1) - 1) & 1, p.status, s_abort, 0x4000);
-            if (!ok) break;
-          }
-          mbar_expect_tx(bar_k + st, L::kKVBytes);
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += v;
+    }
+    if (lane == 31) s_scan[warp] = incl;
+    __syncthreads();
+    int pos = incl - cnt;
+    for (int k = 0; k < warp && k < 4; ++k) pos += s_scan[k];
+    for (int j = j0; j < j1; ++j) {
+      uint32_t any = 0;
+      for (int k = 0; k < tile_words; ++k) any |= s_member[j * tile_words + k];
+      if (any) s_tiles[pos++] = (uint16_t)j;
+    }
+    if (tid == 0) *s_ntiles = s_scan[0] + s_scan[1] + s_scan[2] + s_scan[3];
+    __syncthreads();
+  };
+
+  int sent_k = 0, sent_v = 0, sent_q = 0;     // producer: loads sent so far (key tiles, row tiles)
+  int c = 0, it = 0;                          // running counts of key tiles and of live row tiles
+  bool ok = true;
+  // softmax threads: row of a tile = thread index
+  const int row = tid & (kFwdSoftmax - 1);
+  const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+  const int g = row / p.nq, ql = row % p.nq;
+
+  for (int w0 = blockIdx.x; w0 < n_work; w0 += kSel ? gridDim.x : n_work) {
+    if (kSel) build_list(w0);
+    const int w_end = kSel ? w0 + 1 : n_work;
+    if (warp == 4) {
+      // ---- producer -------------------------------------------------------------------------
+      if (lane == 0) {
+        for (int w = w0; ok && w < w_end; w += gridDim.x) {
+          const Tile x = tile_of(w);
+          if (x.n_tiles == 0) continue;
+          const int b = x.bh / p.Hkv, hkv = x.bh % p.Hkv;
+          if (it > 0) ok = mbar_wait(q_free, (it - 1) & 1, p.status, s_abort, 0x8000);
+          if (!ok) break;
+          mbar_expect_tx(bar_q, L::kQBytes);
 #pragma unroll
           for (int s = 0; s < kSlabs; ++s)
-            tma_load_3d(sK + st * L::kKVBytes + s * (kKeys * 128), &tm_k, bar_k + st, s * 64,
-                        x.first_key + i * kKeys, x.bh);
-          last_k[st] = c;
-          if (c >= 2) {
-            ok = mbar_wait(v_free + st, ((c >> 1) - 1) & 1, p.status, s_abort, 0x4000);
+            tma_load_3d(sQ + s * (kRows * 128), &tm_q, bar_q, s * 64, x.t0, b * p.Hq + hkv * p.G);
+          sent_q = ++it;
+          for (int i = 0; i < x.n_tiles; ++i, ++c) {
+            const int st = c % kStages, use = c / kStages, key0 = key0_of(x, i);
+            // a stage is free once the MMAs of the tile kStages back, which read it, are done
+            if (use > 0) ok = mbar_wait(k_free + st, (use - 1) & 1, p.status, s_abort, 0x4000);
             if (!ok) break;
-          }
-          if (!(p.debug_starve && c == 1)) {           // test only: this tile's wait has to run out
-            mbar_expect_tx(bar_v + st, L::kKVBytes);
+            mbar_expect_tx(bar_k + st, L::kKVBytes);
 #pragma unroll
             for (int s = 0; s < kSlabs; ++s)
-              tma_load_3d(sV + st * L::kKVBytes + s * (kKeys * 128), &tm_v, bar_v + st, s * 64,
-                          x.first_key + i * kKeys, x.bh);
-            last_v[st] = c;
+              tma_load_3d(sK + st * L::kKVBytes + s * (kKeys * 128), &tm_k, bar_k + st, s * 64, key0, x.bh);
+            sent_k = c + 1;
+            if (use > 0) ok = mbar_wait(v_free + st, (use - 1) & 1, p.status, s_abort, 0x4000);
+            if (!ok) break;
+            if (!(p.debug_starve && c == 1)) {           // test only: this tile's wait has to run out
+              mbar_expect_tx(bar_v + st, L::kKVBytes);
+#pragma unroll
+              for (int s = 0; s < kSlabs; ++s)
+                tma_load_3d(sV + st * L::kKVBytes + s * (kKeys * 128), &tm_v, bar_v + st, s * 64, key0, x.bh);
+              sent_v = c + 1;
+            }
           }
         }
-        ++it;
       }
-    }
-  } else if (warp == 5) {
-    // ---- MMA issuer ------------------------------------------------------------------------
-    if (lane == 0) {
-      int c = 0, it = 0;
-      bool ok = true;
-      auto issue_s = [&](int cc) {   // S = Q K^T for running key tile cc, Q from tensor memory
-        const uint32_t ka = desc_lo_kmajor(smem_u32(sK + (cc & 1) * L::kKVBytes));
+    } else if (warp == 5) {
+      // ---- MMA issuer ------------------------------------------------------------------------
+      if (lane == 0) {
+        auto issue_s = [&](int cc, bool last) {   // S = Q K^T of running key tile cc
+          const int st = cc % kStages;
+          const uint32_t qa = desc_lo_kmajor(smem_u32(sQ)), ka = desc_lo_kmajor(smem_u32(sK + st * L::kKVBytes));
 #pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) {
-          const uint32_t slab = kk >> 2, in = (kk & 3) * 32;
-          mma_ts(tmem + kColS, tmem + kColQ + kk * 8, desc_at(ka, slab * (kKeys * 128) + in), kIdescQK, kk > 0);
-        }
-        tc_commit(bar_s);
-        tc_commit(k_free + (cc & 1));
-      };
-      for (int w = blockIdx.x; ok && w < n_work; w += gridDim.x) {
-        const Tile x = tile_of(w);
-        if (x.n_tiles == 0) continue;
-        ok = mbar_wait(bar_qt, it & 1, p.status, s_abort, 0x8000) &&
-             mbar_wait(bar_k + (c & 1), (c >> 1) & 1, p.status, s_abort, 2);
-        if (!ok) break;
-        tc_fence_after();
-        issue_s(c);                                     // (after the last PV of the previous row tile: P lies over S)
-        for (int i = 0; i < x.n_tiles; ++i, ++c) {
-          ok = mbar_wait(bar_p, c & 1, p.status, s_abort, 0x2000) &&
-               mbar_wait(bar_v + (c & 1), (c >> 1) & 1, p.status, s_abort, 16);
+          for (int kk = 0; kk < D / 16; ++kk) {
+            const uint32_t slab = kk >> 2, in = (kk & 3) * 32;
+            mma_ss(tmem + kColS + (cc & 1) * kKeys, desc_at(qa, slab * (kRows * 128) + in),
+                   desc_at(ka, slab * (kKeys * 128) + in), kIdescQK, kk > 0);
+          }
+          tc_commit(bar_s + (cc & 1));
+          tc_commit(k_free + st);
+          if (last) tc_commit(q_free);
+        };
+        for (int w = w0; ok && w < w_end; w += gridDim.x) {
+          const Tile x = tile_of(w);
+          if (x.n_tiles == 0) continue;
+          ok = mbar_wait(bar_q, it & 1, p.status, s_abort, 1) &&
+               mbar_wait(bar_k + c % kStages, (c / kStages) & 1, p.status, s_abort, 2);
+          // An S MMA overwrites the P of two key tiles back: that tile's PV has to be complete (MMAs of
+          // different shapes and operand sources are not ordered by their issue).  Here every earlier
+          // one is waited for; the threads that write the last row tile's output wait for it as well.
+          if (ok && c > 0) ok = mbar_wait(bar_o + ((c - 1) & 1), ((c - 1) >> 1) & 1, p.status, s_abort, 0x2000);
           if (!ok) break;
           tc_fence_after();
-          {                                             // O (+)= P V
-            const uint32_t va = desc_lo_mnmajor(smem_u32(sV + (c & 1) * L::kKVBytes), kKeys * 128);
+          issue_s(c, x.n_tiles == 1);
+          for (int i = 0; i < x.n_tiles; ++i, ++c) {
+            if (i + 1 < x.n_tiles) {
+              ok = mbar_wait(bar_k + (c + 1) % kStages, ((c + 1) / kStages) & 1, p.status, s_abort, 2);
+              if (ok && i > 0) ok = mbar_wait(bar_o + ((c - 1) & 1), ((c - 1) >> 1) & 1, p.status, s_abort, 0x2000);
+              if (!ok) break;
+              tc_fence_after();
+              issue_s(c + 1, i + 2 == x.n_tiles);
+            }
+            const int st = c % kStages;
+            ok = mbar_wait(bar_p + (c & 1), (c >> 1) & 1, p.status, s_abort, 0x2000) &&
+                 mbar_wait(bar_v + st, (c / kStages) & 1, p.status, s_abort, 16);
+            if (!ok) break;
+            tc_fence_after();
+            const uint32_t va = desc_lo_mnmajor(smem_u32(sV + st * L::kKVBytes), kKeys * 128);   // O (+)= P V
 #pragma unroll
             for (int kk = 0; kk < kKeys / 16; ++kk)
-              mma_ts(tmem + kColO, tmem + kColS + kk * 8, desc_at(va, kk * 2048), kIdescPV, (i > 0) || (kk > 0));
-            tc_commit(bar_o);
-            tc_commit(v_free + (c & 1));
+              mma_ts(tmem + kColO, tmem + kColS + (c & 1) * kKeys + kk * 8, desc_at(va, kk * 2048), kIdescPV, (i > 0) || (kk > 0));
+            tc_commit(bar_o + (c & 1));
+            tc_commit(v_free + st);
           }
-          if (i + 1 < x.n_tiles) {
-            ok = mbar_wait(bar_k + ((c + 1) & 1), ((c + 1) >> 1) & 1, p.status, s_abort, 2);
-            if (!ok) break;
-            issue_s(c + 1);
-          }
+          ++it;
         }
-        ++it;
       }
-      tc_commit(bar_drain);
-      if (!mbar_wait(bar_drain, 0, p.status, s_abort, 0x1000)) mbar_wait_drain(bar_drain, 0);
-    }
-  } else {
-    // ---- softmax: thread = row ---------------------------------------------------------------
-    const int row = tid;
-    const uint32_t lane_base = tmem + ((uint32_t)(warp * 32) << 16);
-    const int g = row / p.nq, ql = row % p.nq;
-    auto q_to_tmem = [&]() {       // this thread's row of the Q tile: shared memory -> tensor memory
-#pragma unroll
-      for (int sl = 0; sl < kSlabs; ++sl) {
-        const uint8_t* src = sQ + sl * (kRows * 128) + row * 128;
-        uint32_t qv[32];
-#pragma unroll
-        for (int cch = 0; cch < 8; ++cch) {
-          const uint4 u = *reinterpret_cast<const uint4*>(src + ((cch ^ (row & 7)) << 4));
-          qv[4 * cch + 0] = u.x; qv[4 * cch + 1] = u.y; qv[4 * cch + 2] = u.z; qv[4 * cch + 3] = u.w;
-        }
-        tmem_st32(lane_base + kColQ + sl * 32, qv);
-      }
-      tmem_wait_st();
-      tc_fence_before();
-      mbar_arrive(bar_qt);
-    };
-    int c = 0, it = 0;
-    bool ok = true;
-    // the first live row tile's Q
-    int w = blockIdx.x;
-    Tile x = tile_of(w < n_work ? w : 0);
-    auto skip_empty = [&]() {      // rows without a key: zeros, no barrier is touched
-      while (w < n_work && x.n_tiles == 0) {
+    } else {
+      // ---- softmax: thread = row ---------------------------------------------------------------
+      for (int w = w0; w < w_end; w += gridDim.x) {
+        const Tile x = tile_of(w);
         const int t = x.t0 + ql;
-        if (g < p.G && t < p.T) {
-          const int head = (x.bh % p.Hkv) * p.G + g, b = x.bh / p.Hkv;
-          uint4* dst = reinterpret_cast<uint4*>(p.o + ((size_t)(b * p.Hq + head) * p.T + t) * D);
-#pragma unroll
-          for (int v4 = 0; v4 < D / 8; ++v4) dst[v4] = make_uint4(0, 0, 0, 0);
-          p.lse[(size_t)(b * p.Hq + head) * p.T + t] = kLseEmpty;
-        }
-        w += gridDim.x;
-        if (w < n_work) x = tile_of(w);
-      }
-    };
-    skip_empty();
-    if (w < n_work) {
-      ok = mbar_wait(bar_q, 0, p.status, s_abort, 1);
-      q_to_tmem();
-    }
-    while (w < n_work) {
-      const int t = x.t0 + ql;
-      const bool row_ok = (g < p.G) && (t < p.T);
-      const int b = x.bh / p.Hkv, head = (x.bh % p.Hkv) * p.G + g;
-      float m_used = -INFINITY, l_sum = 0.f;
-      for (int i = 0; i < x.n_tiles; ++i, ++c) {
-        const int key0 = x.first_key + i * kKeys;
-        ok = mbar_wait(bar_s, c & 1, p.status, s_abort, 4) && ok;
-        if (!__all_sync(0xffffffffu, ok)) break;              // the whole warp leaves together
-        tc_fence_after();
-        uint32_t r[64];
-        tmem_ld32(lane_base + kColS, r);
-        tmem_ld32(lane_base + kColS + 32, r + 32);
-        tmem_wait_ld();
-        int lo = 0, hi = -1;
-        if (row_ok) {
-          if (p.kind == 0) {
-            lo = max(0, t - p.window + 1 - key0);
-            hi = min(kKeys - 1, t - key0);
-          } else {
-            hi = min(kKeys - 1, cmp_visible(t, p.block_size, p.window, p.Lk) - 1 - key0);
-          }
-        }
-        float xs[64];
-        float tmax = -INFINITY;
-        if (lo <= 0 && hi >= kKeys - 1) {
-#pragma unroll
-          for (int cc = 0; cc < 64; ++cc) {
-            xs[cc] = __uint_as_float(r[cc]) * p.scale_log2;
-            tmax = fmaxf(tmax, xs[cc]);
-          }
-        } else {
-#pragma unroll
-          for (int cc = 0; cc < 64; ++cc) {
-            xs[cc] = (cc >= lo && cc <= hi) ? __uint_as_float(r[cc]) * p.scale_log2 : -INFINITY;
-            tmax = fmaxf(tmax, xs[cc]);
-          }
-        }
-        float alpha = 1.f;
-        bool rescale = false;
-        if (tmax > m_used + 8.f) {              // also the first finite maximum (m_used = -inf)
-          if (m_used != -INFINITY) {
-            alpha = ex2(m_used - tmax);
-            rescale = true;
-            l_sum *= alpha;
-          }
-          m_used = tmax;
-        }
-        const float msub = (m_used == -INFINITY) ? 0.f : m_used;
-        float psum = 0.f;
-        uint32_t pk[32];
-#pragma unroll
-        for (int cc = 0; cc < 32; ++cc) {
-          const float p0 = ex2(xs[2 * cc] - msub), p1 = ex2(xs[2 * cc + 1] - msub);
-          psum += p0 + p1;
-          pk[cc] = pack_bf16(p0, p1);
-        }
-        l_sum += psum;
-        // O may be touched once PV of the tile before is done; only a warp that has to rescale waits
-        if (i > 0 && __any_sync(0xffffffffu, rescale)) {
-          ok = mbar_wait(bar_o, (c - 1) & 1, p.status, s_abort, 8);
-          if (!__all_sync(0xffffffffu, ok)) break;
-          tc_fence_after();
-#pragma unroll
-          for (int cc = 0; cc < D / 32; ++cc) {
-            uint32_t o32[32];
-            tmem_ld32(lane_base + kColO + cc * 32, o32);
-            tmem_wait_ld();
-#pragma unroll
-            for (int e = 0; e < 32; ++e) o32[e] = __float_as_uint(__uint_as_float(o32[e]) * alpha);
-            tmem_st32(lane_base + kColO + cc * 32, o32);
-          }
-        }
-        tmem_st32(lane_base + kColS, pk);        // over the S columns this thread has just read
-        tmem_wait_st();
-        tc_fence_before();
-        mbar_arrive(bar_p);
-      }
-      if (!__all_sync(0xffffffffu, ok)) break;
-      // next live row tile: its Q goes into tensor memory now (every S of this tile is done: the
-      // last one was read above), so that its first S runs while this tile's output is written
-      const int w_cur = w;
-      const Tile x_cur = x;
-      w += gridDim.x;
-      if (w < n_work) x = tile_of(w);
-      skip_empty();
-      ++it;
-      if (w < n_work) {
-        ok = mbar_wait(bar_q, it & 1, p.status, s_abort, 1);
-        if (!__all_sync(0xffffffffu, ok)) break;
-        q_to_tmem();
-      }
-      (void)w_cur;
-      // ---- this tile's output: the last PV, then O / l -------------------------------------
-      ok = mbar_wait(bar_o, (c - 1) & 1, p.status, s_abort, 8);
-      if (!__all_sync(0xffffffffu, ok)) break;
-      tc_fence_after();
-      {
-        const float inv = l_sum > 0.f ? 1.f / l_sum : 0.f;
+        const bool row_ok = (g < p.G) && (t < p.T);
+        const int b = x.bh / p.Hkv, head = (x.bh % p.Hkv) * p.G + g;
         __nv_bfloat16* orow = p.o + ((size_t)(b * p.Hq + head) * p.T + t) * D;
+        float* lrow = p.lse + (size_t)(b * p.Hq + head) * p.T + t;
+        if (x.n_tiles == 0) {                       // rows without a key: zeros, no barrier is touched
+          if (row_ok) {
+            uint4* dst = reinterpret_cast<uint4*>(orow);
+#pragma unroll
+            for (int v4 = 0; v4 < D / 8; ++v4) dst[v4] = make_uint4(0, 0, 0, 0);
+            *lrow = kLseEmpty;
+          }
+          continue;
+        }
+        float m_used = -INFINITY, l_sum = 0.f;      // m_used in units of raw scores
+        for (int i = 0; i < x.n_tiles; ++i, ++c) {
+          const int key0 = key0_of(x, i);
+          // valid columns of this row in this tile: one range [lo, hi] and, for selection, 16-column groups
+          int lo = 0, hi = -1;
+          uint32_t groups = 0xfu;
+          if (row_ok) {
+            if (kSel) {
+              hi = min(kKeys - 1, t - key0);
+              const uint32_t* mem = s_member + (key0 / kKeys) * tile_words + (ql >> 5);
+              if (p.n_sub == 1) {
+                if (!((mem[0] >> (ql & 31)) & 1u)) hi = -1;
+              } else {
+                groups = 0u;
+                for (int k = 0; k < p.n_sub; ++k)
+                  if ((mem[k * p.nw] >> (ql & 31)) & 1u) groups |= ((1u << (p.block_size >> 4)) - 1u) << (k * (p.block_size >> 4));
+              }
+            } else if (p.kind == 0) {
+              lo = max(0, t - p.window + 1 - key0);
+              hi = min(kKeys - 1, t - key0);
+            } else {
+              hi = min(kKeys - 1, cmp_visible(t, p.block_size, p.window, p.Lk) - 1 - key0);
+            }
+          }
+          ok = mbar_wait(bar_s + (c & 1), (c >> 1) & 1, p.status, s_abort, 4) && ok;
+          if (!__all_sync(0xffffffffu, ok)) break;              // the whole warp leaves together
+          tc_fence_after();
+          const uint32_t s_base = lane_base + kColS + (c & 1) * kKeys;
+          uint32_t r[64];
+          tmem_ld32(s_base, r);
+          tmem_ld32(s_base + 32, r + 32);
+          tmem_wait_ld();
+          if (!(lo <= 0 && hi >= kKeys - 1 && groups == 0xfu)) {
+#pragma unroll
+            for (int cc = 0; cc < 64; ++cc)
+              if (!(cc >= lo && cc <= hi && ((groups >> (cc >> 4)) & 1u))) r[cc] = 0xff800000u;   // -inf
+          }
+          float tmax[4];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) tmax[k] = __uint_as_float(r[k]);
+#pragma unroll
+          for (int cc = 4; cc < 64; ++cc) tmax[cc & 3] = fmaxf(tmax[cc & 3], __uint_as_float(r[cc]));
+          const float tm = fmaxf(fmaxf(tmax[0], tmax[1]), fmaxf(tmax[2], tmax[3]));
+          // the running maximum is only raised when it grows by more than 8 powers of two
+          float alpha = 1.f;
+          bool rescale = false;
+          if ((tm - m_used) * p.scale_log2 > 8.f) {              // also the first finite maximum (m_used = -inf)
+            if (m_used != -INFINITY) {
+              alpha = ex2((m_used - tm) * p.scale_log2);
+              rescale = true;
+              l_sum *= alpha;
+            }
+            m_used = tm;
+          }
+          const float msub = (m_used == -INFINITY) ? 0.f : m_used * p.scale_log2;
+          const uint64_t sc2 = pack_f32x2(p.scale_log2, p.scale_log2), mn2 = pack_f32x2(-msub, -msub);
+          uint64_t ps[2] = {0ull, 0ull};
+          uint32_t pk[32];
+#pragma unroll
+          for (int cc = 0; cc < 32; ++cc) {
+            float p0, p1;
+            unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(r[2 * cc]), __uint_as_float(r[2 * cc + 1])), sc2, mn2), p0, p1);
+            p0 = ex2(p0);
+            p1 = ex2(p1);
+            ps[cc & 1] = add_f32x2(ps[cc & 1], pack_f32x2(p0, p1));
+            pk[cc] = pack_bf16(p0, p1);
+          }
+          float s0, s1;
+          unpack_f32x2(add_f32x2(ps[0], ps[1]), s0, s1);
+          l_sum += s0 + s1;
+          // O may be touched once PV of the tile before is done; only a warp that has to rescale waits
+          if (i > 0 && __any_sync(0xffffffffu, rescale)) {
+            ok = mbar_wait(bar_o + ((c - 1) & 1), ((c - 1) >> 1) & 1, p.status, s_abort, 8);
+            if (!__all_sync(0xffffffffu, ok)) break;
+            tc_fence_after();
+#pragma unroll
+            for (int cc = 0; cc < D / 32; ++cc) {
+              uint32_t o32[32];
+              tmem_ld32(lane_base + kColO + cc * 32, o32);
+              tmem_wait_ld();
+#pragma unroll
+              for (int e = 0; e < 32; ++e) o32[e] = __float_as_uint(__uint_as_float(o32[e]) * alpha);
+              tmem_st32(lane_base + kColO + cc * 32, o32);
+            }
+          }
+          tmem_st32(s_base, pk);                   // over the S columns this thread has just read
+          tmem_wait_st();
+          tc_fence_before();
+          mbar_arrive(bar_p + (c & 1));
+        }
+        if (!__all_sync(0xffffffffu, ok)) break;
+        // ---- this row tile's output: the last PV, then O / l -------------------------------------
+        ok = mbar_wait(bar_o + ((c - 1) & 1), ((c - 1) >> 1) & 1, p.status, s_abort, 8);
+        if (!__all_sync(0xffffffffu, ok)) break;
+        tc_fence_after();
+        const float inv = l_sum > 0.f ? 1.f / l_sum : 0.f;
 #pragma unroll
         for (int cc = 0; cc < D / 32; ++cc) {
           uint32_t o32[32];
@@ -788,13 +453,17 @@ tc_fwd_range_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             }
           }
         }
-        if (row_ok)
-          p.lse[(size_t)(b * p.Hq + head) * p.T + t] =
-              l_sum > 0.f ? (m_used + log2f(l_sum)) * kLn2 : kLseEmpty;
-        (void)x_cur;
+        if (row_ok) *lrow = l_sum > 0.f ? (m_used * p.scale_log2 + log2f(l_sum)) * kLn2 : kLseEmpty;
+        tc_fence_before();     // the O columns are read: the next row tile's first PV (behind this thread's next P) may overwrite them
       }
-      tc_fence_before();     // the O columns are read: the next tile's first PV (behind this thread's next P) may overwrite them
     }
+    // the row tile's list may be overwritten once every role is through with it
+    if (kSel && __syncthreads_or(*s_abort)) break;
+  }
+  if (warp == 5 && lane == 0) {
+    // the tensor pipe is idle before tensor memory is given back, whatever happened
+    tc_commit(bar_drain);
+    if (!mbar_wait(bar_drain, 0, p.status, s_abort, 0x1000)) mbar_wait_drain(bar_drain, 0);
   }
 
   // ---- teardown -------------------------------------------------------------------------------
@@ -802,17 +471,14 @@ tc_fwd_range_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   __syncthreads();
   tc_fence_after();
   if (*s_abort) {
-    // Give-up path.  The producer waits (bounded) for the loads still on their way into this
-    // CTA's shared memory; the MMA thread has waited for the tensor pipe above.
+    // Give-up path: nothing more is written.  The producer waits (bounded) for the loads still on
+    // their way into this CTA's shared memory; the MMA thread has waited for the tensor pipe above.
     if (warp == 4 && lane == 0) {
-      if (q_sent > 0) mbar_wait_drain(bar_q, (q_sent - 1) & 1);
-#pragma unroll
-      for (int st = 0; st < 2; ++st) {
-        if (last_k[st] >= 0) mbar_wait_drain(bar_k + st, (last_k[st] >> 1) & 1);
-        if (last_v[st] >= 0) mbar_wait_drain(bar_v + st, (last_v[st] >> 1) & 1);
-      }
+      if (sent_q > 0) mbar_wait_drain(bar_q, (sent_q - 1) & 1);
+      for (int k = max(0, sent_k - kStages); k < sent_k; ++k) mbar_wait_drain(bar_k + k % kStages, (k / kStages) & 1);
+      for (int k = max(0, sent_v - kStages); k < sent_v; ++k)
+        if (!(p.debug_starve && k == 1)) mbar_wait_drain(bar_v + k % kStages, (k / kStages) & 1);
     }
-    if (warp == 5 && lane == 0) mbar_wait_drain(bar_drain, 0);
     __syncthreads();
   }
   if (warp == 0) tmem_dealloc(tmem, kTmemCols);
@@ -832,7 +498,7 @@ bool tc_shape_ok(const NsaDims& d, int block_size) {
   const int nq = tc::kRows / tc::group_pad(G);
   const int nb = (d.T + tc::kKeys - 1) / tc::kKeys;
   if (nb > 65535) return false;
-  if (tc::fwd_smem_bytes(d.D, nb, nq >= 32 ? nq / 32 : 1, tc::kKeys / block_size, 2) > 112 * 1024) return false;
+  if (tc::fwd_smem_bytes(d.D, nb, nq >= 32 ? nq / 32 : 1, tc::kKeys / block_size, 2) > 224 * 1024) return false;
   return true;
 }
 
@@ -864,31 +530,20 @@ static int launch_fwd(const AttnArgs& a, const SelPlanHeader* plan, int force, c
   if (rc == NSA_OK) rc = make_map(&tm_v, a.v, a.D, a.Lk, a.B * a.Hkv, kKeys, 1);
   if (rc != NSA_OK) return rc;
   const size_t smem = fwd_smem_bytes(a.D, p.nb_sel, p.nw, p.n_sub, a.kind);
-  if (a.kind != 2) {
-    // window / compression: persistent CTAs, two per SM, each walking its share of the row tiles
-    const int sms = sm_count();
-    const long long n_work = (long long)p.n_qtiles * a.B * a.Hkv;
-    if (n_work == 0) return NSA_OK;
-    const unsigned g1 = (unsigned)(n_work < 2LL * sms ? n_work : 2LL * sms);
-    KernelScope ks(branch_name(kFwdNames, a.kind), st);
-    if (a.D == 128) {
-      NSA_CUDA_OK(func_smem((const void*)tc_fwd_range_kernel<128>, smem));
-      tc_fwd_range_kernel<128><<<g1, kFwdThreads, smem, st>>>(tm_q, tm_k, tm_v, p);
-    } else {
-      NSA_CUDA_OK(func_smem((const void*)tc_fwd_range_kernel<64>, smem));
-      tc_fwd_range_kernel<64><<<g1, kFwdThreads, smem, st>>>(tm_q, tm_k, tm_v, p);
-    }
-    NSA_LAUNCH_OK("tc_fwd_range_kernel");
+  // persistent CTAs, two per SM, each walking its share of the row tiles
+  const long long n_work = (long long)p.n_qtiles * a.B * a.Hkv;
+  if (n_work == 0) return NSA_OK;
+  NSA_CHECK_ARG(n_work < (1LL << 31), "too many row tiles");
+  const unsigned grid = (unsigned)std::min<long long>(n_work, 2LL * sm_count());
+  KernelScope ks(branch_name(kFwdNames, a.kind), st);
+  auto go = [&](auto kernel) -> int {
+    NSA_CUDA_OK(func_smem((const void*)kernel, smem));
+    kernel<<<grid, kFwdThreads, smem, st>>>(tm_q, tm_k, tm_v, p);
     return NSA_OK;
-  }
-  dim3 grid(p.n_qtiles, a.B * a.Hkv);
-  if (a.D == 128) {
-    NSA_CUDA_OK(func_smem((const void*)tc_fwd_kernel<128>, smem));
-    { KernelScope ks(branch_name(kFwdNames, a.kind), st); tc_fwd_kernel<128><<<grid, kFwdThreads, smem, st>>>(tm_q, tm_k, tm_v, p); }
-  } else {
-    NSA_CUDA_OK(func_smem((const void*)tc_fwd_kernel<64>, smem));
-    { KernelScope ks(branch_name(kFwdNames, a.kind), st); tc_fwd_kernel<64><<<grid, kFwdThreads, smem, st>>>(tm_q, tm_k, tm_v, p); }
-  }
+  };
+  if (a.D == 128) rc = a.kind == 2 ? go(tc_fwd_kernel<128, true>) : go(tc_fwd_kernel<128, false>);
+  else rc = a.kind == 2 ? go(tc_fwd_kernel<64, true>) : go(tc_fwd_kernel<64, false>);
+  if (rc != NSA_OK) return rc;
   NSA_LAUNCH_OK("tc_fwd_kernel");
   return NSA_OK;
 }
