@@ -1,8 +1,9 @@
 // tcgen05 / TMEM attention kernels for sm_100a.
 //
-// One CTA owns a tile of 128 rows = nq consecutive query tokens x the Gp query heads of one
-// (batch, kv head) group (row r -> head r / nq, token r % nq), so the heads of a GQA group
-// share every K/V tile.  The CTA walks a list of 64-key tiles:
+// One CTA owns a tile of 128 rows = nq consecutive query tokens x the G query heads of one
+// (batch, kv head) group (row r -> token r / G, head r % G), so the heads of a GQA group share
+// every K/V tile; nq = 128 / G, so a group of 3 fills 126 rows (padded to 4, as an earlier version had
+// it, it filled 96).  The CTA walks a list of 64-key tiles:
 //   window      the tiles covering [t_first - W + 1, t_last]
 //   compression the tiles covering summaries [0, (t_last + 1) / Bsz - 1]
 //   selection   the 64-key tiles holding blocks (of 16, 32 or 64 tokens) listed for the tile's nq
@@ -27,13 +28,14 @@ struct FwdArgs {
   __nv_bfloat16* o;
   float* lse;
   int* status;
-  int B, Hq, Hkv, T, Lk, S, G, Gp, nq;
+  int B, Hq, Hkv, T, Lk, S, G, nq;
   int kind, window, block_size;
   const SelPlanHeader* plan;         // selection: statistics for the variant choice (null: this kernel serves the call)
   int force;
+  int nq_union;              // queries per query tile in the plan's statistics (G padded to a power of two)
   int debug_starve;          // test only: the V load of the second key tile is never sent
   int n_qtiles, nb_sel;      // nb_sel = ceil(T / 64) key tiles a selection list may name
-  int nw;                    // 32-bit membership words per block = max(1, nq / 32)
+  int nw;                    // 32-bit membership words per block = ceil(nq / 32)
   int n_sub;                 // selection: list blocks per 64-key tile (64 / block_size)
   float scale_log2;
 };
@@ -132,7 +134,7 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   const int tile_words = p.n_sub * p.nw;
   uint16_t* s_tiles = (uint16_t*)(s_member + (kSel ? p.nb_sel * tile_words : 0));
 
-  if (kSel && p.plan != nullptr && prefer_pairs(p.plan, p.nq, p.force))
+  if (kSel && p.plan != nullptr && prefer_pairs(p.plan, p.nq_union, p.force))
     return;   // the block-outer variant serves this call: leave before anything is set up
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) {
@@ -229,7 +231,7 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   // softmax threads: row of a tile = thread index
   const int row = tid & (kFwdSoftmax - 1);
   const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) * 32) << 16);
-  const int g = row / p.nq, ql = row % p.nq;
+  const int ql = row / p.G, g = row % p.G;
 
   for (int w0 = blockIdx.x; w0 < n_work; w0 += kSel ? gridDim.x : n_work) {
     if (kSel) build_list(w0);
@@ -243,10 +245,10 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           const int b = x.bh / p.Hkv, hkv = x.bh % p.Hkv;
           if (it > 0) ok = mbar_wait(q_free, (it - 1) & 1, p.status, s_abort, 0x8000);
           if (!ok) break;
-          mbar_expect_tx(bar_q, L::kQBytes);
+          mbar_expect_tx(bar_q, (uint32_t)(p.nq * p.G * 128 * kSlabs));
 #pragma unroll
           for (int s = 0; s < kSlabs; ++s)
-            tma_load_3d(sQ + s * (kRows * 128), &tm_q, bar_q, s * 64, x.t0, b * p.Hq + hkv * p.G);
+            tma_load_3d(sQ + s * (kRows * 128), &tm_q, bar_q, s * 64, b * p.Hq + hkv * p.G, x.t0);
           sent_q = ++it;
           for (int i = 0; i < x.n_tiles; ++i, ++c) {
             const int st = c % kStages, use = c / kStages, key0 = key0_of(x, i);
@@ -326,7 +328,7 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       for (int w = w0; w < w_end; w += gridDim.x) {
         const Tile x = tile_of(w);
         const int t = x.t0 + ql;
-        const bool row_ok = (g < p.G) && (t < p.T);
+        const bool row_ok = ql < p.nq && t < p.T;
         const int b = x.bh / p.Hkv, head = (x.bh % p.Hkv) * p.G + g;
         __nv_bfloat16* orow = p.o + ((size_t)(b * p.Hq + head) * p.T + t) * D;
         float* lrow = p.lse + (size_t)(b * p.Hq + head) * p.T + t;
@@ -362,6 +364,7 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
             } else {
               hi = min(kKeys - 1, cmp_visible(t, p.block_size, p.window, p.Lk) - 1 - key0);
             }
+            if (lo > hi) { lo = 0; hi = -1; }
           }
           ok = mbar_wait(bar_s + (c & 1), (c >> 1) & 1, p.status, s_abort, 4) && ok;
           if (!__all_sync(0xffffffffu, ok)) break;              // the whole warp leaves together
@@ -371,17 +374,32 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           tmem_ld32(s_base, r);
           tmem_ld32(s_base + 32, r + 32);
           tmem_wait_ld();
-          if (!(lo <= 0 && hi >= kKeys - 1 && groups == 0xfu)) {
+          // A row that attends the whole tile or none of it, or whole 16-column groups of it, needs no
+          // work per element: a group it does not attend gets the exponent 0 * s - inf.  Only rows whose
+          // range ends inside the tile mask their columns one by one.
+          if (!(lo <= 0 && (hi >= kKeys - 1 || hi < 0))) {
 #pragma unroll
             for (int cc = 0; cc < 64; ++cc)
-              if (!(cc >= lo && cc <= hi && ((groups >> (cc >> 4)) & 1u))) r[cc] = 0xff800000u;   // -inf
+              if (cc < lo || cc > hi) r[cc] = __float_as_uint(-3.0e38f);   // finite: 0 * r has to be 0
           }
-          float tmax[4];
+          float tmax[4];                      // of the four column groups
 #pragma unroll
-          for (int k = 0; k < 4; ++k) tmax[k] = __uint_as_float(r[k]);
+          for (int k = 0; k < 4; ++k) {
+            float m0 = __uint_as_float(r[16 * k]), m1 = __uint_as_float(r[16 * k + 1]);
 #pragma unroll
-          for (int cc = 4; cc < 64; ++cc) tmax[cc & 3] = fmaxf(tmax[cc & 3], __uint_as_float(r[cc]));
-          const float tm = fmaxf(fmaxf(tmax[0], tmax[1]), fmaxf(tmax[2], tmax[3]));
+            for (int cc = 2; cc < 16; cc += 2) {
+              m0 = fmaxf(m0, __uint_as_float(r[16 * k + cc]));
+              m1 = fmaxf(m1, __uint_as_float(r[16 * k + cc + 1]));
+            }
+            tmax[k] = fmaxf(m0, m1);
+          }
+          if (hi < 0) groups = 0u;
+          if (kSel) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) tmax[k] = ((groups >> k) & 1u) ? tmax[k] : -INFINITY;
+          }
+          float tm = fmaxf(fmaxf(tmax[0], tmax[1]), fmaxf(tmax[2], tmax[3]));
+          if (!kSel) tm = hi < 0 ? -INFINITY : tm;
           // the running maximum is only raised when it grows by more than 8 powers of two
           float alpha = 1.f;
           bool rescale = false;
@@ -394,13 +412,21 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
             m_used = tm;
           }
           const float msub = (m_used == -INFINITY) ? 0.f : m_used * p.scale_log2;
-          const uint64_t sc2 = pack_f32x2(p.scale_log2, p.scale_log2), mn2 = pack_f32x2(-msub, -msub);
+          uint64_t sc2[kSel ? 4 : 1], mn2[kSel ? 4 : 1];
+#pragma unroll
+          for (int k = 0; k < (kSel ? 4 : 1); ++k) {
+            const bool on = (groups >> k) & 1u;
+            const float sc = on ? p.scale_log2 : 0.f, mn = on ? -msub : -INFINITY;
+            sc2[k] = pack_f32x2(sc, sc);
+            mn2[k] = pack_f32x2(mn, mn);
+          }
           uint64_t ps[2] = {0ull, 0ull};
           uint32_t pk[32];
 #pragma unroll
           for (int cc = 0; cc < 32; ++cc) {
             float p0, p1;
-            unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(r[2 * cc]), __uint_as_float(r[2 * cc + 1])), sc2, mn2), p0, p1);
+            unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(r[2 * cc]), __uint_as_float(r[2 * cc + 1])), sc2[kSel ? cc >> 3 : 0],
+                                   mn2[kSel ? cc >> 3 : 0]), p0, p1);
             p0 = ex2(p0);
             p1 = ex2(p1);
             ps[cc & 1] = add_f32x2(ps[cc & 1], pack_f32x2(p0, p1));
@@ -495,10 +521,10 @@ bool tc_shape_ok(const NsaDims& d, int block_size) {
   const int G = d.Hq / d.Hkv;
   if (G < 2 || G > 128) return false;   // the backward tiles hold at most 64 queries
   if (d.T < 1) return false;
-  const int nq = tc::kRows / tc::group_pad(G);
+  const int nq = tc::kRows / G;
   const int nb = (d.T + tc::kKeys - 1) / tc::kKeys;
   if (nb > 65535) return false;
-  if (tc::fwd_smem_bytes(d.D, nb, nq >= 32 ? nq / 32 : 1, tc::kKeys / block_size, 2) > 224 * 1024) return false;
+  if (tc::fwd_smem_bytes(d.D, nb, (nq + 31) / 32, tc::kKeys / block_size, 2) > 224 * 1024) return false;
   return true;
 }
 
@@ -507,7 +533,7 @@ int get_option_debug_starve_load();   // api.cu
 static int launch_fwd(const AttnArgs& a, const SelPlanHeader* plan, int force, cudaStream_t st) {
   using namespace tc;
   FwdArgs p;
-  p.plan = plan; p.force = force;
+  p.plan = plan; p.force = force; p.nq_union = kRows / group_pad(a.Hq / a.Hkv);
   p.debug_starve = get_option_debug_starve_load();
   p.block_idx = a.block_idx;
   p.o = (__nv_bfloat16*)a.o;
@@ -516,16 +542,15 @@ static int launch_fwd(const AttnArgs& a, const SelPlanHeader* plan, int force, c
   if (!p.status) { set_error("device status word unavailable"); return NSA_ERR_CUDA; }
   p.B = a.B; p.Hq = a.Hq; p.Hkv = a.Hkv; p.T = a.T; p.Lk = a.Lk; p.S = a.S;
   p.G = a.Hq / a.Hkv;
-  p.Gp = group_pad(p.G);
-  p.nq = kRows / p.Gp;
+  p.nq = kRows / p.G;
   p.kind = a.kind; p.window = a.window; p.block_size = a.block_size;
   p.n_qtiles = (a.T + p.nq - 1) / p.nq;
   p.nb_sel = (a.T + kKeys - 1) / kKeys;
-  p.nw = p.nq >= 32 ? p.nq / 32 : 1;
+  p.nw = (p.nq + 31) / 32;
   p.n_sub = a.kind == 2 ? kKeys / a.block_size : 1;
   p.scale_log2 = a.scale * kLog2e;
   CUtensorMap tm_q, tm_k, tm_v;
-  int rc = make_map(&tm_q, a.q, a.D, a.T, a.B * a.Hq, p.nq, p.Gp);
+  int rc = make_map_query_rows(&tm_q, a.q, a.D, a.T, a.B * a.Hq, p.G, p.nq);
   if (rc == NSA_OK) rc = make_map(&tm_k, a.k, a.D, a.Lk, a.B * a.Hkv, kKeys, 1);
   if (rc == NSA_OK) rc = make_map(&tm_v, a.v, a.D, a.Lk, a.B * a.Hkv, kKeys, 1);
   if (rc != NSA_OK) return rc;
