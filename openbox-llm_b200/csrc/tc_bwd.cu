@@ -537,18 +537,35 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
 }
 
 // ---- the same backward with the issuing taken out of the compute groups ---------------------------
-// Two row tiles are in flight (shared memory holds no more: Q, dO, P, dS of a tile are 96 KB), one
-// per slot.  Three producer warps refill a slot's Q / dO the moment its MMAs are done; one thread
-// issues whichever batch of MMAs is ready next (S / dP of the tile that has landed, or dV / dK / dQ
-// of the tile whose probabilities are written); each slot has a compute group of 256 threads (two
-// warps per TMEM lane quadrant, half of the key columns each) that turns S / dP into P / dS and,
-// while the slot's next tile is on its way, moves the tile's dQ from TMEM to the staging tile and
-// stores it.  Each hand-over is an mbarrier with a bounded wait.  The tensor pipe needs about 2.9 k
-// cycles per row tile (80-100 cycles per MMA instruction: their shared-memory operands, not the
-// arithmetic); the aim of this arrangement is to keep it fed.
-constexpr int kB2Threads = 640;   // 2 x 8 compute warps, 3 producer warps, MMA warp
+// A slot holds what one row tile needs in shared memory (Q, dO, P, dS); two fit at D = 128 (96 KB each),
+// three at D = 64 (64 KB).  Three producer warps refill a slot's Q / dO the moment its dV / dK MMAs
+// are done; one thread issues whichever batch of MMAs is ready next (S / dP of the tile that has
+// landed, or dV / dK / dQ of the tile whose probabilities are written); two compute groups of 256
+// threads (two warps per TMEM lane quadrant, half of the key columns each) take alternate tiles,
+// turn S / dP into P / dS and, once the MMAs are done, move the tile's dQ from TMEM to the staging tile
+// (its P / dS region) and store it.  Each hand-over is an mbarrier with a bounded wait.
+//
+// What bounds it is shared memory: the five products read 224 KB of operands per row tile at D = 128
+// (168 KB at D = 64), the gathered rows, P / dS and the staging tile add 160 (112) KB, 3.1 k (2.2 k)
+// cycles at 128 bytes per clock.  The chain of one tile (gather, S / dP, arithmetic, dV / dK / dQ, dQ out)
+// is two to three times that long, so what counts is how many tiles overlap: with three slots the
+// gather and the S / dP of a group's next tile run while its last one is in its MMAs.  D = 64 also
+// computes dV^T and dK^T in one product, [dO | Q]^T [P | dS] (their tiles are neighbours): the two
+// off-diagonal quarters are wasted, but the operands are read once, 8 KB a step instead of 12.
+constexpr int kB2Threads = 640;   // 2 x 8 compute warps, 3 producer warps, MMA warp (a 21st warp would cost 16 registers each)
 constexpr int kB2Producers = 3;
 constexpr int kB2Compute = 16;    // compute warps
+
+template <int D> struct Bwd2 {
+  static constexpr int kSlabs = D / 64;
+  static constexpr int kSlots = D == 64 ? 3 : 2;
+  static constexpr int kKVBytes = kKeys * 128 * kSlabs;
+  static constexpr int kRowBytes = kRows * 128 * kSlabs;            // Q or dO
+  static constexpr int kSlotBytes = 2 * kRowBytes + 2 * kPBytes;    // dO, Q, P, dS
+  static constexpr int kBars = 2 + 7 * kSlots;
+  static constexpr size_t kSmem = 2 * kKVBytes + (size_t)kSlots * kSlotBytes + 256 /*barriers*/ +
+                                  (size_t)kSlots * 128 * 4 /*partial rows of a ragged tile*/ + 1024 /*alignment slack*/;
+};
 
 template <int D>
 __global__ void __launch_bounds__(kB2Threads, 1)
@@ -556,31 +573,36 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
                const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
                const __grid_constant__ CUtensorMap tm_q_run, const __grid_constant__ CUtensorMap tm_do_run,
                const __grid_constant__ CUtensorMap tm_dq, const BwdArgs p) {
-  constexpr int kSlabs = D / 64;
-  constexpr int kKVBytes = kKeys * 128 * kSlabs;
+  using L = Bwd2<D>;
+  constexpr int kSlabs = L::kSlabs, kSlots = L::kSlots, kKVBytes = L::kKVBytes;
   constexpr uint32_t kTmemCols = 512;
-  constexpr uint32_t kColDV = 256, kColDK = 320;   // slot s: S at 128 s, dP at 128 s + 64, dQ over both
+  // slot s: S at 128 s, dP at 128 s + 64, dQ over both; then dV^T and dK^T: at D = 128 64 columns each, at D = 64
+  // the diagonal quarters of one 128 x 128 product (dV^T: lanes 0-63, columns 0-63; dK^T: lanes 64-127,
+  // columns 64-127)
+  constexpr uint32_t kColDV = 128 * kSlots, kColDK = kColDV + 64;
   constexpr uint32_t kIdescS = idesc_bf16(128, kKeys, 0, 0);
-  constexpr uint32_t kIdescT = idesc_bf16(128, kKeys, 1, 1);
+  constexpr uint32_t kIdescT = idesc_bf16(128, D == 64 ? 128 : kKeys, 1, 1);
   constexpr uint32_t kIdescDQ = idesc_bf16(128, D, 0, 1);
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   uint8_t* sK = smem;
   uint8_t* sV = sK + kKVBytes;
-  uint8_t* sGroup = sV + kKVBytes;
-  uint64_t* bars = (uint64_t*)(sGroup + 2 * kGroupBytes);
+  uint8_t* sSlot = sV + kKVBytes;
+  uint64_t* bars = (uint64_t*)(sSlot + kSlots * L::kSlotBytes);
   uint64_t* bar_kv = bars + 0;
-  uint64_t* g_full = bars + 1;       // [2] Q / dO of the slot have landed
-  uint64_t* sp_full = bars + 3;      // [2] S / dP of the slot are in TMEM
-  uint64_t* pds_full = bars + 5;     // [2] P / dS of the slot are in shared memory (128 arrivals)
-  uint64_t* acc_full = bars + 7;     // [2] dV / dK / dQ MMAs of the slot are done
-  uint64_t* dq_read = bars + 9;      // [2] dQ of the slot has left TMEM (256 arrivals)
-  uint64_t* qdo_free = bars + 13;    // [2] the dV / dK MMAs of the slot are done: Q / dO may be refilled
-  uint64_t* bar_drain = bars + 11;
-  uint32_t* s_tmem = (uint32_t*)(bars + 16);
+  uint64_t* bar_drain = bars + 1;
+  uint64_t* g_full = bars + 2;                    // [kSlots] Q / dO of the slot have landed
+  uint64_t* sp_full = g_full + kSlots;            // S / dP of the slot are in TMEM
+  uint64_t* pds_full = sp_full + kSlots;          // P / dS of the slot are in shared memory (256 arrivals)
+  uint64_t* qdo_free = pds_full + kSlots;         // the dV / dK MMAs of the slot are done: Q / dO may be refilled
+  uint64_t* acc_full = qdo_free + kSlots;         // dV / dK / dQ MMAs of the slot are done
+  uint64_t* dq_read = acc_full + kSlots;          // dQ of the slot has left TMEM (256 arrivals)
+  uint64_t* stage_free = dq_read + kSlots;        // dQ of the slot has left its staging tile: P / dS may be written
+  uint32_t* s_tmem = (uint32_t*)(bars + L::kBars);
   volatile int* s_abort = (volatile int*)(s_tmem + 1);
-  uint32_t* s_prow = (uint32_t*)(s_tmem + 4);        // [2][128] partial row of each tile row (ragged tile), per slot
+  uint32_t* s_prow = (uint32_t*)(bars + 32);      // [kSlots][128] partial row of each tile row (ragged tile)
+  static_assert(L::kBars * 8 + 8 <= 256, "barrier region");
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
@@ -630,28 +652,33 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
 
   if (tid == 0) {
     int bad = (*(volatile int*)p.status != 0) ? 1 : 0;
-    if ((size_t)((uint8_t*)(s_prow + 256) - smem_raw) > bwd_smem_bytes(D)) {
+    if ((size_t)((uint8_t*)(s_prow + kSlots * 128) - smem_raw) > L::kSmem) {
       atomicOr(p.status, 256);   // the shared-memory window is less aligned than assumed
       bad = 1;
     }
     *s_abort = bad;
     mbar_init(bar_kv, 1);
-    for (int s = 0; s < 2; ++s) {
-      mbar_init(g_full + s, 1); mbar_init(sp_full + s, 1); mbar_init(pds_full + s, 256);
-      mbar_init(acc_full + s, 1); mbar_init(dq_read + s, 256); mbar_init(qdo_free + s, 1);
-    }
     mbar_init(bar_drain, 1);
+    for (int s = 0; s < kSlots; ++s) {
+      mbar_init(g_full + s, 1); mbar_init(sp_full + s, 1); mbar_init(pds_full + s, 256); mbar_init(qdo_free + s, 1);
+      mbar_init(acc_full + s, 1); mbar_init(dq_read + s, 256); mbar_init(stage_free + s, 1);
+    }
     fence_barrier_init();
     prefetch_tensormap(&tm_k); prefetch_tensormap(&tm_v);
     prefetch_tensormap(&tm_q); prefetch_tensormap(&tm_do); prefetch_tensormap(&tm_dq);
   }
   __syncthreads();
   if (*s_abort) return;
-  // Rows past nq * G of a tile (and, for D = 64, the second slab) are never loaded: keep them 0.
-  for (int i = tid; i < 2 * 2 * kRowTileBytes / 16; i += kB2Threads) {
-    const int buf = i / (kRowTileBytes / 16), o16 = i % (kRowTileBytes / 16);
-    uint8_t* base = sGroup + (buf >> 1) * kGroupBytes + (buf & 1) * kRowTileBytes;
-    *reinterpret_cast<uint4*>(base + o16 * 16) = make_uint4(0, 0, 0, 0);
+  // rows past nq * G of a tile are never loaded, and dV / dK sum over all 128: keep them zero
+  {
+    // (merged boxes lay the two slabs of a row side by side: one run of 256-byte rows)
+    const int r0 = p.nq * p.G, row_bytes = p.merged ? 256 : 128;
+    const int n = (kRows - r0) * row_bytes / 16, runs = 2 * L::kRowBytes / (kRows * row_bytes);
+    for (int i = tid; i < runs * kSlots * n; i += kB2Threads) {
+      const int part = i / n, slot = part / runs;
+      uint8_t* base = sSlot + slot * L::kSlotBytes + (part % runs) * (kRows * row_bytes);
+      *reinterpret_cast<uint4*>(base + r0 * row_bytes + (i % n) * 16) = make_uint4(0, 0, 0, 0);
+    }
   }
   fence_proxy_async();
   if (warp == 0) {
@@ -706,12 +733,12 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
     const uint64_t pol_keep = l2_policy_evict_normal();   // gathered q / dO rows: read again by other blocks
     int issued = 0;                                  // tiles whose loads this warp has sent off
     for (int k = 0; k < n_tiles; ++k) {
-      const int sb = k & 1;
-      // the slot's Q / dO are free once the dV / dK MMAs of tile k-2 are done (dQ reads dS and K only)
-      if (k >= 2) mbar_wait(qdo_free + sb, ((k >> 1) - 1) & 1, p.status, s_abort, 128);
+      const int sb = k % kSlots, u = k / kSlots;
+      // the slot's Q / dO are free once the dV / dK MMAs of its last tile are done (dQ reads dS and K only)
+      if (u > 0) mbar_wait(qdo_free + sb, (u - 1) & 1, p.status, s_abort, 128);
       if (__any_sync(0xffffffffu, *s_abort)) break;           // the whole warp leaves together
-      uint8_t* sQ = sGroup + sb * kGroupBytes;
-      uint8_t* sDO = sQ + kRowTileBytes;
+      uint8_t* sDO = sSlot + sb * L::kSlotBytes;
+      uint8_t* sQ = sDO + L::kRowBytes;
       if (pw == 0 && lane == 0) mbar_expect_tx(g_full + sb, gather_bytes);
       __syncwarp();
       if (p.kind != 2) {
@@ -754,7 +781,7 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
       // give-up path: the loads still on their way into this CTA's shared memory land (bounded
       // wait on the last phase of each slot) before the CTA ends
       mbar_wait_drain(bar_kv, 0);
-      for (int k = max(0, issued - 2); k < issued; ++k) mbar_wait_drain(g_full + (k & 1), (k >> 1) & 1);
+      for (int k = max(0, issued - kSlots); k < issued; ++k) mbar_wait_drain(g_full + k % kSlots, (k / kSlots) & 1);
     }
   } else if (warp == kB2Compute + kB2Producers) {
     // ---- MMA issuer: whichever batch is ready next ---------------------------------------------
@@ -764,18 +791,18 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
       const uint32_t kb = desc_lo_mnmajor(smem_u32(sK), kKeys * 128);
       const uint32_t q_slab = p.merged ? 1024u : (uint32_t)(kRows * 128), q_sbo = p.merged ? 2048u : 1024u;
       int next_a = 0, next_b = 0;                    // next tile for S / dP, next tile for dV / dK / dQ
+      int sa = 0, ua = 0, sbb = 0, ub = 0;           // their slots and the slots' use counts
       long long idle_since = clock64();
       uint32_t polls = 0;
       while (next_b < n_tiles) {
         bool progressed = false;
         if (next_a < n_tiles) {
-          const int k = next_a, sb = k & 1, u = k >> 1;
-          // Q / dO have landed; dQ of tile k-2, which lies over the slot's S / dP columns, has been read
-          if (mbar_try_wait(g_full + sb, u & 1) && (k < 2 || mbar_try_wait(dq_read + sb, (u - 1) & 1))) {
+          // Q / dO have landed; dQ of the slot's last tile, which lies over its S / dP columns, has been read
+          if (mbar_try_wait(g_full + sa, ua & 1) && (ua == 0 || mbar_try_wait(dq_read + sa, (ua - 1) & 1))) {
             tc_fence_after();
-            const uint8_t* sQ = sGroup + sb * kGroupBytes;
-            const uint32_t qa = desc_lo_kmajor(smem_u32(sQ)), da = desc_lo_kmajor(smem_u32(sQ + kRowTileBytes));
-            const uint32_t colS = tmem + sb * 128, colDP = colS + 64;
+            const uint8_t* sDO = sSlot + sa * L::kSlotBytes;
+            const uint32_t qa = desc_lo_kmajor(smem_u32(sDO + L::kRowBytes)), da = desc_lo_kmajor(smem_u32(sDO));
+            const uint32_t colS = tmem + sa * 128, colDP = colS + 64;
 #pragma unroll
             for (int kk = 0; kk < D / 16; ++kk) {
               const uint32_t slab = kk >> 2, in = (kk & 3) * 32;
@@ -788,34 +815,44 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
               mma_ss(colDP, desc_at_sbo(da, slab * q_slab + in, q_sbo), desc_at(va, slab * (kKeys * 128) + in),
                      kIdescS, kk > 0);
             }
-            tc_commit(sp_full + sb);
+            tc_commit(sp_full + sa);
             ++next_a;
+            if (++sa == kSlots) { sa = 0; ++ua; }
             progressed = true;
           }
         }
         if (next_b < next_a) {
-          const int k = next_b, sb = k & 1, u = k >> 1;
-          if (mbar_try_wait(pds_full + sb, u & 1)) {
+          if (mbar_try_wait(pds_full + sbb, ub & 1)) {
             tc_fence_after();
-            const uint8_t* sQ = sGroup + sb * kGroupBytes;
-            const uint8_t* sP = sQ + 2 * kRowTileBytes;
+            const uint8_t* sDO = sSlot + sbb * L::kSlotBytes;
+            const uint8_t* sP = sDO + 2 * L::kRowBytes;
             const uint8_t* sDS = sP + kPBytes;
-            const uint32_t qa = desc_lo_mnmajor(smem_u32(sQ), q_slab);
-            const uint32_t da = desc_lo_mnmajor(smem_u32(sQ + kRowTileBytes), q_slab);
-            const uint32_t pa = desc_lo_mnmajor(smem_u32(sP), 0), dsa = desc_lo_mnmajor(smem_u32(sDS), 0);
             const uint32_t dsk = desc_lo_kmajor(smem_u32(sDS));
+            if (D == 64) {
+              // A: the dO and Q tiles as two 64-column slabs, B: the P and dS tiles likewise
+              const uint32_t da = desc_lo_mnmajor(smem_u32(sDO), L::kRowBytes);
+              const uint32_t pa = desc_lo_mnmajor(smem_u32(sP), kPBytes);
 #pragma unroll
-            for (int kk = 0; kk < kRows / 16; ++kk)        // contraction over the 128 rows, 16 a step
-              mma_ss(tmem + kColDV, desc_at_sbo(da, kk * 2 * q_sbo, q_sbo), desc_at(pa, kk * 2048), kIdescT, 1);
+              for (int kk = 0; kk < kRows / 16; ++kk)        // contraction over the 128 rows, 16 a step
+                mma_ss(tmem + kColDV, desc_at(da, kk * 2048), desc_at(pa, kk * 2048), kIdescT, 1);
+            } else {
+              const uint32_t da = desc_lo_mnmajor(smem_u32(sDO), q_slab);
+              const uint32_t qa = desc_lo_mnmajor(smem_u32(sDO + L::kRowBytes), q_slab);
+              const uint32_t pa = desc_lo_mnmajor(smem_u32(sP), 0), dsa = desc_lo_mnmajor(smem_u32(sDS), 0);
 #pragma unroll
-            for (int kk = 0; kk < kRows / 16; ++kk)
-              mma_ss(tmem + kColDK, desc_at_sbo(qa, kk * 2 * q_sbo, q_sbo), desc_at(dsa, kk * 2048), kIdescT, 1);
-            tc_commit(qdo_free + sb);
+              for (int kk = 0; kk < kRows / 16; ++kk)
+                mma_ss(tmem + kColDV, desc_at_sbo(da, kk * 2 * q_sbo, q_sbo), desc_at(pa, kk * 2048), kIdescT, 1);
+#pragma unroll
+              for (int kk = 0; kk < kRows / 16; ++kk)
+                mma_ss(tmem + kColDK, desc_at_sbo(qa, kk * 2 * q_sbo, q_sbo), desc_at(dsa, kk * 2048), kIdescT, 1);
+            }
+            tc_commit(qdo_free + sbb);
 #pragma unroll
             for (int kk = 0; kk < kKeys / 16; ++kk)        // contraction over the 64 keys
-              mma_ss(tmem + sb * 128, desc_at(dsk, kk * 32), desc_at(kb, kk * 2048), kIdescDQ, kk > 0);
-            tc_commit(acc_full + sb);
+              mma_ss(tmem + sbb * 128, desc_at(dsk, kk * 32), desc_at(kb, kk * 2048), kIdescDQ, kk > 0);
+            tc_commit(acc_full + sbb);
             ++next_b;
+            if (++sbb == kSlots) { sbb = 0; ++ub; }
             progressed = true;
           }
         }
@@ -832,17 +869,13 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
       if (!mbar_wait(bar_drain, 0, p.status, s_abort, 4096)) mbar_wait_drain(bar_drain, 0);
     }
   } else if (warp < kB2Compute) {
-    // ---- compute group of slot sb: S, dP -> P, dS; then the tile's dQ out -----------------------------
-    const int sb = warp >> 3, wg = warp & 7, lt = (warp & 7) * 32 + lane;
+    // ---- compute group `grp`: tiles grp, grp + 2, ... -------------------------------------------------
+    const int grp = warp >> 3, wg = warp & 7, lt = (warp & 7) * 32 + lane;
     const int quad = wg & 3, half = wg >> 2;           // TMEM lane quadrant, key-column half
     const int row = quad * 32 + lane;
     const int ql = row / p.G, g = row % p.G;
     const int head = hkv * p.G + g;
     const bool row_slot_ok = ql < p.nq;
-    uint8_t* sP = sGroup + sb * kGroupBytes + 2 * kRowTileBytes;
-    uint8_t* sDS = sP + kPBytes;
-    uint32_t* s_prow_g = s_prow + sb * 128;
-    const uint32_t lane_base = tmem + ((uint32_t)(quad * 32) << 16) + sb * 128;
     // query of this thread's row in tile k (selection: with the tile's column groups it attends in
     // the bits above the position), -1: no row
     auto row_query = [&](int k) -> int {
@@ -852,16 +885,20 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
       return t_lo + qi;
     };
     auto row_index = [&](int t) -> size_t { return (size_t)(b * p.Hq + head) * p.T + (t & (int)kPairPosMask); };
-    int t_cur = sb < n_tiles ? row_query(sb) : -1;
-    int t_nxt = sb + 2 < n_tiles ? row_query(sb + 2) : -1;
+    int t_cur = grp < n_tiles ? row_query(grp) : -1;
+    int t_nxt = grp + 2 < n_tiles ? row_query(grp + 2) : -1;
     float lse_cur = 0.f, delta_cur = 0.f, gate_cur = 1.f;
     if (t_cur >= 0) {
       lse_cur = __ldg(p.lse + row_index(t_cur));
       delta_cur = __ldg(p.delta + row_index(t_cur));
       if (p.row_scale) gate_cur = __ldg(p.row_scale + row_index(t_cur));
     }
-    for (int k = sb; k < n_tiles; k += 2) {
-      const int u = k >> 1, i = rt_begin + k;
+    // A given-up wait does not part a group: its warps go on to the barrier below, which decides for all.
+    for (int k = grp; k < n_tiles; k += 2) {
+      const int sb = k % kSlots, u = k / kSlots;
+      uint8_t* sP = sSlot + sb * L::kSlotBytes + 2 * L::kRowBytes;
+      uint8_t* sDS = sP + kPBytes;
+      const uint32_t lane_base = tmem + ((uint32_t)(quad * 32) << 16) + sb * 128;
       const int t_nn = (k + 4 < n_tiles) ? row_query(k + 4) : -1;
       float lse_nxt = 0.f, delta_nxt = 0.f, gate_nxt = 1.f;
       if (t_nxt >= 0) {
@@ -889,9 +926,14 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
       // every column of this thread's half is attended (the usual case away from the diagonal)?
       const bool all_cols = lo <= half * 32 && hi >= half * 32 + 31 && groups == 0x3u;
       mbar_wait(sp_full + sb, u & 1, p.status, s_abort, 64);
-      // the P / dS tiles double as the dQ staging tile: this group's store of tile k-2 has read it
-      if (lt == 0) bulk_wait_read();
-      if (named_or_b(1 + sb, 256, *s_abort)) break;            // the whole group leaves together
+      // the P / dS tiles double as the dQ staging tile: the store of the slot's last tile has read it
+      // (the thread that stored says so, below)
+      if (lt == 0 && k > grp) {
+        bulk_wait_read();
+        mbar_arrive(stage_free + (k - 2) % kSlots);
+      }
+      if (u > 0) mbar_wait(stage_free + sb, (u - 1) & 1, p.status, s_abort, 64);
+      __syncwarp();
       tc_fence_after();
       {
         uint32_t rs[32], rp[32];
@@ -915,8 +957,8 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
               const int c = half * 32 + c2 * 2 + e;
-              const bool ok = (c >= lo) && (c <= hi) && ((groups >> (c2 >> 3)) & 1u);
-              const float pr = ok ? ex2(fmaf(__uint_as_float(rs[c2 * 2 + e]), p.scale_log2, -lse2)) : 0.f;
+              const bool in = (c >= lo) && (c <= hi) && ((groups >> (c2 >> 3)) & 1u);
+              const float pr = in ? ex2(fmaf(__uint_as_float(rs[c2 * 2 + e]), p.scale_log2, -lse2)) : 0.f;
               pv[e] = pr;
               dv[e] = pr * fmaf(__uint_as_float(rp[c2 * 2 + e]), dscale, -ddelta);
             }
@@ -937,7 +979,10 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
       mbar_arrive(pds_full + sb);
       // ---- the tile's dQ: TMEM -> bf16 -> staging tile (the P / dS region, free once the MMAs are
       // done) -> partial buffer, while the producers fetch the slot's next tile
+      const int i = rt_begin + k;
+      uint8_t* stage = sP;
       mbar_wait(acc_full + sb, u & 1, p.status, s_abort, 128);
+      __syncwarp();
       tc_fence_after();
 #pragma unroll
       for (int cc = 0; cc < D / 64; ++cc) {          // this thread's half of the D columns
@@ -951,8 +996,8 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
         }
 #pragma unroll
         for (int v4 = 0; v4 < 4; ++v4) {
-          const uint32_t chunk = (uint32_t)((col0 >> 3) + v4);
-          st_shared_v4(smem_u32(sP) + (chunk >> 3) * (kRows * 128) + row * 128 + (((chunk & 7) ^ (row & 7)) << 4),
+          const uint32_t ch = (uint32_t)((col0 >> 3) + v4);
+          st_shared_v4(smem_u32(stage) + (ch >> 3) * (kRows * 128) + row * 128 + (((ch & 7) ^ (row & 7)) << 4),
                        pack_bf16(__uint_as_float(r32[v4 * 8 + 0]), __uint_as_float(r32[v4 * 8 + 1])),
                        pack_bf16(__uint_as_float(r32[v4 * 8 + 2]), __uint_as_float(r32[v4 * 8 + 3])),
                        pack_bf16(__uint_as_float(r32[v4 * 8 + 4]), __uint_as_float(r32[v4 * 8 + 5])),
@@ -960,6 +1005,7 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
         }
       }
       const bool full_tile = (i + 1) * p.nq <= n_q;
+      uint32_t* prow_s = s_prow + sb * 128;
       if (!full_tile && half == 0) {
         uint32_t prow = 0xffffffffu;
         const int qi = i * p.nq + ql;
@@ -971,10 +1017,10 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
             prow = (uint32_t)((((size_t)bh * p.T + t_lo + qi) * p.n_slots + slot) * p.G + g);
           }
         }
-        s_prow_g[row] = prow;
+        prow_s[row] = prow;
       }
       fence_proxy_async();
-      if (named_or_b(1 + sb, 256, *s_abort)) break;
+      if (named_or_b(1 + grp, 256, *s_abort)) break;           // the whole group leaves together
       if (full_tile) {
         // its rows are consecutive in the partial buffer: one TMA store per slab
         if (lt == 0) {
@@ -983,17 +1029,17 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
           const int outer = p.kind == 2 ? 0 : bh;
 #pragma unroll
           for (int sl = 0; sl < kSlabs; ++sl)
-            tma_store_5d_hint(&tm_dq, sP + sl * (kRows * 128), sl * 64, 0, slot, mid, outer, l2_policy_evict_first());
+            tma_store_5d_hint(&tm_dq, stage + sl * (kRows * 128), sl * 64, 0, slot, mid, outer, l2_policy_evict_first());
           bulk_commit();
         }
-      } else {   // the ragged last tile: 16 lanes write the 256 (D = 128) or 128 bytes of one row
+      } else {   // the ragged last tile: whole rows out by hand, 16 bytes a lane
         constexpr int kChunks = D / 8;
         constexpr int kRowsPerPass = 256 / kChunks;
         const int c = lt % kChunks;
         for (int r = lt / kChunks; r < kRows; r += kRowsPerPass) {
-          const uint32_t prow = s_prow_g[r];
+          const uint32_t prow = prow_s[r];
           if (prow != 0xffffffffu) {
-            const uint4 v = *reinterpret_cast<const uint4*>(sP + (c >> 3) * (kRows * 128) + r * 128 +
+            const uint4 v = *reinterpret_cast<const uint4*>(stage + (c >> 3) * (kRows * 128) + r * 128 +
                                                             (((c & 7) ^ (r & 7)) << 4));
             *reinterpret_cast<uint4*>(p.dq_part + (size_t)prow * D + c * 8) = v;
           }
@@ -1009,15 +1055,17 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
   tc_fence_after();
   if (warp < kB2Compute && ((warp >> 2) & 1) == 0 && !*s_abort) {
     const int grp = warp >> 3, quad = warp & 3;
-    const uint32_t col = grp == 0 ? kColDV : kColDK;
-    const uint32_t lane_base = tmem + ((uint32_t)(quad * 32) << 16);
-    const int d = quad * 32 + lane;
+    // D = 64: dV^T sits in lanes 0-63, dK^T in lanes 64-127
+    const bool mine = D == 128 || (quad >> 1) == grp;
+    if (mine) {
+      const uint32_t col = grp == 0 ? kColDV : kColDK;
+      const uint32_t lane_base = tmem + ((uint32_t)(quad * 32) << 16);
+      const int d = (D == 128 ? quad : quad & 1) * 32 + lane;
 #pragma unroll
-    for (int hc = 0; hc < 2; ++hc) {
-      uint32_t r32[32];
-      tmem_ld32(lane_base + col + hc * 32, r32);
-      tmem_wait_ld();
-      if (d < D) {
+      for (int hc = 0; hc < 2; ++hc) {
+        uint32_t r32[32];
+        tmem_ld32(lane_base + col + hc * 32, r32);
+        tmem_wait_ld();
 #pragma unroll
         for (int c = 0; c < 32; ++c) {
           const int key = key0 + hc * 32 + c;
@@ -1376,11 +1424,11 @@ int tc_attn_bwd(const AttnArgs& a, void* ws, size_t ws_bytes, cudaStream_t st) {
   if ((get_option_bwd_kernel() == 1 || a.kind == 2) && !p.dq_acc_mode) {   // compute groups relieved of the issuing
     KernelScope ks(branch_name(kBwdNames, a.kind), st);
     if (a.D == 128) {
-      NSA_CUDA_OK(func_smem((const void*)tc_bwd2_kernel<128>, smem));
-      tc_bwd2_kernel<128><<<grid, kB2Threads, smem, st>>>(tm_k, tm_v, tm_q, tm_do, tm_q_run, tm_do_run, tm_dq, p);
+      NSA_CUDA_OK(func_smem((const void*)tc_bwd2_kernel<128>, Bwd2<128>::kSmem));
+      tc_bwd2_kernel<128><<<grid, kB2Threads, Bwd2<128>::kSmem, st>>>(tm_k, tm_v, tm_q, tm_do, tm_q_run, tm_do_run, tm_dq, p);
     } else {
-      NSA_CUDA_OK(func_smem((const void*)tc_bwd2_kernel<64>, smem));
-      tc_bwd2_kernel<64><<<grid, kB2Threads, smem, st>>>(tm_k, tm_v, tm_q, tm_do, tm_q_run, tm_do_run, tm_dq, p);
+      NSA_CUDA_OK(func_smem((const void*)tc_bwd2_kernel<64>, Bwd2<64>::kSmem));
+      tc_bwd2_kernel<64><<<grid, kB2Threads, Bwd2<64>::kSmem, st>>>(tm_k, tm_v, tm_q, tm_do, tm_q_run, tm_do_run, tm_dq, p);
     }
   } else if (a.D == 128) {
     NSA_CUDA_OK(func_smem((const void*)tc_bwd_kernel<128>, smem));
