@@ -46,6 +46,7 @@ struct BwdArgs {
   float* dv_acc;
   int* status;
   int split_chunk;             // row tiles per CTA when split
+  int csize;                   // CTAs per cluster
   int B, Hq, Hkv, T, Lk, G, nq;
   int kind, window, block_size;
   int n_ktiles, n_slots;
@@ -556,6 +557,27 @@ constexpr int kB2Threads = 640;   // 2 x 8 compute warps, 3 producer warps, MMA 
 constexpr int kB2Producers = 3;
 constexpr int kB2Compute = 16;    // compute warps
 
+// Cluster helpers.  Every thread of every CTA of the cluster takes part in the barrier.
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t peer_addr(const void* p, int rank) {
+  uint32_t a;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ int ld_peer_s32(const int* p, int rank) {
+  int v;
+  asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(peer_addr(p, rank)) : "memory");
+  return v;
+}
+__device__ __forceinline__ float4 ld_peer_f32x4(const float* p, int rank) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "r"(peer_addr(p, rank)) : "memory");
+  return v;
+}
+
 template <int D> struct Bwd2 {
   static constexpr int kSlabs = D / 64;
   static constexpr int kSlots = D == 64 ? 3 : 2;
@@ -567,7 +589,7 @@ template <int D> struct Bwd2 {
                                   (size_t)kSlots * 128 * 4 /*partial rows of a ragged tile*/ + 1024 /*alignment slack*/;
 };
 
-template <int D>
+template <int D, bool kCluster>
 __global__ void __launch_bounds__(kB2Threads, 1)
 tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
@@ -606,10 +628,13 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
-  int4 item = make_int4((int)blockIdx.y, (int)blockIdx.x, 0, 1);
-  if (p.kind == 2) {                                 // selection: one work item per CTA
-    if ((int)(blockIdx.x % p.plan.max_items) >= p.plan.n_items[blockIdx.x / p.plan.max_items]) return;
-    item = p.plan.items[blockIdx.x];
+  // one key tile (or selection work item) per cluster of csize CTAs, which share its row tiles out
+  const int csize = kCluster ? p.csize : 1, rank = kCluster ? (int)blockIdx.x % csize : 0;
+  const int work = kCluster ? (int)blockIdx.x / csize : (int)blockIdx.x;
+  int4 item = make_int4((int)blockIdx.y, work, 0, 1);
+  if (p.kind == 2) {
+    if (work % p.plan.max_items >= p.plan.n_items[work / p.plan.max_items]) return;
+    item = p.plan.items[work];
   }
   const int j = item.y;                              // key tile
   const int bh = item.x;
@@ -631,12 +656,14 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
   n_q = max(n_q, 0);
   const int n_rt_all = (n_q + p.nq - 1) / p.nq;
   const int chunk = p.kind == 2 ? kSelChunkTiles : ((int)gridDim.z > 1 ? p.split_chunk : n_rt_all);
-  const int rt_begin = p.kind == 2 ? item.z : (int)blockIdx.z * chunk;
-  const int rt_end = min(n_rt_all, rt_begin + chunk);
+  const int rt_first = p.kind == 2 ? item.z : (int)blockIdx.z * chunk;
+  const int rt_last = min(n_rt_all, rt_first + chunk);
   const bool split = p.kind == 2 ? item.w > 1 : gridDim.z > 1;
-  const int n_tiles = rt_end - rt_begin;
+  const int per_cta = kCluster ? (max(0, rt_last - rt_first) + csize - 1) / csize : rt_last - rt_first;
+  const int rt_begin = rt_first + rank * per_cta;
+  int n_tiles = max(0, min(rt_last, rt_begin + per_cta) - rt_begin);
 
-  if (n_tiles <= 0) {
+  if (rt_last <= rt_first) {
     if (!split && n_rt_all == 0) {   // nobody attends these keys: their gradients are zero
       for (int i = tid; i < kKeys * D / 8; i += blockDim.x) {
         const int key = key0 + i / (D / 8);
@@ -668,7 +695,10 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
     prefetch_tensormap(&tm_q); prefetch_tensormap(&tm_do); prefetch_tensormap(&tm_dq);
   }
   __syncthreads();
-  if (*s_abort) return;
+  if (*s_abort) {
+    if (!kCluster) return;
+    n_tiles = 0;             // the cluster's other CTAs read this one's flag at the end: it stays
+  }
   // rows past nq * G of a tile are never loaded, and dV / dK sum over all 128: keep them zero
   {
     // (merged boxes lay the two slabs of a row side by side: one run of 256-byte rows)
@@ -1053,6 +1083,7 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
   // ---- dK^T, dV^T: lane = d, column = key; compute group 0 writes dV, group 1 writes dK ----------
   __syncthreads();           // the MMA thread has seen the tensor pipe drain (bar_drain)
   tc_fence_after();
+  float* s_acc = reinterpret_cast<float*>(sSlot);      // cluster: [dV, dK][64 keys][D], over the slots
   if (warp < kB2Compute && ((warp >> 2) & 1) == 0 && !*s_abort) {
     const int grp = warp >> 3, quad = warp & 3;
     // D = 64: dV^T sits in lanes 0-63, dK^T in lanes 64-127
@@ -1069,7 +1100,9 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
 #pragma unroll
         for (int c = 0; c < 32; ++c) {
           const int key = key0 + hc * 32 + c;
-          if (key < p.Lk) {
+          if (kCluster) {
+            s_acc[(grp * kKeys + hc * 32 + c) * D + d] = __uint_as_float(r32[c]);
+          } else if (key < p.Lk) {
             const size_t o = ((size_t)bh * p.Lk + key) * D + d;
             if (split) atomicAdd((grp == 0 ? p.dv_acc : p.dk_acc) + o, __uint_as_float(r32[c]));
             else (grp == 0 ? p.dv : p.dk)[o] = __float2bfloat16_rn(__uint_as_float(r32[c]));
@@ -1077,6 +1110,35 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
         }
       }
     }
+  }
+  if (kCluster) {
+    // the CTAs of the cluster add their accumulators, each a share of the keys, in rank order
+    cluster_sync();
+    int aborted = 0;
+    for (int r = 0; r < csize; ++r) aborted |= ld_peer_s32(const_cast<int*>(s_abort), r);
+    if (!aborted) {
+      const int n = 2 * kKeys * D / 4 / csize;           // float4s per CTA
+      for (int i = tid; i < n; i += kB2Threads) {
+        const int e = (rank * n + i) * 4;
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int r = 0; r < csize; ++r) {
+          const float4 v = ld_peer_f32x4(s_acc + e, r);
+          acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+        }
+        const int which = e / (kKeys * D), key = key0 + (e / D) % kKeys, d = e % D;
+        if (key < p.Lk) {
+          const size_t o = ((size_t)bh * p.Lk + key) * D + d;
+          if (split) {
+            float* dst = (which == 0 ? p.dv_acc : p.dk_acc) + o;
+            atomicAdd(dst, acc.x); atomicAdd(dst + 1, acc.y); atomicAdd(dst + 2, acc.z); atomicAdd(dst + 3, acc.w);
+          } else {
+            *reinterpret_cast<uint2*>((which == 0 ? p.dv : p.dk) + o) =
+                make_uint2(pack_bf16(acc.x, acc.y), pack_bf16(acc.z, acc.w));
+          }
+        }
+      }
+    }
+    cluster_sync();            // nobody leaves while its memory is read
   }
   tc_fence_before();
   __syncthreads();
@@ -1282,6 +1344,7 @@ static const char* const kRedNames[3] = {"dq_reduce_win", "dq_reduce_cmp", "dq_r
 
 struct BwdPlan {
   int n_ktiles, n_slots, nq, n_splits, split_chunk;
+  int csize;                 // CTAs that share the row tiles of one key tile
   size_t off_acc;
   size_t cap_pairs;          // selection: pairs the CSR may hold
   SelPlanLayout layout;      // selection
@@ -1317,16 +1380,27 @@ static BwdPlan plan_bwd(const AttnArgs& a) {
     pl.layout = sel_plan_layout((int)units, a.T, a.S, pl.nq);
     off += pl.layout.total;
   }
-  // compression: a few key tiles are attended by (almost) every query; split their row tiles
+  // Fewer key tiles than SMs: a cluster of CTAs shares the row tiles of each and adds its dK / dV through
+  // distributed shared memory, as long as a CTA keeps 8 row tiles or so (a CTA costs about as much as
+  // two before its first).  More than that many CTAs gain nothing, and clusters leave SMs of a
+  // GPC over, so big problems do without.
+  const int max_rt = a.kind == 0 ? (a.window + kKeys - 2 + pl.nq) / pl.nq : (a.T + pl.nq - 1) / pl.nq;
+  const int item_rt = a.kind == 2 ? (max_rt < kSelChunkTiles ? max_rt : kSelChunkTiles) : max_rt;
+  const long long base = (long long)units * pl.n_ktiles;
+  pl.csize = 1;
+  while (!a.dq_acc && pl.csize < 8 && base * pl.csize * 2 <= sm_count() + 20 && item_rt >= 8 * pl.csize) pl.csize *= 2;
+  // compression: a few key tiles are attended by (almost) every query; what a cluster does not make
+  // short enough goes in chunks of 48 row tiles whose dK / dV meet in fp32 accumulators
   pl.n_splits = 1;
   pl.split_chunk = 0;
   pl.off_acc = off;
   if (a.kind == 1) {
-    const int max_rt = (a.T + pl.nq - 1) / pl.nq;
     pl.split_chunk = 48;
-    pl.n_splits = (max_rt + pl.split_chunk - 1) / pl.split_chunk;
-    if (pl.n_splits > 1) off += 2 * align_up((size_t)a.B * a.Hkv * a.Lk * a.D * sizeof(float), 256);
-    else pl.n_splits = 1;
+    if (max_rt > pl.split_chunk * pl.csize) {
+      pl.csize = 1;
+      pl.n_splits = (max_rt + pl.split_chunk - 1) / pl.split_chunk;
+      off += 2 * align_up((size_t)a.B * a.Hkv * a.Lk * a.D * sizeof(float), 256);
+    }
   }
   // selection: blocks split over several work items use the same accumulators
   if (a.kind == 2) off += 2 * align_up((size_t)a.B * a.Hkv * a.Lk * a.D * sizeof(float), 256);
@@ -1368,6 +1442,7 @@ int tc_attn_bwd(const AttnArgs& a, void* ws, size_t ws_bytes, cudaStream_t st) {
   p.merged = (a.kind == 2 && a.D == 128 && G % 8 == 0 && get_option_merged_boxes()) ? 1 : 0;
   p.scale = a.scale; p.scale_log2 = a.scale * kLog2e;
   p.split_chunk = pl.split_chunk;
+  p.csize = pl.csize;
   const size_t n_kv = (size_t)a.B * a.Hkv * a.Lk * a.D;
   p.dk_acc = (float*)(base + pl.off_acc);
   p.dv_acc = (float*)(base + pl.off_acc + align_up(n_kv * sizeof(float), 256));
@@ -1421,15 +1496,29 @@ int tc_attn_bwd(const AttnArgs& a, void* ws, size_t ws_bytes, cudaStream_t st) {
   dim3 grid(pl.n_ktiles, a.B * a.Hkv, pl.n_splits);
   if (a.kind == 2)
     grid = dim3((unsigned)((size_t)a.B * a.Hkv * pl.layout.max_items));
-  if ((get_option_bwd_kernel() == 1 || a.kind == 2) && !p.dq_acc_mode) {   // compute groups relieved of the issuing
+  const bool roles = (get_option_bwd_kernel() == 1 || a.kind == 2) && !p.dq_acc_mode;   // compute groups relieved of the issuing
+  if (roles) {
     KernelScope ks(branch_name(kBwdNames, a.kind), st);
-    if (a.D == 128) {
-      NSA_CUDA_OK(func_smem((const void*)tc_bwd2_kernel<128>, Bwd2<128>::kSmem));
-      tc_bwd2_kernel<128><<<grid, kB2Threads, Bwd2<128>::kSmem, st>>>(tm_k, tm_v, tm_q, tm_do, tm_q_run, tm_do_run, tm_dq, p);
-    } else {
-      NSA_CUDA_OK(func_smem((const void*)tc_bwd2_kernel<64>, Bwd2<64>::kSmem));
-      tc_bwd2_kernel<64><<<grid, kB2Threads, Bwd2<64>::kSmem, st>>>(tm_k, tm_v, tm_q, tm_do, tm_q_run, tm_do_run, tm_dq, p);
-    }
+    grid.x *= (unsigned)pl.csize;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(kB2Threads);
+    cfg.dynamicSmemBytes = a.D == 128 ? Bwd2<128>::kSmem : Bwd2<64>::kSmem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = (unsigned)pl.csize;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = pl.csize > 1 ? 1 : 0;
+    auto go = [&](auto kernel) -> int {
+      NSA_CUDA_OK(func_smem((const void*)kernel, cfg.dynamicSmemBytes));
+      NSA_CUDA_OK(cudaLaunchKernelEx(&cfg, kernel, tm_k, tm_v, tm_q, tm_do, tm_q_run, tm_do_run, tm_dq, p));
+      return NSA_OK;
+    };
+    if (a.D == 128) rc = pl.csize > 1 ? go(tc_bwd2_kernel<128, true>) : go(tc_bwd2_kernel<128, false>);
+    else rc = pl.csize > 1 ? go(tc_bwd2_kernel<64, true>) : go(tc_bwd2_kernel<64, false>);
+    if (rc != NSA_OK) return rc;
   } else if (a.D == 128) {
     NSA_CUDA_OK(func_smem((const void*)tc_bwd_kernel<128>, smem));
     KernelScope ks(branch_name(kBwdNames, a.kind), st);
