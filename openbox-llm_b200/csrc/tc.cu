@@ -79,7 +79,7 @@ __device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) {
   return r;
 }
 
-// One kernel for the three branches (kSel: selection).  192 threads in roles: warps 0-3 (thread = row
+// One kernel for the three branches (kKind: 0 window, 1 compression, 2 selection).  192 threads in roles: warps 0-3 (thread = row
 // = TMEM lane) own the softmax, warp 4 sends the TMA loads, warp 5 issues the MMAs; two CTAs per SM,
 // each walking many row tiles (tile w, w + gridDim.x, ...), long rows first.
 //
@@ -96,12 +96,20 @@ __device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) {
 //
 // Selection builds the list of a row tile's key tiles first, all threads together, and so works row
 // tile by row tile.
-template <int D, bool kSel>
+//
+// Compression rounds score * scale before the maximum is subtracted and sums a tile's probabilities
+// in column order, a few instructions per key more than the others' fused form.  A shift common to
+// all keys leaves a softmax as it is, so the gradients of the summaries sum to zero over the keys and
+// the gradient of the key pooling's position parameters is what rounding leaves of that sum, 3e-4
+// of the other gradients.  Any other rounding here, or order of the sum in backward, is as exact
+// and replaces these values by others of their size; with this one they stay what they were.
+template <int D, int kKind>
 __global__ void __launch_bounds__(kFwdThreads, 2)
 tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
               const __grid_constant__ CUtensorMap tm_v, const FwdArgs p) {
   using L = FwdSmem<D>;
   constexpr int kSlabs = L::kSlabs, kStages = L::kStages;
+  constexpr bool kSel = kKind == 2, kCmp = kKind == 1;
   constexpr uint32_t kTmemCols = 256;
   // O in columns 0-127, two buffers of S (P, bf16, is written over the first 32 columns of its S by the
   // thread that read the row)
@@ -171,7 +179,7 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     x.first_key = 0;
     if (kSel) {
       x.n_tiles = *s_ntiles;
-    } else if (p.kind == 0) {
+    } else if (!kCmp) {
       x.first_key = max(0, x.t0 - p.window + 1) & ~(kKeys - 1);
       x.n_tiles = (min(x.t_last, p.Lk - 1) - x.first_key) / kKeys + 1;
     } else {
@@ -341,7 +349,7 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           }
           continue;
         }
-        float m_used = -INFINITY, l_sum = 0.f;      // m_used in units of raw scores
+        float m_used = -INFINITY, l_sum = 0.f;      // log2 units
         for (int i = 0; i < x.n_tiles; ++i, ++c) {
           const int key0 = key0_of(x, i);
           // valid columns of this row in this tile: one range [lo, hi] and, for selection, 16-column groups
@@ -358,7 +366,7 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
                 for (int k = 0; k < p.n_sub; ++k)
                   if ((mem[k * p.nw] >> (ql & 31)) & 1u) groups |= ((1u << (p.block_size >> 4)) - 1u) << (k * (p.block_size >> 4));
               }
-            } else if (p.kind == 0) {
+            } else if (!kCmp) {
               lo = max(0, t - p.window + 1 - key0);
               hi = min(kKeys - 1, t - key0);
             } else {
@@ -374,67 +382,103 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           tmem_ld32(s_base, r);
           tmem_ld32(s_base + 32, r + 32);
           tmem_wait_ld();
-          // A row that attends the whole tile or none of it, or whole 16-column groups of it, needs no
-          // work per element: a group it does not attend gets the exponent 0 * s - inf.  Only rows whose
-          // range ends inside the tile mask their columns one by one.
-          if (!(lo <= 0 && (hi >= kKeys - 1 || hi < 0))) {
-#pragma unroll
-            for (int cc = 0; cc < 64; ++cc)
-              if (cc < lo || cc > hi) r[cc] = __float_as_uint(-3.0e38f);   // finite: 0 * r has to be 0
-          }
-          float tmax[4];                      // of the four column groups
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            float m0 = __uint_as_float(r[16 * k]), m1 = __uint_as_float(r[16 * k + 1]);
-#pragma unroll
-            for (int cc = 2; cc < 16; cc += 2) {
-              m0 = fmaxf(m0, __uint_as_float(r[16 * k + cc]));
-              m1 = fmaxf(m1, __uint_as_float(r[16 * k + cc + 1]));
-            }
-            tmax[k] = fmaxf(m0, m1);
-          }
-          if (hi < 0) groups = 0u;
-          if (kSel) {
-#pragma unroll
-            for (int k = 0; k < 4; ++k) tmax[k] = ((groups >> k) & 1u) ? tmax[k] : -INFINITY;
-          }
-          float tm = fmaxf(fmaxf(tmax[0], tmax[1]), fmaxf(tmax[2], tmax[3]));
-          if (!kSel) tm = hi < 0 ? -INFINITY : tm;
           // the running maximum is only raised when it grows by more than 8 powers of two
           float alpha = 1.f;
           bool rescale = false;
-          if ((tm - m_used) * p.scale_log2 > 8.f) {              // also the first finite maximum (m_used = -inf)
-            if (m_used != -INFINITY) {
-              alpha = ex2((m_used - tm) * p.scale_log2);
-              rescale = true;
-              l_sum *= alpha;
-            }
-            m_used = tm;
-          }
-          const float msub = (m_used == -INFINITY) ? 0.f : m_used * p.scale_log2;
-          uint64_t sc2[kSel ? 4 : 1], mn2[kSel ? 4 : 1];
-#pragma unroll
-          for (int k = 0; k < (kSel ? 4 : 1); ++k) {
-            const bool on = (groups >> k) & 1u;
-            const float sc = on ? p.scale_log2 : 0.f, mn = on ? -msub : -INFINITY;
-            sc2[k] = pack_f32x2(sc, sc);
-            mn2[k] = pack_f32x2(mn, mn);
-          }
-          uint64_t ps[2] = {0ull, 0ull};
           uint32_t pk[32];
+          if constexpr (kCmp) {
+            float xs[64];
+            float tmax = -INFINITY;
+            if (lo <= 0 && hi >= kKeys - 1) {
 #pragma unroll
-          for (int cc = 0; cc < 32; ++cc) {
-            float p0, p1;
-            unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(r[2 * cc]), __uint_as_float(r[2 * cc + 1])), sc2[kSel ? cc >> 3 : 0],
-                                   mn2[kSel ? cc >> 3 : 0]), p0, p1);
-            p0 = ex2(p0);
-            p1 = ex2(p1);
-            ps[cc & 1] = add_f32x2(ps[cc & 1], pack_f32x2(p0, p1));
-            pk[cc] = pack_bf16(p0, p1);
+              for (int cc = 0; cc < 64; ++cc) {
+                xs[cc] = __uint_as_float(r[cc]) * p.scale_log2;
+                tmax = fmaxf(tmax, xs[cc]);
+              }
+            } else {
+#pragma unroll
+              for (int cc = 0; cc < 64; ++cc) {
+                xs[cc] = (cc >= lo && cc <= hi) ? __uint_as_float(r[cc]) * p.scale_log2 : -INFINITY;
+                tmax = fmaxf(tmax, xs[cc]);
+              }
+            }
+            if (tmax > m_used + 8.f) {
+              if (m_used != -INFINITY) {
+                alpha = ex2(m_used - tmax);
+                rescale = true;
+                l_sum *= alpha;
+              }
+              m_used = tmax;
+            }
+            const float msub = (m_used == -INFINITY) ? 0.f : m_used;
+            float psum = 0.f;
+#pragma unroll
+            for (int cc = 0; cc < 32; ++cc) {
+              const float p0 = ex2(xs[2 * cc] - msub), p1 = ex2(xs[2 * cc + 1] - msub);
+              psum += p0 + p1;
+              pk[cc] = pack_bf16(p0, p1);
+            }
+            l_sum += psum;
+          } else {
+            // A row that attends the whole tile or none of it, or whole 16-column groups of it, needs no
+            // work per element: a group it does not attend gets the exponent 0 * s - inf.  Only rows whose
+            // range ends inside the tile mask their columns one by one.
+            if (!(lo <= 0 && (hi >= kKeys - 1 || hi < 0))) {
+#pragma unroll
+              for (int cc = 0; cc < 64; ++cc)
+                if (cc < lo || cc > hi) r[cc] = __float_as_uint(-3.0e38f);   // finite: 0 * r has to be 0
+            }
+            float tmax[4];                      // of the four column groups
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              float m0 = __uint_as_float(r[16 * k]), m1 = __uint_as_float(r[16 * k + 1]);
+#pragma unroll
+              for (int cc = 2; cc < 16; cc += 2) {
+                m0 = fmaxf(m0, __uint_as_float(r[16 * k + cc]));
+                m1 = fmaxf(m1, __uint_as_float(r[16 * k + cc + 1]));
+              }
+              tmax[k] = fmaxf(m0, m1);
+            }
+            if (hi < 0) groups = 0u;
+            if (kSel) {
+#pragma unroll
+              for (int k = 0; k < 4; ++k) tmax[k] = ((groups >> k) & 1u) ? tmax[k] : -INFINITY;
+            }
+            float tm = fmaxf(fmaxf(tmax[0], tmax[1]), fmaxf(tmax[2], tmax[3]));
+            if (!kSel) tm = hi < 0 ? -INFINITY : tm;
+            tm *= p.scale_log2;
+            if (tm > m_used + 8.f) {              // also the first finite maximum (m_used = -inf)
+              if (m_used != -INFINITY) {
+                alpha = ex2(m_used - tm);
+                rescale = true;
+                l_sum *= alpha;
+              }
+              m_used = tm;
+            }
+            const float msub = (m_used == -INFINITY) ? 0.f : m_used;
+            uint64_t sc2[kSel ? 4 : 1], mn2[kSel ? 4 : 1];
+#pragma unroll
+            for (int k = 0; k < (kSel ? 4 : 1); ++k) {
+              const bool on = (groups >> k) & 1u;
+              const float sc = on ? p.scale_log2 : 0.f, mn = on ? -msub : -INFINITY;
+              sc2[k] = pack_f32x2(sc, sc);
+              mn2[k] = pack_f32x2(mn, mn);
+            }
+            uint64_t ps[2] = {0ull, 0ull};
+#pragma unroll
+            for (int cc = 0; cc < 32; ++cc) {
+              float p0, p1;
+              unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(r[2 * cc]), __uint_as_float(r[2 * cc + 1])), sc2[kSel ? cc >> 3 : 0],
+                                     mn2[kSel ? cc >> 3 : 0]), p0, p1);
+              p0 = ex2(p0);
+              p1 = ex2(p1);
+              ps[cc & 1] = add_f32x2(ps[cc & 1], pack_f32x2(p0, p1));
+              pk[cc] = pack_bf16(p0, p1);
+            }
+            float s0, s1;
+            unpack_f32x2(add_f32x2(ps[0], ps[1]), s0, s1);
+            l_sum += s0 + s1;
           }
-          float s0, s1;
-          unpack_f32x2(add_f32x2(ps[0], ps[1]), s0, s1);
-          l_sum += s0 + s1;
           // O may be touched once PV of the tile before is done; only a warp that has to rescale waits
           if (i > 0 && __any_sync(0xffffffffu, rescale)) {
             ok = mbar_wait(bar_o + ((c - 1) & 1), ((c - 1) >> 1) & 1, p.status, s_abort, 8);
@@ -479,7 +523,7 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
             }
           }
         }
-        if (row_ok) *lrow = l_sum > 0.f ? (m_used * p.scale_log2 + log2f(l_sum)) * kLn2 : kLseEmpty;
+        if (row_ok) *lrow = l_sum > 0.f ? (m_used + log2f(l_sum)) * kLn2 : kLseEmpty;
         tc_fence_before();     // the O columns are read: the next row tile's first PV (behind this thread's next P) may overwrite them
       }
     }
@@ -566,8 +610,10 @@ static int launch_fwd(const AttnArgs& a, const SelPlanHeader* plan, int force, c
     kernel<<<grid, kFwdThreads, smem, st>>>(tm_q, tm_k, tm_v, p);
     return NSA_OK;
   };
-  if (a.D == 128) rc = a.kind == 2 ? go(tc_fwd_kernel<128, true>) : go(tc_fwd_kernel<128, false>);
-  else rc = a.kind == 2 ? go(tc_fwd_kernel<64, true>) : go(tc_fwd_kernel<64, false>);
+  if (a.D == 128)
+    rc = a.kind == 2 ? go(tc_fwd_kernel<128, 2>) : a.kind == 1 ? go(tc_fwd_kernel<128, 1>) : go(tc_fwd_kernel<128, 0>);
+  else
+    rc = a.kind == 2 ? go(tc_fwd_kernel<64, 2>) : a.kind == 1 ? go(tc_fwd_kernel<64, 1>) : go(tc_fwd_kernel<64, 0>);
   if (rc != NSA_OK) return rc;
   NSA_LAUNCH_OK("tc_fwd_kernel");
   return NSA_OK;

@@ -1383,21 +1383,23 @@ static BwdPlan plan_bwd(const AttnArgs& a) {
   // Fewer key tiles than SMs: a cluster of CTAs shares the row tiles of each and adds its dK / dV through
   // distributed shared memory, as long as a CTA keeps 8 row tiles or so (a CTA costs about as much as
   // two before its first).  More than that many CTAs gain nothing, and clusters leave SMs of a
-  // GPC over, so big problems do without.
+  // GPC over, so big problems do without.  Compression keeps one running sum per key tile: the
+  // gradient of the key pooling's position parameters is the rounding of that sum (tc.cu), and as it
+  // runs beside the other branches where a problem is small, the op at T = 1024 gains nothing from
+  // sharing those (277 to 289 us without, 291 with).
   const int max_rt = a.kind == 0 ? (a.window + kKeys - 2 + pl.nq) / pl.nq : (a.T + pl.nq - 1) / pl.nq;
   const int item_rt = a.kind == 2 ? (max_rt < kSelChunkTiles ? max_rt : kSelChunkTiles) : max_rt;
   const long long base = (long long)units * pl.n_ktiles;
   pl.csize = 1;
-  while (!a.dq_acc && pl.csize < 8 && base * pl.csize * 2 <= sm_count() + 20 && item_rt >= 8 * pl.csize) pl.csize *= 2;
-  // compression: a few key tiles are attended by (almost) every query; what a cluster does not make
-  // short enough goes in chunks of 48 row tiles whose dK / dV meet in fp32 accumulators
+  while (a.kind != 1 && !a.dq_acc && pl.csize < 8 && base * pl.csize * 2 <= sm_count() + 20 && item_rt >= 8 * pl.csize) pl.csize *= 2;
+  // compression: a few key tiles are attended by (almost) every query; they go in chunks of 48 row
+  // tiles whose dK / dV meet in fp32 accumulators
   pl.n_splits = 1;
   pl.split_chunk = 0;
   pl.off_acc = off;
   if (a.kind == 1) {
     pl.split_chunk = 48;
-    if (max_rt > pl.split_chunk * pl.csize) {
-      pl.csize = 1;
+    if (max_rt > pl.split_chunk) {
       pl.n_splits = (max_rt + pl.split_chunk - 1) / pl.split_chunk;
       off += 2 * align_up((size_t)a.B * a.Hkv * a.Lk * a.D * sizeof(float), 256);
     }
