@@ -1,5 +1,6 @@
 // Bandwidth-bound companions of the attention kernels: compression pooling, block scoring +
 // top-n, block->query CSR inversion and the sigmoid gate combine.
+#include <type_traits>
 #include <atomic>
 
 #include "pool.cuh"
@@ -982,45 +983,61 @@ namespace {
 // A row of the fused projection holds, for one token: q (Hq*D), then kc, vc, ks, vs, kw, vw (Hkv*D
 // each), then the gate logits (3*Hq, padded to a multiple of 8 elements).  `to_heads`: rows -> q
 // [B,Hq,T,D], kv [6][B,Hkv,T,D], gate [B,Hq,T,3]; else the other way (gradients), the padding zeroed.
-template <typename T, typename V>   // V: the 16-byte vector of T
-__global__ void split_heads_kernel(T* __restrict__ y, T* __restrict__ q, T* __restrict__ kv, T* __restrict__ gate,
-                                   int B, int Tn, int Hq, int Hkv, int D, int W, int to_heads, size_t n_vec) {
+// Bound by the one pass over both sides.  A thread moves one 16-byte column of K consecutive tokens: where the
+// column goes is worked out once for K loads in flight, and the K pieces it touches on the head-major
+// side follow one another: 59 us for 8 x 4096 rows of 2344 bf16, 87 with K = 1.
+template <typename T, typename V, int K>   // V: the 16-byte vector of T
+__global__ void __launch_bounds__(256)
+split_heads_kernel(T* __restrict__ y, T* __restrict__ q, T* __restrict__ kv, T* __restrict__ gate, int B, int Tn, int Hq,
+                   int Hkv, int D, int W, int to_heads, size_t n_items) {
   constexpr int kPer = 16 / (int)sizeof(T);                 // elements per vector
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n_vec) return;
-  const int wv = W / kPer;
+  if (i >= n_items) return;
+  const int wv = W / kPer, chunks = (Tn + K - 1) / K;
   const int col = (int)(i % wv) * kPer;
-  const size_t bt = i / wv;
-  const int t = (int)(bt % Tn), b = (int)(bt / Tn);
-  V* row = reinterpret_cast<V*>(y + bt * W + col);
+  const size_t bc = i / wv;
+  const int t0 = (int)(bc % chunks) * K, b = (int)(bc / chunks);
+  const int n = min(K, Tn - t0);
+  T* row = y + ((size_t)b * Tn + t0) * W + col;
   const int n_attn = (Hq + 6 * Hkv) * D;
   if (col < n_attn) {
     T* dst;
     if (col < Hq * D) {
       const int h = col / D, d = col % D;
-      dst = q + (((size_t)b * Hq + h) * Tn + t) * D + d;
+      dst = q + (((size_t)b * Hq + h) * Tn + t0) * D + d;
     } else {
       const int c2 = col - Hq * D;
       const int which = c2 / (Hkv * D), c3 = c2 % (Hkv * D);
       const int h = c3 / D, d = c3 % D;
-      dst = kv + ((((size_t)which * B + b) * Hkv + h) * Tn + t) * D + d;
+      dst = kv + ((((size_t)which * B + b) * Hkv + h) * Tn + t0) * D + d;
     }
-    if (to_heads) *reinterpret_cast<V*>(dst) = *row;
-    else *row = *reinterpret_cast<const V*>(dst);
-  } else {
-    T tmp[kPer];
-    if (to_heads) *reinterpret_cast<V*>(tmp) = *row;
+    const T* from = to_heads ? row : dst;
+    T* to = to_heads ? dst : row;
+    const size_t from_ld = to_heads ? W : D, to_ld = to_heads ? D : W;
+    V v[K];
 #pragma unroll
-    for (int e = 0; e < kPer; ++e) {
-      const int c = col - n_attn + e;                       // h * 3 + branch
-      if (c < 3 * Hq) {
-        T* g = gate + ((((size_t)b * Hq + c / 3) * Tn + t) * 3 + c % 3);
-        if (to_heads) *g = tmp[e]; else tmp[e] = *g;
-      } else if (!to_heads) {
-        tmp[e] = T(0.f);
+    for (int k = 0; k < K; ++k)
+      if (k < n) v[k] = __ldcs(reinterpret_cast<const V*>(from + k * from_ld));
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+      if (k < n) *reinterpret_cast<V*>(to + k * to_ld) = v[k];
+  } else {
+#pragma unroll 1
+    for (int k = 0; k < n; ++k, row += W) {
+      alignas(16) T tmp[kPer];
+      if (to_heads) *reinterpret_cast<V*>(tmp) = *reinterpret_cast<const V*>(row);
+#pragma unroll
+      for (int e = 0; e < kPer; ++e) {
+        const int c = col - n_attn + e;                       // h * 3 + branch
+        if (c < 3 * Hq) {
+          T* g = gate + ((((size_t)b * Hq + c / 3) * Tn + t0 + k) * 3 + c % 3);
+          if (to_heads) *g = tmp[e]; else tmp[e] = *g;
+        } else if (!to_heads) {
+          tmp[e] = T(0.f);
+        }
       }
+      if (!to_heads) *reinterpret_cast<V*>(row) = *reinterpret_cast<const V*>(tmp);
     }
-    if (!to_heads) *row = *reinterpret_cast<const V*>(tmp);
   }
 }
 
@@ -1065,14 +1082,21 @@ static int split_or_merge(void* y, void* q, void* kv, void* gate, int B, int T, 
   NSA_CHECK_ARG(y && q && kv && gate, "null tensor");
   cudaStream_t st = (cudaStream_t)stream;
   KernelScope ks(to_heads ? "split_heads_kernel" : "merge_heads_kernel", st);
+  // eight tokens a thread where that still gives every SM its 2048 threads
+  const int wv = dtype == NSA_DTYPE_BF16 ? W / 8 : W / 4;
+  const size_t wide = (size_t)B * ((T + 7) / 8) * wv;
+  const bool use_wide = wide >= (size_t)sm_count() * 2048;
+  const size_t n = use_wide ? wide : rows * wv;
+  auto go = [&](auto kernel, auto* yp) {
+    using E = std::remove_pointer_t<decltype(yp)>;
+    kernel<<<blocks_for(n, 256), 256, 0, st>>>(yp, (E*)q, (E*)kv, (E*)gate, B, T, Hq, Hkv, D, W, to_heads, n);
+  };
   if (dtype == NSA_DTYPE_BF16) {
-    const size_t n = rows * (W / 8);
-    split_heads_kernel<__nv_bfloat16, uint4><<<blocks_for(n, 256), 256, 0, st>>>(
-        (__nv_bfloat16*)y, (__nv_bfloat16*)q, (__nv_bfloat16*)kv, (__nv_bfloat16*)gate, B, T, Hq, Hkv, D, W, to_heads, n);
+    if (use_wide) go(split_heads_kernel<__nv_bfloat16, uint4, 8>, (__nv_bfloat16*)y);
+    else go(split_heads_kernel<__nv_bfloat16, uint4, 1>, (__nv_bfloat16*)y);
   } else {
-    const size_t n = rows * (W / 4);
-    split_heads_kernel<float, float4><<<blocks_for(n, 256), 256, 0, st>>>(
-        (float*)y, (float*)q, (float*)kv, (float*)gate, B, T, Hq, Hkv, D, W, to_heads, n);
+    if (use_wide) go(split_heads_kernel<float, float4, 8>, (float*)y);
+    else go(split_heads_kernel<float, float4, 1>, (float*)y);
   }
   NSA_LAUNCH_OK("split_heads_kernel");
   return NSA_OK;

@@ -112,3 +112,21 @@ def test_learned_pooling_backward(geom):
     for a, b, name in zip(got[1:], ref[1:], ("d_intra", "d_logits", "d_proj")):
         bound = 1e-4 * max(1.0, b.grad.abs().max().item())
         assert (a.grad.cpu() - b.grad).abs().max().item() <= bound, name
+
+
+# eight tokens a thread (many rows) and one (few); lengths that end inside a group of eight
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32], ids=str)
+@pytest.mark.parametrize("B,T,Hq,Hkv,D", [(2, 4141, 12, 4, 64), (3, 8, 5, 1, 32), (1, 4103, 16, 4, 128), (2, 9, 8, 2, 64)])
+def test_projection_rows_to_heads_and_back(B, T, Hq, Hkv, D, dtype):
+    ops = pkg().ops
+    W = ops.fused_projection_width(Hq, Hkv, D)
+    n = (Hq + 6 * Hkv) * D
+    y = torch.randn(B, T, W, device="cuda").to(dtype)
+    q, kv, gate = ops.split_heads(y, Hq, Hkv, D)
+    assert torch.equal(q, y[..., :Hq * D].view(B, T, Hq, D).transpose(1, 2))
+    assert torch.equal(kv, y[..., Hq * D:n].reshape(B, T, 6, Hkv, D).permute(2, 0, 3, 1, 4))
+    assert torch.equal(gate, y[..., n:n + 3 * Hq].reshape(B, T, Hq, 3).transpose(1, 2))
+    back = torch.full_like(y, float("nan"))
+    ops._split_heads_launch(back, q, kv, gate, Hq, Hkv, D, True)
+    assert torch.equal(back[..., :n + 3 * Hq], y[..., :n + 3 * Hq])
+    assert (back[..., n + 3 * Hq:] == 0).all()
