@@ -1243,16 +1243,21 @@ __global__ void dq_reduce3_kernel(const Reduce3Args a) {
   const size_t row_elems = (size_t)a.G * D;              // elements of one partial row (all heads)
   const size_t in_row = (size_t)g * D + v * 8;           // this thread's first head inside a row
   const size_t head_step = (size_t)Gp * D;               // to its next head
-  // eight partial rows per trip: their loads are issued before the first is added
-  constexpr int kTrip = 8;
-  auto add_rows = [&](const __nv_bfloat16* part, const long long (&rows)[kTrip]) {
+  // Rows per trip: 8 for one or two heads; three heads hold three loads per row, and an empty place costs as
+  // many instructions as a row (a window of 512 touches 9 key tiles, a query sees few tiles of
+  // summaries).  Groups of 3 at 8 x 4096 tokens: 277 us with a thread per head, 257 so; at two heads
+  // shorter trips gain 1 % at T = 32768 and cost 4 of 13 us at T = 1024.
+  constexpr int kTripSel = HG == 3 ? 4 : 8, kTripWin = HG == 3 ? 3 : 8, kTripCmp = HG == 3 ? 2 : 8;
+  // a trip of N partial rows: their loads are issued before the first is added
+  auto add_rows = [&](const __nv_bfloat16* part, const auto& rows) {
+    constexpr int kTrip = sizeof(rows) / sizeof(rows[0]);
     uint4 u[kTrip][HG];
 #pragma unroll
     for (int k = 0; k < kTrip; ++k) {
       const __nv_bfloat16* src = part + (size_t)(rows[k] >= 0 ? rows[k] : 0) * row_elems + in_row;
 #pragma unroll
       for (int h = 0; h < HG; ++h)
-        u[k][h] = rows[k] >= 0 ? __ldg(reinterpret_cast<const uint4*>(src + h * head_step))
+        u[k][h] = rows[k] >= 0 ? __ldcs(reinterpret_cast<const uint4*>(src + h * head_step))
                                : make_uint4(0u, 0u, 0u, 0u);
     }
 #pragma unroll
@@ -1279,29 +1284,29 @@ __global__ void dq_reduce3_kernel(const Reduce3Args a) {
   }
   if (a.part_slc) {
     const int32_t* ps = a.pair_of_slot + (size_t)qrow * a.S;
-    for (int s0 = 0; s0 < a.S; s0 += kTrip) {
-      long long rows[kTrip];
+    for (int s0 = 0; s0 < a.S; s0 += kTripSel) {
+      long long rows[kTripSel];
 #pragma unroll
-      for (int k = 0; k < kTrip; ++k) rows[k] = s0 + k < a.S ? (long long)__ldg(ps + s0 + k) : -1;
+      for (int k = 0; k < kTripSel; ++k) rows[k] = s0 + k < a.S ? (long long)__ldg(ps + s0 + k) : -1;
       add_rows(a.part_slc, rows);
     }
   }
   if (a.part_win) {
     const int first = max(0, t - a.window + 1) >> 6, last = t >> 6;
-    for (int j0 = first; j0 <= last; j0 += kTrip) {
-      long long rows[kTrip];
+    for (int j0 = first; j0 <= last; j0 += kTripWin) {
+      long long rows[kTripWin];
 #pragma unroll
-      for (int k = 0; k < kTrip; ++k) rows[k] = j0 + k <= last ? qrow * a.slots_win + (j0 + k) % a.slots_win : -1;
+      for (int k = 0; k < kTripWin; ++k) rows[k] = j0 + k <= last ? qrow * a.slots_win + (j0 + k) % a.slots_win : -1;
       add_rows(a.part_win, rows);
     }
   }
   if (a.part_cmp) {
     const int n_vis = cmp_visible(t, a.cmp_len, a.cmp_stride, a.Lk_cmp);
     const int last = n_vis > 0 ? (n_vis - 1) >> 6 : -1;
-    for (int j0 = 0; j0 <= last; j0 += kTrip) {
-      long long rows[kTrip];
+    for (int j0 = 0; j0 <= last; j0 += kTripCmp) {
+      long long rows[kTripCmp];
 #pragma unroll
-      for (int k = 0; k < kTrip; ++k) rows[k] = j0 + k <= last ? qrow * a.slots_cmp + j0 + k : -1;
+      for (int k = 0; k < kTripCmp; ++k) rows[k] = j0 + k <= last ? qrow * a.slots_cmp + j0 + k : -1;
       add_rows(a.part_cmp, rows);
     }
   }
@@ -1595,16 +1600,18 @@ int tc_dq_reduce3(const AttnArgs& base, int Lk_cmp, int cmp_len, int cmp_stride,
     r.part_win = (const __nv_bfloat16*)((const char*)ws_win + pl.off_part);
     r.slots_win = pl.n_slots;
   }
-  const int hg = r.G % 2 == 0 ? 2 : 1;                    // heads of a query served by one thread
+  const int hg = r.G % 2 == 0 ? 2 : (r.G % 3 == 0 ? 3 : 1);   // heads of a query served by one thread
   const size_t nthreads = (size_t)r.B * r.Hkv * r.T * (r.G / hg) * (base.D / 8);
   if (nthreads == 0) return NSA_OK;
   const unsigned grid = (unsigned)((nthreads + 255) / 256);
   KernelScope ks("dq_reduce3", st);
   if (base.D == 128) {
     if (hg == 2) dq_reduce3_kernel<128, 2><<<grid, 256, 0, st>>>(r);
+    else if (hg == 3) dq_reduce3_kernel<128, 3><<<grid, 256, 0, st>>>(r);
     else dq_reduce3_kernel<128, 1><<<grid, 256, 0, st>>>(r);
   } else {
     if (hg == 2) dq_reduce3_kernel<64, 2><<<grid, 256, 0, st>>>(r);
+    else if (hg == 3) dq_reduce3_kernel<64, 3><<<grid, 256, 0, st>>>(r);
     else dq_reduce3_kernel<64, 1><<<grid, 256, 0, st>>>(r);
   }
   NSA_LAUNCH_OK("dq_reduce3_kernel");
