@@ -751,9 +751,9 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
     const int n_ops = p.nq * per_q;                  // selection: the boxes of a tile
     constexpr int kRounds = (kMaxNq * kSlabs * 2 + 32 * kB2Producers - 1) / (32 * kB2Producers);
     auto box_of = [&](int r) -> int { return (r * 32 + lane) * kB2Producers + pw; };
-    auto tq_of = [&](int k, int o) -> int {          // query position of box o of tile k (none: past T, zeros)
+    auto tq_of = [&](int k, int o) -> int {          // pair of box o of tile k (none: past T, zeros)
       const int qi = (rt_begin + k) * p.nq + o / per_q;
-      return (o < n_ops && qi < n_q) ? (int)(ldg_s32_now(p.plan.pairs + pair_base + qi) & kPairPosMask) : p.T;
+      return (o < n_ops && qi < n_q) ? ldg_s32_now(p.plan.pairs + pair_base + qi) : p.T;
     };
     int tq[kRounds];
     if (p.kind == 2) {
@@ -786,18 +786,19 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
 #pragma unroll
         for (int r = 0; r < kRounds; ++r) {
           const int o = box_of(r);
+          const int t_box = (int)(tq[r] & kPairPosMask);   // here: not where the load would be waited for
           if (o < n_ops && p.merged) {
             tma_load_5d_hint(((o & 1) ? sDO : sQ) + (o >> 1) * (p.G / 8) * 2048, (o & 1) ? &tm_do : &tm_q, g_full + sb,
-                             0, 0, 0, tq[r], (b * p.Hq + hkv * p.G) >> 3, pol_keep);
+                             0, 0, 0, t_box, (b * p.Hq + hkv * p.G) >> 3, pol_keep);
           } else if (o < n_ops) {
             const int qq = o / (kSlabs * 2), kx = o % (kSlabs * 2);
             const int s = kx >> 1;
             if (kx & 1)
               tma_load_3d(sDO + s * (kRows * 128) + qq * p.G * 128, &tm_do, g_full + sb, s * 64,
-                          b * p.Hq + hkv * p.G, tq[r]);
+                          b * p.Hq + hkv * p.G, t_box);
             else
               tma_load_3d(sQ + s * (kRows * 128) + qq * p.G * 128, &tm_q, g_full + sb, s * 64,
-                          b * p.Hq + hkv * p.G, tq[r]);
+                          b * p.Hq + hkv * p.G, t_box);
           }
         }
         if (k + 1 < n_tiles) {

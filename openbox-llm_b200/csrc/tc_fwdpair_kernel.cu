@@ -157,10 +157,12 @@ tc_fwdpair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
     const int per_q = p.merged ? 1 : kSlabs;
     const int n_ops = p.nq * per_q;                  // at most 128: up to two per lane of the three warps
     const int o0 = lane * kPairProducers + pw, o1 = o0 + 32 * kPairProducers;   // this lane's boxes
-    // query position of one of this lane's boxes in tile k (a missing query reads past T: zeros)
+    // pair of one of this lane's boxes in tile k (a missing query reads past T: zeros).  The position is
+    // taken out of it when the box is sent: taken out here, the warp waits for the load before it looks at
+    // the next tile (8 x 32768 tokens, 16 heads: 4.80 ms so and 4.53 as it is)
     auto tq_of = [&](int k, int o) -> int {
       const int qi = (item.z + k) * p.nq + o / per_q;
-      return (o < n_ops && qi < n_q) ? (int)(ldg_s32_now(p.plan.pairs + pair_base + qi) & kPairPosMask) : p.T;
+      return (o < n_ops && qi < n_q) ? ldg_s32_now(p.plan.pairs + pair_base + qi) : p.T;
     };
     int tq0 = tq_of(0, o0), tq1 = tq_of(0, o1);
     for (int k = 0; k < n_tiles; ++k) {
@@ -174,7 +176,7 @@ tc_fwdpair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
       uint8_t* dst = sQ + st * kQBytes;
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
-        const int o = r ? o1 : o0, tq = r ? tq1 : tq0;
+        const int o = r ? o1 : o0, tq = (int)((r ? tq1 : tq0) & kPairPosMask);
         if (o < n_ops) {
           if (p.merged) {
             tma_load_5d_hint(dst + o * (p.G / 8) * 2048, &tm_q, q_full + st, 0, 0, 0, tq, (b * p.Hq + hkv * p.G) >> 3,
