@@ -36,7 +36,8 @@ extern "C" {
 #define NSA_MODE_COMPRESS_STRIDED 3   /* no counterpart in the reference: `window` is the summary stride */
 
 /* which kernel family serves a call */
-#define NSA_IMPL_AUTO 0   /* tcgen05 kernels when the shape allows, else the SIMT kernels */
+#define NSA_IMPL_AUTO 0   /* tcgen05 kernels when the shape allows, else the SIMT kernels; selection on blocks
+                             of 16 or 32 tokens always SIMT, whose arithmetic is fp32 throughout */
 #define NSA_IMPL_SIMT 1   /* CUDA-core kernels: any dtype, D in {16,32,64,128}, any G and block size */
 #define NSA_IMPL_TC   2   /* tcgen05/TMEM kernels only; NSA_ERR_UNSUPPORTED if the shape does not fit */
 
@@ -100,9 +101,9 @@ int nsa_selection_bwd(const void* q, const void* k, const void* v, const int32_t
 
 /* The tcgen05 selection kernels walk the block list block by block: the queries of each block (what
  * nsa_fsa.py:14-64 builds), the (query, slot) -> pair map and a work list, which nsa_selection_fwd
- * and nsa_selection_bwd each build inside their workspace.  A caller that runs both on one block list (every training step)
- * can build them once into a buffer of nsa_selection_plan_bytes bytes (0: shape not served by the
- * tcgen05 kernels) and hand it to the *_planned forms, which read it instead of building
+ * and nsa_selection_bwd each build inside their workspace.  A caller that runs both on one block list
+ * (every training step) can build them once into a buffer of nsa_selection_plan_bytes bytes (0: NSA_IMPL_AUTO does not run
+ * this call on the tcgen05 kernels) and hand it to the *_planned forms, which read it instead of building
  * their own.  The reference builds its CSR once per forward and once per backward
  * (nsa_selection_kernel.py:199-201, nsa_selection_backward.py:356-358); no counterpart for the
  * reuse. */

@@ -131,9 +131,15 @@ AttnArgs base_args(const NsaDims* d, int Lk) {
   return a;
 }
 
+// NSA_IMPL_AUTO leaves selection on blocks of 16 and 32 tokens to the CUDA cores, whose probabilities, dS and
+// partial sums are fp32; the tcgen05 kernels keep P, dS and the dQ partials in bf16, which on these
+// blocks a caller asks for with NSA_IMPL_TC.  Against 64-bit arithmetic (T of 130 to 2047, D of 64
+// and 128) o and dq are off by 1.66e-3 and 1.7e-3 here, the rounding of a bf16 result, and by 2.1e-3 to 2.6e-3
+// and 2.6e-3 to 2.9e-3 there.  The price is time: the whole op forward + backward on 16-token blocks,
+// 2 x 1024 tokens, 16 heads of 128, takes 1.26 ms, on the tensor cores 0.33.
 bool use_tc(const NsaDims* d, int block_size, int impl, int* err) {
   *err = NSA_OK;
-  if (impl == NSA_IMPL_SIMT) return false;
+  if (impl == NSA_IMPL_SIMT || (impl == NSA_IMPL_AUTO && (block_size == 16 || block_size == 32))) return false;
   const bool ok = tc_shape_ok(*d, block_size);
   if (impl == NSA_IMPL_TC && !ok) {
     set_error("shape not served by the tcgen05 kernels (bf16, D in {64,128}, blocks of 16, 32 or 64 tokens, 2 to 128 query heads per kv head)");
@@ -456,7 +462,7 @@ extern "C" int nsa_selection_plan_build(const int32_t* block_idx, const NsaDims*
   int rc = check_sel(dims, S, block_size);
   if (rc != NSA_OK) return rc;
   NSA_CHECK_ARG(S > 0 && block_idx && plan, "null block_idx or plan");
-  NSA_CHECK_ARG(use_tc(dims, block_size, NSA_IMPL_AUTO, &rc), "a selection plan needs a shape the tcgen05 kernels serve");
+  NSA_CHECK_ARG(use_tc(dims, block_size, NSA_IMPL_AUTO, &rc), "a selection plan needs a call that NSA_IMPL_AUTO gives to the tcgen05 kernels");
   AttnArgs a = base_args(dims, dims->T);
   a.block_idx = block_idx; a.kind = 2; a.S = S; a.block_size = block_size;
   return tc_sel_plan_build(a, plan, plan_bytes, (cudaStream_t)stream);
@@ -534,7 +540,7 @@ extern "C" int nsa_dq_reduce3(const NsaDims* dims, int Lk_cmp, int cmp_len, int 
   int rc = check_dims(dims);
   if (rc != NSA_OK) return rc;
   NSA_CHECK_ARG(dq, "null dq");
-  NSA_CHECK_ARG(use_tc(dims, block_size, NSA_IMPL_AUTO, &rc), "nsa_dq_reduce3 needs a shape the tcgen05 kernels serve");
+  NSA_CHECK_ARG(tc_shape_ok(*dims, block_size), "nsa_dq_reduce3 needs a shape the tcgen05 kernels serve");
   if (cmp_stride <= 0) cmp_stride = cmp_len;
   NSA_CHECK_ARG(!ws_cmp || (Lk_cmp > 0 && cmp_len > 0 && cmp_stride <= cmp_len), "bad compression geometry");
   NSA_CHECK_ARG(!ws_slc || S > 0, "bad S");
@@ -549,7 +555,7 @@ extern "C" int nsa_dq_finish(const NsaDims* dims, int S, int block_size, const f
   int rc = check_dims(dims);
   if (rc != NSA_OK) return rc;
   NSA_CHECK_ARG(dq && dq_acc, "null dq or accumulator");
-  NSA_CHECK_ARG(use_tc(dims, block_size, NSA_IMPL_AUTO, &rc), "nsa_dq_finish needs a shape the tcgen05 kernels serve");
+  NSA_CHECK_ARG(tc_shape_ok(*dims, block_size), "nsa_dq_finish needs a shape the tcgen05 kernels serve");
   NSA_CHECK_ARG(!ws_slc || S > 0, "bad S");
   const AttnArgs a = base_args(dims, dims->T);
   return tc_dq_reduce3(a, 0, 0, 0, S, block_size, 1, nullptr, ws_slc, nullptr, nullptr, dq_acc, dq, (cudaStream_t)stream);

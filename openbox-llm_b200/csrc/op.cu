@@ -114,7 +114,13 @@ struct OpPlan {
   size_t row_stat, dk_cmp, dv_cmp, acc, acc_bytes, d_pooled, ws_pool, ws_pool_bytes, dq_acc, dq3, ws[3], ws_bytes[3], bwd_ws;
 };
 
-// mode argument of the range entry points for the compression branch
+// the selection branch of a call as the tcgen05 plan sees it
+AttnArgs sel_args(const NsaAttentionDesc* d, const int32_t* block_idx) {
+  AttnArgs a = base_args(&d->dims, d->dims.T);
+  a.block_idx = block_idx; a.kind = 2; a.S = d->n_sel; a.block_size = d->block_size;
+  return a;
+}
+
 int op_plan(const NsaAttentionDesc* d, OpPlan* p) {
   int rc = check_dims(&d->dims);
   if (rc != NSA_OK) return rc;
@@ -146,7 +152,7 @@ int op_plan(const NsaAttentionDesc* d, OpPlan* p) {
   p->lse3 = s.take(3 * p->rows * sizeof(float));
   p->pooled = s.take(grad && p->fast_pool ? 2 * p->n_c * sizeof(float) : 0);
   p->fwd_ws = nsa_selection_fwd_workspace_bytes(&m, p->S, d->block_size, d->impl);
-  if (p->fused && (grad || p->fwd_ws > 0)) p->plan_bytes = nsa_selection_plan_bytes(&m, p->S, d->block_size);
+  if (p->fused && (grad || p->fwd_ws > 0)) p->plan_bytes = tc_sel_plan_bytes(sel_args(d, nullptr));
   p->plan = s.take(p->plan_bytes);
   p->saved_total = s.off;
   if (!grad) return NSA_OK;
@@ -245,7 +251,7 @@ extern "C" int nsa_attention_fwd(const NsaAttentionDesc* d, const NsaAttentionTe
   NSA_TRY(nsa_range_attn_fwd(t->q, t->kw, t->vw, o[2], lse[2], &m, m.T, NSA_MODE_WINDOW, d->window, 0, d->impl, fork.stream(0)));
   // the selection branch with its plan; with given lists it waits for nothing
   auto selection = [&](cudaStream_t s) -> int {
-    if (plan) NSA_TRY(nsa_selection_plan_build(t->block_idx, &m, p.S, d->block_size, plan, p.plan_bytes, s));
+    if (plan) NSA_TRY(tc_sel_plan_build(sel_args(d, t->block_idx), plan, p.plan_bytes, s));
     if (plan && p.fwd_ws)
       return nsa_selection_fwd_planned(t->q, t->ks, t->vs, t->block_idx, o[1], lse[1], &m, p.S, d->block_size,
                                        workspace, workspace_bytes, plan, s);
@@ -280,7 +286,7 @@ extern "C" int nsa_attention_fwd(const NsaAttentionDesc* d, const NsaAttentionTe
                                       d->impl == NSA_IMPL_TC ? NSA_IMPL_AUTO : d->impl, stream));
     if (plan && !p.fwd_ws) {      // only the backward reads the plan: it is built beside the forward kernel
       NSA_TRY(fork.begin());
-      NSA_TRY(nsa_selection_plan_build(t->block_idx, &m, p.S, d->block_size, plan, p.plan_bytes, fork.stream(1)));
+      NSA_TRY(tc_sel_plan_build(sel_args(d, t->block_idx), plan, p.plan_bytes, fork.stream(1)));
       NSA_TRY(nsa_selection_fwd(t->q, t->ks, t->vs, t->block_idx, o[1], lse[1], &m, p.S, d->block_size, nullptr, 0,
                                 d->impl, stream));
     } else {

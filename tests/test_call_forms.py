@@ -1,0 +1,68 @@
+"""Forms of a call that choose a path without changing the mathematics: block sizes, views, streams,
+refused arguments, non-finite values where nothing attends them."""
+import pytest
+import torch
+
+from oracle import nsa_oracle as O
+from tests.util import cfg_id, dev, make_inputs, pkg
+
+pytestmark = pytest.mark.gpu
+
+
+def _selection_64(t, idx, bs):
+    """Selection attention and its gradients in 64-bit arithmetic, dense, on the CPU."""
+    q, k, v, do = (t[n].double() for n in ("q", "ks", "vs", "do"))
+    B, Hq, T, D = q.shape
+    G = Hq // k.shape[1]
+    kk, vv = k.repeat_interleave(G, 1), v.repeat_interleave(G, 1)
+    keep = torch.zeros(B, k.shape[1], T, T + bs, dtype=torch.bool)
+    for s in range(idx.shape[-1]):
+        for e in range(bs):
+            pos = idx[..., s].long() * bs + e
+            ok = (idx[..., s] >= 0) & (pos <= torch.arange(T))
+            keep.scatter_(3, torch.where(ok, pos, T + e % bs)[..., None], True)
+    keep = keep[..., :T].repeat_interleave(G, 1)
+    s = (q @ kk.transpose(-1, -2) * D ** -0.5).masked_fill(~keep, float("-inf"))
+    lse = torch.logsumexp(s, -1)
+    p = torch.where(keep, (s - lse[..., None]).exp(), torch.zeros(()).double())
+    o = p @ vv
+    delta = (do * o).sum(-1)
+    ds = p * (do @ vv.transpose(-1, -2) - delta[..., None]) * D ** -0.5
+    fold = lambda x: x.view(B, k.shape[1], G, T, D).sum(2)
+    return o, lse, delta, ds @ kk, fold(ds.transpose(-1, -2) @ q), fold(p.transpose(-1, -2) @ do)
+
+
+@pytest.mark.parametrize("c", [dict(B=1, Hq=4, Hkv=2, D=64, T=200, block_size=16, S=3),
+                               dict(B=1, Hq=8, Hkv=2, D=128, T=330, block_size=16, S=2),
+                               dict(B=2, Hq=6, Hkv=2, D=64, T=256, block_size=32, S=4)], ids=cfg_id)
+def test_small_blocks_are_fp32_arithmetic(c):
+    """Selection on 16- and 32-token blocks by default: every result is the 64-bit value rounded to bf16 (8
+    significant bits: half a step is at most 2^-8 of the value), plus what fp32 arithmetic leaves: sums
+    of a few hundred terms and exponents of up to 2^3, each good to 2^-24, under 2e-5 of the largest
+    value.  Probabilities in bf16 (2^-9 of the largest terms) miss that wherever terms cancel."""
+    nsa = pkg()
+    t = make_inputs(c, torch.bfloat16, seed=3)
+    bs, idx = c["block_size"], t["block_idx"]
+    o64, lse64, delta, dq64, dk64, dv64 = _selection_64(t, idx, bs)
+    live = torch.isfinite(lse64)
+    q, k, v, do = (dev(t[n], torch.bfloat16) for n in ("q", "ks", "vs", "do"))
+
+    def close(got, want, what):
+        bound = 2.0 ** -8 * want.abs() + 2e-5 * want.abs().max()
+        assert ((got.double().cpu() - want).abs() <= bound).all(), what
+
+    o, lse = nsa.selection_forward_triton(q, k, v, idx.cuda(), bs, return_lse=True)
+    close(o, o64, "o")
+    close(nsa.selection_attn_triton(q, k, v, idx.cuda(), bs), o64, "o through autograd")
+    ones = torch.ones_like(lse)
+    lse_in = torch.where(live, lse64, torch.full_like(lse64, O.LSE_EMPTY)).float().cuda()
+    grads = nsa.ops._selection_backward(q, k, v, idx.cuda(), bs, do, o, lse_in, ones, delta.float().cuda())
+    for got, want, what in zip(grads, (dq64, dk64, dv64), ("dq", "dk", "dv")):
+        close(got, want, what)
+    # the whole op, its gate open for the selection branch alone
+    gate = torch.tensor([-1e4, 1e4, -1e4]).expand(*t["gate"].shape).bfloat16().cuda()
+    ins = [dev(t[n], torch.bfloat16) for n in ("q", "kc", "vc", "ks", "vs", "kw", "vw")]
+    close(nsa.nsa_fused_forward(*ins, gate, idx.cuda(), bs, 64), o64, "o of the whole op")
+    ins = [x.requires_grad_(True) for x in ins]
+    close(nsa.nsa_fused_forward(*ins, gate, idx.cuda(), bs, 64), o64, "o of the whole op, training")
+    assert nsa.lib().nsa_device_status(None) == 0
