@@ -38,6 +38,8 @@ struct FwdArgs {
   int nw;                    // 32-bit membership words per block = ceil(nq / 32)
   int n_sub;                 // selection: list blocks per 64-key tile (64 / block_size)
   float scale_log2;
+  float neg_zero;            // -0: what a product is added to where it has to be rounded by itself (a packed mul
+                             //     and the add after it are merged into one fma, whatever their rounding says)
 };
 
 // D = 128: Q 32 KB + two stages of K and V = 96 KB, two CTAs per SM.  D = 64: four stages in 80 KB.
@@ -97,12 +99,12 @@ __device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) {
 // Selection builds the list of a row tile's key tiles first, all threads together, and so works row
 // tile by row tile.
 //
-// Compression rounds score * scale before the maximum is subtracted and sums a tile's probabilities
-// in column order, a few instructions per key more than the others' fused form.  A shift common to
-// all keys leaves a softmax as it is, so the gradients of the summaries sum to zero over the keys and
-// the gradient of the key pooling's position parameters is what rounding leaves of that sum, 3e-4
-// of the other gradients.  Any other rounding here, or order of the sum in backward, is as exact
-// and replaces these values by others of their size; with this one they stay what they were.
+// Score * scale is rounded before the maximum is subtracted, and a tile's probabilities are summed in
+// column order: the three branches give the same bits on the same keys.  (A shift common to all keys
+// leaves a softmax as it is, so the gradients of the summaries sum to zero over the keys and the
+// gradient of the key pooling's position parameters is what rounding leaves of that sum, 3e-4 of the
+// other gradients.  Any other rounding here, or order of the sum in backward, is as exact and replaces
+// these values by others of their size.)
 template <int D, int kKind>
 __global__ void __launch_bounds__(kFwdThreads, 2)
 tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
@@ -464,20 +466,19 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
               sc2[k] = pack_f32x2(sc, sc);
               mn2[k] = pack_f32x2(mn, mn);
             }
-            uint64_t ps[2] = {0ull, 0ull};
+            const uint64_t nz2 = pack_f32x2(p.neg_zero, p.neg_zero);
+            float psum = 0.f;
 #pragma unroll
             for (int cc = 0; cc < 32; ++cc) {
               float p0, p1;
-              unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(r[2 * cc]), __uint_as_float(r[2 * cc + 1])), sc2[kSel ? cc >> 3 : 0],
-                                     mn2[kSel ? cc >> 3 : 0]), p0, p1);
+              unpack_f32x2(add_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(r[2 * cc]), __uint_as_float(r[2 * cc + 1])),
+                                               sc2[kSel ? cc >> 3 : 0], nz2), mn2[kSel ? cc >> 3 : 0]), p0, p1);
               p0 = ex2(p0);
               p1 = ex2(p1);
-              ps[cc & 1] = add_f32x2(ps[cc & 1], pack_f32x2(p0, p1));
+              psum += p0 + p1;
               pk[cc] = pack_bf16(p0, p1);
             }
-            float s0, s1;
-            unpack_f32x2(add_f32x2(ps[0], ps[1]), s0, s1);
-            l_sum += s0 + s1;
+            l_sum += psum;
           }
           // O may be touched once PV of the tile before is done; only a warp that has to rescale waits
           if (i > 0 && __any_sync(0xffffffffu, rescale)) {
@@ -593,6 +594,7 @@ static int launch_fwd(const AttnArgs& a, const SelPlanHeader* plan, int force, c
   p.nw = (p.nq + 31) / 32;
   p.n_sub = a.kind == 2 ? kKeys / a.block_size : 1;
   p.scale_log2 = a.scale * kLog2e;
+  p.neg_zero = -0.f;
   CUtensorMap tm_q, tm_k, tm_v;
   int rc = make_map_query_rows(&tm_q, a.q, a.D, a.T, a.B * a.Hq, p.G, p.nq);
   if (rc == NSA_OK) rc = make_map(&tm_k, a.k, a.D, a.Lk, a.B * a.Hkv, kKeys, 1);

@@ -66,3 +66,21 @@ def test_small_blocks_are_fp32_arithmetic(c):
     ins = [x.requires_grad_(True) for x in ins]
     close(nsa.nsa_fused_forward(*ins, gate, idx.cuda(), bs, 64), o64, "o of the whole op, training")
     assert nsa.lib().nsa_device_status(None) == 0
+
+
+@pytest.mark.parametrize("c", [dict(B=1, Hq=8, Hkv=2, D=64, T=1000), dict(B=2, Hq=16, Hkv=1, D=128, T=448),
+                               dict(B=1, Hq=6, Hkv=2, D=64, T=333)], ids=str)
+def test_branches_round_alike(c):
+    """The three branches on the same keys give the same bits: a window over everything, summaries of one
+    token each, and a list of every block (query-outer kernel) are one attention in one order."""
+    nsa = pkg()
+    B, Hq, Hkv, D, T = (c[n] for n in ("B", "Hq", "Hkv", "D", "T"))
+    g = torch.Generator().manual_seed(8)
+    q, k, v = (torch.randn(B, h, T, D, generator=g).bfloat16().cuda() for h in (Hq, Hkv, Hkv))
+    o, lse = nsa.range_attn_forward(q, k, v, nsa.MODE_COMPRESS, 0, 1)
+    idx = torch.arange((T + 63) // 64, dtype=torch.int32, device="cuda").expand(B, Hkv, T, -1).contiguous()
+    nsa.set_option("sel_fwd_variant", 1)
+    for o2, lse2 in (nsa.range_attn_forward(q, k, v, nsa.MODE_WINDOW, T, 0),
+                     nsa.selection_forward_triton(q, k, v, idx, 64, return_lse=True)):
+        assert torch.equal(o, o2) and torch.equal(lse, lse2)
+    assert nsa.lib().nsa_device_status(None) == 0
