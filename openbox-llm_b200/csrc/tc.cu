@@ -388,98 +388,48 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           float alpha = 1.f;
           bool rescale = false;
           uint32_t pk[32];
-          if constexpr (kCmp) {
-            float xs[64];
-            float tmax = -INFINITY;
-            if (lo <= 0 && hi >= kKeys - 1) {
+          // Masking is by select: what a row does not attend may be infinite or NaN.  A row that attends the
+          // whole tile or none of it needs no work per element (none: its P is set to zero below); only
+          // rows whose range ends inside the tile, or that attend some 16-column groups of it, do.
+          const bool none = hi < 0;
+          if (!(lo <= 0 && (hi >= kKeys - 1 || none) && (!kSel || groups == 0xfu))) {
 #pragma unroll
-              for (int cc = 0; cc < 64; ++cc) {
-                xs[cc] = __uint_as_float(r[cc]) * p.scale_log2;
-                tmax = fmaxf(tmax, xs[cc]);
-              }
-            } else {
-#pragma unroll
-              for (int cc = 0; cc < 64; ++cc) {
-                xs[cc] = (cc >= lo && cc <= hi) ? __uint_as_float(r[cc]) * p.scale_log2 : -INFINITY;
-                tmax = fmaxf(tmax, xs[cc]);
-              }
-            }
-            if (tmax > m_used + 8.f) {
-              if (m_used != -INFINITY) {
-                alpha = ex2(m_used - tmax);
-                rescale = true;
-                l_sum *= alpha;
-              }
-              m_used = tmax;
-            }
-            const float msub = (m_used == -INFINITY) ? 0.f : m_used;
-            float psum = 0.f;
-#pragma unroll
-            for (int cc = 0; cc < 32; ++cc) {
-              const float p0 = ex2(xs[2 * cc] - msub), p1 = ex2(xs[2 * cc + 1] - msub);
-              psum += p0 + p1;
-              pk[cc] = pack_bf16(p0, p1);
-            }
-            l_sum += psum;
-          } else {
-            // A row that attends the whole tile or none of it, or whole 16-column groups of it, needs no
-            // work per element: a group it does not attend gets the exponent 0 * s - inf.  Only rows whose
-            // range ends inside the tile mask their columns one by one.
-            if (!(lo <= 0 && (hi >= kKeys - 1 || hi < 0))) {
-#pragma unroll
-              for (int cc = 0; cc < 64; ++cc)
-                if (cc < lo || cc > hi) r[cc] = __float_as_uint(-3.0e38f);   // finite: 0 * r has to be 0
-            }
-            float tmax[4];                      // of the four column groups
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              float m0 = __uint_as_float(r[16 * k]), m1 = __uint_as_float(r[16 * k + 1]);
-#pragma unroll
-              for (int cc = 2; cc < 16; cc += 2) {
-                m0 = fmaxf(m0, __uint_as_float(r[16 * k + cc]));
-                m1 = fmaxf(m1, __uint_as_float(r[16 * k + cc + 1]));
-              }
-              tmax[k] = fmaxf(m0, m1);
-            }
-            if (hi < 0) groups = 0u;
-            if (kSel) {
-#pragma unroll
-              for (int k = 0; k < 4; ++k) tmax[k] = ((groups >> k) & 1u) ? tmax[k] : -INFINITY;
-            }
-            float tm = fmaxf(fmaxf(tmax[0], tmax[1]), fmaxf(tmax[2], tmax[3]));
-            if (!kSel) tm = hi < 0 ? -INFINITY : tm;
-            tm *= p.scale_log2;
-            if (tm > m_used + 8.f) {              // also the first finite maximum (m_used = -inf)
-              if (m_used != -INFINITY) {
-                alpha = ex2(m_used - tm);
-                rescale = true;
-                l_sum *= alpha;
-              }
-              m_used = tm;
-            }
-            const float msub = (m_used == -INFINITY) ? 0.f : m_used;
-            uint64_t sc2[kSel ? 4 : 1], mn2[kSel ? 4 : 1];
-#pragma unroll
-            for (int k = 0; k < (kSel ? 4 : 1); ++k) {
-              const bool on = (groups >> k) & 1u;
-              const float sc = on ? p.scale_log2 : 0.f, mn = on ? -msub : -INFINITY;
-              sc2[k] = pack_f32x2(sc, sc);
-              mn2[k] = pack_f32x2(mn, mn);
-            }
-            const uint64_t nz2 = pack_f32x2(p.neg_zero, p.neg_zero);
-            float psum = 0.f;
-#pragma unroll
-            for (int cc = 0; cc < 32; ++cc) {
-              float p0, p1;
-              unpack_f32x2(add_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(r[2 * cc]), __uint_as_float(r[2 * cc + 1])),
-                                               sc2[kSel ? cc >> 3 : 0], nz2), mn2[kSel ? cc >> 3 : 0]), p0, p1);
-              p0 = ex2(p0);
-              p1 = ex2(p1);
-              psum += p0 + p1;
-              pk[cc] = pack_bf16(p0, p1);
-            }
-            l_sum += psum;
+            for (int cc = 0; cc < 64; ++cc)
+              if (cc < lo || cc > hi || (kSel && !((groups >> (cc >> 4)) & 1u))) r[cc] = __float_as_uint(-INFINITY);
           }
+          float tmax[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+          for (int cc = 0; cc < 64; ++cc) tmax[cc & 3] = fmaxf(tmax[cc & 3], __uint_as_float(r[cc]));
+          // (the scale is positive: the largest scaled score is the scaled largest score)
+          const float tm = none ? -INFINITY : fmaxf(fmaxf(tmax[0], tmax[1]), fmaxf(tmax[2], tmax[3])) * p.scale_log2;
+          if (tm > m_used + 8.f) {                 // also the first finite maximum (m_used = -inf)
+            if (m_used != -INFINITY) {
+              alpha = ex2(m_used - tm);
+              rescale = true;
+              l_sum *= alpha;
+            }
+            m_used = tm;
+          }
+          const float msub = (m_used == -INFINITY) ? 0.f : m_used;
+          const uint64_t nz2 = pack_f32x2(p.neg_zero, p.neg_zero);
+          const uint64_t sc2 = pack_f32x2(p.scale_log2, p.scale_log2), mn2 = pack_f32x2(-msub, -msub);
+          float psum = 0.f;
+#pragma unroll
+          for (int cc = 0; cc < 32; ++cc) {
+            float p0, p1;
+            unpack_f32x2(add_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(r[2 * cc]), __uint_as_float(r[2 * cc + 1])), sc2, nz2),
+                                   mn2), p0, p1);
+            p0 = ex2(p0);
+            p1 = ex2(p1);
+            psum += p0 + p1;
+            pk[cc] = pack_bf16(p0, p1);
+          }
+          if (none) {
+            psum = 0.f;
+#pragma unroll
+            for (int cc = 0; cc < 32; ++cc) pk[cc] = 0u;
+          }
+          l_sum += psum;
           // O may be touched once PV of the tile before is done; only a warp that has to rescale waits
           if (i > 0 && __any_sync(0xffffffffu, rescale)) {
             ok = mbar_wait(bar_o + ((c - 1) & 1), ((c - 1) >> 1) & 1, p.status, s_abort, 8);

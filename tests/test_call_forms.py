@@ -84,3 +84,48 @@ def test_branches_round_alike(c):
                      nsa.selection_forward_triton(q, k, v, idx, 64, return_lse=True)):
         assert torch.equal(o, o2) and torch.equal(lse, lse2)
     assert nsa.lib().nsa_device_status(None) == 0
+
+
+def _attends(kind, T, W, bs, idx, key):
+    """[B, Hkv, T] bool (or [T] for the window and compression): does the row of query t attend `key`?"""
+    t = torch.arange(T)
+    if kind == "window":
+        return (t >= key) & (t - key < W)
+    if kind == "compression":
+        return t >= (key + 1) * bs - 1
+    return (idx == key // bs).any(-1) & (t >= key)
+
+
+@pytest.mark.parametrize("bad", [float("inf"), float("-inf"), float("nan")], ids=str)
+@pytest.mark.parametrize("Hq,Hkv,D,bs", [(8, 2, 64, 64), (16, 1, 128, 64), (6, 2, 64, 16)])
+def test_forward_keeps_non_finite_keys_to_their_rows(Hq, Hkv, D, bs, bad):
+    """tcgen05 forward: a key that is infinite or NaN reaches the rows that attend it and no other; all other
+    rows keep their bits."""
+    nsa = pkg()
+    nsa.set_impl("tc")
+    B, T, W, S = 1, 500, 70, 3
+    c = dict(B=B, Hq=Hq, Hkv=Hkv, D=D, T=T, block_size=bs, S=S)
+    t = make_inputs(c, torch.bfloat16, seed=12)
+    q, k, v = (dev(t[n], torch.bfloat16) for n in ("q", "ks", "vs"))
+    idx = t["block_idx"]
+    n_cmp = T // bs
+
+    def runs(k):
+        yield "window", nsa.range_attn_forward(q, k, v, nsa.MODE_WINDOW, W, 0)
+        yield "compression", nsa.range_attn_forward(q, k[:, :, :n_cmp], v[:, :, :n_cmp], nsa.MODE_COMPRESS, 0, bs)
+        for variant in (1, 2):
+            nsa.set_option("sel_fwd_variant", variant)
+            yield "selection", nsa.selection_forward_triton(q, k, v, idx.cuda(), bs, return_lse=True)
+
+    clean = list(runs(k))
+    for key in (3, 66, 127, 300):
+        k2 = k.clone()
+        k2[:, :, key, 5] = bad
+        for (kind, (o, lse)), (_, (o2, lse2)) in zip(clean, runs(k2)):
+            if kind == "compression" and key >= n_cmp:
+                continue
+            hit = _attends(kind, T, W, bs, idx, key)
+            hit = (hit if hit.dim() == 3 else hit.expand(B, Hkv, T)).repeat_interleave(Hq // Hkv, 1).cuda()
+            assert hit.any() and not hit.all()
+            assert torch.equal(o[~hit], o2[~hit]) and torch.equal(lse[~hit], lse2[~hit]), (kind, key)
+    assert nsa.lib().nsa_device_status(None) == 0
