@@ -128,7 +128,7 @@ int op_plan(const NsaAttentionDesc* d, OpPlan* p) {
   NSA_CHECK_ARG(d->learned || (d->cmp_len == d->block_size && d->cmp_stride == d->block_size),
                 "mean pooling is defined on the aligned grid only");
   NSA_CHECK_ARG(d->block_size >= 16, "block_size must be >= 16");
-  NSA_CHECK_ARG(d->n_sel >= 0, "bad n_sel");
+  NSA_CHECK_ARG(d->n_sel >= (d->given_lists ? 0 : 1), "bad n_sel: the scorer picks at least one block");
   const NsaDims& m = d->dims;
   memset(p, 0, sizeof(*p));
   p->es = m.dtype == NSA_DTYPE_BF16 ? 2 : 4;
