@@ -764,6 +764,10 @@ bool tc_topn_ok(const NsaDims& d, int n_blk, int n_sel, int cmp_len, int stride,
 int tc_topn(const void* q, const void* k_cmp, const float* lse, int32_t* block_idx, float* imp_out,
             const NsaDims& d, int n_blk, int block_size, int n_sel, int n_init, int n_local, int stride,
             int sel_block, int imp_cols, cudaStream_t st);
+// shared memory of the CUDA-core scorer: four warps, each with a query and the importances of its row
+static size_t topn_smem(const NsaDims& d, int n_cmp, int sel_block) {
+  return (size_t)4 * (d.D + n_cmp + (d.T + sel_block - 1) / sel_block + 1) * sizeof(float);
+}
 }
 
 extern "C" int nsa_topn_blocks(const void* q, const void* k_cmp, const float* lse_cmp,
@@ -781,17 +785,36 @@ extern "C" int nsa_topn_blocks_forced(const void* q, const void* k_cmp, const fl
                                  block_size, block_size, n_sel, n_init, n_local, impl, stream);
 }
 
+namespace nsa {
+// What the scorer asks of a call's sizes, checked before anything is launched.
+int topn_check(const NsaDims* dims, int n_cmp, int cmp_len, int cmp_stride, int sel_block, int n_sel, int n_init,
+               int n_local, int impl) {
+  NSA_CHECK_ARG(n_init >= 0 && n_local >= 0 && n_init < (1 << 18) && n_local < (1 << 18), "bad forced block counts");
+  NSA_CHECK_ARG(dims->Hkv > 0 && dims->Hq % dims->Hkv == 0, "Hq must be a multiple of Hkv");
+  NSA_CHECK_ARG(cmp_len > 0 && n_sel > 0 && n_cmp >= 0, "bad block_size/n_sel/n_blk");
+  NSA_CHECK_ARG(cmp_stride > 0 && cmp_stride <= cmp_len && cmp_len % cmp_stride == 0 && sel_block > 0 &&
+                sel_block % cmp_stride == 0, "summary length and selection block must be multiples of the stride");
+  if ((size_t)dims->B * dims->Hkv * dims->T == 0) return NSA_OK;
+  if (impl != NSA_IMPL_SIMT) {
+    if (tc_topn_ok(*dims, n_cmp, n_sel, cmp_len, cmp_stride, sel_block)) return NSA_OK;
+    if (impl == NSA_IMPL_TC) {
+      set_error("scoring shape not served by the tcgen05 kernel");
+      return NSA_ERR_UNSUPPORTED;
+    }
+  }
+  NSA_CHECK_ARG(topn_smem(*dims, n_cmp, sel_block) <= 200 * 1024, "n_blk %d too large for the scoring kernel", n_cmp);
+  return NSA_OK;
+}
+}  // namespace nsa
+
 extern "C" int nsa_topn_blocks_general(const void* q, const void* k_cmp, const float* lse_cmp,
                                        int32_t* block_idx, float* importance_out, const NsaDims* dims,
                                        int n_cmp, int cmp_len, int cmp_stride, int sel_block, int n_sel,
                                        int n_init, int n_local, int impl, void* stream) {
   const int n_blk = n_cmp, block_size = cmp_len;
   NSA_CHECK_ARG(dims && q && lse_cmp && block_idx && (k_cmp || n_blk == 0), "null argument");
-  NSA_CHECK_ARG(n_init >= 0 && n_local >= 0 && n_init < (1 << 18) && n_local < (1 << 18), "bad forced block counts");
-  NSA_CHECK_ARG(dims->Hkv > 0 && dims->Hq % dims->Hkv == 0, "Hq must be a multiple of Hkv");
-  NSA_CHECK_ARG(block_size > 0 && n_sel > 0 && n_blk >= 0, "bad block_size/n_sel/n_blk");
-  NSA_CHECK_ARG(cmp_stride > 0 && cmp_stride <= cmp_len && cmp_len % cmp_stride == 0 && sel_block > 0 &&
-                sel_block % cmp_stride == 0, "summary length and selection block must be multiples of the stride");
+  const int rc = topn_check(dims, n_cmp, cmp_len, cmp_stride, sel_block, n_sel, n_init, n_local, impl);
+  if (rc != NSA_OK) return rc;
   const bool aligned = cmp_len == cmp_stride && cmp_stride == sel_block;
   const int n_sblk = (dims->T + sel_block - 1) / sel_block;
   const int imp_cols = aligned ? n_blk : n_sblk;     // the aligned call keeps its [.., n_blk] layout
@@ -799,17 +822,10 @@ extern "C" int nsa_topn_blocks_general(const void* q, const void* k_cmp, const f
   cudaStream_t st = (cudaStream_t)stream;
   const size_t units = (size_t)dims->B * dims->Hkv * dims->T;
   if (units == 0) return NSA_OK;
-  if (impl != NSA_IMPL_SIMT) {
-    if (tc_topn_ok(*dims, n_blk, n_sel, cmp_len, cmp_stride, sel_block))
-      return tc_topn(q, k_cmp, lse_cmp, block_idx, importance_out, *dims, n_blk, block_size, n_sel, n_init,
-                     n_local, cmp_stride, sel_block, imp_cols, st);
-    if (impl == NSA_IMPL_TC) {
-      set_error("scoring shape not served by the tcgen05 kernel");
-      return NSA_ERR_UNSUPPORTED;
-    }
-  }
-  const size_t sm = (size_t)4 * (D + n_blk + n_sblk + 1) * sizeof(float);
-  NSA_CHECK_ARG(sm <= 200 * 1024, "n_blk %d too large for the scoring kernel", n_blk);
+  if (impl != NSA_IMPL_SIMT && tc_topn_ok(*dims, n_blk, n_sel, cmp_len, cmp_stride, sel_block))
+    return tc_topn(q, k_cmp, lse_cmp, block_idx, importance_out, *dims, n_blk, block_size, n_sel, n_init,
+                   n_local, cmp_stride, sel_block, imp_cols, st);
+  const size_t sm = topn_smem(*dims, n_blk, sel_block);
   const float scale = 1.0f / sqrtf((float)D);
   const unsigned grid = blocks_for(units, 4);
 #define NSA_TOPN(TT, DD)                                                                        \

@@ -59,7 +59,8 @@ SideStreams* side_streams() {
   return &s;
 }
 
-// Forks the side streams off `main` and joins them again.  Off (everything on `main`) when the
+// Forks the side streams off `main` and joins them again; a call that fails in between joins them as it
+// returns, since its caller gives back the memory they work in.  Off (everything on `main`) when the
 // call fills the GPU by itself, when launches are being timed, or when a side stream is inside
 // somebody else's stream capture.
 class Fork {
@@ -74,26 +75,39 @@ class Fork {
       if (cudaStreamIsCapturing(side_->st[k], &theirs) != cudaSuccess ||
           (theirs != cudaStreamCaptureStatusNone && mine == cudaStreamCaptureStatusNone)) { drop(); return; }
   }
+  ~Fork() {
+    if (open_ && rejoin() != cudaSuccess) cudaGetLastError();   // the failure that led here is the one to report
+  }
+  Fork(const Fork&) = delete;
+  Fork& operator=(const Fork&) = delete;
   cudaStream_t stream(int k) const { return side_ ? side_->st[k] : main_; }
   int begin() {                                    // the side streams see what `main` holds so far
     if (!side_) return NSA_OK;
+    open_ = true;
     NSA_CUDA_OK(cudaEventRecord(side_->begin, main_));
     for (int k = 0; k < 2; ++k) NSA_CUDA_OK(cudaStreamWaitEvent(side_->st[k], side_->begin, 0));
     return NSA_OK;
   }
   int join() {
-    if (!side_) return NSA_OK;
-    for (int k = 0; k < 2; ++k) {
-      NSA_CUDA_OK(cudaEventRecord(side_->end[k], side_->st[k]));
-      NSA_CUDA_OK(cudaStreamWaitEvent(main_, side_->end[k], 0));
-    }
+    if (open_) NSA_CUDA_OK(rejoin());
     return NSA_OK;
   }
 
  private:
   void drop() { cudaGetLastError(); side_ = nullptr; }
+  cudaError_t rejoin() {
+    open_ = false;
+    cudaError_t rc = cudaSuccess;
+    for (int k = 0; k < 2; ++k) {                  // one stream's error does not leave the other unjoined
+      cudaError_t e = cudaEventRecord(side_->end[k], side_->st[k]);
+      if (e == cudaSuccess) e = cudaStreamWaitEvent(main_, side_->end[k], 0);
+      if (e != cudaSuccess) rc = e;
+    }
+    return rc;
+  }
   cudaStream_t main_;
   SideStreams* side_ = nullptr;
+  bool open_ = false;       // forked and not joined yet
 };
 
 struct Carver {
@@ -114,6 +128,10 @@ struct OpPlan {
   size_t row_stat, dk_cmp, dv_cmp, acc, acc_bytes, d_pooled, ws_pool, ws_pool_bytes, dq_acc, dq3, ws[3], ws_bytes[3], bwd_ws;
 };
 
+// impl chooses the attention kernels; lists longer than the tensor-core scorer keeps (16) are scored on
+// the CUDA cores even where it names the former
+int score_impl(const NsaAttentionDesc* d) { return d->impl == NSA_IMPL_TC ? NSA_IMPL_AUTO : d->impl; }
+
 // the selection branch of a call as the tcgen05 plan sees it
 AttnArgs sel_args(const NsaAttentionDesc* d, const int32_t* block_idx) {
   AttnArgs a = base_args(&d->dims, d->dims.T);
@@ -128,7 +146,13 @@ int op_plan(const NsaAttentionDesc* d, OpPlan* p) {
   NSA_CHECK_ARG(d->learned || (d->cmp_len == d->block_size && d->cmp_stride == d->block_size),
                 "mean pooling is defined on the aligned grid only");
   NSA_CHECK_ARG(d->block_size >= 16, "block_size must be >= 16");
+  NSA_CHECK_ARG(d->window >= 1, "window must be >= 1");
   NSA_CHECK_ARG(d->n_sel >= (d->given_lists ? 0 : 1), "bad n_sel: the scorer picks at least one block");
+  if (!d->given_lists) {
+    rc = topn_check(&d->dims, pool_count(d->dims.T, d->cmp_len, d->cmp_stride), d->cmp_len, d->cmp_stride, d->block_size,
+                    d->n_sel, d->n_init, d->n_local, score_impl(d));
+    if (rc != NSA_OK) return rc;
+  }
   const NsaDims& m = d->dims;
   memset(p, 0, sizeof(*p));
   p->es = m.dtype == NSA_DTYPE_BF16 ? 2 : 4;
@@ -278,12 +302,8 @@ extern "C" int nsa_attention_fwd(const NsaAttentionDesc* d, const NsaAttentionTe
   NSA_TRY(nsa_range_attn_fwd(t->q, k_cmp, v_cmp, o[0], lse[0], &m, p.n_cmp, NSA_MODE_COMPRESS_STRIDED, d->cmp_stride,
                              d->cmp_len, d->impl, stream));
   if (!d->given_lists) {
-    // impl chooses the attention kernels; lists longer than the tensor-core scorer keeps (16) are scored
-    // on the CUDA cores even where it names the former
-    if (p.S > 0)
-      NSA_TRY(nsa_topn_blocks_general(t->q, k_cmp, lse[0], t->block_idx, nullptr, &m, p.n_cmp, d->cmp_len, d->cmp_stride,
-                                      d->block_size, p.S, d->n_init, d->n_local,
-                                      d->impl == NSA_IMPL_TC ? NSA_IMPL_AUTO : d->impl, stream));
+    NSA_TRY(nsa_topn_blocks_general(t->q, k_cmp, lse[0], t->block_idx, nullptr, &m, p.n_cmp, d->cmp_len, d->cmp_stride,
+                                      d->block_size, p.S, d->n_init, d->n_local, score_impl(d), stream));
     if (plan && !p.fwd_ws) {      // only the backward reads the plan: it is built beside the forward kernel
       NSA_TRY(fork.begin());
       NSA_TRY(tc_sel_plan_build(sel_args(d, t->block_idx), plan, p.plan_bytes, fork.stream(1)));

@@ -27,3 +27,53 @@ def test_sizes_of_a_valid_call():
 
 def test_scored_lists_need_a_slot():
     assert _sizes(n_sel=0) == -1
+
+
+@pytest.mark.parametrize("bad", [dict(cmp_stride=12), dict(cmp_stride=24), dict(block_size=40), dict(n_init=-1),
+                                 dict(n_local=1 << 18), dict(window=0), dict(T=1 << 20, dtype=1, n_sel=17)], ids=str)
+def test_bad_arguments_are_refused_before_any_launch(bad):
+    """What the scorer and the branches require is checked with the sizes: no kernel of a refused call runs."""
+    assert _sizes(**bad) == -1
+
+
+def _inputs(B, Hq, Hkv, T, D, seed=4):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    mk = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
+    return [mk(B, Hq, T, D)] + [mk(B, Hkv, T, D) for _ in range(6)] + [mk(B, Hq, T, 3)]
+
+
+def _off_by_one(t):
+    """The same values in a contiguous view that starts one element into its buffer."""
+    buf = t.new_empty(t.numel() + 1)
+    view = buf[1:].view(t.shape)
+    view.copy_(t)
+    return view
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("grad", [False, True])
+def test_a_call_that_fails_midway_joins_its_side_streams(grad):
+    """ks at an odd address is refused by its tensor map (on the host) after the window kernel has gone to
+    a side stream.  Under capture an unjoined side stream makes the capture fail; outside, the
+    caller's stream waits for the side streams' work, and the next call is right."""
+    nsa = pkg()
+    L = importlib.import_module("openbox-llm_b200._lib")
+    ins = [x.requires_grad_(grad) for x in _inputs(1, 16, 4, 512, 64)]
+    want = nsa.nsa_attention(*ins, 64, 4, 128)
+    bad = list(ins)
+    bad[3] = _off_by_one(ins[3].detach()).requires_grad_(grad)
+
+    def refused():
+        with pytest.raises(L.NsaError):
+            nsa.nsa_attention(*bad, 64, 4, 128)
+
+    refused()
+    assert torch.equal(nsa.nsa_attention(*ins, 64, 4, 128), want)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        refused()
+        out = nsa.nsa_attention(*ins, 64, 4, 128)
+    graph.replay()
+    assert torch.equal(out, want)
+    assert nsa.lib().nsa_device_status(None) == 0
