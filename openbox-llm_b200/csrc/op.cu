@@ -61,8 +61,8 @@ SideStreams* side_streams() {
 
 // Forks the side streams off `main` and joins them again; a call that fails in between joins them as it
 // returns, since its caller gives back the memory they work in.  Off (everything on `main`) when the
-// call fills the GPU by itself, when launches are being timed, or when a side stream is inside
-// somebody else's stream capture.
+// call fills the GPU by itself, when launches are being timed, or when a side stream is inside a
+// stream capture that `main` is not part of.
 class Fork {
  public:
   Fork(cudaStream_t main, bool want) : main_(main) {
@@ -70,10 +70,11 @@ class Fork {
     side_ = side_streams();
     if (!side_) return;
     cudaStreamCaptureStatus mine, theirs;
-    if (cudaStreamIsCapturing(main, &mine) != cudaSuccess) { drop(); return; }
+    unsigned long long my_id = 0, their_id = 0;
+    if (cudaStreamGetCaptureInfo(main, &mine, &my_id) != cudaSuccess) { drop(); return; }
     for (int k = 0; k < 2; ++k)
-      if (cudaStreamIsCapturing(side_->st[k], &theirs) != cudaSuccess ||
-          (theirs != cudaStreamCaptureStatusNone && mine == cudaStreamCaptureStatusNone)) { drop(); return; }
+      if (cudaStreamGetCaptureInfo(side_->st[k], &theirs, &their_id) != cudaSuccess ||
+          (theirs != cudaStreamCaptureStatusNone && (mine != theirs || my_id != their_id))) { drop(); return; }
   }
   ~Fork() {
     if (open_ && rejoin() != cudaSuccess) cudaGetLastError();   // the failure that led here is the one to report
