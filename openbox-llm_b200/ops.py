@@ -15,6 +15,7 @@ import ctypes
 import functools
 
 import torch
+from torch.autograd import forward_ad
 
 from . import _lib as L
 
@@ -654,8 +655,11 @@ class _NSAAttention(torch.autograd.Function):
 
 
 def _op(q, kv, gate_logits, block_idx, block_size, n_sel, window, forced, comp):
-    """The whole op, through autograd only where a gradient is asked for."""
-    if torch.is_grad_enabled() and any(t.requires_grad for t in (q, *kv, gate_logits, *(comp or ()))):
+    """The whole op: through the autograd node where a gradient is asked for, and inside a forward-mode
+    level, where the node refuses a tangent that the bare call would drop.  The bare call spares a short
+    forward 9 us of 66 (512 tokens, 16 heads)."""
+    if (torch.is_grad_enabled() and any(t.requires_grad for t in (q, *kv, gate_logits, *(comp or ())))) or (
+            getattr(forward_ad, "_current_level", 0) >= 0):
         return _NSAAttention.apply(q, *kv, gate_logits, block_size, n_sel, window, block_idx, forced, *(comp or ()))
     return _op_forward(q, kv, gate_logits, block_idx, block_size, n_sel, window, forced, comp, False)[:2]
 

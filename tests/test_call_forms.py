@@ -129,3 +129,26 @@ def test_forward_keeps_non_finite_keys_to_their_rows(Hq, Hkv, D, bs, bad):
             assert hit.any() and not hit.all()
             assert torch.equal(o[~hit], o2[~hit]) and torch.equal(lse[~hit], lse2[~hit]), (kind, key)
     assert nsa.lib().nsa_device_status(None) == 0
+
+
+def test_forward_mode_derivatives_are_refused():
+    """There is no forward-mode derivative of the op: a tangent raises instead of being dropped, also where
+    no input requires a gradient."""
+    import torch.autograd.forward_ad as fwd
+    nsa = pkg()
+    c = dict(B=1, Hq=4, Hkv=2, D=64, T=192, block_size=64, S=2)
+    t = make_inputs(c, torch.bfloat16, seed=1)
+    ins = [dev(t[n], torch.bfloat16) for n in ("q", "kc", "vc", "ks", "vs", "kw", "vw", "gate")]
+    idx = t["block_idx"].cuda()
+    want = nsa.nsa_fused_forward(*ins, idx, 64, 64)
+    assert not want.requires_grad
+    with fwd.dual_level():
+        for at in (0, 3, 7):
+            dual = list(ins)
+            dual[at] = fwd.make_dual(ins[at], torch.ones_like(ins[at]))
+            for call in (lambda: nsa.nsa_fused_forward(*dual, idx, 64, 64), lambda: nsa.nsa_attention(*dual, 64, 2, 64)):
+                with pytest.raises(NotImplementedError):
+                    call()
+                with torch.no_grad(), pytest.raises(NotImplementedError):
+                    call()
+        assert torch.equal(nsa.nsa_fused_forward(*ins, idx, 64, 64), want)
