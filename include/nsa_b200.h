@@ -172,7 +172,8 @@ typedef struct NsaAttentionDesc {
 
 typedef struct NsaAttentionTensors {
   const void *q, *kc, *vc, *ks, *vs, *kw, *vw, *gate;
-  const float* comp[6];               /* K side intra_pos, pool_logits, proj; V side the same */
+  const float* comp[6];               /* K side intra_pos, pool_logits, proj; V side the same.  kc, vc, intra_pos
+                                         and proj start on a 16-byte boundary (else NSA_ERR_BAD_ARG) */
   int32_t* block_idx;
   void* out;
   const void* d_out;                  /* from here on: backward only */

@@ -585,7 +585,7 @@ __global__ void gate_bwd_rows_kernel(const T* __restrict__ oc, const T* __restri
 // rows of whole, aligned 16-byte vectors: the kernels of pool.cu
 inline bool pool_vec_ok(int D, int dtype, const void* a, const void* b) {
   const int per = dtype == NSA_DTYPE_BF16 ? 8 : 4;
-  return D % per == 0 && (((uintptr_t)a | (uintptr_t)b) & 15) == 0;
+  return D % per == 0 && aligned16(a, b);
 }
 
 inline unsigned blocks_for(size_t n, int per) { return (unsigned)((n + per - 1) / per); }
@@ -655,7 +655,7 @@ extern "C" int nsa_block_compress_strided_fwd(const void* x, const float* intra_
   if (ctas == 0) return NSA_OK;
   cudaStream_t st = (cudaStream_t)stream;
   const size_t sm = (size_t)(block_size + D) * sizeof(float);
-  if (pool_learned_ok(D, block_size, dtype)) {
+  if (pool_learned_ok(D, block_size, dtype) && aligned16(x, intra_pos, proj_w, out)) {
     PoolSides p = {};
     p.n = 1; p.x[0] = x; p.intra[0] = intra_pos; p.logits[0] = pool_logits; p.proj[0] = proj_w; p.out[0] = out;
     return pool_learned_fwd(p, B, Hkv, T, D, block_size, stride, st);
@@ -707,7 +707,7 @@ extern "C" int nsa_block_compress_strided_bwd(const void* x, const float* intra_
   float* d_pooled = pooled + rows * D;
   float* sum_dp = d_pooled + rows * D;
   float* d_w = sum_dp + D;
-  if (pool_learned_ok(D, block_size, dtype)) {
+  if (pool_learned_ok(D, block_size, dtype) && aligned16(x, intra_pos, proj_w, d_out, dx, workspace)) {
     PoolSides p = {};
     p.n = 1; p.x[0] = x; p.intra[0] = intra_pos; p.logits[0] = pool_logits; p.proj[0] = proj_w; p.pooled[0] = pooled;
     p.d_out[0] = d_out; p.dx[0] = dx; p.d_pooled[0] = d_pooled; p.acc[0] = sum_dp;

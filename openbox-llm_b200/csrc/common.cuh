@@ -56,6 +56,7 @@ constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;
 
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
+template <typename... P> inline bool aligned16(const P*... p) { return ((... | (uintptr_t)p) & 15) == 0; }
 
 __device__ __forceinline__ float to_float(float x) { return x; }
 __device__ __forceinline__ float to_float(__nv_bfloat16 x) { return __bfloat162float(x); }

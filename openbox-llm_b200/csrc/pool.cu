@@ -496,6 +496,14 @@ __global__ void mean_bwd_kernel(const PoolSides s, int T_, int Dv, int len, int 
   reinterpret_cast<uint4*>(s.dx[blockIdx.y])[i] = Vec<T>::pack(g);
 }
 
+// an argument error where a side's rows or matrices do not start on a 16-byte boundary
+int check_vectors(const PoolSides& s) {
+  for (int k = 0; k < s.n; ++k)
+    NSA_CHECK_ARG(aligned16(s.x[k], s.intra[k], s.proj[k], s.out[k], s.pooled[k], s.d_out[k], s.dx[k], s.d_pooled[k]),
+                  "pooling: K, V and the pooling parameters must start on a 16-byte boundary");
+  return NSA_OK;
+}
+
 template <int D, int R>
 int launch_pool_fwd(const PoolSides& s, int T, int len, int stride, int n_sum, int rows, cudaStream_t st) {
   const size_t smem = (PoolFwdSmem<D, R>::kFloats + 2 * (size_t)len) * sizeof(float);
@@ -529,6 +537,7 @@ bool pool_learned_ok(int D, int len, int dtype) {
 size_t pool_acc_floats(int D, int len) { return ((size_t)D * D + D + len + 1 + 63) / 64 * 64; }
 
 int pool_learned_fwd(const PoolSides& s, int B, int H, int T, int D, int len, int stride, cudaStream_t st) {
+  if (int bad = check_vectors(s)) return bad;
   const int n_sum = pool_count(T, len, stride);
   const size_t rows = (size_t)B * H * n_sum;
   if (rows == 0) return NSA_OK;
@@ -547,6 +556,7 @@ int pool_learned_fwd(const PoolSides& s, int B, int H, int T, int D, int len, in
 }
 
 int pool_learned_bwd(const PoolSides& s, int B, int H, int T, int D, int len, int stride, cudaStream_t st) {
+  if (int bad = check_vectors(s)) return bad;
   const int n_sum = pool_count(T, len, stride);
   const size_t rows = (size_t)B * H * n_sum;
   NSA_CHECK_ARG(rows < (1u << 30), "too many summaries");
@@ -580,6 +590,7 @@ int pool_learned_bwd(const PoolSides& s, int B, int H, int T, int D, int len, in
 }
 
 int pool_mean_fwd(const PoolSides& s, int B, int H, int T, int D, int len, int dtype, cudaStream_t st) {
+  if (int bad = check_vectors(s)) return bad;
   const int n_sum = T / len;
   const size_t rows = (size_t)B * H * n_sum;
   if (rows == 0) return NSA_OK;
@@ -594,6 +605,7 @@ int pool_mean_fwd(const PoolSides& s, int B, int H, int T, int D, int len, int d
 }
 
 int pool_mean_bwd(const PoolSides& s, int B, int H, int T, int D, int len, int dtype, cudaStream_t st) {
+  if (int bad = check_vectors(s)) return bad;
   const int n_sum = T / len;
   const int Dv = dtype == NSA_DTYPE_BF16 ? D / 8 : D / 4;
   const size_t n = (size_t)B * H * T * Dv;

@@ -7,7 +7,9 @@
 namespace nsa {
 
 // One or two tensors pooled with the same geometry (the keys and the values of the compression
-// branch), each with its own parameters.
+// branch), each with its own parameters.  x, dx, out, d_out, pooled, d_pooled, intra and proj are read and
+// written as 16-byte vectors: the calls below refuse other addresses, the entry points that take them
+// go to the scalar kernels of aux.cu instead.
 struct PoolSides {
   int n;                         // 1 or 2
   const void* x[2];              // [B, H, T, D]

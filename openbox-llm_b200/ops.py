@@ -558,6 +558,11 @@ def _op_desc(B, Hq, Hkv, T, D, dtype, block_size, n_sel, window, n_init, n_local
     return (d, *(x.value for x in sizes))
 
 
+def _aligned(t):
+    """t, or a copy of it where it does not start on a 16-byte boundary."""
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
 def _op_forward(q, kv, gate_logits, block_idx, block_size, n_sel, window, forced, comp, need_grad):
     """Forward of the whole op: (out, block_idx, what backward needs).  forced = (n_init, n_local,
     summary length, summary stride); comp: the six compressor parameters, or None for mean pooling."""
@@ -591,6 +596,9 @@ def _op_forward(q, kv, gate_logits, block_idx, block_size, n_sel, window, forced
         with torch.cuda.device(dev):
             return _op_forward(q, kv, gate_logits, block_idx, block_size, n_sel, window, forced, comp, need_grad)
     tensors = [t if t.is_contiguous() else t.contiguous() for t in tensors[:8]]
+    # the pooling reads these as 16-byte vectors; a view may start anywhere
+    tensors[1:3] = map(_aligned, tensors[1:3])
+    cp = [_aligned(t) for t in cp]
     if not given:
         block_idx = torch.empty(B, Hkv, T, n_sel, device=dev, dtype=torch.int32)
     desc, saved_bytes, fwd_bytes, bwd_bytes = _op_desc(
@@ -629,7 +637,7 @@ class _NSAAttention(torch.autograd.Function):
         desc, bwd_bytes, gate_dtype, comp_dtypes = ctx.cfg
         if d_out is None:
             return (None,) * (13 + len(comp_dtypes))
-        kept = ctx.saved_tensors
+        kept = [_aligned(t) for t in ctx.saved_tensors]
         tensors, block_idx, saved, cp = kept[:8], kept[8], kept[9], kept[10:]
         dev = saved.device
         if torch.cuda.current_device() != dev.index:
@@ -638,7 +646,7 @@ class _NSAAttention(torch.autograd.Function):
         if d_out.device != dev:
             raise L.NsaError(f"libnsa_b200: tensors on different devices ({dev} and {d_out.device})")
         assert d_out.dtype == tensors[0].dtype
-        d_out = d_out.contiguous()
+        d_out = _aligned(d_out.contiguous())
         grads = [torch.empty_like(t) for t in tensors]
         d_cp = [torch.empty_like(t) for t in cp]
         ws = L.workspace(bwd_bytes, dev)

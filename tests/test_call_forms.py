@@ -4,9 +4,15 @@ import pytest
 import torch
 
 from oracle import nsa_oracle as O
-from tests.util import cfg_id, dev, make_inputs, pkg
+from tests.util import cfg_id, check, dev, make_inputs, pkg
 
 pytestmark = pytest.mark.gpu
+
+
+def _shifted(t, by=1):
+    """The same values in a contiguous view that starts `by` elements into its buffer."""
+    view = t.new_empty(t.numel() + by)[by:].view(t.shape)
+    return view.copy_(t)
 
 
 def _selection_64(t, idx, bs):
@@ -152,3 +158,71 @@ def test_forward_mode_derivatives_are_refused():
                 with torch.no_grad(), pytest.raises(NotImplementedError):
                     call()
         assert torch.equal(nsa.nsa_fused_forward(*ins, idx, 64, 64), want)
+
+
+@pytest.mark.parametrize("dtype,D,by", [(torch.bfloat16, 64, 1), (torch.bfloat16, 128, 4), (torch.float32, 64, 1),
+                                        (torch.float32, 32, 3), (torch.bfloat16, 16, 3)], ids=str)
+def test_pooled_tensors_and_parameters_may_start_anywhere(dtype, D, by):
+    """kc, vc and the compressor's parameters as contiguous views at any element offset (a slice of a flat
+    buffer): the results are those of aligned tensors."""
+    nsa = pkg()
+    bs = 64
+    c = dict(B=2, Hq=4, Hkv=2, D=D, T=330, block_size=bs, S=2)
+    t = make_inputs(c, dtype, seed=6)
+    ins = [dev(t[n], dtype) for n in ("q", "kc", "vc", "ks", "vs", "kw", "vw", "gate")]
+    do, idx = dev(t["do"], dtype), t["block_idx"].cuda()
+    g = torch.Generator().manual_seed(3)
+    comp = {}
+    for p in ("k", "v"):
+        comp[p + "_intra"] = 0.1 * torch.randn(bs, D, generator=g).cuda()
+        comp[p + "_logits"] = 0.3 * torch.randn(bs, generator=g).cuda()
+        comp[p + "_proj"] = (torch.randn(D, D, generator=g) * D ** -0.5).cuda()
+    moved = [x if i not in (1, 2) else _shifted(x, by) for i, x in enumerate(ins)]
+    moved_comp = {n: _shifted(x, by) for n, x in comp.items()}
+
+    def op(xs, cp, learned):
+        xs = [x.detach().requires_grad_(True) for x in xs]
+        cp = {n: x.detach().requires_grad_(True) for n, x in cp.items()}
+        leaves = xs + (list(cp.values()) if learned else [])
+        with torch.no_grad():
+            bare = (nsa.nsa_attention(*xs, bs, 2, 70, compressor=cp) if learned else
+                    nsa.nsa_fused_forward(*xs, idx, bs, 70))
+        out = (nsa.nsa_attention(*xs, bs, 2, 70, compressor=cp) if learned else
+               nsa.nsa_fused_forward(*xs, idx, bs, 70))
+        assert torch.equal(bare, out)
+        return [out.detach(), *torch.autograd.grad(out, leaves, do if xs[1].data_ptr() % 16 == 0 else _shifted(do, by))]
+
+    for learned in (False, True):
+        want, got = op(ins, comp, learned), op(moved, moved_comp, learned)
+        assert torch.equal(want[0], got[0]), learned
+        for i, (a, b) in enumerate(zip(got[1:], want[1:])):
+            # sums that meet by atomics differ in their order alone: a bf16 step, or 1e-5 for fp32 (d k_intra
+            # is zero but for rounding)
+            bound = (2.0 ** -7 if b.dtype == torch.bfloat16 else 1e-5) * max(b.float().abs().max().item(), 1e-1)
+            assert (a.float() - b.float()).abs().max().item() <= bound, (learned, i)
+
+    # the pooling by itself, forward and backward; the scalar kernels add the window in another order
+    for x, m in zip(ins[1:3], moved[1:3]):
+        check(nsa.block_mean_pool(m, bs), nsa.block_mean_pool(x, bs).float().cpu(), dtype, "mean pool")
+        both = []
+        for y, cp in ((x, comp), (m, moved_comp)):
+            y = y.detach().requires_grad_(True)
+            ps = [cp["k_" + n].detach().requires_grad_(True) for n in ("intra", "logits", "proj")]
+            s = nsa.block_compress(y, *ps, bs)
+            both.append([s.detach(), *torch.autograd.grad(s, [y, *ps], torch.ones_like(s))])
+        for a, b in zip(*both):
+            check(b, a.float().cpu(), b.dtype, "learned pool")
+    assert nsa.lib().nsa_device_status(None) == 0
+
+
+def test_unaligned_rows_are_refused_by_the_c_call():
+    """The C entry point cannot copy: it refuses kc off a 16-byte boundary, before any of its rows is read."""
+    from tests.test_refused_calls import _inputs
+    from tests.test_streams import _forward_call
+    ins = _inputs(1, 8, 2, 512, 64)
+    launch, _ = _forward_call([ins[0], _shifted(ins[1]), *ins[2:]])
+    assert launch(torch.cuda.current_stream().cuda_stream) == -1
+    launch, out = _forward_call(ins)
+    assert launch(torch.cuda.current_stream().cuda_stream) == 0
+    torch.cuda.synchronize()
+    assert torch.isfinite(out).all() and out.abs().sum() > 0
