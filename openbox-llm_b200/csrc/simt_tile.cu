@@ -186,6 +186,29 @@ __device__ __forceinline__ void row_range(const AttnArgs& a, int t, int& lo, int
   else if (a.kind == 1) hi = cmp_visible(t, a.block_size, a.window, a.Lk) - 1;
 }
 
+// Whether a value of the tile that this thread has put into shared memory is infinite or NaN; the loop is load_keys'.
+template <typename T, int D, int kThreads>
+__device__ __forceinline__ bool non_finite(const float* tile) {
+  constexpr int LD = D + kPad, kPer = D / (sizeof(T) == 4 ? 4 : 8), kVec = sizeof(T) == 4 ? 1 : 2;
+  float z = 0.f;                                         // x * 0: 0 or NaN
+#pragma unroll
+  for (int i = threadIdx.x; i < kK * kPer; i += kThreads) {
+#pragma unroll
+    for (int k = 0; k < kVec; ++k) {
+      const float4 v = *reinterpret_cast<const float4*>(tile + (i / kPer) * LD + (i % kPer) * 4 * kVec + 4 * k);
+      z = fmaf(v.x, 0.f, z); z = fmaf(v.y, 0.f, z); z = fmaf(v.z, 0.f, z); z = fmaf(v.w, 0.f, z);
+    }
+  }
+  return z != 0.f;
+}
+
+// What stands for a key that a row does not attend in the tile of P: the sign tells it from a probability of
+// zero.  As a factor it is a zero, as long as the other factor is finite; a tile that holds a value
+// that is not goes through loops that leave these keys out, so that such a value stays with the rows
+// (and keys) that it belongs to.
+constexpr float kMasked = -0.f;
+__device__ __forceinline__ bool attended(float p) { return __float_as_uint(p) != 0x80000000u; }
+
 template <int D> constexpr size_t fwd_floats() { return (size_t)3 * kR * (D + kPad) + (size_t)kR * kPLd; }
 template <int D> constexpr size_t bwd_floats() { return (size_t)4 * kR * (D + kPad) + (size_t)2 * kR * kPLd; }
 
@@ -280,12 +303,12 @@ simt_tile_fwd_kernel(const AttnArgs a) {
     for (int i = 0; i < 8; ++i) {
       const int ql = (row0 + ty + 8 * i) / G - t_first;
       float mx = -INFINITY;
+      bool ok[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        bool ok = tok[j] >= lo[i] && tok[j] <= hi[i];
-        if (a.kind == 2) ok = ok && ((mk[j] >> ql) & 1ull);
-        s[i][j] = ok ? s[i][j] : -INFINITY;
-        mx = fmaxf(mx, s[i][j]);
+        ok[j] = tok[j] >= lo[i] && tok[j] <= hi[i];
+        if (a.kind == 2) ok[j] = ok[j] && ((mk[j] >> ql) & 1ull);
+        mx = fmaxf(mx, ok[j] ? s[i][j] : -INFINITY);
       }
 #pragma unroll
       for (int w = 8; w >= 1; w >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, w));
@@ -298,7 +321,7 @@ simt_tile_fwd_kernel(const AttnArgs a) {
       for (int c = 0; c < C; ++c) o[i][c] *= alpha;
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        const float p = expf(s[i][j] - ms);              // masked: 0
+        const float p = ok[j] ? expf(s[i][j] - m_new) : kMasked;
         l[i] += p;
         sP[(ty + 8 * i) * kPLd + tx + 16 * j] = p;
       }
@@ -308,7 +331,20 @@ simt_tile_fwd_kernel(const AttnArgs a) {
     if (kt + 1 < n_kt) load_keys<T, D, kFwdThreads>(sK, kbase, ki->tok[buf ^ 1]);
     cp_commit();
     cp_wait<1>();
-    __syncthreads();
+    if (__syncthreads_or(non_finite<T, D, kFwdThreads>(sV))) {
+#pragma unroll 1
+      for (int k = 0; k < kK; ++k) {
+        float v[C];
+        load_cols<C>(sV + k * LD, tx, v);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const float p = sP[(ty + 8 * i) * kPLd + k];
+          if (attended(p))
+#pragma unroll
+            for (int c = 0; c < C; ++c) o[i][c] = fmaf(p, v[c], o[i][c]);
+        }
+      }
+    } else
 #pragma unroll 2
     for (int k = 0; k < kK; k += 4) {
       float v[4][C];
@@ -378,12 +414,13 @@ simt_tile_bwd_kernel(const AttnArgs a) {
   float* dvb = a.dv_acc + kvoff;
   if (n_kt > 0) fill_keys(a, tk, sl, ki, 0, 0);
   // Q (scaled), dO (times the gate of a gated branch), lse and delta; four threads per row
+  bool rows_bad;                        // a value of Q or dO is infinite or NaN
   {
     const int r = tid >> 2, part = tid & 3;
     const bool in = row0 + r < n_rows;
     const size_t row = in ? row_ptr(r) : 0;
     const float rs = in && a.row_scale ? a.row_scale[row] : 1.f;
-    float dot = 0.f;
+    float dot = 0.f, z = 0.f;
     for (int c = part * 8; c < D; c += 32) {
       float q[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, g[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
       if (in) {
@@ -391,7 +428,10 @@ simt_tile_bwd_kernel(const AttnArgs a) {
         load8(reinterpret_cast<const T*>(a.d_o) + row * D + c, g);
       }
 #pragma unroll
-      for (int e = 0; e < 8; ++e) { q[e] *= a.scale; g[e] *= rs; }
+      for (int e = 0; e < 8; ++e) {
+        q[e] *= a.scale; g[e] *= rs;
+        z = fmaf(q[e], 0.f, z); z = fmaf(g[e], 0.f, z);
+      }
       if (in && !a.row_dot) {
         float o[8];
         load8(reinterpret_cast<const T*>(a.o) + row * D + c, o);
@@ -407,8 +447,9 @@ simt_tile_bwd_kernel(const AttnArgs a) {
       s_lse[r] = in ? a.lse[row] : 0.f;
       s_delta[r] = in ? (a.row_dot ? rs * a.row_dot[row] : dot) : 0.f;
     }
+    rows_bad = z != 0.f;
   }
-  __syncthreads();
+  rows_bad = __syncthreads_or(rows_bad);
   int lo[4], hi[4];
   float lse[4], delta[4], dq[4][C];
 #pragma unroll
@@ -429,7 +470,7 @@ simt_tile_bwd_kernel(const AttnArgs a) {
   for (int kt = 0; kt < n_kt; ++kt) {
     const int buf = kt & 1;
     cp_wait<0>();
-    __syncthreads();
+    const bool bad = __syncthreads_or(non_finite<T, D, kBwdThreads>(sK) || non_finite<T, D, kBwdThreads>(sV)) || rows_bad;
     float s[4][4], dp[4][4];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
@@ -464,15 +505,29 @@ simt_tile_bwd_kernel(const AttnArgs a) {
       for (int i = 0; i < 4; ++i) {
         bool ok = tok >= lo[i] && tok <= hi[i];
         if (a.kind == 2) ok = ok && ((mk >> ((row0 + ty + 16 * i) / G - t_first)) & 1ull);
-        const float p = ok ? expf(s[i][j] - lse[i]) : 0.f;
+        const float p = ok ? expf(s[i][j] - lse[i]) : kMasked;
         sP[(ty + 16 * i) * kPLd + tx + 16 * j] = p;
-        sDS[(ty + 16 * i) * kPLd + tx + 16 * j] = p * (dp[i][j] - delta[i]);
+        sDS[(ty + 16 * i) * kPLd + tx + 16 * j] = ok ? p * (dp[i][j] - delta[i]) : 0.f;
       }
     }
     if (kt + 1 < n_kt) fill_keys(a, tk, sl, ki, buf ^ 1, kt + 1);
     __syncthreads();
     if (kt + 1 < n_kt) load_keys<T, D, kBwdThreads>(sV, vbase, ki->tok[buf ^ 1]);
     // dQ += dS K
+    if (bad) {
+#pragma unroll 1
+      for (int k = 0; k < kK; ++k) {
+        float v[C];
+        load_cols<C>(sK + k * LD, tx, v);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float ds = sDS[(ty + 16 * i) * kPLd + k];
+          if (attended(sP[(ty + 16 * i) * kPLd + k]))
+#pragma unroll
+            for (int c = 0; c < C; ++c) dq[i][c] = fmaf(ds, v[c], dq[i][c]);
+        }
+      }
+    } else
 #pragma unroll 2
     for (int k = 0; k < kK; k += 4) {
       float v[4][C];
@@ -501,6 +556,20 @@ simt_tile_bwd_kernel(const AttnArgs a) {
       for (int e = 0; e < 4; ++e)
 #pragma unroll
         for (int c = 0; c < C; ++c) acc[e][c] = 0.f;
+      if (bad) {
+#pragma unroll 1
+        for (int r = 0; r < kR; ++r) {
+          float v[C];
+          load_cols<C>(x + r * LD, tx, v);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float we = w[r * kPLd + ty * 4 + e];
+            if (attended(sP[r * kPLd + ty * 4 + e]))
+#pragma unroll
+              for (int c = 0; c < C; ++c) acc[e][c] = fmaf(we, v[c], acc[e][c]);
+          }
+        }
+      } else
 #pragma unroll 4
       for (int r = 0; r < kR; ++r) {
         const float4 p = *reinterpret_cast<const float4*>(w + r * kPLd + ty * 4);

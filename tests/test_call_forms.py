@@ -226,3 +226,53 @@ def test_unaligned_rows_are_refused_by_the_c_call():
     assert launch(torch.cuda.current_stream().cuda_stream) == 0
     torch.cuda.synchronize()
     assert torch.isfinite(out).all() and out.abs().sum() > 0
+
+
+@pytest.mark.parametrize("where", ["k", "v", "q", "do"])
+@pytest.mark.parametrize("dtype,D,bad", [(torch.float32, 64, float("nan")), (torch.float32, 16, float("inf")),
+                                         (torch.float32, 128, float("-inf")), (torch.bfloat16, 32, float("inf"))], ids=str)
+def test_cuda_core_tiles_keep_non_finite_values_to_their_rows(dtype, D, bad, where):
+    """CUDA-core tiles of 64 rows x 64 keys, forward and backward: a value that is infinite or NaN reaches the rows
+    that attend its key (k, v) or its own row (q, dO), and the gradients of the keys those rows
+    attend; everything else is what it is without that value."""
+    nsa = pkg()
+    nsa.set_impl("simt")
+    Hq, Hkv, T, bs, S, W = 4, 2, 200, 16, 4, 40
+    G = Hq // Hkv
+    t = make_inputs(dict(B=1, Hq=Hq, Hkv=Hkv, D=D, T=T, block_size=bs, S=S), dtype, seed=9)
+    q, k, v, do = (dev(t[n], dtype) for n in ("q", "ks", "vs", "do"))
+    idx = t["block_idx"]
+    tt, kk = torch.arange(T)[:, None], torch.arange(T)[None, :]
+    keep = {"window": ((tt >= kk) & (tt - kk < W)).expand(Hkv, T, T),
+            "compression": (tt >= (kk + 1) * 3 - 1).expand(Hkv, T, T),
+            "selection": (idx[0, :, :, None, :] == (kk // bs)[None, :, :, None]).any(-1) & (tt >= kk)}
+
+    def run(kind, q, k, v, do):
+        if kind == "selection":
+            o, lse = nsa.selection_forward_triton(q, k, v, idx.cuda(), bs, return_lse=True)
+            return o, lse, nsa.ops._selection_backward(q, k, v, idx.cuda(), bs, do, o, lse)
+        mode, w = (nsa.MODE_WINDOW, W) if kind == "window" else (nsa.MODE_COMPRESS, 3)
+        o, lse = nsa.range_attn_forward(q, k, v, mode, w, w)
+        return o, lse, nsa.range_attn_backward(q, k, v, o, lse, do, mode, w, w)
+
+    for kind, m in keep.items():
+        o, lse, (dq, dk, dv) = run(kind, q, k, v, do)
+        for at in (2, 61, 130):
+            x = {"q": q, "k": k, "v": v, "do": do}
+            x[where] = x[where].clone()
+            x[where][:, :, at, 3] = bad
+            o2, lse2, (dq2, dk2, dv2) = run(kind, **x)
+            rows = m[:, :, at] if where in "kv" else (torch.arange(T) == at).expand(Hkv, T)      # [Hkv, T]
+            keys = (m & rows[:, :, None]).any(1)
+            if where in "kv":
+                keys[:, at] = True
+            assert not rows.all() and not keys.all()
+            r = rows.repeat_interleave(G, 0)[None].cuda()
+            if where != "do":
+                assert torch.equal(o[~r], o2[~r]) and torch.equal(lse[~r], lse2[~r]), (kind, at)
+            assert torch.equal(dq[~r], dq2[~r]), (kind, at)
+            # the keys' sums meet by atomics, in any order: 1e-5 of the largest, and a bf16 step
+            step = 2.0 ** -7 if dtype == torch.bfloat16 else 0.0
+            for a, b in ((dk, dk2), (dv, dv2)):
+                a, b = a[0][~keys.cuda()].float(), b[0][~keys.cuda()].float()
+                assert ((a - b).abs() <= step * a.abs() + 1e-5 * a.abs().max()).all(), (kind, at)
