@@ -89,6 +89,7 @@ struct SelList {           // selection only, in shared memory
   unsigned long long mask[kMaxBlocks];   // queries of the tile that list a block
   uint16_t list[kMaxBlocks];             // the listed blocks, ascending
   int n_list;
+  int repeats;                           // some query lists a block more than once
 };
 
 // shared memory of one tile's key bookkeeping, double buffered: the next tile is fetched ahead
@@ -109,13 +110,16 @@ __device__ __forceinline__ TileKeys tile_keys(const AttnArgs& a, int bh, int t_f
   } else {
     const int n_blk = (t_last + a.block_size) / a.block_size;   // blocks that start at or before t_last
     for (int i = threadIdx.x; i < n_blk; i += kThreads) sl->mask[i] = 0ull;
+    if (threadIdx.x == 0) sl->repeats = 0;
     __syncthreads();
     const int32_t* idx = a.block_idx + ((size_t)bh * a.T + t_first) * a.S;
     const int n_e = (t_last - t_first + 1) * a.S;
     for (int e = threadIdx.x; e < n_e; e += kThreads) {
       const int ql = e / a.S;
       const int blk = __ldg(idx + e);
-      if (blk >= 0 && (long long)blk * a.block_size <= t_first + ql) atomicOr(&sl->mask[blk], 1ull << ql);
+      if (blk >= 0 && (long long)blk * a.block_size <= t_first + ql &&
+          (atomicOr(&sl->mask[blk], 1ull << ql) >> ql & 1ull))
+        sl->repeats = 1;
     }
     __syncthreads();
     if (threadIdx.x < 32) {
@@ -133,6 +137,17 @@ __device__ __forceinline__ TileKeys tile_keys(const AttnArgs& a, int bh, int t_f
     k.n = sl->n_list * a.block_size;
   }
   return k;
+}
+
+// How often query t lists the block of token tok.  A block listed twice counts twice, as it does in the
+// row kernels, which go through the slots one by one.
+__device__ __forceinline__ int times_listed(const AttnArgs& a, int bh, int t, int tok) {
+  const int32_t* slot = a.block_idx + ((size_t)bh * a.T + t) * a.S;
+  const int blk = tok / a.block_size;
+  int n = 0;
+#pragma unroll 1
+  for (int s = 0; s < a.S; ++s) n += __ldg(slot + s) == blk;
+  return n;
 }
 
 // token and membership of key tile i's keys (threads 0..63)
@@ -238,6 +253,7 @@ simt_tile_fwd_kernel(const AttnArgs a) {
     return ((size_t)b * a.Hq + hkv * G + f % G) * a.T + f / G;
   };
   const TileKeys tk = tile_keys<kFwdThreads>(a, bh, t_first, t_last, sl);
+  const bool repeats = a.kind == 2 && sl->repeats;
   const int n_kt = (tk.n + kK - 1) / kK;
   const T* kbase = reinterpret_cast<const T*>(a.k) + (size_t)bh * a.Lk * D;
   const T* vbase = reinterpret_cast<const T*>(a.v) + (size_t)bh * a.Lk * D;
@@ -326,6 +342,21 @@ simt_tile_fwd_kernel(const AttnArgs a) {
         sP[(ty + 8 * i) * kPLd + tx + 16 * j] = p;
       }
     }
+    if (repeats) {                        // this thread's places once more
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+#pragma unroll 1
+        for (int j = 0; j < 4; ++j) {
+          float* p = sP + (ty + 8 * i) * kPLd + tx + 16 * j;
+          const float one = *p;
+          const int n = attended(one) ? times_listed(a, bh, (row0 + ty + 8 * i) / G, ki->tok[buf][tx + 16 * j]) : 1;
+          if (n > 1) {
+            *p = one * (float)n;
+            l[i] += one * (float)(n - 1);
+          }
+        }
+      }
+    }
     if (kt + 1 < n_kt) fill_keys(a, tk, sl, ki, buf ^ 1, kt + 1);
     __syncthreads();
     if (kt + 1 < n_kt) load_keys<T, D, kFwdThreads>(sK, kbase, ki->tok[buf ^ 1]);
@@ -406,6 +437,7 @@ simt_tile_bwd_kernel(const AttnArgs a) {
     return ((size_t)b * a.Hq + hkv * G + f % G) * a.T + f / G;
   };
   const TileKeys tk = tile_keys<kBwdThreads>(a, bh, t_first, t_last, sl);
+  const bool repeats = a.kind == 2 && sl->repeats;
   const int n_kt = (tk.n + kK - 1) / kK;
   const size_t kvoff = (size_t)bh * a.Lk * D;
   const T* kbase = reinterpret_cast<const T*>(a.k) + kvoff;
@@ -508,6 +540,14 @@ simt_tile_bwd_kernel(const AttnArgs a) {
         const float p = ok ? expf(s[i][j] - lse[i]) : kMasked;
         sP[(ty + 16 * i) * kPLd + tx + 16 * j] = p;
         sDS[(ty + 16 * i) * kPLd + tx + 16 * j] = ok ? p * (dp[i][j] - delta[i]) : 0.f;
+      }
+    }
+    if (repeats) {                        // this thread's places once more
+#pragma unroll 1
+      for (int e = 0; e < 16; ++e) {
+        const int at = (ty + 16 * (e >> 2)) * kPLd + tx + 16 * (e & 3);
+        const int n = attended(sP[at]) ? times_listed(a, bh, (row0 + ty + 16 * (e >> 2)) / G, ki->tok[buf][tx + 16 * (e & 3)]) : 1;
+        if (n > 1) { sP[at] *= (float)n; sDS[at] *= (float)n; }
       }
     }
     if (kt + 1 < n_kt) fill_keys(a, tk, sl, ki, buf ^ 1, kt + 1);

@@ -276,3 +276,36 @@ def test_cuda_core_tiles_keep_non_finite_values_to_their_rows(dtype, D, bad, whe
             for a, b in ((dk, dk2), (dv, dv2)):
                 a, b = a[0][~keys.cuda()].float(), b[0][~keys.cuda()].float()
                 assert ((a - b).abs() <= step * a.abs() + 1e-5 * a.abs().max()).all(), (kind, at)
+
+
+@pytest.mark.parametrize("T", [128, 250, 448, 640], ids=lambda T: f"T{T}")
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16], ids=str)
+def test_repeated_blocks_count_alike_both_ways(dtype, T):
+    """A list that names a block more than once: on the CUDA cores every slot counts, whichever of the row
+    and tile kernels serves a direction (8 to 40 blocks for 4 slots: tiles up to 16 forward and 32 backward)."""
+    nsa = pkg()
+    nsa.set_impl("simt")
+    B, Hq, Hkv, D, bs, S = 1, 6, 2, 32, 16, 4
+    t = make_inputs(dict(B=B, Hq=Hq, Hkv=Hkv, D=D, T=T, block_size=bs, S=S), dtype, seed=2)
+    idx = t["block_idx"].clone()
+    idx[:, :, ::3, 2] = idx[:, :, ::3, 0]
+    idx[:, 1, 5::7, 1:] = idx[:, 1, 5::7, :1]
+    q, k, v, do = (t[n].double() for n in ("q", "ks", "vs", "do"))
+    tt, kk = torch.arange(T)[:, None], torch.arange(T)[None, :]
+    times = ((idx[:, :, :, None, :] == (kk // bs)[None, None, :, :, None]).sum(-1) * (tt >= kk)).repeat_interleave(Hq // Hkv, 1)
+    kx, vx = (x.repeat_interleave(Hq // Hkv, 1) for x in (k, v))
+    s = (q @ kx.transpose(-1, -2) * D ** -0.5).masked_fill(times == 0, float("-inf"))
+    lse = (torch.logsumexp(s + times.double().clamp(min=1).log(), -1))
+    live = torch.isfinite(lse)
+    p = torch.where(times > 0, times * (s - torch.where(live, lse, torch.zeros_like(lse))[..., None]).exp(), torch.zeros_like(s))
+    o = p @ vx
+    ds = p * (do @ vx.transpose(-1, -2) - (do * o).sum(-1, keepdim=True)) * D ** -0.5
+    fold = lambda x: x.view(B, Hkv, -1, T, D).sum(2)
+    want = (ds @ kx, fold(ds.transpose(-1, -2) @ q), fold(p.transpose(-1, -2) @ do))
+    dq_, dk_, dv_ = (dev(t[n], dtype) for n in ("q", "ks", "vs"))
+    got_o, got_lse = nsa.selection_forward_triton(dq_, dk_, dv_, idx.cuda(), bs, return_lse=True)
+    check(got_o, o.float(), dtype, "repeats o")
+    assert (got_lse.cpu()[live].double() - lse[live]).abs().max().item() <= 1e-4
+    grads = nsa.ops._selection_backward(dq_, dk_, dv_, idx.cuda(), bs, dev(t["do"], dtype), got_o, got_lse)
+    for g, w, n in zip(grads, want, ("dq", "dk", "dv")):
+        check(g, w.float(), dtype, f"repeats {n}", abs32=4e-3)
