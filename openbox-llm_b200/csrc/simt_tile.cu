@@ -244,9 +244,9 @@ simt_tile_fwd_kernel(const AttnArgs a) {
   KeyInfo* ki = reinterpret_cast<KeyInfo*>(sP + kR * kPLd);
   SelList* sl = reinterpret_cast<SelList*>(ki + 1);
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  const int bh = blockIdx.y, b = bh / a.Hkv, hkv = bh % a.Hkv, G = a.Hq / a.Hkv;
-  const int row0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * kR;      // long rows first
-  const int n_rows = a.T * G;
+  const int G = a.Hq / a.Hkv, n_rows = a.T * G, tiles = (n_rows + kR - 1) / kR;
+  const int bh = blockIdx.x / tiles, b = bh / a.Hkv, hkv = bh % a.Hkv;
+  const int row0 = (tiles - 1 - (int)blockIdx.x % tiles) * kR;       // long rows first
   const int t_first = row0 / G, t_last = (min(row0 + kR, n_rows) - 1) / G;
   auto row_ptr = [&](int r) -> size_t {                              // row r of the tile in [B, Hq, T]
     const int f = row0 + r;
@@ -428,9 +428,9 @@ simt_tile_bwd_kernel(const AttnArgs a) {
   SelList* sl = reinterpret_cast<SelList*>(ki + 1);
   __shared__ float s_lse[kR], s_delta[kR];
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  const int bh = blockIdx.y, b = bh / a.Hkv, hkv = bh % a.Hkv, G = a.Hq / a.Hkv;
-  const int row0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * kR;
-  const int n_rows = a.T * G;
+  const int G = a.Hq / a.Hkv, n_rows = a.T * G, tiles = (n_rows + kR - 1) / kR;
+  const int bh = blockIdx.x / tiles, b = bh / a.Hkv, hkv = bh % a.Hkv;
+  const int row0 = (tiles - 1 - (int)blockIdx.x % tiles) * kR;
   const int t_first = row0 / G, t_last = (min(row0 + kR, n_rows) - 1) / G;
   auto row_ptr = [&](int r) -> size_t {
     const int f = row0 + r;
@@ -637,12 +637,15 @@ simt_tile_bwd_kernel(const AttnArgs a) {
     }
 }
 
+long long n_tiles(const AttnArgs& a) {
+  return ((long long)a.T * (a.Hq / a.Hkv) + kR - 1) / kR * a.B * a.Hkv;
+}
+
 size_t extra_smem(const AttnArgs& a) { return sizeof(KeyInfo) + (a.kind == 2 ? sizeof(SelList) : 0); }
 
 template <typename T, int D>
 int launch(const AttnArgs& a, bool bwd, cudaStream_t st) {
-  const int G = a.Hq / a.Hkv;
-  const dim3 grid((unsigned)(((long long)a.T * G + kR - 1) / kR), a.B * a.Hkv);
+  const unsigned grid = (unsigned)n_tiles(a);         // in x, which takes any number of units
   if (!bwd) {
     const size_t smem = fwd_floats<D>() * sizeof(float) + extra_smem(a);
     NSA_CUDA_OK(func_smem((const void*)simt_tile_fwd_kernel<T, D>, smem));
@@ -680,7 +683,7 @@ bool simt_tile_ok(const AttnArgs& a, bool bwd) {
   const uintptr_t p = (uintptr_t)a.q | (uintptr_t)a.k | (uintptr_t)a.v | (uintptr_t)a.o | (uintptr_t)a.d_o |
                       (uintptr_t)a.dq | (uintptr_t)a.dk_acc | (uintptr_t)a.dv_acc;
   if (p & 15) return false;
-  if ((long long)a.T * (a.Hq / a.Hkv) >= (1LL << 31) - kR) return false;
+  if ((long long)a.T * (a.Hq / a.Hkv) >= (1LL << 31) - kR || n_tiles(a) >= (1LL << 31)) return false;
   if (a.kind != 2) return true;
   const int n_blk = (a.T + a.block_size - 1) / a.block_size;
   return n_blk <= kMaxBlocks && n_blk <= (bwd ? 8LL : 4LL) * a.S;

@@ -309,3 +309,25 @@ def test_repeated_blocks_count_alike_both_ways(dtype, T):
     grads = nsa.ops._selection_backward(dq_, dk_, dv_, idx.cuda(), bs, dev(t["do"], dtype), got_o, got_lse)
     for g, w, n in zip(grads, want, ("dq", "dk", "dv")):
         check(g, w.float(), dtype, f"repeats {n}", abs32=4e-3)
+
+
+def test_more_units_than_a_grid_dimension_holds():
+    """B x Hkv above 65535 on the CUDA cores, forward and backward: the last units are those of a small call."""
+    nsa = pkg()
+    B, H, T, D, bs, S = 8193, 8, 20, 16, 16, 1
+    g = torch.Generator(device="cuda").manual_seed(5)
+    q, k, v, do = (torch.randn(B, H, T, D, generator=g, device="cuda") for _ in range(4))
+    idx = torch.where(torch.arange(T, device="cuda") >= 15, 0, -1).to(torch.int32)[:, None].expand(B, H, T, S).contiguous()
+
+    def run(sl):
+        a, b, c, d = (x[sl].contiguous() for x in (q, k, v, do))
+        i = idx[sl].contiguous()
+        o, lse = nsa.range_attn_forward(a, b, c, nsa.MODE_WINDOW, 7, 0)
+        out = [o, lse, *nsa.range_attn_backward(a, b, c, o, lse, d, nsa.MODE_WINDOW, 7, 0)]
+        o, lse = nsa.selection_forward_triton(a, b, c, i, bs, return_lse=True)
+        return out + [o, lse, *nsa.ops._selection_backward(a, b, c, i, bs, d, o, lse)]
+
+    assert B * H > 65535
+    for a, b in zip(run(slice(None)), run(slice(B - 2, B))):
+        assert torch.equal(a[B - 2:], b)
+    assert nsa.lib().nsa_device_status(None) == 0
