@@ -544,6 +544,7 @@ def heads_to_tokens(x):
 def nsa_fused_forward(q, kc, vc, ks, vs, kw, vw, gate_logits, block_idx, block_size, window):
     """nsa_fused_kernel.py:560-573: the three branches with a given block_idx, mean pooling."""
     bs = int(block_size)
+    assert q.stride(-1) == 1
     return _op(q, (kc, vc, ks, vs, kw, vw), gate_logits, block_idx, bs, 0, window, (0, 0, bs, bs), None)[0]
 
 
@@ -578,6 +579,8 @@ def _op_forward(q, kv, gate_logits, block_idx, block_size, n_sel, window, forced
     for t in kv:
         assert t.shape == shape and t.dtype == q.dtype
         tensors.append(t)
+    # as _check_qkv: the rows of the attention calls are dense (the pooling takes any kc, vc)
+    assert all(t.stride(-1) == 1 for t in kv[2:])
     gate = gate_logits if gate_logits.dtype == q.dtype else gate_logits.to(q.dtype)
     tensors.append(gate)
     given = block_idx is not None

@@ -331,3 +331,23 @@ def test_more_units_than_a_grid_dimension_holds():
     for a, b in zip(run(slice(None)), run(slice(B - 2, B))):
         assert torch.equal(a[B - 2:], b)
     assert nsa.lib().nsa_device_status(None) == 0
+
+
+def test_attention_rows_have_to_be_dense():
+    """The attention calls ask for stride(-1) == 1, the whole op too: q of the drop-in call, K and V of the
+    selection and window branches.  The pooled pair may be any view."""
+    nsa = pkg()
+    t = make_inputs(dict(B=1, Hq=4, Hkv=2, D=64, T=192, block_size=64, S=2), torch.bfloat16, seed=1)
+    ins = [dev(t[n], torch.bfloat16) for n in ("q", "kc", "vc", "ks", "vs", "kw", "vw", "gate")]
+    idx = t["block_idx"].cuda()
+    want = nsa.nsa_fused_forward(*ins, idx, 64, 64)
+    for i in range(7):
+        xs = list(ins)
+        xs[i] = ins[i].transpose(-1, -2).contiguous().transpose(-1, -2)
+        calls = [lambda: nsa.nsa_fused_forward(*xs, idx, 64, 64), lambda: nsa.nsa_attention(*xs, 64, 2, 64, block_idx=idx)]
+        for call, refused in zip(calls, (i in (0, 3, 4, 5, 6), i >= 3)):
+            if refused:
+                with pytest.raises(AssertionError):
+                    call()
+            else:
+                assert torch.equal(call(), want)
