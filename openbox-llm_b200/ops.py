@@ -574,13 +574,11 @@ def _op_forward(q, kv, gate_logits, block_idx, block_size, n_sel, window, forced
     assert Hq % Hkv == 0, "GQA needs Hq divisible by Hkv"
     assert D in (16, 32, 64, 128), "head dim must be a power of two <= 128"
     assert block_size >= 16, "block_size must be >= 16 (tl.dot inner dim)"
-    shape, dev = (B, Hkv, T, D), q.device
-    tensors = [q]
+    dev = q.device
+    tensors = [q, *kv]
+    assert kv[0].shape == (B, Hkv, T, D)          # and the other five like it (_op)
     for t in kv:
-        assert t.shape == shape and t.dtype == q.dtype
-        tensors.append(t)
-    # as _check_qkv: the rows of the attention calls are dense (the pooling takes any kc, vc)
-    assert all(t.stride(-1) == 1 for t in kv[2:])
+        assert t.dtype == q.dtype
     gate = gate_logits if gate_logits.dtype == q.dtype else gate_logits.to(q.dtype)
     tensors.append(gate)
     given = block_idx is not None
@@ -598,10 +596,15 @@ def _op_forward(q, kv, gate_logits, block_idx, block_size, n_sel, window, forced
     if torch.cuda.current_device() != dev.index:
         with torch.cuda.device(dev):
             return _op_forward(q, kv, gate_logits, block_idx, block_size, n_sel, window, forced, comp, need_grad)
-    tensors = [t if t.is_contiguous() else t.contiguous() for t in tensors[:8]]
+    for i, t in enumerate(tensors[:8]):
+        if not t.is_contiguous():
+            # as _check_qkv: the rows of the attention calls are dense (the pooling takes any kc, vc)
+            assert i not in (3, 4, 5, 6) or t.stride(-1) == 1
+            tensors[i] = t.contiguous()
     # the pooling reads these as 16-byte vectors; a view may start anywhere
     tensors[1:3] = map(_aligned, tensors[1:3])
     cp = [_aligned(t) for t in cp]
+    tensors = tensors[:8]
     if not given:
         block_idx = torch.empty(B, Hkv, T, n_sel, device=dev, dtype=torch.int32)
     desc, saved_bytes, fwd_bytes, bwd_bytes = _op_desc(
@@ -640,7 +643,9 @@ class _NSAAttention(torch.autograd.Function):
         desc, bwd_bytes, gate_dtype, comp_dtypes = ctx.cfg
         if d_out is None:
             return (None,) * (13 + len(comp_dtypes))
-        kept = [_aligned(t) for t in ctx.saved_tensors]
+        kept = ctx.saved_tensors
+        if any(t.data_ptr() % 16 for t in kept):
+            kept = [_aligned(t) for t in kept]
         tensors, block_idx, saved, cp = kept[:8], kept[8], kept[9], kept[10:]
         dev = saved.device
         if torch.cuda.current_device() != dev.index:
@@ -665,10 +670,36 @@ class _NSAAttention(torch.autograd.Function):
         return (*grads, None, None, None, None, None, *d_cp)
 
 
+def _op_in_parts(q, kv, gate_logits, block_idx, block_size, n_sel, window, forced, comp):
+    """The op out of the calls of its parts, for K / V tensors that do not share one shape: a pooled or windowed
+    pair of another length, branches with other numbers of kv heads."""
+    kc, vc, ks, vs, kw, vw = kv
+    n_init, n_local, cl, cs = forced
+    if comp is None:
+        assert cl == cs == block_size, "mean pooling is defined on the aligned grid only"
+        k_cmp, v_cmp = block_mean_pool(kc, block_size), block_mean_pool(vc, block_size)
+    else:
+        k_cmp, v_cmp = (block_compress(x, *comp[3 * i:3 * i + 3], cl, cs) for i, x in enumerate((kc, vc)))
+    o_cmp = compression_attn_triton(q, k_cmp, v_cmp, cl, cs)
+    if block_idx is None:
+        with torch.no_grad():
+            _, lse = range_attn_forward(q, k_cmp, v_cmp, MODE_COMPRESS_STRIDED, cs, cl)
+        block_idx = topn_blocks(q, k_cmp, lse, block_size, n_sel, n_init_blocks=n_init, n_local_blocks=n_local,
+                                cmp_len=cl, cmp_stride=cs)
+    else:
+        block_idx = block_idx.to(torch.int32).contiguous()
+    assert ks.shape[2] == q.shape[2], "selection keys and queries are the same tokens"
+    o_slc = selection_attn_triton(q, ks, vs, block_idx, block_size)
+    return gate_combine(o_cmp, o_slc, window_attn_triton(q, kw, vw, window), gate_logits), block_idx
+
+
 def _op(q, kv, gate_logits, block_idx, block_size, n_sel, window, forced, comp):
     """The whole op: through the autograd node where a gradient is asked for, and inside a forward-mode
     level, where the node refuses a tangent that the bare call would drop.  The bare call spares a short
     forward 9 us of 66 (512 tokens, 16 heads)."""
+    kc, vc, ks, vs, kw, vw = kv
+    if not (kc.shape == vc.shape == ks.shape == vs.shape == kw.shape == vw.shape and kc.shape[2] == q.shape[2]):
+        return _op_in_parts(q, kv, gate_logits, block_idx, block_size, n_sel, window, forced, comp)
     if (torch.is_grad_enabled() and any(t.requires_grad for t in (q, *kv, gate_logits, *(comp or ())))) or (
             getattr(forward_ad, "_current_level", 0) >= 0):
         return _NSAAttention.apply(q, *kv, gate_logits, block_size, n_sel, window, block_idx, forced, *(comp or ()))

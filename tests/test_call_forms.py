@@ -351,3 +351,33 @@ def test_attention_rows_have_to_be_dense():
                     call()
             else:
                 assert torch.equal(call(), want)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16], ids=str)
+def test_branches_of_different_shapes(dtype):
+    """One kv head for the pooled pair, two for the selected one, and a window pair that is longer than q:
+    nsa_fused_forward takes them, forward and backward; with all K / V alike in value it is the plain call."""
+    nsa = pkg()
+    B, Hq, T, D, bs, W = 1, 4, 192, 64, 64, 100
+    t = make_inputs(dict(B=B, Hq=Hq, Hkv=2, D=D, T=T, block_size=bs, S=2), dtype, seed=4)
+    q, kc, vc, ks, vs, kw, vw, gate, do = (dev(t[n], dtype) for n in ("q", "kc", "vc", "ks", "vs", "kw", "vw", "gate", "do"))
+    idx = t["block_idx"].cuda()
+    kc, vc = kc[:, :1].contiguous(), vc[:, :1].contiguous()
+    same = [x.requires_grad_(True) for x in (q, kc.expand(-1, 2, -1, -1).contiguous(), vc.expand(-1, 2, -1, -1).contiguous(),
+                                             ks, vs, kw, vw, gate)]
+    want = nsa.nsa_fused_forward(*same, idx, bs, W)
+    dwant = torch.autograd.grad(want, same, do)
+    longer = [torch.cat([x.detach(), torch.full_like(x[:, :, :64], 3.0)], 2) for x in (kw, vw)]
+    mixed = [x.detach().requires_grad_(True) for x in (q, kc, vc, ks, vs, *longer, gate)]
+    got = nsa.nsa_fused_forward(*mixed, idx, bs, W)
+    dgot = list(torch.autograd.grad(got, mixed, do))
+    check(got, want.detach().float().cpu(), dtype, "mixed shapes out")
+    assert all((d[:, :, T:] == 0).all() for d in dgot[5:7])
+    dgot[5:7] = [d[:, :, :T] for d in dgot[5:7]]
+    for i, (a, b) in enumerate(zip(dgot, dwant)):
+        b = b.float().sum(1, keepdim=True) if i in (1, 2) else b.float()
+        # (dq: three roundings instead of one; d kc, d vc: two heads summed after rounding)
+        assert (a.float() - b).norm() <= (2.0 ** -6 if dtype == torch.bfloat16 else 1e-5) * b.norm(), i
+    out, lists = nsa.nsa_attention(*[x.detach() for x in mixed], bs, 2, W, block_idx=idx, return_block_idx=True)
+    assert torch.equal(out, got) and torch.equal(lists, idx.int())
+    assert nsa.lib().nsa_device_status(None) == 0
