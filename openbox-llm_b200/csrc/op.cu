@@ -71,10 +71,16 @@ class Fork {
     if (!side_) return;
     cudaStreamCaptureStatus mine, theirs;
     unsigned long long my_id = 0, their_id = 0;
-    if (cudaStreamGetCaptureInfo(main, &mine, &my_id) != cudaSuccess) { drop(); return; }
-    for (int k = 0; k < 2; ++k)
-      if (cudaStreamGetCaptureInfo(side_->st[k], &theirs, &their_id) != cudaSuccess ||
-          (theirs != cudaStreamCaptureStatusNone && (mine != theirs || my_id != their_id))) { drop(); return; }
+    if (cudaStreamIsCapturing(main, &mine) != cudaSuccess) { drop(); return; }
+    for (int k = 0; k < 2; ++k) {
+      if (cudaStreamIsCapturing(side_->st[k], &theirs) != cudaSuccess) { drop(); return; }
+      if (theirs == cudaStreamCaptureStatusNone) continue;
+      if (cudaStreamGetCaptureInfo(main, &mine, &my_id) != cudaSuccess ||
+          cudaStreamGetCaptureInfo(side_->st[k], &theirs, &their_id) != cudaSuccess || mine != theirs || my_id != their_id) {
+        drop();
+        return;
+      }
+    }
   }
   ~Fork() {
     if (open_ && rejoin() != cudaSuccess) cudaGetLastError();   // the failure that led here is the one to report

@@ -601,10 +601,13 @@ def _op_forward(q, kv, gate_logits, block_idx, block_size, n_sel, window, forced
             # as _check_qkv: the rows of the attention calls are dense (the pooling takes any kc, vc)
             assert i not in (3, 4, 5, 6) or t.stride(-1) == 1
             tensors[i] = t.contiguous()
-    # the pooling reads these as 16-byte vectors; a view may start anywhere
-    tensors[1:3] = map(_aligned, tensors[1:3])
-    cp = [_aligned(t) for t in cp]
     tensors = tensors[:8]
+    in_ptrs, cp_ptrs = [t.data_ptr() for t in tensors], [t.data_ptr() for t in cp]
+    # the pooling reads these as 16-byte vectors; a view may start anywhere
+    if any(p % 16 for p in (in_ptrs[1], in_ptrs[2], *cp_ptrs)):
+        tensors[1:3] = map(_aligned, tensors[1:3])
+        cp = [_aligned(t) for t in cp]
+        in_ptrs, cp_ptrs = [t.data_ptr() for t in tensors], [t.data_ptr() for t in cp]
     if not given:
         block_idx = torch.empty(B, Hkv, T, n_sel, device=dev, dtype=torch.int32)
     desc, saved_bytes, fwd_bytes, bwd_bytes = _op_desc(
@@ -616,8 +619,7 @@ def _op_forward(q, kv, gate_logits, block_idx, block_size, n_sel, window, forced
     if need_grad and fwd_bytes:
         ws = L.workspace(fwd_bytes, dev)
         ws_ptr = ws.data_ptr()
-    ptrs = L.OP_TENSORS(*[t.data_ptr() for t in tensors], *([t.data_ptr() for t in cp] or (None,) * 6),
-                        block_idx.data_ptr(), out.data_ptr())
+    ptrs = L.OP_TENSORS(*in_ptrs, *(cp_ptrs or (None,) * 6), block_idx.data_ptr(), out.data_ptr())
     L.check(L.lib().nsa_attention_fwd(desc, ptrs, saved.data_ptr(), ws_ptr, fwd_bytes, L.raw_stream(dev)))
     if L.CHECK_STATUS_EVERY_CALL:
         L.check_device_status()
