@@ -383,27 +383,21 @@ __global__ void csr_scan_kernel(const int32_t* __restrict__ counts, int32_t* __r
 __global__ void csr_fill_kernel(const int32_t* __restrict__ idx, const uint32_t* __restrict__ bitmap,
                                 const int32_t* __restrict__ prefix, const int32_t* __restrict__ row_start,
                                 int32_t* __restrict__ q_of_block, int32_t* __restrict__ pair_bh,
-                                int32_t* __restrict__ pair_of_slot, int T_, int S, int bs, int n_blk,
-                                int words, size_t n_entries) {
+                                int T_, int S, int bs, int n_blk, int words, size_t n_entries) {
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n_entries) return;
   const int j = idx[i];
   const int slot = (int)(i % S);
   const int t = (int)((i / S) % T_);
   const size_t bh = i / ((size_t)S * T_);
-  int p = -1;
-  if (j >= 0 && j < n_blk && (long long)j * bs <= t) {
-    bool dup = false;
-    for (int s2 = 0; s2 < slot; ++s2) dup |= idx[i - slot + s2] == j;
-    if (!dup) {
-      const size_t row = bh * n_blk + j;
-      const uint32_t bits = bitmap[row * words + (t >> 5)];
-      p = row_start[row] + prefix[row * words + (t >> 5)] + __popc(bits & ((1u << (t & 31)) - 1u));
-      q_of_block[p] = t;
-      pair_bh[p] = (int)bh;
-    }
-  }
-  if (pair_of_slot) pair_of_slot[i] = p;
+  if (j < 0 || j >= n_blk || (long long)j * bs > t) return;
+  for (int s2 = 0; s2 < slot; ++s2)
+    if (idx[i - slot + s2] == j) return;
+  const size_t row = bh * n_blk + j;
+  const uint32_t bits = bitmap[row * words + (t >> 5)];
+  const int p = row_start[row] + prefix[row * words + (t >> 5)] + __popc(bits & ((1u << (t & 31)) - 1u));
+  q_of_block[p] = t;
+  pair_bh[p] = (int)bh;
 }
 
 // ------------------------------------------------------------------------------------------
@@ -869,12 +863,10 @@ extern "C" size_t nsa_csr_workspace_bytes(int B, int Hkv, int T, int S, int bloc
 }
 
 namespace nsa {
-// CSR over n_blk blocks (the public entry point uses T / block_size, as the reference does;
-// the tcgen05 backward also counts a ragged tail block).  pair_of_slot, when given, receives
-// for every (b, hkv, t, slot) the pair index of that selection or -1.
-int build_csr_internal(const int32_t* block_idx, int B, int Hkv, int T, int S, int block_size,
-                       int n_blk, int32_t* q_of_block, int32_t* block_offsets, int32_t* pair_bh,
-                       int32_t* pair_of_slot, void* workspace, size_t workspace_bytes, cudaStream_t st) {
+// CSR over the T / block_size complete blocks, as the reference builds it
+static int build_csr(const int32_t* block_idx, int B, int Hkv, int T, int S, int block_size, int32_t* q_of_block,
+                     int32_t* block_offsets, int32_t* pair_bh, void* workspace, size_t workspace_bytes, cudaStream_t st) {
+  const int n_blk = T / block_size;
   const size_t rows = (size_t)B * Hkv * n_blk;
   const int words = (T + 31) / 32;
   if ((size_t)B * Hkv == 0) return NSA_OK;
@@ -901,7 +893,7 @@ int build_csr_internal(const int32_t* block_idx, int B, int Hkv, int T, int S, i
   { KernelScope ks("csr_scan_kernel", st); csr_scan_kernel<<<1, 1024, 0, st>>>(counts, block_offsets, row_start, n_blk, rows); }
   if (n_entries) {
     KernelScope ks("csr_fill_kernel", st);
-    csr_fill_kernel<<<blocks_for(n_entries, 256), 256, 0, st>>>(block_idx, bitmap, prefix, row_start, q_of_block, pair_bh, pair_of_slot, T, S, block_size, n_blk, words, n_entries);
+    csr_fill_kernel<<<blocks_for(n_entries, 256), 256, 0, st>>>(block_idx, bitmap, prefix, row_start, q_of_block, pair_bh, T, S, block_size, n_blk, words, n_entries);
   }
   NSA_LAUNCH_OK("csr kernels");
   return NSA_OK;
@@ -913,9 +905,8 @@ extern "C" int nsa_build_block_to_query_csr(const int32_t* block_idx, int B, int
                                             int32_t* block_offsets, int32_t* pair_bh, void* workspace,
                                             size_t workspace_bytes, void* stream) {
   NSA_CHECK_ARG(block_size > 0 && B >= 0 && Hkv >= 0 && T >= 0 && S >= 0, "bad sizes");
-  return build_csr_internal(block_idx, B, Hkv, T, S, block_size, T / block_size, q_of_block,
-                            block_offsets, pair_bh, nullptr, workspace, workspace_bytes,
-                            (cudaStream_t)stream);
+  return build_csr(block_idx, B, Hkv, T, S, block_size, q_of_block, block_offsets, pair_bh, workspace, workspace_bytes,
+                   (cudaStream_t)stream);
 }
 
 // ---- CSR without caller-provided scratch -----------------------------------------------------
@@ -951,9 +942,8 @@ extern "C" int nsa_build_block_to_query_csr_noalloc(const int32_t* block_idx, in
     NSA_CUDA_OK(cudaGetSymbolAddress(&scratch, g_csr_builtin_scratch));
     scratch_of_device[dev].store(scratch, std::memory_order_release);
   }
-  return build_csr_internal(block_idx, B, Hkv, T, S, block_size, T / block_size, q_of_block,
-                            block_offsets, pair_bh, nullptr, scratch,
-                            kCsrBuiltinScratchBytes, (cudaStream_t)stream);
+  return build_csr(block_idx, B, Hkv, T, S, block_size, q_of_block, block_offsets, pair_bh, scratch,
+                   kCsrBuiltinScratchBytes, (cudaStream_t)stream);
 }
 
 extern "C" int nsa_gate_combine_bwd_rows(const void* o_cmp, const void* o_slc, const void* o_win,

@@ -2,8 +2,7 @@
 //
 // One CTA owns a tile of 128 rows = nq consecutive query tokens x the G query heads of one
 // (batch, kv head) group (row r -> token r / G, head r % G), so the heads of a GQA group share
-// every K/V tile; nq = 128 / G, so a group of 3 fills 126 rows (padded to 4, as an earlier version had
-// it, it filled 96).  The CTA walks a list of 64-key tiles:
+// every K/V tile; nq = 128 / G, so a group of 3 fills 126 rows.  The CTA walks a list of 64-key tiles:
 //   window      the tiles covering [t_first - W + 1, t_last]
 //   compression the tiles covering summaries [0, (t_last + 1) / Bsz - 1]
 //   selection   the 64-key tiles holding blocks (of 16, 32 or 64 tokens) listed for the tile's nq

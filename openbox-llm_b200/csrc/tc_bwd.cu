@@ -1388,8 +1388,11 @@ static BwdPlan plan_bwd(const AttnArgs& a) {
   }
   // Fewer key tiles than SMs: a cluster of CTAs shares the row tiles of each and adds its dK / dV through
   // distributed shared memory, as long as a CTA keeps 8 row tiles or so (a CTA costs about as much as
-  // two before its first).  More than that many CTAs gain nothing, and clusters leave SMs of a
-  // GPC over, so big problems do without.  Compression keeps one running sum per key tile: the
+  // two before its first).  The line is 20 CTAs above one per SM: key tiles are unequal (the last ones have
+  // few queries left), so the CTAs over the line start as the short ones end.  At 76 to 84 key tiles
+  // (152 to 168 CTAs in pairs) window and selection take 40 to 61 and 77 to 107 us in pairs, 49 to 66 and 102
+  // to 153 without (D of 64 and 128, groups of 4).  More CTAs than that gain nothing, and clusters
+  // leave SMs of a GPC over, so big problems do without.  Compression keeps one running sum per key tile: the
   // gradient of the key pooling's position parameters is the rounding of that sum (tc.cu), and as it
   // runs beside the other branches where a problem is small, the op at T = 1024 gains nothing from
   // sharing those (277 to 289 us without, 291 with).
