@@ -113,7 +113,7 @@ struct AttnArgs {
 };
 int simt_attn_fwd(const AttnArgs& a, int dtype, cudaStream_t st);
 int simt_attn_bwd(const AttnArgs& a, int dtype, cudaStream_t st);
-bool simt_tile_ok(const AttnArgs& a, bool bwd);                                  // simt_tile.cu
+bool simt_tile_ok(const AttnArgs& a, int dtype, bool bwd);                                  // simt_tile.cu
 int simt_tile_fwd(const AttnArgs& a, int dtype, cudaStream_t st);
 int simt_tile_bwd(const AttnArgs& a, int dtype, cudaStream_t st);
 int cast_f32_to(const float* src, void* dst, size_t n, int dtype, cudaStream_t st);

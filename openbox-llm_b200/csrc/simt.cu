@@ -2,7 +2,7 @@
 // They serve every dtype / head dim / group size / block size the boundary accepts
 // (nsa_selection_kernel.py:187-188).  The tiled kernels of simt_tile.cu take over wherever a tile's
 // rows share enough keys (every window and compression call, selection unless there are many more
-// blocks than list slots), the tcgen05 kernels for the bf16 shapes that fill a tensor-core tile.
+// blocks than list slots or too few tiles for the SMs), the tcgen05 kernels for the bf16 shapes that fill a tensor-core tile.
 //
 // The three branches differ only in which keys a row visits:
 //   window      keys [max(0,t-W+1), t]                         (nsa_fused_kernel.py:588-589)
@@ -261,13 +261,13 @@ int launch_bwd(const AttnArgs& a, cudaStream_t st) {
 
 int simt_attn_fwd(const AttnArgs& a, int dtype, cudaStream_t st) {
   if ((size_t)a.B * a.Hq * a.T == 0) return NSA_OK;
-  if (simt_tile_ok(a, false)) return simt_tile_fwd(a, dtype, st);
+  if (simt_tile_ok(a, dtype, false)) return simt_tile_fwd(a, dtype, st);
   return dtype == NSA_DTYPE_BF16 ? launch_fwd<__nv_bfloat16>(a, st) : launch_fwd<float>(a, st);
 }
 
 int simt_attn_bwd(const AttnArgs& a, int dtype, cudaStream_t st) {
   if ((size_t)a.B * a.Hq * a.T == 0) return NSA_OK;
-  if (simt_tile_ok(a, true)) return simt_tile_bwd(a, dtype, st);
+  if (simt_tile_ok(a, dtype, true)) return simt_tile_bwd(a, dtype, st);
   return dtype == NSA_DTYPE_BF16 ? launch_bwd<__nv_bfloat16>(a, st) : launch_bwd<float>(a, st);
 }
 

@@ -678,15 +678,21 @@ int launch_d(const AttnArgs& a, bool bwd, cudaStream_t st) {
 // average over a causal sequence), where a row at a time goes through its own blocks only.  At 64
 // blocks of 16 tokens, 8 list slots, D = 128 and lists that share little (B=2, T=1024, 16 heads) the
 // forward tile took 0.62 ms against 0.36, the backward tile 0.81 against 0.91: the lines are drawn at 4
-// and 8 blocks per list slot.  Rows must be whole 16-byte vectors.
-bool simt_tile_ok(const AttnArgs& a, bool bwd) {
+// and 8 blocks per list slot.  And a tile is one long chain through its keys, while the row kernels spread
+// its work over 64 warps: with fewer tiles than a GPU holds, the rows end sooner.  At 4 blocks per slot
+// the two take the same time at 1.5 tiles per SM forward and 0.75 backward in bf16, 0.75 and 0.5 in fp32
+// (bf16, 256 tokens, blocks of 16, D = 64: 32 tiles 42 and 70 us, rows 15 and 28; 256 tiles 51 and 118, rows
+// 55 and 115; fp32, 512 tokens, blocks of 32: 384 tiles 110 and 240, rows 214 and 496).
+// Rows must be whole 16-byte vectors.
+bool simt_tile_ok(const AttnArgs& a, int dtype, bool bwd) {
   const uintptr_t p = (uintptr_t)a.q | (uintptr_t)a.k | (uintptr_t)a.v | (uintptr_t)a.o | (uintptr_t)a.d_o |
                       (uintptr_t)a.dq | (uintptr_t)a.dk_acc | (uintptr_t)a.dv_acc;
   if (p & 15) return false;
   if ((long long)a.T * (a.Hq / a.Hkv) >= (1LL << 31) - kR || n_tiles(a) >= (1LL << 31)) return false;
   if (a.kind != 2) return true;
   const int n_blk = (a.T + a.block_size - 1) / a.block_size;
-  return n_blk <= kMaxBlocks && n_blk <= (bwd ? 8LL : 4LL) * a.S;
+  const int quarters = dtype == NSA_DTYPE_BF16 ? (bwd ? 3 : 6) : (bwd ? 2 : 3);      // of the tiles per SM
+  return n_blk <= kMaxBlocks && n_blk <= (bwd ? 8LL : 4LL) * a.S && 4 * n_tiles(a) >= (long long)quarters * sm_count();
 }
 
 int simt_tile_fwd(const AttnArgs& a, int dtype, cudaStream_t st) {

@@ -4,6 +4,7 @@ import pytest
 import torch
 
 from oracle import nsa_oracle as O
+from tests.test_small_blocks_and_tiles import TILES, _branch
 from tests.util import cfg_id, check, dev, make_inputs, pkg
 
 pytestmark = pytest.mark.gpu
@@ -237,11 +238,11 @@ def test_cuda_core_tiles_keep_non_finite_values_to_their_rows(dtype, D, bad, whe
     attend; everything else is what it is without that value."""
     nsa = pkg()
     nsa.set_impl("simt")
-    Hq, Hkv, T, bs, S, W = 4, 2, 200, 16, 4, 40
+    B, Hq, Hkv, T, bs, S, W = 22, 4, 2, 200, 16, 4, 40          # 22 x 14 tiles: two for every SM
     G = Hq // Hkv
-    t = make_inputs(dict(B=1, Hq=Hq, Hkv=Hkv, D=D, T=T, block_size=bs, S=S), dtype, seed=9)
+    t = make_inputs(dict(B=B, Hq=Hq, Hkv=Hkv, D=D, T=T, block_size=bs, S=S), dtype, seed=9)
     q, k, v, do = (dev(t[n], dtype) for n in ("q", "ks", "vs", "do"))
-    idx = t["block_idx"]
+    idx = t["block_idx"][:1].expand(B, -1, -1, -1).contiguous()
     tt, kk = torch.arange(T)[:, None], torch.arange(T)[None, :]
     keep = {"window": ((tt >= kk) & (tt - kk < W)).expand(Hkv, T, T),
             "compression": (tt >= (kk + 1) * 3 - 1).expand(Hkv, T, T),
@@ -267,25 +268,26 @@ def test_cuda_core_tiles_keep_non_finite_values_to_their_rows(dtype, D, bad, whe
             if where in "kv":
                 keys[:, at] = True
             assert not rows.all() and not keys.all()
-            r = rows.repeat_interleave(G, 0)[None].cuda()
+            r, u = ~rows.repeat_interleave(G, 0).cuda(), ~keys.cuda()
             if where != "do":
-                assert torch.equal(o[~r], o2[~r]) and torch.equal(lse[~r], lse2[~r]), (kind, at)
-            assert torch.equal(dq[~r], dq2[~r]), (kind, at)
+                assert torch.equal(o[:, r], o2[:, r]) and torch.equal(lse[:, r], lse2[:, r]), (kind, at)
+            assert torch.equal(dq[:, r], dq2[:, r]), (kind, at)
             # the keys' sums meet by atomics, in any order: 1e-5 of the largest, and a bf16 step
             step = 2.0 ** -7 if dtype == torch.bfloat16 else 0.0
             for a, b in ((dk, dk2), (dv, dv2)):
-                a, b = a[0][~keys.cuda()].float(), b[0][~keys.cuda()].float()
+                a, b = a[:, u].float(), b[:, u].float()
                 assert ((a - b).abs() <= step * a.abs() + 1e-5 * a.abs().max()).all(), (kind, at)
 
 
-@pytest.mark.parametrize("T", [128, 250, 448, 640], ids=lambda T: f"T{T}")
+@pytest.mark.parametrize("B,T", [(1, 128), (28, 128), (14, 250), (8, 448), (6, 640)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16], ids=str)
-def test_repeated_blocks_count_alike_both_ways(dtype, T):
+def test_repeated_blocks_count_alike_both_ways(dtype, B, T):
     """A list that names a block more than once: on the CUDA cores every slot counts, whichever of the row
-    and tile kernels serves a direction (8 to 40 blocks for 4 slots: tiles up to 16 forward and 32 backward)."""
+    and tile kernels serves a direction (8 to 40 blocks for 4 slots: tiles up to 16 forward and 32
+    backward, where there are tiles enough, here 300 and more but for the first)."""
     nsa = pkg()
     nsa.set_impl("simt")
-    B, Hq, Hkv, D, bs, S = 1, 6, 2, 32, 16, 4
+    Hq, Hkv, D, bs, S = 6, 2, 32, 16, 4
     t = make_inputs(dict(B=B, Hq=Hq, Hkv=Hkv, D=D, T=T, block_size=bs, S=S), dtype, seed=2)
     idx = t["block_idx"].clone()
     idx[:, :, ::3, 2] = idx[:, :, ::3, 0]
@@ -311,8 +313,20 @@ def test_repeated_blocks_count_alike_both_ways(dtype, T):
         check(g, w.float(), dtype, f"repeats {n}", abs32=4e-3)
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16], ids=["f32", "bf16"])
+@pytest.mark.parametrize("c", TILES, ids=cfg_id)
+def test_cuda_core_selection_tiles_fill_the_gpu(c, dtype):
+    """The selection tiles serve calls with tiles enough for the SMs: the shapes that end inside a tile, on a batch
+    that has two tiles per SM, against the oracle."""
+    G = c["Hq"] // c["Hkv"]
+    per_batch = (c["T"] * G + 63) // 64 * c["Hkv"]
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    _branch(dict(c, B=(2 * sms + per_batch - 1) // per_batch), dtype, "simt", None, "full tiles")
+
+
 def test_more_units_than_a_grid_dimension_holds():
-    """B x Hkv above 65535 on the CUDA cores, forward and backward: the last units are those of a small call."""
+    """B x Hkv above 65535 on the CUDA cores, forward and backward: the last units are those of a
+    call with 320 units (tiles enough to take the same kernels)."""
     nsa = pkg()
     B, H, T, D, bs, S = 8193, 8, 20, 16, 16, 1
     g = torch.Generator(device="cuda").manual_seed(5)
@@ -328,8 +342,8 @@ def test_more_units_than_a_grid_dimension_holds():
         return out + [o, lse, *nsa.ops._selection_backward(a, b, c, i, bs, d, o, lse)]
 
     assert B * H > 65535
-    for a, b in zip(run(slice(None)), run(slice(B - 2, B))):
-        assert torch.equal(a[B - 2:], b)
+    for a, b in zip(run(slice(None)), run(slice(B - 40, B))):
+        assert torch.equal(a[B - 40:], b)
     assert nsa.lib().nsa_device_status(None) == 0
 
 
