@@ -131,12 +131,11 @@ AttnArgs base_args(const NsaDims* d, int Lk) {
   return a;
 }
 
-// NSA_IMPL_AUTO leaves selection on blocks of 16 and 32 tokens to the CUDA cores, whose probabilities, dS and
-// partial sums are fp32; the tcgen05 kernels keep P, dS and the dQ partials in bf16, which on these
-// blocks a caller asks for with NSA_IMPL_TC.  Against 64-bit arithmetic (T of 130 to 2047, D of 64
-// and 128) o and dq are off by 1.66e-3 and 1.7e-3 here, the rounding of a bf16 result, and by 2.1e-3 to 2.6e-3
-// and 2.6e-3 to 2.9e-3 there.  The price is time: the whole op forward + backward on 16-token blocks,
-// 2 x 1024 tokens, 16 heads of 128, takes 1.30 ms, on the tensor cores 0.30.
+// Selection on blocks of 16 and 32 tokens is fp32 arithmetic under NSA_IMPL_AUTO: through the two-term tcgen05 kernels
+// (use_two_term) where they serve the call, else on the CUDA cores.  NSA_IMPL_TC asks for the plain
+// tcgen05 kernels, which keep P, dS and the dQ partials in bf16: against 64-bit arithmetic (T of 130 to 2047, D of 64
+// and 128) o and dq are off by 2.1e-3 to 2.6e-3 and 2.6e-3 to 2.9e-3 there, by 1.66e-3 and 1.7e-3, the rounding of
+// a bf16 result, otherwise.
 bool use_tc(const NsaDims* d, int block_size, int impl, int* err) {
   *err = NSA_OK;
   if (impl == NSA_IMPL_SIMT || (impl == NSA_IMPL_AUTO && (block_size == 16 || block_size == 32))) return false;
@@ -146,6 +145,15 @@ bool use_tc(const NsaDims* d, int block_size, int impl, int* err) {
     *err = NSA_ERR_UNSUPPORTED;
   }
   return ok;
+}
+
+// Selection on blocks of 16 and 32 tokens through the tcgen05 kernels with P and dS in two bf16 terms (16 significant
+// bits; K, V, Q and dO are bf16 as they are).  The backward keeps fp32 dQ partials of S rows per query: beyond
+// 8 GB of them (half of what the bf16 partials of 64-token blocks take at 8 x 32768 tokens, 16 heads of 128, 16 blocks a
+// list) the CUDA-core kernels, which need none, serve the call.
+bool use_two_term(const NsaDims* d, int block_size, int S, int impl, bool bwd) {
+  if (impl != NSA_IMPL_AUTO || (block_size != 16 && block_size != 32) || S < 1 || !tc_shape_ok(*d, block_size)) return false;
+  return !bwd || (double)d->B * d->Hq * d->T * S * d->D * sizeof(float) <= 8e9;
 }
 
 // backward through the SIMT kernels: dq direct, dk/dv via fp32 accumulators
@@ -442,7 +450,8 @@ static int selection_fwd_impl(const void* q, const void* k, const void* v,
   a.q = q; a.k = k; a.v = v; a.o = o; a.lse = lse; a.block_idx = block_idx;
   a.kind = 2; a.S = S; a.block_size = block_size;
   a.sel_plan = plan;
-  if (use_tc(dims, block_size, impl, &rc) && S > 0)
+  a.two_term = use_two_term(dims, block_size, S, impl, false) && aligned16(q, k, v, o);
+  if (a.two_term || (use_tc(dims, block_size, impl, &rc) && S > 0))
     return tc_sel_fwd(a, workspace, workspace_bytes, (cudaStream_t)stream);
   if (rc != NSA_OK) return rc;
   return simt_attn_fwd(a, dims->dtype, (cudaStream_t)stream);
@@ -473,9 +482,10 @@ extern "C" size_t nsa_selection_bwd_workspace_bytes(const NsaDims* dims, int S, 
   if (check_sel(dims, S, block_size) != NSA_OK) return 0;
   int rc;
   size_t need = simt_bwd_ws(dims, dims->T);
-  if (use_tc(dims, block_size, impl, &rc)) {
+  const bool two_term = use_two_term(dims, block_size, S, impl, true);
+  if (two_term || use_tc(dims, block_size, impl, &rc)) {
     AttnArgs a = base_args(dims, dims->T);
-    a.kind = 2; a.S = S; a.block_size = block_size;
+    a.kind = 2; a.S = S; a.block_size = block_size; a.two_term = two_term;
     need = need > tc_attn_bwd_workspace(a) ? need : tc_attn_bwd_workspace(a);
   }
   return need;
@@ -523,7 +533,9 @@ static int selection_bwd_impl(const void* q, const void* k, const void* v,
   a.block_idx = block_idx; a.kind = 2; a.S = S; a.block_size = block_size;
   a.row_scale = row_scale; a.row_dot = row_dot;
   NSA_CHECK_ARG((row_scale == nullptr) == (row_dot == nullptr), "row_scale and row_dot go together");
-  if (use_tc(dims, block_size, impl, &rc) && S > 0) {
+  a.two_term = dq && use_two_term(dims, block_size, S, impl, true) && aligned16(q, k, v, d_o, dq, dk, dv) &&
+               (row_dot || aligned16(o));
+  if (a.two_term || (use_tc(dims, block_size, impl, &rc) && S > 0)) {
     a.dk_acc = (float*)dk;
     a.dv_acc = (float*)dv;
     a.sel_plan = plan;

@@ -105,6 +105,7 @@ struct AttnArgs {
   const float* row_scale; const float* row_dot;   // backward of a gated branch (may be null)
   float* dq_acc;     // tcgen05 window / compression backward: fp32 accumulator [B*Hkv][T][G][D] that takes dQ (or null)
   const void* sel_plan;   // tcgen05 selection: plan built earlier (tc_sel_plan_build), or null
+  bool two_term;          // tcgen05 selection on 16- and 32-token blocks: P and dS in two bf16 terms, dQ partials in fp32
   bool plan_kept;         // the plan outlives the dQ reduction: the backward need not copy its pair map
   int B, Hq, Hkv, T, Lk, D, S;
   int kind;          // 0 window, 1 compress, 2 selection

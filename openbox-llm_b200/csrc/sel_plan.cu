@@ -42,7 +42,7 @@ plan_count_kernel(const int32_t* __restrict__ block_idx, int32_t* __restrict__ c
                   int nq_union) {
   extern __shared__ uint32_t bm[];
   const int chunk = blockIdx.x, unit = blockIdx.y;
-  if (chunk == 0 && unit == 0 && threadIdx.x == 0) { hdr->union_tiles = 0ull; hdr->pairs = 0ull; }
+  if (chunk == 0 && unit == 0 && threadIdx.x == 0) { hdr->union_tiles = 0ull; hdr->pairs = 0ull; hdr->repeats = 0ull; }
   const int t0 = chunk * cw * 32, n_q = min(T - t0, cw * 32);
   mark_chunk(block_idx + ((size_t)unit * T + t0) * S, bm, t0, n_q, S, block_size, n_kt, cw);
   int uni = 0;
@@ -184,8 +184,8 @@ plan_scan_kernel(int32_t* __restrict__ counts, const int32_t* __restrict__ union
 template <bool kMatch>
 __global__ void __launch_bounds__(kThreads)
 plan_fill_kernel(const int32_t* __restrict__ block_idx, const int32_t* __restrict__ starts,
-                 int32_t* __restrict__ pairs, int32_t* __restrict__ pair_of_slot, int T, int S, int block_size,
-                 int n_kt, int cw, int n_chunks) {
+                 int32_t* __restrict__ pairs, int32_t* __restrict__ pair_of_slot, SelPlanHeader* __restrict__ hdr, int T, int S,
+                 int block_size, int n_kt, int cw, int n_chunks) {
   extern __shared__ uint32_t bm[];
   uint16_t* before = reinterpret_cast<uint16_t*>(bm + n_kt * cw);   // [word][tile]: queries in earlier words
   const int chunk = blockIdx.x, unit = blockIdx.y;
@@ -215,13 +215,17 @@ plan_fill_kernel(const int32_t* __restrict__ block_idx, const int32_t* __restric
     if (kMatch) {
       const uint32_t peers = __match_any_sync(0xffffffffu, j < 0 ? -1 - (int)threadIdx.x : (ql << 16) | j);
       dup = (peers & ((1u << (threadIdx.x & 31)) - 1u)) != 0u;
-      if (block_size < kKeysPerTile) groups = __reduce_or_sync(peers, groups);
+      if (block_size < kKeysPerTile) {
+        groups = __reduce_or_sync(peers, groups);
+        if (j >= 0 && __popc(peers) * __popc(one) != __popc(groups)) hdr->repeats = 1ull;
+      }
     } else if (j >= 0) {
       const int32_t* row = idx + ql * S;
       for (int s = 0; s < S; ++s) {
         const int b2 = __ldg(row + s);
         if (tile_of(b2, t, block_size) != j) continue;
         dup |= s < slot;
+        if (block_size < kKeysPerTile && s < slot && b2 == blk) hdr->repeats = 1ull;
         groups |= one << ((b2 * block_size - j * kKeysPerTile) >> 4);
       }
     }
@@ -294,10 +298,10 @@ int sel_plan_build(const int32_t* block_idx, void* base, const SelPlanLayout& l,
     plan_scan_kernel<<<units, kScanThreads, 0, st>>>(counts, unions, p, T, S, l.n_ktiles, l.n_chunks, nq); }
   { KernelScope ks("plan_fill_kernel", st);
     if (match)
-      plan_fill_kernel<true><<<grid, kThreads, smem + smem / 2, st>>>(block_idx, counts, p.pairs, p.pair_of_slot, T, S,
+      plan_fill_kernel<true><<<grid, kThreads, smem + smem / 2, st>>>(block_idx, counts, p.pairs, p.pair_of_slot, p.hdr, T, S,
                                                                       block_size, l.n_ktiles, l.chunk_words, l.n_chunks);
     else
-      plan_fill_kernel<false><<<grid, kThreads, smem + smem / 2, st>>>(block_idx, counts, p.pairs, p.pair_of_slot, T, S,
+      plan_fill_kernel<false><<<grid, kThreads, smem + smem / 2, st>>>(block_idx, counts, p.pairs, p.pair_of_slot, p.hdr, T, S,
                                                                        block_size, l.n_ktiles, l.chunk_words, l.n_chunks); }
   NSA_LAUNCH_OK("selection plan kernels");
   return NSA_OK;

@@ -25,7 +25,8 @@ constexpr int kSelChunkTiles = 128;
 struct SelPlanHeader {
   unsigned long long union_tiles;   // distinct (query tile, key tile) pairs of the query-outer kernel
   unsigned long long pairs;         // pairs over all units
-  unsigned long long pad[30];
+  unsigned long long repeats;       // not 0: some query names a block of 16 or 32 tokens more than once
+  unsigned long long pad[29];
 };
 
 // device pointers into a plan buffer

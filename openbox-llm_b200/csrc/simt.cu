@@ -262,12 +262,14 @@ int launch_bwd(const AttnArgs& a, cudaStream_t st) {
 int simt_attn_fwd(const AttnArgs& a, int dtype, cudaStream_t st) {
   if ((size_t)a.B * a.Hq * a.T == 0) return NSA_OK;
   if (simt_tile_ok(a, dtype, false)) return simt_tile_fwd(a, dtype, st);
+  NSA_CHECK_ARG(aligned16(a.k), "k has to start on a 16-byte boundary");              // read as 16-byte vectors
   return dtype == NSA_DTYPE_BF16 ? launch_fwd<__nv_bfloat16>(a, st) : launch_fwd<float>(a, st);
 }
 
 int simt_attn_bwd(const AttnArgs& a, int dtype, cudaStream_t st) {
   if ((size_t)a.B * a.Hq * a.T == 0) return NSA_OK;
   if (simt_tile_ok(a, dtype, true)) return simt_tile_bwd(a, dtype, st);
+  NSA_CHECK_ARG(aligned16(a.k, a.v), "k and v have to start on a 16-byte boundary");
   return dtype == NSA_DTYPE_BF16 ? launch_bwd<__nv_bfloat16>(a, st) : launch_bwd<float>(a, st);
 }
 

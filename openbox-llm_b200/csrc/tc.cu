@@ -16,6 +16,7 @@
 // accumulator in TMEM is rescaled rarely.
 #include <algorithm>
 
+#include "sel_row.cuh"
 #include "tc_common.cuh"
 #include "tc_host.cuh"
 
@@ -37,6 +38,9 @@ struct FwdArgs {
   int nw;                    // 32-bit membership words per block = ceil(nq / 32)
   int n_sub;                 // selection: list blocks per 64-key tile (64 / block_size)
   float scale_log2;
+  const __nv_bfloat16* q;    // two-term selection: the rows that are done again one by one
+  const __nv_bfloat16* k;
+  const __nv_bfloat16* v;
   float neg_zero;            // -0: what a product is added to where it has to be rounded by itself (a packed mul
                              //     and the add after it are merged into one fma, whatever their rounding says)
 };
@@ -104,7 +108,12 @@ __device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) {
 // gradient of the key pooling's position parameters is what rounding leaves of that sum, 3e-4 of the
 // other gradients.  Any other rounding here, or order of the sum in backward, is as exact and replaces
 // these values by others of their size.)
-template <int D, int kKind>
+//
+// kTwoTerm (selection on 16- and 32-token blocks, whose results are fp32 arithmetic rounded once): P goes to the
+// tensor cores as two bf16 terms, P - bf16(P) behind bf16(P), 16 significant bits in the 64 columns that S leaves
+// behind, at the price of a second product.  A block listed twice counts twice; a row whose result is not finite
+// (V of a key it does not attend may be infinite: zero times that is NaN) is done again by itself.
+template <int D, int kKind, bool kTwoTerm>
 __global__ void __launch_bounds__(kFwdThreads, 2)
 tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
               const __grid_constant__ CUtensorMap tm_v, const FwdArgs p) {
@@ -138,6 +147,7 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   uint32_t* s_tmem = (uint32_t*)(bars + L::kBars);
   volatile int* s_abort = (volatile int*)(s_tmem + 1);
   int* s_ntiles = (int*)(s_tmem + 2);
+  int* s_repeats = (int*)(s_tmem + 3);              // two-term: a query of the row tile lists a block more than once
   int* s_scan = (int*)(s_tmem + 4);                 // [129]
   uint32_t* s_member = (uint32_t*)(s_scan + 132);   // [nb_sel][n_sub][nw]   (selection only)
   const int tile_words = p.n_sub * p.nw;
@@ -196,6 +206,7 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     const int bh = w % units, t0 = (p.n_qtiles - 1 - w / units) * p.nq, t_last = min(p.T - 1, t0 + p.nq - 1);
     const int n_vis = t_last / kKeys + 1;              // key tiles that start at or before the last query
     for (int i = tid; i < n_vis * tile_words; i += kFwdThreads) s_member[i] = 0u;
+    if (kTwoTerm && tid == 0) *s_repeats = 0;
     __syncthreads();
     const int32_t* idx = p.block_idx + ((size_t)bh * p.T + t0) * p.S;
     const int n_entries = (t_last - t0 + 1) * p.S;
@@ -203,8 +214,10 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       const int q_local = e / p.S;
       const int blk = __ldg(idx + e);
       // list block blk = part blk % n_sub of key tile blk / n_sub
-      if (blk >= 0 && (long long)blk * p.block_size <= t0 + q_local)
-        atomicOr(&s_member[blk * p.nw + (q_local >> 5)], 1u << (q_local & 31));
+      if (blk >= 0 && (long long)blk * p.block_size <= t0 + q_local) {
+        const uint32_t was = atomicOr(&s_member[blk * p.nw + (q_local >> 5)], 1u << (q_local & 31));
+        if (kTwoTerm && (was >> (q_local & 31) & 1u)) *s_repeats = 1;
+      }
     }
     __syncthreads();
     const int per = (n_vis + 127) / 128;               // the first 128 threads scan `per` tiles each
@@ -326,6 +339,10 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
 #pragma unroll
             for (int kk = 0; kk < kKeys / 16; ++kk)
               mma_ts(tmem + kColO, tmem + kColS + (c & 1) * kKeys + kk * 8, desc_at(va, kk * 2048), kIdescPV, (i > 0) || (kk > 0));
+            if (kTwoTerm)
+#pragma unroll
+              for (int kk = 0; kk < kKeys / 16; ++kk)
+                mma_ts(tmem + kColO, tmem + kColS + (c & 1) * kKeys + 32 + kk * 8, desc_at(va, kk * 2048), kIdescPV, 1);
             tc_commit(bar_o + (c & 1));
             tc_commit(v_free + st);
           }
@@ -351,6 +368,8 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           continue;
         }
         float m_used = -INFINITY, l_sum = 0.f;      // log2 units
+        bool listed = false;                        // two-term: the row attends a key
+        const bool repeats = kTwoTerm && *s_repeats;
         for (int i = 0; i < x.n_tiles; ++i, ++c) {
           const int key0 = key0_of(x, i);
           // valid columns of this row in this tile: one range [lo, hi] and, for selection, 16-column groups
@@ -391,6 +410,7 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           // whole tile or none of it needs no work per element (none: its P is set to zero below); only
           // rows whose range ends inside the tile, or that attend some 16-column groups of it, do.
           const bool none = hi < 0;
+          if (kTwoTerm) listed |= !none && groups != 0u;
           if (!(lo <= 0 && (hi >= kKeys - 1 || none) && (!kSel || groups == 0xfu))) {
 #pragma unroll
             for (int cc = 0; cc < 64; ++cc)
@@ -413,6 +433,12 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           const uint64_t nz2 = pack_f32x2(p.neg_zero, p.neg_zero);
           const uint64_t sc2 = pack_f32x2(p.scale_log2, p.scale_log2), mn2 = pack_f32x2(-msub, -msub);
           float psum = 0.f;
+          float times[4] = {1.f, 1.f, 1.f, 1.f};     // how often the row's list names the block of a 16-column group
+          if (kTwoTerm && repeats && !none) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+              times[k] = (float)times_listed(p.block_idx + ((size_t)x.bh * p.T + t) * p.S, p.S, (key0 + 16 * k) / p.block_size);
+          }
 #pragma unroll
           for (int cc = 0; cc < 32; ++cc) {
             float p0, p1;
@@ -420,13 +446,23 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
                                    mn2), p0, p1);
             p0 = ex2(p0);
             p1 = ex2(p1);
+            if (kTwoTerm && repeats) {
+              const float n = times[cc >> 3];
+              p0 *= n;
+              p1 *= n;
+            }
             psum += p0 + p1;
             pk[cc] = pack_bf16(p0, p1);
+            if (kTwoTerm)
+              r[cc] = pack_bf16(p0 - __uint_as_float(pk[cc] << 16), p1 - __uint_as_float(pk[cc] & 0xffff0000u));
           }
           if (none) {
             psum = 0.f;
 #pragma unroll
             for (int cc = 0; cc < 32; ++cc) pk[cc] = 0u;
+            if (kTwoTerm)
+#pragma unroll
+              for (int cc = 0; cc < 32; ++cc) r[cc] = 0u;
           }
           l_sum += psum;
           // O may be touched once PV of the tile before is done; only a warp that has to rescale waits
@@ -445,6 +481,7 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
             }
           }
           tmem_st32(s_base, pk);                   // over the S columns this thread has just read
+          if (kTwoTerm) tmem_st32(s_base + 32, r);
           tmem_wait_st();
           tc_fence_before();
           mbar_arrive(bar_p + (c & 1));
@@ -455,11 +492,15 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         if (!__all_sync(0xffffffffu, ok)) break;
         tc_fence_after();
         const float inv = l_sum > 0.f ? 1.f / l_sum : 0.f;
+        float nan_sum = 0.f;                         // x * 0: 0 or NaN
 #pragma unroll
         for (int cc = 0; cc < D / 32; ++cc) {
           uint32_t o32[32];
           tmem_ld32(lane_base + kColO + cc * 32, o32);
           tmem_wait_ld();
+          if (kTwoTerm)
+#pragma unroll
+            for (int e = 0; e < 32; ++e) nan_sum = fmaf(__uint_as_float(o32[e]), 0.f, nan_sum);
           if (row_ok) {
             uint4* dst = reinterpret_cast<uint4*>(orow + cc * 32);
 #pragma unroll
@@ -474,6 +515,10 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           }
         }
         if (row_ok) *lrow = l_sum > 0.f ? (m_used + log2f(l_sum)) * kLn2 : kLseEmpty;
+        if (kTwoTerm && row_ok && listed && !(nan_sum == 0.f && l_sum > 0.f && l_sum < INFINITY))
+          sel_row_forward<D>(p.q + ((size_t)(b * p.Hq + head) * p.T + t) * D, p.k + (size_t)x.bh * p.Lk * D,
+                             p.v + (size_t)x.bh * p.Lk * D, p.block_idx + ((size_t)x.bh * p.T + t) * p.S, p.S, p.block_size,
+                             t, p.scale_log2, orow, lrow);
         tc_fence_before();     // the O columns are read: the next row tile's first PV (behind this thread's next P) may overwrite them
       }
     }
@@ -544,6 +589,7 @@ static int launch_fwd(const AttnArgs& a, const SelPlanHeader* plan, int force, c
   p.n_sub = a.kind == 2 ? kKeys / a.block_size : 1;
   p.scale_log2 = a.scale * kLog2e;
   p.neg_zero = -0.f;
+  p.q = (const __nv_bfloat16*)a.q; p.k = (const __nv_bfloat16*)a.k; p.v = (const __nv_bfloat16*)a.v;
   CUtensorMap tm_q, tm_k, tm_v;
   int rc = make_map_query_rows(&tm_q, a.q, a.D, a.T, a.B * a.Hq, p.G, p.nq);
   if (rc == NSA_OK) rc = make_map(&tm_k, a.k, a.D, a.Lk, a.B * a.Hkv, kKeys, 1);
@@ -561,10 +607,12 @@ static int launch_fwd(const AttnArgs& a, const SelPlanHeader* plan, int force, c
     kernel<<<grid, kFwdThreads, smem, st>>>(tm_q, tm_k, tm_v, p);
     return NSA_OK;
   };
-  if (a.D == 128)
-    rc = a.kind == 2 ? go(tc_fwd_kernel<128, 2>) : a.kind == 1 ? go(tc_fwd_kernel<128, 1>) : go(tc_fwd_kernel<128, 0>);
+  if (a.two_term)
+    rc = a.D == 128 ? go(tc_fwd_kernel<128, 2, true>) : go(tc_fwd_kernel<64, 2, true>);
+  else if (a.D == 128)
+    rc = a.kind == 2 ? go(tc_fwd_kernel<128, 2, false>) : a.kind == 1 ? go(tc_fwd_kernel<128, 1, false>) : go(tc_fwd_kernel<128, 0, false>);
   else
-    rc = a.kind == 2 ? go(tc_fwd_kernel<64, 2>) : a.kind == 1 ? go(tc_fwd_kernel<64, 1>) : go(tc_fwd_kernel<64, 0>);
+    rc = a.kind == 2 ? go(tc_fwd_kernel<64, 2, false>) : a.kind == 1 ? go(tc_fwd_kernel<64, 1, false>) : go(tc_fwd_kernel<64, 0, false>);
   if (rc != NSA_OK) return rc;
   NSA_LAUNCH_OK("tc_fwd_kernel");
   return NSA_OK;

@@ -26,6 +26,9 @@
 //                accumulator [units][T][G][D] by TMA reduce-add.  Consecutive key tiles hit the same
 //                consecutive query rows at nearby times, so the adds meet in L2 and no partial
 //                buffer exists; the order of the adds, hence the last bits of dq, is not fixed.
+#include <type_traits>
+
+#include "sel_row.cuh"
 #include "tc_common.cuh"
 #include "tc_host.cuh"
 
@@ -34,21 +37,24 @@ namespace tc {
 
 struct BwdArgs {
   const __nv_bfloat16* q;
+  const __nv_bfloat16* k;
+  const __nv_bfloat16* v;
   const __nv_bfloat16* d_o;
+  const int32_t* block_idx;    // two-term selection
   const float* lse;
   const float* delta;          // sum_d dO * O per row (unscaled)
   const float* row_scale;      // gate value per row of a gated branch, or null
   SelPlan plan;                // selection
   __nv_bfloat16* dk;
   __nv_bfloat16* dv;
-  __nv_bfloat16* dq_part;
+  void* dq_part;               // bf16, fp32 for two-term selection
   float* dk_acc;               // fp32 accumulators, used when the row tiles of a key tile are split
   float* dv_acc;
   int* status;
   int split_chunk;             // row tiles per CTA when split
   int csize;                   // CTAs per cluster
   int B, Hq, Hkv, T, Lk, G, nq;
-  int kind, window, block_size;
+  int kind, window, block_size, S;
   int n_ktiles, n_slots;
   int merged;                  // selection: one TMA box per (query, tensor) brings both 64-column slabs
   int dq_acc_mode;             // 1: dQ tiles are added to the fp32 accumulator (window / compression)
@@ -484,7 +490,7 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
           if (prow != 0xffffffffu) {
             const uint4 v = *reinterpret_cast<const uint4*>(sP + (c >> 3) * (kRows * 128) + r * 128 +
                                                             (((c & 7) ^ (r & 7)) << 4));
-            *reinterpret_cast<uint4*>(p.dq_part + (size_t)prow * D + c * 8) = v;
+            *reinterpret_cast<uint4*>((__nv_bfloat16*)p.dq_part + (size_t)prow * D + c * 8) = v;
           }
         }
       }
@@ -578,24 +584,96 @@ __device__ __forceinline__ float4 ld_peer_f32x4(const float* p, int rank) {
   return v;
 }
 
-template <int D> struct Bwd2 {
+//
+// kTwoTerm: selection on 16- and 32-token blocks, whose results are fp32 arithmetic rounded once.  P and dS go to
+// the tensor cores as two bf16 terms each (16 significant bits; the second adds three products of eight), the dQ
+// partials stay fp32, a block listed twice counts twice and what comes out non-finite is done again row by
+// row (sel_row.cuh).  P and dS take 64 KB of a slot, as much as its fp32 staging tile, so one slot fits at D = 128 and
+// two at D = 64.  The whole op on 16-token blocks, forward + backward (2 x 1024 tokens, 16 heads of 128, 8 blocks a
+// list): selection backward 157 us against 795 for the CUDA-core tiles, forward 37 against 367, the pass 356 against 1299.
+template <int D, bool kTwoTerm> struct Bwd2 {
   static constexpr int kSlabs = D / 64;
-  static constexpr int kSlots = D == 64 ? 3 : 2;
+  static constexpr int kTerms = kTwoTerm ? 2 : 1;
+  static constexpr int kSlots = (D == 64 ? 3 : 2) - (kTwoTerm ? 1 : 0);
   static constexpr int kKVBytes = kKeys * 128 * kSlabs;
   static constexpr int kRowBytes = kRows * 128 * kSlabs;            // Q or dO
-  static constexpr int kSlotBytes = 2 * kRowBytes + 2 * kPBytes;    // dO, Q, P, dS
+  static constexpr int kSlotBytes = 2 * kRowBytes + 2 * kTerms * kPBytes;    // dO, Q, P, dS (and P, dS: second terms)
   static constexpr int kBars = 2 + 7 * kSlots;
   static constexpr size_t kSmem = 2 * kKVBytes + (size_t)kSlots * kSlotBytes + 256 /*barriers*/ +
                                   (size_t)kSlots * 128 * 4 /*partial rows of a ragged tile*/ + 1024 /*alignment slack*/;
 };
 
-template <int D, bool kCluster>
+// dK and dV of one work item in scalar fp32, a warp to a row, into acc [dV, dK][64 keys][D] in shared memory, for
+// a tile whose sums are not finite (two-term selection).
+template <int D>
+__device__ __noinline__ void sel_tile_dkdv(const BwdArgs& p, float* acc, int bh, int j, int pair_first, int n_rows,
+                                           int n_threads) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int b = bh / p.Hkv, hkv = bh % p.Hkv, key0 = j * kKeys;
+  for (int i = threadIdx.x; i < 2 * kKeys * D; i += n_threads) acc[i] = 0.f;
+  __syncthreads();
+  for (int r = warp; r < n_rows; r += n_threads / 32) {
+    const int pair = __ldg(p.plan.pairs + pair_first + r / p.G);
+    const int t = pair & (int)kPairPosMask;
+    const size_t row = ((size_t)b * p.Hq + hkv * p.G + r % p.G) * p.T + t;
+    const float gate = p.row_scale ? p.row_scale[row] : 1.f;
+    const float lse2 = p.lse[row] * kLog2e - __log2f(gate), delta = p.delta[row];
+    float q[D / 32], g[D / 32];
+    for (int e = 0; e < D / 32; ++e) {
+      q[e] = to_float(p.q[row * D + lane + 32 * e]);
+      g[e] = to_float(p.d_o[row * D + lane + 32 * e]);
+    }
+    const int32_t* list = p.block_idx + ((size_t)bh * p.T + t) * p.S;
+    for (int c = 0; c < kKeys && key0 + c <= t; ++c) {
+      if (!(((uint32_t)pair >> (kPairPosBits + (c >> 4))) & 1u)) continue;
+      const size_t key = ((size_t)bh * p.Lk + key0 + c) * D;
+      float x = 0.f, y = 0.f;
+      for (int e = 0; e < D / 32; ++e) {
+        x = fmaf(q[e], to_float(p.k[key + lane + 32 * e]), x);
+        y = fmaf(g[e], to_float(p.v[key + lane + 32 * e]), y);
+      }
+      x = warp_sum(x);
+      y = warp_sum(y);
+      const float pr = (float)times_listed(list, p.S, (key0 + c) / p.block_size) * exp2f(fmaf(x, p.scale_log2, -lse2));
+      const float ds = pr * (y - delta) * p.scale;
+      for (int e = 0; e < D / 32; ++e) {
+        atomicAdd(acc + c * D + lane + 32 * e, pr * g[e]);
+        atomicAdd(acc + (kKeys + c) * D + lane + 32 * e, ds * q[e]);
+      }
+    }
+  }
+  __syncthreads();
+}
+
+// 32 columns of a row's dQ against one key tile in scalar fp32 (two-term selection, result not finite).
+template <int D>
+__device__ __noinline__ void sel_row_dq(const BwdArgs& p, float* acc, int bh, int head, int pair, int key0, int col0) {
+  const int t = pair & (int)kPairPosMask;
+  const size_t row = ((size_t)(bh / p.Hkv) * p.Hq + head) * p.T + t;
+  const float gate = p.row_scale ? p.row_scale[row] : 1.f;
+  const float lse2 = p.lse[row] * kLog2e - __log2f(gate), delta = p.delta[row];
+  const int32_t* list = p.block_idx + ((size_t)bh * p.T + t) * p.S;
+#pragma unroll 1
+  for (int e = 0; e < 32; ++e) acc[e] = 0.f;
+#pragma unroll 1
+  for (int c = 0; c < kKeys && key0 + c <= t; ++c) {
+    if (!(((uint32_t)pair >> (kPairPosBits + (c >> 4))) & 1u)) continue;
+    const size_t key = ((size_t)bh * p.Lk + key0 + c) * D;
+    const float x = dot_rows<D>(p.q + row * D, p.k + key), y = dot_rows<D>(p.d_o + row * D, p.v + key);
+    const float pr = (float)times_listed(list, p.S, (key0 + c) / p.block_size) * exp2f(fmaf(x, p.scale_log2, -lse2));
+    const float ds = pr * (y - delta) * p.scale;
+#pragma unroll 1
+    for (int e = 0; e < 32; ++e) acc[e] = fmaf(ds, to_float(p.k[key + col0 + e]), acc[e]);
+  }
+}
+
+template <int D, bool kCluster, bool kTwoTerm>
 __global__ void __launch_bounds__(kB2Threads, 1)
 tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
                const __grid_constant__ CUtensorMap tm_q_run, const __grid_constant__ CUtensorMap tm_do_run,
-               const __grid_constant__ CUtensorMap tm_dq, const BwdArgs p) {
-  using L = Bwd2<D>;
+               const __grid_constant__ CUtensorMap tm_dq, const __grid_constant__ BwdArgs p) {
+  using L = Bwd2<D, kTwoTerm>;
   constexpr int kSlabs = L::kSlabs, kSlots = L::kSlots, kKVBytes = L::kKVBytes;
   constexpr uint32_t kTmemCols = 512;
   // slot s: S at 128 s, dP at 128 s + 64, dQ over both; then dV^T and dK^T: at D = 128 64 columns each, at D = 64
@@ -857,30 +935,35 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
             tc_fence_after();
             const uint8_t* sDO = sSlot + sbb * L::kSlotBytes;
             const uint8_t* sP = sDO + 2 * L::kRowBytes;
-            const uint8_t* sDS = sP + kPBytes;
+            const uint8_t* sDS = sP + kPBytes;       // (two-term: P, dS, then their second terms)
             const uint32_t dsk = desc_lo_kmajor(smem_u32(sDS));
-            if (D == 64) {
-              // A: the dO and Q tiles as two 64-column slabs, B: the P and dS tiles likewise
-              const uint32_t da = desc_lo_mnmajor(smem_u32(sDO), L::kRowBytes);
-              const uint32_t pa = desc_lo_mnmajor(smem_u32(sP), kPBytes);
 #pragma unroll
-              for (int kk = 0; kk < kRows / 16; ++kk)        // contraction over the 128 rows, 16 a step
-                mma_ss(tmem + kColDV, desc_at(da, kk * 2048), desc_at(pa, kk * 2048), kIdescT, 1);
-            } else {
-              const uint32_t da = desc_lo_mnmajor(smem_u32(sDO), q_slab);
-              const uint32_t qa = desc_lo_mnmajor(smem_u32(sDO + L::kRowBytes), q_slab);
-              const uint32_t pa = desc_lo_mnmajor(smem_u32(sP), 0), dsa = desc_lo_mnmajor(smem_u32(sDS), 0);
+            for (uint32_t term = 0; term < L::kTerms * 2 * kPBytes; term += 2 * kPBytes) {
+              if (D == 64) {
+                // A: the dO and Q tiles as two 64-column slabs, B: the P and dS tiles likewise
+                const uint32_t da = desc_lo_mnmajor(smem_u32(sDO), L::kRowBytes);
+                const uint32_t pa = desc_lo_mnmajor(smem_u32(sP), kPBytes);
 #pragma unroll
-              for (int kk = 0; kk < kRows / 16; ++kk)
-                mma_ss(tmem + kColDV, desc_at_sbo(da, kk * 2 * q_sbo, q_sbo), desc_at(pa, kk * 2048), kIdescT, 1);
+                for (int kk = 0; kk < kRows / 16; ++kk)        // contraction over the 128 rows, 16 a step
+                  mma_ss(tmem + kColDV, desc_at(da, kk * 2048), desc_at(pa, term + kk * 2048), kIdescT, 1);
+              } else {
+                const uint32_t da = desc_lo_mnmajor(smem_u32(sDO), q_slab);
+                const uint32_t qa = desc_lo_mnmajor(smem_u32(sDO + L::kRowBytes), q_slab);
+                const uint32_t pa = desc_lo_mnmajor(smem_u32(sP), 0), dsa = desc_lo_mnmajor(smem_u32(sDS), 0);
 #pragma unroll
-              for (int kk = 0; kk < kRows / 16; ++kk)
-                mma_ss(tmem + kColDK, desc_at_sbo(qa, kk * 2 * q_sbo, q_sbo), desc_at(dsa, kk * 2048), kIdescT, 1);
+                for (int kk = 0; kk < kRows / 16; ++kk)
+                  mma_ss(tmem + kColDV, desc_at_sbo(da, kk * 2 * q_sbo, q_sbo), desc_at(pa, term + kk * 2048), kIdescT, 1);
+#pragma unroll
+                for (int kk = 0; kk < kRows / 16; ++kk)
+                  mma_ss(tmem + kColDK, desc_at_sbo(qa, kk * 2 * q_sbo, q_sbo), desc_at(dsa, term + kk * 2048), kIdescT, 1);
+              }
             }
             tc_commit(qdo_free + sbb);
 #pragma unroll
-            for (int kk = 0; kk < kKeys / 16; ++kk)        // contraction over the 64 keys
-              mma_ss(tmem + sbb * 128, desc_at(dsk, kk * 32), desc_at(kb, kk * 2048), kIdescDQ, kk > 0);
+            for (uint32_t term = 0; term < L::kTerms * 2 * kPBytes; term += 2 * kPBytes)
+#pragma unroll
+              for (int kk = 0; kk < kKeys / 16; ++kk)        // contraction over the 64 keys
+                mma_ss(tmem + sbb * 128, desc_at(dsk, term + kk * 32), desc_at(kb, kk * 2048), kIdescDQ, term > 0 || kk > 0);
             tc_commit(acc_full + sbb);
             ++next_b;
             if (++sbb == kSlots) { sbb = 0; ++ub; }
@@ -916,21 +999,26 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
       return t_lo + qi;
     };
     auto row_index = [&](int t) -> size_t { return (size_t)(b * p.Hq + head) * p.T + (t & (int)kPairPosMask); };
-    int t_cur = grp < n_tiles ? row_query(grp) : -1;
-    int t_nxt = grp + 2 < n_tiles ? row_query(grp + 2) : -1;
+    // With one slot one group does every tile: a group that skipped the other's use of the slot would wait for
+    // a phase two ahead, which a parity does not tell from the one before.
+    constexpr int kGroups = kSlots == 1 ? 1 : 2;
+    const int k_end = grp < kGroups ? n_tiles : 0;
+    int t_cur = grp < k_end ? row_query(grp) : -1;
+    int t_nxt = grp + kGroups < k_end ? row_query(grp + kGroups) : -1;
     float lse_cur = 0.f, delta_cur = 0.f, gate_cur = 1.f;
     if (t_cur >= 0) {
       lse_cur = __ldg(p.lse + row_index(t_cur));
       delta_cur = __ldg(p.delta + row_index(t_cur));
       if (p.row_scale) gate_cur = __ldg(p.row_scale + row_index(t_cur));
     }
+    const bool repeats = kTwoTerm && __ldg(&p.plan.hdr->repeats) != 0ull;
     // A given-up wait does not part a group: its warps go on to the barrier below, which decides for all.
-    for (int k = grp; k < n_tiles; k += 2) {
+    for (int k = grp; k < k_end; k += kGroups) {
       const int sb = k % kSlots, u = k / kSlots;
       uint8_t* sP = sSlot + sb * L::kSlotBytes + 2 * L::kRowBytes;
       uint8_t* sDS = sP + kPBytes;
       const uint32_t lane_base = tmem + ((uint32_t)(quad * 32) << 16) + sb * 128;
-      const int t_nn = (k + 4 < n_tiles) ? row_query(k + 4) : -1;
+      const int t_nn = (k + 2 * kGroups < k_end) ? row_query(k + 2 * kGroups) : -1;
       float lse_nxt = 0.f, delta_nxt = 0.f, gate_nxt = 1.f;
       if (t_nxt >= 0) {
         lse_nxt = ldg_f32_now(p.lse + row_index(t_nxt));
@@ -955,13 +1043,19 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
       const float lse2 = lse_cur * kLog2e - __log2f(gate_cur);
       const float dscale = p.scale, ddelta = delta_cur * p.scale;
       // every column of this thread's half is attended (the usual case away from the diagonal)?
-      const bool all_cols = lo <= half * 32 && hi >= half * 32 + 31 && groups == 0x3u;
+      const bool all_cols = lo <= half * 32 && hi >= half * 32 + 31 && groups == 0x3u && !repeats;
+      float times[2] = {1.f, 1.f};                   // how often the row's list names the blocks of its column groups
+      if (kTwoTerm && repeats && t_cur >= 0) {
+        const int32_t* list = p.block_idx + ((size_t)bh * p.T + (t_cur & (int)kPairPosMask)) * p.S;
+#pragma unroll
+        for (int e = 0; e < 2; ++e) times[e] = (float)times_listed(list, p.S, (key0 + half * 32 + 16 * e) / p.block_size);
+      }
       mbar_wait(sp_full + sb, u & 1, p.status, s_abort, 64);
       // the P / dS tiles double as the dQ staging tile: the store of the slot's last tile has read it
       // (the thread that stored says so, below)
       if (lt == 0 && k > grp) {
         bulk_wait_read();
-        mbar_arrive(stage_free + (k - 2) % kSlots);
+        mbar_arrive(stage_free + (k - kGroups) % kSlots);
       }
       if (u > 0) mbar_wait(stage_free + sb, (u - 1) & 1, p.status, s_abort, 64);
       __syncwarp();
@@ -972,14 +1066,22 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
         tmem_ld32(lane_base + 64 + half * 32, rp);
         tmem_wait_ld();
         uint32_t pp[16], pd[16];
+        uint32_t pp2[kTwoTerm ? 16 : 1], pd2[kTwoTerm ? 16 : 1];   // second terms
+        auto put = [&](int c2, float p0, float p1, float d0, float d1) {
+          pp[c2] = pack_bf16(p0, p1);
+          pd[c2] = pack_bf16(d0, d1);
+          if (kTwoTerm) {
+            pp2[c2] = pack_bf16(p0 - __uint_as_float(pp[c2] << 16), p1 - __uint_as_float(pp[c2] & 0xffff0000u));
+            pd2[c2] = pack_bf16(d0 - __uint_as_float(pd[c2] << 16), d1 - __uint_as_float(pd[c2] & 0xffff0000u));
+          }
+        };
         if (__all_sync(0xffffffffu, all_cols)) {
 #pragma unroll
           for (int c2 = 0; c2 < 16; ++c2) {
             const float p0 = ex2(fmaf(__uint_as_float(rs[c2 * 2]), p.scale_log2, -lse2));
             const float p1 = ex2(fmaf(__uint_as_float(rs[c2 * 2 + 1]), p.scale_log2, -lse2));
-            pp[c2] = pack_bf16(p0, p1);
-            pd[c2] = pack_bf16(p0 * fmaf(__uint_as_float(rp[c2 * 2]), dscale, -ddelta),
-                               p1 * fmaf(__uint_as_float(rp[c2 * 2 + 1]), dscale, -ddelta));
+            put(c2, p0, p1, p0 * fmaf(__uint_as_float(rp[c2 * 2]), dscale, -ddelta),
+                p1 * fmaf(__uint_as_float(rp[c2 * 2 + 1]), dscale, -ddelta));
           }
         } else {
 #pragma unroll
@@ -989,12 +1091,13 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
             for (int e = 0; e < 2; ++e) {
               const int c = half * 32 + c2 * 2 + e;
               const bool in = (c >= lo) && (c <= hi) && ((groups >> (c2 >> 3)) & 1u);
-              const float pr = in ? ex2(fmaf(__uint_as_float(rs[c2 * 2 + e]), p.scale_log2, -lse2)) : 0.f;
+              float pr = in ? ex2(fmaf(__uint_as_float(rs[c2 * 2 + e]), p.scale_log2, -lse2)) : 0.f;
+              if (kTwoTerm) pr *= times[c2 >> 3];
               pv[e] = pr;
               dv[e] = pr * fmaf(__uint_as_float(rp[c2 * 2 + e]), dscale, -ddelta);
+              if (kTwoTerm && !in) dv[e] = 0.f;      // (dP of a key that is not attended may be infinite)
             }
-            pp[c2] = pack_bf16(pv[0], pv[1]);
-            pd[c2] = pack_bf16(dv[0], dv[1]);
+            put(c2, pv[0], pv[1], dv[0], dv[1]);
           }
         }
         const uint32_t p_row = smem_u32(sP) + row * 128, ds_row = smem_u32(sDS) + row * 128;
@@ -1003,6 +1106,10 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
           const uint32_t chunk16 = (uint32_t)((half * 4 + k4) ^ (row & 7)) << 4;
           st_shared_v4(p_row + chunk16, pp[k4 * 4], pp[k4 * 4 + 1], pp[k4 * 4 + 2], pp[k4 * 4 + 3]);
           st_shared_v4(ds_row + chunk16, pd[k4 * 4], pd[k4 * 4 + 1], pd[k4 * 4 + 2], pd[k4 * 4 + 3]);
+          if (kTwoTerm) {
+            st_shared_v4(p_row + 2 * kPBytes + chunk16, pp2[k4 * 4], pp2[k4 * 4 + 1], pp2[k4 * 4 + 2], pp2[k4 * 4 + 3]);
+            st_shared_v4(ds_row + 2 * kPBytes + chunk16, pd2[k4 * 4], pd2[k4 * 4 + 1], pd2[k4 * 4 + 2], pd2[k4 * 4 + 3]);
+          }
         }
       }
       fence_proxy_async();
@@ -1024,6 +1131,24 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
         if (cc == D / 64 - 1) {            // dQ is in registers: S / dP of the slot's next tile may land
           tc_fence_before();
           mbar_arrive(dq_read + sb);
+        }
+        if (kTwoTerm) {                    // fp32 staging: slabs of 128 rows x 32 columns
+          float z = 0.f;                   // x * 0: 0 or NaN
+#pragma unroll
+          for (int e = 0; e < 32; ++e) z = fmaf(__uint_as_float(r32[e]), 0.f, z);
+          if (t_cur >= 0 && z != 0.f) {
+            float again[32];
+            sel_row_dq<D>(p, again, bh, head, t_cur, key0, col0);
+#pragma unroll
+            for (int e = 0; e < 32; ++e) r32[e] = __float_as_uint(again[e]);
+          }
+          __syncwarp();
+          const uint32_t rbase = smem_u32(stage) + (col0 >> 5) * (kRows * 128) + row * 128;
+#pragma unroll
+          for (int c = 0; c < 8; ++c)
+            st_shared_v4(rbase + (((uint32_t)c ^ (uint32_t)(row & 7)) << 4), r32[c * 4], r32[c * 4 + 1], r32[c * 4 + 2],
+                         r32[c * 4 + 3]);
+          continue;
         }
 #pragma unroll
         for (int v4 = 0; v4 < 4; ++v4) {
@@ -1058,13 +1183,14 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
           const int slot = p.kind == 2 ? 0 : (p.kind == 0 ? j % p.n_slots : j);
           const int mid = p.kind == 2 ? pair_base + i * p.nq : t_lo + i * p.nq;
           const int outer = p.kind == 2 ? 0 : bh;
+          constexpr int kParts = kTwoTerm ? D / 32 : kSlabs;
 #pragma unroll
-          for (int sl = 0; sl < kSlabs; ++sl)
-            tma_store_5d_hint(&tm_dq, stage + sl * (kRows * 128), sl * 64, 0, slot, mid, outer, l2_policy_evict_first());
+          for (int sl = 0; sl < kParts; ++sl)
+            tma_store_5d_hint(&tm_dq, stage + sl * (kRows * 128), sl * (D / kParts), 0, slot, mid, outer, l2_policy_evict_first());
           bulk_commit();
         }
       } else {   // the ragged last tile: whole rows out by hand, 16 bytes a lane
-        constexpr int kChunks = D / 8;
+        constexpr int kChunks = kTwoTerm ? D / 4 : D / 8;
         constexpr int kRowsPerPass = 256 / kChunks;
         const int c = lt % kChunks;
         for (int r = lt / kChunks; r < kRows; r += kRowsPerPass) {
@@ -1072,7 +1198,7 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
           if (prow != 0xffffffffu) {
             const uint4 v = *reinterpret_cast<const uint4*>(stage + (c >> 3) * (kRows * 128) + r * 128 +
                                                             (((c & 7) ^ (r & 7)) << 4));
-            *reinterpret_cast<uint4*>(p.dq_part + (size_t)prow * D + c * 8) = v;
+            *reinterpret_cast<uint4*>((char*)p.dq_part + ((size_t)prow * kChunks + c) * 16) = v;
           }
         }
       }
@@ -1084,8 +1210,39 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
   // ---- dK^T, dV^T: lane = d, column = key; compute group 0 writes dV, group 1 writes dK ----------
   __syncthreads();           // the MMA thread has seen the tensor pipe drain (bar_drain)
   tc_fence_after();
+  bool redone = false;
   float* s_acc = reinterpret_cast<float*>(sSlot);      // cluster: [dV, dK][64 keys][D], over the slots
-  if (warp < kB2Compute && ((warp >> 2) & 1) == 0 && !*s_abort) {
+  if (kTwoTerm) {
+    // sums that are not finite are formed again, leaving out what a row does not attend
+    float z = 0.f;
+    if (warp < kB2Compute && ((warp >> 2) & 1) == 0 && !*s_abort) {
+      const uint32_t lb = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+      const bool mine = D == 128 || ((warp & 3) >> 1) == (warp >> 3);
+      uint32_t r32[32];
+#pragma unroll
+      for (int hc = 0; hc < 2; ++hc) {
+        tmem_ld32(lb + (warp >> 3 ? kColDK : kColDV) + hc * 32, r32);
+        tmem_wait_ld();
+#pragma unroll
+        for (int c = 0; c < 32; ++c)
+          if (mine) z = fmaf(__uint_as_float(r32[c]), 0.f, z);
+      }
+    }
+    if (__syncthreads_or(z != 0.f)) {
+      const int first = rt_begin * p.nq, rows = max(0, min(n_tiles * p.nq, n_q - first)) * p.G;
+      sel_tile_dkdv<D>(p, s_acc, bh, j, pair_base + first, rows, kB2Threads);
+      if (!kCluster && !*s_abort)
+        for (int i = tid; i < 2 * kKeys * D; i += kB2Threads) {
+          const int which = i / (kKeys * D), key = key0 + (i / D) % kKeys;
+          if (key >= p.Lk) continue;
+          const size_t o = ((size_t)bh * p.Lk + key) * D + i % D;
+          if (split) atomicAdd((which == 0 ? p.dv_acc : p.dk_acc) + o, s_acc[i]);
+          else (which == 0 ? p.dv : p.dk)[o] = __float2bfloat16_rn(s_acc[i]);
+        }
+      redone = true;
+    }
+  }
+  if (!redone && warp < kB2Compute && ((warp >> 2) & 1) == 0 && !*s_abort) {
     const int grp = warp >> 3, quad = warp & 3;
     // D = 64: dV^T sits in lanes 0-63, dK^T in lanes 64-127
     const bool mine = D == 128 || (quad >> 1) == grp;
@@ -1163,8 +1320,8 @@ __global__ void delta_kernel(const __nv_bfloat16* __restrict__ d_o, const __nv_b
 }
 
 // dq[b, hkv*G+g, t, :] = sum over the partial slots of query (bh, t); one thread per 8 elements
-template <int D>
-__global__ void dq_reduce_kernel(const __nv_bfloat16* __restrict__ part, const int32_t* __restrict__ pair_of_slot,
+template <int D, bool kF32>
+__global__ void dq_reduce_kernel(const void* __restrict__ part, const int32_t* __restrict__ pair_of_slot,
                                  __nv_bfloat16* __restrict__ dq, int B, int Hq, int Hkv, int T, int G,
                                  int kind, int window, int block_size, int Lk, int n_slots, int S) {
   constexpr int kVec = D / 8;
@@ -1179,7 +1336,14 @@ __global__ void dq_reduce_kernel(const __nv_bfloat16* __restrict__ part, const i
 #pragma unroll
   for (int e = 0; e < 8; ++e) acc[e] = 0.f;
   auto add = [&](size_t row_index) {
-    const uint4 u = __ldg(reinterpret_cast<const uint4*>(part + (row_index * G + g) * D + v * 8));
+    if (kF32) {
+      const float4* src = reinterpret_cast<const float4*>((const float*)part + (row_index * G + g) * D + v * 8);
+      const float4 a = __ldcs(src), b = __ldcs(src + 1);
+      acc[0] += a.x; acc[1] += a.y; acc[2] += a.z; acc[3] += a.w;
+      acc[4] += b.x; acc[5] += b.y; acc[6] += b.z; acc[7] += b.w;
+      return;
+    }
+    const uint4 u = __ldg(reinterpret_cast<const uint4*>((const __nv_bfloat16*)part + (row_index * G + g) * D + v * 8));
     const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
@@ -1214,7 +1378,7 @@ __global__ void dq_reduce_kernel(const __nv_bfloat16* __restrict__ part, const i
 // of query (bh, t) are added in fp32 and rounded once.  A branch whose buffer is null is absent.
 struct Reduce3Args {
   const __nv_bfloat16* part_cmp; int slots_cmp, Lk_cmp, cmp_len, cmp_stride;
-  const __nv_bfloat16* part_slc; const int32_t* pair_of_slot; int S;
+  const void* part_slc; const int32_t* pair_of_slot; int S;     // fp32 where the kernel is kF32
   const __nv_bfloat16* part_win; int slots_win, window;
   const float* acc;            // fp32 accumulator [units][T][G][D] holding the window + compression part, or null
   __nv_bfloat16* dq;
@@ -1225,7 +1389,7 @@ struct Reduce3Args {
 // query share the partial rows, so their index loads and address arithmetic are paid once.  The
 // kernel moves 32 GB at the benchmark shape and was held back by its instruction count, not by
 // memory, when every thread served a single head.
-template <int D, int HG>
+template <int D, int HG, bool kF32>
 __global__ void dq_reduce3_kernel(const Reduce3Args a) {
   constexpr int kVec = D / 8;
   const int Gp = a.G / HG;                               // head groups per query
@@ -1289,7 +1453,33 @@ __global__ void dq_reduce3_kernel(const Reduce3Args a) {
       long long rows[kTripSel];
 #pragma unroll
       for (int k = 0; k < kTripSel; ++k) rows[k] = s0 + k < a.S ? (long long)__ldg(ps + s0 + k) : -1;
-      add_rows(a.part_slc, rows);
+      if (!kF32) {
+        add_rows((const __nv_bfloat16*)a.part_slc, rows);
+        continue;
+      }
+#pragma unroll
+      for (int k0 = 0; k0 < kTripSel; k0 += 4) {       // fp32 rows are twice as wide: half a trip at a time
+        float4 f[4][HG][2];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const long long row = rows[k0 + k];
+          const float* src = (const float*)a.part_slc + (size_t)(row >= 0 ? row : 0) * row_elems + in_row;
+#pragma unroll
+          for (int h = 0; h < HG; ++h)
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+              f[k][h][e] = row >= 0 ? __ldcs(reinterpret_cast<const float4*>(src + h * head_step) + e) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+#pragma unroll
+          for (int h = 0; h < HG; ++h)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              acc[h][4 * e] += f[k][h][e].x; acc[h][4 * e + 1] += f[k][h][e].y;
+              acc[h][4 * e + 2] += f[k][h][e].z; acc[h][4 * e + 3] += f[k][h][e].w;
+            }
+      }
     }
   }
   if (a.part_win) {
@@ -1380,7 +1570,7 @@ static BwdPlan plan_bwd(const AttnArgs& a) {
   }
   size_t off = 0;
   pl.off_delta = off; off += align_up((size_t)a.B * a.Hq * a.T * sizeof(float), 256);
-  pl.off_part = off; off += align_up(part_rows * G * a.D * 2, 256);
+  pl.off_part = off; off += align_up(part_rows * G * a.D * (a.two_term ? 4 : 2), 256);
   pl.off_plan = off;
   if (a.kind == 2) {
     pl.layout = sel_plan_layout((int)units, a.T, a.S, pl.nq);
@@ -1436,13 +1626,17 @@ int tc_attn_bwd(const AttnArgs& a, void* ws, size_t ws_bytes, cudaStream_t st) {
   const int G = a.Hq / a.Hkv;
   BwdArgs p;
   p.q = (const __nv_bfloat16*)a.q;
+  p.k = (const __nv_bfloat16*)a.k;
+  p.v = (const __nv_bfloat16*)a.v;
+  p.block_idx = a.block_idx;
+  p.S = a.S;
   p.d_o = (const __nv_bfloat16*)a.d_o;
   p.lse = a.lse;
   p.delta = a.row_dot ? a.row_dot : (float*)(base + pl.off_delta);
   p.row_scale = a.row_scale;
   p.dk = (__nv_bfloat16*)a.dk_acc;     // the API passes the dk / dv outputs through these fields
   p.dv = (__nv_bfloat16*)a.dv_acc;
-  p.dq_part = (__nv_bfloat16*)(base + pl.off_part);
+  p.dq_part = base + pl.off_part;
   p.plan = SelPlan{};
   p.status = device_status_ptr();
   if (!p.status) { set_error("device status word unavailable"); return NSA_ERR_CUDA; }
@@ -1498,7 +1692,7 @@ int tc_attn_bwd(const AttnArgs& a, void* ws, size_t ws_bytes, cudaStream_t st) {
     rc = make_map_dq_acc(&tm_dqacc, a.dq_acc, a.D, G, (size_t)a.T, (size_t)a.B * a.Hkv, pl.nq);
     tm_dq = tm_dqacc;        // the partial-tile map is not used in this mode
   } else if (rc == NSA_OK) {
-    rc = a.kind == 2 ? make_map_partial(&tm_dq, p.dq_part, a.D, G, 1, pl.cap_pairs ? pl.cap_pairs : 1, 1, pl.nq)
+    rc = a.kind == 2 ? make_map_partial(&tm_dq, p.dq_part, a.D, G, 1, pl.cap_pairs ? pl.cap_pairs : 1, 1, pl.nq, a.two_term)
                      : make_map_partial(&tm_dq, p.dq_part, a.D, G, pl.n_slots, a.T, (size_t)a.B * a.Hkv, pl.nq);
     tm_dqacc = tm_dq;        // likewise
   }
@@ -1514,7 +1708,8 @@ int tc_attn_bwd(const AttnArgs& a, void* ws, size_t ws_bytes, cudaStream_t st) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(kB2Threads);
-    cfg.dynamicSmemBytes = a.D == 128 ? Bwd2<128>::kSmem : Bwd2<64>::kSmem;
+    cfg.dynamicSmemBytes = a.two_term ? (a.D == 128 ? Bwd2<128, true>::kSmem : Bwd2<64, true>::kSmem)
+                                      : (a.D == 128 ? Bwd2<128, false>::kSmem : Bwd2<64, false>::kSmem);
     cfg.stream = st;
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeClusterDimension;
@@ -1527,8 +1722,14 @@ int tc_attn_bwd(const AttnArgs& a, void* ws, size_t ws_bytes, cudaStream_t st) {
       NSA_CUDA_OK(cudaLaunchKernelEx(&cfg, kernel, tm_k, tm_v, tm_q, tm_do, tm_q_run, tm_do_run, tm_dq, p));
       return NSA_OK;
     };
-    if (a.D == 128) rc = pl.csize > 1 ? go(tc_bwd2_kernel<128, true>) : go(tc_bwd2_kernel<128, false>);
-    else rc = pl.csize > 1 ? go(tc_bwd2_kernel<64, true>) : go(tc_bwd2_kernel<64, false>);
+    if (a.two_term) {
+      if (a.D == 128) rc = pl.csize > 1 ? go(tc_bwd2_kernel<128, true, true>) : go(tc_bwd2_kernel<128, false, true>);
+      else rc = pl.csize > 1 ? go(tc_bwd2_kernel<64, true, true>) : go(tc_bwd2_kernel<64, false, true>);
+    } else if (a.D == 128) {
+      rc = pl.csize > 1 ? go(tc_bwd2_kernel<128, true, false>) : go(tc_bwd2_kernel<128, false, false>);
+    } else {
+      rc = pl.csize > 1 ? go(tc_bwd2_kernel<64, true, false>) : go(tc_bwd2_kernel<64, false, false>);
+    }
     if (rc != NSA_OK) return rc;
   } else if (a.D == 128) {
     NSA_CUDA_OK(func_smem((const void*)tc_bwd_kernel<128>, smem));
@@ -1556,14 +1757,12 @@ int tc_attn_bwd(const AttnArgs& a, void* ws, size_t ws_bytes, cudaStream_t st) {
   const unsigned rgrid = (unsigned)((nthreads + 255) / 256);
   {
     KernelScope ks(branch_name(kRedNames, a.kind), st);
-    if (a.D == 128)
-      dq_reduce_kernel<128><<<rgrid, 256, 0, st>>>(p.dq_part, p.plan.pair_of_slot, (__nv_bfloat16*)a.dq, a.B, a.Hq,
-                                                  a.Hkv, a.T, G, a.kind, a.window, a.block_size, a.Lk,
-                                                  pl.n_slots, a.S);
-    else
-      dq_reduce_kernel<64><<<rgrid, 256, 0, st>>>(p.dq_part, p.plan.pair_of_slot, (__nv_bfloat16*)a.dq, a.B, a.Hq,
-                                                 a.Hkv, a.T, G, a.kind, a.window, a.block_size, a.Lk,
-                                                 pl.n_slots, a.S);
+    auto go = [&](auto kernel) {
+      kernel<<<rgrid, 256, 0, st>>>(p.dq_part, p.plan.pair_of_slot, (__nv_bfloat16*)a.dq, a.B, a.Hq, a.Hkv, a.T, G, a.kind,
+                                    a.window, a.block_size, a.Lk, pl.n_slots, a.S);
+    };
+    if (a.two_term) { if (a.D == 128) go(dq_reduce_kernel<128, true>); else go(dq_reduce_kernel<64, true>); }
+    else { if (a.D == 128) go(dq_reduce_kernel<128, false>); else go(dq_reduce_kernel<64, false>); }
   }
   NSA_LAUNCH_OK("dq_reduce_kernel");
   return NSA_OK;
@@ -1580,14 +1779,15 @@ int tc_dq_reduce3(const AttnArgs& base, int Lk_cmp, int cmp_len, int cmp_stride,
   using namespace tc;
   Reduce3Args r;
   r.acc = dq_acc;
-  r.part_cmp = r.part_slc = r.part_win = nullptr;
+  r.part_cmp = r.part_win = nullptr;
+  r.part_slc = nullptr;
   r.pair_of_slot = nullptr;
   r.slots_cmp = r.slots_win = 1;
   r.Lk_cmp = Lk_cmp; r.cmp_len = cmp_len; r.cmp_stride = cmp_stride; r.S = S; r.window = window;
   r.dq = (__nv_bfloat16*)dq;
   r.B = base.B; r.Hq = base.Hq; r.Hkv = base.Hkv; r.T = base.T; r.G = base.Hq / base.Hkv;
   if (ws_cmp) {
-    AttnArgs a = base; a.kind = 1; a.Lk = Lk_cmp; a.block_size = cmp_len; a.window = cmp_stride;
+    AttnArgs a = base; a.two_term = false; a.kind = 1; a.Lk = Lk_cmp; a.block_size = cmp_len; a.window = cmp_stride;
     const BwdPlan pl = plan_bwd(a);
     r.part_cmp = (const __nv_bfloat16*)((const char*)ws_cmp + pl.off_part);
     r.slots_cmp = pl.n_slots;
@@ -1595,11 +1795,11 @@ int tc_dq_reduce3(const AttnArgs& base, int Lk_cmp, int cmp_len, int cmp_stride,
   if (ws_slc) {
     AttnArgs a = base; a.kind = 2; a.Lk = base.T; a.S = S; a.block_size = block_size;
     const BwdPlan pl = plan_bwd(a);
-    r.part_slc = (const __nv_bfloat16*)((const char*)ws_slc + pl.off_part);
+    r.part_slc = (const char*)ws_slc + pl.off_part;
     r.pair_of_slot = pos ? pos : sel_plan_at((const char*)ws_slc + pl.off_plan, pl.layout).pair_of_slot;
   }
   if (ws_win) {
-    AttnArgs a = base; a.kind = 0; a.Lk = base.T; a.window = window;
+    AttnArgs a = base; a.two_term = false; a.kind = 0; a.Lk = base.T; a.window = window;
     const BwdPlan pl = plan_bwd(a);
     r.part_win = (const __nv_bfloat16*)((const char*)ws_win + pl.off_part);
     r.slots_win = pl.n_slots;
@@ -1609,15 +1809,16 @@ int tc_dq_reduce3(const AttnArgs& base, int Lk_cmp, int cmp_len, int cmp_stride,
   if (nthreads == 0) return NSA_OK;
   const unsigned grid = (unsigned)((nthreads + 255) / 256);
   KernelScope ks("dq_reduce3", st);
-  if (base.D == 128) {
-    if (hg == 2) dq_reduce3_kernel<128, 2><<<grid, 256, 0, st>>>(r);
-    else if (hg == 3) dq_reduce3_kernel<128, 3><<<grid, 256, 0, st>>>(r);
-    else dq_reduce3_kernel<128, 1><<<grid, 256, 0, st>>>(r);
-  } else {
-    if (hg == 2) dq_reduce3_kernel<64, 2><<<grid, 256, 0, st>>>(r);
-    else if (hg == 3) dq_reduce3_kernel<64, 3><<<grid, 256, 0, st>>>(r);
-    else dq_reduce3_kernel<64, 1><<<grid, 256, 0, st>>>(r);
-  }
+  auto go = [&](auto kernel) { kernel<<<grid, 256, 0, st>>>(r); };
+  auto by_heads = [&](auto f32) {
+    constexpr bool kF32 = decltype(f32)::value;
+    if (base.D == 128) {
+      if (hg == 2) go(dq_reduce3_kernel<128, 2, kF32>); else if (hg == 3) go(dq_reduce3_kernel<128, 3, kF32>); else go(dq_reduce3_kernel<128, 1, kF32>);
+    } else {
+      if (hg == 2) go(dq_reduce3_kernel<64, 2, kF32>); else if (hg == 3) go(dq_reduce3_kernel<64, 3, kF32>); else go(dq_reduce3_kernel<64, 1, kF32>);
+    }
+  };
+  if (base.two_term) by_heads(std::true_type()); else by_heads(std::false_type());
   NSA_LAUNCH_OK("dq_reduce3_kernel");
   return NSA_OK;
 }

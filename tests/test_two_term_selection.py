@@ -1,0 +1,134 @@
+"""Selection on 16- and 32-token blocks by default: the tcgen05 kernels with P and dS in two bf16 terms against the
+CUDA-core kernels (fp32 throughout) and against 64-bit arithmetic, over the forms of a call that both accept."""
+import pytest
+import torch
+
+from tests.test_call_forms import _selection_64, _shifted
+from tests.util import cfg_id, dev, make_inputs, pkg
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(autouse=True)
+def _reset():
+    yield
+    pkg().set_impl("auto")
+
+
+def _both(q, k, v, do, idx, bs):
+    """[o, dq, dk, dv, lse] by default and on the CUDA cores, both backward from the latter's o and LSE."""
+    nsa = pkg()
+    out = []
+    for impl in ("simt", "auto"):
+        nsa.set_impl(impl)
+        o, lse = nsa.selection_forward_triton(q, k, v, idx, bs, return_lse=True)
+        o_in, lse_in = (out[0][0], out[0][4]) if out else (o, lse)
+        out.append([o, *nsa.ops._selection_backward(q, k, v, idx, bs, do, o_in, lse_in), lse])
+    assert nsa.lib().nsa_device_status(None) == 0
+    return out[1], out[0]
+
+
+def _close(got, want, what):
+    """Two bf16 roundings of the same value, each half a step (2^-9), and fp32 sums whose terms are up to the
+    largest entry: 2e-5 of it."""
+    for a, b, n in zip(got, want, ("o", "dq", "dk", "dv")):
+        a, b = a.double(), b.double()
+        fin = torch.isfinite(b)
+        assert torch.equal(torch.isfinite(a), fin), (what, n)
+        a, b = a[fin], b[fin]
+        assert ((a - b).abs() <= 2.0 ** -7 * b.abs() + 2e-5 * b.abs().max()).all(), (what, n)
+    a, b = got[4], want[4]
+    fin = torch.isfinite(b)
+    assert torch.equal(torch.isfinite(a), fin) and ((a - b)[fin].abs() <= 1e-5 * b[fin].abs().clamp(min=1)).all(), (what, "lse")
+
+
+# one key tile and less; tiles and row tiles that end ragged; 2, 3, 4, 16 and 64 heads a group; few key tiles with many
+# rows (clusters); work items that are split (a block that every query lists, more than 128 row tiles)
+SHAPES = [dict(B=1, Hq=4, Hkv=2, D=64, T=17, block_size=16, S=1),
+          dict(B=1, Hq=8, Hkv=2, D=128, T=64, block_size=16, S=3),
+          dict(B=2, Hq=6, Hkv=2, D=64, T=129, block_size=32, S=2),
+          dict(B=2, Hq=12, Hkv=4, D=128, T=447, block_size=16, S=8),
+          dict(B=1, Hq=16, Hkv=1, D=128, T=833, block_size=32, S=5),
+          dict(B=1, Hq=64, Hkv=1, D=64, T=321, block_size=16, S=40),
+          dict(B=1, Hq=16, Hkv=1, D=64, T=1100, block_size=16, S=4),
+          dict(B=1, Hq=16, Hkv=1, D=128, T=1100, block_size=16, S=4)]
+
+
+@pytest.mark.parametrize("c", SHAPES, ids=cfg_id)
+def test_against_the_cuda_cores_and_64_bits(c):
+    t = make_inputs(c, torch.bfloat16, seed=4)
+    bs, idx = c["block_size"], t["block_idx"].clone()
+    if c["T"] > 1000:
+        idx[..., -1] = torch.where((idx == 0).any(-1), idx[..., -1], torch.zeros_like(idx[..., -1]))
+    ins = [dev(t[n], torch.bfloat16) for n in ("q", "ks", "vs", "do")]
+    got, want = _both(*ins, idx.cuda(), bs)
+    _close(got, want, "auto against simt")
+    if c["T"] > 500:
+        return
+    o64, _, _, dq64, dk64, dv64 = _selection_64(t, idx, bs)
+    for a, b, r, n in zip(got, want, (o64, dq64, dk64, dv64), ("o", "dq", "dk", "dv")):
+        e = [((x.double().cpu() - r).norm() / r.norm().clamp(min=1e-300)).item() for x in (a, b)]
+        # a bf16 result is off by its rounding whoever computes it; 2 % for which way the ties of few values fall
+        assert e[0] <= 1.02 * e[1] + 1e-6, (n, e)
+
+
+@pytest.mark.parametrize("where", ["k", "v", "q", "do"])
+@pytest.mark.parametrize("D,Hkv,bad", [(64, 2, float("inf")), (128, 1, float("nan")), (64, 1, float("-inf"))], ids=str)
+def test_non_finite_values_stay_with_their_rows(D, Hkv, bad, where):
+    """A value that is infinite or NaN reaches what attends it, as it does in the CUDA-core kernels, and no more."""
+    c = dict(B=1, Hq=8, Hkv=Hkv, D=D, T=200, block_size=16, S=3)
+    t = make_inputs(c, torch.bfloat16, seed=9)
+    x = {n: dev(t[m], torch.bfloat16) for n, m in (("q", "q"), ("k", "ks"), ("v", "vs"), ("do", "do"))}
+    idx = t["block_idx"].cuda()
+    for at in (2, 61, 130):
+        y = dict(x)
+        y[where] = x[where].clone()
+        y[where][:, :, at, 3] = bad
+        _close(*_both(**y, idx=idx, bs=16), (where, at))
+
+
+@pytest.mark.parametrize("bs,S", [(16, 4), (32, 3)])
+@pytest.mark.parametrize("D", [64, 128])
+def test_repeated_blocks_count_as_often_as_listed(D, bs, S):
+    c = dict(B=2, Hq=6, Hkv=2, D=D, T=333, block_size=bs, S=S)
+    t = make_inputs(c, torch.bfloat16, seed=2)
+    idx = t["block_idx"].clone()
+    idx[:, :, ::3, 2] = idx[:, :, ::3, 0]
+    idx[:, 1, 5::7, 1:] = idx[:, 1, 5::7, :1]
+    ins = [dev(t[n], torch.bfloat16) for n in ("q", "ks", "vs", "do")]
+    _close(*_both(*ins, idx.cuda(), bs), "repeats")
+
+
+def test_views_off_a_16_byte_boundary():
+    """What the tensor cores load by TMA starts on a 16-byte boundary: q, v and dO that do not leave the call to the
+    CUDA cores, whose row kernels read them by elements; K (and V in backward), which they read as
+    16-byte vectors, are refused."""
+    nsa = pkg()
+    c = dict(B=1, Hq=8, Hkv=2, D=64, T=200, block_size=16, S=3)
+    t = make_inputs(c, torch.bfloat16, seed=1)
+    q, k, v, do = (dev(t[n], torch.bfloat16) for n in ("q", "ks", "vs", "do"))
+    idx = t["block_idx"].cuda()
+    nsa.set_impl("simt")
+    o, lse = nsa.selection_forward_triton(q, k, v, idx, 16, return_lse=True)
+    grads = nsa.ops._selection_backward(q, k, v, idx, 16, do, o, lse)
+    nsa.set_impl("auto")
+    for x in ((_shifted(q), k, v), (q, k, _shifted(v))):
+        for a, b in zip(nsa.selection_forward_triton(*x, idx, 16, return_lse=True), (o, lse)):
+            assert torch.equal(a, b)
+    for x in ((_shifted(q), k, v, do), (q, k, v, _shifted(do))):
+        got = nsa.ops._selection_backward(*x[:3], idx, 16, x[3], o, lse)
+        assert torch.equal(got[0], grads[0])
+        for a, b in zip(got[1:], grads[1:]):                     # sums that meet by atomics, rounded to bf16
+            assert ((a.float() - b.float()).abs() <= 2.0 ** -7 * b.float().abs() + 1e-5 * b.float().abs().max()).all()
+    with pytest.raises(nsa._lib.NsaError):
+        nsa.selection_forward_triton(q, _shifted(k), v, idx, 16)
+    for x in ((q, _shifted(k), v), (q, k, _shifted(v))):
+        with pytest.raises(nsa._lib.NsaError):
+            nsa.ops._selection_backward(*x, idx, 16, do, o, lse)
+    # the whole op, forward
+    ins = [dev(t[n], torch.bfloat16) for n in ("q", "kc", "vc", "ks", "vs", "kw", "vw", "gate")]
+    want = nsa.nsa_fused_forward(*ins, idx, 16, 64)
+    ins[4] = _shifted(ins[4])
+    got = nsa.nsa_fused_forward(*ins, idx, 16, 64)
+    assert ((got.float() - want.float()).abs() <= 2.0 ** -6 * want.float().abs().clamp(min=1)).all()
+    assert nsa.lib().nsa_device_status(None) == 0
