@@ -11,6 +11,10 @@
 // backward, add every key's gradient by its own atomics; here one vector atomic per (row tile, key)
 // does, and window / compression / selection at B=1, T=2048, 8 heads of 64 in fp32 go from
 // 1.6 / 3.8 ms (forward / backward, three branches) to 0.42 / 0.68 ms.
+// A row tile is one chain through its key tiles: where tiles are few a cluster of 2 or 4 CTAs shares
+// it, every CTA its key tiles, and adds up O (by its maximum) or dQ through distributed shared memory in
+// rank order; at that size selection goes from 299 / 453 us to 187 / 353.
+#include "cluster.cuh"
 #include "common.cuh"
 
 namespace nsa {
@@ -85,12 +89,21 @@ struct TileKeys {
   int first, n;            // window / compression: first key and their number; selection: 0, keys of the union
 };
 
-struct SelList {           // selection only, in shared memory
-  unsigned long long mask[kMaxBlocks];   // queries of the tile that list a block
-  uint16_t list[kMaxBlocks];             // the listed blocks, ascending
-  int n_list;
-  int repeats;                           // some query lists a block more than once
+struct SelList {           // selection only, in shared memory: as many blocks as the sequence has
+  unsigned long long* mask;   // queries of the tile that list a block
+  int* n_list;
+  int* repeats;               // not 0: some query lists a block more than once
+  uint16_t* list;             // the listed blocks, ascending
 };
+__host__ __device__ __forceinline__ int sel_blocks(const AttnArgs& a) { return (a.T + a.block_size - 1) / a.block_size; }
+__device__ __forceinline__ SelList sel_list(const AttnArgs& a, void* at) {
+  SelList s;
+  s.mask = (unsigned long long*)at;
+  s.n_list = (int*)(s.mask + (a.kind == 2 ? sel_blocks(a) : 0));
+  s.repeats = s.n_list + 1;
+  s.list = (uint16_t*)(s.n_list + 2);
+  return s;
+}
 
 // shared memory of one tile's key bookkeeping, double buffered: the next tile is fetched ahead
 struct KeyInfo {
@@ -99,7 +112,7 @@ struct KeyInfo {
 };
 
 template <int kThreads>
-__device__ __forceinline__ TileKeys tile_keys(const AttnArgs& a, int bh, int t_first, int t_last, SelList* sl) {
+__device__ __forceinline__ TileKeys tile_keys(const AttnArgs& a, int bh, int t_first, int t_last, const SelList& sl) {
   TileKeys k;
   k.first = 0; k.n = 0;
   if (a.kind == 0) {
@@ -109,8 +122,8 @@ __device__ __forceinline__ TileKeys tile_keys(const AttnArgs& a, int bh, int t_f
     k.n = cmp_visible(t_last, a.block_size, a.window, a.Lk);   // compression: window holds the stride
   } else {
     const int n_blk = (t_last + a.block_size) / a.block_size;   // blocks that start at or before t_last
-    for (int i = threadIdx.x; i < n_blk; i += kThreads) sl->mask[i] = 0ull;
-    if (threadIdx.x == 0) sl->repeats = 0;
+    for (int i = threadIdx.x; i < n_blk; i += kThreads) sl.mask[i] = 0ull;
+    if (threadIdx.x == 0) *sl.repeats = 0;
     __syncthreads();
     const int32_t* idx = a.block_idx + ((size_t)bh * a.T + t_first) * a.S;
     const int n_e = (t_last - t_first + 1) * a.S;
@@ -118,23 +131,23 @@ __device__ __forceinline__ TileKeys tile_keys(const AttnArgs& a, int bh, int t_f
       const int ql = e / a.S;
       const int blk = __ldg(idx + e);
       if (blk >= 0 && (long long)blk * a.block_size <= t_first + ql &&
-          (atomicOr(&sl->mask[blk], 1ull << ql) >> ql & 1ull))
-        sl->repeats = 1;
+          (atomicOr(&sl.mask[blk], 1ull << ql) >> ql & 1ull))
+        *sl.repeats = 1;
     }
     __syncthreads();
     if (threadIdx.x < 32) {
       int n = 0;
       for (int b0 = 0; b0 < n_blk; b0 += 32) {
         const int b = b0 + threadIdx.x;
-        const bool on = b < n_blk && sl->mask[b] != 0ull;
+        const bool on = b < n_blk && sl.mask[b] != 0ull;
         const unsigned m = __ballot_sync(0xffffffffu, on);
-        if (on) sl->list[n + __popc(m & ((1u << threadIdx.x) - 1u))] = (uint16_t)b;
+        if (on) sl.list[n + __popc(m & ((1u << threadIdx.x) - 1u))] = (uint16_t)b;
         n += __popc(m);
       }
-      if (threadIdx.x == 0) sl->n_list = n;
+      if (threadIdx.x == 0) *sl.n_list = n;
     }
     __syncthreads();
-    k.n = sl->n_list * a.block_size;
+    k.n = *sl.n_list * a.block_size;
   }
   return k;
 }
@@ -151,16 +164,16 @@ __device__ __forceinline__ int times_listed(const AttnArgs& a, int bh, int t, in
 }
 
 // token and membership of key tile i's keys (threads 0..63)
-__device__ __forceinline__ void fill_keys(const AttnArgs& a, const TileKeys& tk, const SelList* sl, KeyInfo* ki, int buf, int i) {
+__device__ __forceinline__ void fill_keys(const AttnArgs& a, const TileKeys& tk, const SelList& sl, KeyInfo* ki, int buf, int i) {
   if (threadIdx.x >= kK) return;
   const int k = i * kK + threadIdx.x;
   int tok = -1;
   unsigned long long m = 0ull;
   if (k < tk.n) {
     if (a.kind == 2) {
-      const int b = sl->list[k / a.block_size];
+      const int b = sl.list[k / a.block_size];
       tok = b * a.block_size + k % a.block_size;
-      m = sl->mask[b];
+      m = sl.mask[b];
       if (tok >= a.T) tok = -1;
     } else {
       tok = tk.first + k;
@@ -234,7 +247,7 @@ constexpr int kBwdThreads = 256;
 // S and D / 16 columns of O.  V travels while S is computed, the next K while O is.
 template <typename T, int D>
 __global__ void __launch_bounds__(kFwdThreads)
-simt_tile_fwd_kernel(const AttnArgs a) {
+simt_tile_fwd_kernel(const AttnArgs a, const int csize) {
   constexpr int LD = D + kPad, C = D / 16;
   extern __shared__ float4 sm4[];
   float* sQ = reinterpret_cast<float*>(sm4);
@@ -242,18 +255,19 @@ simt_tile_fwd_kernel(const AttnArgs a) {
   float* sV = sK + kK * LD;
   float* sP = sV + kK * LD;
   KeyInfo* ki = reinterpret_cast<KeyInfo*>(sP + kR * kPLd);
-  SelList* sl = reinterpret_cast<SelList*>(ki + 1);
+  const SelList sl = sel_list(a, ki + 1);
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   const int G = a.Hq / a.Hkv, n_rows = a.T * G, tiles = (n_rows + kR - 1) / kR;
-  const int bh = blockIdx.x / tiles, b = bh / a.Hkv, hkv = bh % a.Hkv;
-  const int row0 = (tiles - 1 - (int)blockIdx.x % tiles) * kR;       // long rows first
+  const int rank = (int)blockIdx.x & (csize - 1), work = (int)blockIdx.x / csize;    // the cluster's CTAs take its key tiles in turn
+  const int bh = work / tiles, b = bh / a.Hkv, hkv = bh % a.Hkv;
+  const int row0 = (tiles - 1 - work % tiles) * kR;                  // long rows first
   const int t_first = row0 / G, t_last = (min(row0 + kR, n_rows) - 1) / G;
   auto row_ptr = [&](int r) -> size_t {                              // row r of the tile in [B, Hq, T]
     const int f = row0 + r;
     return ((size_t)b * a.Hq + hkv * G + f % G) * a.T + f / G;
   };
   const TileKeys tk = tile_keys<kFwdThreads>(a, bh, t_first, t_last, sl);
-  const bool repeats = a.kind == 2 && sl->repeats;
+  const bool repeats = a.kind == 2 && *sl.repeats;
   const int n_kt = (tk.n + kK - 1) / kK;
   const T* kbase = reinterpret_cast<const T*>(a.k) + (size_t)bh * a.Lk * D;
   const T* vbase = reinterpret_cast<const T*>(a.v) + (size_t)bh * a.Lk * D;
@@ -279,16 +293,17 @@ simt_tile_fwd_kernel(const AttnArgs a) {
 #pragma unroll
     for (int c = 0; c < C; ++c) o[i][c] = 0.f;
   }
-  if (n_kt > 0) {
-    fill_keys(a, tk, sl, ki, 0, 0);
+  if (rank < n_kt) {
+    fill_keys(a, tk, sl, ki, 0, rank);
     __syncthreads();
     load_keys<T, D, kFwdThreads>(sK, kbase, ki->tok[0]);
     cp_commit();
     load_keys<T, D, kFwdThreads>(sV, vbase, ki->tok[0]);
     cp_commit();
   }
-  for (int kt = 0; kt < n_kt; ++kt) {
-    const int buf = kt & 1;
+  int buf = 0;
+  for (int kt = rank; kt < n_kt; kt += csize, buf ^= 1) {
+    const bool more = kt + csize < n_kt;
     cp_wait<1>();
     __syncthreads();
     float s[8][4];
@@ -359,9 +374,9 @@ simt_tile_fwd_kernel(const AttnArgs a) {
         }
       }
     }
-    if (kt + 1 < n_kt) fill_keys(a, tk, sl, ki, buf ^ 1, kt + 1);
+    if (more) fill_keys(a, tk, sl, ki, buf ^ 1, kt + csize);
     __syncthreads();
-    if (kt + 1 < n_kt) load_keys<T, D, kFwdThreads>(sK, kbase, ki->tok[buf ^ 1]);
+    if (more) load_keys<T, D, kFwdThreads>(sK, kbase, ki->tok[buf ^ 1]);
     cp_commit();
     cp_wait<1>();
     if (__syncthreads_or(non_finite<T, D, kFwdThreads>(sV))) {
@@ -394,14 +409,49 @@ simt_tile_fwd_kernel(const AttnArgs a) {
       }
     }
     __syncthreads();
-    if (kt + 1 < n_kt) load_keys<T, D, kFwdThreads>(sV, vbase, ki->tok[buf ^ 1]);
+    if (more) load_keys<T, D, kFwdThreads>(sV, vbase, ki->tok[buf ^ 1]);
     cp_commit();
   }
   cp_wait<0>();
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
+  for (int i = 0; i < 8; ++i)
 #pragma unroll
     for (int w = 8; w >= 1; w >>= 1) l[i] += __shfl_xor_sync(0xffffffffu, l[i], w);
+  if (csize > 1) {
+    // every CTA leaves what its keys gave (O over the K tile; m and l over P); the rows are dealt out for the sum
+    float* sO = sK;
+    float* sM = sP;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+#pragma unroll
+      for (int c = 0; c < C; ++c) sO[(ty + 8 * i) * LD + col_of<C>(tx, c)] = o[i][c];
+      if (tx == 0) { sM[ty + 8 * i] = m[i]; sM[kR + ty + 8 * i] = l[i]; }
+    }
+    cluster_sync();
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      if ((i & (csize - 1)) != rank) continue;
+      const int r = ty + 8 * i;
+      float mx = -INFINITY;
+      for (int k = 0; k < csize; ++k) mx = fmaxf(mx, ld_peer_f32(sM + r, k));
+      const float ms = mx == -INFINITY ? 0.f : mx;
+      l[i] = 0.f;
+#pragma unroll
+      for (int c = 0; c < C; ++c) o[i][c] = 0.f;
+      for (int k = 0; k < csize; ++k) {
+        const float w = expf(ld_peer_f32(sM + r, k) - ms);
+        l[i] = fmaf(w, ld_peer_f32(sM + kR + r, k), l[i]);
+#pragma unroll
+        for (int c = 0; c < C; ++c) o[i][c] = fmaf(w, ld_peer_f32(sO + r * LD + col_of<C>(tx, c), k), o[i][c]);
+      }
+      m[i] = mx;
+    }
+    cluster_sync();                       // nobody leaves while its memory is read
+  }
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    if ((i & (csize - 1)) != rank) continue;
     if (row0 + ty + 8 * i < n_rows) {
       const size_t row = row_ptr(ty + 8 * i);
       const float inv = l[i] > 0.f ? 1.f / l[i] : 0.f;
@@ -417,7 +467,7 @@ simt_tile_fwd_kernel(const AttnArgs a) {
 // columns of dQ (rows ty + 16 i) and of dK / dV (keys 4 ty + e), which leave by vector atomics.
 template <typename T, int D>
 __global__ void __launch_bounds__(kBwdThreads, D <= 64 ? 2 : 1)
-simt_tile_bwd_kernel(const AttnArgs a) {
+simt_tile_bwd_kernel(const AttnArgs a, const int csize) {
   constexpr int LD = D + kPad, C = D / 16;
   extern __shared__ float4 sm4[];
   float* sQ = reinterpret_cast<float*>(sm4);
@@ -427,26 +477,27 @@ simt_tile_bwd_kernel(const AttnArgs a) {
   float* sP = sV + kK * LD;
   float* sDS = sP + kR * kPLd;
   KeyInfo* ki = reinterpret_cast<KeyInfo*>(sDS + kR * kPLd);
-  SelList* sl = reinterpret_cast<SelList*>(ki + 1);
+  const SelList sl = sel_list(a, ki + 1);
   __shared__ float s_lse[kR], s_delta[kR];
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   const int G = a.Hq / a.Hkv, n_rows = a.T * G, tiles = (n_rows + kR - 1) / kR;
-  const int bh = blockIdx.x / tiles, b = bh / a.Hkv, hkv = bh % a.Hkv;
-  const int row0 = (tiles - 1 - (int)blockIdx.x % tiles) * kR;
+  const int rank = (int)blockIdx.x & (csize - 1), work = (int)blockIdx.x / csize;
+  const int bh = work / tiles, b = bh / a.Hkv, hkv = bh % a.Hkv;
+  const int row0 = (tiles - 1 - work % tiles) * kR;
   const int t_first = row0 / G, t_last = (min(row0 + kR, n_rows) - 1) / G;
   auto row_ptr = [&](int r) -> size_t {
     const int f = row0 + r;
     return ((size_t)b * a.Hq + hkv * G + f % G) * a.T + f / G;
   };
   const TileKeys tk = tile_keys<kBwdThreads>(a, bh, t_first, t_last, sl);
-  const bool repeats = a.kind == 2 && sl->repeats;
+  const bool repeats = a.kind == 2 && *sl.repeats;
   const int n_kt = (tk.n + kK - 1) / kK;
   const size_t kvoff = (size_t)bh * a.Lk * D;
   const T* kbase = reinterpret_cast<const T*>(a.k) + kvoff;
   const T* vbase = reinterpret_cast<const T*>(a.v) + kvoff;
   float* dkb = a.dk_acc + kvoff;
   float* dvb = a.dv_acc + kvoff;
-  if (n_kt > 0) fill_keys(a, tk, sl, ki, 0, 0);
+  if (rank < n_kt) fill_keys(a, tk, sl, ki, 0, rank);
   // Q (scaled), dO (times the gate of a gated branch), lse and delta; four threads per row
   bool rows_bad;                        // a value of Q or dO is infinite or NaN
   {
@@ -496,13 +547,14 @@ simt_tile_bwd_kernel(const AttnArgs a) {
 #pragma unroll
     for (int c = 0; c < C; ++c) dq[i][c] = 0.f;
   }
-  if (n_kt > 0) {
+  if (rank < n_kt) {
     load_keys<T, D, kBwdThreads>(sV, vbase, ki->tok[0]);
     load_keys<T, D, kBwdThreads>(sK, kbase, ki->tok[0]);
     cp_commit();
   }
-  for (int kt = 0; kt < n_kt; ++kt) {
-    const int buf = kt & 1;
+  int buf = 0;
+  for (int kt = rank; kt < n_kt; kt += csize, buf ^= 1) {
+    const bool more = kt + csize < n_kt;
     cp_wait<0>();
     const bool bad = __syncthreads_or(non_finite<T, D, kBwdThreads>(sK) || non_finite<T, D, kBwdThreads>(sV)) || rows_bad;
     float s[4][4], dp[4][4];
@@ -553,9 +605,9 @@ simt_tile_bwd_kernel(const AttnArgs a) {
         if (n > 1) { sP[at] *= (float)n; sDS[at] *= (float)n; }
       }
     }
-    if (kt + 1 < n_kt) fill_keys(a, tk, sl, ki, buf ^ 1, kt + 1);
+    if (more) fill_keys(a, tk, sl, ki, buf ^ 1, kt + csize);
     __syncthreads();
-    if (kt + 1 < n_kt) load_keys<T, D, kBwdThreads>(sV, vbase, ki->tok[buf ^ 1]);
+    if (more) load_keys<T, D, kBwdThreads>(sV, vbase, ki->tok[buf ^ 1]);
     // dQ += dS K
     if (bad) {
 #pragma unroll 1
@@ -587,7 +639,7 @@ simt_tile_bwd_kernel(const AttnArgs a) {
       }
     }
     __syncthreads();
-    if (kt + 1 < n_kt) load_keys<T, D, kBwdThreads>(sK, kbase, ki->tok[buf ^ 1]);
+    if (more) load_keys<T, D, kBwdThreads>(sK, kbase, ki->tok[buf ^ 1]);
     cp_commit();
     // dV += P^T dO and dK += dS^T Q (Q carries the scale), one after the other to spare registers
 #pragma unroll
@@ -631,9 +683,28 @@ simt_tile_bwd_kernel(const AttnArgs a) {
       }
     }
   }
+  if (csize > 1) {                        // dQ of the cluster's CTAs, over their K tiles, in rank order
+    float* sD = sK;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int c = 0; c < C; ++c) sD[(ty + 16 * i) * LD + col_of<C>(tx, c)] = dq[i][c];
+    cluster_sync();
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      if ((i & (csize - 1)) != rank) continue;
+#pragma unroll
+      for (int c = 0; c < C; ++c) {
+        dq[i][c] = 0.f;
+        for (int k = 0; k < csize; ++k) dq[i][c] += ld_peer_f32(sD + (ty + 16 * i) * LD + col_of<C>(tx, c), k);
+      }
+    }
+    cluster_sync();                       // nobody leaves while its memory is read
+  }
 #pragma unroll
   for (int i = 0; i < 4; ++i)
-    if (row0 + ty + 16 * i < n_rows) {
+    if ((i & (csize - 1)) == rank && row0 + ty + 16 * i < n_rows) {
 #pragma unroll
       for (int c = 0; c < C; ++c) dq[i][c] *= a.scale;
       store_cols<C>(reinterpret_cast<T*>(a.dq) + row_ptr(ty + 16 * i) * D, tx, dq[i]);
@@ -644,21 +715,51 @@ long long n_tiles(const AttnArgs& a) {
   return ((long long)a.T * (a.Hq / a.Hkv) + kR - 1) / kR * a.B * a.Hkv;
 }
 
-size_t extra_smem(const AttnArgs& a) { return sizeof(KeyInfo) + (a.kind == 2 ? sizeof(SelList) : 0); }
+size_t extra_smem(const AttnArgs& a) { return sizeof(KeyInfo) + 16 + (a.kind == 2 ? (size_t)sel_blocks(a) * 10 : 0); }
+
+// CTAs that share a row tile, each taking every csize-th key tile.  A row tile is one long chain; with few of them the
+// longest is what the call waits for.  The lines, in row tiles per SM (fp32, D = 64, 8 heads on 2; alone | 2 | 4 CTAs a
+// tile, us): selection at 0.86 forward 132 | 93 | 66, backward 232 | 180 | 125; at 1.7 310 | 189 | 182 and
+// 640 | 355 | 399; at 6.9 650 | 615 | 678 and 1507 | 1345 | 1499; at 21 1648 | 1691 | 2021 and 3935 | 3994 | 4467.
+// Window (chains of 9 key tiles) at 0.4 69 | 44 | 37 and 109 | 64 | 55; at 1.3 101 | 78 | 90 and 196 | 145 | 159; at 1.7
+// 103 | 98 | 121 and 199 | 215 | 225.  At D = 128 a tile has an SM to itself: sharing only fills idle SMs.
+int cluster_size(const AttnArgs& a) {
+  const long long tiles = n_tiles(a), sms = sm_count();
+  const int n_kt = ((a.kind == 0 ? a.window + kR / (a.Hq / a.Hkv) : a.Lk) + kK - 1) / kK;
+  int csize = 1;
+  if (a.D > 64) csize = 4 * tiles <= sms ? 4 : 2 * tiles <= sms ? 2 : 1;
+  else if (a.kind == 2) csize = tiles <= sms ? 4 : tiles <= 7 * sms ? 2 : 1;
+  else csize = 2 * tiles <= sms ? 4 : 3 * tiles <= 4 * sms ? 2 : 1;
+  while (csize > 1 && n_kt < 2 * csize) csize >>= 1;
+  return csize;
+}
 
 template <typename T, int D>
 int launch(const AttnArgs& a, bool bwd, cudaStream_t st) {
-  const unsigned grid = (unsigned)n_tiles(a);         // in x, which takes any number of units
+  const int csize = cluster_size(a);
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = (unsigned)csize;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)n_tiles(a) * csize);   // in x, which takes any number of units
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = csize > 1 ? 1 : 0;
   if (!bwd) {
     const size_t smem = fwd_floats<D>() * sizeof(float) + extra_smem(a);
     NSA_CUDA_OK(func_smem((const void*)simt_tile_fwd_kernel<T, D>, smem));
     KernelScope ks(branch_name(kFwdNames, a.kind), st);
-    simt_tile_fwd_kernel<T, D><<<grid, kFwdThreads, smem, st>>>(a);
+    cfg.blockDim = dim3(kFwdThreads);
+    cfg.dynamicSmemBytes = smem;
+    NSA_CUDA_OK(cudaLaunchKernelEx(&cfg, simt_tile_fwd_kernel<T, D>, a, csize));
   } else {
     const size_t smem = bwd_floats<D>() * sizeof(float) + extra_smem(a);
     NSA_CUDA_OK(func_smem((const void*)simt_tile_bwd_kernel<T, D>, smem));
     KernelScope ks(branch_name(kBwdNames, a.kind), st);
-    simt_tile_bwd_kernel<T, D><<<grid, kBwdThreads, smem, st>>>(a);
+    cfg.blockDim = dim3(kBwdThreads);
+    cfg.dynamicSmemBytes = smem;
+    NSA_CUDA_OK(cudaLaunchKernelEx(&cfg, simt_tile_bwd_kernel<T, D>, a, csize));
   }
   NSA_LAUNCH_OK("simt_tile kernel");
   return NSA_OK;
@@ -681,11 +782,11 @@ int launch_d(const AttnArgs& a, bool bwd, cudaStream_t st) {
 // average over a causal sequence), where a row at a time goes through its own blocks only.  At 64
 // blocks of 16 tokens, 8 list slots, D = 128 and lists that share little (B=2, T=1024, 16 heads) the
 // forward tile took 0.62 ms against 0.36, the backward tile 0.81 against 0.91: the lines are drawn at 4
-// and 8 blocks per list slot.  And a tile is one long chain through its keys, while the row kernels spread
-// its work over 64 warps: with fewer tiles than a GPU holds, the rows end sooner.  At 4 blocks per slot
-// the two take the same time at 1.5 tiles per SM forward and 0.75 backward in bf16, 0.75 and 0.5 in fp32
-// (bf16, 256 tokens, blocks of 16, D = 64: 32 tiles 42 and 70 us, rows 15 and 28; 256 tiles 51 and 118, rows
-// 55 and 115; fp32, 512 tokens, blocks of 32: 384 tiles 110 and 240, rows 214 and 496).
+// and 8 blocks per list slot.  And a tile is a chain through its keys, which four CTAs share
+// at most, while the row kernels spread its work over 64 warps: with few tiles the rows end sooner.  In
+// row tiles per SM (8 heads on 2, tile | rows, us): fp32, D = 64, blocks of 64, at 0.11 forward 29 | 27 and backward 41 | 33,
+// at 0.22 33 | 42 and 44 | 73, at 0.43 39 | 125 and 62 | 251; fp32, blocks of 32, 4 listed, at 0.43 38 | 50 and 63 | 101;
+// bf16, blocks of 16, 4 listed, at 0.22 34 | 25 and 47 | 31; blocks of 32, 8 listed, at 0.65 57 | 86 and 84 | 165.
 // Rows must be whole 16-byte vectors.
 bool simt_tile_ok(const AttnArgs& a, int dtype, bool bwd) {
   const uintptr_t p = (uintptr_t)a.q | (uintptr_t)a.k | (uintptr_t)a.v | (uintptr_t)a.o | (uintptr_t)a.d_o |
@@ -694,8 +795,7 @@ bool simt_tile_ok(const AttnArgs& a, int dtype, bool bwd) {
   if ((long long)a.T * (a.Hq / a.Hkv) >= (1LL << 31) - kR || n_tiles(a) >= (1LL << 31)) return false;
   if (a.kind != 2) return true;
   const int n_blk = (a.T + a.block_size - 1) / a.block_size;
-  const int quarters = dtype == NSA_DTYPE_BF16 ? (bwd ? 3 : 6) : (bwd ? 2 : 3);      // of the tiles per SM
-  return n_blk <= kMaxBlocks && n_blk <= (bwd ? 8LL : 4LL) * a.S && 4 * n_tiles(a) >= (long long)quarters * sm_count();
+  return n_blk <= kMaxBlocks && n_blk <= (bwd ? 8LL : 4LL) * a.S && (dtype == NSA_DTYPE_BF16 ? 2 : 5) * n_tiles(a) >= sm_count();
 }
 
 int simt_tile_fwd(const AttnArgs& a, int dtype, cudaStream_t st) {

@@ -28,6 +28,7 @@
 //                buffer exists; the order of the adds, hence the last bits of dq, is not fixed.
 #include <type_traits>
 
+#include "cluster.cuh"
 #include "sel_row.cuh"
 #include "tc_common.cuh"
 #include "tc_host.cuh"
@@ -563,28 +564,6 @@ constexpr int kB2Threads = 640;   // 2 x 8 compute warps, 3 producer warps, MMA 
 constexpr int kB2Producers = 3;
 constexpr int kB2Compute = 16;    // compute warps
 
-// Cluster helpers.  Every thread of every CTA of the cluster takes part in the barrier.
-__device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
-}
-__device__ __forceinline__ uint32_t peer_addr(const void* p, int rank) {
-  uint32_t a;
-  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
-  return a;
-}
-__device__ __forceinline__ int ld_peer_s32(const int* p, int rank) {
-  int v;
-  asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(peer_addr(p, rank)) : "memory");
-  return v;
-}
-__device__ __forceinline__ float4 ld_peer_f32x4(const float* p, int rank) {
-  float4 v;
-  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-               : "r"(peer_addr(p, rank)) : "memory");
-  return v;
-}
-
-//
 // kTwoTerm: selection on 16- and 32-token blocks, whose results are fp32 arithmetic rounded once.  P and dS go to
 // the tensor cores as two bf16 terms each (16 significant bits; the second adds three products of eight), the dQ
 // partials stay fp32, a block listed twice counts twice and what comes out non-finite is done again row by

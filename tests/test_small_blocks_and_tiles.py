@@ -86,6 +86,32 @@ def test_cuda_core_tiles(c, dtype):
             check(g, r, dtype, f"window {W} {n}", abs32=4e-3)
 
 
+# few row tiles with long chains: clusters of 4 and 2 CTAs share one (the first tiles leave some of them without a
+# key tile), at D = 64 and 128; lengths that end inside a tile
+@pytest.mark.parametrize("c", [dict(B=1, Hq=8, Hkv=2, D=64, T=530, block_size=64, S=6),
+                               dict(B=2, Hq=6, Hkv=2, D=64, T=1001, block_size=32, S=12),
+                               dict(B=1, Hq=4, Hkv=1, D=128, T=530, block_size=64, S=6),
+                               dict(B=1, Hq=4, Hkv=1, D=128, T=1090, block_size=64, S=5),
+                               dict(B=1, Hq=12, Hkv=4, D=16, T=700, block_size=48, S=5)], ids=cfg_id)
+def test_cuda_core_tiles_shared_by_clusters(c):
+    nsa = pkg()
+    _branch(c, torch.float32, "simt", None, "cluster")
+    t = make_inputs(c, torch.float32, seed=6)
+    q, k, v, do = (dev(t[n], torch.float32) for n in ("q", "kw", "vw", "do"))
+    for W in (300, c["T"]):
+        keep = O.window_keep_fn(c["T"], W)
+        o_ref, lse_ref = O.stream_attn_forward(t["q"], t["kw"], t["vw"], keep)
+        grads_ref = O.stream_attn_backward(t["q"], t["kw"], t["vw"], o_ref, lse_ref, t["do"], keep)
+        o, lse = nsa.range_attn_forward(q, k, v, nsa.MODE_WINDOW, W, 0)
+        check(o, o_ref, torch.float32, f"cluster window {W} o")
+        assert (lse.cpu() - lse_ref).abs().max().item() <= 1e-4
+        grads = nsa.range_attn_backward(q, k, v, o, lse, do, nsa.MODE_WINDOW, W, 0)
+        for g, r, n in zip(grads, grads_ref, ("dq", "dk", "dv")):
+            check(g, r, torch.float32, f"cluster window {W} {n}", abs32=4e-3)
+        again = nsa.range_attn_backward(q, k, v, o, lse, do, nsa.MODE_WINDOW, W, 0)
+        assert torch.equal(grads[0], again[0])           # dq adds up in rank order
+
+
 # one summary row and many (2 and 8 rows per CTA, several groups per persistent CTA), windows longer
 # than one pass of a CTA, a tail after the last window
 @pytest.mark.parametrize("geom", [(1, 1, 64, 64, 64), (2, 3, 2500, 64, 64), (1, 2, 700, 128, 200), (1, 4, 333, 32, 48),
