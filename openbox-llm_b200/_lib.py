@@ -2,6 +2,7 @@
 call fails, an exception is raised."""
 import ctypes
 import functools
+import importlib.util
 import os
 
 import torch
@@ -111,6 +112,25 @@ def lib():
             name, _, value = item.partition("=")
             check(handle.nsa_set_option(name.strip().encode(), int(value)))
     return _lib
+
+
+_ext = None
+EXT_PATH = os.path.join(_HERE, "csrc", "_nsa_torch.so")
+
+
+def torch_op():
+    """The autograd nodes in C++ (csrc/torch_op.cpp); raise if they have not been built."""
+    global _ext
+    if _ext is None:
+        lib()
+        if not os.path.exists(EXT_PATH):
+            raise NsaError(f"{EXT_PATH} is missing: build it with `python {_HERE}/build.py`")
+        spec = importlib.util.spec_from_file_location("_nsa_torch", EXT_PATH)
+        mod = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(mod)
+        mod.set_error(NsaError)
+        _ext = mod
+    return _ext
 
 
 def check(rc):

@@ -1,0 +1,292 @@
+// Autograd nodes of the whole op and of the projection layer in C++.  What a short call costs is host work: with
+// 1024 tokens the op's kernels take 150 us forward + backward, while its Python nodes, their tensors and
+// the ctypes calls took 350.  The nodes here do what those of ops.py and module.py do for the usual form of a call
+// (dense CUDA tensors of one device and type that start on 16-byte boundaries, no dispatch mode, transform or
+// trace under way); for every other form the entry points return None and the Python nodes serve it.
+#include <Python.h>
+
+#include <ATen/ATen.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
+#include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/custom_function.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include "../../include/nsa_b200.h"
+
+namespace {
+
+using at::Tensor;
+using torch::autograd::AutogradContext;
+using torch::autograd::variable_list;
+
+PyObject* g_error = nullptr;             // NsaError of the Python package
+
+[[noreturn]] void raise_error(int rc) {
+  PyGILState_STATE s = PyGILState_Ensure();
+  const std::string msg = "libnsa_b200 error " + std::to_string(rc) + ": " + nsa_last_error();
+  PyErr_SetString(g_error, msg.c_str());
+  python_error err;
+  err.persist();
+  PyGILState_Release(s);
+  throw std::move(err);
+}
+void check(int rc) {
+  if (rc != NSA_OK) raise_error(rc);
+}
+
+void* raw_stream(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
+Tensor bytes_like(size_t n, const Tensor& t) { return at::empty({(int64_t)n}, t.options().dtype(at::kByte)); }
+
+// A dense CUDA tensor of the given type on device `dev` that starts on a 16-byte boundary and that no Python-side
+// dispatch stands behind.
+bool plain(const Tensor& t, at::ScalarType dtype, at::Device dev) {
+  return t.defined() && t.layout() == at::kStrided && t.device() == dev && t.scalar_type() == dtype && t.numel() > 0 &&
+         t.is_contiguous() && !t.is_neg() && !t.unsafeGetTensorImpl()->is_python_dispatch() &&
+         (reinterpret_cast<uintptr_t>(t.unsafeGetTensorImpl()->data()) & 15) == 0;
+}
+// No functorch transform and no dispatch mode sees the tensors of this call.
+bool plain_state() {
+  return !c10::impl::TorchDispatchModeTLS::any_modes_set() &&
+         !c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode);
+}
+
+// The tensors of a call in the order of NsaAttentionTensors: q, kc, vc, ks, vs, kw, vw, gate; the compressor's.
+struct Call {
+  NsaAttentionDesc d;
+  Tensor in[8], comp[6], block_idx;
+};
+
+// Sizes that belong together; what is refused here gets its message from the Python side.
+bool fill_desc(Call& c, const int* ints, bool learned, bool given) {
+  const Tensor& q = c.in[0];
+  if (q.dim() != 4 || c.in[1].dim() != 4 || (q.scalar_type() != at::kBFloat16 && q.scalar_type() != at::kFloat)) return false;
+  const int64_t B = q.size(0), Hq = q.size(1), T = q.size(2), D = q.size(3), Hkv = c.in[1].size(1);
+  if (Hkv < 1 || Hq % Hkv || (D != 16 && D != 32 && D != 64 && D != 128) || ints[0] < 16 || T > INT32_MAX) return false;
+  c.d.dims = {(int32_t)B, (int32_t)Hq, (int32_t)Hkv, (int32_t)T, (int32_t)D,
+              q.scalar_type() == at::kBFloat16 ? NSA_DTYPE_BF16 : NSA_DTYPE_F32};
+  c.d.block_size = ints[0]; c.d.n_sel = ints[1]; c.d.window = ints[2];
+  c.d.n_init = ints[3]; c.d.n_local = ints[4]; c.d.cmp_len = ints[5]; c.d.cmp_stride = ints[6];
+  c.d.dq_accumulator = ints[7]; c.d.impl = ints[8];
+  c.d.learned = learned; c.d.given_lists = given; c.d.need_grad = 0;
+  if (!learned && (ints[5] != ints[0] || ints[6] != ints[0])) return false;
+  if (given) {
+    const auto s = c.block_idx.sizes();
+    if (s.size() != 4 || s[0] != B || s[1] != Hkv || s[2] != T) return false;
+    c.d.n_sel = (int32_t)s[3];
+  } else if (ints[1] < 1) {
+    return false;
+  }
+  return true;
+}
+bool comp_ok(const Call& c, at::Device dev) {
+  const int64_t n = c.d.cmp_len, D = c.d.dims.D;
+  for (int k = 0; k < 6; ++k)
+    if (!plain(c.comp[k], at::kFloat, dev) || c.comp[k].numel() != (k % 3 == 0 ? n * D : k % 3 == 1 ? n : D * D)) return false;
+  return true;
+}
+
+NsaAttentionTensors pointers(const Tensor* in, const Tensor* comp, const Tensor& block_idx, bool learned) {
+  NsaAttentionTensors t = {};
+  const void** p[8] = {&t.q, &t.kc, &t.vc, &t.ks, &t.vs, &t.kw, &t.vw, &t.gate};
+  for (int k = 0; k < 8; ++k) *p[k] = in[k].data_ptr();
+  for (int k = 0; k < 6 && learned; ++k) t.comp[k] = comp[k].data_ptr<float>();
+  t.block_idx = block_idx.data_ptr<int32_t>();
+  return t;
+}
+
+// out; `saved` keeps what backward reads.  Makes c.block_idx where the scorer writes it.
+Tensor op_forward(Call& c, bool need_grad, Tensor* saved) {
+  const Tensor& q = c.in[0];
+  c.d.need_grad = need_grad;
+  if (!c.d.given_lists) c.block_idx = at::empty({c.d.dims.B, c.d.dims.Hkv, c.d.dims.T, c.d.n_sel}, q.options().dtype(at::kInt));
+  size_t keep, fwd, bwd;
+  check(nsa_attention_sizes(&c.d, &keep, &fwd, &bwd));
+  Tensor out = at::empty(q.sizes(), q.options());
+  Tensor mem = bytes_like(keep + (need_grad ? 0 : fwd) + 1, q), ws;
+  void* ws_ptr = (char*)mem.data_ptr() + keep;
+  if (need_grad && fwd) {
+    ws = bytes_like(fwd, q);
+    ws_ptr = ws.data_ptr();
+  }
+  NsaAttentionTensors t = pointers(c.in, c.comp, c.block_idx, c.d.learned);
+  t.out = out.data_ptr();
+  check(nsa_attention_fwd(&c.d, &t, mem.data_ptr(), ws_ptr, fwd, raw_stream(q)));
+  *saved = mem;
+  return out;
+}
+
+// d_in: the eight gradients, allocated by the caller
+void op_backward(const NsaAttentionDesc& d, const Tensor* in, const Tensor* comp, const Tensor& block_idx, const Tensor& saved,
+                 const Tensor& d_out, const Tensor* d_in, Tensor* d_comp) {
+  size_t keep, fwd, bwd;
+  check(nsa_attention_sizes(&d, &keep, &fwd, &bwd));
+  NsaAttentionTensors t = pointers(in, comp, block_idx, d.learned);
+  t.d_out = d_out.data_ptr();
+  void** p[8] = {&t.dq, &t.dkc, &t.dvc, &t.dks, &t.dvs, &t.dkw, &t.dvw, &t.d_gate};
+  for (int k = 0; k < 8; ++k) *p[k] = d_in[k].data_ptr();
+  for (int k = 0; k < 6 && d.learned; ++k) {
+    d_comp[k] = at::empty_like(comp[k]);
+    t.d_comp[k] = d_comp[k].data_ptr<float>();
+  }
+  Tensor ws = bytes_like(bwd + 1, d_out);
+  check(nsa_attention_bwd(&d, &t, saved.data_ptr(), ws.data_ptr(), bwd, raw_stream(d_out)));
+}
+
+// A descriptor travels to the backward as a list of integers.
+std::vector<int64_t> pack(const NsaAttentionDesc& d) {
+  const int32_t* p = reinterpret_cast<const int32_t*>(&d);
+  return std::vector<int64_t>(p, p + sizeof(d) / sizeof(int32_t));
+}
+NsaAttentionDesc unpack(AutogradContext* ctx) {
+  NsaAttentionDesc d;
+  const auto v = ctx->saved_data["desc"].toIntVector();
+  for (size_t k = 0; k < v.size(); ++k) reinterpret_cast<int32_t*>(&d)[k] = (int32_t)v[k];
+  return d;
+}
+// what a saved-tensor hook gave back may lie anywhere
+Tensor aligned(const Tensor& t) {
+  const Tensor c = t.contiguous();
+  return (reinterpret_cast<uintptr_t>(c.data_ptr()) & 15) ? c.clone() : c;
+}
+
+// ---- the whole op -------------------------------------------------------------------------------------
+struct OpNode {
+  template <typename... A>
+  static Tensor run(AutogradContext* ctx, Call* c, const A&...) {
+    Tensor saved;
+    Tensor out = op_forward(*c, true, &saved);
+    variable_list keep(c->in, c->in + 8);
+    keep.push_back(c->block_idx);
+    keep.push_back(saved);
+    if (c->d.learned) keep.insert(keep.end(), c->comp, c->comp + 6);
+    ctx->save_for_backward(std::move(keep));
+    ctx->saved_data["desc"] = pack(c->d);
+    ctx->set_materialize_grads(false);
+    return out;
+  }
+  static variable_list grads(AutogradContext* ctx, const variable_list& g) {
+    const NsaAttentionDesc d = unpack(ctx);
+    const int n = d.learned ? 14 : 8;
+    variable_list res(1 + n);                   // the call structure has no gradient
+    if (!g[0].defined()) return res;
+    variable_list kept = ctx->get_saved_variables();
+    for (Tensor& t : kept) t = aligned(t);
+    TORCH_CHECK(g[0].device() == kept[9].device(), "libnsa_b200: tensors on different devices");
+    TORCH_CHECK(g[0].scalar_type() == kept[0].scalar_type(), "libnsa_b200: the gradient's type is not the output's");
+    const Tensor d_out = aligned(g[0]);
+    Tensor d_in[8], d_comp[6];
+    for (int k = 0; k < 8; ++k) d_in[k] = at::empty_like(kept[k]);
+    op_backward(d, kept.data(), kept.data() + 10, kept[8], kept[9], d_out, d_in, d_comp);
+    for (int k = 0; k < 8; ++k) res[1 + k] = d_in[k];
+    for (int k = 8; k < n; ++k) res[1 + k] = d_comp[k - 8];
+    return res;
+  }
+};
+struct OpMean : torch::autograd::Function<OpMean> {
+  static Tensor forward(AutogradContext* ctx, Call* c, const Tensor& q, const Tensor& kc, const Tensor& vc, const Tensor& ks,
+                        const Tensor& vs, const Tensor& kw, const Tensor& vw, const Tensor& gate) {
+    return OpNode::run(ctx, c);
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list g) { return OpNode::grads(ctx, g); }
+};
+struct OpLearned : torch::autograd::Function<OpLearned> {
+  static Tensor forward(AutogradContext* ctx, Call* c, const Tensor& q, const Tensor& kc, const Tensor& vc, const Tensor& ks,
+                        const Tensor& vs, const Tensor& kw, const Tensor& vw, const Tensor& gate, const Tensor& c0,
+                        const Tensor& c1, const Tensor& c2, const Tensor& c3, const Tensor& c4, const Tensor& c5) {
+    return OpNode::run(ctx, c);
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list g) { return OpNode::grads(ctx, g); }
+};
+
+bool tensor_arg(PyObject* o, Tensor* t) {
+  if (!THPVariable_CheckExact(o)) return false;
+  *t = THPVariable_Unpack(o);
+  return true;
+}
+bool int_args(PyObject* const* a, int n, int* out) {
+  for (int k = 0; k < n; ++k) {
+    const long v = PyLong_AsLong(a[k]);
+    if (v == -1 && PyErr_Occurred()) { PyErr_Clear(); return false; }
+    if (v < INT32_MIN || v > INT32_MAX) return false;
+    out[k] = (int)v;
+  }
+  return true;
+}
+PyObject* none() { Py_RETURN_NONE; }
+
+// op(q, kc, vc, ks, vs, kw, vw, gate, block_idx | None, compressor tuple | None, block_size, n_sel, window, n_init,
+//    n_local, cmp_len, cmp_stride, dq_accumulator, impl) -> (out, block_idx), or None where the call is not plain
+PyObject* py_op(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  if (n != 19 || !plain_state()) return none();
+  Call c;
+  for (int k = 0; k < 8; ++k)
+    if (!tensor_arg(a[k], &c.in[k])) return none();
+  const bool given = a[8] != Py_None, learned = a[9] != Py_None;
+  if (given && !tensor_arg(a[8], &c.block_idx)) return none();
+  if (learned) {
+    if (!PyTuple_Check(a[9]) || PyTuple_GET_SIZE(a[9]) != 6) return none();
+    for (int k = 0; k < 6; ++k)
+      if (!tensor_arg(PyTuple_GET_ITEM(a[9], k), &c.comp[k])) return none();
+  }
+  int ints[9];
+  if (!int_args(a + 10, 9, ints)) return none();
+  const Tensor& q = c.in[0];
+  if (!q.defined() || !q.is_cuda() || q.device().index() != c10::cuda::current_device()) return none();
+  for (int k = 0; k < 8; ++k)
+    if (!plain(c.in[k], q.scalar_type(), q.device())) return none();
+  if (given && !(c.block_idx.device() == q.device() && c.block_idx.scalar_type() == at::kInt && c.block_idx.is_contiguous())) return none();
+  if (!fill_desc(c, ints, learned, given)) return none();
+  const NsaDims& m = c.d.dims;
+  for (int k = 1; k < 7; ++k)
+    if (c.in[k].sizes() != at::IntArrayRef({m.B, m.Hkv, m.T, m.D})) return none();
+  if (c.in[7].sizes() != at::IntArrayRef({m.B, m.Hq, m.T, 3})) return none();
+  if (learned && !comp_ok(c, q.device())) return none();
+  bool need = false;
+  if (at::GradMode::is_enabled()) {
+    for (const Tensor& t : c.in) need |= t.requires_grad();
+    for (int k = 0; k < 6 && learned; ++k) need |= c.comp[k].requires_grad();
+  }
+  Tensor out;
+  {
+    pybind11::gil_scoped_release no_gil;
+    if (!need) {
+      Tensor saved;
+      at::NoGradGuard no_grad;
+      out = op_forward(c, false, &saved);
+    } else if (learned) {
+      out = OpLearned::apply(&c, c.in[0], c.in[1], c.in[2], c.in[3], c.in[4], c.in[5], c.in[6], c.in[7], c.comp[0], c.comp[1],
+                             c.comp[2], c.comp[3], c.comp[4], c.comp[5]);
+    } else {
+      out = OpMean::apply(&c, c.in[0], c.in[1], c.in[2], c.in[3], c.in[4], c.in[5], c.in[6], c.in[7]);
+    }
+  }
+  PyObject* o = THPVariable_Wrap(out);
+  if (!o) return nullptr;
+  PyObject* idx = given ? (Py_INCREF(a[8]), a[8]) : THPVariable_Wrap(c.block_idx);
+  if (!idx) { Py_DECREF(o); return nullptr; }
+  PyObject* res = PyTuple_Pack(2, o, idx);
+  Py_DECREF(o);
+  Py_DECREF(idx);
+  return res;
+  END_HANDLE_TH_ERRORS
+}
+
+PyObject* py_set_error(PyObject*, PyObject* cls) {
+  Py_INCREF(cls);
+  g_error = cls;
+  return none();
+}
+
+PyMethodDef kMethods[] = {
+    {"op", (PyCFunction)(void (*)(void))py_op, METH_FASTCALL, "whole op, or None where the call is not plain"},
+    {"set_error", py_set_error, METH_O, "exception class of failed library calls"},
+    {nullptr, nullptr, 0, nullptr}};
+PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_nsa_torch", nullptr, -1, kMethods};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__nsa_torch() { return PyModule_Create(&kModule); }

@@ -696,14 +696,19 @@ def _op_in_parts(q, kv, gate_logits, block_idx, block_size, n_sel, window, force
 
 
 def _op(q, kv, gate_logits, block_idx, block_size, n_sel, window, forced, comp):
-    """The whole op: through the autograd node where a gradient is asked for, and inside a forward-mode
-    level, where the node refuses a tangent that the bare call would drop.  The bare call spares a short
-    forward 9 us of 66 (512 tokens, 16 heads)."""
+    """The whole op.  The usual form of a call goes to the node in C++ (csrc/torch_op.cpp, which says what that form is);
+    every other one through the Python node where a gradient is asked for, and inside a forward-mode level,
+    where the node refuses a tangent that the bare call would drop."""
     kc, vc, ks, vs, kw, vw = kv
+    dual = getattr(forward_ad, "_current_level", 0) >= 0
+    if not dual and not L.CHECK_STATUS_EVERY_CALL and torch._C._get_tracing_state() is None:
+        res = L.torch_op().op(q, kc, vc, ks, vs, kw, vw, gate_logits, block_idx, comp, block_size, n_sel, window, *forced,
+                              int(_dq_accumulator), L.IMPL[_impl])
+        if res is not None:
+            return res
     if not (kc.shape == vc.shape == ks.shape == vs.shape == kw.shape == vw.shape and kc.shape[2] == q.shape[2]):
         return _op_in_parts(q, kv, gate_logits, block_idx, block_size, n_sel, window, forced, comp)
-    if (torch.is_grad_enabled() and any(t.requires_grad for t in (q, *kv, gate_logits, *(comp or ())))) or (
-            getattr(forward_ad, "_current_level", 0) >= 0):
+    if (torch.is_grad_enabled() and any(t.requires_grad for t in (q, *kv, gate_logits, *(comp or ())))) or dual:
         return _NSAAttention.apply(q, *kv, gate_logits, block_size, n_sel, window, block_idx, forced, *(comp or ()))
     return _op_forward(q, kv, gate_logits, block_idx, block_size, n_sel, window, forced, comp, False)[:2]
 
