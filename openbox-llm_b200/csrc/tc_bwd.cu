@@ -1520,6 +1520,7 @@ static const char* const kRedNames[3] = {"dq_reduce_win", "dq_reduce_cmp", "dq_r
 struct BwdPlan {
   int n_ktiles, n_slots, nq, n_splits, split_chunk;
   int csize;                 // CTAs that share the row tiles of one key tile
+  bool sel_split;            // selection: a key tile that every query lists would be more than one work item
   size_t off_acc;
   size_t cap_pairs;          // selection: pairs the CSR may hold
   SelPlanLayout layout;      // selection
@@ -1582,8 +1583,10 @@ static BwdPlan plan_bwd(const AttnArgs& a) {
       off += 2 * align_up((size_t)a.B * a.Hkv * a.Lk * a.D * sizeof(float), 256);
     }
   }
-  // selection: blocks split over several work items use the same accumulators
-  if (a.kind == 2) off += 2 * align_up((size_t)a.B * a.Hkv * a.Lk * a.D * sizeof(float), 256);
+  // selection: blocks split over several work items use the same accumulators (launches and memory that up to
+  // kSelChunkTiles row tiles of queries, 4096 tokens at groups of 4, a call does without)
+  pl.sel_split = a.kind == 2 && max_rt > kSelChunkTiles;
+  if (pl.sel_split) off += 2 * align_up((size_t)a.B * a.Hkv * a.Lk * a.D * sizeof(float), 256);
   pl.total = off;
   return pl;
 }
@@ -1652,6 +1655,8 @@ int tc_attn_bwd(const AttnArgs& a, void* ws, size_t ws_bytes, cudaStream_t st) {
                                   pl.cap_pairs * sizeof(int32_t), cudaMemcpyDeviceToDevice, st));
     }
     p.plan = sel_plan_at(plan_mem, pl.layout);
+  }
+  if (pl.sel_split) {
     KernelScope ks("sel_split_blocks_kernel", st);
     sel_split_blocks_kernel<<<dim3(pl.n_ktiles, a.B * a.Hkv), 256, 0, st>>>(p.plan.offsets, p.dk_acc, p.dv_acc, p.dk, p.dv,
                                                                         pl.n_ktiles, pl.nq, a.Lk, a.D, 0);
@@ -1720,7 +1725,7 @@ int tc_attn_bwd(const AttnArgs& a, void* ws, size_t ws_bytes, cudaStream_t st) {
     tc_bwd_kernel<64><<<grid, 512, smem, st>>>(tm_k, tm_v, tm_q_run, tm_do_run, tm_dq, tm_dqacc, p);
   }
   NSA_LAUNCH_OK("tc_bwd_kernel");
-  if (a.kind == 2) {
+  if (pl.sel_split) {
     KernelScope ks("sel_split_blocks_kernel", st);
     sel_split_blocks_kernel<<<dim3(pl.n_ktiles, a.B * a.Hkv), 256, 0, st>>>(p.plan.offsets, p.dk_acc, p.dv_acc, p.dk, p.dv,
                                                                         pl.n_ktiles, pl.nq, a.Lk, a.D, 1);
