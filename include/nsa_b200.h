@@ -309,6 +309,16 @@ int nsa_merge_heads(const void* dq, const void* dkv, const void* dgate, void* dy
 int nsa_swap_heads_tokens(const void* src, void* dst, int B, int H, int T, int D, int dtype, int to_tokens,
                           void* stream);
 
+/* fp32 -> bf16 (round to nearest) of up to NSA_MAX_CAST_SEGMENTS arrays of n elements in one launch; a null src writes
+ * zeros.  What a layer's projection GEMMs read under bf16 autocast: x and the weights. */
+#define NSA_MAX_CAST_SEGMENTS 16
+typedef struct NsaCastSegment {
+  const float* src;
+  void* dst;
+  size_t n;
+} NsaCastSegment;
+int nsa_cast_bf16_segments(const NsaCastSegment* segs, int n, void* stream);
+
 /* ---- gate combine ---------------------------------------------------------------------------
  * Replaces the sigmoid blend nsa_model.py:366-368 / nsa_fused_kernel.py:572-573 and its
  * autograd backward: out = sum_i sigmoid(gate[...,i]) * o_i; d_gate is float32-accumulated

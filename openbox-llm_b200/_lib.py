@@ -90,6 +90,7 @@ SIGNATURES = {
     "nsa_split_heads": (_i, [_vp] * 4 + [_i] * 6 + [_vp]),
     "nsa_merge_heads": (_i, [_vp] * 4 + [_i] * 6 + [_vp]),
     "nsa_swap_heads_tokens": (_i, [_vp, _vp] + [_i] * 6 + [_vp]),
+    "nsa_cast_bf16_segments": (_i, [_vp, _i, _vp]),
     "nsa_gate_combine_fwd": (_i, [_vp] * 5 + [_dp, _vp]),
     "nsa_gate_combine_bwd": (_i, [_vp] * 9 + [_dp, _vp]),
 }

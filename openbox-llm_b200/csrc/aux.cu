@@ -1071,8 +1071,57 @@ __global__ void swap_heads_tokens_kernel(const V* __restrict__ src, V* __restric
   }
   dst[i] = __ldg(src + s);
 }
+
+// fp32 arrays -> bf16, several in one launch: what the projection GEMMs of a layer read (x, the eight weights one behind
+// the other, the bias row, out_proj's weight).  A thread takes 8 elements of one array; an array without a source is
+// filled with zeros.  Bound by the pass over x at training sizes, by launches at small ones, where torch's two
+// concatenations, fills and three casts were seven kernels.
+struct CastSegs {
+  NsaCastSegment s[NSA_MAX_CAST_SEGMENTS];
+  size_t first[NSA_MAX_CAST_SEGMENTS + 1];       // first item (of 8 elements) of a segment
+  int n;
+};
+__global__ void __launch_bounds__(256) cast_segments_kernel(const __grid_constant__ CastSegs c) {
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= c.first[c.n]) return;
+  int k = 0;
+  while (i >= c.first[k + 1]) ++k;
+  const NsaCastSegment& s = c.s[k];
+  const size_t e0 = (i - c.first[k]) * 8;
+  const float* src = s.src + e0;
+  __nv_bfloat16* dst = (__nv_bfloat16*)s.dst + e0;
+  if (e0 + 8 <= s.n && ((((uintptr_t)s.src | (uintptr_t)s.dst) & 15) == 0)) {
+    float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+    if (s.src) {
+      a = __ldcs(reinterpret_cast<const float4*>(src));
+      b = __ldcs(reinterpret_cast<const float4*>(src) + 1);
+    }
+    __nv_bfloat162 h[4] = {__floats2bfloat162_rn(a.x, a.y), __floats2bfloat162_rn(a.z, a.w), __floats2bfloat162_rn(b.x, b.y),
+                           __floats2bfloat162_rn(b.z, b.w)};
+    *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(h);
+  } else {
+    for (size_t e = 0; e < 8 && e0 + e < s.n; ++e) dst[e] = __float2bfloat16_rn(s.src ? src[e] : 0.f);
+  }
+}
 }  // namespace
 }  // namespace nsa
+
+extern "C" int nsa_cast_bf16_segments(const NsaCastSegment* segs, int n, void* stream) {
+  NSA_CHECK_ARG(segs && n >= 0 && n <= NSA_MAX_CAST_SEGMENTS, "bad segments");
+  CastSegs c;
+  c.n = n;
+  c.first[0] = 0;
+  for (int k = 0; k < n; ++k) {
+    NSA_CHECK_ARG(segs[k].n == 0 || segs[k].dst, "null destination");
+    c.s[k] = segs[k];
+    c.first[k + 1] = c.first[k] + (segs[k].n + 7) / 8;
+  }
+  if (c.first[n] == 0) return NSA_OK;
+  KernelScope ks("cast_segments_kernel", (cudaStream_t)stream);
+  cast_segments_kernel<<<blocks_for(c.first[n], 256), 256, 0, (cudaStream_t)stream>>>(c);
+  NSA_LAUNCH_OK("cast_segments_kernel");
+  return NSA_OK;
+}
 
 extern "C" int nsa_fused_projection_width(int Hq, int Hkv, int D) {
   return (Hq + 6 * Hkv) * D + (3 * Hq + 7) / 8 * 8;

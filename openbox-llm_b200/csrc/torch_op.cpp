@@ -60,13 +60,11 @@ struct Call {
 };
 
 // Sizes that belong together; what is refused here gets its message from the Python side.
-bool fill_desc(Call& c, const int* ints, bool learned, bool given) {
-  const Tensor& q = c.in[0];
-  if (q.dim() != 4 || c.in[1].dim() != 4 || (q.scalar_type() != at::kBFloat16 && q.scalar_type() != at::kFloat)) return false;
-  const int64_t B = q.size(0), Hq = q.size(1), T = q.size(2), D = q.size(3), Hkv = c.in[1].size(1);
-  if (Hkv < 1 || Hq % Hkv || (D != 16 && D != 32 && D != 64 && D != 128) || ints[0] < 16 || T > INT32_MAX) return false;
+bool fill_desc(Call& c, int64_t B, int64_t Hq, int64_t Hkv, int64_t T, int64_t D, at::ScalarType dtype, const int* ints,
+               bool learned, bool given) {
+  if ((dtype != at::kBFloat16 && dtype != at::kFloat) || Hkv < 1 || Hq % Hkv || (D != 16 && D != 32 && D != 64 && D != 128) || ints[0] < 16 || T > INT32_MAX) return false;
   c.d.dims = {(int32_t)B, (int32_t)Hq, (int32_t)Hkv, (int32_t)T, (int32_t)D,
-              q.scalar_type() == at::kBFloat16 ? NSA_DTYPE_BF16 : NSA_DTYPE_F32};
+              dtype == at::kBFloat16 ? NSA_DTYPE_BF16 : NSA_DTYPE_F32};
   c.d.block_size = ints[0]; c.d.n_sel = ints[1]; c.d.window = ints[2];
   c.d.n_init = ints[3]; c.d.n_local = ints[4]; c.d.cmp_len = ints[5]; c.d.cmp_stride = ints[6];
   c.d.dq_accumulator = ints[7]; c.d.impl = ints[8];
@@ -201,6 +199,119 @@ struct OpLearned : torch::autograd::Function<OpLearned> {
   static variable_list backward(AutogradContext* ctx, variable_list g) { return OpNode::grads(ctx, g); }
 };
 
+// ---- the layer under bf16 autocast: projections, op and out_proj in one node ----------------------------
+// One launch casts x and the nine weights, laid out as the GEMMs read them; the gradients of x and the
+// weights leave their GEMMs in fp32, the K / V gradients of the six branches land in one buffer and the bias
+// row is summed over its own columns.  In place of torch's nodes and modules: 8 x 4096 tokens, 12 heads
+// of 64, forward + backward 3165 -> 2984 us; 256 tokens, forward, 271 -> 94.
+struct Layer {
+  Call c;
+  Tensor x, w[8], bias, w_out;
+  int64_t B, T, dm, width, n_attn;
+};
+struct LayerNode : torch::autograd::Function<LayerNode> {
+  static Tensor run(Layer& l, bool need_grad, variable_list* keep) {
+    const NsaDims& m = l.c.d.dims;
+    const auto opt = l.x.options().dtype(at::kBFloat16);
+    const int64_t rows = l.B * l.T, hd = (int64_t)m.Hq * m.D;
+    Tensor xb = l.x.scalar_type() == at::kBFloat16 ? l.x.view({rows, l.dm}) : at::empty({rows, l.dm}, opt);
+    Tensor w = at::empty({l.width, l.dm}, opt), bias = at::empty({l.width}, opt), w_out = at::empty({l.dm, hd}, opt);
+    NsaCastSegment s[NSA_MAX_CAST_SEGMENTS];
+    int n = 0;
+    auto seg = [&](const float* src, void* dst, int64_t e) { s[n++] = NsaCastSegment{src, dst, (size_t)e}; };
+    if (l.x.scalar_type() == at::kFloat) seg(l.x.data_ptr<float>(), xb.data_ptr(), xb.numel());
+    char* at_w = (char*)w.data_ptr();
+    int64_t row = 0;
+    for (int k = 0; k < 8; ++k) {
+      seg(l.w[k].data_ptr<float>(), at_w + row * l.dm * 2, l.w[k].numel());
+      row += l.w[k].size(0);
+    }
+    seg(nullptr, at_w + row * l.dm * 2, (l.width - row) * l.dm);
+    char* at_b = (char*)bias.data_ptr();
+    seg(nullptr, at_b, l.n_attn);
+    seg(l.bias.data_ptr<float>(), at_b + l.n_attn * 2, l.bias.numel());
+    seg(nullptr, at_b + row * 2, l.width - row);
+    seg(l.w_out.data_ptr<float>(), w_out.data_ptr(), w_out.numel());
+    check(nsa_cast_bf16_segments(s, n, raw_stream(l.x)));
+    Tensor y = at::addmm(bias, xb, w.t());
+    Call& c = l.c;
+    c.in[0] = at::empty({m.B, m.Hq, m.T, m.D}, opt);
+    Tensor kv = at::empty({6, m.B, m.Hkv, m.T, m.D}, opt);
+    c.in[7] = at::empty({m.B, m.Hq, m.T, 3}, opt);
+    for (int k = 0; k < 6; ++k) c.in[1 + k] = kv.select(0, k);
+    check(nsa_split_heads(y.data_ptr(), c.in[0].data_ptr(), kv.data_ptr(), c.in[7].data_ptr(), m.B, m.T, m.Hq, m.Hkv, m.D,
+                          NSA_DTYPE_BF16, raw_stream(l.x)));
+    Tensor saved;
+    Tensor o = op_forward(c, need_grad, &saved);
+    Tensor tokens = at::empty({rows, hd}, opt);
+    check(nsa_swap_heads_tokens(o.data_ptr(), tokens.data_ptr(), m.B, m.Hq, m.T, m.D, NSA_DTYPE_BF16, 1, raw_stream(l.x)));
+    Tensor out = at::mm(tokens, w_out.t()).view({l.B, l.T, l.dm});
+    if (keep) {
+      *keep = {c.in[0], kv, c.in[7], c.block_idx, saved, xb, w, w_out, tokens};
+      keep->insert(keep->end(), c.comp, c.comp + 6);
+    }
+    return out;
+  }
+  static Tensor forward(AutogradContext* ctx, Layer* l, const Tensor& x, const Tensor& w0, const Tensor& w1, const Tensor& w2,
+                        const Tensor& w3, const Tensor& w4, const Tensor& w5, const Tensor& w6, const Tensor& w7,
+                        const Tensor& bias, const Tensor& w_out, const Tensor& c0, const Tensor& c1, const Tensor& c2,
+                        const Tensor& c3, const Tensor& c4, const Tensor& c5) {
+    variable_list keep;
+    Tensor out = run(*l, true, &keep);
+    ctx->save_for_backward(std::move(keep));
+    ctx->saved_data["desc"] = pack(l->c.d);
+    ctx->saved_data["x_bf16"] = x.scalar_type() == at::kBFloat16;
+    ctx->set_materialize_grads(false);
+    return out;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list g) {
+    c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::autocast_dispatch_keyset);
+    variable_list res(18);                      // l, x, w[8], bias, w_out, comp[6]
+    if (!g[0].defined()) return res;
+    const NsaAttentionDesc d = unpack(ctx);
+    const NsaDims& m = d.dims;
+    variable_list kept = ctx->get_saved_variables();
+    for (Tensor& t : kept) t = aligned(t);
+    const Tensor &kv = kept[1], &xb = kept[5], &w = kept[6], &w_out = kept[7], &tokens = kept[8];
+    Tensor in[8];
+    in[0] = kept[0];
+    in[7] = kept[2];
+    for (int k = 0; k < 6; ++k) in[1 + k] = kv.select(0, k);
+    const int64_t rows = (int64_t)m.B * m.T, hd = (int64_t)m.Hq * m.D, dm = xb.size(1), width = w.size(0);
+    const auto opt = xb.options();
+    const Tensor dy = aligned(g[0].to(at::kBFloat16)).view({rows, dm});
+    if (ctx->needs_input_grad(10)) res[11] = at::mm(dy.t(), tokens, at::kFloat);
+    Tensor d_tokens = at::mm(dy, w_out), d_out = at::empty({m.B, m.Hq, m.T, m.D}, opt);
+    check(nsa_swap_heads_tokens(d_tokens.data_ptr(), d_out.data_ptr(), m.B, m.Hq, m.T, m.D, NSA_DTYPE_BF16, 0, raw_stream(dy)));
+    Tensor d_in[8], d_comp[6], d_kv = at::empty_like(kv);
+    d_in[0] = at::empty_like(in[0]);
+    d_in[7] = at::empty_like(in[7]);
+    for (int k = 0; k < 6; ++k) d_in[1 + k] = d_kv.select(0, k);
+    op_backward(d, in, kept.data() + 9, kept[3], kept[4], d_out, d_in, d_comp);
+    Tensor d_rows = at::empty({rows, width}, opt);
+    check(nsa_merge_heads(d_in[0].data_ptr(), d_kv.data_ptr(), d_in[7].data_ptr(), d_rows.data_ptr(), m.B, m.T, m.Hq, m.Hkv, m.D,
+                          NSA_DTYPE_BF16, raw_stream(dy)));
+    if (ctx->needs_input_grad(0)) {
+      Tensor dx = ctx->saved_data["x_bf16"].toBool() ? at::mm(d_rows, w) : at::mm(d_rows, w, at::kFloat);
+      res[1] = dx.view({m.B, m.T, dm});
+    }
+    bool any = false;
+    for (int k = 0; k < 8; ++k) any |= ctx->needs_input_grad(1 + k);
+    if (any) {
+      const Tensor dw = at::mm(d_rows.t(), xb, at::kFloat);
+      int64_t row = 0;
+      for (int k = 0; k < 8; ++k) {
+        const int64_t n = k == 0 ? hd : k < 7 ? (int64_t)m.Hkv * m.D : 3 * m.Hq;
+        res[2 + k] = dw.narrow(0, row, n);
+        row += n;
+      }
+    }
+    if (ctx->needs_input_grad(9)) res[10] = d_rows.narrow(1, hd + 6 * (int64_t)m.Hkv * m.D, 3 * m.Hq).sum({0}, false, at::kFloat);
+    for (int k = 0; k < 6; ++k) res[12 + k] = d_comp[k];
+    return res;
+  }
+};
+
 bool tensor_arg(PyObject* o, Tensor* t) {
   if (!THPVariable_CheckExact(o)) return false;
   *t = THPVariable_Unpack(o);
@@ -239,7 +350,9 @@ PyObject* py_op(PyObject*, PyObject* const* a, Py_ssize_t n) {
   for (int k = 0; k < 8; ++k)
     if (!plain(c.in[k], q.scalar_type(), q.device())) return none();
   if (given && !(c.block_idx.device() == q.device() && c.block_idx.scalar_type() == at::kInt && c.block_idx.is_contiguous())) return none();
-  if (!fill_desc(c, ints, learned, given)) return none();
+  if (q.dim() != 4 || c.in[1].dim() != 4 ||
+      !fill_desc(c, q.size(0), q.size(1), c.in[1].size(1), q.size(2), q.size(3), q.scalar_type(), ints, learned, given))
+    return none();
   const NsaDims& m = c.d.dims;
   for (int k = 1; k < 7; ++k)
     if (c.in[k].sizes() != at::IntArrayRef({m.B, m.Hkv, m.T, m.D})) return none();
@@ -275,6 +388,64 @@ PyObject* py_op(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
+// layer(x, (q, kc, vc, ks, vs, kw, vw, gate weights), gate bias, out weight, compressor tuple, block_idx | None, Hq, Hkv,
+//       then the integers of op()) -> y, or None where the call is not plain
+PyObject* py_layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  if (n != 17 || !plain_state()) return none();
+  Layer l;
+  Call& c = l.c;
+  if (!tensor_arg(a[0], &l.x) || !PyTuple_Check(a[1]) || PyTuple_GET_SIZE(a[1]) != 8 || !PyTuple_Check(a[4]) ||
+      PyTuple_GET_SIZE(a[4]) != 6 || !tensor_arg(a[2], &l.bias) || !tensor_arg(a[3], &l.w_out))
+    return none();
+  for (int k = 0; k < 8; ++k)
+    if (!tensor_arg(PyTuple_GET_ITEM(a[1], k), &l.w[k])) return none();
+  for (int k = 0; k < 6; ++k)
+    if (!tensor_arg(PyTuple_GET_ITEM(a[4], k), &c.comp[k])) return none();
+  const bool given = a[5] != Py_None;
+  if (given && !tensor_arg(a[5], &c.block_idx)) return none();
+  int ints[11];
+  if (!int_args(a + 6, 11, ints)) return none();
+  const int64_t Hq = ints[0], Hkv = ints[1];
+  const Tensor& x = l.x;
+  if (!x.defined() || !x.is_cuda() || x.device().index() != c10::cuda::current_device() || x.dim() != 3 || Hq < 1 || Hkv < 1) return none();
+  const at::Device dev = x.device();
+  l.B = x.size(0); l.T = x.size(1); l.dm = x.size(2);
+  if (!plain(x, x.scalar_type(), dev) || (x.scalar_type() != at::kFloat && x.scalar_type() != at::kBFloat16)) return none();
+  const int64_t D = l.w[0].dim() == 2 ? l.w[0].size(0) / Hq : 0;
+  if (D < 16 || D % 8 || l.dm % 8) return none();
+  l.n_attn = (Hq + 6 * Hkv) * D;
+  l.width = nsa_fused_projection_width((int)Hq, (int)Hkv, (int)D);
+  for (int k = 0; k < 8; ++k) {
+    const int64_t r = k == 0 ? Hq * D : k < 7 ? Hkv * D : 3 * Hq;
+    if (!plain(l.w[k], at::kFloat, dev) || l.w[k].sizes() != at::IntArrayRef({r, l.dm})) return none();
+  }
+  if (!plain(l.bias, at::kFloat, dev) || l.bias.sizes() != at::IntArrayRef({3 * Hq})) return none();
+  if (!plain(l.w_out, at::kFloat, dev) || l.w_out.sizes() != at::IntArrayRef({l.dm, Hq * D})) return none();
+  if (given && !(c.block_idx.device() == dev && c.block_idx.scalar_type() == at::kInt && c.block_idx.is_contiguous())) return none();
+  if (!fill_desc(c, l.B, Hq, Hkv, l.T, D, at::kBFloat16, ints + 2, true, given) || !comp_ok(c, dev)) return none();
+  bool need = false;
+  if (at::GradMode::is_enabled()) {
+    need = x.requires_grad() || l.bias.requires_grad() || l.w_out.requires_grad();
+    for (const Tensor& t : l.w) need |= t.requires_grad();
+    for (const Tensor& t : c.comp) need |= t.requires_grad();
+  }
+  Tensor out;
+  {
+    pybind11::gil_scoped_release no_gil;
+    c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::autocast_dispatch_keyset);
+    if (need) {
+      out = LayerNode::apply(&l, x, l.w[0], l.w[1], l.w[2], l.w[3], l.w[4], l.w[5], l.w[6], l.w[7], l.bias, l.w_out, c.comp[0],
+                             c.comp[1], c.comp[2], c.comp[3], c.comp[4], c.comp[5]);
+    } else {
+      at::NoGradGuard no_grad;
+      out = LayerNode::run(l, false, nullptr);
+    }
+  }
+  return THPVariable_Wrap(out);
+  END_HANDLE_TH_ERRORS
+}
+
 PyObject* py_set_error(PyObject*, PyObject* cls) {
   Py_INCREF(cls);
   g_error = cls;
@@ -283,6 +454,7 @@ PyObject* py_set_error(PyObject*, PyObject* cls) {
 
 PyMethodDef kMethods[] = {
     {"op", (PyCFunction)(void (*)(void))py_op, METH_FASTCALL, "whole op, or None where the call is not plain"},
+    {"layer", (PyCFunction)(void (*)(void))py_layer, METH_FASTCALL, "layer under bf16 autocast, or None where the call is not plain"},
     {"set_error", py_set_error, METH_O, "exception class of failed library calls"},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_nsa_torch", nullptr, -1, kMethods};

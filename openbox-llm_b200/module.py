@@ -10,13 +10,16 @@ gate projection as eight GEMMs, each followed by its own transpose + copy.  Here
 (still eight parameters with the reference's names) are applied as one GEMM, one kernel pass turns
 its rows into the head-major tensors the attention kernels read and one pass brings the output back
 for out_proj; the backward likewise (one pass assembling the gradient rows, one dgrad and one wgrad
-GEMM).  `fused_projection=False` keeps the eight separate projections.
+GEMM).  `fused_projection=False` keeps the eight separate projections.  Under bf16 autocast the layer is one autograd
+node (csrc/torch_op.cpp) around the same passes and GEMMs.
 """
 import torch
 import torch.nn as nn
 import torch.nn.functional as F
+from torch.nn.modules.module import _has_any_global_hook
 
-from .ops import fused_projection_width, heads_to_tokens, nsa_attention, split_heads
+from . import _lib as L
+from .ops import fused_projection_width, heads_to_tokens, nsa_attention, one_node_ok, split_heads, switches
 
 
 class _Compressor(nn.Module):
@@ -62,11 +65,30 @@ class NSAAttentionB200(nn.Module):
         B, T, _ = x.shape
         return x.view(B, T, n_heads, self.dh).transpose(1, 2).contiguous()
 
+    def _one_node(self, x, block_idx):
+        """The layer as one node, where it is what a call of its modules comes to: bf16 autocast, fp32 weights, an
+        out_proj that is a plain Linear without hooks; None where it is not."""
+        o = self.out_proj
+        if not (one_node_ok() and torch.is_autocast_enabled("cuda") and torch.get_autocast_dtype("cuda") is torch.bfloat16
+                and type(o) is nn.Linear and o.bias is None and not _has_any_global_hook()
+                and not (o._forward_hooks or o._forward_pre_hooks or o._backward_hooks or o._backward_pre_hooks)):
+            return None
+        k, v = self.comp_k, self.comp_v
+        return L.torch_op().layer(
+            x, (self.q_proj.weight, self.k_cmp.weight, self.v_cmp.weight, self.k_slc.weight, self.v_slc.weight,
+                self.k_win.weight, self.v_win.weight, self.gate.weight), self.gate.bias, o.weight,
+            (k.intra_pos, k.pool_logits, k.proj.weight, v.intra_pos, v.pool_logits, v.proj.weight), block_idx, self.Hq, self.Hkv,
+            self.block_size, self.n_sel, self.window, self.n_init_blocks, self.n_local_blocks, self.cmp_len, self.cmp_stride,
+            *switches())
+
     def forward(self, x, block_idx=None):
         """x [B,T,d_model] -> [B,T,d_model].  `block_idx` overrides the scorer's pick."""
         B, T, _ = x.shape
         fused = self.fused_projection and x.is_cuda and self.dh % 8 == 0
         if fused:
+            y = self._one_node(x, block_idx)
+            if y is not None:
+                return y
             # one GEMM for the eight projections, one pass to head-major layout
             ws = [p.weight for p in (self.q_proj, self.k_cmp, self.v_cmp, self.k_slc, self.v_slc,
                                      self.k_win, self.v_win, self.gate)]

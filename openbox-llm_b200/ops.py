@@ -695,20 +695,34 @@ def _op_in_parts(q, kv, gate_logits, block_idx, block_size, n_sel, window, force
     return gate_combine(o_cmp, o_slc, window_attn_triton(q, kw, vw, window), gate_logits), block_idx
 
 
+def _dual_level():
+    return getattr(forward_ad, "_current_level", 0) >= 0
+
+
+def one_node_ok():
+    """Whether the nodes in C++ may serve a call: outside of forward-mode levels and traces, and without a look at the
+    device status after every call."""
+    return not _dual_level() and not L.CHECK_STATUS_EVERY_CALL and torch._C._get_tracing_state() is None
+
+
+def switches():
+    """The process-wide choices a call goes by: dQ accumulator, kernel family."""
+    return int(_dq_accumulator), L.IMPL[_impl]
+
+
 def _op(q, kv, gate_logits, block_idx, block_size, n_sel, window, forced, comp):
     """The whole op.  The usual form of a call goes to the node in C++ (csrc/torch_op.cpp, which says what that form is);
     every other one through the Python node where a gradient is asked for, and inside a forward-mode level,
     where the node refuses a tangent that the bare call would drop."""
     kc, vc, ks, vs, kw, vw = kv
-    dual = getattr(forward_ad, "_current_level", 0) >= 0
-    if not dual and not L.CHECK_STATUS_EVERY_CALL and torch._C._get_tracing_state() is None:
+    if one_node_ok():
         res = L.torch_op().op(q, kc, vc, ks, vs, kw, vw, gate_logits, block_idx, comp, block_size, n_sel, window, *forced,
-                              int(_dq_accumulator), L.IMPL[_impl])
+                              *switches())
         if res is not None:
             return res
     if not (kc.shape == vc.shape == ks.shape == vs.shape == kw.shape == vw.shape and kc.shape[2] == q.shape[2]):
         return _op_in_parts(q, kv, gate_logits, block_idx, block_size, n_sel, window, forced, comp)
-    if (torch.is_grad_enabled() and any(t.requires_grad for t in (q, *kv, gate_logits, *(comp or ())))) or dual:
+    if (torch.is_grad_enabled() and any(t.requires_grad for t in (q, *kv, gate_logits, *(comp or ())))) or _dual_level():
         return _NSAAttention.apply(q, *kv, gate_logits, block_size, n_sel, window, block_idx, forced, *(comp or ()))
     return _op_forward(q, kv, gate_logits, block_idx, block_size, n_sel, window, forced, comp, False)[:2]
 
