@@ -452,28 +452,33 @@ template <> struct Vec<float> {
   }
 };
 
+// A warp to a summary: Dv lanes side by side on a token's 16-byte vectors, 32 / Dv tokens at a time, whose sums meet by
+// shuffles.  A thread that walked all tokens of its columns waited for one load chain of 64 in four: 21 us for
+// 2 x 4 x 4096 tokens of 64 bf16, 5 so.
 template <typename T>
-__global__ void mean_fwd_kernel(const PoolSides s, int T_, int Dv, int len, int n_sum, size_t n_out) {
+__global__ void mean_fwd_kernel(const PoolSides s, int T_, int Dv, int len, int n_sum, size_t rows) {
   constexpr int N = Vec<T>::N;
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n_out) return;
-  const int d = (int)(i % Dv);
-  const size_t row = i / Dv;
+  const size_t row = (size_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (row >= rows) return;
+  const int lane = threadIdx.x & 31, d = lane & (Dv - 1), step = 32 / Dv;      // Dv: a power of two up to 32
   const size_t bh = row / n_sum, j = row % n_sum;
   const uint4* p = reinterpret_cast<const uint4*>(s.x[blockIdx.y]) + (bh * T_ + j * len) * Dv + d;
   float a[N];
 #pragma unroll
   for (int e = 0; e < N; ++e) a[e] = 0.f;
-#pragma unroll 16
-  for (int r = 0; r < len; ++r) {
+#pragma unroll 8
+  for (int r = lane / Dv; r < len; r += step) {
     float f[N];
     Vec<T>::unpack(__ldg(p + (size_t)r * Dv), f);
 #pragma unroll
     for (int e = 0; e < N; ++e) a[e] += f[e];
   }
+  for (int o = Dv; o < 32; o <<= 1)
+#pragma unroll
+    for (int e = 0; e < N; ++e) a[e] += __shfl_xor_sync(0xffffffffu, a[e], o);
 #pragma unroll
   for (int e = 0; e < N; ++e) a[e] /= (float)len;
-  reinterpret_cast<uint4*>(s.out[blockIdx.y])[i] = Vec<T>::pack(a);
+  if (lane < Dv) reinterpret_cast<uint4*>(s.out[blockIdx.y])[row * Dv + d] = Vec<T>::pack(a);
 }
 
 template <typename T>
@@ -595,11 +600,10 @@ int pool_mean_fwd(const PoolSides& s, int B, int H, int T, int D, int len, int d
   const size_t rows = (size_t)B * H * n_sum;
   if (rows == 0) return NSA_OK;
   const int Dv = dtype == NSA_DTYPE_BF16 ? D / 8 : D / 4;
-  const size_t n = rows * Dv;
   KernelScope ks("mean_pool_fwd_kernel", st);
-  const dim3 grid((unsigned)((n + 63) / 64), s.n);
-  if (dtype == NSA_DTYPE_BF16) mean_fwd_kernel<__nv_bfloat16><<<grid, 64, 0, st>>>(s, T, Dv, len, n_sum, n);
-  else mean_fwd_kernel<float><<<grid, 64, 0, st>>>(s, T, Dv, len, n_sum, n);
+  const dim3 grid((unsigned)((rows + 3) / 4), s.n);
+  if (dtype == NSA_DTYPE_BF16) mean_fwd_kernel<__nv_bfloat16><<<grid, 128, 0, st>>>(s, T, Dv, len, n_sum, rows);
+  else mean_fwd_kernel<float><<<grid, 128, 0, st>>>(s, T, Dv, len, n_sum, rows);
   NSA_LAUNCH_OK("mean_pool_fwd_kernel");
   return NSA_OK;
 }

@@ -1,10 +1,11 @@
-// Builds the index structures of sel_plan.cuh in three launches whatever the size: count, scan,
-// fill.  A CTA of the first and the last takes a chunk of consecutive queries of one unit and
+// Builds the index structures of sel_plan.cuh in three launches, count, scan and fill, or in one where the sequence
+// is short.  A CTA of the first and the last takes a chunk of consecutive queries of one unit and
 // marks its list entries in a bitmap [key tile][query] in shared memory, from which ranks are
 // population counts; nothing but the counts and the results touches global memory.  At 16 units of
 // 32768 queries x 16 slots: 0.17 ms, against 0.30 ms and eight launches with the bitmap in global
 // memory (bound by the scattered 4-byte stores of the pairs); at 4 units of 1024 queries 16 us,
 // bound by latency.
+#include "cluster.cuh"
 #include "sel_plan.cuh"
 
 namespace nsa {
@@ -24,10 +25,10 @@ __device__ __forceinline__ int tile_of(int blk, int t, int block_size) {
 // one or two queries, so they fall into different banks.
 __device__ __forceinline__ void mark_chunk(const int32_t* __restrict__ idx, uint32_t* bm, int t0, int n_q, int S,
                                            int block_size, int n_kt, int cw) {
-  for (int i = threadIdx.x; i < n_kt * cw; i += kThreads) bm[i] = 0u;
+  for (int i = threadIdx.x; i < n_kt * cw; i += blockDim.x) bm[i] = 0u;
   __syncthreads();
 #pragma unroll 4
-  for (int e = threadIdx.x; e < n_q * S; e += kThreads) {
+  for (int e = threadIdx.x; e < n_q * S; e += blockDim.x) {
     const int ql = e / S;
     const int j = tile_of(__ldg(idx + e), t0 + ql, block_size);
     if (j >= 0) atomicOr(&bm[(ql >> 5) * n_kt + j], 1u << (ql & 31));
@@ -182,29 +183,12 @@ plan_scan_kernel(int32_t* __restrict__ counts, const int32_t* __restrict__ union
 // kMatch: a query's S entries sit in one warp (S divides 32), so the entries of one query that
 // name the same tile find one another by a warp match instead of reading the list again.
 template <bool kMatch>
-__global__ void __launch_bounds__(kThreads)
-plan_fill_kernel(const int32_t* __restrict__ block_idx, const int32_t* __restrict__ starts,
-                 int32_t* __restrict__ pairs, int32_t* __restrict__ pair_of_slot, SelPlanHeader* __restrict__ hdr, int T, int S,
-                 int block_size, int n_kt, int cw, int n_chunks) {
-  extern __shared__ uint32_t bm[];
-  uint16_t* before = reinterpret_cast<uint16_t*>(bm + n_kt * cw);   // [word][tile]: queries in earlier words
-  const int chunk = blockIdx.x, unit = blockIdx.y;
-  const int t0 = chunk * cw * 32, n_q = min(T - t0, cw * 32);
-  const int32_t* idx = block_idx + ((size_t)unit * T + t0) * S;
-  mark_chunk(idx, bm, t0, n_q, S, block_size, n_kt, cw);
-  for (int j = threadIdx.x; j < n_kt; j += kThreads) {
-    int run = 0;
-    for (int w = 0; w < cw; ++w) {
-      before[w * n_kt + j] = (uint16_t)run;
-      run += __popc(bm[w * n_kt + j]);
-    }
-  }
-  __syncthreads();
-  const int32_t* st = starts + ((size_t)unit * n_chunks + chunk) * n_kt;
-  int32_t* pos = pair_of_slot + ((size_t)unit * T + t0) * S;
+__device__ __forceinline__ void fill_chunk(const int32_t* __restrict__ idx, const uint32_t* bm, const uint16_t* before,
+                                           const int32_t* st, int32_t* __restrict__ pairs, int32_t* __restrict__ pos,
+                                           SelPlanHeader* __restrict__ hdr, int t0, int n_q, int S, int block_size, int n_kt) {
   const uint32_t one = (1u << (block_size >> 4)) - 1u;              // column groups of one block
   const int n_e = n_q * S;
-  for (int e0 = 0; e0 < n_e; e0 += kThreads) {
+  for (int e0 = 0; e0 < n_e; e0 += blockDim.x) {
     const int e = e0 + threadIdx.x;
     const bool in = e < n_e;
     const int ql = in ? e / S : 0, t = t0 + ql, slot = e - ql * S;
@@ -232,11 +216,120 @@ plan_fill_kernel(const int32_t* __restrict__ block_idx, const int32_t* __restric
     int r = -1;
     if (j >= 0 && !dup) {
       const int at = (ql >> 5) * n_kt + j;
-      r = __ldg(st + j) + before[at] + __popc(bm[at] & ((1u << (ql & 31)) - 1u));
+      r = st[j] + before[at] + __popc(bm[at] & ((1u << (ql & 31)) - 1u));
       pairs[r] = (int32_t)((uint32_t)t | (groups << kPairPosBits));
     }
     if (in) pos[e] = r;
   }
+}
+
+template <bool kMatch>
+__global__ void __launch_bounds__(kThreads)
+plan_fill_kernel(const int32_t* __restrict__ block_idx, const int32_t* __restrict__ starts,
+                 int32_t* __restrict__ pairs, int32_t* __restrict__ pair_of_slot, SelPlanHeader* __restrict__ hdr, int T, int S,
+                 int block_size, int n_kt, int cw, int n_chunks) {
+  extern __shared__ uint32_t bm[];
+  uint16_t* before = reinterpret_cast<uint16_t*>(bm + n_kt * cw);   // [word][tile]: queries in earlier words
+  const int chunk = blockIdx.x, unit = blockIdx.y;
+  const int t0 = chunk * cw * 32, n_q = min(T - t0, cw * 32);
+  const int32_t* idx = block_idx + ((size_t)unit * T + t0) * S;
+  mark_chunk(idx, bm, t0, n_q, S, block_size, n_kt, cw);
+  for (int j = threadIdx.x; j < n_kt; j += kThreads) {
+    int run = 0;
+    for (int w = 0; w < cw; ++w) {
+      before[w * n_kt + j] = (uint16_t)run;
+      run += __popc(bm[w * n_kt + j]);
+    }
+  }
+  __syncthreads();
+  fill_chunk<kMatch>(idx, bm, before, starts + ((size_t)unit * n_chunks + chunk) * n_kt, pairs,
+                     pair_of_slot + ((size_t)unit * T + t0) * S, hdr, t0, n_q, S, block_size, n_kt);
+}
+
+// The three steps in one launch for sequences of up to kClusterChunk * kClusterSize tokens: a cluster to a unit, whose
+// CTAs take a chunk of queries each and read one another's counts through distributed shared memory, so that nothing
+// but the results touches global memory.  The header is zeroed before.  At 4 units of 1024 queries x 16 slots
+// 8 us against 14 for the three kernels and the gaps between them; at 4096 queries 22 against 18, at 8192 38
+// against 22: eight CTAs a unit are then too few.
+constexpr int kClusterSize = 8;
+constexpr int kClusterChunk = 256;            // queries
+constexpr int kClusterThreads = 1024;
+template <bool kMatch>
+__global__ void __launch_bounds__(kClusterThreads)
+plan_cluster_kernel(const int32_t* __restrict__ block_idx, SelPlan p, int T, int S, int block_size, int n_kt, int cw, int nq,
+                    int nq_union) {
+  extern __shared__ uint32_t bm[];
+  int32_t* cnt = reinterpret_cast<int32_t*>(bm + n_kt * cw);         // [n_kt] pairs of this chunk
+  int32_t* st = cnt + n_kt;                                          // [n_kt] first pair of this chunk
+  uint16_t* before = reinterpret_cast<uint16_t*>(st + n_kt);         // [word][tile]: queries in earlier words
+  __shared__ int warp_sums[32];
+  const int rank = (int)blockIdx.x % kClusterSize, unit = (int)blockIdx.x / kClusterSize, tid = threadIdx.x;
+  const int t0 = min(T, rank * cw * 32), n_q = min(T - t0, cw * 32);
+  const int32_t* idx = block_idx + ((size_t)unit * T + t0) * S;
+  mark_chunk(idx, bm, t0, n_q, S, block_size, n_kt, cw);
+  int uni = 0;
+  const int per = nq_union < 32 ? nq_union : 32, tw = nq_union > 32 ? nq_union / 32 : 1;
+  const uint32_t mask = per == 32 ? 0xffffffffu : (1u << per) - 1u;
+  for (int j = tid; j < n_kt; j += kClusterThreads) {
+    int c = 0;
+    uint32_t run = 0u;
+    for (int w = 0; w < cw; ++w) {
+      const uint32_t b = bm[w * n_kt + j];
+      before[w * n_kt + j] = (uint16_t)c;
+      c += __popc(b);
+      if (per < 32) {
+        for (int k = 0; k < 32; k += per) uni += ((b >> k) & mask) != 0u;
+      } else {
+        run |= b;
+        if ((w + 1) % tw == 0 || w + 1 == cw) { uni += run != 0u; run = 0u; }
+      }
+    }
+    cnt[j] = c;
+  }
+  cluster_sync();
+  int pair_carry = unit * T * S, item_carry = 0;
+  int32_t* off = p.offsets + (size_t)unit * (n_kt + 1);
+  int4* items = p.items + (size_t)unit * p.max_items;
+  for (int j0 = 0; j0 < n_kt; j0 += kClusterThreads) {
+    const int j = j0 + tid;
+    int earlier = 0, all = 0;
+    if (j < n_kt) {
+#pragma unroll
+      for (int r = 0; r < kClusterSize; ++r) {
+        const int v = ld_peer_s32(cnt + j, r);
+        if (r < rank) earlier += v;
+        all += v;
+      }
+    }
+    const int n_rt = (all + nq - 1) / nq;
+    const int n_it = j < n_kt ? max(1, (n_rt + kSelChunkTiles - 1) / kSelChunkTiles) : 0;
+    int total, total_it;
+    const int start = pair_carry + block_scan(all, warp_sums, &total);
+    const int first = item_carry + block_scan(n_it, warp_sums, &total_it);
+    if (j < n_kt) {
+      st[j] = start + earlier;
+      if (rank == 0) {
+        off[j] = start;
+        for (int k = 0; k < n_it && first + k < p.max_items; ++k)
+          items[first + k] = make_int4(unit, j, k * kSelChunkTiles, n_it);
+      }
+    }
+    pair_carry += total;
+    item_carry += total_it;
+  }
+  int uni_total;
+  block_scan(uni, warp_sums, &uni_total);
+  if (tid == 0) {
+    if (rank == 0) {
+      off[n_kt] = pair_carry;
+      p.n_items[unit] = min(item_carry, p.max_items);
+      atomicAdd(&p.hdr->pairs, (unsigned long long)(pair_carry - unit * T * S));
+    }
+    atomicAdd(&p.hdr->union_tiles, (unsigned long long)uni_total);
+  }
+  __syncthreads();
+  fill_chunk<kMatch>(idx, bm, before, st, p.pairs, p.pair_of_slot + ((size_t)unit * T + t0) * S, p.hdr, t0, n_q, S, block_size, n_kt);
+  cluster_sync();                            // nobody leaves while its counts are read
 }
 
 }  // namespace
@@ -288,6 +381,30 @@ int sel_plan_build(const int32_t* block_idx, void* base, const SelPlanLayout& l,
   const size_t smem = (size_t)l.n_ktiles * l.chunk_words * 4;
   const dim3 grid(l.n_chunks, units);
   const bool match = S <= 32 && 32 % S == 0 && l.n_ktiles < (1 << 16);
+  if (T <= kClusterChunk * kClusterSize && units <= 64) {       // (more units: the three kernels fill the GPU)
+    // chunks of whole query tiles of the union count (at most 64 queries), so that none is counted twice
+    const int cw = ((T + kClusterSize - 1) / kClusterSize + 63) / 64 * 2;
+    const size_t smem1 = (size_t)l.n_ktiles * (cw * 6 + 8);
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = kClusterSize;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)units * kClusterSize);
+    cfg.blockDim = dim3(kClusterThreads);
+    cfg.dynamicSmemBytes = smem1;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    NSA_CUDA_OK(cudaMemsetAsync(p.hdr, 0, sizeof(SelPlanHeader), st));
+    KernelScope ks("plan_cluster_kernel", st);
+    auto go = [&](auto kernel) -> int {
+      NSA_CUDA_OK(func_smem((const void*)kernel, smem1));
+      NSA_CUDA_OK(cudaLaunchKernelEx(&cfg, kernel, block_idx, p, T, S, block_size, l.n_ktiles, cw, nq, nq_union));
+      return NSA_OK;
+    };
+    return match ? go(plan_cluster_kernel<true>) : go(plan_cluster_kernel<false>);
+  }
   NSA_CUDA_OK(func_smem((const void*)plan_count_kernel, smem));
   NSA_CUDA_OK(match ? func_smem((const void*)plan_fill_kernel<true>, smem + smem / 2)
                     : func_smem((const void*)plan_fill_kernel<false>, smem + smem / 2));

@@ -1282,75 +1282,27 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
   if (warp == 0) tmem_dealloc(tmem, kTmemCols);
 }
 
-// delta[b,h,t] = sum_d dO * O (fp32), one warp per row
+// delta[b,h,t] = sum_d dO * O (fp32), D / 8 lanes to a row, one 16-byte vector of each: bound by the pass over both (16
+// heads x 8192 rows of 64: 6 us, 18 with a warp to a row).
+template <int D>
 __global__ void delta_kernel(const __nv_bfloat16* __restrict__ d_o, const __nv_bfloat16* __restrict__ o,
-                             float* __restrict__ delta, size_t rows, int D) {
-  const size_t row = (size_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (row >= rows) return;
+                             float* __restrict__ delta, size_t rows, bool vec) {
+  constexpr int kLanes = D / 8;
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x, row = i / kLanes;
   float s = 0.f;
-  for (int d = lane * 2; d < D; d += 64) {
-    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(d_o + row * D + d));
-    const float2 c = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(o + row * D + d));
-    s = fmaf(a.x, c.x, fmaf(a.y, c.y, s));
-  }
-  s = warp_sum(s);
-  if (lane == 0) delta[row] = s;
-}
-
-// dq[b, hkv*G+g, t, :] = sum over the partial slots of query (bh, t); one thread per 8 elements
-template <int D, bool kF32>
-__global__ void dq_reduce_kernel(const void* __restrict__ part, const int32_t* __restrict__ pair_of_slot,
-                                 __nv_bfloat16* __restrict__ dq, int B, int Hq, int Hkv, int T, int G,
-                                 int kind, int window, int block_size, int Lk, int n_slots, int S) {
-  constexpr int kVec = D / 8;
-  const size_t gid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const size_t total = (size_t)B * Hkv * T * G * kVec;
-  if (gid >= total) return;
-  const int v = (int)(gid % kVec);
-  const int g = (int)((gid / kVec) % G);
-  const int t = (int)((gid / ((size_t)kVec * G)) % T);
-  const size_t bh = gid / ((size_t)kVec * G * T);
-  float acc[8];
+  if (row < rows && !vec) {                          // tensors off a 16-byte boundary
+    for (int e = 0; e < 8; ++e) s = fmaf(to_float(d_o[i * 8 + e]), to_float(o[i * 8 + e]), s);
+  } else if (row < rows) {
+    const uint4 x = __ldg(reinterpret_cast<const uint4*>(d_o) + i), y = __ldg(reinterpret_cast<const uint4*>(o) + i);
+    const uint32_t a[4] = {x.x, x.y, x.z, x.w}, c[4] = {y.x, y.y, y.z, y.w};
 #pragma unroll
-  for (int e = 0; e < 8; ++e) acc[e] = 0.f;
-  auto add = [&](size_t row_index) {
-    if (kF32) {
-      const float4* src = reinterpret_cast<const float4*>((const float*)part + (row_index * G + g) * D + v * 8);
-      const float4 a = __ldcs(src), b = __ldcs(src + 1);
-      acc[0] += a.x; acc[1] += a.y; acc[2] += a.z; acc[3] += a.w;
-      acc[4] += b.x; acc[5] += b.y; acc[6] += b.z; acc[7] += b.w;
-      return;
-    }
-    const uint4 u = __ldg(reinterpret_cast<const uint4*>((const __nv_bfloat16*)part + (row_index * G + g) * D + v * 8));
-    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float2 f = __bfloat1622float2(h[e]);
-      acc[2 * e] += f.x;
-      acc[2 * e + 1] += f.y;
-    }
-  };
-  if (kind == 2) {
-    const int32_t* ps = pair_of_slot + (bh * T + t) * S;
-    for (int s = 0; s < S; ++s) {
-      const int pr = __ldg(ps + s);
-      if (pr >= 0) add((size_t)pr);
-    }
-  } else {
-    int first, last;   // key tiles this query attends
-    if (kind == 0) { first = max(0, t - window + 1) >> 6; last = t >> 6; }
-    else { first = 0; last = cmp_visible(t, block_size, window, Lk) - 1; last = last < 0 ? -1 : last >> 6; }
-    for (int jt = first; jt <= last; ++jt) {
-      const int slot = kind == 0 ? jt % n_slots : jt;
-      add((bh * T + t) * n_slots + slot);
-    }
+    for (int e = 0; e < 4; ++e)
+      s = fmaf(__uint_as_float(a[e] << 16), __uint_as_float(c[e] << 16),
+               fmaf(__uint_as_float(a[e] & 0xffff0000u), __uint_as_float(c[e] & 0xffff0000u), s));
   }
-  const int b = (int)(bh / Hkv), hkv = (int)(bh % Hkv);
-  uint4 u;
-  u.x = pack_bf16(acc[0], acc[1]); u.y = pack_bf16(acc[2], acc[3]);
-  u.z = pack_bf16(acc[4], acc[5]); u.w = pack_bf16(acc[6], acc[7]);
-  *reinterpret_cast<uint4*>(dq + (((size_t)b * Hq + hkv * G + g) * T + t) * D + v * 8) = u;
+#pragma unroll
+  for (int w = kLanes / 2; w > 0; w >>= 1) s += __shfl_xor_sync(0xffffffffu, s, w);
+  if (row < rows && i % kLanes == 0) delta[row] = s;
 }
 
 // dq of the whole op in one pass: the partials of the compression, selection and window branches
@@ -1488,6 +1440,35 @@ __global__ void dq_reduce3_kernel(const Reduce3Args a) {
     u.z = pack_bf16(acc[h][4], acc[h][5]); u.w = pack_bf16(acc[h][6], acc[h][7]);
     *reinterpret_cast<uint4*>(a.dq + (((size_t)b * a.Hq + hkv * a.G + g + h * Gp) * a.T + t) * D + v * 8) = u;
   }
+}
+
+static Reduce3Args reduce_args(const AttnArgs& a, void* dq) {
+  Reduce3Args r = {};
+  r.slots_cmp = r.slots_win = 1;
+  r.dq = (__nv_bfloat16*)dq;
+  r.B = a.B; r.Hq = a.Hq; r.Hkv = a.Hkv; r.T = a.T; r.G = a.Hq / a.Hkv;
+  return r;
+}
+
+// f32: the selection's partials are fp32 (two-term)
+static int reduce_launch(const Reduce3Args& r, int D, bool f32, const char* name, cudaStream_t st) {
+  const int hg = r.G % 2 == 0 ? 2 : (r.G % 3 == 0 ? 3 : 1);   // heads of a query served by one thread
+  const size_t nthreads = (size_t)r.B * r.Hkv * r.T * (r.G / hg) * (D / 8);
+  if (nthreads == 0) return NSA_OK;
+  const unsigned grid = (unsigned)((nthreads + 255) / 256);
+  KernelScope ks(name, st);
+  auto go = [&](auto kernel) { kernel<<<grid, 256, 0, st>>>(r); };
+  auto by_heads = [&](auto f32) {
+    constexpr bool kF32 = decltype(f32)::value;
+    if (D == 128) {
+      if (hg == 2) go(dq_reduce3_kernel<128, 2, kF32>); else if (hg == 3) go(dq_reduce3_kernel<128, 3, kF32>); else go(dq_reduce3_kernel<128, 1, kF32>);
+    } else {
+      if (hg == 2) go(dq_reduce3_kernel<64, 2, kF32>); else if (hg == 3) go(dq_reduce3_kernel<64, 3, kF32>); else go(dq_reduce3_kernel<64, 1, kF32>);
+    }
+  };
+  if (f32) by_heads(std::true_type()); else by_heads(std::false_type());
+  NSA_LAUNCH_OK("dq_reduce3_kernel");
+  return NSA_OK;
 }
 
 // Selection blocks whose row tiles were split over several work items collect dK / dV in the fp32
@@ -1639,9 +1620,10 @@ int tc_attn_bwd(const AttnArgs& a, void* ws, size_t ws_bytes, cudaStream_t st) {
   const size_t rows = (size_t)a.B * a.Hq * a.T;
   if (!a.row_dot) {
     KernelScope ks("delta_kernel", st);
-    delta_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, st>>>((const __nv_bfloat16*)a.d_o,
-                                                             (const __nv_bfloat16*)a.o,
-                                                             (float*)(base + pl.off_delta), rows, a.D);
+    const unsigned dgrid = (unsigned)((rows * (a.D / 8) + 255) / 256);
+    const auto *d_o = (const __nv_bfloat16*)a.d_o, *o = (const __nv_bfloat16*)a.o;
+    if (a.D == 128) delta_kernel<128><<<dgrid, 256, 0, st>>>(d_o, o, (float*)(base + pl.off_delta), rows, aligned16(d_o, o));
+    else delta_kernel<64><<<dgrid, 256, 0, st>>>(d_o, o, (float*)(base + pl.off_delta), rows, aligned16(d_o, o));
   }
   NSA_LAUNCH_OK("delta_kernel");
   if (a.kind == 2) {
@@ -1737,21 +1719,14 @@ int tc_attn_bwd(const AttnArgs& a, void* ws, size_t ws_bytes, cudaStream_t st) {
     if (rc2 != NSA_OK) return rc2;
   }
   if (!a.dq) return NSA_OK;   // the partials stay in the workspace (or the accumulator) for tc_dq_reduce3
-  const size_t nthreads = (size_t)a.B * a.Hkv * a.T * G * (a.D / 8);
-  const unsigned rgrid = (unsigned)((nthreads + 255) / 256);
-  {
-    KernelScope ks(branch_name(kRedNames, a.kind), st);
-    auto go = [&](auto kernel) {
-      kernel<<<rgrid, 256, 0, st>>>(p.dq_part, p.plan.pair_of_slot, (__nv_bfloat16*)a.dq, a.B, a.Hq, a.Hkv, a.T, G, a.kind,
-                                    a.window, a.block_size, a.Lk, pl.n_slots, a.S);
-    };
-    if (a.two_term) { if (a.D == 128) go(dq_reduce_kernel<128, true>); else go(dq_reduce_kernel<64, true>); }
-    else { if (a.D == 128) go(dq_reduce_kernel<128, false>); else go(dq_reduce_kernel<64, false>); }
-  }
-  NSA_LAUNCH_OK("dq_reduce_kernel");
-  return NSA_OK;
+  Reduce3Args r = reduce_args(a, a.dq);
+  if (a.kind == 0) { r.part_win = (const __nv_bfloat16*)p.dq_part; r.slots_win = pl.n_slots; r.window = a.window; }
+  else if (a.kind == 1) {
+    r.part_cmp = (const __nv_bfloat16*)p.dq_part; r.slots_cmp = pl.n_slots;
+    r.Lk_cmp = a.Lk; r.cmp_len = a.block_size; r.cmp_stride = a.window;
+  } else { r.part_slc = p.dq_part; r.pair_of_slot = p.plan.pair_of_slot; r.S = a.S; }
+  return reduce_launch(r, a.D, a.two_term, branch_name(kRedNames, a.kind), st);
 }
-
 
 // dq of the whole op from the three branch workspaces (each written by tc_attn_bwd with a null
 // dq) and / or the fp32 accumulator: `base` carries B, Hq, Hkv, T, D; a null workspace means the
@@ -1761,15 +1736,9 @@ int tc_dq_reduce3(const AttnArgs& base, int Lk_cmp, int cmp_len, int cmp_stride,
                   int window, const void* ws_cmp, const void* ws_slc, const void* ws_win,
                   const int32_t* pos, const float* dq_acc, void* dq, cudaStream_t st) {
   using namespace tc;
-  Reduce3Args r;
+  Reduce3Args r = reduce_args(base, dq);
   r.acc = dq_acc;
-  r.part_cmp = r.part_win = nullptr;
-  r.part_slc = nullptr;
-  r.pair_of_slot = nullptr;
-  r.slots_cmp = r.slots_win = 1;
   r.Lk_cmp = Lk_cmp; r.cmp_len = cmp_len; r.cmp_stride = cmp_stride; r.S = S; r.window = window;
-  r.dq = (__nv_bfloat16*)dq;
-  r.B = base.B; r.Hq = base.Hq; r.Hkv = base.Hkv; r.T = base.T; r.G = base.Hq / base.Hkv;
   if (ws_cmp) {
     AttnArgs a = base; a.two_term = false; a.kind = 1; a.Lk = Lk_cmp; a.block_size = cmp_len; a.window = cmp_stride;
     const BwdPlan pl = plan_bwd(a);
@@ -1788,23 +1757,7 @@ int tc_dq_reduce3(const AttnArgs& base, int Lk_cmp, int cmp_len, int cmp_stride,
     r.part_win = (const __nv_bfloat16*)((const char*)ws_win + pl.off_part);
     r.slots_win = pl.n_slots;
   }
-  const int hg = r.G % 2 == 0 ? 2 : (r.G % 3 == 0 ? 3 : 1);   // heads of a query served by one thread
-  const size_t nthreads = (size_t)r.B * r.Hkv * r.T * (r.G / hg) * (base.D / 8);
-  if (nthreads == 0) return NSA_OK;
-  const unsigned grid = (unsigned)((nthreads + 255) / 256);
-  KernelScope ks("dq_reduce3", st);
-  auto go = [&](auto kernel) { kernel<<<grid, 256, 0, st>>>(r); };
-  auto by_heads = [&](auto f32) {
-    constexpr bool kF32 = decltype(f32)::value;
-    if (base.D == 128) {
-      if (hg == 2) go(dq_reduce3_kernel<128, 2, kF32>); else if (hg == 3) go(dq_reduce3_kernel<128, 3, kF32>); else go(dq_reduce3_kernel<128, 1, kF32>);
-    } else {
-      if (hg == 2) go(dq_reduce3_kernel<64, 2, kF32>); else if (hg == 3) go(dq_reduce3_kernel<64, 3, kF32>); else go(dq_reduce3_kernel<64, 1, kF32>);
-    }
-  };
-  if (base.two_term) by_heads(std::true_type()); else by_heads(std::false_type());
-  NSA_LAUNCH_OK("dq_reduce3_kernel");
-  return NSA_OK;
+  return reduce_launch(r, base.D, base.two_term, "dq_reduce3", st);
 }
 
 }  // namespace nsa
