@@ -87,29 +87,30 @@ class Fork {
     }
   }
   ~Fork() {
-    if (open_ && rejoin() != cudaSuccess) cudaGetLastError();   // the failure that led here is the one to report
+    if (rejoin(open_) != cudaSuccess) cudaGetLastError();       // the failure that led here is the one to report
   }
   Fork(const Fork&) = delete;
   Fork& operator=(const Fork&) = delete;
   cudaStream_t stream(int k) const { return side_ ? side_->st[k] : main_; }
   int begin() {                                    // the side streams see what `main` holds so far
     if (!side_) return NSA_OK;
-    open_ = true;
+    open_ = 3;
     NSA_CUDA_OK(cudaEventRecord(side_->begin, main_));
     for (int k = 0; k < 2; ++k) NSA_CUDA_OK(cudaStreamWaitEvent(side_->st[k], side_->begin, 0));
     return NSA_OK;
   }
-  int join() {
-    if (open_) NSA_CUDA_OK(rejoin());
+  int join(int which = 3) {                        // `main` waits for the side streams of the mask
+    NSA_CUDA_OK(rejoin(open_ & which));
     return NSA_OK;
   }
 
  private:
   void drop() { cudaGetLastError(); side_ = nullptr; }
-  cudaError_t rejoin() {
-    open_ = false;
+  cudaError_t rejoin(int which) {
+    open_ &= ~which;
     cudaError_t rc = cudaSuccess;
     for (int k = 0; k < 2; ++k) {                  // one stream's error does not leave the other unjoined
+      if (!(which >> k & 1)) continue;
       cudaError_t e = cudaEventRecord(side_->end[k], side_->st[k]);
       if (e == cudaSuccess) e = cudaStreamWaitEvent(main_, side_->end[k], 0);
       if (e != cudaSuccess) rc = e;
@@ -118,7 +119,7 @@ class Fork {
   }
   cudaStream_t main_;
   SideStreams* side_ = nullptr;
-  bool open_ = false;       // forked and not joined yet
+  int open_ = 0;            // side streams that are forked and not joined yet
 };
 
 struct Carver {
@@ -287,17 +288,23 @@ extern "C" int nsa_attention_fwd(const NsaAttentionDesc* d, const NsaAttentionTe
   void* plan = p.plan_bytes ? sv + p.plan : nullptr;
   Fork fork(st, small_problem(d));
   NSA_TRY(fork.begin());
-  NSA_TRY(nsa_range_attn_fwd(t->q, t->kw, t->vw, o[2], lse[2], &m, m.T, NSA_MODE_WINDOW, d->window, 0, d->impl, fork.stream(0)));
-  // the selection branch with its plan; with given lists it waits for nothing
+  auto window = [&]() -> int {
+    return nsa_range_attn_fwd(t->q, t->kw, t->vw, o[2], lse[2], &m, m.T, NSA_MODE_WINDOW, d->window, 0, d->impl, fork.stream(0));
+  };
+  auto build_plan = [&](cudaStream_t s) -> int {
+    return plan ? tc_sel_plan_build(sel_args(d, t->block_idx), plan, p.plan_bytes, s) : NSA_OK;
+  };
   auto selection = [&](cudaStream_t s) -> int {
-    if (plan) NSA_TRY(tc_sel_plan_build(sel_args(d, t->block_idx), plan, p.plan_bytes, s));
     if (plan && p.fwd_ws)
       return nsa_selection_fwd_planned(t->q, t->ks, t->vs, t->block_idx, o[1], lse[1], &m, p.S, d->block_size,
                                        workspace, workspace_bytes, plan, s);
     return nsa_selection_fwd(t->q, t->ks, t->vs, t->block_idx, o[1], lse[1], &m, p.S, d->block_size, workspace,
                              workspace_bytes, d->impl, s);
   };
-  if (d->given_lists) NSA_TRY(selection(fork.stream(1)));
+  // Given lists: their plan, a chain of small kernels, goes ahead of what fills the GPU beside it, and the
+  // selection behind that.  Lists of the scorer: the window beside the chain that leads to them.
+  if (d->given_lists) NSA_TRY(build_plan(fork.stream(1)));
+  else NSA_TRY(window());
   if (p.fast_pool) {
     PoolSides s = op_sides(d, t);
     s.out[0] = k_cmp; s.out[1] = v_cmp;
@@ -316,20 +323,26 @@ extern "C" int nsa_attention_fwd(const NsaAttentionDesc* d, const NsaAttentionTe
   }
   NSA_TRY(nsa_range_attn_fwd(t->q, k_cmp, v_cmp, o[0], lse[0], &m, p.n_cmp, NSA_MODE_COMPRESS_STRIDED, d->cmp_stride,
                              d->cmp_len, d->impl, stream));
-  if (!d->given_lists) {
+  if (d->given_lists) {
+    NSA_TRY(window());
+    NSA_TRY(selection(fork.stream(1)));
+    NSA_TRY(fork.join());
+  } else {
     NSA_TRY(nsa_topn_blocks_general(t->q, k_cmp, lse[0], t->block_idx, nullptr, &m, p.n_cmp, d->cmp_len, d->cmp_stride,
                                       d->block_size, p.S, d->n_init, d->n_local, score_impl(d), stream));
     if (plan && !p.fwd_ws) {      // only the backward reads the plan: it is built beside the forward kernel
       NSA_TRY(fork.begin());
-      NSA_TRY(tc_sel_plan_build(sel_args(d, t->block_idx), plan, p.plan_bytes, fork.stream(1)));
+      NSA_TRY(build_plan(fork.stream(1)));
       NSA_TRY(nsa_selection_fwd(t->q, t->ks, t->vs, t->block_idx, o[1], lse[1], &m, p.S, d->block_size, nullptr, 0,
                                 d->impl, stream));
     } else {
+      NSA_TRY(build_plan(st));
       NSA_TRY(selection(st));
     }
+    NSA_TRY(fork.join(1));
   }
-  NSA_TRY(fork.join());
-  return nsa_gate_combine_fwd(o[0], o[1], o[2], t->gate, t->out, &m, stream);
+  NSA_TRY(nsa_gate_combine_fwd(o[0], o[1], o[2], t->gate, t->out, &m, stream));
+  return fork.join();                    // a plan that only the backward reads
 }
 
 extern "C" int nsa_attention_bwd(const NsaAttentionDesc* d, const NsaAttentionTensors* t, const void* saved,

@@ -13,7 +13,6 @@ namespace {
 
 constexpr int kKeysPerTile = 64;
 constexpr int kThreads = 256;
-constexpr int kScanThreads = 1024;
 
 // key tile of a list entry of query t, -1 when the entry is empty or lies after t
 __device__ __forceinline__ int tile_of(int blk, int t, int block_size) {
@@ -75,7 +74,8 @@ plan_count_kernel(const int32_t* __restrict__ block_idx, int32_t* __restrict__ c
   if (threadIdx.x == 0) unions[unit * n_chunks + chunk] = s_uni;
 }
 
-// exclusive scan of v over the CTA; *total gets the sum
+// exclusive scan of v over the CTA's NT threads; *total gets the sum
+template <int NT>
 __device__ __forceinline__ int block_scan(int v, int* warp_sums, int* total) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int incl = v;
@@ -87,7 +87,7 @@ __device__ __forceinline__ int block_scan(int v, int* warp_sums, int* total) {
   if (lane == 31) warp_sums[warp] = incl;
   __syncthreads();
   if (warp == 0) {
-    int w = lane < kScanThreads / 32 ? warp_sums[lane] : 0;
+    int w = lane < NT / 32 ? warp_sums[lane] : 0;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const int u = __shfl_up_sync(0xffffffffu, w, o);
@@ -97,28 +97,30 @@ __device__ __forceinline__ int block_scan(int v, int* warp_sums, int* total) {
   }
   __syncthreads();
   const int before = warp ? warp_sums[warp - 1] : 0;
-  *total = warp_sums[kScanThreads / 32 - 1];
+  *total = warp_sums[NT / 32 - 1];
   __syncthreads();
   return before + incl - v;
 }
 
 // One CTA per unit: offsets of the key tiles, the start of every (chunk, tile) run in place of its
-// count, and the work items in (tile, chunk) order.  Up to 1024 tiles a pass; with fewer tiles the
-// chunks are dealt out over groups of threads, so the column sums are not one long chain of loads.
-__global__ void __launch_bounds__(kScanThreads)
+// count, and the work items in (tile, chunk) order.  Up to NT tiles a pass; with fewer tiles the
+// chunks are dealt out over groups of threads, so the column sums are not one long chain of loads.  256 threads of
+// at most 48 registers find room beside two CTAs of the window kernel on an SM; 1024 wait until they are done.
+template <int NT>
+__global__ void __launch_bounds__(NT, NT == 256 ? 5 : 1)
 plan_scan_kernel(int32_t* __restrict__ counts, const int32_t* __restrict__ unions, SelPlan p, int T, int S,
                  int n_kt, int n_chunks, int nq) {
-  constexpr int kBatch = 16;                  // loads in flight per thread
+  constexpr int kBatch = NT == 256 ? 8 : 16;  // loads in flight per thread
   __shared__ int warp_sums[32];
-  __shared__ int part_sum[kScanThreads];
+  __shared__ int part_sum[NT];
   const int unit = blockIdx.x, tid = threadIdx.x;
   int32_t* cnt = counts + (size_t)unit * n_chunks * n_kt;
   int pair_carry = unit * T * S, item_carry = 0;
   int32_t* off = p.offsets + (size_t)unit * (n_kt + 1);
   int4* items = p.items + (size_t)unit * p.max_items;
   int width = 32;                             // tiles per pass, a power of two
-  while (width < kScanThreads && width < n_kt) width <<= 1;
-  const int parts = kScanThreads / width, part = tid / width;
+  while (width < NT && width < n_kt) width <<= 1;
+  const int parts = NT / width, part = tid / width;
   const int per = (n_chunks + parts - 1) / parts;
   const int c0 = min(n_chunks, part * per), c1 = min(n_chunks, c0 + per);
   for (int j0 = 0; j0 < n_kt; j0 += width) {
@@ -141,8 +143,8 @@ plan_scan_kernel(int32_t* __restrict__ counts, const int32_t* __restrict__ union
     // at least one item, so that a tile nobody lists still gets its zero gradients
     const int n_it = first_part ? max(1, (n_rt + kSelChunkTiles - 1) / kSelChunkTiles) : 0;
     int total, total_it;
-    const int start = pair_carry + block_scan(first_part ? all : 0, warp_sums, &total);
-    const int first = item_carry + block_scan(n_it, warp_sums, &total_it);
+    const int start = pair_carry + block_scan<NT>(first_part ? all : 0, warp_sums, &total);
+    const int first = item_carry + block_scan<NT>(n_it, warp_sums, &total_it);
     if (first_part) {
       off[j] = start;
       for (int k = 0; k < n_it && first + k < p.max_items; ++k)
@@ -168,9 +170,9 @@ plan_scan_kernel(int32_t* __restrict__ counts, const int32_t* __restrict__ union
     item_carry += total_it;
   }
   int uni = 0;
-  for (int c = tid; c < n_chunks; c += kScanThreads) uni += unions[unit * n_chunks + c];
+  for (int c = tid; c < n_chunks; c += NT) uni += unions[unit * n_chunks + c];
   int uni_total;
-  block_scan(uni, warp_sums, &uni_total);
+  block_scan<NT>(uni, warp_sums, &uni_total);
   if (tid == 0) {
     off[n_kt] = pair_carry;
     p.n_items[unit] = min(item_carry, p.max_items);
@@ -304,8 +306,8 @@ plan_cluster_kernel(const int32_t* __restrict__ block_idx, SelPlan p, int T, int
     const int n_rt = (all + nq - 1) / nq;
     const int n_it = j < n_kt ? max(1, (n_rt + kSelChunkTiles - 1) / kSelChunkTiles) : 0;
     int total, total_it;
-    const int start = pair_carry + block_scan(all, warp_sums, &total);
-    const int first = item_carry + block_scan(n_it, warp_sums, &total_it);
+    const int start = pair_carry + block_scan<kClusterThreads>(all, warp_sums, &total);
+    const int first = item_carry + block_scan<kClusterThreads>(n_it, warp_sums, &total_it);
     if (j < n_kt) {
       st[j] = start + earlier;
       if (rank == 0) {
@@ -318,7 +320,7 @@ plan_cluster_kernel(const int32_t* __restrict__ block_idx, SelPlan p, int T, int
     item_carry += total_it;
   }
   int uni_total;
-  block_scan(uni, warp_sums, &uni_total);
+  block_scan<kClusterThreads>(uni, warp_sums, &uni_total);
   if (tid == 0) {
     if (rank == 0) {
       off[n_kt] = pair_carry;
@@ -412,7 +414,8 @@ int sel_plan_build(const int32_t* block_idx, void* base, const SelPlanLayout& l,
     plan_count_kernel<<<grid, kThreads, smem, st>>>(block_idx, counts, unions, p.hdr, T, S, block_size, l.n_ktiles,
                                                     l.chunk_words, l.n_chunks, nq_union); }
   { KernelScope ks("plan_scan_kernel", st);
-    plan_scan_kernel<<<units, kScanThreads, 0, st>>>(counts, unions, p, T, S, l.n_ktiles, l.n_chunks, nq); }
+    if (l.n_ktiles <= 256) plan_scan_kernel<256><<<units, 256, 0, st>>>(counts, unions, p, T, S, l.n_ktiles, l.n_chunks, nq);
+    else plan_scan_kernel<1024><<<units, 1024, 0, st>>>(counts, unions, p, T, S, l.n_ktiles, l.n_chunks, nq); }
   { KernelScope ks("plan_fill_kernel", st);
     if (match)
       plan_fill_kernel<true><<<grid, kThreads, smem + smem / 2, st>>>(block_idx, counts, p.pairs, p.pair_of_slot, p.hdr, T, S,
