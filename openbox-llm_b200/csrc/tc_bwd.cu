@@ -1321,7 +1321,8 @@ struct Reduce3Args {
 // kernel moves 32 GB at the benchmark shape and was held back by its instruction count, not by
 // memory, when every thread served a single head.
 template <int D, int HG, bool kF32>
-__global__ void dq_reduce3_kernel(const Reduce3Args a) {
+__global__ void __launch_bounds__(256, 3)
+dq_reduce3_kernel(const Reduce3Args a) {
   constexpr int kVec = D / 8;
   const int Gp = a.G / HG;                               // head groups per query
   const size_t gid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1339,11 +1340,12 @@ __global__ void dq_reduce3_kernel(const Reduce3Args a) {
   const size_t row_elems = (size_t)a.G * D;              // elements of one partial row (all heads)
   const size_t in_row = (size_t)g * D + v * 8;           // this thread's first head inside a row
   const size_t head_step = (size_t)Gp * D;               // to its next head
-  // Rows per trip: 8 for one or two heads; three heads hold three loads per row, and an empty place costs as
-  // many instructions as a row (a window of 512 touches 9 key tiles, a query sees few tiles of
-  // summaries).  Groups of 3 at 8 x 4096 tokens: 277 us with a thread per head, 257 so; at two heads
-  // shorter trips gain 1 % at T = 32768 and cost 4 of 13 us at T = 1024.
-  constexpr int kTripSel = HG == 3 ? 4 : 8, kTripWin = HG == 3 ? 3 : 8, kTripCmp = HG == 3 ? 2 : 8;
+  // Rows per trip and CTAs per SM (three: 80 registers, which hold the loads of a trip; without the bound the
+  // compiler took 70 and issued them in turns).  An empty place costs as many instructions as a row (a window
+  // of 512 touches 9 key tiles, a query sees few tiles of summaries).  Two heads at 8 x 32768 tokens: trips of
+  // 8 rows in 5.24 ms, of 4 in 4.90 (5.33 with five CTAs, which spill), unbounded 5.76; groups of 3 at 8 x 4096:
+  // 203 us, unbounded 257.
+  constexpr int kTripSel = HG == 1 ? 8 : 4, kTripWin = HG == 3 ? 3 : kTripSel, kTripCmp = HG == 3 ? 2 : kTripSel;
   // a trip of N partial rows: their loads are issued before the first is added
   auto add_rows = [&](const __nv_bfloat16* part, const auto& rows) {
     constexpr int kTrip = sizeof(rows) / sizeof(rows[0]);

@@ -18,10 +18,12 @@ namespace tc {
 
 // o[b, hkv*G+g, t, :] and lse from the per-(pair, head) partials of query (bh, t).  Bound by the one pass
 // over the partials: a thread owns 8 columns of H neighbouring heads, whose partial rows lie side by
-// side and share the index loads and the addresses, and has 4 H 16-byte loads in flight.  At 8 x 32768
-// tokens, 16 heads of 128: 19 GB in 3.42 ms (3.54 with a thread per head); 64 heads x 65536: 3.49 (3.60).
+// side and share the index loads and the addresses, and has 4 H 16-byte loads in flight.  Three CTAs of 80
+// registers share an SM, which is what the pass needs in flight: at 8 x 32768 tokens, 16 heads of 128, 19 GB in
+// 3.02 ms, 3.58 with two CTAs of 110; 64 heads x 65536 2.97, 3.43 (3.45 with four CTAs of 64 registers, which spill, 3.36
+// and 3.00 with two slots a trip and three or four CTAs, 3.51 with eight).
 template <int D, int H>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 3)
 sel_combine_kernel(const __nv_bfloat16* __restrict__ o_part, const float* __restrict__ ml,
                    const int32_t* __restrict__ pair_of_slot, const SelPlanHeader* __restrict__ hdr,
                    __nv_bfloat16* __restrict__ o, float* __restrict__ lse, int B, int Hq, int Hkv, int T, int G, int S,
