@@ -1,9 +1,12 @@
 // Bandwidth-bound companions of the attention kernels: compression pooling, block scoring +
 // top-n, block->query CSR inversion and the sigmoid gate combine.
+#include <algorithm>
 #include <type_traits>
 #include <atomic>
 
+#include "op.cuh"
 #include "pool.cuh"
+#include "tc_common.cuh"
 
 namespace nsa {
 namespace {
@@ -463,25 +466,30 @@ __device__ __forceinline__ void load8(const __nv_bfloat16* p, float* f) {
   }
 }
 
-__global__ void gate_fwd_vec_kernel(const __nv_bfloat16* __restrict__ oc, const __nv_bfloat16* __restrict__ os,
-                                    const __nv_bfloat16* __restrict__ ow, const __nv_bfloat16* __restrict__ gate,
-                                    __nv_bfloat16* __restrict__ out, size_t rows, int VL) {
-  const size_t gid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const size_t row = gid / VL;
-  if (row >= rows) return;
-  const size_t i = gid * 8;
-  float a[8], b[8], c[8];
-  load8(oc + i, a); load8(os + i, b); load8(ow + i, c);
-  const float g0 = sigmoidf_(__bfloat162float(gate[row * 3 + 0]));
-  const float g1 = sigmoidf_(__bfloat162float(gate[row * 3 + 1]));
-  const float g2 = sigmoidf_(__bfloat162float(gate[row * 3 + 2]));
-  uint4 r;
-  __nv_bfloat162* rs = reinterpret_cast<__nv_bfloat162*>(&r);
+// (Where the merge may have blended, a grid of 16 CTAs per SM strides over the rows: a grid of a CTA for every 256
+// vectors took 148 us to come and go at 65536 tokens, 64 heads of 128.)
+__global__ void __launch_bounds__(256)
+gate_fwd_vec_kernel(const __nv_bfloat16* __restrict__ oc, const __nv_bfloat16* __restrict__ os,
+                    const __nv_bfloat16* __restrict__ ow, const __nv_bfloat16* __restrict__ gate,
+                    __nv_bfloat16* __restrict__ out, size_t rows, int VL, const SelPlanHeader* __restrict__ hdr, int nq_union,
+                    int force) {
+  if (hdr != nullptr && tc::prefer_pairs(hdr, nq_union, force)) return;   // the merge of the selection has blended
+  const size_t n = rows * VL, stride = (size_t)gridDim.x * blockDim.x;
+  for (size_t gid = (size_t)blockIdx.x * blockDim.x + threadIdx.x; gid < n; gid += stride) {
+    const size_t row = gid / VL, i = gid * 8;
+    float a[8], b[8], c[8];
+    load8(oc + i, a); load8(os + i, b); load8(ow + i, c);
+    const float g0 = sigmoidf_(__bfloat162float(gate[row * 3 + 0]));
+    const float g1 = sigmoidf_(__bfloat162float(gate[row * 3 + 1]));
+    const float g2 = sigmoidf_(__bfloat162float(gate[row * 3 + 2]));
+    uint4 r;
+    __nv_bfloat162* rs = reinterpret_cast<__nv_bfloat162*>(&r);
 #pragma unroll
-  for (int e = 0; e < 4; ++e)
-    rs[e] = __floats2bfloat162_rn(g0 * a[2 * e] + g1 * b[2 * e] + g2 * c[2 * e],
-                                  g0 * a[2 * e + 1] + g1 * b[2 * e + 1] + g2 * c[2 * e + 1]);
-  *reinterpret_cast<uint4*>(out + i) = r;
+    for (int e = 0; e < 4; ++e)
+      rs[e] = __floats2bfloat162_rn(g0 * a[2 * e] + g1 * b[2 * e] + g2 * c[2 * e],
+                                    g0 * a[2 * e + 1] + g1 * b[2 * e + 1] + g2 * c[2 * e + 1]);
+    *reinterpret_cast<uint4*>(out + i) = r;
+  }
 }
 
 // One 16-byte vector of each of the four tensors a thread; three lanes of a row finish a branch each.  Bound by the
@@ -1195,12 +1203,19 @@ extern "C" int nsa_swap_heads_tokens(const void* src, void* dst, int B, int H, i
 extern "C" int nsa_gate_combine_fwd(const void* o_cmp, const void* o_slc, const void* o_win,
                                     const void* gate_logits, void* out, const NsaDims* dims,
                                     void* stream) {
+  return nsa::gate_fwd_unless_blended(o_cmp, o_slc, o_win, gate_logits, out, dims, nsa::SelChoice{}, stream);
+}
+
+int nsa::gate_fwd_unless_blended(const void* o_cmp, const void* o_slc, const void* o_win, const void* gate_logits, void* out,
+                                 const NsaDims* dims, const SelChoice& choice, void* stream) {
   NSA_CHECK_ARG(dims, "null dims");
   const size_t rows = (size_t)dims->B * dims->Hq * dims->T;
   if (rows == 0) return NSA_OK;
   cudaStream_t st = (cudaStream_t)stream;
+  unsigned grid = blocks_for(rows * (dims->D / 8), 256);
+  if (choice.hdr) grid = std::min(grid, 16u * (unsigned)sm_count());
   if (gate_vec_ok(dims->D, dims->dtype))
-    { KernelScope ks("gate_fwd_kernel", st); gate_fwd_vec_kernel<<<blocks_for(rows * (dims->D / 8), 256), 256, 0, st>>>((const __nv_bfloat16*)o_cmp, (const __nv_bfloat16*)o_slc, (const __nv_bfloat16*)o_win, (const __nv_bfloat16*)gate_logits, (__nv_bfloat16*)out, rows, dims->D / 8); }
+    { KernelScope ks("gate_fwd_kernel", st); gate_fwd_vec_kernel<<<grid, 256, 0, st>>>((const __nv_bfloat16*)o_cmp, (const __nv_bfloat16*)o_slc, (const __nv_bfloat16*)o_win, (const __nv_bfloat16*)gate_logits, (__nv_bfloat16*)out, rows, dims->D / 8, choice.hdr, choice.nq_union, choice.force); }
   else if (dims->dtype == NSA_DTYPE_BF16)
     { KernelScope ks("gate_fwd_kernel", st); gate_fwd_kernel<<<blocks_for(rows, 8), 256, 0, st>>>((const __nv_bfloat16*)o_cmp, (const __nv_bfloat16*)o_slc, (const __nv_bfloat16*)o_win, (const __nv_bfloat16*)gate_logits, (__nv_bfloat16*)out, rows, dims->D); }
   else

@@ -106,6 +106,11 @@ struct AttnArgs {
   float* dq_acc;     // tcgen05 window / compression backward: fp32 accumulator [B*Hkv][T][G][D] that takes dQ (or null)
   const void* sel_plan;   // tcgen05 selection: plan built earlier (tc_sel_plan_build), or null
   bool two_term;          // tcgen05 selection on 16- and 32-token blocks: P and dS in two bf16 terms, dQ partials in fp32
+  // tcgen05 selection: where the block-outer kernel serves the call its merge blends the three branches as well
+  // (gate logits, the other branches' outputs, the op's output; null g_out: it does not) and keeps `o` only
+  // where o_kept says so
+  const void *g_cmp, *g_win, *g_logits;
+  void *g_out, *o_kept;
   bool plan_kept;         // the plan outlives the dQ reduction: the backward need not copy its pair map
   int B, Hq, Hkv, T, Lk, D, S;
   int kind;          // 0 window, 1 compress, 2 selection
@@ -125,6 +130,9 @@ int tc_attn_fwd(const AttnArgs& a, cudaStream_t st);
 size_t tc_sel_fwd_workspace(const AttnArgs& a);
 int tc_sel_fwd(const AttnArgs& a, void* ws, size_t ws_bytes, cudaStream_t st);
 size_t tc_sel_plan_bytes(const AttnArgs& a);
+// what decides on the device which of the two forward kernels serves a planned call
+struct SelChoice { const struct SelPlanHeader* hdr; int nq_union, force; };
+SelChoice tc_sel_choice(const AttnArgs& a, const void* plan);
 int tc_sel_plan_build(const AttnArgs& a, void* plan, size_t plan_bytes, cudaStream_t st);
 const int32_t* sel_plan_pair_map(const AttnArgs& a, int S, int block_size, const void* plan);
 size_t tc_attn_bwd_workspace(const AttnArgs& a);

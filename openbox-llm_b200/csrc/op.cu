@@ -91,6 +91,7 @@ class Fork {
   }
   Fork(const Fork&) = delete;
   Fork& operator=(const Fork&) = delete;
+  bool active() const { return side_ != nullptr; }
   cudaStream_t stream(int k) const { return side_ ? side_->st[k] : main_; }
   int begin() {                                    // the side streams see what `main` holds so far
     if (!side_) return NSA_OK;
@@ -294,10 +295,18 @@ extern "C" int nsa_attention_fwd(const NsaAttentionDesc* d, const NsaAttentionTe
   auto build_plan = [&](cudaStream_t s) -> int {
     return plan ? tc_sel_plan_build(sel_args(d, t->block_idx), plan, p.plan_bytes, s) : NSA_OK;
   };
+  SelChoice choice = {};
   auto selection = [&](cudaStream_t s) -> int {
-    if (plan && p.fwd_ws)
-      return nsa_selection_fwd_planned(t->q, t->ks, t->vs, t->block_idx, o[1], lse[1], &m, p.S, d->block_size,
-                                       workspace, workspace_bytes, plan, s);
+    if (plan && p.fwd_ws) {
+      AttnArgs a = sel_args(d, t->block_idx);
+      a.q = t->q; a.k = t->ks; a.v = t->vs; a.o = o[1]; a.lse = lse[1]; a.sel_plan = plan;
+      if (!fork.active()) {              // the other branches lie before this one: its merge can blend them
+        a.g_cmp = o[0]; a.g_win = o[2]; a.g_logits = t->gate; a.g_out = t->out;
+        a.o_kept = d->need_grad ? o[1] : nullptr;
+        choice = tc_sel_choice(a, plan);
+      }
+      return tc_sel_fwd(a, workspace, workspace_bytes, s);
+    }
     return nsa_selection_fwd(t->q, t->ks, t->vs, t->block_idx, o[1], lse[1], &m, p.S, d->block_size, workspace,
                              workspace_bytes, d->impl, s);
   };
@@ -341,7 +350,7 @@ extern "C" int nsa_attention_fwd(const NsaAttentionDesc* d, const NsaAttentionTe
     }
     NSA_TRY(fork.join(1));
   }
-  NSA_TRY(nsa_gate_combine_fwd(o[0], o[1], o[2], t->gate, t->out, &m, stream));
+  NSA_TRY(gate_fwd_unless_blended(o[0], o[1], o[2], t->gate, t->out, &m, choice, stream));
   return fork.join();                    // a plan that only the backward reads
 }
 

@@ -10,5 +10,8 @@ bool use_tc(const NsaDims* d, int block_size, int impl, int* err);
 bool use_two_term(const NsaDims* d, int block_size, int S, int impl, bool bwd);
 int topn_check(const NsaDims* dims, int n_cmp, int cmp_len, int cmp_stride, int sel_block, int n_sel, int n_init,
                int n_local, int impl);   // aux.cu
+// nsa_gate_combine_fwd, unless the block-outer kernel has served the selection (a choice without header: always)
+int gate_fwd_unless_blended(const void* o_cmp, const void* o_slc, const void* o_win, const void* gate_logits, void* out,
+                            const NsaDims* dims, const SelChoice& choice, void* stream);   // aux.cu
 bool profiling();     // every launch is bracketed by events on its stream: branches must not overlap
 }  // namespace nsa

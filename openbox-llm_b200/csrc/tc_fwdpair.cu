@@ -22,12 +22,19 @@ namespace tc {
 // registers share an SM, which is what the pass needs in flight: at 8 x 32768 tokens, 16 heads of 128, 19 GB in
 // 3.02 ms, 3.58 with two CTAs of 110; 64 heads x 65536 2.97, 3.43 (3.45 with four CTAs of 64 registers, which spill, 3.36
 // and 3.00 with two slots a trip and three or four CTAs, 3.51 with eight).
+//
+// Where the whole op asks for it (gb.out) the gate blend is done here too: o_slc need not be read back (nor written,
+// when no backward follows).
+struct GateBlend {
+  const __nv_bfloat16 *cmp, *win, *logits;
+  __nv_bfloat16* out;
+};
 template <int D, int H>
 __global__ void __launch_bounds__(256, 3)
 sel_combine_kernel(const __nv_bfloat16* __restrict__ o_part, const float* __restrict__ ml,
                    const int32_t* __restrict__ pair_of_slot, const SelPlanHeader* __restrict__ hdr,
-                   __nv_bfloat16* __restrict__ o, float* __restrict__ lse, int B, int Hq, int Hkv, int T, int G, int S,
-                   int nq_union, int force) {
+                   __nv_bfloat16* __restrict__ o, float* __restrict__ lse, const GateBlend gb, int B, int Hq, int Hkv, int T,
+                   int G, int S, int nq_union, int force) {
   if (!prefer_pairs(hdr, nq_union, force)) return;
   constexpr int kVec = D / 8;
   const int groups = G / H;
@@ -102,7 +109,23 @@ sel_combine_kernel(const __nv_bfloat16* __restrict__ o_part, const float* __rest
     uint4 u;
     u.x = pack_bf16(acc[h][0] * inv, acc[h][1] * inv); u.y = pack_bf16(acc[h][2] * inv, acc[h][3] * inv);
     u.z = pack_bf16(acc[h][4] * inv, acc[h][5] * inv); u.w = pack_bf16(acc[h][6] * inv, acc[h][7] * inv);
-    *reinterpret_cast<uint4*>(o + orow * D + v * 8) = u;
+    if (o) *reinterpret_cast<uint4*>(o + orow * D + v * 8) = u;
+    if (gb.out) {
+      const uint4 c = __ldcs(reinterpret_cast<const uint4*>(gb.cmp + orow * D + v * 8));
+      const uint4 w = __ldcs(reinterpret_cast<const uint4*>(gb.win + orow * D + v * 8));
+      float gate[3];
+#pragma unroll
+      for (int k = 0; k < 3; ++k) gate[k] = 1.f / (1.f + expf(-__bfloat162float(gb.logits[orow * 3 + k])));
+      const uint32_t xc[4] = {c.x, c.y, c.z, c.w}, xs[4] = {u.x, u.y, u.z, u.w}, xw[4] = {w.x, w.y, w.z, w.w};
+      uint32_t r[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        r[e] = pack_bf16(gate[0] * __uint_as_float(xc[e] << 16) + gate[1] * __uint_as_float(xs[e] << 16) +
+                             gate[2] * __uint_as_float(xw[e] << 16),
+                         gate[0] * __uint_as_float(xc[e] & 0xffff0000u) + gate[1] * __uint_as_float(xs[e] & 0xffff0000u) +
+                             gate[2] * __uint_as_float(xw[e] & 0xffff0000u));
+      *reinterpret_cast<uint4*>(gb.out + orow * D + v * 8) = make_uint4(r[0], r[1], r[2], r[3]);
+    }
     if (v == 0) lse[orow] = L[h] > 0.f ? (M[h] + log2f(L[h])) * kLn2 : kLseEmpty;
   }
 }
@@ -154,6 +177,10 @@ const int32_t* sel_plan_pair_map(const AttnArgs& base, int S, int block_size, co
   return sel_plan_at(plan, tc::plan_pairs(a).layout).pair_of_slot;
 }
 
+SelChoice tc_sel_choice(const AttnArgs& a, const void* plan) {
+  return {sel_plan_at(plan, tc::plan_pairs(a).layout).hdr, tc::kRows / tc::group_pad(a.Hq / a.Hkv), get_option_sel_fwd()};
+}
+
 int tc_sel_plan_build(const AttnArgs& a, void* plan, size_t plan_bytes, cudaStream_t st) {
   using namespace tc;
   const PairPlan pl = plan_pairs(a);
@@ -200,7 +227,10 @@ int tc_sel_fwd(const AttnArgs& a, void* ws, size_t ws_bytes, cudaStream_t st) {
   auto combine = [&](auto kernel) {
     KernelScope ks("sel_combine_kernel", st);
     kernel<<<cgrid, 256, 0, st>>>((const __nv_bfloat16*)(base + pl.off_part), (const float*)(base + pl.off_ml),
-                                  plan.pair_of_slot, plan.hdr, (__nv_bfloat16*)a.o, a.lse, a.B, a.Hq, a.Hkv, a.T, G, a.S,
+                                  plan.pair_of_slot, plan.hdr, (__nv_bfloat16*)(a.g_out ? a.o_kept : a.o), a.lse,
+                                  GateBlend{(const __nv_bfloat16*)a.g_cmp, (const __nv_bfloat16*)a.g_win,
+                                            (const __nv_bfloat16*)a.g_logits, (__nv_bfloat16*)a.g_out},
+                                  a.B, a.Hq, a.Hkv, a.T, G, a.S,
                                   nq_union, force);
   };
   if (a.D == 128) { if (H == 2) combine(sel_combine_kernel<128, 2>); else combine(sel_combine_kernel<128, 1>); }

@@ -159,3 +159,30 @@ def test_layer_is_what_its_modules_give(B, T, Hq, Hkv, dh, bs, x_dtype):
             # bf16 rounding of the entries and of what they are sums of; k_intra is zero but for rounding
             assert (a.float() - b.float()).norm() <= 2.0 ** -6 * b.float().norm() + 1e-3, i
     assert pkg().lib().nsa_device_status(None) == 0
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_blend_in_the_merge(D):
+    """A call that fills the GPU blends the branches where the selection's partials are merged, if the block-outer kernel
+    served it, and by the gate kernel if the query-outer one did: the same output but for the partials' rounding to bf16
+    (2^-9 of each term), bit for bit the same with and without a backward to come."""
+    nsa = pkg()
+    B, Hq, Hkv, T = 1, 16, 2, 12352
+    g = torch.Generator("cuda").manual_seed(2)
+    mk = lambda h, n=D: torch.randn(B, h, T, n, generator=g, device="cuda").bfloat16()
+    ins = [mk(Hq), *[mk(Hkv) for _ in range(6)], mk(Hq, 3)]
+    outs = []
+    for variant in (1, 2, 0):
+        nsa.set_option("sel_fwd_variant", variant)
+        try:
+            out, idx = nsa.nsa_attention(*ins, 64, 16, 512, return_block_idx=True)
+            xs = [x.detach().requires_grad_(True) for x in ins]
+            assert torch.equal(nsa.nsa_attention(*xs, 64, 16, 512), out)
+            assert torch.equal(nsa.nsa_attention(*ins, 64, 16, 512, block_idx=idx), out)
+        finally:
+            nsa.set_option("sel_fwd_variant", 0)
+        outs.append(out.float())
+    assert torch.equal(outs[2], outs[0]) or torch.equal(outs[2], outs[1])
+    assert not torch.equal(outs[0], outs[1])
+    assert (outs[0] - outs[1]).abs().max() <= 2.0 ** -6 and (outs[0] - outs[1]).norm() <= 2.0 ** -8 * outs[0].norm()
+    assert nsa.lib().nsa_device_status(None) == 0
