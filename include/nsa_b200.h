@@ -37,7 +37,8 @@ extern "C" {
 
 /* which kernel family serves a call */
 #define NSA_IMPL_AUTO 0   /* tcgen05 kernels when the shape allows, else the SIMT kernels; selection on blocks
-                             of 16 or 32 tokens always SIMT, whose arithmetic is fp32 throughout */
+                             of 16 or 32 tokens with P and dS in two bf16 terms and fp32 dQ partials, or SIMT,
+                             whose arithmetic is fp32 throughout */
 #define NSA_IMPL_SIMT 1   /* CUDA-core kernels: any dtype, D in {16,32,64,128}, any G and block size */
 #define NSA_IMPL_TC   2   /* tcgen05/TMEM kernels only; NSA_ERR_UNSUPPORTED if the shape does not fit */
 
