@@ -53,6 +53,7 @@ struct BwdArgs {
   float* dv_acc;
   int* status;
   int split_chunk;             // row tiles per CTA when split
+  size_t acc_stride;           // compression, few chunks: floats between their accumulators (0: one for all, by atomics)
   int csize;                   // CTAs per cluster
   int B, Hq, Hkv, T, Lk, G, nq;
   int kind, window, block_size, S;
@@ -1241,7 +1242,8 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
             s_acc[(grp * kKeys + hc * 32 + c) * D + d] = __uint_as_float(r32[c]);
           } else if (key < p.Lk) {
             const size_t o = ((size_t)bh * p.Lk + key) * D + d;
-            if (split) atomicAdd((grp == 0 ? p.dv_acc : p.dk_acc) + o, __uint_as_float(r32[c]));
+            if (split && p.acc_stride) (grp == 0 ? p.dv_acc : p.dk_acc)[blockIdx.z * p.acc_stride + o] = __uint_as_float(r32[c]);
+            else if (split) atomicAdd((grp == 0 ? p.dv_acc : p.dk_acc) + o, __uint_as_float(r32[c]));
             else (grp == 0 ? p.dv : p.dk)[o] = __float2bfloat16_rn(__uint_as_float(r32[c]));
           }
         }
@@ -1497,6 +1499,32 @@ __global__ void sel_split_blocks_kernel(const int32_t* __restrict__ offsets, flo
   }
 }
 
+// dK and dV of the compression branch from the accumulators of up to kOrderedChunks chunks of row tiles, in a fixed order: the
+// last chunk of a key tile, which may be short, then the others as they come.  (The order in which atomics end up
+// when the CTAs run side by side; the gradient of the key pooling's position parameters is the rounding of
+// these sums, and 1e-2 of it moves with their order.)
+constexpr int kOrderedChunks = 4;
+__global__ void __launch_bounds__(256)
+cmp_chunks_kernel(const float* __restrict__ dk_acc, const float* __restrict__ dv_acc, __nv_bfloat16* __restrict__ dk,
+                  __nv_bfloat16* __restrict__ dv, size_t n8, size_t stride, int T, int Lk, int D, int cmp_len, int cmp_stride,
+                  int nq, int chunk) {
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n8) return;
+  const float* src = (blockIdx.y ? dv_acc : dk_acc) + i * 8;
+  const int key0 = (int)((i * 8 / D) % Lk) & ~(kKeys - 1);
+  const int n_q = max(0, T - (key0 * cmp_stride + cmp_len - 1));
+  const int chunks = ((n_q + nq - 1) / nq + chunk - 1) / chunk;
+  float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  for (int k = 0; k < chunks; ++k) {
+    const float4* row = reinterpret_cast<const float4*>(src + (size_t)(k == 0 ? chunks - 1 : k - 1) * stride);
+    const float4 a = __ldg(row), b = __ldg(row + 1);
+    acc[0] += a.x; acc[1] += a.y; acc[2] += a.z; acc[3] += a.w;
+    acc[4] += b.x; acc[5] += b.y; acc[6] += b.z; acc[7] += b.w;
+  }
+  *reinterpret_cast<uint4*>((blockIdx.y ? dv : dk) + i * 8) =
+      make_uint4(pack_bf16(acc[0], acc[1]), pack_bf16(acc[2], acc[3]), pack_bf16(acc[4], acc[5]), pack_bf16(acc[6], acc[7]));
+}
+
 static const char* const kBwdNames[3] = {"tc_bwd_win", "tc_bwd_cmp", "tc_bwd_slc"};
 static const char* const kRedNames[3] = {"dq_reduce_win", "dq_reduce_cmp", "dq_reduce_slc"};
 
@@ -1563,7 +1591,8 @@ static BwdPlan plan_bwd(const AttnArgs& a) {
     pl.split_chunk = 48;
     if (max_rt > pl.split_chunk) {
       pl.n_splits = (max_rt + pl.split_chunk - 1) / pl.split_chunk;
-      off += 2 * align_up((size_t)a.B * a.Hkv * a.Lk * a.D * sizeof(float), 256);
+      const size_t n_acc = pl.n_splits <= kOrderedChunks ? (size_t)pl.n_splits : 1;
+      off += 2 * align_up(n_acc * a.B * a.Hkv * a.Lk * a.D * sizeof(float), 256);
     }
   }
   // selection: blocks split over several work items use the same accumulators (launches and memory that up to
@@ -1614,9 +1643,12 @@ int tc_attn_bwd(const AttnArgs& a, void* ws, size_t ws_bytes, cudaStream_t st) {
   p.split_chunk = pl.split_chunk;
   p.csize = pl.csize;
   const size_t n_kv = (size_t)a.B * a.Hkv * a.Lk * a.D;
+  const bool roles = (get_option_bwd_kernel() == 1 || a.kind == 2) && !p.dq_acc_mode;   // compute groups relieved of the issuing
+  const bool ordered = roles && pl.n_splits > 1 && pl.n_splits <= kOrderedChunks && aligned16(p.dk, p.dv);
+  p.acc_stride = ordered ? n_kv : 0;
   p.dk_acc = (float*)(base + pl.off_acc);
-  p.dv_acc = (float*)(base + pl.off_acc + align_up(n_kv * sizeof(float), 256));
-  if (pl.n_splits > 1)
+  p.dv_acc = (float*)(base + pl.off_acc + align_up((ordered ? (size_t)pl.n_splits : 1) * n_kv * sizeof(float), 256));
+  if (pl.n_splits > 1 && !ordered)
     NSA_CUDA_OK(cudaMemsetAsync(base + pl.off_acc, 0, 2 * align_up(n_kv * sizeof(float), 256), st));
 
   const size_t rows = (size_t)a.B * a.Hq * a.T;
@@ -1669,7 +1701,6 @@ int tc_attn_bwd(const AttnArgs& a, void* ws, size_t ws_bytes, cudaStream_t st) {
   dim3 grid(pl.n_ktiles, a.B * a.Hkv, pl.n_splits);
   if (a.kind == 2)
     grid = dim3((unsigned)((size_t)a.B * a.Hkv * pl.layout.max_items));
-  const bool roles = (get_option_bwd_kernel() == 1 || a.kind == 2) && !p.dq_acc_mode;   // compute groups relieved of the issuing
   if (roles) {
     KernelScope ks(branch_name(kBwdNames, a.kind), st);
     grid.x *= (unsigned)pl.csize;
@@ -1715,7 +1746,13 @@ int tc_attn_bwd(const AttnArgs& a, void* ws, size_t ws_bytes, cudaStream_t st) {
                                                                         pl.n_ktiles, pl.nq, a.Lk, a.D, 1);
     NSA_LAUNCH_OK("sel_split_blocks_kernel");
   }
-  if (pl.n_splits > 1) {
+  if (ordered) {
+    KernelScope ks("cmp_chunks_kernel", st);
+    cmp_chunks_kernel<<<dim3((unsigned)((n_kv / 8 + 255) / 256), 2), 256, 0, st>>>(p.dk_acc, p.dv_acc, p.dk, p.dv, n_kv / 8, n_kv, a.T,
+                                                                                  a.Lk, a.D, a.block_size, a.window, pl.nq,
+                                                                                  pl.split_chunk);
+    NSA_LAUNCH_OK("cmp_chunks_kernel");
+  } else if (pl.n_splits > 1) {
     int rc2 = cast_f32_to(p.dk_acc, p.dk, n_kv, NSA_DTYPE_BF16, st);
     if (rc2 == NSA_OK) rc2 = cast_f32_to(p.dv_acc, p.dv, n_kv, NSA_DTYPE_BF16, st);
     if (rc2 != NSA_OK) return rc2;

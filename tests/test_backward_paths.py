@@ -257,3 +257,29 @@ def test_selection_plan_gives_the_same_results():
         for a, b in zip(g0[1:], g1[1:]):
             assert (a.float() - b.float()).abs().max().item() <= 2.0 ** -7 * max(b.float().abs().max().item(), 1e-6)
     assert nsa.lib().nsa_device_status(None) == 0
+
+
+@pytest.mark.parametrize("G,D,T,stride", [(4, 64, 1537, 16), (16, 128, 900, 32), (16, 64, 1400, 64), (2, 64, 9600, 64)])
+def test_compression_chunks_add_up_in_order(G, D, T, stride):
+    """49 to 192 row tiles of queries: two to four chunks a key tile, the last of them short, tiles with fewer chunks than
+    the first; the same bits on every run."""
+    nsa = pkg()
+    n = (T - stride) // stride + 1
+    g = torch.Generator().manual_seed(7)
+    q, do = (torch.randn(1, G, T, D, generator=g).bfloat16() for _ in range(2))
+    k, v = (torch.randn(1, 1, n, D, generator=g).bfloat16() for _ in range(2))
+    keep = torch.arange(T)[:, None] >= (torch.arange(n)[None, :] + 1) * stride - 1
+    live = keep.any(1)
+    s = (q.double() @ k.double().transpose(-1, -2) * D ** -0.5).masked_fill(~keep, float("-inf"))
+    p = torch.where(keep, torch.softmax(s.masked_fill(~live[:, None], 0.), -1), torch.zeros(()).double())
+    o64 = p @ v.double()
+    ds = p * (do.double() @ v.double().transpose(-1, -2) - (do.double() * o64).sum(-1, keepdim=True)) * D ** -0.5
+    want = (ds @ k.double(), (ds.transpose(-1, -2) @ q.double()).sum(1, keepdim=True), (p.transpose(-1, -2) @ do.double()).sum(1, keepdim=True))
+    args = [x.cuda() for x in (q, k, v)]
+    o, lse = nsa.range_attn_forward(*args, nsa.MODE_COMPRESS, 0, stride)
+    runs = [nsa.range_attn_backward(*args, o, lse, do.cuda(), nsa.MODE_COMPRESS, 0, stride) for _ in range(3)]
+    for got, ref in zip(runs[0], want):
+        assert (got.double().cpu() - ref).norm() <= 1e-2 * ref.norm()      # P and dS in bf16, as everywhere
+    for other in runs[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(runs[0][1:], other[1:]))
+    assert nsa.lib().nsa_device_status(None) == 0
