@@ -37,8 +37,8 @@ extern "C" {
 
 /* which kernel family serves a call */
 #define NSA_IMPL_AUTO 0   /* tcgen05 kernels when the shape allows, else the SIMT kernels; selection on blocks
-                             of 16 or 32 tokens with P and dS in two bf16 terms and fp32 dQ partials, or SIMT,
-                             whose arithmetic is fp32 throughout */
+                             of 16 or 32 tokens with P and dS in three bf16 terms (24 bits) and fp32 dQ
+                             partials, or, small calls among them, SIMT, whose arithmetic is fp32 throughout */
 #define NSA_IMPL_SIMT 1   /* CUDA-core kernels: any dtype, D in {16,32,64,128}, any G and block size */
 #define NSA_IMPL_TC   2   /* tcgen05/TMEM kernels only; NSA_ERR_UNSUPPORTED if the shape does not fit */
 
@@ -366,6 +366,8 @@ int nsa_profile_summary(char* buf, size_t cap);
  * its query-outer kernel (cheap when neighbouring queries share blocks) and its block-outer
  * kernel (cheap when they do not); 1 / 2 force one of them.  No counterpart in the reference
  * beyond its USE_FSA_FWD module flag (nsa_selection_kernel.py:48).
+ * "small_blocks_tc" (0 / 1): with 1 selection on blocks of 16 and 32 tokens goes to the tcgen05 kernels
+ * whatever the size of the call; with 0 (default) small calls stay on the CUDA cores.
  * "debug_starve_load" (0 / 1, tests only): with 1 the tcgen05 window / compression / query-outer
  * forward kernel never sends the load of its second V tile, so that CTA's bounded wait runs out
  * after about a second: it raises the status word, waits for what it has in flight, gives its

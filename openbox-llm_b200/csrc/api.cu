@@ -110,6 +110,7 @@ static std::atomic<int> g_opt_merged{1};
 int get_option_merged_boxes() { return g_opt_merged.load(); }
 static std::atomic<int> g_opt_starve{0};
 int get_option_debug_starve_load() { return g_opt_starve.load(); }
+static std::atomic<int> g_opt_small_blocks_tc{0};
 
 int check_dims(const NsaDims* d) {
   NSA_CHECK_ARG(d != nullptr, "dims is null");
@@ -131,8 +132,8 @@ AttnArgs base_args(const NsaDims* d, int Lk) {
   return a;
 }
 
-// Selection on blocks of 16 and 32 tokens is fp32 arithmetic under NSA_IMPL_AUTO: through the two-term tcgen05 kernels
-// (use_two_term) where they serve the call, else on the CUDA cores.  NSA_IMPL_TC asks for the plain
+// Selection on blocks of 16 and 32 tokens is fp32 arithmetic under NSA_IMPL_AUTO: through the three-term tcgen05 kernels
+// (use_three_term) or on the CUDA cores.  NSA_IMPL_TC asks for the plain
 // tcgen05 kernels, which keep P, dS and the dQ partials in bf16: against 64-bit arithmetic (T of 130 to 2047, D of 64
 // and 128) o and dq are off by 2.1e-3 to 2.6e-3 and 2.6e-3 to 2.9e-3 there, by 1.66e-3 and 1.7e-3, the rounding of
 // a bf16 result, otherwise.
@@ -147,12 +148,18 @@ bool use_tc(const NsaDims* d, int block_size, int impl, int* err) {
   return ok;
 }
 
-// Selection on blocks of 16 and 32 tokens through the tcgen05 kernels with P and dS in two bf16 terms (16 significant
-// bits; K, V, Q and dO are bf16 as they are).  The backward keeps fp32 dQ partials of S rows per query: beyond
-// 8 GB of them (half of what the bf16 partials of 64-token blocks take at 8 x 32768 tokens, 16 heads of 128, 16 blocks a
-// list) the CUDA-core kernels, which need none, serve the call.
-bool use_two_term(const NsaDims* d, int block_size, int S, int impl, bool bwd) {
+// Selection on blocks of 16 and 32 tokens through the tcgen05 kernels with P and dS in three bf16 terms (the 24
+// significant bits of fp32; K, V, Q and dO are bf16 as they are).
+// Small calls stay on the CUDA cores, where a forward with its backward ends sooner.  In products per matrix (rows x
+// listed keys x D; us on the CUDA cores | the tensor cores, forward and backward): 8.4 M (8 heads of 64, 256 tokens,
+// 4 blocks of 16) 15 + 28 | 13 + 43, 12.6 M (384 tokens) 17 + 45 | 16 + 48, 16.8 M (512 tokens) 19 + 42 | 19 + 40, 33 M (256
+// tokens, 8 blocks of 32) 29 + 54 | 13 + 43.
+// The backward keeps fp32 dQ partials of S rows per query: beyond 8 GB of them (half of what the bf16 partials of
+// 64-token blocks take at 8 x 32768 tokens, 16 heads of 128, 16 blocks a list) the CUDA-core kernels, which need none,
+// serve the call.
+bool use_three_term(const NsaDims* d, int block_size, int S, int impl, bool bwd) {
   if (impl != NSA_IMPL_AUTO || (block_size != 16 && block_size != 32) || S < 1 || !tc_shape_ok(*d, block_size)) return false;
+  if ((double)d->B * d->Hq * d->T * S * block_size * d->D <= 12e6 && !g_opt_small_blocks_tc.load()) return false;
   return !bwd || (double)d->B * d->Hq * d->T * S * d->D * sizeof(float) <= 8e9;
 }
 
@@ -219,6 +226,10 @@ extern "C" int nsa_set_option(const char* name, int value) {
   }
   if (name && strcmp(name, "debug_starve_load") == 0 && value >= 0 && value <= 1) {
     g_opt_starve.store(value);
+    return NSA_OK;
+  }
+  if (name && strcmp(name, "small_blocks_tc") == 0 && value >= 0 && value <= 1) {
+    g_opt_small_blocks_tc.store(value);
     return NSA_OK;
   }
   set_error("unknown option or value");
@@ -450,8 +461,8 @@ static int selection_fwd_impl(const void* q, const void* k, const void* v,
   a.q = q; a.k = k; a.v = v; a.o = o; a.lse = lse; a.block_idx = block_idx;
   a.kind = 2; a.S = S; a.block_size = block_size;
   a.sel_plan = plan;
-  a.two_term = use_two_term(dims, block_size, S, impl, false) && aligned16(q, k, v, o);
-  if (a.two_term || (use_tc(dims, block_size, impl, &rc) && S > 0))
+  a.three_term = use_three_term(dims, block_size, S, impl, false) && aligned16(q, k, v, o);
+  if (a.three_term || (use_tc(dims, block_size, impl, &rc) && S > 0))
     return tc_sel_fwd(a, workspace, workspace_bytes, (cudaStream_t)stream);
   if (rc != NSA_OK) return rc;
   return simt_attn_fwd(a, dims->dtype, (cudaStream_t)stream);
@@ -482,10 +493,10 @@ extern "C" size_t nsa_selection_bwd_workspace_bytes(const NsaDims* dims, int S, 
   if (check_sel(dims, S, block_size) != NSA_OK) return 0;
   int rc;
   size_t need = simt_bwd_ws(dims, dims->T);
-  const bool two_term = use_two_term(dims, block_size, S, impl, true);
-  if (two_term || use_tc(dims, block_size, impl, &rc)) {
+  const bool three_term = use_three_term(dims, block_size, S, impl, true);
+  if (three_term || use_tc(dims, block_size, impl, &rc)) {
     AttnArgs a = base_args(dims, dims->T);
-    a.kind = 2; a.S = S; a.block_size = block_size; a.two_term = two_term;
+    a.kind = 2; a.S = S; a.block_size = block_size; a.three_term = three_term;
     need = need > tc_attn_bwd_workspace(a) ? need : tc_attn_bwd_workspace(a);
   }
   return need;
@@ -533,9 +544,9 @@ static int selection_bwd_impl(const void* q, const void* k, const void* v,
   a.block_idx = block_idx; a.kind = 2; a.S = S; a.block_size = block_size;
   a.row_scale = row_scale; a.row_dot = row_dot;
   NSA_CHECK_ARG((row_scale == nullptr) == (row_dot == nullptr), "row_scale and row_dot go together");
-  a.two_term = dq && use_two_term(dims, block_size, S, impl, true) && aligned16(q, k, v, d_o, dq, dk, dv) &&
+  a.three_term = dq && use_three_term(dims, block_size, S, impl, true) && aligned16(q, k, v, d_o, dq, dk, dv) &&
                (row_dot || aligned16(o));
-  if (a.two_term || (use_tc(dims, block_size, impl, &rc) && S > 0)) {
+  if (a.three_term || (use_tc(dims, block_size, impl, &rc) && S > 0)) {
     a.dk_acc = (float*)dk;
     a.dv_acc = (float*)dv;
     a.sel_plan = plan;

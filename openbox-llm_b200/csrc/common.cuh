@@ -105,7 +105,7 @@ struct AttnArgs {
   const float* row_scale; const float* row_dot;   // backward of a gated branch (may be null)
   float* dq_acc;     // tcgen05 window / compression backward: fp32 accumulator [B*Hkv][T][G][D] that takes dQ (or null)
   const void* sel_plan;   // tcgen05 selection: plan built earlier (tc_sel_plan_build), or null
-  bool two_term;          // tcgen05 selection on 16- and 32-token blocks: P and dS in two bf16 terms, dQ partials in fp32
+  bool three_term;          // tcgen05 selection on 16- and 32-token blocks: P and dS in three bf16 terms, dQ partials in fp32
   // tcgen05 selection: where the block-outer kernel serves the call its merge blends the three branches as well
   // (gate logits, the other branches' outputs, the op's output; null g_out: it does not) and keeps `o` only
   // where o_kept says so

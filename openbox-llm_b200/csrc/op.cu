@@ -131,7 +131,7 @@ struct Carver {
 struct OpPlan {
   int n_cmp, S, es;
   bool fused;              // the three backward kernels leave their dQ partials to one reduction
-  bool two_term;           // selection on 16- and 32-token blocks on the tensor cores (api.cu), with fp32 partials
+  bool three_term;           // selection on 16- and 32-token blocks on the tensor cores (api.cu), with fp32 partials
   bool acc_mode;           // fused, and window and compression add to one fp32 dQ accumulator
   bool fast_pool;
   size_t n_q, n_kv, n_c, rows;    // elements of q, of one K/V tensor, of one summary tensor; rows of q
@@ -181,8 +181,8 @@ int op_plan(const NsaAttentionDesc* d, OpPlan* p) {
   int err;
   const bool tc = use_tc(&m, d->block_size, d->impl, &err);
   if (err != NSA_OK) return err;
-  p->two_term = use_two_term(&m, d->block_size, p->S, d->impl, true);
-  p->fused = (tc || p->two_term) && p->S > 0;
+  p->three_term = use_three_term(&m, d->block_size, p->S, d->impl, true);
+  p->fused = (tc || p->three_term) && p->S > 0;
   p->acc_mode = tc && p->fused && d->dq_accumulator;
   const bool grad = d->need_grad != 0;
 
@@ -212,7 +212,7 @@ int op_plan(const NsaAttentionDesc* d, OpPlan* p) {
   }
   const bool acc_mode = p->acc_mode;
   if (acc_mode) p->dq_acc = w.take(p->n_q * sizeof(float));
-  if (!p->fused || p->two_term) p->dq3 = w.take(3 * p->n_q * p->es);
+  if (!p->fused || p->three_term) p->dq3 = w.take(3 * p->n_q * p->es);
   p->ws_bytes[0] = acc_mode ? nsa_range_attn_bwd_acc_workspace_bytes(&m, p->n_cmp, NSA_MODE_COMPRESS_STRIDED, d->cmp_stride)
                             : nsa_range_attn_bwd_workspace_bytes(&m, p->n_cmp, NSA_MODE_COMPRESS_STRIDED, d->cmp_stride, d->impl);
   p->ws_bytes[1] = nsa_selection_bwd_workspace_bytes(&m, p->S, d->block_size, d->impl);
@@ -392,8 +392,8 @@ extern "C" int nsa_attention_bwd(const NsaAttentionDesc* d, const NsaAttentionTe
   void* dk_cmp = w + p.dk_cmp;
   void* dv_cmp = w + p.dv_cmp;
   const bool acc_mode = p.acc_mode;
-  // tensors off a 16-byte boundary keep the two-term selection, which loads by TMA, from serving the call
-  const bool fused = p.fused && !(p.two_term && !aligned16(t->q, t->ks, t->vs, t->d_out, t->dq, t->dks, t->dvs));
+  // tensors off a 16-byte boundary keep the three-term selection, which loads by TMA, from serving the call
+  const bool fused = p.fused && !(p.three_term && !aligned16(t->q, t->ks, t->vs, t->d_out, t->dq, t->dks, t->dvs));
   float* dq_acc = (float*)(w + p.dq_acc);
   void* ws[3];
   void* dq[3];             // where a branch puts its own dq (null: partials stay in its workspace)
@@ -444,7 +444,7 @@ extern "C" int nsa_attention_bwd(const NsaAttentionDesc* d, const NsaAttentionTe
   // selection
   if (fused) {
     AttnArgs a = base_args(&m, m.T);
-    a.two_term = p.two_term;
+    a.three_term = p.three_term;
     a.q = t->q; a.k = t->ks; a.v = t->vs; a.o = (void*)o[1]; a.lse = (float*)lse[1]; a.d_o = t->d_out; a.dq = nullptr;
     a.block_idx = t->block_idx; a.kind = 2; a.S = p.S; a.block_size = d->block_size;
     a.row_scale = rs[1]; a.row_dot = rd[1];
@@ -466,7 +466,7 @@ extern "C" int nsa_attention_bwd(const NsaAttentionDesc* d, const NsaAttentionTe
   if (!fused) return nsa_sum3(dq[0], dq[1], dq[2], t->dq, p.n_q, m.dtype, stream);
   // the three branches left their dQ partials in their workspaces (or two of them in the accumulator)
   AttnArgs a = base_args(&m, m.T);
-  a.two_term = p.two_term;
+  a.three_term = p.three_term;
   const int32_t* pos = sel_plan_pair_map(a, p.S, d->block_size, sv + p.plan);
   if (acc_mode)
     return tc_dq_reduce3(a, 0, 0, 0, p.S, d->block_size, 1, nullptr, ws[1], nullptr, pos, dq_acc, t->dq, st);

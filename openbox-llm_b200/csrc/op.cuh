@@ -7,7 +7,7 @@ namespace nsa {
 int check_dims(const NsaDims* d);
 AttnArgs base_args(const NsaDims* d, int Lk);
 bool use_tc(const NsaDims* d, int block_size, int impl, int* err);
-bool use_two_term(const NsaDims* d, int block_size, int S, int impl, bool bwd);
+bool use_three_term(const NsaDims* d, int block_size, int S, int impl, bool bwd);
 int topn_check(const NsaDims* dims, int n_cmp, int cmp_len, int cmp_stride, int sel_block, int n_sel, int n_init,
                int n_local, int impl);   // aux.cu
 // nsa_gate_combine_fwd, unless the block-outer kernel has served the selection (a choice without header: always)

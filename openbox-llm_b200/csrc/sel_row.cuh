@@ -1,4 +1,4 @@
-// Selection attention of single rows in scalar fp32, for the rows and key tiles that the two-term tcgen05 kernels
+// Selection attention of single rows in scalar fp32, for the rows and key tiles that the three-term tcgen05 kernels
 // cannot finish: a product of a masked probability (zero) with a value that is infinite or NaN is NaN, so where such a
 // value sits in a tile every row of the tile would carry it.  What comes out non-finite there is computed
 // again here from the row's own list, key by key, and stays with what attends the value.  Speed does not matter.

@@ -38,7 +38,7 @@ struct FwdArgs {
   int nw;                    // 32-bit membership words per block = ceil(nq / 32)
   int n_sub;                 // selection: list blocks per 64-key tile (64 / block_size)
   float scale_log2;
-  const __nv_bfloat16* q;    // two-term selection: the rows that are done again one by one
+  const __nv_bfloat16* q;    // three-term selection: the rows that are done again one by one
   const __nv_bfloat16* k;
   const __nv_bfloat16* v;
   float neg_zero;            // -0: what a product is added to where it has to be rounded by itself (a packed mul
@@ -52,7 +52,7 @@ template <int D> struct FwdSmem {
   static constexpr int kQBytes = kRows * 128 * kSlabs;
   static constexpr int kKVBytes = kKeys * 128 * kSlabs;
   static constexpr int kFixed = kQBytes + 2 * kStages * kKVBytes;
-  static constexpr int kBars = 9 + 4 * kStages;
+  static constexpr int kBars = 9 + 4 * kStages + (D == 128 ? 4 : 0);
 };
 
 __host__ __device__ inline size_t fwd_smem_bytes(int D, int nb_sel, int nw, int n_sub, int kind) {
@@ -109,11 +109,15 @@ __device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) {
 // other gradients.  Any other rounding here, or order of the sum in backward, is as exact and replaces
 // these values by others of their size.)
 //
-// kTwoTerm (selection on 16- and 32-token blocks, whose results are fp32 arithmetic rounded once): P goes to the
-// tensor cores as two bf16 terms, P - bf16(P) behind bf16(P), 16 significant bits in the 64 columns that S leaves
-// behind, at the price of a second product.  A block listed twice counts twice; a row whose result is not finite
-// (V of a key it does not attend may be infinite: zero times that is NaN) is done again by itself.
-template <int D, int kKind, bool kTwoTerm>
+// kThreeTerm (selection on 16- and 32-token blocks, whose results are fp32 arithmetic rounded once): P goes to the
+// tensor cores as three bf16 terms, each what the ones before it leave of P: all 24 bits of an fp32 value, at the price
+// of two more products.  The first two take the 64 columns that S leaves behind; the third has 32 columns of its own at
+// D = 64, those that O does not use, and at D = 128, where tensor memory is full, follows into the columns of the first
+// as soon as that one's product is done.  2 x 1024 tokens, 16 heads of 128, 8 blocks of 16 a list: 42 us (50 with columns
+// for all terms, which leave room for one CTA an SM; 32 with two terms, whose 16 bits show in sums that cancel; 27
+// with one).  A block listed twice counts twice; a row whose result is not finite (V of a key it does not attend may be
+// infinite: zero times that is NaN) is done again by itself.
+template <int D, int kKind, bool kThreeTerm>
 __global__ void __launch_bounds__(kFwdThreads, 2)
 tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
               const __grid_constant__ CUtensorMap tm_v, const FwdArgs p) {
@@ -121,9 +125,10 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   constexpr int kSlabs = L::kSlabs, kStages = L::kStages;
   constexpr bool kSel = kKind == 2, kCmp = kKind == 1;
   constexpr uint32_t kTmemCols = 256;
+  constexpr bool kLate = kThreeTerm && D == 128;    // the third term of P waits for the first to be used
   // O in columns 0-127, two buffers of S (P, bf16, is written over the first 32 columns of its S by the
-  // thread that read the row)
-  constexpr uint32_t kColO = 0, kColS = 128;
+  // thread that read the row; three-term: over all 64, and the third term of buffer b at kColP3 + b * kP3Step)
+  constexpr uint32_t kColO = 0, kColS = 128, kColP3 = kLate ? kColS : 64, kP3Step = kLate ? kKeys : 32;
   constexpr uint32_t kIdescQK = idesc_bf16(128, kKeys, 0, 0);
   constexpr uint32_t kIdescPV = idesc_bf16(128, D, 0, 1);
 
@@ -144,10 +149,12 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   uint64_t* bar_v = bar_k + kStages;           // [kStages] V stage landed
   uint64_t* k_free = bar_v + kStages;          // [kStages] the S MMA that read the stage is done
   uint64_t* v_free = k_free + kStages;         // [kStages] the PV MMA that read the stage is done
+  uint64_t* bar_p1 = v_free + kStages;         // kLate: [2] the product of P's first term is done
+  uint64_t* bar_p3 = bar_p1 + 2;               // kLate: [2] the 128 rows of the third term are written
   uint32_t* s_tmem = (uint32_t*)(bars + L::kBars);
   volatile int* s_abort = (volatile int*)(s_tmem + 1);
   int* s_ntiles = (int*)(s_tmem + 2);
-  int* s_repeats = (int*)(s_tmem + 3);              // two-term: a query of the row tile lists a block more than once
+  int* s_repeats = (int*)(s_tmem + 3);              // three-term: a query of the row tile lists a block more than once
   int* s_scan = (int*)(s_tmem + 4);                 // [129]
   uint32_t* s_member = (uint32_t*)(s_scan + 132);   // [nb_sel][n_sub][nw]   (selection only)
   const int tile_words = p.n_sub * p.nw;
@@ -163,6 +170,8 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     for (int k = 0; k < 2; ++k) { mbar_init(bar_s + k, 1); mbar_init(bar_p + k, kFwdSoftmax); mbar_init(bar_o + k, 1); }
     mbar_init(bar_drain, 1);
     for (int k = 0; k < 4 * kStages; ++k) mbar_init(bar_k + k, 1);
+    if (kLate)
+      for (int k = 0; k < 2; ++k) { mbar_init(bar_p1 + k, 1); mbar_init(bar_p3 + k, kFwdSoftmax); }
     fence_barrier_init();
     prefetch_tensormap(&tm_q); prefetch_tensormap(&tm_k); prefetch_tensormap(&tm_v);
   }
@@ -206,7 +215,7 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     const int bh = w % units, t0 = (p.n_qtiles - 1 - w / units) * p.nq, t_last = min(p.T - 1, t0 + p.nq - 1);
     const int n_vis = t_last / kKeys + 1;              // key tiles that start at or before the last query
     for (int i = tid; i < n_vis * tile_words; i += kFwdThreads) s_member[i] = 0u;
-    if (kTwoTerm && tid == 0) *s_repeats = 0;
+    if (kThreeTerm && tid == 0) *s_repeats = 0;
     __syncthreads();
     const int32_t* idx = p.block_idx + ((size_t)bh * p.T + t0) * p.S;
     const int n_entries = (t_last - t0 + 1) * p.S;
@@ -216,7 +225,7 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       // list block blk = part blk % n_sub of key tile blk / n_sub
       if (blk >= 0 && (long long)blk * p.block_size <= t0 + q_local) {
         const uint32_t was = atomicOr(&s_member[blk * p.nw + (q_local >> 5)], 1u << (q_local & 31));
-        if (kTwoTerm && (was >> (q_local & 31) & 1u)) *s_repeats = 1;
+        if (kThreeTerm && (was >> (q_local & 31) & 1u)) *s_repeats = 1;
       }
     }
     __syncthreads();
@@ -339,10 +348,20 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
 #pragma unroll
             for (int kk = 0; kk < kKeys / 16; ++kk)
               mma_ts(tmem + kColO, tmem + kColS + (c & 1) * kKeys + kk * 8, desc_at(va, kk * 2048), kIdescPV, (i > 0) || (kk > 0));
-            if (kTwoTerm)
+            if (kThreeTerm) {
+              if (kLate) tc_commit(bar_p1 + (c & 1));
 #pragma unroll
               for (int kk = 0; kk < kKeys / 16; ++kk)
                 mma_ts(tmem + kColO, tmem + kColS + (c & 1) * kKeys + 32 + kk * 8, desc_at(va, kk * 2048), kIdescPV, 1);
+              if (kLate) {
+                ok = mbar_wait(bar_p3 + (c & 1), (c >> 1) & 1, p.status, s_abort, 0x2000);
+                if (!ok) break;
+                tc_fence_after();
+              }
+#pragma unroll
+              for (int kk = 0; kk < kKeys / 16; ++kk)
+                mma_ts(tmem + kColO, tmem + kColP3 + (c & 1) * kP3Step + kk * 8, desc_at(va, kk * 2048), kIdescPV, 1);
+            }
             tc_commit(bar_o + (c & 1));
             tc_commit(v_free + st);
           }
@@ -368,8 +387,8 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           continue;
         }
         float m_used = -INFINITY, l_sum = 0.f;      // log2 units
-        bool listed = false;                        // two-term: the row attends a key
-        const bool repeats = kTwoTerm && *s_repeats;
+        bool listed = false;                        // three-term: the row attends a key
+        const bool repeats = kThreeTerm && *s_repeats;
         for (int i = 0; i < x.n_tiles; ++i, ++c) {
           const int key0 = key0_of(x, i);
           // valid columns of this row in this tile: one range [lo, hi] and, for selection, 16-column groups
@@ -410,7 +429,7 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           // whole tile or none of it needs no work per element (none: its P is set to zero below); only
           // rows whose range ends inside the tile, or that attend some 16-column groups of it, do.
           const bool none = hi < 0;
-          if (kTwoTerm) listed |= !none && groups != 0u;
+          if (kThreeTerm) listed |= !none && groups != 0u;
           if (!(lo <= 0 && (hi >= kKeys - 1 || none) && (!kSel || groups == 0xfu))) {
 #pragma unroll
             for (int cc = 0; cc < 64; ++cc)
@@ -434,7 +453,7 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           const uint64_t sc2 = pack_f32x2(p.scale_log2, p.scale_log2), mn2 = pack_f32x2(-msub, -msub);
           float psum = 0.f;
           float times[4] = {1.f, 1.f, 1.f, 1.f};     // how often the row's list names the block of a 16-column group
-          if (kTwoTerm && repeats && !none) {
+          if (kThreeTerm && repeats && !none) {
 #pragma unroll
             for (int k = 0; k < 4; ++k)
               times[k] = (float)times_listed(p.block_idx + ((size_t)x.bh * p.T + t) * p.S, p.S, (key0 + 16 * k) / p.block_size);
@@ -446,25 +465,40 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
                                    mn2), p0, p1);
             p0 = ex2(p0);
             p1 = ex2(p1);
-            if (kTwoTerm && repeats) {
+            if (kThreeTerm && repeats) {
               const float n = times[cc >> 3];
               p0 *= n;
               p1 *= n;
             }
             psum += p0 + p1;
             pk[cc] = pack_bf16(p0, p1);
-            if (kTwoTerm)
-              r[cc] = pack_bf16(p0 - __uint_as_float(pk[cc] << 16), p1 - __uint_as_float(pk[cc] & 0xffff0000u));
+            if (kThreeTerm) {                      // what the first term leaves, exactly
+              r[2 * cc] = __float_as_uint(p0 - __uint_as_float(pk[cc] << 16));
+              r[2 * cc + 1] = __float_as_uint(p1 - __uint_as_float(pk[cc] & 0xffff0000u));
+            }
           }
           if (none) {
             psum = 0.f;
 #pragma unroll
             for (int cc = 0; cc < 32; ++cc) pk[cc] = 0u;
-            if (kTwoTerm)
+            if (kThreeTerm)
 #pragma unroll
-              for (int cc = 0; cc < 32; ++cc) r[cc] = 0u;
+              for (int cc = 0; cc < 64; ++cc) r[cc] = 0u;
           }
           l_sum += psum;
+          if constexpr (kThreeTerm) {              // (before the rescaling below needs the registers)
+            tmem_st32(s_base, pk);
+#pragma unroll
+            for (int cc = 0; cc < 32; ++cc) {
+              pk[cc] = pack_bf16(__uint_as_float(r[2 * cc]), __uint_as_float(r[2 * cc + 1]));
+              r[2 * cc] = __float_as_uint(__uint_as_float(r[2 * cc]) - __uint_as_float(pk[cc] << 16));
+              r[2 * cc + 1] = __float_as_uint(__uint_as_float(r[2 * cc + 1]) - __uint_as_float(pk[cc] & 0xffff0000u));
+            }
+            tmem_st32(s_base + 32, pk);
+#pragma unroll
+            for (int cc = 0; cc < 32; ++cc) pk[cc] = pack_bf16(__uint_as_float(r[2 * cc]), __uint_as_float(r[2 * cc + 1]));
+            if (!kLate) tmem_st32(lane_base + kColP3 + (c & 1) * kP3Step, pk);
+          }
           // O may be touched once PV of the tile before is done; only a warp that has to rescale waits
           if (i > 0 && __any_sync(0xffffffffu, rescale)) {
             ok = mbar_wait(bar_o + ((c - 1) & 1), ((c - 1) >> 1) & 1, p.status, s_abort, 8);
@@ -480,11 +514,19 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
               tmem_st32(lane_base + kColO + cc * 32, o32);
             }
           }
-          tmem_st32(s_base, pk);                   // over the S columns this thread has just read
-          if (kTwoTerm) tmem_st32(s_base + 32, r);
+          if (!kThreeTerm) tmem_st32(s_base, pk);  // over the S columns this thread has just read
           tmem_wait_st();
           tc_fence_before();
           mbar_arrive(bar_p + (c & 1));
+          if constexpr (kLate) {
+            ok = mbar_wait(bar_p1 + (c & 1), (c >> 1) & 1, p.status, s_abort, 8);
+            if (!__all_sync(0xffffffffu, ok)) break;
+            tc_fence_after();
+            tmem_st32(lane_base + kColP3 + (c & 1) * kP3Step, pk);
+            tmem_wait_st();
+            tc_fence_before();
+            mbar_arrive(bar_p3 + (c & 1));
+          }
         }
         if (!__all_sync(0xffffffffu, ok)) break;
         // ---- this row tile's output: the last PV, then O / l -------------------------------------
@@ -498,7 +540,7 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           uint32_t o32[32];
           tmem_ld32(lane_base + kColO + cc * 32, o32);
           tmem_wait_ld();
-          if (kTwoTerm)
+          if (kThreeTerm)
 #pragma unroll
             for (int e = 0; e < 32; ++e) nan_sum = fmaf(__uint_as_float(o32[e]), 0.f, nan_sum);
           if (row_ok) {
@@ -515,7 +557,7 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           }
         }
         if (row_ok) *lrow = l_sum > 0.f ? (m_used + log2f(l_sum)) * kLn2 : kLseEmpty;
-        if (kTwoTerm && row_ok && listed && !(nan_sum == 0.f && l_sum > 0.f && l_sum < INFINITY))
+        if (kThreeTerm && row_ok && listed && !(nan_sum == 0.f && l_sum > 0.f && l_sum < INFINITY))
           sel_row_forward<D>(p.q + ((size_t)(b * p.Hq + head) * p.T + t) * D, p.k + (size_t)x.bh * p.Lk * D,
                              p.v + (size_t)x.bh * p.Lk * D, p.block_idx + ((size_t)x.bh * p.T + t) * p.S, p.S, p.block_size,
                              t, p.scale_log2, orow, lrow);
@@ -607,7 +649,7 @@ static int launch_fwd(const AttnArgs& a, const SelPlanHeader* plan, int force, c
     kernel<<<grid, kFwdThreads, smem, st>>>(tm_q, tm_k, tm_v, p);
     return NSA_OK;
   };
-  if (a.two_term)
+  if (a.three_term)
     rc = a.D == 128 ? go(tc_fwd_kernel<128, 2, true>) : go(tc_fwd_kernel<64, 2, true>);
   else if (a.D == 128)
     rc = a.kind == 2 ? go(tc_fwd_kernel<128, 2, false>) : a.kind == 1 ? go(tc_fwd_kernel<128, 1, false>) : go(tc_fwd_kernel<128, 0, false>);

@@ -41,14 +41,14 @@ struct BwdArgs {
   const __nv_bfloat16* k;
   const __nv_bfloat16* v;
   const __nv_bfloat16* d_o;
-  const int32_t* block_idx;    // two-term selection
+  const int32_t* block_idx;    // three-term selection
   const float* lse;
   const float* delta;          // sum_d dO * O per row (unscaled)
   const float* row_scale;      // gate value per row of a gated branch, or null
   SelPlan plan;                // selection
   __nv_bfloat16* dk;
   __nv_bfloat16* dv;
-  void* dq_part;               // bf16, fp32 for two-term selection
+  void* dq_part;               // bf16, fp32 for three-term selection
   float* dk_acc;               // fp32 accumulators, used when the row tiles of a key tile are split
   float* dv_acc;
   int* status;
@@ -565,26 +565,26 @@ constexpr int kB2Threads = 640;   // 2 x 8 compute warps, 3 producer warps, MMA 
 constexpr int kB2Producers = 3;
 constexpr int kB2Compute = 16;    // compute warps
 
-// kTwoTerm: selection on 16- and 32-token blocks, whose results are fp32 arithmetic rounded once.  P and dS go to
-// the tensor cores as two bf16 terms each (16 significant bits; the second adds three products of eight), the dQ
-// partials stay fp32, a block listed twice counts twice and what comes out non-finite is done again row by
-// row (sel_row.cuh).  P and dS take 64 KB of a slot, as much as its fp32 staging tile, so one slot fits at D = 128 and
-// two at D = 64.  The whole op on 16-token blocks, forward + backward (2 x 1024 tokens, 16 heads of 128, 8 blocks a
-// list): selection backward 157 us against 795 for the CUDA-core tiles, forward 37 against 367, the pass 356 against 1299.
-template <int D, bool kTwoTerm> struct Bwd2 {
+// kThreeTerm: selection on 16- and 32-token blocks, whose results are fp32 arithmetic rounded once.  P and dS go to
+// the tensor cores as three bf16 terms each, all 24 bits of the fp32 values (two more of each of the three products they
+// enter), the dQ partials stay fp32, a block listed twice counts twice and what comes out non-finite is done again row by
+// row (sel_row.cuh).  P and dS take 96 KB of a slot, so one slot fits.  The whole op on 16-token blocks, forward + backward (2 x 1024 tokens, 16 heads of 128, 8 blocks a
+// list): selection backward with its plan and dQ sum 199 us against 799 on the CUDA cores (182 with two terms), forward
+// 42 against 360, the pass 345 against 1300.
+template <int D, bool kThreeTerm> struct Bwd2 {
   static constexpr int kSlabs = D / 64;
-  static constexpr int kTerms = kTwoTerm ? 2 : 1;
-  static constexpr int kSlots = (D == 64 ? 3 : 2) - (kTwoTerm ? 1 : 0);
+  static constexpr int kTerms = kThreeTerm ? 3 : 1;
+  static constexpr int kSlots = kThreeTerm ? 1 : D == 64 ? 3 : 2;
   static constexpr int kKVBytes = kKeys * 128 * kSlabs;
   static constexpr int kRowBytes = kRows * 128 * kSlabs;            // Q or dO
-  static constexpr int kSlotBytes = 2 * kRowBytes + 2 * kTerms * kPBytes;    // dO, Q, P, dS (and P, dS: second terms)
+  static constexpr int kSlotBytes = 2 * kRowBytes + 2 * kTerms * kPBytes;    // dO, Q, P, dS (and P, dS: further terms)
   static constexpr int kBars = 2 + 7 * kSlots;
   static constexpr size_t kSmem = 2 * kKVBytes + (size_t)kSlots * kSlotBytes + 256 /*barriers*/ +
                                   (size_t)kSlots * 128 * 4 /*partial rows of a ragged tile*/ + 1024 /*alignment slack*/;
 };
 
 // dK and dV of one work item in scalar fp32, a warp to a row, into acc [dV, dK][64 keys][D] in shared memory, for
-// a tile whose sums are not finite (two-term selection).
+// a tile whose sums are not finite (three-term selection).
 template <int D>
 __device__ __noinline__ void sel_tile_dkdv(const BwdArgs& p, float* acc, int bh, int j, int pair_first, int n_rows,
                                            int n_threads) {
@@ -625,7 +625,7 @@ __device__ __noinline__ void sel_tile_dkdv(const BwdArgs& p, float* acc, int bh,
   __syncthreads();
 }
 
-// 32 columns of a row's dQ against one key tile in scalar fp32 (two-term selection, result not finite).
+// 32 columns of a row's dQ against one key tile in scalar fp32 (three-term selection, result not finite).
 template <int D>
 __device__ __noinline__ void sel_row_dq(const BwdArgs& p, float* acc, int bh, int head, int pair, int key0, int col0) {
   const int t = pair & (int)kPairPosMask;
@@ -647,13 +647,13 @@ __device__ __noinline__ void sel_row_dq(const BwdArgs& p, float* acc, int bh, in
   }
 }
 
-template <int D, bool kCluster, bool kTwoTerm>
+template <int D, bool kCluster, bool kThreeTerm>
 __global__ void __launch_bounds__(kB2Threads, 1)
 tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
                const __grid_constant__ CUtensorMap tm_q_run, const __grid_constant__ CUtensorMap tm_do_run,
                const __grid_constant__ CUtensorMap tm_dq, const __grid_constant__ BwdArgs p) {
-  using L = Bwd2<D, kTwoTerm>;
+  using L = Bwd2<D, kThreeTerm>;
   constexpr int kSlabs = L::kSlabs, kSlots = L::kSlots, kKVBytes = L::kKVBytes;
   constexpr uint32_t kTmemCols = 512;
   // slot s: S at 128 s, dP at 128 s + 64, dQ over both; then dV^T and dK^T: at D = 128 64 columns each, at D = 64
@@ -915,7 +915,7 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
             tc_fence_after();
             const uint8_t* sDO = sSlot + sbb * L::kSlotBytes;
             const uint8_t* sP = sDO + 2 * L::kRowBytes;
-            const uint8_t* sDS = sP + kPBytes;       // (two-term: P, dS, then their second terms)
+            const uint8_t* sDS = sP + kPBytes;       // (three-term: P, dS, then their further terms)
             const uint32_t dsk = desc_lo_kmajor(smem_u32(sDS));
 #pragma unroll
             for (uint32_t term = 0; term < L::kTerms * 2 * kPBytes; term += 2 * kPBytes) {
@@ -991,7 +991,7 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
       delta_cur = __ldg(p.delta + row_index(t_cur));
       if (p.row_scale) gate_cur = __ldg(p.row_scale + row_index(t_cur));
     }
-    const bool repeats = kTwoTerm && __ldg(&p.plan.hdr->repeats) != 0ull;
+    const bool repeats = kThreeTerm && __ldg(&p.plan.hdr->repeats) != 0ull;
     // A given-up wait does not part a group: its warps go on to the barrier below, which decides for all.
     for (int k = grp; k < k_end; k += kGroups) {
       const int sb = k % kSlots, u = k / kSlots;
@@ -1025,7 +1025,7 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
       // every column of this thread's half is attended (the usual case away from the diagonal)?
       const bool all_cols = lo <= half * 32 && hi >= half * 32 + 31 && groups == 0x3u && !repeats;
       float times[2] = {1.f, 1.f};                   // how often the row's list names the blocks of its column groups
-      if (kTwoTerm && repeats && t_cur >= 0) {
+      if (kThreeTerm && repeats && t_cur >= 0) {
         const int32_t* list = p.block_idx + ((size_t)bh * p.T + (t_cur & (int)kPairPosMask)) * p.S;
 #pragma unroll
         for (int e = 0; e < 2; ++e) times[e] = (float)times_listed(list, p.S, (key0 + half * 32 + 16 * e) / p.block_size);
@@ -1046,14 +1046,15 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
         tmem_ld32(lane_base + 64 + half * 32, rp);
         tmem_wait_ld();
         uint32_t pp[16], pd[16];
-        uint32_t pp2[kTwoTerm ? 16 : 1], pd2[kTwoTerm ? 16 : 1];   // second terms
+        // the values as bf16; three-term: they stay in fp32 where S and dP were, for the terms to be taken off
         auto put = [&](int c2, float p0, float p1, float d0, float d1) {
+          if (kThreeTerm) {
+            rs[c2 * 2] = __float_as_uint(p0); rs[c2 * 2 + 1] = __float_as_uint(p1);
+            rp[c2 * 2] = __float_as_uint(d0); rp[c2 * 2 + 1] = __float_as_uint(d1);
+            return;
+          }
           pp[c2] = pack_bf16(p0, p1);
           pd[c2] = pack_bf16(d0, d1);
-          if (kTwoTerm) {
-            pp2[c2] = pack_bf16(p0 - __uint_as_float(pp[c2] << 16), p1 - __uint_as_float(pp[c2] & 0xffff0000u));
-            pd2[c2] = pack_bf16(d0 - __uint_as_float(pd[c2] << 16), d1 - __uint_as_float(pd[c2] & 0xffff0000u));
-          }
         };
         if (__all_sync(0xffffffffu, all_cols)) {
 #pragma unroll
@@ -1072,10 +1073,10 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
               const int c = half * 32 + c2 * 2 + e;
               const bool in = (c >= lo) && (c <= hi) && ((groups >> (c2 >> 3)) & 1u);
               float pr = in ? ex2(fmaf(__uint_as_float(rs[c2 * 2 + e]), p.scale_log2, -lse2)) : 0.f;
-              if (kTwoTerm) pr *= times[c2 >> 3];
+              if (kThreeTerm) pr *= times[c2 >> 3];
               pv[e] = pr;
               dv[e] = pr * fmaf(__uint_as_float(rp[c2 * 2 + e]), dscale, -ddelta);
-              if (kTwoTerm && !in) dv[e] = 0.f;      // (dP of a key that is not attended may be infinite)
+              if (kThreeTerm && !in) dv[e] = 0.f;      // (dP of a key that is not attended may be infinite)
             }
             put(c2, pv[0], pv[1], dv[0], dv[1]);
           }
@@ -1084,12 +1085,26 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
 #pragma unroll
         for (int k4 = 0; k4 < 4; ++k4) {
           const uint32_t chunk16 = (uint32_t)((half * 4 + k4) ^ (row & 7)) << 4;
+          if (kThreeTerm) {
+            auto terms = [&](uint32_t at, uint32_t* v) {         // eight fp32 values; what a term leaves is exact
+#pragma unroll
+              for (int term = 0; term < L::kTerms; ++term) {
+                uint32_t b[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                  b[e] = pack_bf16(__uint_as_float(v[2 * e]), __uint_as_float(v[2 * e + 1]));
+                  v[2 * e] = __float_as_uint(__uint_as_float(v[2 * e]) - __uint_as_float(b[e] << 16));
+                  v[2 * e + 1] = __float_as_uint(__uint_as_float(v[2 * e + 1]) - __uint_as_float(b[e] & 0xffff0000u));
+                }
+                st_shared_v4(at + term * 2 * kPBytes, b[0], b[1], b[2], b[3]);
+              }
+            };
+            terms(p_row + chunk16, rs + k4 * 8);
+            terms(ds_row + chunk16, rp + k4 * 8);
+            continue;
+          }
           st_shared_v4(p_row + chunk16, pp[k4 * 4], pp[k4 * 4 + 1], pp[k4 * 4 + 2], pp[k4 * 4 + 3]);
           st_shared_v4(ds_row + chunk16, pd[k4 * 4], pd[k4 * 4 + 1], pd[k4 * 4 + 2], pd[k4 * 4 + 3]);
-          if (kTwoTerm) {
-            st_shared_v4(p_row + 2 * kPBytes + chunk16, pp2[k4 * 4], pp2[k4 * 4 + 1], pp2[k4 * 4 + 2], pp2[k4 * 4 + 3]);
-            st_shared_v4(ds_row + 2 * kPBytes + chunk16, pd2[k4 * 4], pd2[k4 * 4 + 1], pd2[k4 * 4 + 2], pd2[k4 * 4 + 3]);
-          }
         }
       }
       fence_proxy_async();
@@ -1112,7 +1127,7 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
           tc_fence_before();
           mbar_arrive(dq_read + sb);
         }
-        if (kTwoTerm) {                    // fp32 staging: slabs of 128 rows x 32 columns
+        if (kThreeTerm) {                    // fp32 staging: slabs of 128 rows x 32 columns
           float z = 0.f;                   // x * 0: 0 or NaN
 #pragma unroll
           for (int e = 0; e < 32; ++e) z = fmaf(__uint_as_float(r32[e]), 0.f, z);
@@ -1163,14 +1178,14 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
           const int slot = p.kind == 2 ? 0 : (p.kind == 0 ? j % p.n_slots : j);
           const int mid = p.kind == 2 ? pair_base + i * p.nq : t_lo + i * p.nq;
           const int outer = p.kind == 2 ? 0 : bh;
-          constexpr int kParts = kTwoTerm ? D / 32 : kSlabs;
+          constexpr int kParts = kThreeTerm ? D / 32 : kSlabs;
 #pragma unroll
           for (int sl = 0; sl < kParts; ++sl)
             tma_store_5d_hint(&tm_dq, stage + sl * (kRows * 128), sl * (D / kParts), 0, slot, mid, outer, l2_policy_evict_first());
           bulk_commit();
         }
       } else {   // the ragged last tile: whole rows out by hand, 16 bytes a lane
-        constexpr int kChunks = kTwoTerm ? D / 4 : D / 8;
+        constexpr int kChunks = kThreeTerm ? D / 4 : D / 8;
         constexpr int kRowsPerPass = 256 / kChunks;
         const int c = lt % kChunks;
         for (int r = lt / kChunks; r < kRows; r += kRowsPerPass) {
@@ -1192,7 +1207,7 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
   tc_fence_after();
   bool redone = false;
   float* s_acc = reinterpret_cast<float*>(sSlot);      // cluster: [dV, dK][64 keys][D], over the slots
-  if (kTwoTerm) {
+  if (kThreeTerm) {
     // sums that are not finite are formed again, leaving out what a row does not attend
     float z = 0.f;
     if (warp < kB2Compute && ((warp >> 2) & 1) == 0 && !*s_abort) {
@@ -1454,7 +1469,7 @@ static Reduce3Args reduce_args(const AttnArgs& a, void* dq) {
   return r;
 }
 
-// f32: the selection's partials are fp32 (two-term)
+// f32: the selection's partials are fp32 (three-term)
 static int reduce_launch(const Reduce3Args& r, int D, bool f32, const char* name, cudaStream_t st) {
   const int hg = r.G % 2 == 0 ? 2 : (r.G % 3 == 0 ? 3 : 1);   // heads of a query served by one thread
   const size_t nthreads = (size_t)r.B * r.Hkv * r.T * (r.G / hg) * (D / 8);
@@ -1561,7 +1576,7 @@ static BwdPlan plan_bwd(const AttnArgs& a) {
   }
   size_t off = 0;
   pl.off_delta = off; off += align_up((size_t)a.B * a.Hq * a.T * sizeof(float), 256);
-  pl.off_part = off; off += align_up(part_rows * G * a.D * (a.two_term ? 4 : 2), 256);
+  pl.off_part = off; off += align_up(part_rows * G * a.D * (a.three_term ? 4 : 2), 256);
   pl.off_plan = off;
   if (a.kind == 2) {
     pl.layout = sel_plan_layout((int)units, a.T, a.S, pl.nq);
@@ -1692,7 +1707,7 @@ int tc_attn_bwd(const AttnArgs& a, void* ws, size_t ws_bytes, cudaStream_t st) {
     rc = make_map_dq_acc(&tm_dqacc, a.dq_acc, a.D, G, (size_t)a.T, (size_t)a.B * a.Hkv, pl.nq);
     tm_dq = tm_dqacc;        // the partial-tile map is not used in this mode
   } else if (rc == NSA_OK) {
-    rc = a.kind == 2 ? make_map_partial(&tm_dq, p.dq_part, a.D, G, 1, pl.cap_pairs ? pl.cap_pairs : 1, 1, pl.nq, a.two_term)
+    rc = a.kind == 2 ? make_map_partial(&tm_dq, p.dq_part, a.D, G, 1, pl.cap_pairs ? pl.cap_pairs : 1, 1, pl.nq, a.three_term)
                      : make_map_partial(&tm_dq, p.dq_part, a.D, G, pl.n_slots, a.T, (size_t)a.B * a.Hkv, pl.nq);
     tm_dqacc = tm_dq;        // likewise
   }
@@ -1707,7 +1722,7 @@ int tc_attn_bwd(const AttnArgs& a, void* ws, size_t ws_bytes, cudaStream_t st) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(kB2Threads);
-    cfg.dynamicSmemBytes = a.two_term ? (a.D == 128 ? Bwd2<128, true>::kSmem : Bwd2<64, true>::kSmem)
+    cfg.dynamicSmemBytes = a.three_term ? (a.D == 128 ? Bwd2<128, true>::kSmem : Bwd2<64, true>::kSmem)
                                       : (a.D == 128 ? Bwd2<128, false>::kSmem : Bwd2<64, false>::kSmem);
     cfg.stream = st;
     cudaLaunchAttribute attr;
@@ -1721,7 +1736,7 @@ int tc_attn_bwd(const AttnArgs& a, void* ws, size_t ws_bytes, cudaStream_t st) {
       NSA_CUDA_OK(cudaLaunchKernelEx(&cfg, kernel, tm_k, tm_v, tm_q, tm_do, tm_q_run, tm_do_run, tm_dq, p));
       return NSA_OK;
     };
-    if (a.two_term) {
+    if (a.three_term) {
       if (a.D == 128) rc = pl.csize > 1 ? go(tc_bwd2_kernel<128, true, true>) : go(tc_bwd2_kernel<128, false, true>);
       else rc = pl.csize > 1 ? go(tc_bwd2_kernel<64, true, true>) : go(tc_bwd2_kernel<64, false, true>);
     } else if (a.D == 128) {
@@ -1764,7 +1779,7 @@ int tc_attn_bwd(const AttnArgs& a, void* ws, size_t ws_bytes, cudaStream_t st) {
     r.part_cmp = (const __nv_bfloat16*)p.dq_part; r.slots_cmp = pl.n_slots;
     r.Lk_cmp = a.Lk; r.cmp_len = a.block_size; r.cmp_stride = a.window;
   } else { r.part_slc = p.dq_part; r.pair_of_slot = p.plan.pair_of_slot; r.S = a.S; }
-  return reduce_launch(r, a.D, a.two_term, branch_name(kRedNames, a.kind), st);
+  return reduce_launch(r, a.D, a.three_term, branch_name(kRedNames, a.kind), st);
 }
 
 // dq of the whole op from the three branch workspaces (each written by tc_attn_bwd with a null
@@ -1779,7 +1794,7 @@ int tc_dq_reduce3(const AttnArgs& base, int Lk_cmp, int cmp_len, int cmp_stride,
   r.acc = dq_acc;
   r.Lk_cmp = Lk_cmp; r.cmp_len = cmp_len; r.cmp_stride = cmp_stride; r.S = S; r.window = window;
   if (ws_cmp) {
-    AttnArgs a = base; a.two_term = false; a.kind = 1; a.Lk = Lk_cmp; a.block_size = cmp_len; a.window = cmp_stride;
+    AttnArgs a = base; a.three_term = false; a.kind = 1; a.Lk = Lk_cmp; a.block_size = cmp_len; a.window = cmp_stride;
     const BwdPlan pl = plan_bwd(a);
     r.part_cmp = (const __nv_bfloat16*)((const char*)ws_cmp + pl.off_part);
     r.slots_cmp = pl.n_slots;
@@ -1791,12 +1806,12 @@ int tc_dq_reduce3(const AttnArgs& base, int Lk_cmp, int cmp_len, int cmp_stride,
     r.pair_of_slot = pos ? pos : sel_plan_at((const char*)ws_slc + pl.off_plan, pl.layout).pair_of_slot;
   }
   if (ws_win) {
-    AttnArgs a = base; a.two_term = false; a.kind = 0; a.Lk = base.T; a.window = window;
+    AttnArgs a = base; a.three_term = false; a.kind = 0; a.Lk = base.T; a.window = window;
     const BwdPlan pl = plan_bwd(a);
     r.part_win = (const __nv_bfloat16*)((const char*)ws_win + pl.off_part);
     r.slots_win = pl.n_slots;
   }
-  return reduce_launch(r, base.D, base.two_term, "dq_reduce3", st);
+  return reduce_launch(r, base.D, base.three_term, "dq_reduce3", st);
 }
 
 }  // namespace nsa

@@ -162,9 +162,9 @@ int tc_fwdpair_launch(const AttnArgs& a, const SelPlan& plan, void* o_part, floa
 // A query tile meets at most the key tiles there are, and a full list names S of them: where there
 // are no more than 3.5 S key tiles the query-outer kernel is the cheaper one whatever the lists say
 // (prefer_pairs), so the call is that one kernel and needs neither plan nor workspace.
-// The two-term form exists query-outer only.
+// The three-term form exists query-outer only.
 static bool query_outer_only(const AttnArgs& a) {
-  return a.two_term || (get_option_sel_fwd() == 0 && 2LL * ((a.T + tc::kKeys - 1) / tc::kKeys) <= 7LL * a.S);
+  return a.three_term || (get_option_sel_fwd() == 0 && 2LL * ((a.T + tc::kKeys - 1) / tc::kKeys) <= 7LL * a.S);
 }
 
 size_t tc_sel_fwd_workspace(const AttnArgs& a) { return query_outer_only(a) ? 0 : tc::plan_pairs(a).total; }

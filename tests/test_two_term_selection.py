@@ -1,5 +1,6 @@
-"""Selection on 16- and 32-token blocks by default: the tcgen05 kernels with P and dS in two bf16 terms against the
-CUDA-core kernels (fp32 throughout) and against 64-bit arithmetic, over the forms of a call that both accept."""
+"""Selection on 16- and 32-token blocks by default: the tcgen05 kernels with P and dS in bf16 terms (three of them: the 24
+bits of fp32) against the CUDA-core kernels (fp32 throughout) and against 64-bit arithmetic, over the forms of a call
+that both accept; at small sizes too, which go to the CUDA cores otherwise."""
 import pytest
 import torch
 
@@ -11,7 +12,9 @@ pytestmark = pytest.mark.gpu
 
 @pytest.fixture(autouse=True)
 def _reset():
+    pkg().set_option("small_blocks_tc", 1)
     yield
+    pkg().set_option("small_blocks_tc", 0)
     pkg().set_impl("auto")
 
 
@@ -132,3 +135,33 @@ def test_views_off_a_16_byte_boundary():
     got = nsa.nsa_fused_forward(*ins, idx, 16, 64)
     assert ((got.float() - want.float()).abs() <= 2.0 ** -6 * want.float().abs().clamp(min=1)).all()
     assert nsa.lib().nsa_device_status(None) == 0
+
+
+@pytest.mark.parametrize("D,bs,S", [(64, 16, 4), (128, 16, 8), (64, 32, 4), (128, 32, 4)])
+def test_sums_that_cancel_keep_the_bits_of_fp32(D, bs, S):
+    """Scores close to one another and values that are +64 and -64 in turn: what is left of the sum is 2^-9 of its terms, so
+    that 16 bits of P show (12 % over the rounding of the result, where fp32 stays within 1 %)."""
+    T = 300
+    g = torch.Generator().manual_seed(3)
+    q, do = (torch.randn(1, 8, T, D, generator=g).bfloat16() for _ in range(2))
+    k, v = (torch.randn(1, 2, T, D, generator=g).bfloat16() for _ in range(2))
+    q = q / 512
+    v[..., 0] = torch.where(torch.arange(T) % 2 == 0, 64., -64.)
+    c = dict(B=1, Hq=8, Hkv=2, D=D, T=T, block_size=bs, S=S)
+    idx = make_inputs(c, torch.bfloat16, seed=1)["block_idx"]
+    got, want = _both(*(x.cuda() for x in (q, k, v, do)), idx.cuda(), bs)
+    o64 = _selection_64(dict(q=q, ks=k, vs=v, do=do), idx, bs)[0][..., 0]
+    err = [((x[0][..., 0].double().cpu() - o64).norm() / o64.norm()).item() for x in (got, want)]
+    assert err[0] <= 1.03 * err[1], err
+
+
+def test_small_calls_give_the_bits_of_the_cuda_cores():
+    """The layer's default sizes, and one size past the line."""
+    nsa = pkg()
+    nsa.set_option("small_blocks_tc", 0)
+    for T, same in ((256, True), (500, False)):
+        t = make_inputs(dict(B=1, Hq=8, Hkv=2, D=64, T=T, block_size=16, S=4), torch.bfloat16, seed=3)
+        ins = [dev(t[n], torch.bfloat16) for n in ("q", "ks", "vs", "do")]
+        got, want = _both(*ins, t["block_idx"].cuda(), 16)
+        assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1]) or not same
+        _close(got, want, T)
