@@ -606,7 +606,8 @@ extern "C" int nsa_block_mean_pool_fwd(const void* x, void* out, int B, int Hkv,
   const size_t n = (size_t)B * Hkv * n_blk * D;
   if (n == 0) return NSA_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  if (pool_vec_ok(D, dtype, x, out)) {
+  // Head sizes that do not fill a warp evenly (24, 48, 80, 96; above 128 fp32 or 256 bf16) go by elements.
+  if (pool_vec_ok(D, dtype, x, out) && pool_mean_ok(D, dtype)) {
     PoolSides p = {};
     p.n = 1; p.x[0] = x; p.out[0] = out;
     return pool_mean_fwd(p, B, Hkv, T, D, block_size, dtype, st);

@@ -460,7 +460,7 @@ __global__ void mean_fwd_kernel(const PoolSides s, int T_, int Dv, int len, int 
   constexpr int N = Vec<T>::N;
   const size_t row = (size_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= rows) return;
-  const int lane = threadIdx.x & 31, d = lane & (Dv - 1), step = 32 / Dv;      // Dv: a power of two up to 32
+  const int lane = threadIdx.x & 31, d = lane & (Dv - 1), step = 32 / Dv;      // Dv: a power of two up to 32 (pool_mean_ok)
   const size_t bh = row / n_sum, j = row % n_sum;
   const uint4* p = reinterpret_cast<const uint4*>(s.x[blockIdx.y]) + (bh * T_ + j * len) * Dv + d;
   float a[N];
@@ -594,8 +594,16 @@ int pool_learned_bwd(const PoolSides& s, int B, int H, int T, int D, int len, in
   return NSA_OK;
 }
 
+// Rows of 1, 2, 4 ... 32 vectors of 16 bytes, which is how mean_fwd_kernel lays a token over the lanes of a warp.
+bool pool_mean_ok(int D, int dtype) {
+  const int per = dtype == NSA_DTYPE_BF16 ? 8 : 4;
+  const int Dv = D / per;
+  return D > 0 && D % per == 0 && Dv <= 32 && (Dv & (Dv - 1)) == 0;
+}
+
 int pool_mean_fwd(const PoolSides& s, int B, int H, int T, int D, int len, int dtype, cudaStream_t st) {
   if (int bad = check_vectors(s)) return bad;
+  NSA_CHECK_ARG(pool_mean_ok(D, dtype), "mean pooling by warps: rows have to be 1, 2, 4 ... 32 vectors of 16 bytes");
   const int n_sum = T / len;
   const size_t rows = (size_t)B * H * n_sum;
   if (rows == 0) return NSA_OK;

@@ -32,6 +32,7 @@ bool pool_learned_ok(int D, int len, int dtype);
 size_t pool_acc_floats(int D, int len);        // accumulators and the arrival counter of one side
 int pool_learned_fwd(const PoolSides& s, int B, int H, int T, int D, int len, int stride, cudaStream_t st);
 int pool_learned_bwd(const PoolSides& s, int B, int H, int T, int D, int len, int stride, cudaStream_t st);
+bool pool_mean_ok(int D, int dtype);           // sizes that pool_mean_fwd takes
 int pool_mean_fwd(const PoolSides& s, int B, int H, int T, int D, int len, int dtype, cudaStream_t st);
 int pool_mean_bwd(const PoolSides& s, int B, int H, int T, int D, int len, int dtype, cudaStream_t st);
 
