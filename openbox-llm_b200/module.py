@@ -17,9 +17,25 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 from torch.nn.modules.module import _has_any_global_hook
+from torch.utils._device import DeviceContext
 
 from . import _lib as L
 from .ops import fused_projection_width, heads_to_tokens, nsa_attention, one_node_ok, split_heads, switches
+
+_LINEAR, _LINEAR_FORWARD = F.linear, nn.Linear.forward
+
+
+def _plain_linear(m):
+    """Whether calling m is F.linear and nothing else: no other class, hook, or patched forward."""
+    return (type(m) is nn.Linear and getattr(m.forward, "__func__", None) is _LINEAR_FORWARD and F.linear is _LINEAR
+            and not _has_any_global_hook()
+            and not (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks))
+
+
+def _function_modes():
+    """Whether a TorchFunctionMode is active that may look at calls (the default-device mode only sees factories)."""
+    return any(type(torch._C._get_function_stack_at(i)) is not DeviceContext
+               for i in range(torch._C._len_torch_function_stack()))
 
 
 class _Compressor(nn.Module):
@@ -67,11 +83,10 @@ class NSAAttentionB200(nn.Module):
 
     def _one_node(self, x, block_idx):
         """The layer as one node, where it is what a call of its modules comes to: bf16 autocast, fp32 weights, an
-        out_proj that is a plain Linear without hooks; None where it is not."""
+        out_proj that is a plain Linear, nobody who watches torch's functions; None where it is not."""
         o = self.out_proj
         if not (one_node_ok() and torch.is_autocast_enabled("cuda") and torch.get_autocast_dtype("cuda") is torch.bfloat16
-                and type(o) is nn.Linear and o.bias is None and not _has_any_global_hook()
-                and not (o._forward_hooks or o._forward_pre_hooks or o._backward_hooks or o._backward_pre_hooks)):
+                and _plain_linear(o) and o.bias is None and not _function_modes()):
             return None
         k, v = self.comp_k, self.comp_v
         return L.torch_op().layer(

@@ -186,3 +186,48 @@ def test_blend_in_the_merge(D):
     assert not torch.equal(outs[0], outs[1])
     assert (outs[0] - outs[1]).abs().max() <= 2.0 ** -6 and (outs[0] - outs[1]).norm() <= 2.0 ** -8 * outs[0].norm()
     assert nsa.lib().nsa_device_status(None) == 0
+
+
+def _layer(dh=64, Hq=8, Hkv=2):
+    mod = importlib.import_module("openbox-llm_b200.module")
+    torch.manual_seed(3)
+    layer = mod.NSAAttentionB200(Hq * dh, Hq, Hkv, block_size=64, n_selected_blocks=2, window=40).cuda()
+    for n, p in layer.named_parameters():
+        p.data.normal_(0, 0.02)
+    return layer, torch.randn(2, 200, Hq * dh, device="cuda")
+
+
+def test_out_proj_is_called_where_it_is_more_than_a_linear(monkeypatch):
+    """A forward set on the instance or the class, a replaced F.linear and an active TorchFunctionMode take part in the call as
+    they do in a call of the modules; the default-device mode does not keep the node away."""
+    layer, x = _layer()
+    lin = torch.nn.Linear.forward
+
+    def call():
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            return layer(x)
+    want = call()
+    assert "LayerNode" in want.grad_fn.name()
+    with torch.device("cuda"):
+        assert "LayerNode" in call().grad_fn.name()
+    layer.out_proj.forward = lambda t: lin(layer.out_proj, t) + 1
+    assert torch.equal(call(), want + 1)
+    del layer.out_proj.forward
+    assert torch.equal(call(), want)
+    with monkeypatch.context() as m:
+        m.setattr(torch.nn.Linear, "forward", lambda self, t: lin(self, t) + 1)
+        assert torch.equal(call(), want + 1)
+    seen = []
+    with monkeypatch.context() as m:
+        real = torch.nn.functional.linear
+        m.setattr(torch.nn.functional, "linear", lambda *a, **k: (seen.append(a[1].shape), real(*a, **k))[1])
+        assert torch.equal(call(), want)
+    assert len(seen) == 2
+
+    class Mode(torch.overrides.TorchFunctionMode):
+        def __torch_function__(self, func, types, args=(), kwargs=None):
+            seen.append(func)
+            return func(*args, **(kwargs or {}))
+    with Mode():
+        assert torch.equal(call(), want)
+    assert seen.count(torch.nn.functional.linear) == 2
