@@ -146,6 +146,7 @@ NsaAttentionDesc unpack(AutogradContext* ctx) {
 }
 // what a saved-tensor hook gave back may lie anywhere
 Tensor aligned(const Tensor& t) {
+  if (!t.defined()) return t;
   const Tensor c = t.contiguous();
   return (reinterpret_cast<uintptr_t>(c.data_ptr()) & 15) ? c.clone() : c;
 }
@@ -210,6 +211,7 @@ struct Layer {
   int64_t B, T, dm, width, n_attn;
 };
 struct LayerNode : torch::autograd::Function<LayerNode> {
+  // keep: what the backward reads; a GEMM's operand only where the gradient that reads it is asked for
   static Tensor run(Layer& l, bool need_grad, variable_list* keep) {
     const NsaDims& m = l.c.d.dims;
     const auto opt = l.x.options().dtype(at::kBFloat16);
@@ -247,7 +249,10 @@ struct LayerNode : torch::autograd::Function<LayerNode> {
     check(nsa_swap_heads_tokens(o.data_ptr(), tokens.data_ptr(), m.B, m.Hq, m.T, m.D, NSA_DTYPE_BF16, 1, raw_stream(l.x)));
     Tensor out = at::mm(tokens, w_out.t()).view({l.B, l.T, l.dm});
     if (keep) {
-      *keep = {c.in[0], kv, c.in[7], c.block_idx, saved, xb, w, w_out, tokens};
+      bool weights = false;
+      for (const Tensor& t : l.w) weights |= t.requires_grad();
+      *keep = {c.in[0], kv, c.in[7], c.block_idx, saved, weights ? xb : Tensor(), l.x.requires_grad() ? w : Tensor(), w_out,
+               l.w_out.requires_grad() ? tokens : Tensor()};
       keep->insert(keep->end(), c.comp, c.comp + 6);
     }
     return out;
@@ -268,6 +273,12 @@ struct LayerNode : torch::autograd::Function<LayerNode> {
     c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::autocast_dispatch_keyset);
     variable_list res(18);                      // l, x, w[8], bias, w_out, comp[6]
     if (!g[0].defined()) return res;
+    // x: 0, w: 1..8, bias: 9, w_out: 10, comp: 11..16.  Nothing is done for what no one asks for.
+    bool dw_any = false, rows_any = ctx->needs_input_grad(0) || ctx->needs_input_grad(9), op_any = false;
+    for (int k = 1; k < 9; ++k) dw_any |= ctx->needs_input_grad(k);
+    rows_any |= dw_any;
+    for (int k = 11; k < 17; ++k) op_any |= ctx->needs_input_grad(k);
+    op_any |= rows_any;
     const NsaAttentionDesc d = unpack(ctx);
     const NsaDims& m = d.dims;
     variable_list kept = ctx->get_saved_variables();
@@ -277,10 +288,12 @@ struct LayerNode : torch::autograd::Function<LayerNode> {
     in[0] = kept[0];
     in[7] = kept[2];
     for (int k = 0; k < 6; ++k) in[1 + k] = kv.select(0, k);
-    const int64_t rows = (int64_t)m.B * m.T, hd = (int64_t)m.Hq * m.D, dm = xb.size(1), width = w.size(0);
-    const auto opt = xb.options();
+    const int64_t rows = (int64_t)m.B * m.T, hd = (int64_t)m.Hq * m.D, dm = w_out.size(0);
+    const int64_t width = nsa_fused_projection_width(m.Hq, m.Hkv, m.D);
+    const auto opt = kv.options();
     const Tensor dy = aligned(g[0].to(at::kBFloat16)).view({rows, dm});
     if (ctx->needs_input_grad(10)) res[11] = at::mm(dy.t(), tokens, at::kFloat);
+    if (!op_any) return res;
     Tensor d_tokens = at::mm(dy, w_out), d_out = at::empty({m.B, m.Hq, m.T, m.D}, opt);
     check(nsa_swap_heads_tokens(d_tokens.data_ptr(), d_out.data_ptr(), m.B, m.Hq, m.T, m.D, NSA_DTYPE_BF16, 0, raw_stream(dy)));
     Tensor d_in[8], d_comp[6], d_kv = at::empty_like(kv);
@@ -288,6 +301,8 @@ struct LayerNode : torch::autograd::Function<LayerNode> {
     d_in[7] = at::empty_like(in[7]);
     for (int k = 0; k < 6; ++k) d_in[1 + k] = d_kv.select(0, k);
     op_backward(d, in, kept.data() + 9, kept[3], kept[4], d_out, d_in, d_comp);
+    for (int k = 0; k < 6; ++k) res[12 + k] = d_comp[k];
+    if (!rows_any) return res;
     Tensor d_rows = at::empty({rows, width}, opt);
     check(nsa_merge_heads(d_in[0].data_ptr(), d_kv.data_ptr(), d_in[7].data_ptr(), d_rows.data_ptr(), m.B, m.T, m.Hq, m.Hkv, m.D,
                           NSA_DTYPE_BF16, raw_stream(dy)));
@@ -295,9 +310,7 @@ struct LayerNode : torch::autograd::Function<LayerNode> {
       Tensor dx = ctx->saved_data["x_bf16"].toBool() ? at::mm(d_rows, w) : at::mm(d_rows, w, at::kFloat);
       res[1] = dx.view({m.B, m.T, dm});
     }
-    bool any = false;
-    for (int k = 0; k < 8; ++k) any |= ctx->needs_input_grad(1 + k);
-    if (any) {
+    if (dw_any) {
       const Tensor dw = at::mm(d_rows.t(), xb, at::kFloat);
       int64_t row = 0;
       for (int k = 0; k < 8; ++k) {
@@ -307,7 +320,6 @@ struct LayerNode : torch::autograd::Function<LayerNode> {
       }
     }
     if (ctx->needs_input_grad(9)) res[10] = d_rows.narrow(1, hd + 6 * (int64_t)m.Hkv * m.D, 3 * m.Hq).sum({0}, false, at::kFloat);
-    for (int k = 0; k < 6; ++k) res[12 + k] = d_comp[k];
     return res;
   }
 };
@@ -426,9 +438,10 @@ PyObject* py_layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (!fill_desc(c, l.B, Hq, Hkv, l.T, D, at::kBFloat16, ints + 2, true, given) || !comp_ok(c, dev)) return none();
   bool need = false;
   if (at::GradMode::is_enabled()) {
-    need = x.requires_grad() || l.bias.requires_grad() || l.w_out.requires_grad();
+    need = x.requires_grad() || l.bias.requires_grad();
     for (const Tensor& t : l.w) need |= t.requires_grad();
     for (const Tensor& t : c.comp) need |= t.requires_grad();
+    if (!need && l.w_out.requires_grad()) return none();      // the op has no backward then: out_proj is a node by itself
   }
   Tensor out;
   {

@@ -231,3 +231,50 @@ def test_out_proj_is_called_where_it_is_more_than_a_linear(monkeypatch):
     with Mode():
         assert torch.equal(call(), want)
     assert seen.count(torch.nn.functional.linear) == 2
+
+
+def test_frozen_parameters_cost_nothing():
+    """With only out_proj trainable, or some other part of the layer, what a forward keeps and what a backward launches is no
+    more than what the modules keep and launch, and the gradients are theirs."""
+    nsa = pkg()
+    layer, x = _layer()
+    x = torch.cat([x] * 8)                       # 2.5 MB of activations a tensor: the weights are smaller
+    do = torch.randn_like(x).bfloat16()
+    names = [n for n, _ in layer.named_parameters()]
+    parts = {"out_proj": ["out_proj.weight"], "compressor": [n for n in names if n.startswith("comp_")], "x": ["x"],
+             "bias": ["gate.bias"], "weights": ["q_proj.weight", "v_win.weight"], "out_proj and compressor": ["out_proj.weight", "comp_k.proj.weight"]}
+
+    requested = lambda: torch.cuda.memory_stats()["requested_bytes.all.current"]     # without what the allocator rounds up
+
+    def run(what, asked=None):
+        leaves = []
+        for n, p in layer.named_parameters():
+            p.requires_grad_(n in what)
+            if n in what and n in (asked or what):
+                leaves.append(p)
+        xs = x.detach().requires_grad_("x" in what)
+        if "x" in (asked or what):
+            leaves.append(xs)
+        torch.cuda.synchronize()
+        base = requested()
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            y = layer(xs)
+        held, before = requested() - base, nsa.lib().nsa_launch_count()
+        g = torch.autograd.grad(y, leaves, do)
+        return y.detach(), g, held, nsa.lib().nsa_launch_count() - before
+
+    for name, what in parts.items():
+        run(what)
+        got = run(what)
+        hook = layer.out_proj.register_forward_hook(lambda *a: None)
+        run(what)
+        want = run(what)
+        hook.remove()
+        assert torch.equal(got[0], want[0]), name
+        for a, b in zip(got[1], want[1]):
+            assert a.dtype == b.dtype and (a.float() - b.float()).norm() <= 2.0 ** -6 * b.float().norm() + 1e-3, name
+        assert got[2] <= want[2] + 64 * 1024, (name, got[2], want[2])
+        assert got[3] <= want[3], (name, got[3], want[3])
+    # trainable, but not asked for
+    assert run(names, ["out_proj.weight"])[3] == 0
+    assert run(names, ["out_proj.weight", "comp_v.proj.weight"])[3] < run(names, ["q_proj.weight"])[3]
