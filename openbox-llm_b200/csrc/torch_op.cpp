@@ -151,6 +151,21 @@ Tensor aligned(const Tensor& t) {
   return (reinterpret_cast<uintptr_t>(c.data_ptr()) & 15) ? c.clone() : c;
 }
 
+// The kernels' gradients have no derivative here.  Where a graph of the backward is asked for (create_graph), they
+// come out of nodes that say so when they are differentiated, instead of as constants.
+struct Once : torch::autograd::Function<Once> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& g) { return g.detach(); }
+  static variable_list backward(AutogradContext*, variable_list) {
+    TORCH_CHECK(false, "libnsa_b200: the gradients of the op cannot be differentiated again");
+  }
+};
+variable_list once(variable_list res) {
+  if (at::GradMode::is_enabled())
+    for (Tensor& g : res)
+      if (g.defined()) g = Once::apply(g.detach().requires_grad_(true));
+  return res;
+}
+
 // ---- the whole op -------------------------------------------------------------------------------------
 struct OpNode {
   template <typename... A>
@@ -189,7 +204,7 @@ struct OpMean : torch::autograd::Function<OpMean> {
                         const Tensor& vs, const Tensor& kw, const Tensor& vw, const Tensor& gate) {
     return OpNode::run(ctx, c);
   }
-  static variable_list backward(AutogradContext* ctx, variable_list g) { return OpNode::grads(ctx, g); }
+  static variable_list backward(AutogradContext* ctx, variable_list g) { return once(OpNode::grads(ctx, g)); }
 };
 struct OpLearned : torch::autograd::Function<OpLearned> {
   static Tensor forward(AutogradContext* ctx, Call* c, const Tensor& q, const Tensor& kc, const Tensor& vc, const Tensor& ks,
@@ -197,7 +212,7 @@ struct OpLearned : torch::autograd::Function<OpLearned> {
                         const Tensor& c1, const Tensor& c2, const Tensor& c3, const Tensor& c4, const Tensor& c5) {
     return OpNode::run(ctx, c);
   }
-  static variable_list backward(AutogradContext* ctx, variable_list g) { return OpNode::grads(ctx, g); }
+  static variable_list backward(AutogradContext* ctx, variable_list g) { return once(OpNode::grads(ctx, g)); }
 };
 
 // ---- the layer under bf16 autocast: projections, op and out_proj in one node ----------------------------
@@ -270,6 +285,14 @@ struct LayerNode : torch::autograd::Function<LayerNode> {
     return out;
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
+    variable_list res;
+    {
+      at::NoGradGuard no_grad;
+      res = grads(ctx, g);
+    }
+    return once(std::move(res));
+  }
+  static variable_list grads(AutogradContext* ctx, const variable_list& g) {
     c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::autocast_dispatch_keyset);
     variable_list res(18);                      // l, x, w[8], bias, w_out, comp[6]
     if (!g[0].defined()) return res;

@@ -626,6 +626,18 @@ def _op_forward(q, kv, gate_logits, block_idx, block_size, n_sel, window, forced
     return out, block_idx, (tensors, cp, saved, desc, bwd_bytes)
 
 
+class _Once(torch.autograd.Function):
+    """Gradients that cannot be differentiated again, where a graph of the backward is asked for."""
+
+    @staticmethod
+    def forward(ctx, g):
+        return g.detach()
+
+    @staticmethod
+    def backward(ctx, _):
+        raise RuntimeError("libnsa_b200: the gradients of the op cannot be differentiated again")
+
+
 class _NSAAttention(torch.autograd.Function):
     """The whole op in one node: pooling -> compression attention (+LSE) -> block scoring and
     top-n -> selection attention -> window attention -> gate combine.  Saves q once."""
@@ -669,6 +681,8 @@ class _NSAAttention(torch.autograd.Function):
         if gate_dtype != d_out.dtype:
             grads[7] = grads[7].to(gate_dtype)
         d_cp = [g if g.dtype == t else g.to(t) for g, t in zip(d_cp, comp_dtypes)]
+        if torch.is_grad_enabled():
+            grads, d_cp = ([_Once.apply(g.requires_grad_(True)) for g in gs] for gs in (grads, d_cp))
         return (*grads, None, None, None, None, None, *d_cp)
 
 

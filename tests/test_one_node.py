@@ -278,3 +278,31 @@ def test_frozen_parameters_cost_nothing():
     # trainable, but not asked for
     assert run(names, ["out_proj.weight"])[3] == 0
     assert run(names, ["out_proj.weight", "comp_v.proj.weight"])[3] < run(names, ["q_proj.weight"])[3]
+
+
+def test_gradients_are_not_differentiated_again():
+    """create_graph: the same gradients, which may be used and changed, and an error where a second derivative would have to
+    come through the kernels: in the layer and in the op, through its C++ and its Python node."""
+    nsa = pkg()
+    layer, x = _layer()
+    ins, comp, idx, do = _op_inputs(torch.bfloat16, 64, 64)
+    strided = ins[0].transpose(1, 2).contiguous().transpose(1, 2)        # goes to the Python node
+
+    def the_layer(x):
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            return layer(x)
+    for f, x0 in ((the_layer, x), (lambda q: nsa.nsa_attention(q, *ins[1:], 64, 3, 70, compressor=comp), ins[0]),
+                  (lambda q: nsa.nsa_attention(q, *ins[1:], 64, 3, 70, compressor=comp), strided)):
+        leaf = x0.detach().requires_grad_(True)
+        want, = torch.autograd.grad(f(leaf).float().square().sum(), leaf)
+        y = f(leaf).float().square().sum()
+        g, = torch.autograd.grad(y, leaf, create_graph=True)
+        _close(g.detach(), want, "first")
+        for loss in (g.float().square().sum(), y + g.float().square().sum()):
+            with pytest.raises(RuntimeError, match="differentiated again"):
+                loss.backward(retain_graph=True)
+        leaf.grad = None                        # (what the failed passes reached before they failed)
+        f(leaf).float().square().sum().backward(create_graph=True)
+        with torch.no_grad():
+            leaf.grad.mul_(2.)
+        _close(leaf.grad.detach(), 2 * want, "second")
