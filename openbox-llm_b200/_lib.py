@@ -4,6 +4,7 @@ import ctypes
 import functools
 import importlib.util
 import os
+import warnings
 
 import torch
 
@@ -119,19 +120,31 @@ _ext = None
 EXT_PATH = os.path.join(_HERE, "csrc", "_nsa_torch.so")
 
 
+def _load_ext():
+    if not os.path.exists(EXT_PATH):
+        raise ImportError("it has not been built")
+    spec = importlib.util.spec_from_file_location("_nsa_torch", EXT_PATH)
+    mod = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(mod)
+    if mod.torch_version != torch.__version__:
+        raise ImportError(f"it was built against torch {mod.torch_version}, this is {torch.__version__}")
+    mod.set_error(NsaError)
+    return mod
+
+
 def torch_op():
-    """The autograd nodes in C++ (csrc/torch_op.cpp); raise if they have not been built."""
+    """The autograd nodes in C++ (csrc/torch_op.cpp), or None, with one warning, where they have not been built or were
+    built against another torch: the same kernels are then called by the Python nodes, at the price of host time."""
     global _ext
     if _ext is None:
         lib()
-        if not os.path.exists(EXT_PATH):
-            raise NsaError(f"{EXT_PATH} is missing: build it with `python {_HERE}/build.py`")
-        spec = importlib.util.spec_from_file_location("_nsa_torch", EXT_PATH)
-        mod = importlib.util.module_from_spec(spec)
-        spec.loader.exec_module(mod)
-        mod.set_error(NsaError)
-        _ext = mod
-    return _ext
+        try:
+            _ext = _load_ext()
+        except ImportError as e:
+            warnings.warn(f"libnsa_b200: calls go through the Python nodes, {EXT_PATH} does not serve them: {e}; "
+                          f"build it with `python {_HERE}/build.py`", RuntimeWarning, stacklevel=2)
+            _ext = False
+    return _ext or None
 
 
 def check(rc):

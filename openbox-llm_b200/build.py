@@ -47,17 +47,35 @@ def _compile_ext():
     cuda = os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include") if os.path.sep in _nvcc() else "/usr/local/cuda/include"
     cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-D_GLIBCXX_USE_CXX11_ABI=%d" % _torch()._C._GLIBCXX_USE_CXX11_ABI,
            "-I" + inc, "-I" + os.path.join(inc, "torch", "csrc", "api", "include"), "-I" + sysconfig.get_paths()["include"],
-           "-I" + cuda, "-c", os.path.join(CSRC, "torch_op.cpp"), "-o", EXT_OBJ]
-    return subprocess.run(cmd, capture_output=True, text=True)
+           "-I" + cuda, '-DNSA_TORCH_VERSION="%s"' % _torch().__version__, "-c", os.path.join(CSRC, "torch_op.cpp"), "-o", EXT_OBJ]
+    try:
+        return subprocess.run(cmd, capture_output=True, text=True)
+    except OSError as e:                       # no host compiler by that name
+        return subprocess.CompletedProcess(cmd, 1, "", str(e))
+
+
+def _link_ext(r):
+    if r.returncode == 0:
+        home = os.path.join(os.path.dirname(_torch().__file__), "lib")
+        r = subprocess.run(["g++", "-shared", "-o", EXT, EXT_OBJ, "-L" + CSRC, "-l:libnsa_b200.so", "-Wl,-rpath,$ORIGIN",
+                            "-L" + home, "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python", "-ltorch"],
+                           capture_output=True, text=True)
+    if r.returncode != 0:
+        sys.stderr.write(r.stdout + r.stderr)
+        if os.path.exists(EXT):
+            os.remove(EXT)
+        print("warning: _nsa_torch.so could not be built: calls go through the Python nodes", file=sys.stderr)
 
 
 def build_library(force=False, verbose=False):
-    """Compile every .cu under csrc/ and link libnsa_b200.so.  Skips the work when the
-    sources are unchanged since the last build.  Returns the library path."""
+    """Compile every .cu under csrc/ and link libnsa_b200.so; then _nsa_torch.so, which the package can do without: where
+    it does not build, a warning says so.  Skips the work when the sources are unchanged since the last build.  Returns
+    the library path."""
     stamp_file = os.path.join(CSRC, ".build_stamp")
     stamp = _stamp()
-    if (not force and os.path.exists(LIB) and os.path.exists(EXT) and os.path.exists(stamp_file)
-            and open(stamp_file).read() == stamp):
+    if not force and os.path.exists(LIB) and os.path.exists(stamp_file) and open(stamp_file).read() == stamp:
+        if not os.path.exists(EXT):
+            _link_ext(_compile_ext())
         return LIB
     objs = [os.path.join(CSRC, src[:-3] + ".o") for src in SOURCES]
 
@@ -77,15 +95,7 @@ def build_library(force=False, verbose=False):
     if r.returncode != 0:
         sys.stderr.write(r.stdout + r.stderr)
         raise RuntimeError("link failed")
-    r = ext.result()
-    if r.returncode == 0:
-        home = os.path.join(os.path.dirname(_torch().__file__), "lib")
-        r = subprocess.run(["g++", "-shared", "-o", EXT, EXT_OBJ, "-L" + CSRC, "-l:libnsa_b200.so", "-Wl,-rpath,$ORIGIN",
-                            "-L" + home, "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python", "-ltorch"],
-                           capture_output=True, text=True)
-    if r.returncode != 0:
-        sys.stderr.write(r.stdout + r.stderr)
-        raise RuntimeError("building _nsa_torch failed")
+    _link_ext(ext.result())
     with open(os.path.join(CSRC, "ptxas.log"), "w") as f:
         f.write("\n".join(log))
     with open(stamp_file, "w") as f:

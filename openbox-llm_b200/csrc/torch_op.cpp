@@ -497,4 +497,8 @@ PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_nsa_torch", nullptr, -1, kMethod
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__nsa_torch() { return PyModule_Create(&kModule); }
+PyMODINIT_FUNC PyInit__nsa_torch() {
+  PyObject* m = PyModule_Create(&kModule);
+  if (m && PyModule_AddStringConstant(m, "torch_version", NSA_TORCH_VERSION) != 0) Py_CLEAR(m);
+  return m;
+}

@@ -714,9 +714,10 @@ def _dual_level():
 
 
 def one_node_ok():
-    """Whether the nodes in C++ may serve a call: outside of forward-mode levels and traces, and without a look at the
-    device status after every call."""
-    return not _dual_level() and not L.CHECK_STATUS_EVERY_CALL and torch._C._get_tracing_state() is None
+    """Whether the nodes in C++ may serve a call: where they are built, outside of forward-mode levels and traces, and
+    without a look at the device status after every call."""
+    return (not _dual_level() and not L.CHECK_STATUS_EVERY_CALL and torch._C._get_tracing_state() is None
+            and L.torch_op() is not None)
 
 
 def switches():
