@@ -212,7 +212,7 @@ int op_plan(const NsaAttentionDesc* d, OpPlan* p) {
   }
   const bool acc_mode = p->acc_mode;
   if (acc_mode) p->dq_acc = w.take(p->n_q * sizeof(float));
-  if (!p->fused || p->three_term) p->dq3 = w.take(3 * p->n_q * p->es);
+  if (!p->fused) p->dq3 = w.take(3 * p->n_q * p->es);
   p->ws_bytes[0] = acc_mode ? nsa_range_attn_bwd_acc_workspace_bytes(&m, p->n_cmp, NSA_MODE_COMPRESS_STRIDED, d->cmp_stride)
                             : nsa_range_attn_bwd_workspace_bytes(&m, p->n_cmp, NSA_MODE_COMPRESS_STRIDED, d->cmp_stride, d->impl);
   p->ws_bytes[1] = nsa_selection_bwd_workspace_bytes(&m, p->S, d->block_size, d->impl);
@@ -392,14 +392,14 @@ extern "C" int nsa_attention_bwd(const NsaAttentionDesc* d, const NsaAttentionTe
   void* dk_cmp = w + p.dk_cmp;
   void* dv_cmp = w + p.dv_cmp;
   const bool acc_mode = p.acc_mode;
-  // tensors off a 16-byte boundary keep the three-term selection, which loads by TMA, from serving the call
-  const bool fused = p.fused && !(p.three_term && !aligned16(t->q, t->ks, t->vs, t->d_out, t->dq, t->dks, t->dvs));
+  NSA_CHECK_ARG(!p.three_term || aligned16(t->q, t->ks, t->vs, t->d_out, t->dq),
+                "q, ks, vs, d_out and dq have to start on a 16-byte boundary");
   float* dq_acc = (float*)(w + p.dq_acc);
   void* ws[3];
   void* dq[3];             // where a branch puts its own dq (null: partials stay in its workspace)
   for (int k = 0; k < 3; ++k) {
     ws[k] = w + p.ws[k];
-    dq[k] = fused ? nullptr : w + p.dq3 + k * p.n_q * p.es;
+    dq[k] = p.fused ? nullptr : w + p.dq3 + k * p.n_q * p.es;
   }
   if (p.acc_bytes) NSA_CUDA_OK(cudaMemsetAsync(w + p.acc, 0, p.acc_bytes, st));
   if (acc_mode) NSA_CUDA_OK(cudaMemsetAsync(dq_acc, 0, p.n_q * sizeof(float), st));
@@ -442,7 +442,7 @@ extern "C" int nsa_attention_bwd(const NsaAttentionDesc* d, const NsaAttentionTe
     NSA_TRY(pool_mean_bwd(s, m.B, m.Hkv, m.T, m.D, d->block_size, m.dtype, s_cmp));
   }
   // selection
-  if (fused) {
+  if (p.fused) {
     AttnArgs a = base_args(&m, m.T);
     a.three_term = p.three_term;
     a.q = t->q; a.k = t->ks; a.v = t->vs; a.o = (void*)o[1]; a.lse = (float*)lse[1]; a.d_o = t->d_out; a.dq = nullptr;
@@ -463,7 +463,7 @@ extern "C" int nsa_attention_bwd(const NsaAttentionDesc* d, const NsaAttentionTe
     NSA_TRY(nsa_range_attn_bwd(t->q, t->kw, t->vw, o[2], lse[2], t->d_out, dq[2], t->dkw, t->dvw, &m, m.T,
                                NSA_MODE_WINDOW, d->window, 0, rs[2], rd[2], ws[2], p.ws_bytes[2], d->impl, s_win));
   NSA_TRY(fork.join());
-  if (!fused) return nsa_sum3(dq[0], dq[1], dq[2], t->dq, p.n_q, m.dtype, stream);
+  if (!p.fused) return nsa_sum3(dq[0], dq[1], dq[2], t->dq, p.n_q, m.dtype, stream);
   // the three branches left their dQ partials in their workspaces (or two of them in the accumulator)
   AttnArgs a = base_args(&m, m.T);
   a.three_term = p.three_term;

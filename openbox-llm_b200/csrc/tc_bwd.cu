@@ -727,8 +727,12 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
         const int key = key0 + i / (D / 8);
         if (key < p.Lk) {
           const size_t off = ((size_t)bh * p.Lk + key) * D + (i % (D / 8)) * 8;
-          *reinterpret_cast<uint4*>(p.dk + off) = make_uint4(0, 0, 0, 0);
-          *reinterpret_cast<uint4*>(p.dv + off) = make_uint4(0, 0, 0, 0);
+          if ((((uintptr_t)p.dk | (uintptr_t)p.dv) & 15) == 0) {
+            *reinterpret_cast<uint4*>(p.dk + off) = make_uint4(0, 0, 0, 0);
+            *reinterpret_cast<uint4*>(p.dv + off) = make_uint4(0, 0, 0, 0);
+          } else {                       // a caller's tensor may start anywhere
+            for (int e = 0; e < 8; ++e) p.dk[off + e] = p.dv[off + e] = __float2bfloat16_rn(0.f);
+          }
         }
       }
     }
@@ -1286,8 +1290,13 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
             float* dst = (which == 0 ? p.dv_acc : p.dk_acc) + o;
             atomicAdd(dst, acc.x); atomicAdd(dst + 1, acc.y); atomicAdd(dst + 2, acc.z); atomicAdd(dst + 3, acc.w);
           } else {
-            *reinterpret_cast<uint2*>((which == 0 ? p.dv : p.dk) + o) =
-                make_uint2(pack_bf16(acc.x, acc.y), pack_bf16(acc.z, acc.w));
+            __nv_bfloat16* dst = (which == 0 ? p.dv : p.dk) + o;
+            if (((uintptr_t)dst & 7) == 0) {
+              *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16(acc.x, acc.y), pack_bf16(acc.z, acc.w));
+            } else {                                     // a caller's tensor may start anywhere
+              dst[0] = __float2bfloat16_rn(acc.x); dst[1] = __float2bfloat16_rn(acc.y);
+              dst[2] = __float2bfloat16_rn(acc.z); dst[3] = __float2bfloat16_rn(acc.w);
+            }
           }
         }
       }
