@@ -165,3 +165,36 @@ def test_small_calls_give_the_bits_of_the_cuda_cores():
         got, want = _both(*ins, t["block_idx"].cuda(), 16)
         assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1]) or not same
         _close(got, want, T)
+
+
+# past the plan that one cluster builds (2048 tokens, 64 units); S that divides 32 and S that does not; row tiles of a ragged end
+@pytest.mark.parametrize("B,Hq,Hkv,D,T,bs,S", [(1, 4, 2, 64, 2100, 16, 4), (1, 8, 2, 128, 2100, 32, 5), (1, 4, 1, 64, 2049, 16, 5),
+                                               (33, 4, 2, 64, 130, 16, 4), (33, 6, 2, 64, 130, 32, 3), (17, 8, 4, 128, 130, 16, 8)])
+def test_repeats_are_seen_by_every_plan(B, Hq, Hkv, D, T, bs, S):
+    """Lists without repeats, with one in the last unit alone, with many, and without again, in one piece of memory."""
+    nsa = pkg()
+    t = make_inputs(dict(B=B, Hq=Hq, Hkv=Hkv, D=D, T=T, block_size=bs, S=S), torch.bfloat16, seed=8)
+    q, k, v, do = (dev(t[n], torch.bfloat16) for n in ("q", "ks", "vs", "do"))
+    plain = t["block_idx"].clone()
+    plain = torch.where((plain[..., :, None] == plain[..., None, :]).tril(-1).any(-1), torch.full_like(plain, -1), plain)
+    one, many = plain.clone(), plain.clone()
+    one[-1, -1, T - 3, 1:3] = one[-1, -1, T - 3, :1]
+    many[:, :, ::3, -1] = many[:, :, ::3, 0]
+    many[:, -1, 5::7, 1:] = many[:, -1, 5::7, :1]
+    assert not torch.equal(one, plain) and not torch.equal(many, plain)
+    L, lib = nsa._lib, nsa.lib()
+    dims = L.dims(B, Hq, Hkv, T, D, L.DTYPE_BF16)
+    n = lib.nsa_selection_bwd_workspace_bytes(dims, S, bs, 0)
+    ws = torch.full((n,), 0xa5, dtype=torch.uint8, device="cuda")
+    for idx in (plain, one, many, plain, many):
+        i = idx.int().cuda()
+        nsa.set_impl("simt")
+        o, lse = nsa.selection_forward_triton(q, k, v, i, bs, return_lse=True)
+        want = [o, *nsa.ops._selection_backward(q, k, v, i, bs, do, o, lse), lse]
+        nsa.set_impl("auto")
+        got_o, got_lse = nsa.selection_forward_triton(q, k, v, i, bs, return_lse=True)
+        grads = [torch.empty_like(x) for x in (q, k, v)]
+        L.check(lib.nsa_selection_bwd(*map(L.ptr, (q, k, v, i, o, lse, do, *grads)), dims, S, bs, None, None, L.ptr(ws), n, 0,
+                                      L.stream()))
+        _close([got_o, *grads, got_lse], want, "plan")
+    assert lib.nsa_device_status(None) == 0
