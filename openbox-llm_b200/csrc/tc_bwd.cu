@@ -1366,8 +1366,9 @@ dq_reduce3_kernel(const Reduce3Args a) {
   const size_t row_elems = (size_t)a.G * D;              // elements of one partial row (all heads)
   const size_t in_row = (size_t)g * D + v * 8;           // this thread's first head inside a row
   const size_t head_step = (size_t)Gp * D;               // to its next head
-  // Rows per trip and CTAs per SM (three: 80 registers, which hold the loads of a trip; without the bound the
-  // compiler took 70 and issued them in turns).  An empty place costs as many instructions as a row (a window
+  // Rows per trip and CTAs per SM (three: 80 registers, which hold the loads of a bf16 trip, and of half as many fp32
+  // rows; without the bound the compiler took 70 and issued them in turns).  fp32 rows in trips as long spilled in
+  // groups of 3 and took the same time: 33 us for 4 x 2000 tokens of 12 heads of 64 and 8 slots, 6 TB/s.  An empty place costs as many instructions as a row (a window
   // of 512 touches 9 key tiles, a query sees few tiles of summaries).  Two heads at 8 x 32768 tokens: trips of
   // 8 rows in 5.24 ms, of 4 in 4.90 (5.33 with five CTAs, which spill), unbounded 5.76; groups of 3 at 8 x 4096:
   // 203 us, unbounded 257.
@@ -1408,37 +1409,34 @@ dq_reduce3_kernel(const Reduce3Args a) {
   }
   if (a.part_slc) {
     const int32_t* ps = a.pair_of_slot + (size_t)qrow * a.S;
-    for (int s0 = 0; s0 < a.S; s0 += kTripSel) {
-      long long rows[kTripSel];
+    constexpr int kTrip = kF32 ? kTripSel / 2 : kTripSel;      // fp32 rows are twice as wide
+    for (int s0 = 0; s0 < a.S; s0 += kTrip) {
+      long long rows[kTrip];
 #pragma unroll
-      for (int k = 0; k < kTripSel; ++k) rows[k] = s0 + k < a.S ? (long long)__ldg(ps + s0 + k) : -1;
+      for (int k = 0; k < kTrip; ++k) rows[k] = s0 + k < a.S ? (long long)__ldg(ps + s0 + k) : -1;
       if (!kF32) {
         add_rows((const __nv_bfloat16*)a.part_slc, rows);
         continue;
       }
+      float4 f[kTrip][HG][2];
 #pragma unroll
-      for (int k0 = 0; k0 < kTripSel; k0 += 4) {       // fp32 rows are twice as wide: half a trip at a time
-        float4 f[4][HG][2];
+      for (int k = 0; k < kTrip; ++k) {
+        const float* src = (const float*)a.part_slc + (size_t)(rows[k] >= 0 ? rows[k] : 0) * row_elems + in_row;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const long long row = rows[k0 + k];
-          const float* src = (const float*)a.part_slc + (size_t)(row >= 0 ? row : 0) * row_elems + in_row;
+        for (int h = 0; h < HG; ++h)
 #pragma unroll
-          for (int h = 0; h < HG; ++h)
-#pragma unroll
-            for (int e = 0; e < 2; ++e)
-              f[k][h][e] = row >= 0 ? __ldcs(reinterpret_cast<const float4*>(src + h * head_step) + e) : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-#pragma unroll
-          for (int h = 0; h < HG; ++h)
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-              acc[h][4 * e] += f[k][h][e].x; acc[h][4 * e + 1] += f[k][h][e].y;
-              acc[h][4 * e + 2] += f[k][h][e].z; acc[h][4 * e + 3] += f[k][h][e].w;
-            }
+          for (int e = 0; e < 2; ++e)
+            f[k][h][e] = rows[k] >= 0 ? __ldcs(reinterpret_cast<const float4*>(src + h * head_step) + e) : make_float4(0.f, 0.f, 0.f, 0.f);
       }
+#pragma unroll
+      for (int k = 0; k < kTrip; ++k)
+#pragma unroll
+        for (int h = 0; h < HG; ++h)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            acc[h][4 * e] += f[k][h][e].x; acc[h][4 * e + 1] += f[k][h][e].y;
+            acc[h][4 * e + 2] += f[k][h][e].z; acc[h][4 * e + 3] += f[k][h][e].w;
+          }
     }
   }
   if (a.part_win) {
