@@ -103,8 +103,9 @@ int nsa_selection_bwd(const void* q, const void* k, const void* v, const int32_t
 /* The tcgen05 selection kernels walk the block list block by block: the queries of each block (what
  * nsa_fsa.py:14-64 builds), the (query, slot) -> pair map and a work list, which nsa_selection_fwd
  * and nsa_selection_bwd each build inside their workspace.  A caller that runs both on one block list
- * (every training step) can build them once into a buffer of nsa_selection_plan_bytes bytes (0: NSA_IMPL_AUTO does not run
- * this call on the tcgen05 kernels) and hand it to the *_planned forms, which read it instead of building
+ * (every training step) can build them once into a buffer of nsa_selection_plan_bytes bytes (0: no plan serves this
+ * call under NSA_IMPL_AUTO; it has to be one on blocks of 64 tokens that the tcgen05 kernels take: blocks of 16 and 32
+ * tokens build their own) and hand it to the *_planned forms, which read it instead of building
  * their own.  The reference builds its CSR once per forward and once per backward
  * (nsa_selection_kernel.py:199-201, nsa_selection_backward.py:356-358); no counterpart for the
  * reuse. */
@@ -121,7 +122,8 @@ int nsa_selection_bwd_planned(const void* q, const void* k, const void* v, const
                               void* workspace, size_t workspace_bytes, const void* plan, void* stream);
 
 /* dq of the whole op in one pass (no counterpart in the reference, which adds the three branch
- * gradients with torch).  When the tcgen05 kernels serve a backward call (nsa_tc_supported) its
+ * gradients with torch).  When the tcgen05 kernels serve a backward call (nsa_tc_supported; selection:
+ * on blocks of 64 tokens, or with NSA_IMPL_TC) its
  * `dq` argument may be NULL: the branch's bf16 dQ partials then stay in the call's workspace, and
  * this entry point adds the partials of the compression, selection and window branches of every
  * query in fp32 and writes dq [B,Hq,T,D] once.  ws_* are the workspaces of the three backward

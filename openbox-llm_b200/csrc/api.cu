@@ -482,7 +482,7 @@ extern "C" int nsa_selection_plan_build(const int32_t* block_idx, const NsaDims*
   int rc = check_sel(dims, S, block_size);
   if (rc != NSA_OK) return rc;
   NSA_CHECK_ARG(S > 0 && block_idx && plan, "null block_idx or plan");
-  NSA_CHECK_ARG(use_tc(dims, block_size, NSA_IMPL_AUTO, &rc), "a selection plan needs a call that NSA_IMPL_AUTO gives to the tcgen05 kernels");
+  NSA_CHECK_ARG(use_tc(dims, block_size, NSA_IMPL_AUTO, &rc), "a selection plan needs a call on 64-token blocks that the tcgen05 kernels take");
   AttnArgs a = base_args(dims, dims->T);
   a.block_idx = block_idx; a.kind = 2; a.S = S; a.block_size = block_size;
   return tc_sel_plan_build(a, plan, plan_bytes, (cudaStream_t)stream);
@@ -553,7 +553,7 @@ static int selection_bwd_impl(const void* q, const void* k, const void* v,
     return tc_attn_bwd(a, workspace, workspace_bytes, st);
   }
   if (rc != NSA_OK) return rc;
-  NSA_CHECK_ARG(dq, "dq may be null only when the tcgen05 kernels serve the call");
+  NSA_CHECK_ARG(dq, "dq may be null only where the tcgen05 kernels serve the call: 64-token blocks, or NSA_IMPL_TC");
   return simt_bwd(a, dims, dk, dv, workspace, workspace_bytes, st);
 }
 
