@@ -154,11 +154,14 @@ bool use_tc(const NsaDims* d, int block_size, int impl, int* err) {
 // listed keys x D; us on the CUDA cores | the tensor cores, forward and backward): 8.4 M (8 heads of 64, 256 tokens,
 // 4 blocks of 16) 15 + 28 | 13 + 43, 12.6 M (384 tokens) 17 + 45 | 16 + 48, 16.8 M (512 tokens) 19 + 42 | 19 + 40, 33 M (256
 // tokens, 8 blocks of 32) 29 + 54 | 13 + 43.
+// Lists of more than 32768 keys stay there too: a row that has to be done again (sel_row.cuh) must end within the
+// second that the other roles wait.
 // The backward keeps fp32 dQ partials of S rows per query: beyond 8 GB of them (half of what the bf16 partials of
 // 64-token blocks take at 8 x 32768 tokens, 16 heads of 128, 16 blocks a list) the CUDA-core kernels, which need none,
 // serve the call.
 bool use_three_term(const NsaDims* d, int block_size, int S, int impl, bool bwd) {
   if (impl != NSA_IMPL_AUTO || (block_size != 16 && block_size != 32) || S < 1 || !tc_shape_ok(*d, block_size)) return false;
+  if ((long long)S * block_size > 32768) return false;
   if ((double)d->B * d->Hq * d->T * S * block_size * d->D <= 12e6 && !g_opt_small_blocks_tc.load()) return false;
   return !bwd || (double)d->B * d->Hq * d->T * S * d->D * sizeof(float) <= 8e9;
 }

@@ -583,57 +583,102 @@ template <int D, bool kThreeTerm> struct Bwd2 {
                                   (size_t)kSlots * 128 * 4 /*partial rows of a ragged tile*/ + 1024 /*alignment slack*/;
 };
 
-// dK and dV of one work item in scalar fp32, a warp to a row, into acc [dV, dK][64 keys][D] in shared memory, for
-// a tile whose sums are not finite (three-term selection).
+// dK and dV of one work item in scalar fp32, into acc [dV, dK][64 keys][D] in shared memory, for a tile whose sums are
+// not finite (three-term selection).  A warp has four keys, their K and V rows and their sums in registers, and goes
+// through the rows.
 template <int D>
-__device__ __noinline__ void sel_tile_dkdv(const BwdArgs& p, float* acc, int bh, int j, int pair_first, int n_rows,
-                                           int n_threads) {
+__device__ __noinline__ void sel_tile_dkdv(const BwdArgs& p, float* acc, int bh, int j, int pair_first, int n_rows) {
+  constexpr int N = D / 32;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int b = bh / p.Hkv, hkv = bh % p.Hkv, key0 = j * kKeys;
-  for (int i = threadIdx.x; i < 2 * kKeys * D; i += n_threads) acc[i] = 0.f;
-  __syncthreads();
-  for (int r = warp; r < n_rows; r += n_threads / 32) {
-    const int pair = __ldg(p.plan.pairs + pair_first + r / p.G);
-    const int t = pair & (int)kPairPosMask;
-    const size_t row = ((size_t)b * p.Hq + hkv * p.G + r % p.G) * p.T + t;
-    const float gate = p.row_scale ? p.row_scale[row] : 1.f;
-    const float lse2 = p.lse[row] * kLog2e - __log2f(gate), delta = p.delta[row];
-    float q[D / 32], g[D / 32];
-    for (int e = 0; e < D / 32; ++e) {
-      q[e] = to_float(p.q[row * D + lane + 32 * e]);
-      g[e] = to_float(p.d_o[row * D + lane + 32 * e]);
-    }
-    const int32_t* list = p.block_idx + ((size_t)bh * p.T + t) * p.S;
-    for (int c = 0; c < kKeys && key0 + c <= t; ++c) {
-      if (!(((uint32_t)pair >> (kPairPosBits + (c >> 4))) & 1u)) continue;
-      const size_t key = ((size_t)bh * p.Lk + key0 + c) * D;
-      float x = 0.f, y = 0.f;
-      for (int e = 0; e < D / 32; ++e) {
-        x = fmaf(q[e], to_float(p.k[key + lane + 32 * e]), x);
-        y = fmaf(g[e], to_float(p.v[key + lane + 32 * e]), y);
+  const int b = bh / p.Hkv, hkv = bh % p.Hkv, key0 = j * kKeys, c0 = 4 * warp;
+  if (c0 < kKeys) {
+    const bool repeats = __ldg(&p.plan.hdr->repeats) != 0ull;
+    float k[4][N], v[4][N], dk[4][N], dv[4][N];
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+#pragma unroll
+      for (int e = 0; e < N; ++e) {
+        const size_t at = ((size_t)bh * p.Lk + min(key0 + c0 + c, p.Lk - 1)) * D + lane + 32 * e;
+        k[c][e] = to_float(p.k[at]);
+        v[c][e] = to_float(p.v[at]);
+        dk[c][e] = dv[c][e] = 0.f;
       }
-      x = warp_sum(x);
-      y = warp_sum(y);
-      const float pr = (float)times_listed(list, p.S, (key0 + c) / p.block_size) * exp2f(fmaf(x, p.scale_log2, -lse2));
-      const float ds = pr * (y - delta) * p.scale;
-      for (int e = 0; e < D / 32; ++e) {
-        atomicAdd(acc + c * D + lane + 32 * e, pr * g[e]);
-        atomicAdd(acc + (kKeys + c) * D + lane + 32 * e, ds * q[e]);
+    int pair_l = 0;
+    long long row_l = 0;
+    float lse2_l = 0.f, delta_l = 0.f;
+#pragma unroll 1
+    for (int r = 0; r < n_rows; ++r) {
+      // a lane fetches what 32 rows need before their vectors: one trip to memory for them all
+      if ((r & 31) == 0) {
+        const int rr = min(r + lane, n_rows - 1);
+        pair_l = __ldg(p.plan.pairs + pair_first + rr / p.G);
+        row_l = (b * p.Hq + hkv * p.G + rr % p.G) * (long long)p.T + (pair_l & (int)kPairPosMask);
+        lse2_l = __ldg(p.lse + row_l) * kLog2e - (p.row_scale ? __log2f(__ldg(p.row_scale + row_l)) : 0.f);
+        delta_l = __ldg(p.delta + row_l);
+      }
+      const int pair = __shfl_sync(0xffffffffu, pair_l, r & 31);
+      const int t = pair & (int)kPairPosMask;
+      if (!(((uint32_t)pair >> (kPairPosBits + (c0 >> 4))) & 1u) || key0 + c0 > t) continue;
+      const long long row = __shfl_sync(0xffffffffu, row_l, r & 31);
+      const float lse2 = __shfl_sync(0xffffffffu, lse2_l, r & 31), delta = __shfl_sync(0xffffffffu, delta_l, r & 31);
+      const float times = repeats ? (float)times_listed(p.block_idx + ((size_t)bh * p.T + t) * p.S, p.S, (key0 + c0) / p.block_size) : 1.f;
+      float q[N], g[N];
+#pragma unroll
+      for (int e = 0; e < N; ++e) {
+        q[e] = to_float(p.q[row * D + lane + 32 * e]);
+        g[e] = to_float(p.d_o[row * D + lane + 32 * e]);
+      }
+      float x[4], y[4];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        x[c] = y[c] = 0.f;
+#pragma unroll
+        for (int e = 0; e < N; ++e) {
+          x[c] = fmaf(q[e], k[c][e], x[c]);
+          y[c] = fmaf(g[e], v[c][e], y[c]);
+        }
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          x[c] += __shfl_xor_sync(0xffffffffu, x[c], o);
+          y[c] += __shfl_xor_sync(0xffffffffu, y[c], o);
+        }
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const float pr = times * exp2f(fmaf(x[c], p.scale_log2, -lse2));
+        const float ds = pr * (y[c] - delta) * p.scale;
+        if (key0 + c0 + c <= t) {                          // what is not attended may be infinite or NaN
+#pragma unroll
+          for (int e = 0; e < N; ++e) {
+            dv[c][e] = fmaf(pr, g[e], dv[c][e]);
+            dk[c][e] = fmaf(ds, q[e], dk[c][e]);
+          }
+        }
       }
     }
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+#pragma unroll
+      for (int e = 0; e < N; ++e) {
+        acc[(c0 + c) * D + lane + 32 * e] = dv[c][e];
+        acc[(kKeys + c0 + c) * D + lane + 32 * e] = dk[c][e];
+      }
   }
   __syncthreads();
 }
 
 // 32 columns of a row's dQ against one key tile in scalar fp32 (three-term selection, result not finite).
 template <int D>
-__device__ __noinline__ void sel_row_dq(const BwdArgs& p, float* acc, int bh, int head, int pair, int key0, int col0) {
+__device__ __noinline__ void sel_row_dq(const BwdArgs& p, float* out, int bh, int head, int pair, int key0, int col0) {
   const int t = pair & (int)kPairPosMask;
   const size_t row = ((size_t)(bh / p.Hkv) * p.Hq + head) * p.T + t;
   const float gate = p.row_scale ? p.row_scale[row] : 1.f;
   const float lse2 = p.lse[row] * kLog2e - __log2f(gate), delta = p.delta[row];
   const int32_t* list = p.block_idx + ((size_t)bh * p.T + t) * p.S;
-#pragma unroll 1
+  float acc[32];
+#pragma unroll
   for (int e = 0; e < 32; ++e) acc[e] = 0.f;
 #pragma unroll 1
   for (int c = 0; c < kKeys && key0 + c <= t; ++c) {
@@ -642,9 +687,10 @@ __device__ __noinline__ void sel_row_dq(const BwdArgs& p, float* acc, int bh, in
     const float x = dot_rows<D>(p.q + row * D, p.k + key), y = dot_rows<D>(p.d_o + row * D, p.v + key);
     const float pr = (float)times_listed(list, p.S, (key0 + c) / p.block_size) * exp2f(fmaf(x, p.scale_log2, -lse2));
     const float ds = pr * (y - delta) * p.scale;
-#pragma unroll 1
-    for (int e = 0; e < 32; ++e) acc[e] = fmaf(ds, to_float(p.k[key + col0 + e]), acc[e]);
+    add32_row(ds, p.k + key + col0, acc);
   }
+#pragma unroll
+  for (int e = 0; e < 32; ++e) out[e] = acc[e];
 }
 
 template <int D, bool kCluster, bool kThreeTerm>
@@ -1026,6 +1072,7 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
       // (gate p)^T dO; dS = scale * gate * p * (dP - delta), the constant factors folded once per row
       const float lse2 = lse_cur * kLog2e - __log2f(gate_cur);
       const float dscale = p.scale, ddelta = delta_cur * p.scale;
+      const bool row_again = kThreeTerm && t_cur >= 0 && lse2 == lse2 && ddelta == ddelta;
       // every column of this thread's half is attended (the usual case away from the diagonal)?
       const bool all_cols = lo <= half * 32 && hi >= half * 32 + 31 && groups == 0x3u && !repeats;
       float times[2] = {1.f, 1.f};                   // how often the row's list names the blocks of its column groups
@@ -1135,7 +1182,8 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
           float z = 0.f;                   // x * 0: 0 or NaN
 #pragma unroll
           for (int e = 0; e < 32; ++e) z = fmaf(__uint_as_float(r32[e]), 0.f, z);
-          if (t_cur >= 0 && z != 0.f) {
+          // (a row whose own statistics are NaN has NaN in every column, here as there)
+          if (z != 0.f && row_again) {
             float again[32];
             sel_row_dq<D>(p, again, bh, head, t_cur, key0, col0);
 #pragma unroll
@@ -1229,7 +1277,7 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
     }
     if (__syncthreads_or(z != 0.f)) {
       const int first = rt_begin * p.nq, rows = max(0, min(n_tiles * p.nq, n_q - first)) * p.G;
-      sel_tile_dkdv<D>(p, s_acc, bh, j, pair_base + first, rows, kB2Threads);
+      sel_tile_dkdv<D>(p, s_acc, bh, j, pair_base + first, rows);
       if (!kCluster && !*s_abort)
         for (int i = tid; i < 2 * kKeys * D; i += kB2Threads) {
           const int which = i / (kKeys * D), key = key0 + (i / D) % kKeys;

@@ -34,6 +34,9 @@ def test_lines_of_the_tensor_core_kernels():
     L, lib = pkg()._lib, pkg().lib()
     ws = lambda T, S, D, impl, Hq=16, B=1, bs=16: lib.nsa_selection_bwd_workspace_bytes(
         L.dims(B, Hq, 4, T, D, L.DTYPE_BF16), S, bs, L.IMPL[impl])
+    for S, on in ((1024, True), (1025, False)):              # a list of 32768 keys, and of more
+        auto, simt = ws(64, S, 64, "auto", bs=32), ws(64, S, 64, "simt", bs=32)
+        assert auto >= 16 * 64 * S * 64 * 4 if on else auto == simt
     most = int(8e9 / (16 * 8 * 128 * 4))                     # tokens
     for T, S, D, on in ((most, 8, 128, True), (most + 1, 8, 128, False), (4 * most, 4, 64, True), (4 * most + 4, 4, 64, False),
                         (184, 4, 64, True), (183, 4, 64, False), (2000, 1, 64, True)):
