@@ -725,7 +725,7 @@ size_t extra_smem(const AttnArgs& a) { return sizeof(KeyInfo) + 16 + (a.kind == 
 // 103 | 98 | 121 and 199 | 215 | 225.  At D = 128 a tile has an SM to itself: sharing only fills idle SMs.
 int cluster_size(const AttnArgs& a) {
   const long long tiles = n_tiles(a), sms = sm_count();
-  const int n_kt = ((a.kind == 0 ? a.window + kR / (a.Hq / a.Hkv) : a.Lk) + kK - 1) / kK;
+  const long long n_kt = ((a.kind == 0 ? (long long)a.window + kR / (a.Hq / a.Hkv) : a.Lk) + kK - 1) / kK;    // (any window)
   int csize = 1;
   if (a.D > 64) csize = 4 * tiles <= sms ? 4 : 2 * tiles <= sms ? 2 : 1;
   else if (a.kind == 2) csize = tiles <= sms ? 4 : tiles <= 7 * sms ? 2 : 1;

@@ -34,8 +34,8 @@ def _plain_linear(m):
 
 def _function_modes():
     """Whether a TorchFunctionMode is active that may look at calls (the default-device mode only sees factories)."""
-    return any(type(torch._C._get_function_stack_at(i)) is not DeviceContext
-               for i in range(torch._C._len_torch_function_stack()))
+    n = torch._C._len_torch_function_stack()
+    return n > 0 and any(type(torch._C._get_function_stack_at(i)) is not DeviceContext for i in range(n))
 
 
 class _Compressor(nn.Module):
