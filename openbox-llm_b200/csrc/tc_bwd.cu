@@ -1569,10 +1569,11 @@ __global__ void sel_split_blocks_kernel(const int32_t* __restrict__ offsets, flo
   }
 }
 
-// dK and dV of the compression branch from the accumulators of up to kOrderedChunks chunks of row tiles, in a fixed order: the
-// last chunk of a key tile, which may be short, then the others as they come.  (The order in which atomics end up
-// when the CTAs run side by side; the gradient of the key pooling's position parameters is the rounding of
-// these sums, and 1e-2 of it moves with their order.)
+// dK and dV of the compression branch from the accumulators of up to kOrderedChunks chunks of row tiles, in a fixed order, so
+// that they come out the same on every run: the last chunk of a key tile, then the others as they come.  (Any
+// order is as exact.  This one is what fp32 atomics mostly gave before, and was kept so that results stayed as they were:
+// the gradient of the key pooling's position parameters is the rounding of these sums, and 1e-2 of it moves with the
+// order.  More chunks, beyond 192 row tiles of queries, still meet in atomics.)
 constexpr int kOrderedChunks = 4;
 __global__ void __launch_bounds__(256)
 cmp_chunks_kernel(const float* __restrict__ dk_acc, const float* __restrict__ dv_acc, __nv_bfloat16* __restrict__ dk,
@@ -1643,10 +1644,10 @@ static BwdPlan plan_bwd(const AttnArgs& a) {
   // few queries left), so the CTAs over the line start as the short ones end.  At 76 to 84 key tiles
   // (152 to 168 CTAs in pairs) window and selection take 40 to 61 and 77 to 107 us in pairs, 49 to 66 and 102
   // to 153 without (D of 64 and 128, groups of 4).  More CTAs than that gain nothing, and clusters
-  // leave SMs of a GPC over, so big problems do without.  Compression keeps one running sum per key tile: the
-  // gradient of the key pooling's position parameters is the rounding of that sum (tc.cu), and as it
-  // runs beside the other branches where a problem is small, the op at T = 1024 gains nothing from
-  // sharing those (277 to 289 us without, 291 with).
+  // leave SMs of a GPC over, so big problems do without.  Compression does too: its sums keep one
+  // order, row tiles in turn within a chunk and chunks as cmp_chunks_kernel adds them, since the
+  // gradient of the key pooling's position parameters is the rounding of those sums (tc.cu), and where a problem is small it
+  // runs beside the other branches.
   const int max_rt = a.kind == 0 ? (a.window + kKeys - 2 + pl.nq) / pl.nq : (a.T + pl.nq - 1) / pl.nq;
   const int item_rt = a.kind == 2 ? (max_rt < kSelChunkTiles ? max_rt : kSelChunkTiles) : max_rt;
   const long long base = (long long)units * pl.n_ktiles;

@@ -68,4 +68,4 @@ def test_every_entry(B, Hkv, G, T, S):
                 ok = j >= 0 and 64 * j <= t and j not in named
                 named.add(j)
                 assert pos[u, t, s] == (place[t, j] if ok else -1)
-    assert hdr[0] == union and hdr[1] == n_pairs
+    assert hdr[0] == union and hdr[1] == n_pairs and hdr[2] == 0      # (repeats count on smaller blocks only)

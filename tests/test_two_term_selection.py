@@ -32,14 +32,14 @@ def _both(q, k, v, do, idx, bs):
 
 
 def _close(got, want, what):
-    """Two bf16 roundings of the same value, each half a step (2^-9), and fp32 sums whose terms are up to the
-    largest entry: 2e-5 of it."""
+    """Two bf16 roundings of the same value, each half a step (2^-9), and fp32 sums of up to a few thousand terms as large as the
+    largest entry, 2^-24 off each (and 2^-21 in their exponentials): 4e-6 of it."""
     for a, b, n in zip(got, want, ("o", "dq", "dk", "dv")):
         a, b = a.double(), b.double()
         fin = torch.isfinite(b)
         assert torch.equal(torch.isfinite(a), fin), (what, n)
         a, b = a[fin], b[fin]
-        assert ((a - b).abs() <= 2.0 ** -7 * b.abs() + 2e-5 * b.abs().max()).all(), (what, n)
+        assert ((a - b).abs() <= 2.0 ** -7 * b.abs() + 4e-6 * b.abs().max()).all(), (what, n)
     a, b = got[4], want[4]
     fin = torch.isfinite(b)
     assert torch.equal(torch.isfinite(a), fin) and ((a - b)[fin].abs() <= 1e-5 * b[fin].abs().clamp(min=1)).all(), (what, "lse")
