@@ -126,8 +126,9 @@ def _load_ext():
     spec = importlib.util.spec_from_file_location("_nsa_torch", EXT_PATH)
     mod = importlib.util.module_from_spec(spec)
     spec.loader.exec_module(mod)
-    if mod.torch_version != torch.__version__:
-        raise ImportError(f"it was built against torch {mod.torch_version}, this is {torch.__version__}")
+    built = getattr(mod, "torch_version", "of an unknown version")
+    if built != torch.__version__:
+        raise ImportError(f"it was built against torch {built}, this is {torch.__version__}")
     mod.set_error(NsaError)
     return mod
 
