@@ -305,19 +305,23 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       }
     } else if (warp == 5) {
       // ---- MMA issuer ------------------------------------------------------------------------
-      if (lane == 0) {
+      {
+        const uint32_t lead = elect_one(), tmem_u = uniform(tmem);
+        auto ready = [&](uint64_t* bar, uint32_t parity, int code) -> bool {
+          return __all_sync(0xffffffffu, mbar_wait(bar, parity, p.status, s_abort, code));
+        };
         auto issue_s = [&](int cc, bool last) {   // S = Q K^T of running key tile cc
           const int st = cc % kStages;
           const uint32_t qa = desc_lo_kmajor(smem_u32(sQ)), ka = desc_lo_kmajor(smem_u32(sK + st * L::kKVBytes));
 #pragma unroll
           for (int kk = 0; kk < D / 16; ++kk) {
             const uint32_t slab = kk >> 2, in = (kk & 3) * 32;
-            mma_ss(tmem + kColS + (cc & 1) * kKeys, desc_at(qa, slab * (kRows * 128) + in),
+            mma_ss_by(lead, tmem_u + kColS + (cc & 1) * kKeys, desc_at(qa, slab * (kRows * 128) + in),
                    desc_at(ka, slab * (kKeys * 128) + in), kIdescQK, kk > 0);
           }
-          tc_commit(bar_s + (cc & 1));
-          tc_commit(k_free + st);
-          if (last) tc_commit(q_free);
+          tc_commit_by(lead, bar_s + (cc & 1));
+          tc_commit_by(lead, k_free + st);
+          if (last) tc_commit_by(lead, q_free);
         };
         for (int w = w0; ok && w < w_end; w += gridDim.x) {
           const Tile x = tile_of(w);
@@ -347,12 +351,12 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
             const uint32_t va = desc_lo_mnmajor(smem_u32(sV + st * L::kKVBytes), kKeys * 128);   // O (+)= P V
 #pragma unroll
             for (int kk = 0; kk < kKeys / 16; ++kk)
-              mma_ts(tmem + kColO, tmem + kColS + (c & 1) * kKeys + kk * 8, desc_at(va, kk * 2048), kIdescPV, (i > 0) || (kk > 0));
+              mma_ts_by(lead, tmem_u + kColO, tmem_u + kColS + (c & 1) * kKeys + kk * 8, desc_at(va, kk * 2048), kIdescPV, (i > 0) || (kk > 0));
             if (kThreeTerm) {
-              if (kLate) tc_commit(bar_p1 + (c & 1));
+              if (kLate) tc_commit_by(lead, bar_p1 + (c & 1));
 #pragma unroll
               for (int kk = 0; kk < kKeys / 16; ++kk)
-                mma_ts(tmem + kColO, tmem + kColS + (c & 1) * kKeys + 32 + kk * 8, desc_at(va, kk * 2048), kIdescPV, 1);
+                mma_ts_by(lead, tmem_u + kColO, tmem_u + kColS + (c & 1) * kKeys + 32 + kk * 8, desc_at(va, kk * 2048), kIdescPV, 1);
               if (kLate) {
                 ok = mbar_wait(bar_p3 + (c & 1), (c >> 1) & 1, p.status, s_abort, 0x2000);
                 if (!ok) break;
@@ -360,10 +364,10 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
               }
 #pragma unroll
               for (int kk = 0; kk < kKeys / 16; ++kk)
-                mma_ts(tmem + kColO, tmem + kColP3 + (c & 1) * kP3Step + kk * 8, desc_at(va, kk * 2048), kIdescPV, 1);
+                mma_ts_by(lead, tmem_u + kColO, tmem_u + kColP3 + (c & 1) * kP3Step + kk * 8, desc_at(va, kk * 2048), kIdescPV, 1);
             }
-            tc_commit(bar_o + (c & 1));
-            tc_commit(v_free + st);
+            tc_commit_by(lead, bar_o + (c & 1));
+            tc_commit_by(lead, v_free + st);
           }
           ++it;
         }
@@ -567,9 +571,9 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     // the row tile's list may be overwritten once every role is through with it
     if (kSel && __syncthreads_or(*s_abort)) break;
   }
-  if (warp == 5 && lane == 0) {
+  if (warp == 5) {
     // the tensor pipe is idle before tensor memory is given back, whatever happened
-    tc_commit(bar_drain);
+    tc_commit_by(elect_one(), bar_drain);
     if (!mbar_wait(bar_drain, 0, p.status, s_abort, 0x1000)) mbar_wait_drain(bar_drain, 0);
   }
 

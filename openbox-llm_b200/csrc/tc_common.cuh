@@ -48,14 +48,29 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   return ok != 0;
 }
 
+// The same without the hardware's pause, for a thread that polls several barriers in turn.
+__device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+
 // Bounded wait.  When the limit runs out the kernel raises the device status word, marks the
 // CTA as aborted and every later wait of the CTA returns at once, so the grid drains; other
 // CTAs notice the status word the next time one of their waits is slow.
-// Returns true when the phase completed, false when the wait was given up.
+// Returns true when the phase completed, false when the wait was given up.  The abort flag is read only where the
+// phase is not there at the first look: while the MMAs fetch operands from shared memory a load of the flag takes some
+// 220 cycles (its bandwidth is theirs first), the look at the barrier 30.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* status,
                                           volatile int* s_abort, int code) {
-  if (*s_abort) return false;
   if (mbar_try_wait(bar, parity)) return true;
+  if (*s_abort) return false;
   const long long start = clock64();
   uint32_t polls = 0;
   while (!mbar_try_wait(bar, parity)) {
@@ -287,6 +302,41 @@ __device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_
       "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+
+// The same from a warp whose lanes stay together: `lead` is set in one of them (elect_one), which issues.  Run by a
+// single thread of a warp, addresses and descriptors live in its own registers and have to be moved to the warp's uniform
+// ones for every MMA; with the warp together they are uniform from the start.  The issuing warp shares its scheduler
+// with warps that do arithmetic and gets few of its slots: beside two warps of independent FMAs an MMA of 128 x 64 x 16 came
+// out every 480 cycles from a single thread, every 258 so (every 67 and 61 without them).
+__device__ __forceinline__ uint32_t elect_one() {
+  uint32_t lead;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(lead));
+  return lead;
+}
+__device__ __forceinline__ void mma_ss_by(uint32_t lead, uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                          uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(lead)
+      : "memory");
+}
+__device__ __forceinline__ void mma_ts_by(uint32_t lead, uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc,
+                                          uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
+      "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(lead)
+      : "memory");
+}
+__device__ __forceinline__ void tc_commit_by(uint32_t lead, uint64_t* bar) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar)), "r"(lead)
+      : "memory");
+}
+// a value that all lanes hold, as one the compiler knows to be the same
+__device__ __forceinline__ uint32_t uniform(uint32_t x) { return __reduce_max_sync(0xffffffffu, x); }
 
 // Loads that must be issued where they are written: ptxas otherwise sinks a prefetch down to its
 // first use (a whole loop iteration later) and the warp then waits out the full memory latency.

@@ -167,10 +167,10 @@ tc_fwdpair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
     int tq0 = tq_of(0, o0), tq1 = tq_of(0, o1);
     for (int k = 0; k < n_tiles; ++k) {
       const int st = k % kPairQStages;
-      mbar_wait(q_empty + st, ((k / kPairQStages) + 1) & 1, p.status, s_abort, 512);
+      const bool ok = mbar_wait(q_empty + st, ((k / kPairQStages) + 1) & 1, p.status, s_abort, 512);
       const int tn0 = k + 1 < n_tiles ? tq_of(k + 1, o0) : p.T;          // next tile's positions, ahead
       const int tn1 = k + 1 < n_tiles ? tq_of(k + 1, o1) : p.T;
-      if (__any_sync(0xffffffffu, *s_abort)) break;          // the whole warp leaves together
+      if (!__all_sync(0xffffffffu, ok)) break;               // the whole warp leaves together
       if (pw == 0 && lane == 0) { mbar_expect_tx(q_full + st, gather_bytes); *s_issued = k + 1; }
       __syncwarp();
       uint8_t* dst = sQ + st * kQBytes;
@@ -192,49 +192,50 @@ tc_fwdpair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
     }
   } else if (warp == 12 + kPairProducers) {
     // ---- MMA issuer ------------------------------------------------------------------------
-    if (lane == 0) {
-      mbar_wait(bar_kv, 0, p.status, s_abort, 32);
+    {
+      const uint32_t lead = elect_one(), tmem_u = uniform(tmem);
+      auto ready = [&](uint64_t* bar, uint32_t parity, int code) -> bool {
+        return __all_sync(0xffffffffu, mbar_wait(bar, parity, p.status, s_abort, code));
+      };
+      ready(bar_kv, 0, 32);
       const uint32_t ka = desc_lo_kmajor(smem_u32(sK));
       const uint32_t va = desc_lo_mnmajor(smem_u32(sV), kKeys * 128);
       for (int k = 0; k <= n_tiles; ++k) {
-        if (*s_abort) break;
         if (k < n_tiles) {
           const int st = k % kPairQStages, sb = k & 1;
-          mbar_wait(q_full + st, (k / kPairQStages) & 1, p.status, s_abort, 512);
           // the S / P columns of the slot are free once P V of tile k-2 has completed
-          if (k >= 2) mbar_wait(o_full + sb, ((k >> 1) - 1) & 1, p.status, s_abort, 128);
-          if (*s_abort) break;
+          if (!ready(q_full + st, (k / kPairQStages) & 1, 512) ||
+              (k >= 2 && !ready(o_full + sb, ((k >> 1) - 1) & 1, 128))) break;
           tc_fence_after();
           const uint32_t qa = desc_lo_kmajor(smem_u32(sQ + st * kQBytes));
-          const uint32_t colS = tmem + sb * kSlotCols;
+          const uint32_t colS = tmem_u + sb * kSlotCols;
           // Q tile: slab-major (8-row groups 1024 bytes apart, slabs kRows * 128 apart) or, with merged
           // boxes, the two slabs of an 8-row group side by side (groups 2048 bytes apart)
           const uint32_t q_slab = p.merged ? 1024u : (uint32_t)(kRows * 128), q_sbo = p.merged ? 2048u : 1024u;
 #pragma unroll
           for (int kk = 0; kk < D / 16; ++kk) {
             const uint32_t slab = kk >> 2, in = (kk & 3) * 32;
-            mma_ss(colS, desc_at_sbo(qa, slab * q_slab + in, q_sbo), desc_at(ka, slab * (kKeys * 128) + in),
+            mma_ss_by(lead, colS, desc_at_sbo(qa, slab * q_slab + in, q_sbo), desc_at(ka, slab * (kKeys * 128) + in),
                    kIdescS, kk > 0);
           }
-          tc_commit(q_empty + st);     // the stage may be refilled once S has read it
-          tc_commit(s_full + sb);
+          tc_commit_by(lead, q_empty + st);     // the stage may be refilled once S has read it
+          tc_commit_by(lead, s_full + sb);
         }
         if (k >= 1) {
           const int jt = k - 1, sb = jt & 1;
-          mbar_wait(p_full + sb, (jt >> 1) & 1, p.status, s_abort, 64);
           // the O columns of the slot are free once the epilogue has read O of tile jt-2
-          if (jt >= 2) mbar_wait(o_empty + sb, ((jt >> 1) - 1) & 1, p.status, s_abort, 1024);
-          if (*s_abort) break;
+          if (!ready(p_full + sb, (jt >> 1) & 1, 64) ||
+              (jt >= 2 && !ready(o_empty + sb, ((jt >> 1) - 1) & 1, 1024))) break;
           tc_fence_after();
-          const uint32_t colP = tmem + sb * kSlotCols, colO = colP + 64;
+          const uint32_t colP = tmem_u + sb * kSlotCols, colO = colP + 64;
 #pragma unroll
           for (int kk = 0; kk < kKeys / 16; ++kk)
-            mma_ts(colO, colP + kk * 8, desc_at(va, kk * 2048), kIdescPV, kk > 0);
-          tc_commit(o_full + sb);
+            mma_ts_by(lead, colO, colP + kk * 8, desc_at(va, kk * 2048), kIdescPV, kk > 0);
+          tc_commit_by(lead, o_full + sb);
         }
       }
       // the tensor pipe is idle before TMEM is given back, whatever happened above
-      tc_commit(bar_drain);
+      tc_commit_by(lead, bar_drain);
       if (!mbar_wait(bar_drain, 0, p.status, s_abort, 2048)) mbar_wait_drain(bar_drain, 0);
     }
   } else if (warp < 8) {
@@ -251,12 +252,11 @@ tc_fwdpair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
     };
     int t_cur = sb < n_tiles ? row_query(sb) : -1;
     for (int k = sb; k < n_tiles; k += 2) {
-      if (*s_abort) break;
       const int t_nxt = k + 2 < n_tiles ? row_query(k + 2) : -1;
       const int hi = t_cur >= 0 ? min(kKeys - 1, (int)(t_cur & kPairPosMask) - key0) : -1;
       const uint32_t groups = (uint32_t)t_cur >> kPairPosBits;      // 16-column groups the row attends
-      mbar_wait(s_full + sb, (k >> 1) & 1, p.status, s_abort, 64);
-      if (*s_abort) break;
+      const bool ok = mbar_wait(s_full + sb, (k >> 1) & 1, p.status, s_abort, 64);
+      if (!__all_sync(0xffffffffu, ok)) break;                 // the whole warp leaves together
       tc_fence_after();
       uint32_t r[64];
       tmem_ld32(lane_base, r);
@@ -305,11 +305,11 @@ tc_fwdpair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
     for (int k = 0; k < n_tiles; ++k) {
       const int sb = k & 1;
       const int i = item.z + k;
-      mbar_wait(o_full + sb, (k >> 1) & 1, p.status, s_abort, 128);
+      const bool ok = mbar_wait(o_full + sb, (k >> 1) & 1, p.status, s_abort, 128);
       tc_fence_after();
       // the staging tile of this slot is free once the store of tile k-2 has read it
       if (et == 0 && k >= 2) bulk_wait_read_1();
-      if (named_or(1, 128, *s_abort)) break;                   // the whole group leaves together
+      if (named_or(1, 128, !ok)) break;                        // the whole group leaves together
       uint8_t* stage = sStage + sb * kQBytes;
       const uint32_t lane_base = tmem + ((uint32_t)(quad * 32) << 16) + sb * kSlotCols + 64;
 #pragma unroll
