@@ -92,6 +92,9 @@ __host__ __device__ inline size_t bwd_smem_bytes(int D) {
 __device__ __forceinline__ void group_sync(int group) {
   asm volatile("bar.sync %0, %1;" ::"r"(group + 1), "r"(kGroupThreads) : "memory");
 }
+__device__ __forceinline__ void named_sync_b(int id, int threads) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
 // Named barrier that also tells every thread whether any of them brought a non-zero `pred`: the
 // way a group of warps decides together to leave after a given-up wait.
 __device__ __forceinline__ bool named_or_b(int id, int threads, int pred) {
@@ -546,24 +549,27 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
 }
 
 // ---- the same backward with the issuing taken out of the compute groups ---------------------------
-// A slot holds what one row tile needs in shared memory (Q, dO, P, dS); two fit at D = 128 (96 KB each),
-// three at D = 64 (64 KB).  Three producer warps refill a slot's Q / dO the moment its dV / dK MMAs
-// are done; one thread issues whichever batch of MMAs is ready next (S / dP of the tile that has
-// landed, or dV / dK / dQ of the tile whose probabilities are written); two compute groups of 256
-// threads (two warps per TMEM lane quadrant, half of the key columns each) take alternate tiles,
-// turn S / dP into P / dS and, once the MMAs are done, move the tile's dQ from TMEM to the staging tile
-// (its P / dS region) and store it.  Each hand-over is an mbarrier with a bounded wait.
+// Roles: producer warps fill a ring of Q / dO tiles, one warp issues whichever batch of MMAs is ready next (dP and S of
+// a tile that has landed; dV and dK of a tile whose P / dS are written, which give its dO and Q back one after the other;
+// dQ behind them), eight compute warps (two per TMEM lane quadrant, half of the key columns each) turn S, dP into P, dS,
+// and four warps move dQ from TMEM to a staging tile (the tile's P / dS, which the MMAs are done with) and send it off.
+// Each hand-over is an mbarrier with a bounded wait, and each resource is a ring of its own: Q / dO stages, S / dP
+// columns, P / dS tiles, dQ columns.
 //
-// What bounds it is shared memory: the five products read 224 KB of operands per row tile at D = 128
-// (168 KB at D = 64), the gathered rows, P / dS and the staging tile add 160 (112) KB, 3.1 k (2.2 k)
-// cycles at 128 bytes per clock.  The chain of one tile (gather, S / dP, arithmetic, dV / dK / dQ, dQ out)
-// is two to three times that long, so what counts is how many tiles overlap: with three slots the
-// gather and the S / dP of a group's next tile run while its last one is in its MMAs.  D = 64 also
-// computes dV^T and dK^T in one product, [dO | Q]^T [P | dS] (their tiles are neighbours): the two
+// What bounds it.  At D = 128 shared memory: the five products read 224 KB of operands per row tile, the gathered rows,
+// P / dS and the staging tile add 160 KB, 3.1 k cycles at 128 bytes a clock; the 36 MMAs take 2.4 k by themselves (65 to
+// 70 each, N = 64 or 128 alike).  A row tile takes 3.8 k; with groups that did their own tile's dQ between two tiles'
+// arithmetic it was 4.7 k.  At D = 64 (112 + 80 KB, 1.4 k of MMAs) a selection tile takes as long as its gather: 64 to 84
+// boxes for groups of 4 and 3, and a warp gets one out every 65 cycles, so seven warps do it (8 x 4096 tokens, 12 heads of
+// 64: 604 us, 658 with three; copies of 16 bytes by all lanes instead: 746).  That leaves 96 registers a thread, which
+// costs the compute warps more than it gives where the rows are consecutive or two slabs come in one box: three
+// producers there.  D = 64 computes dV^T and dK^T in one product, [dO | Q]^T [P | dS] (their tiles are neighbours): the two
 // off-diagonal quarters are wasted, but the operands are read once, 8 KB a step instead of 12.
-constexpr int kB2Threads = 640;   // 2 x 8 compute warps, 3 producer warps, MMA warp (a 21st warp would cost 16 registers each)
-constexpr int kB2Producers = 3;
-constexpr int kB2Compute = 16;    // compute warps
+// The issuing warp shares its scheduler with compute warps (mma_ss_by, tc_common.cuh): issued by one thread of it the
+// MMAs came out every 85 to 100 cycles.  Sending dQ from registers straight to global memory (32 bytes a lane) took
+// 10.8 ms instead of 9.3 at 8 x 32768 tokens, 16 heads of 128: its stores hold up those of P and dS.
+constexpr int kB2Compute = 8;     // compute warps
+constexpr int kB2Dq = 4;          // dQ warps; then the producers and one MMA warp
 
 // kThreeTerm: selection on 16- and 32-token blocks, whose results are fp32 arithmetic rounded once.  P and dS go to
 // the tensor cores as three bf16 terms each, all 24 bits of the fp32 values (two more of each of the three products they
@@ -571,16 +577,22 @@ constexpr int kB2Compute = 16;    // compute warps
 // row (sel_row.cuh).  P and dS take 96 KB of a slot, so one slot fits.  The whole op on 16-token blocks, forward + backward (2 x 1024 tokens, 16 heads of 128, 8 blocks a
 // list): selection backward with its plan and dQ sum 199 us against 799 on the CUDA cores (182 with two terms), forward
 // 42 against 360, the pass 345 against 1300.
-template <int D, bool kThreeTerm> struct Bwd2 {
+template <int D, bool kThreeTerm, bool kGather> struct Bwd2 {
   static constexpr int kSlabs = D / 64;
   static constexpr int kTerms = kThreeTerm ? 3 : 1;
-  static constexpr int kSlots = kThreeTerm ? 1 : D == 64 ? 3 : 2;
+  static constexpr int kProducers = kGather ? 7 : 3;
+  static constexpr int kThreads = (kB2Compute + kB2Dq + kProducers + 1) * 32;
+  static constexpr int kStages = kThreeTerm ? (D == 64 ? 2 : 1) : (D == 64 ? 3 : 2);    // Q / dO tiles in shared memory
+  static constexpr int kSets = kThreeTerm ? 1 : (D == 64 ? 3 : 2);                      // P / dS tiles
+  static constexpr int kScores = kStages > 1 ? 2 : 1;                                   // S / dP column sets
+  static constexpr int kDqBufs = D == 64 ? 2 : 1;                                       // dQ column sets
   static constexpr int kKVBytes = kKeys * 128 * kSlabs;
   static constexpr int kRowBytes = kRows * 128 * kSlabs;            // Q or dO
-  static constexpr int kSlotBytes = 2 * kRowBytes + 2 * kTerms * kPBytes;    // dO, Q, P, dS (and P, dS: further terms)
-  static constexpr int kBars = 2 + 7 * kSlots;
-  static constexpr size_t kSmem = 2 * kKVBytes + (size_t)kSlots * kSlotBytes + 256 /*barriers*/ +
-                                  (size_t)kSlots * 128 * 4 /*partial rows of a ragged tile*/ + 1024 /*alignment slack*/;
+  static constexpr int kStageBytes = 2 * kRowBytes;                 // dO, Q
+  static constexpr int kSetBytes = 2 * kTerms * kPBytes;            // P, dS (and P, dS: further terms)
+  static constexpr int kBars = 2 + 4 * kStages + kScores + 2 * kSets + 2 * kDqBufs;
+  static constexpr size_t kSmem = 2 * kKVBytes + (size_t)kStages * kStageBytes + (size_t)kSets * kSetBytes + 256 /*barriers*/ +
+                                  128 * 4 /*partial rows of a ragged tile*/ + 1024 /*alignment slack*/;
 };
 
 // dK and dV of one work item in scalar fp32, into acc [dV, dK][64 keys][D] in shared memory, for a tile whose sums are
@@ -693,19 +705,20 @@ __device__ __noinline__ void sel_row_dq(const BwdArgs& p, float* out, int bh, in
   for (int e = 0; e < 32; ++e) out[e] = acc[e];
 }
 
-template <int D, bool kCluster, bool kThreeTerm>
-__global__ void __launch_bounds__(kB2Threads, 1)
+template <int D, bool kCluster, bool kThreeTerm, bool kGather>
+__global__ void __launch_bounds__(Bwd2<D, kThreeTerm, kGather>::kThreads, 1)
 tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
                const __grid_constant__ CUtensorMap tm_q_run, const __grid_constant__ CUtensorMap tm_do_run,
                const __grid_constant__ CUtensorMap tm_dq, const __grid_constant__ BwdArgs p) {
-  using L = Bwd2<D, kThreeTerm>;
-  constexpr int kSlabs = L::kSlabs, kSlots = L::kSlots, kKVBytes = L::kKVBytes;
+  using L = Bwd2<D, kThreeTerm, kGather>;
+  constexpr int kSlabs = L::kSlabs, kStages = L::kStages, kSets = L::kSets, kScores = L::kScores, kDqBufs = L::kDqBufs;
+  constexpr int kKVBytes = L::kKVBytes, kProducers = L::kProducers, kThreads = L::kThreads;
   constexpr uint32_t kTmemCols = 512;
-  // slot s: S at 128 s, dP at 128 s + 64, dQ over both; then dV^T and dK^T: at D = 128 64 columns each, at D = 64
+  // scores i: S at 128 i, dP at 128 i + 64; then dV^T and dK^T: at D = 128 64 columns each, at D = 64
   // the diagonal quarters of one 128 x 128 product (dV^T: lanes 0-63, columns 0-63; dK^T: lanes 64-127,
-  // columns 64-127)
-  constexpr uint32_t kColDV = 128 * kSlots, kColDK = kColDV + 64;
+  // columns 64-127); then dQ
+  constexpr uint32_t kColDV = 256, kColDK = kColDV + 64, kColDQ = 384;
   constexpr uint32_t kIdescS = idesc_bf16(128, kKeys, 0, 0);
   constexpr uint32_t kIdescT = idesc_bf16(128, D == 64 ? 128 : kKeys, 1, 1);
   constexpr uint32_t kIdescDQ = idesc_bf16(128, D, 0, 1);
@@ -714,20 +727,23 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   uint8_t* sK = smem;
   uint8_t* sV = sK + kKVBytes;
-  uint8_t* sSlot = sV + kKVBytes;
-  uint64_t* bars = (uint64_t*)(sSlot + kSlots * L::kSlotBytes);
+  uint8_t* sRow = sV + kKVBytes;                  // [kStages] dO, Q
+  uint8_t* sPds = sRow + kStages * L::kStageBytes;    // [kSets] P, dS
+  uint64_t* bars = (uint64_t*)(sPds + kSets * L::kSetBytes);
   uint64_t* bar_kv = bars + 0;
   uint64_t* bar_drain = bars + 1;
-  uint64_t* g_full = bars + 2;                    // [kSlots] Q / dO of the slot have landed
-  uint64_t* sp_full = g_full + kSlots;            // S / dP of the slot are in TMEM
-  uint64_t* pds_full = sp_full + kSlots;          // P / dS of the slot are in shared memory (256 arrivals)
-  uint64_t* qdo_free = pds_full + kSlots;         // the dV / dK MMAs of the slot are done: Q / dO may be refilled
-  uint64_t* acc_full = qdo_free + kSlots;         // dV / dK / dQ MMAs of the slot are done
-  uint64_t* dq_read = acc_full + kSlots;          // dQ of the slot has left TMEM (256 arrivals)
-  uint64_t* stage_free = dq_read + kSlots;        // dQ of the slot has left its staging tile: P / dS may be written
+  uint64_t* do_full = bars + 2;                   // [kStages] dO has landed
+  uint64_t* q_full = do_full + kStages;           // [kStages] Q has landed
+  uint64_t* do_free = q_full + kStages;           // [kStages] the dV MMAs are done: dO may be refilled
+  uint64_t* q_free = do_free + kStages;           // [kStages] the dK MMAs are done: Q may be refilled
+  uint64_t* sp_full = q_free + kStages;           // [kScores] S / dP are in TMEM
+  uint64_t* pds_full = sp_full + kScores;         // [kSets] P / dS are in shared memory, S / dP have been read (256 arrivals)
+  uint64_t* pds_free = pds_full + kSets;          // [kSets] dQ has left its staging tile: P / dS may be written
+  uint64_t* acc_full = pds_free + kSets;          // [kDqBufs] all MMAs of the tile are done
+  uint64_t* dq_read = acc_full + kDqBufs;         // [kDqBufs] dQ has left TMEM (128 arrivals)
   uint32_t* s_tmem = (uint32_t*)(bars + L::kBars);
   volatile int* s_abort = (volatile int*)(s_tmem + 1);
-  uint32_t* s_prow = (uint32_t*)(bars + 32);      // [kSlots][128] partial row of each tile row (ragged tile)
+  uint32_t* s_prow = (uint32_t*)(bars + 32);      // [128] partial row of each tile row (ragged tile)
   static_assert(L::kBars * 8 + 8 <= 256, "barrier region");
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -787,17 +803,17 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
 
   if (tid == 0) {
     int bad = (*(volatile int*)p.status != 0) ? 1 : 0;
-    if ((size_t)((uint8_t*)(s_prow + kSlots * 128) - smem_raw) > L::kSmem) {
+    if ((size_t)((uint8_t*)(s_prow + 128) - smem_raw) > L::kSmem) {
       atomicOr(p.status, 256);   // the shared-memory window is less aligned than assumed
       bad = 1;
     }
     *s_abort = bad;
     mbar_init(bar_kv, 1);
     mbar_init(bar_drain, 1);
-    for (int s = 0; s < kSlots; ++s) {
-      mbar_init(g_full + s, 1); mbar_init(sp_full + s, 1); mbar_init(pds_full + s, 256); mbar_init(qdo_free + s, 1);
-      mbar_init(acc_full + s, 1); mbar_init(dq_read + s, 256); mbar_init(stage_free + s, 1);
-    }
+    for (int s = 0; s < 4 * kStages; ++s) mbar_init(do_full + s, 1);
+    for (int s = 0; s < kScores; ++s) mbar_init(sp_full + s, 1);
+    for (int s = 0; s < kSets; ++s) { mbar_init(pds_full + s, kB2Compute * 32); mbar_init(pds_free + s, 1); }
+    for (int s = 0; s < kDqBufs; ++s) { mbar_init(acc_full + s, 1); mbar_init(dq_read + s, kB2Dq * 32); }
     fence_barrier_init();
     prefetch_tensormap(&tm_k); prefetch_tensormap(&tm_v);
     prefetch_tensormap(&tm_q); prefetch_tensormap(&tm_do); prefetch_tensormap(&tm_dq);
@@ -807,45 +823,49 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
     if (!kCluster) return;
     n_tiles = 0;             // the cluster's other CTAs read this one's flag at the end: it stays
   }
-  // rows past nq * G of a tile are never loaded, and dV / dK sum over all 128: keep them zero
-  {
-    // (merged boxes lay the two slabs of a row side by side: one run of 256-byte rows)
-    const int r0 = p.nq * p.G, row_bytes = p.merged ? 256 : 128;
-    const int n = (kRows - r0) * row_bytes / 16, runs = 2 * L::kRowBytes / (kRows * row_bytes);
-    for (int i = tid; i < runs * kSlots * n; i += kB2Threads) {
-      const int part = i / n, slot = part / runs;
-      uint8_t* base = sSlot + slot * L::kSlotBytes + (part % runs) * (kRows * row_bytes);
-      *reinterpret_cast<uint4*>(base + r0 * row_bytes + (i % n) * 16) = make_uint4(0, 0, 0, 0);
+  uint32_t tmem = 0;
+  const bool producer = warp >= kB2Compute + kB2Dq && warp < kB2Compute + kB2Dq + kProducers;
+  if (!producer) {           // the first loads are on their way meanwhile
+    // rows past nq * G of a tile are never loaded, and dV / dK sum over all 128: keep them zero
+    if (warp < kB2Compute + kB2Dq) {
+      // (merged boxes lay the two slabs of a row side by side: one run of 256-byte rows)
+      const int r0 = p.nq * p.G, row_bytes = p.merged ? 256 : 128;
+      const int n = (kRows - r0) * row_bytes / 16, runs = 2 * L::kRowBytes / (kRows * row_bytes);
+      for (int i = tid; i < runs * kStages * n; i += (kB2Compute + kB2Dq) * 32) {
+        const int part = i / n;                        // (stages lie one behind the other)
+        uint8_t* base = sRow + part * (kRows * row_bytes);
+        *reinterpret_cast<uint4*>(base + r0 * row_bytes + (i % n) * 16) = make_uint4(0, 0, 0, 0);
+      }
     }
-  }
-  fence_proxy_async();
-  if (warp == 0) {
-    tmem_alloc(s_tmem, kTmemCols);
-    tmem_relinquish();
-  }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = *s_tmem;
-  // dK^T / dV^T start at zero so that every MMA into them accumulates
-  if (warp < 4) {
-    uint32_t z[32];
+    fence_proxy_async();
+    if (warp == 0) {
+      tmem_alloc(s_tmem, kTmemCols);
+      tmem_relinquish();
+    }
+    tc_fence_before();
+    named_sync_b(2, kThreads - kProducers * 32);
+    tc_fence_after();
+    tmem = *s_tmem;
+    // dK^T / dV^T start at zero so that every MMA into them accumulates
+    if (warp < 4) {
+      uint32_t z[32];
 #pragma unroll
-    for (int c = 0; c < 32; ++c) z[c] = 0u;
-    const uint32_t lb = tmem + ((uint32_t)(warp * 32) << 16);
+      for (int c = 0; c < 32; ++c) z[c] = 0u;
+      const uint32_t lb = tmem + ((uint32_t)(warp * 32) << 16);
 #pragma unroll
-    for (int cc = 0; cc < 4; ++cc) tmem_st32(lb + kColDV + cc * 32, z);
-    tmem_wait_st();
+      for (int cc = 0; cc < 4; ++cc) tmem_st32(lb + kColDV + cc * 32, z);
+      tmem_wait_st();
+    }
+    tc_fence_before();
+    named_sync_b(2, kThreads - kProducers * 32);
+    tc_fence_after();
   }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
 
-  if (warp >= kB2Compute && warp < kB2Compute + kB2Producers) {
+  if (producer) {
     // ---- producers: K / V once, then Q and dO of every tile.  A warp gets a TMA box out every
     // 60-100 cycles whatever its size, so the boxes of a tile are dealt out over three warps
     // (box o to warp o % 3) and, where the shape allows, one box brings both column slabs ---------
-    const int pw = warp - kB2Compute;
+    const int pw = warp - kB2Compute - kB2Dq;
     if (pw == 0 && lane == 0) {
       mbar_expect_tx(bar_kv, 2 * kKVBytes);
 #pragma unroll
@@ -854,11 +874,11 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
         tma_load_3d(sV + s * (kKeys * 128), &tm_v, bar_kv, s * 64, key0, bh);
       }
     }
-    const uint32_t gather_bytes = (uint32_t)(p.nq * p.G * 128 * kSlabs * 2);
-    const int per_q = p.merged ? 2 : kSlabs * 2;     // boxes per query: Q and dO, per slab unless merged
-    const int n_ops = p.nq * per_q;                  // selection: the boxes of a tile
-    constexpr int kRounds = (kMaxNq * kSlabs * 2 + 32 * kB2Producers - 1) / (32 * kB2Producers);
-    auto box_of = [&](int r) -> int { return (r * 32 + lane) * kB2Producers + pw; };
+    const uint32_t tile_bytes = (uint32_t)(p.nq * p.G * 128 * kSlabs);     // of Q or dO
+    const int per_q = p.merged ? 1 : kSlabs;         // boxes per query and tensor: one per slab unless merged
+    const int n_ops = p.nq * per_q;                  // selection: the boxes of a tile, for Q and for dO
+    constexpr int kRounds = (kMaxNq * kSlabs + 32 * kProducers - 1) / (32 * kProducers);
+    auto box_of = [&](int r) -> int { return (r * 32 + lane) * kProducers + pw; };
     auto tq_of = [&](int k, int o) -> int {          // pair of box o of tile k (none: past T, zeros)
       const int qi = (rt_begin + k) * p.nq + o / per_q;
       return (o < n_ops && qi < n_q) ? ldg_s32_now(p.plan.pairs + pair_base + qi) : p.T;
@@ -869,153 +889,173 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
       for (int r = 0; r < kRounds; ++r) tq[r] = tq_of(0, box_of(r));
     }
     const uint64_t pol_keep = l2_policy_evict_normal();   // gathered q / dO rows: read again by other blocks
-    int issued = 0;                                  // tiles whose loads this warp has sent off
+    bool ok = true;
+    int issued = 0;                                  // halves of tiles whose loads this warp has sent off
     for (int k = 0; k < n_tiles; ++k) {
-      const int sb = k % kSlots, u = k / kSlots;
-      // the slot's Q / dO are free once the dV / dK MMAs of its last tile are done (dQ reads dS and K only)
-      if (u > 0) mbar_wait(qdo_free + sb, (u - 1) & 1, p.status, s_abort, 128);
-      if (__any_sync(0xffffffffu, *s_abort)) break;           // the whole warp leaves together
-      uint8_t* sDO = sSlot + sb * L::kSlotBytes;
-      uint8_t* sQ = sDO + L::kRowBytes;
-      if (pw == 0 && lane == 0) mbar_expect_tx(g_full + sb, gather_bytes);
-      __syncwarp();
-      if (p.kind != 2) {
-        // window / compression: the tile's queries are consecutive tokens, one box per slab
-        if (pw == 0 && lane == 0) {
-          const int qi = (rt_begin + k) * p.nq;
-          const int t0 = qi < n_q ? t_lo + qi : p.T;
+      const int sb = k % kStages, u = k / kStages;
+      // dO, which the dV MMAs give back before the dK MMAs do Q (dQ reads dS and K only), then Q
 #pragma unroll
-          for (int s = 0; s < kSlabs; ++s) {
-            tma_load_3d(sQ + s * (kRows * 128), &tm_q_run, g_full + sb, s * 64, b * p.Hq + hkv * p.G, t0);
-            tma_load_3d(sDO + s * (kRows * 128), &tm_do_run, g_full + sb, s * 64, b * p.Hq + hkv * p.G, t0);
+      for (int half = 0; half < 2; ++half) {
+        uint64_t* full = (half ? q_full : do_full) + sb;
+        if (u > 0) ok = mbar_wait((half ? q_free : do_free) + sb, (u - 1) & 1, p.status, s_abort, 128);
+        if (!(ok = __all_sync(0xffffffffu, ok))) break;       // the whole warp leaves together
+        uint8_t* dst = sRow + sb * L::kStageBytes + half * L::kRowBytes;
+        if (pw == 0 && lane == 0) mbar_expect_tx(full, tile_bytes);
+        __syncwarp();
+        if (p.kind != 2) {
+          // window / compression: the tile's queries are consecutive tokens, one box per slab
+          if (pw == 0 && lane == 0) {
+            const int qi = (rt_begin + k) * p.nq;
+            const int t0 = qi < n_q ? t_lo + qi : p.T;
+#pragma unroll
+            for (int s = 0; s < kSlabs; ++s)
+              tma_load_3d(dst + s * (kRows * 128), half ? &tm_q_run : &tm_do_run, full, s * 64, b * p.Hq + hkv * p.G, t0);
+          }
+        } else {
+#pragma unroll
+          for (int r = 0; r < kRounds; ++r) {
+            const int o = box_of(r);
+            const int t_box = (int)(tq[r] & kPairPosMask);   // here: not where the load would be waited for
+            if (o >= n_ops) continue;
+            if (p.merged) {
+              tma_load_5d_hint(dst + o * (p.G / 8) * 2048, half ? &tm_q : &tm_do, full, 0, 0, 0, t_box,
+                               (b * p.Hq + hkv * p.G) >> 3, pol_keep);
+            } else {
+              const int qq = o / kSlabs, s = o % kSlabs;
+              tma_load_3d(dst + s * (kRows * 128) + qq * p.G * 128, half ? &tm_q : &tm_do, full, s * 64,
+                          b * p.Hq + hkv * p.G, t_box);
+            }
           }
         }
-      } else {
-#pragma unroll
-        for (int r = 0; r < kRounds; ++r) {
-          const int o = box_of(r);
-          const int t_box = (int)(tq[r] & kPairPosMask);   // here: not where the load would be waited for
-          if (o < n_ops && p.merged) {
-            tma_load_5d_hint(((o & 1) ? sDO : sQ) + (o >> 1) * (p.G / 8) * 2048, (o & 1) ? &tm_do : &tm_q, g_full + sb,
-                             0, 0, 0, t_box, (b * p.Hq + hkv * p.G) >> 3, pol_keep);
-          } else if (o < n_ops) {
-            const int qq = o / (kSlabs * 2), kx = o % (kSlabs * 2);
-            const int s = kx >> 1;
-            if (kx & 1)
-              tma_load_3d(sDO + s * (kRows * 128) + qq * p.G * 128, &tm_do, g_full + sb, s * 64,
-                          b * p.Hq + hkv * p.G, t_box);
-            else
-              tma_load_3d(sQ + s * (kRows * 128) + qq * p.G * 128, &tm_q, g_full + sb, s * 64,
-                          b * p.Hq + hkv * p.G, t_box);
-          }
-        }
-        if (k + 1 < n_tiles) {
-#pragma unroll
-          for (int r = 0; r < kRounds; ++r) tq[r] = tq_of(k + 1, box_of(r));
-        }
+        issued = 2 * k + half + 1;
       }
-      issued = k + 1;
+      if (!ok) break;
+      if (p.kind == 2 && k + 1 < n_tiles) {
+#pragma unroll
+        for (int r = 0; r < kRounds; ++r) tq[r] = tq_of(k + 1, box_of(r));
+      }
     }
     if (*s_abort && pw == 0 && lane == 0) {
       // give-up path: the loads still on their way into this CTA's shared memory land (bounded
-      // wait on the last phase of each slot) before the CTA ends
+      // wait on the last phase of each stage) before the CTA ends
       mbar_wait_drain(bar_kv, 0);
-      for (int k = max(0, issued - kSlots); k < issued; ++k) mbar_wait_drain(g_full + k % kSlots, (k / kSlots) & 1);
+      for (int h = max(0, issued - 2 * kStages); h < issued; ++h)
+        mbar_wait_drain((h & 1 ? q_full : do_full) + (h >> 1) % kStages, ((h >> 1) / kStages) & 1);
     }
-  } else if (warp == kB2Compute + kB2Producers) {
+  } else if (warp == kB2Compute + kB2Dq + kProducers) {
     // ---- MMA issuer: whichever batch is ready next ---------------------------------------------
-    if (lane == 0) {
+    {
+      const uint32_t lead = elect_one(), tmem_u = uniform(tmem);
+      auto seen = [](uint64_t* bar, uint32_t parity) -> bool { return __all_sync(0xffffffffu, mbar_test_wait(bar, parity)); };
       mbar_wait(bar_kv, 0, p.status, s_abort, 32);
+      __syncwarp();
       const uint32_t ka = desc_lo_kmajor(smem_u32(sK)), va = desc_lo_kmajor(smem_u32(sV));
       const uint32_t kb = desc_lo_mnmajor(smem_u32(sK), kKeys * 128);
       const uint32_t q_slab = p.merged ? 1024u : (uint32_t)(kRows * 128), q_sbo = p.merged ? 2048u : 1024u;
-      int next_a = 0, next_b = 0;                    // next tile for S / dP, next tile for dV / dK / dQ
-      int sa = 0, ua = 0, sbb = 0, ub = 0;           // their slots and the slots' use counts
+      int next_a = 0, next_b = 0, next_c = 0;        // next tile for S / dP, for dV / dK, for dQ
+      int ga = 0, gb = 0;                            // stages of next_a and next_b
+      int pb = 0, pc = 0, dc = 0;                    // P / dS set of next_b and next_c, dQ columns of next_c
+      uint32_t ph_ga = 0, ph_pb = 0, ph_dc = 0;      // phases to wait for (dq_read: of its last use)
+      bool dp_sent = false;                          // dP of next_a is on its way, S not yet
       long long idle_since = clock64();
       uint32_t polls = 0;
-      while (next_b < n_tiles) {
+      while (next_c < n_tiles) {
         bool progressed = false;
-        if (next_a < n_tiles) {
-          // Q / dO have landed; dQ of the slot's last tile, which lies over its S / dP columns, has been read
-          if (mbar_try_wait(g_full + sa, ua & 1) && (ua == 0 || mbar_try_wait(dq_read + sa, (ua - 1) & 1))) {
+        // (P / dS of tile next_a - kScores are written: its S / dP have been read)
+        if (next_a < n_tiles && next_a < next_b + kScores) {
+          const uint8_t* sDO = sRow + ga * L::kStageBytes;
+          const uint32_t colS = tmem_u + (next_a % kScores) * 128, colDP = colS + 64;
+          if (!dp_sent && seen(do_full + ga, ph_ga)) {
             tc_fence_after();
-            const uint8_t* sDO = sSlot + sa * L::kSlotBytes;
-            const uint32_t qa = desc_lo_kmajor(smem_u32(sDO + L::kRowBytes)), da = desc_lo_kmajor(smem_u32(sDO));
-            const uint32_t colS = tmem + sa * 128, colDP = colS + 64;
+            const uint32_t da = desc_lo_kmajor(smem_u32(sDO));
 #pragma unroll
             for (int kk = 0; kk < D / 16; ++kk) {
               const uint32_t slab = kk >> 2, in = (kk & 3) * 32;
-              mma_ss(colS, desc_at_sbo(qa, slab * q_slab + in, q_sbo), desc_at(ka, slab * (kKeys * 128) + in),
+              mma_ss_by(lead, colDP, desc_at_sbo(da, slab * q_slab + in, q_sbo), desc_at(va, slab * (kKeys * 128) + in),
                      kIdescS, kk > 0);
             }
+            dp_sent = progressed = true;
+          }
+          if (dp_sent && seen(q_full + ga, ph_ga)) {
+            tc_fence_after();
+            const uint32_t qa = desc_lo_kmajor(smem_u32(sDO + L::kRowBytes));
 #pragma unroll
             for (int kk = 0; kk < D / 16; ++kk) {
               const uint32_t slab = kk >> 2, in = (kk & 3) * 32;
-              mma_ss(colDP, desc_at_sbo(da, slab * q_slab + in, q_sbo), desc_at(va, slab * (kKeys * 128) + in),
+              mma_ss_by(lead, colS, desc_at_sbo(qa, slab * q_slab + in, q_sbo), desc_at(ka, slab * (kKeys * 128) + in),
                      kIdescS, kk > 0);
             }
-            tc_commit(sp_full + sa);
+            tc_commit_by(lead, sp_full + next_a % kScores);
             ++next_a;
-            if (++sa == kSlots) { sa = 0; ++ua; }
+            if (++ga == kStages) { ga = 0; ph_ga ^= 1; }
+            dp_sent = false;
             progressed = true;
           }
         }
-        if (next_b < next_a) {
-          if (mbar_try_wait(pds_full + sbb, ub & 1)) {
-            tc_fence_after();
-            const uint8_t* sDO = sSlot + sbb * L::kSlotBytes;
-            const uint8_t* sP = sDO + 2 * L::kRowBytes;
-            const uint8_t* sDS = sP + kPBytes;       // (three-term: P, dS, then their further terms)
-            const uint32_t dsk = desc_lo_kmajor(smem_u32(sDS));
+        if (next_b < next_a && seen(pds_full + pb, ph_pb)) {
+          tc_fence_after();
+          const uint8_t* sDO = sRow + gb * L::kStageBytes;
+          const uint8_t* sP = sPds + pb * L::kSetBytes;
+          const uint8_t* sDS = sP + kPBytes;         // (three-term: P, dS, then their further terms)
 #pragma unroll
-            for (uint32_t term = 0; term < L::kTerms * 2 * kPBytes; term += 2 * kPBytes) {
-              if (D == 64) {
-                // A: the dO and Q tiles as two 64-column slabs, B: the P and dS tiles likewise
-                const uint32_t da = desc_lo_mnmajor(smem_u32(sDO), L::kRowBytes);
-                const uint32_t pa = desc_lo_mnmajor(smem_u32(sP), kPBytes);
+          for (uint32_t term = 0; term < L::kTerms * 2 * kPBytes; term += 2 * kPBytes) {
+            if (D == 64) {
+              // A: the dO and Q tiles as two 64-column slabs, B: the P and dS tiles likewise
+              const uint32_t da = desc_lo_mnmajor(smem_u32(sDO), L::kRowBytes);
+              const uint32_t pa = desc_lo_mnmajor(smem_u32(sP), kPBytes);
 #pragma unroll
-                for (int kk = 0; kk < kRows / 16; ++kk)        // contraction over the 128 rows, 16 a step
-                  mma_ss(tmem + kColDV, desc_at(da, kk * 2048), desc_at(pa, term + kk * 2048), kIdescT, 1);
-              } else {
-                const uint32_t da = desc_lo_mnmajor(smem_u32(sDO), q_slab);
-                const uint32_t qa = desc_lo_mnmajor(smem_u32(sDO + L::kRowBytes), q_slab);
-                const uint32_t pa = desc_lo_mnmajor(smem_u32(sP), 0), dsa = desc_lo_mnmajor(smem_u32(sDS), 0);
+              for (int kk = 0; kk < kRows / 16; ++kk)        // contraction over the 128 rows, 16 a step
+                mma_ss_by(lead, tmem_u + kColDV, desc_at(da, kk * 2048), desc_at(pa, term + kk * 2048), kIdescT, 1);
+            } else {
+              const uint32_t da = desc_lo_mnmajor(smem_u32(sDO), q_slab);
+              const uint32_t qa = desc_lo_mnmajor(smem_u32(sDO + L::kRowBytes), q_slab);
+              const uint32_t pa = desc_lo_mnmajor(smem_u32(sP), 0), dsa = desc_lo_mnmajor(smem_u32(sDS), 0);
 #pragma unroll
-                for (int kk = 0; kk < kRows / 16; ++kk)
-                  mma_ss(tmem + kColDV, desc_at_sbo(da, kk * 2 * q_sbo, q_sbo), desc_at(pa, term + kk * 2048), kIdescT, 1);
+              for (int kk = 0; kk < kRows / 16; ++kk)
+                mma_ss_by(lead, tmem_u + kColDV, desc_at_sbo(da, kk * 2 * q_sbo, q_sbo), desc_at(pa, term + kk * 2048), kIdescT, 1);
+              if (term == (L::kTerms - 1) * 2 * kPBytes) tc_commit_by(lead, do_free + gb);
 #pragma unroll
-                for (int kk = 0; kk < kRows / 16; ++kk)
-                  mma_ss(tmem + kColDK, desc_at_sbo(qa, kk * 2 * q_sbo, q_sbo), desc_at(dsa, term + kk * 2048), kIdescT, 1);
-              }
+              for (int kk = 0; kk < kRows / 16; ++kk)
+                mma_ss_by(lead, tmem_u + kColDK, desc_at_sbo(qa, kk * 2 * q_sbo, q_sbo), desc_at(dsa, term + kk * 2048), kIdescT, 1);
             }
-            tc_commit(qdo_free + sbb);
-#pragma unroll
-            for (uint32_t term = 0; term < L::kTerms * 2 * kPBytes; term += 2 * kPBytes)
-#pragma unroll
-              for (int kk = 0; kk < kKeys / 16; ++kk)        // contraction over the 64 keys
-                mma_ss(tmem + sbb * 128, desc_at(dsk, term + kk * 32), desc_at(kb, kk * 2048), kIdescDQ, term > 0 || kk > 0);
-            tc_commit(acc_full + sbb);
-            ++next_b;
-            if (++sbb == kSlots) { sbb = 0; ++ub; }
-            progressed = true;
           }
+          if (D == 64) tc_commit_by(lead, do_free + gb);
+          tc_commit_by(lead, q_free + gb);
+          ++next_b;
+          if (++gb == kStages) gb = 0;
+          if (++pb == kSets) { pb = 0; ph_pb ^= 1; }
+          progressed = true;
+        }
+        if (next_c < next_b && (next_c < kDqBufs || seen(dq_read + dc, ph_dc ^ 1))) {
+          tc_fence_after();
+          const uint32_t dsk = desc_lo_kmajor(smem_u32(sPds + pc * L::kSetBytes + kPBytes));
+#pragma unroll
+          for (uint32_t term = 0; term < L::kTerms * 2 * kPBytes; term += 2 * kPBytes)
+#pragma unroll
+            for (int kk = 0; kk < kKeys / 16; ++kk)          // contraction over the 64 keys
+              mma_ss_by(lead, tmem_u + kColDQ + dc * D, desc_at(dsk, term + kk * 32), desc_at(kb, kk * 2048), kIdescDQ, term > 0 || kk > 0);
+          tc_commit_by(lead, acc_full + dc);
+          ++next_c;
+          if (++pc == kSets) pc = 0;
+          if (++dc == kDqBufs) { dc = 0; ph_dc ^= 1; }
+          progressed = true;
         }
         if (progressed) {
           idle_since = clock64();
         } else if ((++polls & 0xffu) == 0) {
-          if (*s_abort) break;
-          if (*(volatile int*)p.status != 0) { *s_abort = 1; break; }
-          if (clock64() - idle_since > kWaitLimitCycles) { atomicOr(p.status, 2048); *s_abort = 1; break; }
+          bool leave = *s_abort != 0;
+          if (!leave && *(volatile int*)p.status != 0) leave = true;
+          if (!leave && clock64() - idle_since > kWaitLimitCycles) { atomicOr(p.status, 2048); leave = true; }
+          if (__any_sync(0xffffffffu, leave)) { *s_abort = 1; break; }
         }
       }
       // the tensor pipe is idle before TMEM is read for dK / dV and given back, whatever happened
-      tc_commit(bar_drain);
+      tc_commit_by(lead, bar_drain);
       if (!mbar_wait(bar_drain, 0, p.status, s_abort, 4096)) mbar_wait_drain(bar_drain, 0);
     }
   } else if (warp < kB2Compute) {
-    // ---- compute group `grp`: tiles grp, grp + 2, ... -------------------------------------------------
-    const int grp = warp >> 3, wg = warp & 7, lt = (warp & 7) * 32 + lane;
-    const int quad = wg & 3, half = wg >> 2;           // TMEM lane quadrant, key-column half
+    // ---- compute warps: S, dP -> P, dS, tile after tile -------------------------------------------
+    const int quad = warp & 3, half = warp >> 2;       // TMEM lane quadrant, key-column half
     const int row = quad * 32 + lane;
     const int ql = row / p.G, g = row % p.G;
     const int head = hkv * p.G + g;
@@ -1029,12 +1069,8 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
       return t_lo + qi;
     };
     auto row_index = [&](int t) -> size_t { return (size_t)(b * p.Hq + head) * p.T + (t & (int)kPairPosMask); };
-    // With one slot one group does every tile: a group that skipped the other's use of the slot would wait for
-    // a phase two ahead, which a parity does not tell from the one before.
-    constexpr int kGroups = kSlots == 1 ? 1 : 2;
-    const int k_end = grp < kGroups ? n_tiles : 0;
-    int t_cur = grp < k_end ? row_query(grp) : -1;
-    int t_nxt = grp + kGroups < k_end ? row_query(grp + kGroups) : -1;
+    int t_cur = row_query(0);
+    int t_nxt = n_tiles > 1 ? row_query(1) : -1;
     float lse_cur = 0.f, delta_cur = 0.f, gate_cur = 1.f;
     if (t_cur >= 0) {
       lse_cur = __ldg(p.lse + row_index(t_cur));
@@ -1042,13 +1078,11 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
       if (p.row_scale) gate_cur = __ldg(p.row_scale + row_index(t_cur));
     }
     const bool repeats = kThreeTerm && __ldg(&p.plan.hdr->repeats) != 0ull;
-    // A given-up wait does not part a group: its warps go on to the barrier below, which decides for all.
-    for (int k = grp; k < k_end; k += kGroups) {
-      const int sb = k % kSlots, u = k / kSlots;
-      uint8_t* sP = sSlot + sb * L::kSlotBytes + 2 * L::kRowBytes;
+    for (int k = 0; k < n_tiles; ++k) {
+      uint8_t* sP = sPds + (k % kSets) * L::kSetBytes;
       uint8_t* sDS = sP + kPBytes;
-      const uint32_t lane_base = tmem + ((uint32_t)(quad * 32) << 16) + sb * 128;
-      const int t_nn = (k + 2 * kGroups < k_end) ? row_query(k + 2 * kGroups) : -1;
+      const uint32_t lane_base = tmem + ((uint32_t)(quad * 32) << 16) + (k % kScores) * 128;
+      const int t_nn = k + 2 < n_tiles ? row_query(k + 2) : -1;
       float lse_nxt = 0.f, delta_nxt = 0.f, gate_nxt = 1.f;
       if (t_nxt >= 0) {
         lse_nxt = ldg_f32_now(p.lse + row_index(t_nxt));
@@ -1072,7 +1106,6 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
       // (gate p)^T dO; dS = scale * gate * p * (dP - delta), the constant factors folded once per row
       const float lse2 = lse_cur * kLog2e - __log2f(gate_cur);
       const float dscale = p.scale, ddelta = delta_cur * p.scale;
-      const bool row_again = kThreeTerm && t_cur >= 0 && lse2 == lse2 && ddelta == ddelta;
       // every column of this thread's half is attended (the usual case away from the diagonal)?
       const bool all_cols = lo <= half * 32 && hi >= half * 32 + 31 && groups == 0x3u && !repeats;
       float times[2] = {1.f, 1.f};                   // how often the row's list names the blocks of its column groups
@@ -1081,15 +1114,8 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
 #pragma unroll
         for (int e = 0; e < 2; ++e) times[e] = (float)times_listed(list, p.S, (key0 + half * 32 + 16 * e) / p.block_size);
       }
-      mbar_wait(sp_full + sb, u & 1, p.status, s_abort, 64);
-      // the P / dS tiles double as the dQ staging tile: the store of the slot's last tile has read it
-      // (the thread that stored says so, below)
-      if (lt == 0 && k > grp) {
-        bulk_wait_read();
-        mbar_arrive(stage_free + (k - kGroups) % kSlots);
-      }
-      if (u > 0) mbar_wait(stage_free + sb, (u - 1) & 1, p.status, s_abort, 64);
-      __syncwarp();
+      bool ok = mbar_wait(sp_full + k % kScores, (k / kScores) & 1, p.status, s_abort, 64);
+      if (!__all_sync(0xffffffffu, ok)) break;                 // the whole warp leaves together
       tc_fence_after();
       {
         uint32_t rs[32], rp[32];
@@ -1132,6 +1158,9 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
             put(c2, pv[0], pv[1], dv[0], dv[1]);
           }
         }
+        // the P / dS tiles double as the dQ staging tile: the store of the set's last tile has read it
+        if (k >= kSets) ok = mbar_wait(pds_free + k % kSets, ((k / kSets) - 1) & 1, p.status, s_abort, 64);
+        if (!__all_sync(0xffffffffu, ok)) break;
         const uint32_t p_row = smem_u32(sP) + row * 128, ds_row = smem_u32(sDS) + row * 128;
 #pragma unroll
         for (int k4 = 0; k4 < 4; ++k4) {
@@ -1160,34 +1189,48 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
       }
       fence_proxy_async();
       tc_fence_before();
-      mbar_arrive(pds_full + sb);
-      // ---- the tile's dQ: TMEM -> bf16 -> staging tile (the P / dS region, free once the MMAs are
-      // done) -> partial buffer, while the producers fetch the slot's next tile
-      const int i = rt_begin + k;
-      uint8_t* stage = sP;
-      mbar_wait(acc_full + sb, u & 1, p.status, s_abort, 128);
+      mbar_arrive(pds_full + k % kSets);
+      t_cur = t_nxt; t_nxt = t_nn; lse_cur = lse_nxt; delta_cur = delta_nxt; gate_cur = gate_nxt;
+    }
+  } else {
+    // ---- dQ of every tile: TMEM -> bf16 -> staging tile (its P / dS, which the MMAs are done with) -> partial buffer ----
+    const int quad = warp & 3, lt = tid - kB2Compute * 32;
+    const int row = quad * 32 + lane;
+    const int ql = row / p.G, g = row % p.G;
+    const bool row_slot_ok = ql < p.nq;
+    for (int k = 0; k < n_tiles; ++k) {
+      const int dc = k % kDqBufs;
+      const int i = rt_begin + k, qi = i * p.nq + ql;
+      uint8_t* stage = sPds + (k % kSets) * L::kSetBytes;
+      const uint32_t lane_base = tmem + ((uint32_t)(quad * 32) << 16) + kColDQ + dc * D;
+      const bool ok = mbar_wait(acc_full + dc, (k / kDqBufs) & 1, p.status, s_abort, 128);
       __syncwarp();
       tc_fence_after();
 #pragma unroll
-      for (int cc = 0; cc < D / 64; ++cc) {          // this thread's half of the D columns
-        const int col0 = half * (D / 2) + cc * 32;
+      for (int cc = 0; cc < D / 32; ++cc) {
+        const int col0 = cc * 32;
         uint32_t r32[32];
         tmem_ld32(lane_base + col0, r32);
         tmem_wait_ld();
-        if (cc == D / 64 - 1) {            // dQ is in registers: S / dP of the slot's next tile may land
+        if (cc == D / 32 - 1) {            // dQ is in registers: the columns' next dQ may land
           tc_fence_before();
-          mbar_arrive(dq_read + sb);
+          mbar_arrive(dq_read + dc);
         }
         if (kThreeTerm) {                    // fp32 staging: slabs of 128 rows x 32 columns
           float z = 0.f;                   // x * 0: 0 or NaN
 #pragma unroll
           for (int e = 0; e < 32; ++e) z = fmaf(__uint_as_float(r32[e]), 0.f, z);
-          // (a row whose own statistics are NaN has NaN in every column, here as there)
-          if (z != 0.f && row_again) {
-            float again[32];
-            sel_row_dq<D>(p, again, bh, head, t_cur, key0, col0);
+          if (z != 0.f && row_slot_ok && qi < n_q) {
+            const int head = hkv * p.G + g, pair = __ldg(p.plan.pairs + pair_base + qi);
+            const size_t at = (size_t)(b * p.Hq + head) * p.T + (pair & (int)kPairPosMask);
+            const float lse2 = __ldg(p.lse + at) * kLog2e - (p.row_scale ? __log2f(__ldg(p.row_scale + at)) : 0.f);
+            const float ddelta = __ldg(p.delta + at) * p.scale;
+            if (lse2 == lse2 && ddelta == ddelta) {      // (NaN statistics: NaN in every column, here as there)
+              float again[32];
+              sel_row_dq<D>(p, again, bh, head, pair, key0, col0);
 #pragma unroll
-            for (int e = 0; e < 32; ++e) r32[e] = __float_as_uint(again[e]);
+              for (int e = 0; e < 32; ++e) r32[e] = __float_as_uint(again[e]);
+            }
           }
           __syncwarp();
           const uint32_t rbase = smem_u32(stage) + (col0 >> 5) * (kRows * 128) + row * 128;
@@ -1208,10 +1251,8 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
         }
       }
       const bool full_tile = (i + 1) * p.nq <= n_q;
-      uint32_t* prow_s = s_prow + sb * 128;
-      if (!full_tile && half == 0) {
+      if (!full_tile) {
         uint32_t prow = 0xffffffffu;
-        const int qi = i * p.nq + ql;
         if (row_slot_ok && qi < n_q) {
           if (p.kind == 2) {
             prow = (uint32_t)((size_t)(pair_base + qi) * p.G + g);
@@ -1220,10 +1261,10 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
             prow = (uint32_t)((((size_t)bh * p.T + t_lo + qi) * p.n_slots + slot) * p.G + g);
           }
         }
-        prow_s[row] = prow;
+        s_prow[row] = prow;
       }
       fence_proxy_async();
-      if (named_or_b(1 + grp, 256, *s_abort)) break;           // the whole group leaves together
+      if (named_or_b(1, kB2Dq * 32, !ok)) break;               // the whole group leaves together
       if (full_tile) {
         // its rows are consecutive in the partial buffer: one TMA store per slab
         if (lt == 0) {
@@ -1235,13 +1276,15 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
           for (int sl = 0; sl < kParts; ++sl)
             tma_store_5d_hint(&tm_dq, stage + sl * (kRows * 128), sl * (D / kParts), 0, slot, mid, outer, l2_policy_evict_first());
           bulk_commit();
+          bulk_wait_read();
+          mbar_arrive(pds_free + k % kSets);
         }
       } else {   // the ragged last tile: whole rows out by hand, 16 bytes a lane
         constexpr int kChunks = kThreeTerm ? D / 4 : D / 8;
-        constexpr int kRowsPerPass = 256 / kChunks;
+        constexpr int kRowsPerPass = kB2Dq * 32 / kChunks;
         const int c = lt % kChunks;
         for (int r = lt / kChunks; r < kRows; r += kRowsPerPass) {
-          const uint32_t prow = prow_s[r];
+          const uint32_t prow = s_prow[r];
           if (prow != 0xffffffffu) {
             const uint4 v = *reinterpret_cast<const uint4*>(stage + (c >> 3) * (kRows * 128) + r * 128 +
                                                             (((c & 7) ^ (r & 7)) << 4));
@@ -1249,108 +1292,82 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
           }
         }
       }
-      t_cur = t_nxt; t_nxt = t_nn; lse_cur = lse_nxt; delta_cur = delta_nxt; gate_cur = gate_nxt;
     }
-    if (lt == 0) bulk_wait_all();
   }
 
-  // ---- dK^T, dV^T: lane = d, column = key; compute group 0 writes dV, group 1 writes dK ----------
+  // ---- dK^T, dV^T: lane = d, column = key; warps 0-3 have dV, 4-7 dK.  Through shared memory, so that they leave in
+  // rows of a key -----------------------------------------------------------------------------------
   __syncthreads();           // the MMA thread has seen the tensor pipe drain (bar_drain)
   tc_fence_after();
-  bool redone = false;
-  float* s_acc = reinterpret_cast<float*>(sSlot);      // cluster: [dV, dK][64 keys][D], over the slots
-  if (kThreeTerm) {
-    // sums that are not finite are formed again, leaving out what a row does not attend
-    float z = 0.f;
-    if (warp < kB2Compute && ((warp >> 2) & 1) == 0 && !*s_abort) {
-      const uint32_t lb = tmem + ((uint32_t)((warp & 3) * 32) << 16);
-      const bool mine = D == 128 || ((warp & 3) >> 1) == (warp >> 3);
-      uint32_t r32[32];
-#pragma unroll
-      for (int hc = 0; hc < 2; ++hc) {
-        tmem_ld32(lb + (warp >> 3 ? kColDK : kColDV) + hc * 32, r32);
-        tmem_wait_ld();
-#pragma unroll
-        for (int c = 0; c < 32; ++c)
-          if (mine) z = fmaf(__uint_as_float(r32[c]), 0.f, z);
-      }
-    }
-    if (__syncthreads_or(z != 0.f)) {
-      const int first = rt_begin * p.nq, rows = max(0, min(n_tiles * p.nq, n_q - first)) * p.G;
-      sel_tile_dkdv<D>(p, s_acc, bh, j, pair_base + first, rows);
-      if (!kCluster && !*s_abort)
-        for (int i = tid; i < 2 * kKeys * D; i += kB2Threads) {
-          const int which = i / (kKeys * D), key = key0 + (i / D) % kKeys;
-          if (key >= p.Lk) continue;
-          const size_t o = ((size_t)bh * p.Lk + key) * D + i % D;
-          if (split) atomicAdd((which == 0 ? p.dv_acc : p.dk_acc) + o, s_acc[i]);
-          else (which == 0 ? p.dv : p.dk)[o] = __float2bfloat16_rn(s_acc[i]);
-        }
-      redone = true;
-    }
-  }
-  if (!redone && warp < kB2Compute && ((warp >> 2) & 1) == 0 && !*s_abort) {
-    const int grp = warp >> 3, quad = warp & 3;
+  float* s_acc = reinterpret_cast<float*>(sRow);       // [dV, dK][64 keys][D], over the stages
+  float z = 0.f;             // three-term: x * 0 of every sum, 0 or NaN
+  if (warp < 8 && !*s_abort) {
+    const int which = warp >> 2, quad = warp & 3;
     // D = 64: dV^T sits in lanes 0-63, dK^T in lanes 64-127
-    const bool mine = D == 128 || (quad >> 1) == grp;
-    if (mine) {
-      const uint32_t col = grp == 0 ? kColDV : kColDK;
-      const uint32_t lane_base = tmem + ((uint32_t)(quad * 32) << 16);
+    if (D == 128 || (quad >> 1) == which) {
+      const uint32_t lane_base = tmem + ((uint32_t)(quad * 32) << 16) + (which ? kColDK : kColDV);
       const int d = (D == 128 ? quad : quad & 1) * 32 + lane;
 #pragma unroll
       for (int hc = 0; hc < 2; ++hc) {
         uint32_t r32[32];
-        tmem_ld32(lane_base + col + hc * 32, r32);
+        tmem_ld32(lane_base + hc * 32, r32);
         tmem_wait_ld();
 #pragma unroll
         for (int c = 0; c < 32; ++c) {
-          const int key = key0 + hc * 32 + c;
-          if (kCluster) {
-            s_acc[(grp * kKeys + hc * 32 + c) * D + d] = __uint_as_float(r32[c]);
-          } else if (key < p.Lk) {
-            const size_t o = ((size_t)bh * p.Lk + key) * D + d;
-            if (split && p.acc_stride) (grp == 0 ? p.dv_acc : p.dk_acc)[blockIdx.z * p.acc_stride + o] = __uint_as_float(r32[c]);
-            else if (split) atomicAdd((grp == 0 ? p.dv_acc : p.dk_acc) + o, __uint_as_float(r32[c]));
-            else (grp == 0 ? p.dv : p.dk)[o] = __float2bfloat16_rn(__uint_as_float(r32[c]));
-          }
+          s_acc[(which * kKeys + hc * 32 + c) * D + d] = __uint_as_float(r32[c]);
+          if (kThreeTerm) z = fmaf(__uint_as_float(r32[c]), 0.f, z);
         }
       }
     }
   }
+  // sums that are not finite are formed again, leaving out what a row does not attend
+  if (kThreeTerm && __syncthreads_or(z != 0.f)) {
+    const int first = rt_begin * p.nq, rows = max(0, min(n_tiles * p.nq, n_q - first)) * p.G;
+    sel_tile_dkdv<D>(p, s_acc, bh, j, pair_base + first, rows);
+  }
+  // the CTAs of a cluster add their sums, each a share of the keys, in rank order
+  int aborted = 0;
   if (kCluster) {
-    // the CTAs of the cluster add their accumulators, each a share of the keys, in rank order
     cluster_sync();
-    int aborted = 0;
     for (int r = 0; r < csize; ++r) aborted |= ld_peer_s32(const_cast<int*>(s_abort), r);
-    if (!aborted) {
-      const int n = 2 * kKeys * D / 4 / csize;           // float4s per CTA
-      for (int i = tid; i < n; i += kB2Threads) {
-        const int e = (rank * n + i) * 4;
-        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  } else {
+    __syncthreads();
+    aborted = *s_abort;
+  }
+  if (!aborted) {
+    const int n = 2 * kKeys * D / 4 / csize;           // float4s per CTA
+    for (int i = tid; i < n; i += kThreads) {
+      const int e = (rank * n + i) * 4;
+      float4 acc;
+      if (kCluster) {
+        acc = make_float4(0.f, 0.f, 0.f, 0.f);
         for (int r = 0; r < csize; ++r) {
           const float4 v = ld_peer_f32x4(s_acc + e, r);
           acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
         }
-        const int which = e / (kKeys * D), key = key0 + (e / D) % kKeys, d = e % D;
-        if (key < p.Lk) {
-          const size_t o = ((size_t)bh * p.Lk + key) * D + d;
-          if (split) {
-            float* dst = (which == 0 ? p.dv_acc : p.dk_acc) + o;
-            atomicAdd(dst, acc.x); atomicAdd(dst + 1, acc.y); atomicAdd(dst + 2, acc.z); atomicAdd(dst + 3, acc.w);
-          } else {
-            __nv_bfloat16* dst = (which == 0 ? p.dv : p.dk) + o;
-            if (((uintptr_t)dst & 7) == 0) {
-              *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16(acc.x, acc.y), pack_bf16(acc.z, acc.w));
-            } else {                                     // a caller's tensor may start anywhere
-              dst[0] = __float2bfloat16_rn(acc.x); dst[1] = __float2bfloat16_rn(acc.y);
-              dst[2] = __float2bfloat16_rn(acc.z); dst[3] = __float2bfloat16_rn(acc.w);
-            }
+      } else {
+        acc = *reinterpret_cast<const float4*>(s_acc + e);
+      }
+      const int which = e / (kKeys * D), key = key0 + (e / D) % kKeys, d = e % D;
+      if (key < p.Lk) {
+        const size_t o = ((size_t)bh * p.Lk + key) * D + d;
+        if (split) {
+          float* dst = (which == 0 ? p.dv_acc : p.dk_acc) + o;
+          if (p.acc_stride) *reinterpret_cast<float4*>(dst + blockIdx.z * p.acc_stride) = acc;
+          else { atomicAdd(dst, acc.x); atomicAdd(dst + 1, acc.y); atomicAdd(dst + 2, acc.z); atomicAdd(dst + 3, acc.w); }
+        } else {
+          __nv_bfloat16* dst = (which == 0 ? p.dv : p.dk) + o;
+          if (((uintptr_t)dst & 7) == 0) {
+            *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16(acc.x, acc.y), pack_bf16(acc.z, acc.w));
+          } else {                                     // a caller's tensor may start anywhere
+            dst[0] = __float2bfloat16_rn(acc.x); dst[1] = __float2bfloat16_rn(acc.y);
+            dst[2] = __float2bfloat16_rn(acc.z); dst[3] = __float2bfloat16_rn(acc.w);
           }
         }
       }
     }
-    cluster_sync();            // nobody leaves while its memory is read
   }
+  if (kCluster) cluster_sync();            // nobody leaves while its memory is read
   tc_fence_before();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tmem, kTmemCols);
@@ -1618,8 +1635,8 @@ static BwdPlan plan_bwd(const AttnArgs& a) {
   BwdPlan pl;
   const int G = a.Hq / a.Hkv;
   pl.nq = kRows / G;
-  pl.n_ktiles = (a.Lk + kKeys - 1) / kKeys;
   const size_t units = (size_t)a.B * a.Hkv;
+  pl.n_ktiles = (a.Lk + kKeys - 1) / kKeys;
   size_t part_rows;
   if (a.kind == 2) {
     pl.n_slots = a.S;
@@ -1672,6 +1689,77 @@ static BwdPlan plan_bwd(const AttnArgs& a) {
   if (pl.sel_split) off += 2 * align_up((size_t)a.B * a.Hkv * a.Lk * a.D * sizeof(float), 256);
   pl.total = off;
   return pl;
+}
+
+// the kernels with tiles of 64 keys
+static int bwd_narrow(const AttnArgs& a, const BwdArgs& p, const BwdPlan& pl, bool roles, cudaStream_t st) {
+  const int G = p.G;
+  CUtensorMap tm_k, tm_v, tm_q, tm_do;
+  int rc = make_map(&tm_k, a.k, a.D, a.Lk, a.B * a.Hkv, kKeys, 1);
+  if (rc == NSA_OK) rc = make_map(&tm_v, a.v, a.D, a.Lk, a.B * a.Hkv, kKeys, 1);
+  if (rc == NSA_OK) rc = p.merged ? make_map_query_both_slabs(&tm_q, a.q, a.T, a.B * a.Hq, G)
+                                  : make_map_query_rows(&tm_q, a.q, a.D, a.T, a.B * a.Hq, G);
+  if (rc == NSA_OK) rc = p.merged ? make_map_query_both_slabs(&tm_do, a.d_o, a.T, a.B * a.Hq, G)
+                                  : make_map_query_rows(&tm_do, a.d_o, a.D, a.T, a.B * a.Hq, G);
+  CUtensorMap tm_q_run, tm_do_run;
+  if (rc == NSA_OK) rc = make_map_query_rows(&tm_q_run, a.q, a.D, a.T, a.B * a.Hq, G, pl.nq);
+  if (rc == NSA_OK) rc = make_map_query_rows(&tm_do_run, a.d_o, a.D, a.T, a.B * a.Hq, G, pl.nq);
+  CUtensorMap tm_dq, tm_dqacc;
+  if (rc == NSA_OK && p.dq_acc_mode) {
+    rc = make_map_dq_acc(&tm_dqacc, a.dq_acc, a.D, G, (size_t)a.T, (size_t)a.B * a.Hkv, pl.nq);
+    tm_dq = tm_dqacc;        // the partial-tile map is not used in this mode
+  } else if (rc == NSA_OK) {
+    rc = a.kind == 2 ? make_map_partial(&tm_dq, p.dq_part, a.D, G, 1, pl.cap_pairs ? pl.cap_pairs : 1, 1, pl.nq, a.three_term)
+                     : make_map_partial(&tm_dq, p.dq_part, a.D, G, pl.n_slots, a.T, (size_t)a.B * a.Hkv, pl.nq);
+    tm_dqacc = tm_dq;        // likewise
+  }
+  if (rc != NSA_OK) return rc;
+  const size_t smem = bwd_smem_bytes(a.D);
+  dim3 grid(pl.n_ktiles, a.B * a.Hkv, pl.n_splits);
+  if (a.kind == 2)
+    grid = dim3((unsigned)((size_t)a.B * a.Hkv * pl.layout.max_items));
+  if (roles) {
+    KernelScope ks(branch_name(kBwdNames, a.kind), st);
+    grid.x *= (unsigned)pl.csize;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.stream = st;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = (unsigned)pl.csize;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = pl.csize > 1 ? 1 : 0;
+    auto go = [&](auto d, auto three_term, auto gather) -> int {
+      constexpr int D = decltype(d)::value;
+      constexpr bool kThreeTerm = decltype(three_term)::value, kGather = decltype(gather)::value;
+      using L = Bwd2<D, kThreeTerm, kGather>;
+      const auto kernel = pl.csize > 1 ? tc_bwd2_kernel<D, true, kThreeTerm, kGather> : tc_bwd2_kernel<D, false, kThreeTerm, kGather>;
+      cfg.blockDim = dim3(L::kThreads);
+      cfg.dynamicSmemBytes = L::kSmem;
+      NSA_CUDA_OK(func_smem((const void*)kernel, L::kSmem));
+      NSA_CUDA_OK(cudaLaunchKernelEx(&cfg, kernel, tm_k, tm_v, tm_q, tm_do, tm_q_run, tm_do_run, tm_dq, p));
+      return NSA_OK;
+    };
+    auto by_form = [&](auto d) -> int {
+      if (a.three_term) return go(d, std::true_type(), std::false_type());
+      // a box per query and slab: 64 to 256 of them a row tile, more than three warps get out in the time of its MMAs
+      if (a.kind == 2 && !p.merged) return go(d, std::false_type(), std::true_type());
+      return go(d, std::false_type(), std::false_type());
+    };
+    rc = a.D == 128 ? by_form(std::integral_constant<int, 128>()) : by_form(std::integral_constant<int, 64>());
+    if (rc != NSA_OK) return rc;
+  } else if (a.D == 128) {
+    NSA_CUDA_OK(func_smem((const void*)tc_bwd_kernel<128>, smem));
+    KernelScope ks(branch_name(kBwdNames, a.kind), st);
+    tc_bwd_kernel<128><<<grid, 512, smem, st>>>(tm_k, tm_v, tm_q_run, tm_do_run, tm_dq, tm_dqacc, p);
+  } else {
+    NSA_CUDA_OK(func_smem((const void*)tc_bwd_kernel<64>, smem));
+    KernelScope ks(branch_name(kBwdNames, a.kind), st);
+    tc_bwd_kernel<64><<<grid, 512, smem, st>>>(tm_k, tm_v, tm_q_run, tm_do_run, tm_dq, tm_dqacc, p);
+  }
+  NSA_LAUNCH_OK("tc_bwd_kernel");
+  return NSA_OK;
 }
 
 }  // namespace tc
@@ -1748,69 +1836,8 @@ int tc_attn_bwd(const AttnArgs& a, void* ws, size_t ws_bytes, cudaStream_t st) {
     sel_split_blocks_kernel<<<dim3(pl.n_ktiles, a.B * a.Hkv), 256, 0, st>>>(p.plan.offsets, p.dk_acc, p.dv_acc, p.dk, p.dv,
                                                                         pl.n_ktiles, pl.nq, a.Lk, a.D, 0);
   }
-  CUtensorMap tm_k, tm_v, tm_q, tm_do;
-  int rc = make_map(&tm_k, a.k, a.D, a.Lk, a.B * a.Hkv, kKeys, 1);
-  if (rc == NSA_OK) rc = make_map(&tm_v, a.v, a.D, a.Lk, a.B * a.Hkv, kKeys, 1);
-  if (rc == NSA_OK) rc = p.merged ? make_map_query_both_slabs(&tm_q, a.q, a.T, a.B * a.Hq, G)
-                                  : make_map_query_rows(&tm_q, a.q, a.D, a.T, a.B * a.Hq, G);
-  if (rc == NSA_OK) rc = p.merged ? make_map_query_both_slabs(&tm_do, a.d_o, a.T, a.B * a.Hq, G)
-                                  : make_map_query_rows(&tm_do, a.d_o, a.D, a.T, a.B * a.Hq, G);
-  CUtensorMap tm_q_run, tm_do_run;
-  if (rc == NSA_OK) rc = make_map_query_rows(&tm_q_run, a.q, a.D, a.T, a.B * a.Hq, G, pl.nq);
-  if (rc == NSA_OK) rc = make_map_query_rows(&tm_do_run, a.d_o, a.D, a.T, a.B * a.Hq, G, pl.nq);
-  CUtensorMap tm_dq, tm_dqacc;
-  if (rc == NSA_OK && p.dq_acc_mode) {
-    rc = make_map_dq_acc(&tm_dqacc, a.dq_acc, a.D, G, (size_t)a.T, (size_t)a.B * a.Hkv, pl.nq);
-    tm_dq = tm_dqacc;        // the partial-tile map is not used in this mode
-  } else if (rc == NSA_OK) {
-    rc = a.kind == 2 ? make_map_partial(&tm_dq, p.dq_part, a.D, G, 1, pl.cap_pairs ? pl.cap_pairs : 1, 1, pl.nq, a.three_term)
-                     : make_map_partial(&tm_dq, p.dq_part, a.D, G, pl.n_slots, a.T, (size_t)a.B * a.Hkv, pl.nq);
-    tm_dqacc = tm_dq;        // likewise
-  }
+  int rc = bwd_narrow(a, p, pl, roles, st);
   if (rc != NSA_OK) return rc;
-  const size_t smem = bwd_smem_bytes(a.D);
-  dim3 grid(pl.n_ktiles, a.B * a.Hkv, pl.n_splits);
-  if (a.kind == 2)
-    grid = dim3((unsigned)((size_t)a.B * a.Hkv * pl.layout.max_items));
-  if (roles) {
-    KernelScope ks(branch_name(kBwdNames, a.kind), st);
-    grid.x *= (unsigned)pl.csize;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(kB2Threads);
-    cfg.dynamicSmemBytes = a.three_term ? (a.D == 128 ? Bwd2<128, true>::kSmem : Bwd2<64, true>::kSmem)
-                                      : (a.D == 128 ? Bwd2<128, false>::kSmem : Bwd2<64, false>::kSmem);
-    cfg.stream = st;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = (unsigned)pl.csize;
-    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = pl.csize > 1 ? 1 : 0;
-    auto go = [&](auto kernel) -> int {
-      NSA_CUDA_OK(func_smem((const void*)kernel, cfg.dynamicSmemBytes));
-      NSA_CUDA_OK(cudaLaunchKernelEx(&cfg, kernel, tm_k, tm_v, tm_q, tm_do, tm_q_run, tm_do_run, tm_dq, p));
-      return NSA_OK;
-    };
-    if (a.three_term) {
-      if (a.D == 128) rc = pl.csize > 1 ? go(tc_bwd2_kernel<128, true, true>) : go(tc_bwd2_kernel<128, false, true>);
-      else rc = pl.csize > 1 ? go(tc_bwd2_kernel<64, true, true>) : go(tc_bwd2_kernel<64, false, true>);
-    } else if (a.D == 128) {
-      rc = pl.csize > 1 ? go(tc_bwd2_kernel<128, true, false>) : go(tc_bwd2_kernel<128, false, false>);
-    } else {
-      rc = pl.csize > 1 ? go(tc_bwd2_kernel<64, true, false>) : go(tc_bwd2_kernel<64, false, false>);
-    }
-    if (rc != NSA_OK) return rc;
-  } else if (a.D == 128) {
-    NSA_CUDA_OK(func_smem((const void*)tc_bwd_kernel<128>, smem));
-    KernelScope ks(branch_name(kBwdNames, a.kind), st);
-    tc_bwd_kernel<128><<<grid, 512, smem, st>>>(tm_k, tm_v, tm_q_run, tm_do_run, tm_dq, tm_dqacc, p);
-  } else {
-    NSA_CUDA_OK(func_smem((const void*)tc_bwd_kernel<64>, smem));
-    KernelScope ks(branch_name(kBwdNames, a.kind), st);
-    tc_bwd_kernel<64><<<grid, 512, smem, st>>>(tm_k, tm_v, tm_q_run, tm_do_run, tm_dq, tm_dqacc, p);
-  }
-  NSA_LAUNCH_OK("tc_bwd_kernel");
   if (pl.sel_split) {
     KernelScope ks("sel_split_blocks_kernel", st);
     sel_split_blocks_kernel<<<dim3(pl.n_ktiles, a.B * a.Hkv), 256, 0, st>>>(p.plan.offsets, p.dk_acc, p.dv_acc, p.dk, p.dv,
