@@ -26,10 +26,12 @@
 //                accumulator [units][T][G][D] by TMA reduce-add.  Consecutive key tiles hit the same
 //                consecutive query rows at nearby times, so the adds meet in L2 and no partial
 //                buffer exists; the order of the adds, hence the last bits of dq, is not fixed.
+#include <algorithm>
 #include <type_traits>
 
 #include "cluster.cuh"
 #include "sel_row.cuh"
+#include "tc_bwd_wide.cuh"
 #include "tc_common.cuh"
 #include "tc_host.cuh"
 
@@ -1400,6 +1402,7 @@ __global__ void delta_kernel(const __nv_bfloat16* __restrict__ d_o, const __nv_b
 // of query (bh, t) are added in fp32 and rounded once.  A branch whose buffer is null is absent.
 struct Reduce3Args {
   const __nv_bfloat16* part_cmp; int slots_cmp, Lk_cmp, cmp_len, cmp_stride;
+  int shift_win;               // log2 of the keys of a window tile
   const void* part_slc; const int32_t* pair_of_slot; int S;     // fp32 where the kernel is kF32
   const __nv_bfloat16* part_win; int slots_win, window;
   const float* acc;            // fp32 accumulator [units][T][G][D] holding the window + compression part, or null
@@ -1505,7 +1508,7 @@ dq_reduce3_kernel(const Reduce3Args a) {
     }
   }
   if (a.part_win) {
-    const int first = max(0, t - a.window + 1) >> 6, last = t >> 6;
+    const int first = max(0, t - a.window + 1) >> a.shift_win, last = t >> a.shift_win;
     for (int j0 = first; j0 <= last; j0 += kTripWin) {
       long long rows[kTripWin];
 #pragma unroll
@@ -1536,6 +1539,7 @@ dq_reduce3_kernel(const Reduce3Args a) {
 static Reduce3Args reduce_args(const AttnArgs& a, void* dq) {
   Reduce3Args r = {};
   r.slots_cmp = r.slots_win = 1;
+  r.shift_win = 6;
   r.dq = (__nv_bfloat16*)dq;
   r.B = a.B; r.Hq = a.Hq; r.Hkv = a.Hkv; r.T = a.T; r.G = a.Hq / a.Hkv;
   return r;
@@ -1617,6 +1621,7 @@ static const char* const kBwdNames[3] = {"tc_bwd_win", "tc_bwd_cmp", "tc_bwd_slc
 static const char* const kRedNames[3] = {"dq_reduce_win", "dq_reduce_cmp", "dq_reduce_slc"};
 
 struct BwdPlan {
+  bool wide;                 // window: tiles of 128 keys (tc_bwd_wide.cu)
   int n_ktiles, n_slots, nq, n_splits, split_chunk;
   int csize;                 // CTAs that share the row tiles of one key tile
   bool sel_split;            // selection: a key tile that every query lists would be more than one work item
@@ -1631,19 +1636,31 @@ int get_option_merged_boxes();   // api.cu
 int get_option_bwd_kernel();
 namespace tc {
 
+// Window with more tiles of 64 keys than SMs: tiles of 128 (tc_bwd_wide.cu).  A tile of 128 takes 1.5 to 1.7 times as long
+// as one of 64, so it pays where those would need a second wave, and not before: at 32 tiles of 128 keys (64 of 64, in
+// clusters) the window took 45 us for 1024 tokens of 16 heads of 64 and 62 for 2048 of 8 heads of 128, 25 and 33 with tiles
+// of 64; from 128 tiles on it takes 0.65 to 0.7 of their time.  Compression keeps tiles of 64: the gradient of its key
+// pooling's position parameters is the rounding of P and dS, which the products here round in another order.
+static bool use_wide(const AttnArgs& a) {
+  return a.kind == 0 && a.Lk == a.T && !a.dq_acc && get_option_bwd_kernel() == 1 &&
+         (long long)a.B * a.Hkv * ((a.T + kKeys - 1) / kKeys) > sm_count();
+}
+
 static BwdPlan plan_bwd(const AttnArgs& a) {
   BwdPlan pl;
   const int G = a.Hq / a.Hkv;
   pl.nq = kRows / G;
   const size_t units = (size_t)a.B * a.Hkv;
-  pl.n_ktiles = (a.Lk + kKeys - 1) / kKeys;
+  pl.wide = use_wide(a);
+  pl.n_ktiles = (a.Lk + kKeys - 1) / kKeys;        // (the wide kernel has its own)
   size_t part_rows;
   if (a.kind == 2) {
     pl.n_slots = a.S;
     pl.cap_pairs = units * a.T * a.S;
     part_rows = pl.cap_pairs;
   } else {
-    pl.n_slots = a.kind == 0 ? (a.window + kKeys - 2) / kKeys + 1 : pl.n_ktiles;
+    pl.n_slots = a.kind != 0 ? pl.n_ktiles : pl.wide ? (std::min(a.window, a.T) + kWideKeys - 2) / kWideKeys + 1
+                                                     : (a.window + kKeys - 2) / kKeys + 1;
     pl.cap_pairs = 0;
     part_rows = a.dq_acc ? 0 : units * a.T * pl.n_slots;   // accumulator mode: no partial buffer
   }
@@ -1669,7 +1686,7 @@ static BwdPlan plan_bwd(const AttnArgs& a) {
   const int item_rt = a.kind == 2 ? (max_rt < kSelChunkTiles ? max_rt : kSelChunkTiles) : max_rt;
   const long long base = (long long)units * pl.n_ktiles;
   pl.csize = 1;
-  while (a.kind != 1 && !a.dq_acc && pl.csize < 8 && base * pl.csize * 2 <= sm_count() + 20 && item_rt >= 8 * pl.csize) pl.csize *= 2;
+  while (a.kind != 1 && !a.dq_acc && !pl.wide && pl.csize < 8 && base * pl.csize * 2 <= sm_count() + 20 && item_rt >= 8 * pl.csize) pl.csize *= 2;
   // compression: a few key tiles are attended by (almost) every query; they go in chunks of 48 row
   // tiles whose dK / dV meet in fp32 accumulators
   pl.n_splits = 1;
@@ -1836,7 +1853,19 @@ int tc_attn_bwd(const AttnArgs& a, void* ws, size_t ws_bytes, cudaStream_t st) {
     sel_split_blocks_kernel<<<dim3(pl.n_ktiles, a.B * a.Hkv), 256, 0, st>>>(p.plan.offsets, p.dk_acc, p.dv_acc, p.dk, p.dv,
                                                                         pl.n_ktiles, pl.nq, a.Lk, a.D, 0);
   }
-  int rc = bwd_narrow(a, p, pl, roles, st);
+  int rc = NSA_OK;
+  if (pl.wide) {
+    WideArgs w;
+    w.lse = p.lse; w.delta = p.delta; w.row_scale = p.row_scale;
+    w.dk = p.dk; w.dv = p.dv; w.dq_part = (__nv_bfloat16*)p.dq_part;
+    w.status = p.status;
+    w.Hq = a.Hq; w.Hkv = a.Hkv; w.T = a.T; w.G = G; w.nq = pl.nq;
+    w.window = std::min(a.window, a.T); w.n_slots = pl.n_slots;
+    w.scale = p.scale; w.scale_log2 = p.scale_log2;
+    rc = bwd_wide_launch(a, w, branch_name(kBwdNames, a.kind), st);
+  } else {
+    rc = bwd_narrow(a, p, pl, roles, st);
+  }
   if (rc != NSA_OK) return rc;
   if (pl.sel_split) {
     KernelScope ks("sel_split_blocks_kernel", st);
@@ -1857,7 +1886,7 @@ int tc_attn_bwd(const AttnArgs& a, void* ws, size_t ws_bytes, cudaStream_t st) {
   }
   if (!a.dq) return NSA_OK;   // the partials stay in the workspace (or the accumulator) for tc_dq_reduce3
   Reduce3Args r = reduce_args(a, a.dq);
-  if (a.kind == 0) { r.part_win = (const __nv_bfloat16*)p.dq_part; r.slots_win = pl.n_slots; r.window = a.window; }
+  if (a.kind == 0) { r.part_win = (const __nv_bfloat16*)p.dq_part; r.slots_win = pl.n_slots; r.shift_win = pl.wide ? 7 : 6; r.window = a.window; }
   else if (a.kind == 1) {
     r.part_cmp = (const __nv_bfloat16*)p.dq_part; r.slots_cmp = pl.n_slots;
     r.Lk_cmp = a.Lk; r.cmp_len = a.block_size; r.cmp_stride = a.window;
@@ -1893,6 +1922,7 @@ int tc_dq_reduce3(const AttnArgs& base, int Lk_cmp, int cmp_len, int cmp_stride,
     const BwdPlan pl = plan_bwd(a);
     r.part_win = (const __nv_bfloat16*)((const char*)ws_win + pl.off_part);
     r.slots_win = pl.n_slots;
+    r.shift_win = pl.wide ? 7 : 6;
   }
   return reduce_launch(r, base.D, base.three_term, "dq_reduce3", st);
 }
