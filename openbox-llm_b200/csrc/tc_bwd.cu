@@ -1044,7 +1044,9 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
         }
         if (progressed) {
           idle_since = clock64();
-        } else if ((++polls & 0xffu) == 0) {
+          continue;
+        }
+        if ((++polls & 0xffu) == 0) {
           bool leave = *s_abort != 0;
           if (!leave && *(volatile int*)p.status != 0) leave = true;
           if (!leave && clock64() - idle_since > kWaitLimitCycles) { atomicOr(p.status, 2048); leave = true; }
@@ -1108,8 +1110,16 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
       // (gate p)^T dO; dS = scale * gate * p * (dP - delta), the constant factors folded once per row
       const float lse2 = lse_cur * kLog2e - __log2f(gate_cur);
       const float dscale = p.scale, ddelta = delta_cur * p.scale;
-      // every column of this thread's half is attended (the usual case away from the diagonal)?
-      const bool all_cols = lo <= half * 32 && hi >= half * 32 + 31 && groups == 0x3u && !repeats;
+      // the columns of this thread's half that are attended, a bit each: all of them away from the diagonal.  Rows that are
+      // zero in Q and dO (past nq * G of a tile, and selection's past its last query) may count as attending all: two
+      // of them in the last quarter of every tile of three heads had its warps mask every element, 1.7 k cycles a tile
+      // behind the others
+      const int lo_h = min(max(lo - half * 32, 0), 32), hi_h = min(max(hi + 1 - half * 32, 0), 32);
+      uint32_t attended = (hi_h == 32 ? ~0u : (1u << hi_h) - 1u) & ~((lo_h == 32) ? ~0u : (1u << lo_h) - 1u);
+      if (!(groups & 1u)) attended &= 0xffff0000u;
+      if (!(groups & 2u)) attended &= 0x0000ffffu;
+      if (!row_slot_ok || (p.kind == 2 && t_cur < 0)) attended = ~0u;
+      const bool all_cols = attended == ~0u && !repeats;
       float times[2] = {1.f, 1.f};                   // how often the row's list names the blocks of its column groups
       if (kThreeTerm && repeats && t_cur >= 0) {
         const int32_t* list = p.block_idx + ((size_t)bh * p.T + (t_cur & (int)kPairPosMask)) * p.S;
@@ -1149,8 +1159,7 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
             float pv[2], dv[2];
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
-              const int c = half * 32 + c2 * 2 + e;
-              const bool in = (c >= lo) && (c <= hi) && ((groups >> (c2 >> 3)) & 1u);
+              const bool in = (attended >> (c2 * 2 + e)) & 1u;
               float pr = in ? ex2(fmaf(__uint_as_float(rs[c2 * 2 + e]), p.scale_log2, -lse2)) : 0.f;
               if (kThreeTerm) pr *= times[c2 >> 3];
               pv[e] = pr;
