@@ -64,17 +64,16 @@ __device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
 // Bounded wait.  When the limit runs out the kernel raises the device status word, marks the
 // CTA as aborted and every later wait of the CTA returns at once, so the grid drains; other
 // CTAs notice the status word the next time one of their waits is slow.
-// Returns true when the phase completed, false when the wait was given up.  The abort flag is read only where the
-// phase is not there at the first look: while the MMAs fetch operands from shared memory a load of the flag takes some
-// 220 cycles (its bandwidth is theirs first), the look at the barrier 30.
+// Returns true when the phase completed, false when the wait was given up.  The abort flag is read at every 64th look
+// only: while the MMAs fetch operands from shared memory a load of the flag takes some 220 cycles (its bandwidth is
+// theirs first), a look at the barrier 30.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* status,
                                           volatile int* s_abort, int code) {
   if (mbar_try_wait(bar, parity)) return true;
-  if (*s_abort) return false;
   const long long start = clock64();
   uint32_t polls = 0;
   while (!mbar_try_wait(bar, parity)) {
-    if ((++polls & 0xffu) == 0) {
+    if ((++polls & 0x3fu) == 0) {
       if (*s_abort) return false;
       if (*(volatile int*)status != 0) { *s_abort = 1; return false; }
       if (clock64() - start > kWaitLimitCycles) {
