@@ -41,6 +41,8 @@ plan_count_kernel(const int32_t* __restrict__ block_idx, int32_t* __restrict__ c
                   SelPlanHeader* __restrict__ hdr, int T, int S, int block_size, int n_kt, int cw, int n_chunks,
                   int nq_union) {
   extern __shared__ uint32_t bm[];
+  chain_wait();
+  chain_go();
   const int chunk = blockIdx.x, unit = blockIdx.y;
   if (chunk == 0 && unit == 0 && threadIdx.x == 0) { hdr->union_tiles = 0ull; hdr->pairs = 0ull; hdr->repeats = 0ull; }
   const int t0 = chunk * cw * 32, n_q = min(T - t0, cw * 32);
@@ -113,6 +115,8 @@ plan_scan_kernel(int32_t* __restrict__ counts, const int32_t* __restrict__ union
   constexpr int kBatch = NT == 256 ? 8 : 16;  // loads in flight per thread
   __shared__ int warp_sums[32];
   __shared__ int part_sum[NT];
+  chain_wait();
+  chain_go();
   const int unit = blockIdx.x, tid = threadIdx.x;
   int32_t* cnt = counts + (size_t)unit * n_chunks * n_kt;
   int pair_carry = unit * T * S, item_carry = 0;
@@ -231,6 +235,8 @@ plan_fill_kernel(const int32_t* __restrict__ block_idx, const int32_t* __restric
                  int32_t* __restrict__ pairs, int32_t* __restrict__ pair_of_slot, SelPlanHeader* __restrict__ hdr, int T, int S,
                  int block_size, int n_kt, int cw, int n_chunks) {
   extern __shared__ uint32_t bm[];
+  chain_wait();
+  chain_go();
   uint16_t* before = reinterpret_cast<uint16_t*>(bm + n_kt * cw);   // [word][tile]: queries in earlier words
   const int chunk = blockIdx.x, unit = blockIdx.y;
   const int t0 = chunk * cw * 32, n_q = min(T - t0, cw * 32);
@@ -411,18 +417,15 @@ int sel_plan_build(const int32_t* block_idx, void* base, const SelPlanLayout& l,
   NSA_CUDA_OK(match ? func_smem((const void*)plan_fill_kernel<true>, smem + smem / 2)
                     : func_smem((const void*)plan_fill_kernel<false>, smem + smem / 2));
   { KernelScope ks("plan_count_kernel", st);
-    plan_count_kernel<<<grid, kThreads, smem, st>>>(block_idx, counts, unions, p.hdr, T, S, block_size, l.n_ktiles,
-                                                    l.chunk_words, l.n_chunks, nq_union); }
+    NSA_CUDA_OK(launch_chained(plan_count_kernel, grid, kThreads, smem, st, block_idx, counts, unions, p.hdr, T, S, block_size,
+                               l.n_ktiles, l.chunk_words, l.n_chunks, nq_union)); }
   { KernelScope ks("plan_scan_kernel", st);
-    if (l.n_ktiles <= 256) plan_scan_kernel<256><<<units, 256, 0, st>>>(counts, unions, p, T, S, l.n_ktiles, l.n_chunks, nq);
-    else plan_scan_kernel<1024><<<units, 1024, 0, st>>>(counts, unions, p, T, S, l.n_ktiles, l.n_chunks, nq); }
+    const bool small = l.n_ktiles <= 256;
+    NSA_CUDA_OK(launch_chained(small ? plan_scan_kernel<256> : plan_scan_kernel<1024>, units, small ? 256 : 1024, 0, st, counts, unions,
+                               p, T, S, l.n_ktiles, l.n_chunks, nq)); }
   { KernelScope ks("plan_fill_kernel", st);
-    if (match)
-      plan_fill_kernel<true><<<grid, kThreads, smem + smem / 2, st>>>(block_idx, counts, p.pairs, p.pair_of_slot, p.hdr, T, S,
-                                                                      block_size, l.n_ktiles, l.chunk_words, l.n_chunks);
-    else
-      plan_fill_kernel<false><<<grid, kThreads, smem + smem / 2, st>>>(block_idx, counts, p.pairs, p.pair_of_slot, p.hdr, T, S,
-                                                                       block_size, l.n_ktiles, l.chunk_words, l.n_chunks); }
+    NSA_CUDA_OK(launch_chained(match ? plan_fill_kernel<true> : plan_fill_kernel<false>, grid, kThreads, smem + smem / 2, st, block_idx,
+                               counts, p.pairs, p.pair_of_slot, p.hdr, T, S, block_size, l.n_ktiles, l.chunk_words, l.n_chunks)); }
   NSA_LAUNCH_OK("selection plan kernels");
   return NSA_OK;
 }

@@ -160,6 +160,7 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   const int tile_words = p.n_sub * p.nw;
   uint16_t* s_tiles = (uint16_t*)(s_member + (kSel ? p.nb_sel * tile_words : 0));
 
+  if (kSel && p.plan != nullptr) chain_wait();    // the header is read first
   if (kSel && p.plan != nullptr && prefer_pairs(p.plan, p.nq_union, p.force))
     return;   // the block-outer variant serves this call: leave before anything is set up
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -185,6 +186,8 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *s_tmem;
+  if (kSel) chain_wait();
+  else if (kCmp) chain_go();            // the scorer is next
 
   // row tile w of the launch: long rows first, the units of one token range next to each other
   const int units = p.B * p.Hkv;
@@ -659,7 +662,8 @@ static int launch_fwd(const AttnArgs& a, const SelPlanHeader* plan, int force, c
   KernelScope ks(branch_name(kFwdNames, a.kind), st);
   auto go = [&](auto kernel) -> int {
     NSA_CUDA_OK(func_smem((const void*)kernel, smem));
-    kernel<<<grid, kFwdThreads, smem, st>>>(tm_q, tm_k, tm_v, p);
+    if (a.kind == 2) NSA_CUDA_OK(launch_chained(kernel, grid, kFwdThreads, smem, st, tm_q, tm_k, tm_v, p));   // behind scorer or plan
+    else kernel<<<grid, kFwdThreads, smem, st>>>(tm_q, tm_k, tm_v, p);
     return NSA_OK;
   };
   if (a.three_term)

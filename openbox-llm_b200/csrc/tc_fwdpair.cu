@@ -35,6 +35,7 @@ sel_combine_kernel(const __nv_bfloat16* __restrict__ o_part, const float* __rest
                    const int32_t* __restrict__ pair_of_slot, const SelPlanHeader* __restrict__ hdr,
                    __nv_bfloat16* __restrict__ o, float* __restrict__ lse, const GateBlend gb, int B, int Hq, int Hkv, int T,
                    int G, int S, int nq_union, int force) {
+  chain_wait();
   if (!prefer_pairs(hdr, nq_union, force)) return;
   constexpr int kVec = D / 8;
   const int groups = G / H;
@@ -224,17 +225,18 @@ int tc_sel_fwd(const AttnArgs& a, void* ws, size_t ws_bytes, cudaStream_t st) {
   const int H = G % 2 == 0 ? 2 : 1;       // two heads: their statistics are one 16-byte load, aligned for even G
   const size_t nthreads = (size_t)a.B * a.Hkv * a.T * (G / H) * (a.D / 8);
   const unsigned cgrid = (unsigned)((nthreads + 255) / 256);
-  auto combine = [&](auto kernel) {
+  auto combine = [&](auto kernel) -> int {
     KernelScope ks("sel_combine_kernel", st);
-    kernel<<<cgrid, 256, 0, st>>>((const __nv_bfloat16*)(base + pl.off_part), (const float*)(base + pl.off_ml),
-                                  plan.pair_of_slot, plan.hdr, (__nv_bfloat16*)(a.g_out ? a.o_kept : a.o), a.lse,
-                                  GateBlend{(const __nv_bfloat16*)a.g_cmp, (const __nv_bfloat16*)a.g_win,
-                                            (const __nv_bfloat16*)a.g_logits, (__nv_bfloat16*)a.g_out},
-                                  a.B, a.Hq, a.Hkv, a.T, G, a.S,
-                                  nq_union, force);
+    NSA_CUDA_OK(launch_chained(kernel, cgrid, 256, 0, st, (const __nv_bfloat16*)(base + pl.off_part), (const float*)(base + pl.off_ml),
+                               plan.pair_of_slot, plan.hdr, (__nv_bfloat16*)(a.g_out ? a.o_kept : a.o), a.lse,
+                               GateBlend{(const __nv_bfloat16*)a.g_cmp, (const __nv_bfloat16*)a.g_win,
+                                         (const __nv_bfloat16*)a.g_logits, (__nv_bfloat16*)a.g_out},
+                               a.B, a.Hq, a.Hkv, a.T, G, a.S, nq_union, force));
+    return NSA_OK;
   };
-  if (a.D == 128) { if (H == 2) combine(sel_combine_kernel<128, 2>); else combine(sel_combine_kernel<128, 1>); }
-  else { if (H == 2) combine(sel_combine_kernel<64, 2>); else combine(sel_combine_kernel<64, 1>); }
+  if (a.D == 128) rc = H == 2 ? combine(sel_combine_kernel<128, 2>) : combine(sel_combine_kernel<128, 1>);
+  else rc = H == 2 ? combine(sel_combine_kernel<64, 2>) : combine(sel_combine_kernel<64, 1>);
+  if (rc != NSA_OK) return rc;
   NSA_LAUNCH_OK("sel_combine_kernel");
   return NSA_OK;
 }

@@ -43,6 +43,7 @@ tc_score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   constexpr uint32_t kIdescQK = idesc_bf16(128, kKeys, 0, 0);
 
   extern __shared__ uint8_t smem_raw[];
+  chain_wait();
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);   // pointer arithmetic keeps the shared address space
   uint8_t* sQ = smem;
   uint8_t* sK = sQ + kQBytes;                        // 2 stages
@@ -112,6 +113,7 @@ tc_score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     __syncthreads();
     tc_fence_after();
     tmem = *s_tmem;
+    chain_go();
     const uint32_t lane_base = tmem + ((uint32_t)(warp * 32) << 16);
     const float lse2 = row_ok ? __ldg(p.lse + (size_t)(b * p.Hq + hkv * p.G + g) * p.T + t) * kLog2e : 0.f;
 
@@ -316,6 +318,7 @@ tc_score_lanes_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   constexpr int kList = 16;
 
   extern __shared__ uint8_t smem_raw[];
+  chain_wait();
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   uint8_t* sQ = smem;
   uint8_t* sK = sQ + kQBytes;                        // 2 stages
@@ -370,6 +373,7 @@ tc_score_lanes_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *s_tmem;
+    chain_go();
     bool aborted = false;
     int k_loaded = 0, k_seen = 0;   // thread 0: K tiles whose load was issued / whose arrival was seen
     bool q_seen = false;
@@ -590,10 +594,10 @@ static int launch_score_lanes(const void* q, const void* k_cmp, const NsaDims& d
   KernelScope ks("tc_score_topn", st);
   if (p.r == 1 && p.overlap == 0) {
     NSA_CUDA_OK(func_smem((const void*)tc_score_lanes_kernel<D, GP, true>, smem));
-    tc_score_lanes_kernel<D, GP, true><<<dim3(p.n_qtiles, d.B * d.Hkv), 128, smem, st>>>(tm_q, tm_k, p);
+    NSA_CUDA_OK(launch_chained(tc_score_lanes_kernel<D, GP, true>, dim3(p.n_qtiles, d.B * d.Hkv), 128, smem, st, tm_q, tm_k, p));
   } else {
     NSA_CUDA_OK(func_smem((const void*)tc_score_lanes_kernel<D, GP, false>, smem));
-    tc_score_lanes_kernel<D, GP, false><<<dim3(p.n_qtiles, d.B * d.Hkv), 128, smem, st>>>(tm_q, tm_k, p);
+    NSA_CUDA_OK(launch_chained(tc_score_lanes_kernel<D, GP, false>, dim3(p.n_qtiles, d.B * d.Hkv), 128, smem, st, tm_q, tm_k, p));
   }
   return NSA_OK;
 }
@@ -650,11 +654,11 @@ int tc_topn(const void* q, const void* k_cmp, const float* lse, int32_t* block_i
   if (d.D == 128) {
     NSA_CUDA_OK(func_smem((const void*)tc_score_kernel<128>, smem));
     KernelScope ks("tc_score_topn", st);
-    tc_score_kernel<128><<<grid, 128, smem, st>>>(tm_q, tm_k, p);
+    NSA_CUDA_OK(launch_chained(tc_score_kernel<128>, grid, 128, smem, st, tm_q, tm_k, p));
   } else {
     NSA_CUDA_OK(func_smem((const void*)tc_score_kernel<64>, smem));
     KernelScope ks("tc_score_topn", st);
-    tc_score_kernel<64><<<grid, 128, smem, st>>>(tm_q, tm_k, p);
+    NSA_CUDA_OK(launch_chained(tc_score_kernel<64>, grid, 128, smem, st, tm_q, tm_k, p));
   }
   NSA_LAUNCH_OK("tc_score_kernel");
   return NSA_OK;
