@@ -108,6 +108,15 @@ struct KernelScope {
 // 91 against 86.3), both beside the window's kernel.
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void chain_go() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// What the kernel ahead writes is read by plain loads, which stay behind the wait: the read-only path (__ldg, a const
+// __restrict__ argument) takes its data not to change while the kernel is on the GPU, which includes the time before.
+__device__ __forceinline__ int32_t ld_plain(const int32_t* p) { int32_t v; asm volatile("ld.global.s32 %0, [%1];" : "=r"(v) : "l"(p)); return v; }
+__device__ __forceinline__ float ld_plain(const float* p) { float v; asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p)); return v; }
+__device__ __forceinline__ unsigned long long ld_plain(const unsigned long long* p) {
+  unsigned long long v;
+  asm volatile("ld.global.u64 %0, [%1];" : "=l"(v) : "l"(p));
+  return v;
+}
 template <typename... P, typename... A>
 inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, const A&... args) {
   cudaLaunchAttribute attr;

@@ -22,14 +22,14 @@ __device__ __forceinline__ int tile_of(int blk, int t, int block_size) {
 
 // Bitmap words are laid out [word][tile]: the entries a warp marks together name different tiles of
 // one or two queries, so they fall into different banks.
-__device__ __forceinline__ void mark_chunk(const int32_t* __restrict__ idx, uint32_t* bm, int t0, int n_q, int S,
+__device__ __forceinline__ void mark_chunk(const int32_t* idx, uint32_t* bm, int t0, int n_q, int S,
                                            int block_size, int n_kt, int cw) {
   for (int i = threadIdx.x; i < n_kt * cw; i += blockDim.x) bm[i] = 0u;
   __syncthreads();
 #pragma unroll 4
   for (int e = threadIdx.x; e < n_q * S; e += blockDim.x) {
     const int ql = e / S;
-    const int j = tile_of(__ldg(idx + e), t0 + ql, block_size);
+    const int j = tile_of(ld_plain(idx + e), t0 + ql, block_size);
     if (j >= 0) atomicOr(&bm[(ql >> 5) * n_kt + j], 1u << (ql & 31));
   }
   __syncthreads();
@@ -37,7 +37,7 @@ __device__ __forceinline__ void mark_chunk(const int32_t* __restrict__ idx, uint
 
 // counts[unit][chunk][tile] and, per CTA, the distinct (query tile, key tile) pairs
 __global__ void __launch_bounds__(kThreads)
-plan_count_kernel(const int32_t* __restrict__ block_idx, int32_t* __restrict__ counts, int32_t* __restrict__ unions,
+plan_count_kernel(const int32_t* block_idx, int32_t* __restrict__ counts, int32_t* __restrict__ unions,
                   SelPlanHeader* __restrict__ hdr, int T, int S, int block_size, int n_kt, int cw, int n_chunks,
                   int nq_union) {
   extern __shared__ uint32_t bm[];
@@ -110,7 +110,7 @@ __device__ __forceinline__ int block_scan(int v, int* warp_sums, int* total) {
 // at most 48 registers find room beside two CTAs of the window kernel on an SM; 1024 wait until they are done.
 template <int NT>
 __global__ void __launch_bounds__(NT, NT == 256 ? 5 : 1)
-plan_scan_kernel(int32_t* __restrict__ counts, const int32_t* __restrict__ unions, SelPlan p, int T, int S,
+plan_scan_kernel(int32_t* __restrict__ counts, const int32_t* unions, SelPlan p, int T, int S,
                  int n_kt, int n_chunks, int nq) {
   constexpr int kBatch = NT == 256 ? 8 : 16;  // loads in flight per thread
   __shared__ int warp_sums[32];
@@ -189,7 +189,7 @@ plan_scan_kernel(int32_t* __restrict__ counts, const int32_t* __restrict__ union
 // kMatch: a query's S entries sit in one warp (S divides 32), so the entries of one query that
 // name the same tile find one another by a warp match instead of reading the list again.
 template <bool kMatch>
-__device__ __forceinline__ void fill_chunk(const int32_t* __restrict__ idx, const uint32_t* bm, const uint16_t* before,
+__device__ __forceinline__ void fill_chunk(const int32_t* idx, const uint32_t* bm, const uint16_t* before,
                                            const int32_t* st, int32_t* __restrict__ pairs, int32_t* __restrict__ pos,
                                            SelPlanHeader* __restrict__ hdr, int t0, int n_q, int S, int block_size, int n_kt) {
   const uint32_t one = (1u << (block_size >> 4)) - 1u;              // column groups of one block
@@ -198,7 +198,7 @@ __device__ __forceinline__ void fill_chunk(const int32_t* __restrict__ idx, cons
     const int e = e0 + threadIdx.x;
     const bool in = e < n_e;
     const int ql = in ? e / S : 0, t = t0 + ql, slot = e - ql * S;
-    const int blk = in ? __ldg(idx + e) : -1;
+    const int blk = in ? ld_plain(idx + e) : -1;
     const int j = tile_of(blk, t, block_size);
     uint32_t groups = j < 0 ? 0u : one << ((blk * block_size - j * kKeysPerTile) >> 4);
     bool dup = false;
@@ -212,7 +212,7 @@ __device__ __forceinline__ void fill_chunk(const int32_t* __restrict__ idx, cons
     } else if (j >= 0) {
       const int32_t* row = idx + ql * S;
       for (int s = 0; s < S; ++s) {
-        const int b2 = __ldg(row + s);
+        const int b2 = ld_plain(row + s);
         if (tile_of(b2, t, block_size) != j) continue;
         dup |= s < slot;
         if (block_size < kKeysPerTile && s < slot && b2 == blk) hdr->repeats = 1ull;
@@ -231,7 +231,7 @@ __device__ __forceinline__ void fill_chunk(const int32_t* __restrict__ idx, cons
 
 template <bool kMatch>
 __global__ void __launch_bounds__(kThreads)
-plan_fill_kernel(const int32_t* __restrict__ block_idx, const int32_t* __restrict__ starts,
+plan_fill_kernel(const int32_t* block_idx, const int32_t* starts,
                  int32_t* __restrict__ pairs, int32_t* __restrict__ pair_of_slot, SelPlanHeader* __restrict__ hdr, int T, int S,
                  int block_size, int n_kt, int cw, int n_chunks) {
   extern __shared__ uint32_t bm[];
@@ -264,7 +264,7 @@ constexpr int kClusterChunk = 256;            // queries
 constexpr int kClusterThreads = 1024;
 template <bool kMatch>
 __global__ void __launch_bounds__(kClusterThreads)
-plan_cluster_kernel(const int32_t* __restrict__ block_idx, SelPlan p, int T, int S, int block_size, int n_kt, int cw, int nq,
+plan_cluster_kernel(const int32_t* block_idx, SelPlan p, int T, int S, int block_size, int n_kt, int cw, int nq,
                     int nq_union) {
   extern __shared__ uint32_t bm[];
   int32_t* cnt = reinterpret_cast<int32_t*>(bm + n_kt * cw);         // [n_kt] pairs of this chunk

@@ -224,7 +224,7 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     const int n_entries = (t_last - t0 + 1) * p.S;
     for (int e = tid; e < n_entries; e += kFwdThreads) {
       const int q_local = e / p.S;
-      const int blk = __ldg(idx + e);
+      const int blk = ld_plain(idx + e);
       // list block blk = part blk % n_sub of key tile blk / n_sub
       if (blk >= 0 && (long long)blk * p.block_size <= t0 + q_local) {
         const uint32_t was = atomicOr(&s_member[blk * p.nw + (q_local >> 5)], 1u << (q_local & 31));

@@ -367,7 +367,7 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 // take the same time where (query tile, key tile) pairs x nq are 3.0 to 4.6 times the pairs.
 __device__ __forceinline__ bool prefer_pairs(const SelPlanHeader* hdr, int nq, int force) {
   if (force) return force == 2;
-  return 2ull * __ldg(&hdr->union_tiles) * (unsigned long long)nq > 7ull * __ldg(&hdr->pairs);
+  return 2ull * ld_plain(&hdr->union_tiles) * (unsigned long long)nq > 7ull * ld_plain(&hdr->pairs);
 }
 
 // byte offset of element (row, col) inside a 128B-swizzled slab sequence; col in elements

@@ -31,9 +31,9 @@ struct GateBlend {
 };
 template <int D, int H>
 __global__ void __launch_bounds__(256, 3)
-sel_combine_kernel(const __nv_bfloat16* __restrict__ o_part, const float* __restrict__ ml,
-                   const int32_t* __restrict__ pair_of_slot, const SelPlanHeader* __restrict__ hdr,
-                   __nv_bfloat16* __restrict__ o, float* __restrict__ lse, const GateBlend gb, int B, int Hq, int Hkv, int T,
+sel_combine_kernel(const __nv_bfloat16* o_part, const float* ml,
+                   const int32_t* pair_of_slot, const SelPlanHeader* hdr,
+                   __nv_bfloat16* o, float* lse, const GateBlend gb, int B, int Hq, int Hkv, int T,
                    int G, int S, int nq_union, int force) {
   chain_wait();
   if (!prefer_pairs(hdr, nq_union, force)) return;
@@ -59,7 +59,7 @@ sel_combine_kernel(const __nv_bfloat16* __restrict__ o_part, const float* __rest
   for (int s0 = 0; s0 < S; s0 += 4) {
     int pr[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) pr[j] = s0 + j < S ? __ldg(ps + s0 + j) : -1;
+    for (int j = 0; j < 4; ++j) pr[j] = s0 + j < S ? ld_plain(ps + s0 + j) : -1;
     float m[H][4], l[H][4];
     uint4 u[H][4];
 #pragma unroll

@@ -115,7 +115,7 @@ tc_score_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     tmem = *s_tmem;
     chain_go();
     const uint32_t lane_base = tmem + ((uint32_t)(warp * 32) << 16);
-    const float lse2 = row_ok ? __ldg(p.lse + (size_t)(b * p.Hq + hkv * p.G + g) * p.T + t) * kLog2e : 0.f;
+    const float lse2 = row_ok ? ld_plain(p.lse + (size_t)(b * p.Hq + hkv * p.G + g) * p.T + t) * kLog2e : 0.f;
 
     auto load_k = [&](int i) {
       uint64_t* bar = bar_k + (i & 1);
@@ -378,7 +378,7 @@ tc_score_lanes_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     int k_loaded = 0, k_seen = 0;   // thread 0: K tiles whose load was issued / whose arrival was seen
     bool q_seen = false;
     const uint32_t lane_base = tmem + ((uint32_t)(warp * 32) << 16);
-    const float lse2 = row_ok ? __ldg(p.lse + (size_t)(b * p.Hq + hkv * p.G + g) * p.T + t) * kLog2e : 0.f;
+    const float lse2 = row_ok ? ld_plain(p.lse + (size_t)(b * p.Hq + hkv * p.G + g) * p.T + t) * kLog2e : 0.f;
     const int n_vis = t < p.T ? cmp_visible(t, p.block_size, p.stride, p.n_blk) : 0;   // summaries query t sees
     const int my_cur = t / p.sel_block;              // selection block that holds t
     float carry = 0.f;                               // last summary of the previous tile (overlap)
