@@ -101,8 +101,8 @@ struct KernelScope {
 // behind it.  A kernel that allocates tensor memory calls chain_go after that: the next one's CTAs take theirs
 // from the same SMs.
 // Measured (us per call, one after the other -> chained): forward of the operator at T = 512 44.8 -> 39.5, at
-// T = 1024 53.1 -> 48.1, selection at T = 8192 forward and backward 362 -> 350, three branches over given lists
-// at T = 4096 94 -> 88.8 (alone in a graph, where the launches cost nothing, 80 -> 84).
+// T = 1024 53.1 -> 48.1, selection at T = 8192 forward and backward 362 -> 339 (350 with the backward's kernels
+// one after the other), three branches over given lists at T = 4096 94 -> 88.8 (alone in a graph, where the launches cost nothing, 80 -> 84).
 // Plain launches stay where an early CTA takes a place that another stream's kernel would fill: the block-outer
 // selection kernel (chained 98.6 where it is 89.3 plain) and the attention over pooled keys (T = 3000
 // 91 against 86.3), both beside the window's kernel.

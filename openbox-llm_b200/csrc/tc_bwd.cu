@@ -726,6 +726,7 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
   constexpr uint32_t kIdescDQ = idesc_bf16(128, D, 0, 1);
 
   extern __shared__ uint8_t smem_raw[];
+  chain_wait();
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   uint8_t* sK = smem;
   uint8_t* sV = sK + kKVBytes;
@@ -772,8 +773,8 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
     t_lo = key0 * p.window + p.block_size - 1;       // first query that sees summary key0 (window: the stride)
     n_q = p.T - t_lo;
   } else {
-    pair_base = __ldg(p.plan.offsets + (size_t)bh * (p.n_ktiles + 1) + j);
-    n_q = __ldg(p.plan.offsets + (size_t)bh * (p.n_ktiles + 1) + j + 1) - pair_base;
+    pair_base = ld_plain(p.plan.offsets + (size_t)bh * (p.n_ktiles + 1) + j);
+    n_q = ld_plain(p.plan.offsets + (size_t)bh * (p.n_ktiles + 1) + j + 1) - pair_base;
   }
   n_q = max(n_q, 0);
   const int n_rt_all = (n_q + p.nq - 1) / p.nq;
@@ -883,7 +884,7 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
     auto box_of = [&](int r) -> int { return (r * 32 + lane) * kProducers + pw; };
     auto tq_of = [&](int k, int o) -> int {          // pair of box o of tile k (none: past T, zeros)
       const int qi = (rt_begin + k) * p.nq + o / per_q;
-      return (o < n_ops && qi < n_q) ? ldg_s32_now(p.plan.pairs + pair_base + qi) : p.T;
+      return (o < n_ops && qi < n_q) ? ld_plain(p.plan.pairs + pair_base + qi) : p.T;
     };
     int tq[kRounds];
     if (p.kind == 2) {
@@ -1069,7 +1070,7 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
     auto row_query = [&](int k) -> int {
       const int qi = (rt_begin + k) * p.nq + ql;
       if (!row_slot_ok || qi >= n_q) return -1;
-      if (p.kind == 2) return ldg_s32_now(p.plan.pairs + pair_base + qi);
+      if (p.kind == 2) return ld_plain(p.plan.pairs + pair_base + qi);
       return t_lo + qi;
     };
     auto row_index = [&](int t) -> size_t { return (size_t)(b * p.Hq + head) * p.T + (t & (int)kPairPosMask); };
@@ -1077,11 +1078,11 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
     int t_nxt = n_tiles > 1 ? row_query(1) : -1;
     float lse_cur = 0.f, delta_cur = 0.f, gate_cur = 1.f;
     if (t_cur >= 0) {
-      lse_cur = __ldg(p.lse + row_index(t_cur));
-      delta_cur = __ldg(p.delta + row_index(t_cur));
-      if (p.row_scale) gate_cur = __ldg(p.row_scale + row_index(t_cur));
+      lse_cur = ld_plain(p.lse + row_index(t_cur));
+      delta_cur = ld_plain(p.delta + row_index(t_cur));
+      if (p.row_scale) gate_cur = ld_plain(p.row_scale + row_index(t_cur));
     }
-    const bool repeats = kThreeTerm && __ldg(&p.plan.hdr->repeats) != 0ull;
+    const bool repeats = kThreeTerm && ld_plain(&p.plan.hdr->repeats) != 0ull;
     for (int k = 0; k < n_tiles; ++k) {
       uint8_t* sP = sPds + (k % kSets) * L::kSetBytes;
       uint8_t* sDS = sP + kPBytes;
@@ -1089,9 +1090,9 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
       const int t_nn = k + 2 < n_tiles ? row_query(k + 2) : -1;
       float lse_nxt = 0.f, delta_nxt = 0.f, gate_nxt = 1.f;
       if (t_nxt >= 0) {
-        lse_nxt = ldg_f32_now(p.lse + row_index(t_nxt));
-        delta_nxt = ldg_f32_now(p.delta + row_index(t_nxt));
-        if (p.row_scale) gate_nxt = ldg_f32_now(p.row_scale + row_index(t_nxt));
+        lse_nxt = ld_plain(p.lse + row_index(t_nxt));
+        delta_nxt = ld_plain(p.delta + row_index(t_nxt));
+        if (p.row_scale) gate_nxt = ld_plain(p.row_scale + row_index(t_nxt));
       }
       int lo = 0, hi = -1;                           // valid key columns of this row: one range [lo, hi]
       uint32_t groups = 0x3u;                        // and, for selection, the 16-column groups of this thread's half
@@ -1232,10 +1233,10 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
 #pragma unroll
           for (int e = 0; e < 32; ++e) z = fmaf(__uint_as_float(r32[e]), 0.f, z);
           if (z != 0.f && row_slot_ok && qi < n_q) {
-            const int head = hkv * p.G + g, pair = __ldg(p.plan.pairs + pair_base + qi);
+            const int head = hkv * p.G + g, pair = ld_plain(p.plan.pairs + pair_base + qi);
             const size_t at = (size_t)(b * p.Hq + head) * p.T + (pair & (int)kPairPosMask);
-            const float lse2 = __ldg(p.lse + at) * kLog2e - (p.row_scale ? __log2f(__ldg(p.row_scale + at)) : 0.f);
-            const float ddelta = __ldg(p.delta + at) * p.scale;
+            const float lse2 = ld_plain(p.lse + at) * kLog2e - (p.row_scale ? __log2f(ld_plain(p.row_scale + at)) : 0.f);
+            const float ddelta = ld_plain(p.delta + at) * p.scale;
             if (lse2 == lse2 && ddelta == ddelta) {      // (NaN statistics: NaN in every column, here as there)
               float again[32];
               sel_row_dq<D>(p, again, bh, head, pair, key0, col0);
@@ -1387,15 +1388,17 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
 // delta[b,h,t] = sum_d dO * O (fp32), D / 8 lanes to a row, one 16-byte vector of each: bound by the pass over both (16
 // heads x 8192 rows of 64: 6 us, 18 with a warp to a row).
 template <int D>
-__global__ void delta_kernel(const __nv_bfloat16* __restrict__ d_o, const __nv_bfloat16* __restrict__ o,
-                             float* __restrict__ delta, size_t rows, bool vec) {
+__global__ void delta_kernel(const __nv_bfloat16* d_o, const __nv_bfloat16* o,
+                             float* delta, size_t rows, bool vec) {
+  chain_wait();
+  chain_go();
   constexpr int kLanes = D / 8;
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x, row = i / kLanes;
   float s = 0.f;
   if (row < rows && !vec) {                          // tensors off a 16-byte boundary
     for (int e = 0; e < 8; ++e) s = fmaf(to_float(d_o[i * 8 + e]), to_float(o[i * 8 + e]), s);
   } else if (row < rows) {
-    const uint4 x = __ldg(reinterpret_cast<const uint4*>(d_o) + i), y = __ldg(reinterpret_cast<const uint4*>(o) + i);
+    const uint4 x = reinterpret_cast<const uint4*>(d_o)[i], y = reinterpret_cast<const uint4*>(o)[i];
     const uint32_t a[4] = {x.x, x.y, x.z, x.w}, c[4] = {y.x, y.y, y.z, y.w};
 #pragma unroll
     for (int e = 0; e < 4; ++e)
@@ -1426,6 +1429,7 @@ struct Reduce3Args {
 template <int D, int HG, bool kF32>
 __global__ void __launch_bounds__(256, 3)
 dq_reduce3_kernel(const Reduce3Args a) {
+  chain_wait();
   constexpr int kVec = D / 8;
   const int Gp = a.G / HG;                               // head groups per query
   const size_t gid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1479,7 +1483,7 @@ dq_reduce3_kernel(const Reduce3Args a) {
 #pragma unroll
     for (int h = 0; h < HG; ++h) {
       const float4* src = reinterpret_cast<const float4*>(a.acc + (size_t)qrow * row_elems + in_row + h * head_step);
-      const float4 lo = __ldg(src), hi = __ldg(src + 1);
+      const float4 lo = src[0], hi = src[1];
       acc[h][0] = lo.x; acc[h][1] = lo.y; acc[h][2] = lo.z; acc[h][3] = lo.w;
       acc[h][4] = hi.x; acc[h][5] = hi.y; acc[h][6] = hi.z; acc[h][7] = hi.w;
     }
@@ -1490,7 +1494,7 @@ dq_reduce3_kernel(const Reduce3Args a) {
     for (int s0 = 0; s0 < a.S; s0 += kTrip) {
       long long rows[kTrip];
 #pragma unroll
-      for (int k = 0; k < kTrip; ++k) rows[k] = s0 + k < a.S ? (long long)__ldg(ps + s0 + k) : -1;
+      for (int k = 0; k < kTrip; ++k) rows[k] = s0 + k < a.S ? (long long)ld_plain(ps + s0 + k) : -1;
       if (!kF32) {
         add_rows((const __nv_bfloat16*)a.part_slc, rows);
         continue;
@@ -1561,16 +1565,15 @@ static int reduce_launch(const Reduce3Args& r, int D, bool f32, const char* name
   if (nthreads == 0) return NSA_OK;
   const unsigned grid = (unsigned)((nthreads + 255) / 256);
   KernelScope ks(name, st);
-  auto go = [&](auto kernel) { kernel<<<grid, 256, 0, st>>>(r); };
-  auto by_heads = [&](auto f32) {
+  auto go = [&](auto kernel) -> int { NSA_CUDA_OK(launch_chained(kernel, grid, 256, 0, st, r)); return NSA_OK; };
+  auto by_heads = [&](auto f32) -> int {
     constexpr bool kF32 = decltype(f32)::value;
-    if (D == 128) {
-      if (hg == 2) go(dq_reduce3_kernel<128, 2, kF32>); else if (hg == 3) go(dq_reduce3_kernel<128, 3, kF32>); else go(dq_reduce3_kernel<128, 1, kF32>);
-    } else {
-      if (hg == 2) go(dq_reduce3_kernel<64, 2, kF32>); else if (hg == 3) go(dq_reduce3_kernel<64, 3, kF32>); else go(dq_reduce3_kernel<64, 1, kF32>);
-    }
+    if (D == 128)
+      return hg == 2 ? go(dq_reduce3_kernel<128, 2, kF32>) : hg == 3 ? go(dq_reduce3_kernel<128, 3, kF32>) : go(dq_reduce3_kernel<128, 1, kF32>);
+    return hg == 2 ? go(dq_reduce3_kernel<64, 2, kF32>) : hg == 3 ? go(dq_reduce3_kernel<64, 3, kF32>) : go(dq_reduce3_kernel<64, 1, kF32>);
   };
-  if (f32) by_heads(std::true_type()); else by_heads(std::false_type());
+  const int rc = f32 ? by_heads(std::true_type()) : by_heads(std::false_type());
+  if (rc != NSA_OK) return rc;
   NSA_LAUNCH_OK("dq_reduce3_kernel");
   return NSA_OK;
 }
@@ -1578,10 +1581,12 @@ static int reduce_launch(const Reduce3Args& r, int D, bool f32, const char* name
 // Selection blocks whose row tiles were split over several work items collect dK / dV in the fp32
 // accumulators: this kernel clears the accumulator rows of those blocks before the backward
 // kernel (finalize = 0) and turns them into the bf16 outputs after it (finalize = 1).
-__global__ void sel_split_blocks_kernel(const int32_t* __restrict__ offsets, float* __restrict__ dk_acc,
-                                        float* __restrict__ dv_acc, __nv_bfloat16* __restrict__ dk,
-                                        __nv_bfloat16* __restrict__ dv, int n_ktiles, int nq, int Lk, int D,
+__global__ void sel_split_blocks_kernel(const int32_t* offsets, float* dk_acc,
+                                        float* dv_acc, __nv_bfloat16* dk,
+                                        __nv_bfloat16* dv, int n_ktiles, int nq, int Lk, int D,
                                         int finalize) {
+  chain_wait();
+  chain_go();
   const int j = blockIdx.x, bh = blockIdx.y;
   const int n_q = offsets[(size_t)bh * (n_ktiles + 1) + j + 1] - offsets[(size_t)bh * (n_ktiles + 1) + j];
   const int n_rt = (n_q + nq - 1) / nq;
@@ -1750,12 +1755,18 @@ static int bwd_narrow(const AttnArgs& a, const BwdArgs& p, const BwdPlan& pl, bo
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.stream = st;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = (unsigned)pl.csize;
-    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = pl.csize > 1 ? 1 : 0;
+    cudaLaunchAttribute attr[2];
+    cfg.attrs = attr;
+    if (pl.csize > 1) {
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = (unsigned)pl.csize;
+      attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+      cfg.numAttrs = 1;
+    }
+    if (a.kind == 2 && !a.row_dot) {       // a call of its own: the short kernels before it, and no other branch beside it
+      attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
     auto go = [&](auto d, auto three_term, auto gather) -> int {
       constexpr int D = decltype(d)::value;
       constexpr bool kThreeTerm = decltype(three_term)::value, kGather = decltype(gather)::value;
@@ -1841,8 +1852,8 @@ int tc_attn_bwd(const AttnArgs& a, void* ws, size_t ws_bytes, cudaStream_t st) {
     KernelScope ks("delta_kernel", st);
     const unsigned dgrid = (unsigned)((rows * (a.D / 8) + 255) / 256);
     const auto *d_o = (const __nv_bfloat16*)a.d_o, *o = (const __nv_bfloat16*)a.o;
-    if (a.D == 128) delta_kernel<128><<<dgrid, 256, 0, st>>>(d_o, o, (float*)(base + pl.off_delta), rows, aligned16(d_o, o));
-    else delta_kernel<64><<<dgrid, 256, 0, st>>>(d_o, o, (float*)(base + pl.off_delta), rows, aligned16(d_o, o));
+    NSA_CUDA_OK(launch_chained(a.D == 128 ? delta_kernel<128> : delta_kernel<64>, dgrid, 256, 0, st, d_o, o,
+                               (float*)(base + pl.off_delta), rows, aligned16(d_o, o)));
   }
   NSA_LAUNCH_OK("delta_kernel");
   if (a.kind == 2) {
@@ -1859,8 +1870,8 @@ int tc_attn_bwd(const AttnArgs& a, void* ws, size_t ws_bytes, cudaStream_t st) {
   }
   if (pl.sel_split) {
     KernelScope ks("sel_split_blocks_kernel", st);
-    sel_split_blocks_kernel<<<dim3(pl.n_ktiles, a.B * a.Hkv), 256, 0, st>>>(p.plan.offsets, p.dk_acc, p.dv_acc, p.dk, p.dv,
-                                                                        pl.n_ktiles, pl.nq, a.Lk, a.D, 0);
+    NSA_CUDA_OK(launch_chained(sel_split_blocks_kernel, dim3(pl.n_ktiles, a.B * a.Hkv), 256, 0, st, p.plan.offsets, p.dk_acc, p.dv_acc,
+                               p.dk, p.dv, pl.n_ktiles, pl.nq, a.Lk, a.D, 0));
   }
   int rc = NSA_OK;
   if (pl.wide) {
@@ -1878,8 +1889,8 @@ int tc_attn_bwd(const AttnArgs& a, void* ws, size_t ws_bytes, cudaStream_t st) {
   if (rc != NSA_OK) return rc;
   if (pl.sel_split) {
     KernelScope ks("sel_split_blocks_kernel", st);
-    sel_split_blocks_kernel<<<dim3(pl.n_ktiles, a.B * a.Hkv), 256, 0, st>>>(p.plan.offsets, p.dk_acc, p.dv_acc, p.dk, p.dv,
-                                                                        pl.n_ktiles, pl.nq, a.Lk, a.D, 1);
+    NSA_CUDA_OK(launch_chained(sel_split_blocks_kernel, dim3(pl.n_ktiles, a.B * a.Hkv), 256, 0, st, p.plan.offsets, p.dk_acc, p.dv_acc,
+                               p.dk, p.dv, pl.n_ktiles, pl.nq, a.Lk, a.D, 1));
     NSA_LAUNCH_OK("sel_split_blocks_kernel");
   }
   if (ordered) {
