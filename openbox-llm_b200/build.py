@@ -58,7 +58,7 @@ def _link_ext(r):
     if r.returncode == 0:
         home = os.path.join(os.path.dirname(_torch().__file__), "lib")
         r = subprocess.run(["g++", "-shared", "-o", EXT, EXT_OBJ, "-L" + CSRC, "-l:libnsa_b200.so", "-Wl,-rpath,$ORIGIN",
-                            "-L" + home, "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python", "-ltorch"],
+                            "-L" + home, "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-ltorch"],
                            capture_output=True, text=True)
     if r.returncode != 0:
         sys.stderr.write(r.stdout + r.stderr)

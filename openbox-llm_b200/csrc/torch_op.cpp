@@ -6,6 +6,7 @@
 #include <Python.h>
 
 #include <ATen/ATen.h>
+#include <ATen/cuda/EmptyTensor.h>
 #include <c10/core/impl/LocalDispatchKeySet.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAFunctions.h>
@@ -38,7 +39,17 @@ void check(int rc) {
 }
 
 void* raw_stream(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
-Tensor bytes_like(size_t n, const Tensor& t) { return at::empty({(int64_t)n}, t.options().dtype(at::kByte)); }
+// New memory on the device of `t`, without the way through the dispatcher that at::empty takes: a backward makes 15
+// tensors, and calls of some 1024 tokens last as long as their host work.  Operator forward + backward at
+// T = 1024 199 -> 192 us, the layer's forward on 256 tokens 97 -> 92.
+// Where torch fills new memory itself (deterministic algorithms) or something looks on at the calls, it is at::empty.
+Tensor fresh(at::IntArrayRef sizes, at::ScalarType dtype, const Tensor& t) {
+  if (at::globalContext().deterministicAlgorithms() || c10::impl::TorchDispatchModeTLS::any_modes_set())
+    return at::empty(sizes, t.options().dtype(dtype));
+  return Tensor(at::detail::empty_cuda(sizes, dtype, t.device(), std::nullopt));
+}
+Tensor fresh_like(const Tensor& t) { return fresh(t.sizes(), t.scalar_type(), t); }
+Tensor bytes_like(size_t n, const Tensor& t) { return fresh({(int64_t)n}, at::kByte, t); }
 
 // A dense CUDA tensor of the given type on device `dev` that starts on a 16-byte boundary and that no Python-side
 // dispatch stands behind.
@@ -99,10 +110,10 @@ NsaAttentionTensors pointers(const Tensor* in, const Tensor* comp, const Tensor&
 Tensor op_forward(Call& c, bool need_grad, Tensor* saved) {
   const Tensor& q = c.in[0];
   c.d.need_grad = need_grad;
-  if (!c.d.given_lists) c.block_idx = at::empty({c.d.dims.B, c.d.dims.Hkv, c.d.dims.T, c.d.n_sel}, q.options().dtype(at::kInt));
+  if (!c.d.given_lists) c.block_idx = fresh({c.d.dims.B, c.d.dims.Hkv, c.d.dims.T, c.d.n_sel}, at::kInt, q);
   size_t keep, fwd, bwd;
   check(nsa_attention_sizes(&c.d, &keep, &fwd, &bwd));
-  Tensor out = at::empty(q.sizes(), q.options());
+  Tensor out = fresh_like(q);
   Tensor mem = bytes_like(keep + (need_grad ? 0 : fwd) + 1, q), ws;
   void* ws_ptr = (char*)mem.data_ptr() + keep;
   if (need_grad && fwd) {
@@ -126,7 +137,7 @@ void op_backward(const NsaAttentionDesc& d, const Tensor* in, const Tensor* comp
   void** p[8] = {&t.dq, &t.dkc, &t.dvc, &t.dks, &t.dvs, &t.dkw, &t.dvw, &t.d_gate};
   for (int k = 0; k < 8; ++k) *p[k] = d_in[k].data_ptr();
   for (int k = 0; k < 6 && d.learned; ++k) {
-    d_comp[k] = at::empty_like(comp[k]);
+    d_comp[k] = fresh_like(comp[k]);
     t.d_comp[k] = d_comp[k].data_ptr<float>();
   }
   Tensor ws = bytes_like(bwd + 1, d_out);
@@ -192,7 +203,7 @@ struct OpNode {
     TORCH_CHECK(g[0].scalar_type() == kept[0].scalar_type(), "libnsa_b200: the gradient's type is not the output's");
     const Tensor d_out = aligned(g[0]);
     Tensor d_in[8], d_comp[6];
-    for (int k = 0; k < 8; ++k) d_in[k] = at::empty_like(kept[k]);
+    for (int k = 0; k < 8; ++k) d_in[k] = fresh_like(kept[k]);
     op_backward(d, kept.data(), kept.data() + 10, kept[8], kept[9], d_out, d_in, d_comp);
     for (int k = 0; k < 8; ++k) res[1 + k] = d_in[k];
     for (int k = 8; k < n; ++k) res[1 + k] = d_comp[k - 8];
@@ -229,10 +240,10 @@ struct LayerNode : torch::autograd::Function<LayerNode> {
   // keep: what the backward reads; a GEMM's operand only where the gradient that reads it is asked for
   static Tensor run(Layer& l, bool need_grad, variable_list* keep) {
     const NsaDims& m = l.c.d.dims;
-    const auto opt = l.x.options().dtype(at::kBFloat16);
     const int64_t rows = l.B * l.T, hd = (int64_t)m.Hq * m.D;
-    Tensor xb = l.x.scalar_type() == at::kBFloat16 ? l.x.view({rows, l.dm}) : at::empty({rows, l.dm}, opt);
-    Tensor w = at::empty({l.width, l.dm}, opt), bias = at::empty({l.width}, opt), w_out = at::empty({l.dm, hd}, opt);
+    Tensor xb = l.x.scalar_type() == at::kBFloat16 ? l.x.view({rows, l.dm}) : fresh({rows, l.dm}, at::kBFloat16, l.x);
+    Tensor w = fresh({l.width, l.dm}, at::kBFloat16, l.x), bias = fresh({l.width}, at::kBFloat16, l.x),
+           w_out = fresh({l.dm, hd}, at::kBFloat16, l.x);
     NsaCastSegment s[NSA_MAX_CAST_SEGMENTS];
     int n = 0;
     auto seg = [&](const float* src, void* dst, int64_t e) { s[n++] = NsaCastSegment{src, dst, (size_t)e}; };
@@ -252,15 +263,15 @@ struct LayerNode : torch::autograd::Function<LayerNode> {
     check(nsa_cast_bf16_segments(s, n, raw_stream(l.x)));
     Tensor y = at::addmm(bias, xb, w.t());
     Call& c = l.c;
-    c.in[0] = at::empty({m.B, m.Hq, m.T, m.D}, opt);
-    Tensor kv = at::empty({6, m.B, m.Hkv, m.T, m.D}, opt);
-    c.in[7] = at::empty({m.B, m.Hq, m.T, 3}, opt);
+    c.in[0] = fresh({m.B, m.Hq, m.T, m.D}, at::kBFloat16, l.x);
+    Tensor kv = fresh({6, m.B, m.Hkv, m.T, m.D}, at::kBFloat16, l.x);
+    c.in[7] = fresh({m.B, m.Hq, m.T, 3}, at::kBFloat16, l.x);
     for (int k = 0; k < 6; ++k) c.in[1 + k] = kv.select(0, k);
     check(nsa_split_heads(y.data_ptr(), c.in[0].data_ptr(), kv.data_ptr(), c.in[7].data_ptr(), m.B, m.T, m.Hq, m.Hkv, m.D,
                           NSA_DTYPE_BF16, raw_stream(l.x)));
     Tensor saved;
     Tensor o = op_forward(c, need_grad, &saved);
-    Tensor tokens = at::empty({rows, hd}, opt);
+    Tensor tokens = fresh({rows, hd}, at::kBFloat16, l.x);
     check(nsa_swap_heads_tokens(o.data_ptr(), tokens.data_ptr(), m.B, m.Hq, m.T, m.D, NSA_DTYPE_BF16, 1, raw_stream(l.x)));
     Tensor out = at::mm(tokens, w_out.t()).view({l.B, l.T, l.dm});
     if (keep) {
@@ -313,20 +324,19 @@ struct LayerNode : torch::autograd::Function<LayerNode> {
     for (int k = 0; k < 6; ++k) in[1 + k] = kv.select(0, k);
     const int64_t rows = (int64_t)m.B * m.T, hd = (int64_t)m.Hq * m.D, dm = w_out.size(0);
     const int64_t width = nsa_fused_projection_width(m.Hq, m.Hkv, m.D);
-    const auto opt = kv.options();
     const Tensor dy = aligned(g[0].to(at::kBFloat16)).view({rows, dm});
     if (ctx->needs_input_grad(10)) res[11] = at::mm(dy.t(), tokens, at::kFloat);
     if (!op_any) return res;
-    Tensor d_tokens = at::mm(dy, w_out), d_out = at::empty({m.B, m.Hq, m.T, m.D}, opt);
+    Tensor d_tokens = at::mm(dy, w_out), d_out = fresh({m.B, m.Hq, m.T, m.D}, at::kBFloat16, kv);
     check(nsa_swap_heads_tokens(d_tokens.data_ptr(), d_out.data_ptr(), m.B, m.Hq, m.T, m.D, NSA_DTYPE_BF16, 0, raw_stream(dy)));
-    Tensor d_in[8], d_comp[6], d_kv = at::empty_like(kv);
-    d_in[0] = at::empty_like(in[0]);
-    d_in[7] = at::empty_like(in[7]);
+    Tensor d_in[8], d_comp[6], d_kv = fresh_like(kv);
+    d_in[0] = fresh_like(in[0]);
+    d_in[7] = fresh_like(in[7]);
     for (int k = 0; k < 6; ++k) d_in[1 + k] = d_kv.select(0, k);
     op_backward(d, in, kept.data() + 9, kept[3], kept[4], d_out, d_in, d_comp);
     for (int k = 0; k < 6; ++k) res[12 + k] = d_comp[k];
     if (!rows_any) return res;
-    Tensor d_rows = at::empty({rows, width}, opt);
+    Tensor d_rows = fresh({rows, width}, at::kBFloat16, kv);
     check(nsa_merge_heads(d_in[0].data_ptr(), d_kv.data_ptr(), d_in[7].data_ptr(), d_rows.data_ptr(), m.B, m.T, m.Hq, m.Hkv, m.D,
                           NSA_DTYPE_BF16, raw_stream(dy)));
     if (ctx->needs_input_grad(0)) {
