@@ -350,7 +350,7 @@ static int range_attn_bwd(const void* q, const void* k, const void* v, const voi
                           const float* lse, const void* d_o, void* dq, float* dq_acc, void* dk, void* dv,
                           const NsaDims* dims, int Lk, int mode, int window, int block_size,
                           const float* row_scale, const float* row_dot,
-                          void* workspace, size_t workspace_bytes, int impl, void* stream) {
+                          void* workspace, size_t workspace_bytes, int impl, void* stream, bool wide_dq = false) {
   int rc = check_dims(dims);
   if (rc != NSA_OK) return rc;
   NSA_CHECK_ARG(mode == NSA_MODE_WINDOW || mode == NSA_MODE_COMPRESS || mode == NSA_MODE_COMPRESS_STRIDED,
@@ -379,6 +379,7 @@ static int range_attn_bwd(const void* q, const void* k, const void* v, const voi
   }
   a.row_scale = row_scale; a.row_dot = row_dot;
   a.dq_acc = dq_acc;
+  a.wide_dq = wide_dq;
   NSA_CHECK_ARG((row_scale == nullptr) == (row_dot == nullptr), "row_scale and row_dot go together");
   if (use_tc(dims, 64, impl, &rc)) {
     a.dk_acc = (float*)dk;   // tc path writes dk/dv itself; pass the outputs through
@@ -390,6 +391,16 @@ static int range_attn_bwd(const void* q, const void* k, const void* v, const voi
   NSA_CHECK_ARG(dq, "dq may be null only when the tcgen05 kernels serve the call");
   return simt_bwd(a, dims, dk, dv, workspace, workspace_bytes, st);
 }
+
+// the whole op's window backward, whose partials go to tc_dq_reduce3 inside the same call
+namespace nsa {
+int window_bwd(const void* q, const void* k, const void* v, const void* o, const float* lse, const void* d_o, void* dq,
+               void* dk, void* dv, const NsaDims* dims, int window, const float* row_scale, const float* row_dot,
+               void* workspace, size_t workspace_bytes, int impl, cudaStream_t st) {
+  return range_attn_bwd(q, k, v, o, lse, d_o, dq, nullptr, dk, dv, dims, dims->T, NSA_MODE_WINDOW, window, 0, row_scale, row_dot,
+                        workspace, workspace_bytes, impl, st, true);
+}
+}  // namespace nsa
 
 extern "C" int nsa_range_attn_bwd(const void* q, const void* k, const void* v, const void* o,
                                   const float* lse, const void* d_o, void* dq, void* dk, void* dv,

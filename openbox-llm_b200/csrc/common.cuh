@@ -150,6 +150,9 @@ struct AttnArgs {
   const void *g_cmp, *g_win, *g_logits;
   void *g_out, *o_kept;
   bool plan_kept;         // the plan outlives the dQ reduction: the backward need not copy its pair map
+  // window backward without a dq of its own: who reads the partials knows that they may lie in tiles of 128 keys (a caller
+  // who names neither the key count nor the options to nsa_dq_reduce3 gets them in tiles of 64)
+  bool wide_dq;
   int B, Hq, Hkv, T, Lk, D, S;
   int kind;          // 0 window, 1 compress, 2 selection
   int window, block_size;
@@ -175,6 +178,10 @@ int tc_sel_plan_build(const AttnArgs& a, void* plan, size_t plan_bytes, cudaStre
 const int32_t* sel_plan_pair_map(const AttnArgs& a, int S, int block_size, const void* plan);
 size_t tc_attn_bwd_workspace(const AttnArgs& a);
 int tc_attn_bwd(const AttnArgs& a, void* ws, size_t ws_bytes, cudaStream_t st);
+// api.cu: the whole op's window backward (wide_dq); its workspace is nsa_range_attn_bwd's
+int window_bwd(const void* q, const void* k, const void* v, const void* o, const float* lse, const void* d_o, void* dq,
+               void* dk, void* dv, const NsaDims* dims, int window, const float* row_scale, const float* row_dot,
+               void* workspace, size_t workspace_bytes, int impl, cudaStream_t st);
 int tc_dq_reduce3(const AttnArgs& base, int Lk_cmp, int cmp_len, int cmp_stride, int S, int block_size,
                   int window, const void* ws_cmp, const void* ws_slc, const void* ws_win,
                   const int32_t* pos, const float* dq_acc, void* dq, cudaStream_t st);

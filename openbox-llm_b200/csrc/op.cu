@@ -460,13 +460,14 @@ extern "C" int nsa_attention_bwd(const NsaAttentionDesc* d, const NsaAttentionTe
     NSA_TRY(nsa_range_attn_bwd_acc(t->q, t->kw, t->vw, o[2], lse[2], t->d_out, dq_acc, t->dkw, t->dvw, &m, m.T,
                                    NSA_MODE_WINDOW, d->window, 0, rs[2], rd[2], ws[2], p.ws_bytes[2], s_win));
   else
-    NSA_TRY(nsa_range_attn_bwd(t->q, t->kw, t->vw, o[2], lse[2], t->d_out, dq[2], t->dkw, t->dvw, &m, m.T,
-                               NSA_MODE_WINDOW, d->window, 0, rs[2], rd[2], ws[2], p.ws_bytes[2], d->impl, s_win));
+    NSA_TRY(window_bwd(t->q, t->kw, t->vw, o[2], lse[2], t->d_out, dq[2], t->dkw, t->dvw, &m, d->window, rs[2], rd[2],
+                       ws[2], p.ws_bytes[2], d->impl, s_win));
   NSA_TRY(fork.join());
   if (!p.fused) return nsa_sum3(dq[0], dq[1], dq[2], t->dq, p.n_q, m.dtype, stream);
   // the three branches left their dQ partials in their workspaces (or two of them in the accumulator)
   AttnArgs a = base_args(&m, m.T);
   a.three_term = p.three_term;
+  a.wide_dq = true;
   const int32_t* pos = sel_plan_pair_map(a, p.S, d->block_size, sv + p.plan);
   if (acc_mode)
     return tc_dq_reduce3(a, 0, 0, 0, p.S, d->block_size, 1, nullptr, ws[1], nullptr, pos, dq_acc, t->dq, st);

@@ -4,7 +4,7 @@
 // once (TMA), dK^T and dV^T of the tile stay in TMEM for the whole CTA and are written once,
 // with no atomics.  The CTA walks the (query, head) rows that attend the tile, 128 rows at a
 // time (nq queries x the G heads of the group):
-//   window      queries [64 j, 64 j + 63 + W - 1]
+//   window      queries [64 j, 64 j + 63 + W - 1]  (up to a wave of tiles; more go on tiles of 128 keys, use_wide)
 //   compression queries t >= (64 j + 1) * Bsz - 1
 //   selection   the queries that list block j, from the block -> query CSR
 // Q and dO rows arrive by TMA into 128B-swizzled tiles: one box per row tile for the window and
@@ -563,7 +563,7 @@ tc_bwd_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ 
 // 70 each, N = 64 or 128 alike).  A row tile takes 3.8 k; with groups that did their own tile's dQ between two tiles'
 // arithmetic it was 4.7 k.  At D = 64 (112 + 80 KB, 1.4 k of MMAs) a selection tile takes as long as its gather: 64 to 84
 // boxes for groups of 4 and 3, and a warp gets one out every 65 cycles, so seven warps do it (8 x 4096 tokens, 12 heads of
-// 64: 604 us, 658 with three; copies of 16 bytes by all lanes instead: 746).  That leaves 96 registers a thread, which
+// 64: 604 us, 658 with three; copies of 16 bytes by all lanes instead: 746; with masks as bits 520).  That leaves 96 registers a thread, which
 // costs the compute warps more than it gives where the rows are consecutive or two slabs come in one box: three
 // producers there.  D = 64 computes dV^T and dK^T in one product, [dO | Q]^T [P | dS] (their tiles are neighbours): the two
 // off-diagonal quarters are wasted, but the operands are read once, 8 KB a step instead of 12.
@@ -577,8 +577,8 @@ constexpr int kB2Dq = 4;          // dQ warps; then the producers and one MMA wa
 // the tensor cores as three bf16 terms each, all 24 bits of the fp32 values (two more of each of the three products they
 // enter), the dQ partials stay fp32, a block listed twice counts twice and what comes out non-finite is done again row by
 // row (sel_row.cuh).  P and dS take 96 KB of a slot, so one slot fits.  The whole op on 16-token blocks, forward + backward (2 x 1024 tokens, 16 heads of 128, 8 blocks a
-// list): selection backward with its plan and dQ sum 199 us against 799 on the CUDA cores (182 with two terms), forward
-// 42 against 360, the pass 345 against 1300.
+// list): selection backward with its plan and dQ sum 199 us (then a pass of 345) against 799 on the CUDA cores (182 with two terms), forward
+// 42 against 360, the pass 302 against 1300.
 template <int D, bool kThreeTerm, bool kGather> struct Bwd2 {
   static constexpr int kSlabs = D / 64;
   static constexpr int kTerms = kThreeTerm ? 3 : 1;
@@ -1656,7 +1656,7 @@ namespace tc {
 // of 64; from 128 tiles on it takes 0.65 to 0.7 of their time.  Compression keeps tiles of 64: the gradient of its key
 // pooling's position parameters is the rounding of P and dS, which the products here round in another order.
 static bool use_wide(const AttnArgs& a) {
-  return a.kind == 0 && a.Lk == a.T && !a.dq_acc && get_option_bwd_kernel() == 1 &&
+  return a.kind == 0 && a.Lk == a.T && !a.dq_acc && (a.dq || a.wide_dq) && get_option_bwd_kernel() == 1 &&
          (long long)a.B * a.Hkv * ((a.T + kKeys - 1) / kKeys) > sm_count();
 }
 
@@ -1674,7 +1674,7 @@ static BwdPlan plan_bwd(const AttnArgs& a) {
     part_rows = pl.cap_pairs;
   } else {
     pl.n_slots = a.kind != 0 ? pl.n_ktiles : pl.wide ? (std::min(a.window, a.T) + kWideKeys - 2) / kWideKeys + 1
-                                                     : (a.window + kKeys - 2) / kKeys + 1;
+                                                     : (std::min(a.window, a.T) + kKeys - 2) / kKeys + 1;
     pl.cap_pairs = 0;
     part_rows = a.dq_acc ? 0 : units * a.T * pl.n_slots;   // accumulator mode: no partial buffer
   }
@@ -1696,7 +1696,7 @@ static BwdPlan plan_bwd(const AttnArgs& a) {
   // order, row tiles in turn within a chunk and chunks as cmp_chunks_kernel adds them, since the
   // gradient of the key pooling's position parameters is the rounding of those sums (tc.cu), and where a problem is small it
   // runs beside the other branches.
-  const int max_rt = a.kind == 0 ? (a.window + kKeys - 2 + pl.nq) / pl.nq : (a.T + pl.nq - 1) / pl.nq;
+  const int max_rt = a.kind == 0 ? (std::min(a.window, 1 << 30) + kKeys - 2 + pl.nq) / pl.nq : (a.T + pl.nq - 1) / pl.nq;
   const int item_rt = a.kind == 2 ? (max_rt < kSelChunkTiles ? max_rt : kSelChunkTiles) : max_rt;
   const long long base = (long long)units * pl.n_ktiles;
   pl.csize = 1;
@@ -1831,7 +1831,7 @@ int tc_attn_bwd(const AttnArgs& a, void* ws, size_t ws_bytes, cudaStream_t st) {
   p.status = device_status_ptr();
   if (!p.status) { set_error("device status word unavailable"); return NSA_ERR_CUDA; }
   p.B = a.B; p.Hq = a.Hq; p.Hkv = a.Hkv; p.T = a.T; p.Lk = a.Lk; p.G = G; p.nq = pl.nq;
-  p.kind = a.kind; p.window = a.window; p.block_size = a.block_size;
+  p.kind = a.kind; p.window = a.kind == 0 ? std::min(a.window, a.T) : a.window; p.block_size = a.block_size;
   p.n_ktiles = pl.n_ktiles; p.n_slots = pl.n_slots;
   p.dq_acc_mode = (a.dq_acc && a.kind != 2) ? 1 : 0;
   p.merged = (a.kind == 2 && a.D == 128 && G % 8 == 0 && get_option_merged_boxes()) ? 1 : 0;

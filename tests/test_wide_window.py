@@ -103,3 +103,25 @@ def test_gradients_that_start_anywhere():
         want = want or got
         assert all(torch.equal(a, b) for a, b in zip(got, want))
     assert L.lib().nsa_device_status(None) == 0
+
+
+@pytest.mark.parametrize("B,Hq,Hkv,T,Lk,D,window", [(40, 8, 4, 130, 200, 64, 100), (24, 12, 4, 385, 385, 128, 200), (40, 8, 4, 130, 129, 64, 2 ** 31 - 1)])
+def test_partials_for_a_sum_by_hand(B, Hq, Hkv, T, Lk, D, window):
+    """Partials that a caller has added up by nsa_dq_reduce3 lie where that looks for them, whatever the number of keys and
+    the options at that time.  Bound: two bf16 partials' roundings apart."""
+    L = importlib.import_module("openbox-llm_b200._lib")
+    g = torch.Generator("cuda").manual_seed(T + Lk)
+    q, do = (torch.randn(B, Hq, T, D, generator=g, device="cuda").bfloat16() for _ in range(2))
+    k, v = (torch.randn(B, Hkv, Lk, D, generator=g, device="cuda").bfloat16() for _ in range(2))
+    o, lse = nsa.range_attn_forward(q, k, v, nsa.MODE_WINDOW, window, 0)
+    want = nsa.range_attn_backward(q, k, v, o, lse, do, nsa.MODE_WINDOW, window, 0)
+    ws, dk, dv = nsa.range_attn_backward(q, k, v, o, lse, do, nsa.MODE_WINDOW, window, 0, defer_dq=True)
+    dq = torch.empty_like(q)
+    try:
+        L.check(L.lib().nsa_set_option(b"bwd_kernel", 0))
+        L.check(L.lib().nsa_dq_reduce3(L.dims(B, Hq, Hkv, T, D, L.DTYPE_BF16), 0, 0, 0, 0, 64, window, None, None, ws.data_ptr(), dq.data_ptr(),
+                                       L.stream()))
+    finally:
+        L.check(L.lib().nsa_set_option(b"bwd_kernel", 1))
+    for x, y in zip((dq, dk, dv), want):
+        assert rel(x, y.double()) < 2.0 ** -7
