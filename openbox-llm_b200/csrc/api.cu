@@ -296,9 +296,8 @@ extern "C" int nsa_debug_set_device_status(int value, void* stream) {
 }
 
 // ---- range attention -------------------------------------------------------------------------
-extern "C" int nsa_range_attn_fwd(const void* q, const void* k, const void* v, void* o, float* lse,
-                                  const NsaDims* dims, int Lk, int mode, int window, int block_size,
-                                  int impl, void* stream) {
+static int range_attn_fwd(const void* q, const void* k, const void* v, void* o, float* lse, const NsaDims* dims, int Lk, int mode,
+                          int window, int block_size, int impl, bool chained, void* stream) {
   int rc = check_dims(dims);
   if (rc != NSA_OK) return rc;
   NSA_CHECK_ARG(mode == NSA_MODE_WINDOW || mode == NSA_MODE_COMPRESS || mode == NSA_MODE_COMPRESS_STRIDED,
@@ -317,10 +316,23 @@ extern "C" int nsa_range_attn_fwd(const void* q, const void* k, const void* v, v
     NSA_CHECK_ARG(window >= 1 && window <= block_size, "summary stride must be in [1, block_size]");
     a.kind = NSA_MODE_COMPRESS;
   }
+  a.chained = chained;
   if (use_tc(dims, 64, impl, &rc) && Lk > 0) return tc_attn_fwd(a, (cudaStream_t)stream);
   if (rc != NSA_OK) return rc;
   return simt_attn_fwd(a, dims->dtype, (cudaStream_t)stream);
 }
+
+extern "C" int nsa_range_attn_fwd(const void* q, const void* k, const void* v, void* o, float* lse,
+                                  const NsaDims* dims, int Lk, int mode, int window, int block_size,
+                                  int impl, void* stream) {
+  return range_attn_fwd(q, k, v, o, lse, dims, Lk, mode, window, block_size, impl, false, stream);
+}
+namespace nsa {
+int compress_fwd(const void* q, const void* k, const void* v, void* o, float* lse, const NsaDims* dims, int Lk, int stride,
+                 int len, int impl, bool chained, void* stream) {
+  return range_attn_fwd(q, k, v, o, lse, dims, Lk, NSA_MODE_COMPRESS_STRIDED, stride, len, impl, chained, stream);
+}
+}  // namespace nsa
 
 static size_t range_bwd_ws(const NsaDims* dims, int Lk, int mode, int window, int impl, bool acc) {
   if (check_dims(dims) != NSA_OK) return 0;

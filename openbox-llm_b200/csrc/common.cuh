@@ -104,10 +104,12 @@ struct KernelScope {
 // T = 1024 53.1 -> 48.1, selection at T = 8192 forward and backward 362 -> 339 (350 with the backward's kernels
 // one after the other), three branches over given lists at T = 4096 94 -> 88.8 (alone in a graph, where the launches cost nothing, 80 -> 84).
 // Plain launches stay where an early CTA takes a place that another stream's kernel would fill: the block-outer
-// selection kernel (chained 98.6 where it is 89.3 plain) and the attention over pooled keys (T = 3000
-// 91 against 86.3), both beside the window's kernel.
+// selection kernel (chained 98.6 where it is 89.3 plain) and, over given lists, the attention over pooled keys (T = 3000
+// 91 against 86.3), both beside the window's kernel.  With lists of the scorer the window is launched ahead of the
+// pooling, and chained is the better: forward at 512 tokens 39.3 -> 37.9 us, 2 x 300 41.1 -> 38.5, 1024 47.8 -> 46.5.
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void chain_go() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // What the kernel ahead writes is read by plain loads, which stay behind the wait: the read-only path (__ldg, a const
 // __restrict__ argument) takes its data not to change while the kernel is on the GPU, which includes the time before.
 __device__ __forceinline__ int32_t ld_plain(const int32_t* p) { int32_t v; asm volatile("ld.global.s32 %0, [%1];" : "=r"(v) : "l"(p)); return v; }
@@ -153,6 +155,7 @@ struct AttnArgs {
   // window backward without a dq of its own: who reads the partials knows that they may lie in tiles of 128 keys (a caller
   // who names neither the key count nor the options to nsa_dq_reduce3 gets them in tiles of 64)
   bool wide_dq;
+  bool chained;      // tcgen05 compression forward: launched into the end of the pooling (launch_chained)
   int B, Hq, Hkv, T, Lk, D, S;
   int kind;          // 0 window, 1 compress, 2 selection
   int window, block_size;
@@ -178,7 +181,9 @@ int tc_sel_plan_build(const AttnArgs& a, void* plan, size_t plan_bytes, cudaStre
 const int32_t* sel_plan_pair_map(const AttnArgs& a, int S, int block_size, const void* plan);
 size_t tc_attn_bwd_workspace(const AttnArgs& a);
 int tc_attn_bwd(const AttnArgs& a, void* ws, size_t ws_bytes, cudaStream_t st);
-// api.cu: the whole op's window backward (wide_dq); its workspace is nsa_range_attn_bwd's
+// api.cu: the whole op's attention over pooled keys, and its window backward (wide_dq; the workspace is nsa_range_attn_bwd's)
+int compress_fwd(const void* q, const void* k, const void* v, void* o, float* lse, const NsaDims* dims, int Lk, int stride,
+                 int len, int impl, bool chained, void* stream);
 int window_bwd(const void* q, const void* k, const void* v, const void* o, const float* lse, const void* d_o, void* dq,
                void* dk, void* dv, const NsaDims* dims, int window, const float* row_scale, const float* row_dot,
                void* workspace, size_t workspace_bytes, int impl, cudaStream_t st);

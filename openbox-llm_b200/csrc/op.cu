@@ -330,8 +330,7 @@ extern "C" int nsa_attention_fwd(const NsaAttentionDesc* d, const NsaAttentionTe
     s.out[0] = k_cmp; s.out[1] = v_cmp;
     NSA_TRY(pool_mean_fwd(s, m.B, m.Hkv, m.T, m.D, d->block_size, m.dtype, st));
   }
-  NSA_TRY(nsa_range_attn_fwd(t->q, k_cmp, v_cmp, o[0], lse[0], &m, p.n_cmp, NSA_MODE_COMPRESS_STRIDED, d->cmp_stride,
-                             d->cmp_len, d->impl, stream));
+  NSA_TRY(compress_fwd(t->q, k_cmp, v_cmp, o[0], lse[0], &m, p.n_cmp, d->cmp_stride, d->cmp_len, d->impl, !d->given_lists, stream));
   if (d->given_lists) {
     NSA_TRY(window());
     NSA_TRY(selection(fork.stream(1)));

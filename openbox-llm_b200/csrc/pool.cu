@@ -64,6 +64,7 @@ template <int D, int R>
 __global__ void __launch_bounds__(kThreads, 2)
 pool_fwd_kernel(const PoolSides s, int T_, int len, int stride, int n_sum, int rows) {
   extern __shared__ float4 sm4[];
+  chain_go();
   float* sm = reinterpret_cast<float*>(sm4);
   constexpr int VL = D / 8, RG = kThreads / VL, kLd = PoolFwdSmem<D, R>::kProjLd;
   float* projS = sm;
@@ -457,6 +458,7 @@ template <> struct Vec<float> {
 // 2 x 4 x 4096 tokens of 64 bf16, 5 so.
 template <typename T>
 __global__ void mean_fwd_kernel(const PoolSides s, int T_, int Dv, int len, int n_sum, size_t rows) {
+  chain_go();
   constexpr int N = Vec<T>::N;
   const size_t row = (size_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= rows) return;

@@ -186,8 +186,8 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *s_tmem;
-  if (kSel) chain_wait();
-  else if (kCmp) chain_go();            // the scorer is next
+  if (kSel || kCmp) chain_wait();
+  if (kCmp) chain_go();            // the scorer is next
 
   // row tile w of the launch: long rows first, the units of one token range next to each other
   const int units = p.B * p.Hkv;
@@ -662,7 +662,8 @@ static int launch_fwd(const AttnArgs& a, const SelPlanHeader* plan, int force, c
   KernelScope ks(branch_name(kFwdNames, a.kind), st);
   auto go = [&](auto kernel) -> int {
     NSA_CUDA_OK(func_smem((const void*)kernel, smem));
-    if (a.kind == 2) NSA_CUDA_OK(launch_chained(kernel, grid, kFwdThreads, smem, st, tm_q, tm_k, tm_v, p));   // behind scorer or plan
+    if (a.kind == 2 || a.chained)          // behind scorer, plan or pooling
+      NSA_CUDA_OK(launch_chained(kernel, grid, kFwdThreads, smem, st, tm_q, tm_k, tm_v, p));
     else kernel<<<grid, kFwdThreads, smem, st>>>(tm_q, tm_k, tm_v, p);
     return NSA_OK;
   };
