@@ -177,7 +177,7 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     prefetch_tensormap(&tm_q); prefetch_tensormap(&tm_k); prefetch_tensormap(&tm_v);
   }
   __syncthreads();
-  if (*s_abort) return;
+  if (*s_abort) { chain_wait(); return; }      // the kernels behind take its end for that of all before
   if (warp == 0) {
     tmem_alloc(s_tmem, kTmemCols);
     tmem_relinquish();
