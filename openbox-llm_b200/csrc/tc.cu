@@ -310,6 +310,8 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       // ---- MMA issuer ------------------------------------------------------------------------
       {
         const uint32_t lead = elect_one(), tmem_u = uniform(tmem);
+        // Every wait is the whole warp's: the lanes come out of it together and with one answer.  A lane that fell two phases
+        // behind the issuing one would wait for a parity that has come round, up to the limit.
         auto ready = [&](uint64_t* bar, uint32_t parity, int code) -> bool {
           return __all_sync(0xffffffffu, mbar_wait(bar, parity, p.status, s_abort, code));
         };
@@ -329,26 +331,24 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         for (int w = w0; ok && w < w_end; w += gridDim.x) {
           const Tile x = tile_of(w);
           if (x.n_tiles == 0) continue;
-          ok = mbar_wait(bar_q, it & 1, p.status, s_abort, 1) &&
-               mbar_wait(bar_k + c % kStages, (c / kStages) & 1, p.status, s_abort, 2);
+          ok = ready(bar_q, it & 1, 1) && ready(bar_k + c % kStages, (c / kStages) & 1, 2);
           // An S MMA overwrites the P of two key tiles back: that tile's PV has to be complete (MMAs of
           // different shapes and operand sources are not ordered by their issue).  Here every earlier
           // one is waited for; the threads that write the last row tile's output wait for it as well.
-          if (ok && c > 0) ok = mbar_wait(bar_o + ((c - 1) & 1), ((c - 1) >> 1) & 1, p.status, s_abort, 0x2000);
+          if (ok && c > 0) ok = ready(bar_o + ((c - 1) & 1), ((c - 1) >> 1) & 1, 0x2000);
           if (!ok) break;
           tc_fence_after();
           issue_s(c, x.n_tiles == 1);
           for (int i = 0; i < x.n_tiles; ++i, ++c) {
             if (i + 1 < x.n_tiles) {
-              ok = mbar_wait(bar_k + (c + 1) % kStages, ((c + 1) / kStages) & 1, p.status, s_abort, 2);
-              if (ok && i > 0) ok = mbar_wait(bar_o + ((c - 1) & 1), ((c - 1) >> 1) & 1, p.status, s_abort, 0x2000);
+              ok = ready(bar_k + (c + 1) % kStages, ((c + 1) / kStages) & 1, 2);
+              if (ok && i > 0) ok = ready(bar_o + ((c - 1) & 1), ((c - 1) >> 1) & 1, 0x2000);
               if (!ok) break;
               tc_fence_after();
               issue_s(c + 1, i + 2 == x.n_tiles);
             }
             const int st = c % kStages;
-            ok = mbar_wait(bar_p + (c & 1), (c >> 1) & 1, p.status, s_abort, 0x2000) &&
-                 mbar_wait(bar_v + st, (c / kStages) & 1, p.status, s_abort, 16);
+            ok = ready(bar_p + (c & 1), (c >> 1) & 1, 0x2000) && ready(bar_v + st, (c / kStages) & 1, 16);
             if (!ok) break;
             tc_fence_after();
             const uint32_t va = desc_lo_mnmajor(smem_u32(sV + st * L::kKVBytes), kKeys * 128);   // O (+)= P V
@@ -361,7 +361,7 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
               for (int kk = 0; kk < kKeys / 16; ++kk)
                 mma_ts_by(lead, tmem_u + kColO, tmem_u + kColS + (c & 1) * kKeys + 32 + kk * 8, desc_at(va, kk * 2048), kIdescPV, 1);
               if (kLate) {
-                ok = mbar_wait(bar_p3 + (c & 1), (c >> 1) & 1, p.status, s_abort, 0x2000);
+                ok = ready(bar_p3 + (c & 1), (c >> 1) & 1, 0x2000);
                 if (!ok) break;
                 tc_fence_after();
               }

@@ -1,0 +1,24 @@
+"""Rules of the role-split kernels that their sources have to keep (read from the sources: what breaks them may show only as
+a wait that runs into its limit, or not at all)."""
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "openbox-llm_b200", "csrc")
+
+
+def _source(name):
+    return open(os.path.join(CSRC, name)).read()
+
+
+@pytest.mark.parametrize("name", ["tc.cu", "tc_fwdpair_kernel.cu", "tc_bwd.cu", "tc_bwd_wide.cu"])
+def test_a_warp_that_issues_as_one_waits_as_one(name):
+    """A warp whose elected lane issues the MMAs leaves every wait by a vote.  Lanes that waited each for itself could part, and
+    one that fell two phases behind would wait for a parity that has come round.  Barriers of one phase are exempt."""
+    roles = [part for part in re.split(r"\n\s*// ---- ", _source(name)) if "mma_ss_by(" in part]
+    assert roles
+    for role in roles:
+        for line in role.splitlines():
+            if re.search(r"\bmbar_(try_|test_)?wait\(", line):
+                assert "__all_sync(" in line or "bar_kv" in line or "bar_drain" in line, line
