@@ -1112,14 +1112,17 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
       const float lse2 = lse_cur * kLog2e - __log2f(gate_cur);
       const float dscale = p.scale, ddelta = delta_cur * p.scale;
       // the columns of this thread's half that are attended, a bit each: all of them away from the diagonal.  Rows that are
-      // zero in Q and dO (past nq * G of a tile, and selection's past its last query) may count as attending all: two
+      // not there (past nq * G of a tile, and selection's past its last query: zeros in Q and dO) count as attending all: two
       // of them in the last quarter of every tile of three heads had its warps mask every element, 1.7 k cycles a tile
-      // behind the others
+      // behind the others.  What they leave in P and dS is written over with zeros, since zeros times a key that is not finite
+      // are NaN (8 x 4096 tokens, 12 heads of 64: selection 521 us with or without, compression 72 -> 74; zeroed in
+      // registers 532 and 78)
       const int lo_h = min(max(lo - half * 32, 0), 32), hi_h = min(max(hi + 1 - half * 32, 0), 32);
       uint32_t attended = (hi_h == 32 ? ~0u : (1u << hi_h) - 1u) & ~((lo_h == 32) ? ~0u : (1u << lo_h) - 1u);
       if (!(groups & 1u)) attended &= 0xffff0000u;
       if (!(groups & 2u)) attended &= 0x0000ffffu;
-      if (!row_slot_ok || (p.kind == 2 && t_cur < 0)) attended = ~0u;
+      const bool there = row_slot_ok && (p.kind != 2 || t_cur >= 0);
+      if (!there) attended = ~0u;
       const bool all_cols = attended == ~0u && !repeats;
       float times[2] = {1.f, 1.f};                   // how often the row's list names the blocks of its column groups
       if (kThreeTerm && repeats && t_cur >= 0) {
@@ -1197,6 +1200,14 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
           }
           st_shared_v4(p_row + chunk16, pp[k4 * 4], pp[k4 * 4 + 1], pp[k4 * 4 + 2], pp[k4 * 4 + 3]);
           st_shared_v4(ds_row + chunk16, pd[k4 * 4], pd[k4 * 4 + 1], pd[k4 * 4 + 2], pd[k4 * 4 + 3]);
+        }
+        if (!there) {
+#pragma unroll
+          for (int k4 = 0; k4 < 4 * L::kTerms; ++k4) {
+            const uint32_t at = ((uint32_t)((half * 4 + (k4 & 3)) ^ (row & 7)) << 4) + (k4 >> 2) * 2 * kPBytes;
+            st_shared_v4(p_row + at, 0u, 0u, 0u, 0u);
+            st_shared_v4(ds_row + at, 0u, 0u, 0u, 0u);
+          }
         }
       }
       fence_proxy_async();
