@@ -16,6 +16,9 @@
 // Roles: eight compute warps (two per TMEM lane quadrant, half of the rows each), four dQ warps, one warp each for Q,
 // dO, the row statistics and the MMAs.  Each hand-over is an mbarrier with a bounded wait.
 //
+// What is not finite: a V stays with the rows that attend its key, a row of dO (or its delta) or Q reaches dK and dV of the key
+// tiles that its query attends, a K dQ of the rows that share one of its steps of 16 keys: 0 x inf in a product is NaN.
+//
 // What bounds it: at D = 128 the chain S -> p -> dP -> dS of one row tile, whose S and dP fill what TMEM dV and dK leave
 // (4.8 k cycles a row tile, the MMAs alone 2.7 k); at D = 64 the MMAs (4.2 k against 1.8 k by themselves: the warp that
 // issues them shares its scheduler with compute warps, and their operands share shared memory with dS and the tiles
@@ -50,7 +53,8 @@ template <int D> struct Wide {
   static constexpr uint32_t kColP = kOwnP ? kColDQ + D : kColS, kStepP = kOwnP ? 32 : 64;
   static constexpr int kStats = D == 64 ? 4 : 1;                  // row statistics: ring of lse(0), delta(0), lse(1), ...
   static constexpr int kStatBytes = kRows * 16;                   // a row: three bf16 terms of the value, zeros
-  static constexpr int kBars = 2 + 4 * kStages + 7 + kDsTiles + 2 * kStats;
+  static constexpr int kBarS = 2 + 4 * kStages, kBars = kBarS + 7 + kDsTiles + 2 * kStats;
+  static constexpr int kOffDs = 2 * kKVBytes + kStages * 2 * kRowBytes, kOffBars = kOffDs + kDsTiles * kDsBytes + kStageOut + kStats * kStatBytes + 256;
   static constexpr size_t kSmem = 2 * kKVBytes + (size_t)kStages * 2 * kRowBytes + kDsTiles * kDsBytes + kStageOut + kStats * kStatBytes +
                                   256 /*ones*/ + 256 /*barriers*/ + 512 /*alignment slack*/;
 };
@@ -86,6 +90,80 @@ __device__ __forceinline__ bool group_or(int id, int threads, int pred) {
   return out != 0;
 }
 
+// The compute warps' work of a CTA by select: what a key is not attended by may be infinite or NaN.  `smem` and `bars` as in the
+// kernel below.  Not inlined, so that the registers and the schedule of the usual loop stay what they are: as a second form of its
+// body, 8 x 4096 tokens of 12 heads of 64 took 295 us instead of 270, with checks in it 327.
+template <int D>
+__device__ __noinline__ void masked_row_tiles(const WideArgs& p, uint8_t* smem, uint32_t tmem) {
+  using L = Wide<D>;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::kOffBars);
+  uint64_t *s_full = bars + L::kBarS, *dp_full = s_full + 1, *p_full = dp_full + 1, *ds_full = p_full + 1, *ds_free = ds_full + 3;
+  uint64_t* dv_done = ds_free + L::kDsTiles;
+  volatile int* s_abort = reinterpret_cast<volatile int*>(reinterpret_cast<uint32_t*>(bars + L::kBars) + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, quad = warp & 3, half = warp >> 2;
+  const int key0 = blockIdx.x * kWideKeys, kr = quad * 32 + lane, key = key0 + kr;
+  const int n_q = min(p.T - 1, key0 + kWideKeys - 1 + p.window - 1) - key0 + 1, n_tiles = (n_q + p.nq - 1) / p.nq;
+  const uint32_t lane_base = tmem + ((uint32_t)(quad * 32) << 16) + half * 64;
+  const uint32_t p_base = tmem + ((uint32_t)(quad * 32) << 16) + L::kColP + half * L::kStepP;
+#pragma unroll 1
+  for (int k = 0; k < n_tiles; ++k) {
+    const int qi0 = k * p.nq, to_key = key - key0 - qi0;             // queries from the tile's first to the key
+    const uint32_t ds_row = smem_u32(smem + L::kOffDs) + k % L::kDsTiles * L::kDsBytes + half * L::kSlabBytes + kr * 128;
+    const int lo = min(max(to_key, 0), p.nq) * p.G, hi = key >= p.T ? 0 : min(min(p.nq, n_q - qi0), to_key + p.window) * p.G;
+    const int lo_h = min(max(lo - half * 64, 0), 64), hi_h = min(max(hi - half * 64, 0), 64);
+    const uint64_t upto = hi_h == 64 ? ~0ull : (1ull << hi_h) - 1ull;
+    const uint64_t attended = lo_h == 64 ? 0ull : upto >> lo_h << lo_h;
+    bool ok = mbar_wait(s_full, k & 1, p.status, s_abort, 64);
+    if (ok && L::kOwnP && k > 0) ok = mbar_wait(dv_done, (k - 1) & 1, p.status, s_abort, 64);
+    if (!__all_sync(0xffffffffu, ok)) return;                // the whole warp leaves together
+    tc_fence_after();
+    uint32_t pr[64];
+    tmem_ld32(lane_base + L::kColS, pr);
+    tmem_ld32(lane_base + L::kColS + 32, pr + 32);
+    tmem_wait_ld();
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const uint32_t in = (uint32_t)(attended >> (h * 32));
+      uint32_t pk[16];
+#pragma unroll
+      for (int c2 = 0; c2 < 16; ++c2) {
+#pragma unroll
+        for (int c = h * 32 + c2 * 2; c < h * 32 + c2 * 2 + 2; ++c)
+          pr[c] = in >> (c & 31) & 1u ? __float_as_uint(ex2(__uint_as_float(pr[c]) * p.scale_log2)) : 0u;
+        pk[c2] = pack_bf16(__uint_as_float(pr[h * 32 + c2 * 2]), __uint_as_float(pr[h * 32 + c2 * 2 + 1]));
+      }
+      tmem_st16(p_base + h * 16, pk);
+    }
+    tmem_wait_st();
+    tc_fence_before();
+    mbar_arrive(p_full);
+    ok = mbar_wait(dp_full, k & 1, p.status, s_abort, 64);
+    if (ok && k >= L::kDsTiles) ok = mbar_wait(ds_free + k % L::kDsTiles, (k / L::kDsTiles - 1) & 1, p.status, s_abort, 64);
+    if (!__all_sync(0xffffffffu, ok)) return;
+    tc_fence_after();
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const uint32_t in = (uint32_t)(attended >> (h * 32));
+      uint32_t dp[32];
+      tmem_ld32(lane_base + L::kColDP + h * 32, dp);
+      tmem_wait_ld();
+#pragma unroll
+      for (int c = 0; c < 32; ++c)
+        dp[c] = in >> c & 1u ? __float_as_uint(__uint_as_float(pr[h * 32 + c]) * (__uint_as_float(dp[c]) * p.scale)) : 0u;
+#pragma unroll
+      for (int v4 = 0; v4 < 4; ++v4) {
+        uint32_t b[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) b[e] = pack_bf16(__uint_as_float(dp[v4 * 8 + e * 2]), __uint_as_float(dp[v4 * 8 + e * 2 + 1]));
+        st_shared_16b(ds_row + ((uint32_t)((h * 4 + v4) ^ (kr & 7)) << 4), b[0], b[1], b[2], b[3]);
+      }
+    }
+    fence_proxy_async();
+    tc_fence_before();
+    mbar_arrive(ds_full);
+  }
+}
+
 template <int D>
 __global__ void __launch_bounds__(kWideThreads, 1)
 tc_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
@@ -112,7 +190,7 @@ tc_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
   uint64_t* q_full = do_full + kStages;           // [kStages] Q has landed
   uint64_t* do_free = q_full + kStages;           // [kStages] the dV and dP MMAs are done
   uint64_t* q_free = do_free + kStages;           // [kStages] the dK MMAs are done
-  uint64_t* s_full = q_free + kStages;            // S^T is in TMEM
+  uint64_t* s_full = bars + L::kBarS;             // S^T is in TMEM
   uint64_t* dp_full = s_full + 1;                 // dP^T is in TMEM
   uint64_t* p_full = dp_full + 1;                 // P^T is in TMEM (256 arrivals)
   uint64_t* ds_full = p_full + 1;                 // dS is in shared memory, dP has been read (256 arrivals)
@@ -284,7 +362,7 @@ tc_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
         return __all_sync(0xffffffffu, mbar_wait(bar, parity, p.status, s_abort, code));
       };
       // no swizzle: groups of 8 rows x 16 bytes, the statistics' one behind the other, the ones' the same for all rows; the
-      // second half of a step of 16 is zeros there and reads the first half again here
+      // second half of a step of 16 is zeros there and reads the first half again here (so that an infinite delta comes out NaN)
       auto plain = [](const void* t, uint32_t lbo_bytes, uint32_t sbo_bytes) -> uint64_t {
         return (uint64_t)((smem_u32(t) >> 4) & 0x3fffu) | (uint64_t)(lbo_bytes >> 4) << 16 | (uint64_t)(sbo_bytes >> 4) << 32 | 1ull << 46;
       };
@@ -392,13 +470,30 @@ tc_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     const uint32_t lane_base = tmem + ((uint32_t)(quad * 32) << 16) + half * 64;
     const uint32_t p_base = tmem + ((uint32_t)(quad * 32) << 16) + L::kColP + half * L::kStepP;
     const uint32_t ds_row0 = smem_u32(sDs) + half * kSlabBytes + kr * 128;
-    for (int k = 0; k < n_tiles; ++k) {
+    // Where K and V are finite, P = 0 masks dS = P * (dP - delta) as well, and rows past nq * G, zeros in Q and dO, may count
+    // as attended (as others they would have these warps mask every element of every tile).  A K or V that is infinite
+    // or NaN spoils dS of rows that do not attend it, and rows that are not there.  The look at the tile hides behind
+    // the first S.
+    bool odd = false;
+    if (mbar_wait(bar_kv, 0, p.status, s_abort, 32)) {
+      __nv_bfloat162 z(0.f, 0.f);                    // x * 0: 0 or NaN
+#pragma unroll 8
+      for (int i = tid; i < 2 * L::kKVBytes / 16; i += 256) {        // (V lies behind K)
+        const uint4 u = reinterpret_cast<const uint4*>(sK)[i];
+        const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) z = __hfma2(reinterpret_cast<const __nv_bfloat162&>(w[e]), __nv_bfloat162(0.f, 0.f), z);
+      }
+      odd = (reinterpret_cast<const uint32_t&>(z) & 0x7fff7fffu) != 0u;
+    }
+    odd = group_or(3, 256, odd);
+    if (odd) masked_row_tiles<D>(p, smem, tmem);
+    for (int k = odd ? n_tiles : 0; k < n_tiles; ++k) {
       const int qi0 = k * p.nq, t0 = t_lo + qi0;
       const uint32_t ds_row = ds_row0 + k % L::kDsTiles * L::kDsBytes;
       // rows [lo, hi) attend the key
       const int q_end = min(p.nq, n_q - qi0);
       const int q_first = key - t0, q_last = min(q_end, key - t0 + window);
-      // (the rows past nq * G are zeros in Q and dO: attended or not makes no difference)
       const int lo = min(max(q_first, 0), p.nq) * p.G, hi = key >= p.T ? 0 : q_last >= p.nq ? kRows : q_last * p.G;
       // of this warp's half: bit c for row half * 64 + c
       const int lo_h = min(max(lo - half * 64, 0), 64), hi_h = min(max(hi - half * 64, 0), 64);
