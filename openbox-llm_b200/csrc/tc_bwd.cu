@@ -839,6 +839,10 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
         uint8_t* base = sRow + part * (kRows * row_bytes);
         *reinterpret_cast<uint4*>(base + r0 * row_bytes + (i % n) * 16) = make_uint4(0, 0, 0, 0);
       }
+      // nor are P and dS of such rows written, nor dQ over them: times a key that is not finite anything that came of their S
+      // would be NaN (zeros stored over them in the last place cost 1 to 2 % at D = 128)
+      for (int i = tid; i < kSets * (L::kSetBytes / kPBytes) * (kRows - r0) * 8; i += (kB2Compute + kB2Dq) * 32)
+        *reinterpret_cast<uint4*>(sPds + i / ((kRows - r0) * 8) * kPBytes + r0 * 128 + i % ((kRows - r0) * 8) * 16) = make_uint4(0, 0, 0, 0);
     }
     fence_proxy_async();
     if (warp == 0) {
@@ -1111,18 +1115,15 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
       // (gate p)^T dO; dS = scale * gate * p * (dP - delta), the constant factors folded once per row
       const float lse2 = lse_cur * kLog2e - __log2f(gate_cur);
       const float dscale = p.scale, ddelta = delta_cur * p.scale;
-      // the columns of this thread's half that are attended, a bit each: all of them away from the diagonal.  Rows that are
-      // not there (past nq * G of a tile, and selection's past its last query: zeros in Q and dO) count as attending all: two
+      // the columns of this thread's half that are attended, a bit each: all of them away from the diagonal.  Rows past
+      // nq * G of a tile count as attending all, and their rows of P and dS stay the zeros they start as: two
       // of them in the last quarter of every tile of three heads had its warps mask every element, 1.7 k cycles a tile
-      // behind the others.  What they leave in P and dS is written over with zeros, since zeros times a key that is not finite
-      // are NaN (8 x 4096 tokens, 12 heads of 64: selection 521 us with or without, compression 72 -> 74; zeroed in
-      // registers 532 and 78)
+      // behind the others
       const int lo_h = min(max(lo - half * 32, 0), 32), hi_h = min(max(hi + 1 - half * 32, 0), 32);
       uint32_t attended = (hi_h == 32 ? ~0u : (1u << hi_h) - 1u) & ~((lo_h == 32) ? ~0u : (1u << lo_h) - 1u);
       if (!(groups & 1u)) attended &= 0xffff0000u;
       if (!(groups & 2u)) attended &= 0x0000ffffu;
-      const bool there = row_slot_ok && (p.kind != 2 || t_cur >= 0);
-      if (!there) attended = ~0u;
+      if (!row_slot_ok) attended = ~0u;
       const bool all_cols = attended == ~0u && !repeats;
       float times[2] = {1.f, 1.f};                   // how often the row's list names the blocks of its column groups
       if (kThreeTerm && repeats && t_cur >= 0) {
@@ -1191,22 +1192,16 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
                   v[2 * e] = __float_as_uint(__uint_as_float(v[2 * e]) - __uint_as_float(b[e] << 16));
                   v[2 * e + 1] = __float_as_uint(__uint_as_float(v[2 * e + 1]) - __uint_as_float(b[e] & 0xffff0000u));
                 }
-                st_shared_v4(at + term * 2 * kPBytes, b[0], b[1], b[2], b[3]);
+                if (row_slot_ok) st_shared_v4(at + term * 2 * kPBytes, b[0], b[1], b[2], b[3]);
               }
             };
             terms(p_row + chunk16, rs + k4 * 8);
             terms(ds_row + chunk16, rp + k4 * 8);
             continue;
           }
-          st_shared_v4(p_row + chunk16, pp[k4 * 4], pp[k4 * 4 + 1], pp[k4 * 4 + 2], pp[k4 * 4 + 3]);
-          st_shared_v4(ds_row + chunk16, pd[k4 * 4], pd[k4 * 4 + 1], pd[k4 * 4 + 2], pd[k4 * 4 + 3]);
-        }
-        if (!there) {
-#pragma unroll
-          for (int k4 = 0; k4 < 4 * L::kTerms; ++k4) {
-            const uint32_t at = ((uint32_t)((half * 4 + (k4 & 3)) ^ (row & 7)) << 4) + (k4 >> 2) * 2 * kPBytes;
-            st_shared_v4(p_row + at, 0u, 0u, 0u, 0u);
-            st_shared_v4(ds_row + at, 0u, 0u, 0u, 0u);
+          if (row_slot_ok) {
+            st_shared_v4(p_row + chunk16, pp[k4 * 4], pp[k4 * 4 + 1], pp[k4 * 4 + 2], pp[k4 * 4 + 3]);
+            st_shared_v4(ds_row + chunk16, pd[k4 * 4], pd[k4 * 4 + 1], pd[k4 * 4 + 2], pd[k4 * 4 + 3]);
           }
         }
       }
@@ -1259,18 +1254,19 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
           const uint32_t rbase = smem_u32(stage) + (col0 >> 5) * (kRows * 128) + row * 128;
 #pragma unroll
           for (int c = 0; c < 8; ++c)
-            st_shared_v4(rbase + (((uint32_t)c ^ (uint32_t)(row & 7)) << 4), r32[c * 4], r32[c * 4 + 1], r32[c * 4 + 2],
-                         r32[c * 4 + 3]);
+            if (row_slot_ok)
+              st_shared_v4(rbase + (((uint32_t)c ^ (uint32_t)(row & 7)) << 4), r32[c * 4], r32[c * 4 + 1], r32[c * 4 + 2], r32[c * 4 + 3]);
           continue;
         }
 #pragma unroll
         for (int v4 = 0; v4 < 4; ++v4) {
           const uint32_t ch = (uint32_t)((col0 >> 3) + v4);
-          st_shared_v4(smem_u32(stage) + (ch >> 3) * (kRows * 128) + row * 128 + (((ch & 7) ^ (row & 7)) << 4),
-                       pack_bf16(__uint_as_float(r32[v4 * 8 + 0]), __uint_as_float(r32[v4 * 8 + 1])),
-                       pack_bf16(__uint_as_float(r32[v4 * 8 + 2]), __uint_as_float(r32[v4 * 8 + 3])),
-                       pack_bf16(__uint_as_float(r32[v4 * 8 + 4]), __uint_as_float(r32[v4 * 8 + 5])),
-                       pack_bf16(__uint_as_float(r32[v4 * 8 + 6]), __uint_as_float(r32[v4 * 8 + 7])));
+          if (row_slot_ok)
+            st_shared_v4(smem_u32(stage) + (ch >> 3) * (kRows * 128) + row * 128 + (((ch & 7) ^ (row & 7)) << 4),
+                         pack_bf16(__uint_as_float(r32[v4 * 8 + 0]), __uint_as_float(r32[v4 * 8 + 1])),
+                         pack_bf16(__uint_as_float(r32[v4 * 8 + 2]), __uint_as_float(r32[v4 * 8 + 3])),
+                         pack_bf16(__uint_as_float(r32[v4 * 8 + 4]), __uint_as_float(r32[v4 * 8 + 5])),
+                         pack_bf16(__uint_as_float(r32[v4 * 8 + 6]), __uint_as_float(r32[v4 * 8 + 7])));
         }
       }
       const bool full_tile = (i + 1) * p.nq <= n_q;
