@@ -114,6 +114,11 @@ __device__ __forceinline__ void chain_go() { asm volatile("griddepcontrol.launch
 // __restrict__ argument) takes its data not to change while the kernel is on the GPU, which includes the time before.
 __device__ __forceinline__ int32_t ld_plain(const int32_t* p) { int32_t v; asm volatile("ld.global.s32 %0, [%1];" : "=r"(v) : "l"(p)); return v; }
 __device__ __forceinline__ float ld_plain(const float* p) { float v; asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p)); return v; }
+__device__ __forceinline__ uint4 ld_plain(const uint4* p) {
+  uint4 v;
+  asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
 __device__ __forceinline__ unsigned long long ld_plain(const unsigned long long* p) {
   unsigned long long v;
   asm volatile("ld.global.u64 %0, [%1];" : "=l"(v) : "l"(p));

@@ -16,16 +16,16 @@ namespace nsa {
 namespace tc {
 
 // How often a list of S blocks names block `blk`.
-__device__ __forceinline__ int times_listed(const int32_t* __restrict__ row, int S, int blk) {
+__device__ __forceinline__ int times_listed(const int32_t* row, int S, int blk) {
   int n = 0;
 #pragma unroll 1
-  for (int s = 0; s < S; ++s) n += __ldg(row + s) == blk;
+  for (int s = 0; s < S; ++s) n += ld_plain(row + s) == blk;
   return n;
 }
 
 // eight bf16 of an aligned row as floats
-__device__ __forceinline__ void load8_row(const __nv_bfloat16* __restrict__ p, float* f) {
-  const uint4 u = __ldg(reinterpret_cast<const uint4*>(p));
+__device__ __forceinline__ void load8_row(const __nv_bfloat16* p, float* f) {
+  const uint4 u = ld_plain(reinterpret_cast<const uint4*>(p));
   const uint32_t w[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
   for (int e = 0; e < 4; ++e) {
@@ -35,7 +35,7 @@ __device__ __forceinline__ void load8_row(const __nv_bfloat16* __restrict__ p, f
 }
 
 template <int D>
-__device__ __forceinline__ float dot_rows(const __nv_bfloat16* __restrict__ a, const __nv_bfloat16* __restrict__ b) {
+__device__ __forceinline__ float dot_rows(const __nv_bfloat16* a, const __nv_bfloat16* b) {
   float acc[2] = {0.f, 0.f};
 #pragma unroll 2
   for (int d = 0; d < D; d += 8) {
@@ -49,7 +49,7 @@ __device__ __forceinline__ float dot_rows(const __nv_bfloat16* __restrict__ a, c
 }
 
 // acc += w * (32 columns of a row)
-__device__ __forceinline__ void add32_row(float w, const __nv_bfloat16* __restrict__ row, float* acc) {
+__device__ __forceinline__ void add32_row(float w, const __nv_bfloat16* row, float* acc) {
 #pragma unroll
   for (int c = 0; c < 32; c += 8) {
     float x[8];
@@ -72,7 +72,7 @@ __device__ __noinline__ void sel_row_forward(const __nv_bfloat16* q, const __nv_
     for (int e = 0; e < 32; ++e) acc[e] = 0.f;
 #pragma unroll 1
     for (int s = 0; s < S; ++s) {
-      const int blk = __ldg(list + s);
+      const int blk = ld_plain(list + s);
       if (blk < 0 || (long long)blk * block_size > t) continue;
       const int last = min(t, (blk + 1) * block_size - 1);
 #pragma unroll 1

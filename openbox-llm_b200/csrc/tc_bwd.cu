@@ -606,7 +606,7 @@ __device__ __noinline__ void sel_tile_dkdv(const BwdArgs& p, float* acc, int bh,
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int b = bh / p.Hkv, hkv = bh % p.Hkv, key0 = j * kKeys, c0 = 4 * warp;
   if (c0 < kKeys) {
-    const bool repeats = __ldg(&p.plan.hdr->repeats) != 0ull;
+    const bool repeats = ld_plain(&p.plan.hdr->repeats) != 0ull;
     float k[4][N], v[4][N], dk[4][N], dv[4][N];
 #pragma unroll
     for (int c = 0; c < 4; ++c)
@@ -625,10 +625,10 @@ __device__ __noinline__ void sel_tile_dkdv(const BwdArgs& p, float* acc, int bh,
       // a lane fetches what 32 rows need before their vectors: one trip to memory for them all
       if ((r & 31) == 0) {
         const int rr = min(r + lane, n_rows - 1);
-        pair_l = __ldg(p.plan.pairs + pair_first + rr / p.G);
+        pair_l = ld_plain(p.plan.pairs + pair_first + rr / p.G);
         row_l = (b * p.Hq + hkv * p.G + rr % p.G) * (long long)p.T + (pair_l & (int)kPairPosMask);
-        lse2_l = __ldg(p.lse + row_l) * kLog2e - (p.row_scale ? __log2f(__ldg(p.row_scale + row_l)) : 0.f);
-        delta_l = __ldg(p.delta + row_l);
+        lse2_l = ld_plain(p.lse + row_l) * kLog2e - (p.row_scale ? __log2f(ld_plain(p.row_scale + row_l)) : 0.f);
+        delta_l = ld_plain(p.delta + row_l);
       }
       const int pair = __shfl_sync(0xffffffffu, pair_l, r & 31);
       const int t = pair & (int)kPairPosMask;

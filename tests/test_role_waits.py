@@ -22,3 +22,18 @@ def test_a_warp_that_issues_as_one_waits_as_one(name):
         for line in role.splitlines():
             if re.search(r"\bmbar_(try_|test_)?wait\(", line):
                 assert "__all_sync(" in line or "bar_kv" in line or "bar_drain" in line, line
+
+
+READ_ONLY_PATH = r"__ldg\(|ldg_\w+_now\(|ld\.global\.nc|\bconst \w+\s*\* __restrict__"
+
+
+@pytest.mark.parametrize("name", ["sel_row.cuh", "sel_plan.cu", "tc_score.cu", "tc.cu", "tc_fwdpair.cu", "tc_bwd.cu"])
+def test_chained_kernels_read_by_plain_loads(name):
+    """A kernel that is on the GPU before the one ahead has ended reads nothing through the read-only path, which takes its data
+    not to change meanwhile.  Two kernels of the backward are launched plainly."""
+    functions = re.split(r"\n(?=(?:template <[^\n]*>\n)?(?:__global__|__device__) )", _source(name))
+    plain = [f for f in functions if re.search(r"^(tc_bwd_kernel|cmp_chunks_kernel)\(", f, re.M)]
+    assert len(plain) == (2 if name == "tc_bwd.cu" else 0)
+    for f in functions:
+        if f not in plain:
+            assert not re.search(READ_ONLY_PATH, f), re.search(READ_ONLY_PATH, f).group(0)
