@@ -49,3 +49,29 @@ def test_one_behind_the_other_and_each_alone(B, Hq, Hkv, T, D, S):
             assert torch.equal(a, b)
         assert torch.equal(whole[k][0], want[k % 4][0]) and torch.equal(whole[k][1], want[k % 4][1])
     assert nsa.lib().nsa_device_status(None) == 0
+
+
+@pytest.mark.parametrize("B,Hq,Hkv,T,D,S", SHAPES)
+def test_the_backward_of_selection_behind_one_another(B, Hq, Hkv, T, D, S):
+    """Row statistics, plan, backward and dQ sum in a row, of different inputs, against passes that each start on an idle GPU: dq bit for
+    bit, dk and dv up to the order of fp32 adds (2^-7 of the largest entry)."""
+    nsa = pkg()
+    ins = [_inputs(B, Hq, Hkv, T, D, seed=s) for s in range(4)]
+    g = torch.Generator("cuda").manual_seed(9)
+    idx = [torch.randint(-1, (T + 63) // 64, (B, Hkv, T, S), generator=g, device="cuda", dtype=torch.int32) for _ in ins]
+
+    def grads(k):
+        q, _, _, ks, vs = (x.detach().requires_grad_(True) for x in ins[k][:5])
+        return torch.autograd.grad(nsa.selection_attn_triton(q, ks, vs, idx[k], 64), (q, ks, vs), ins[(k + 1) % 4][0].detach())
+
+    want = []
+    for k in range(4):
+        torch.cuda.synchronize()
+        want.append(grads(k))
+    torch.cuda.synchronize()
+    got = [grads(k % 4) for k in range(16)]
+    for k in range(16):
+        assert torch.equal(got[k][0], want[k % 4][0])
+        for a, b in zip(got[k][1:], want[k % 4][1:]):
+            assert (a.float() - b.float()).abs().max() <= 2.0 ** -7 * b.float().abs().max()
+    assert nsa.lib().nsa_device_status(None) == 0

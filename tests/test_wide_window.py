@@ -2,14 +2,15 @@
 row tiles and windows.
 
 The kernel serves windows with more tiles of 64 keys than the GPU has SMs, so the sequences here are short and many.
-P, dS and the partial rows of dQ are bf16 (relative 2^-9 each), everything else fp32: relative L2 of 2^-8 on dv, dk and
-dq, each with a rounding of its own to bf16 (2^-9), within 8e-3."""
+What is rounded to bf16 (relative 2^-9 at most) on the way to a gradient: P, O in delta, dS, the partial rows of dQ, the gradient itself,
+four of them for each of dq, dk and dv at most, independent of one another: relative L2 of 2 x 2^-9.  Measured: 1.7e-3 to 2.9e-3."""
 import importlib
 
 import pytest
 import torch
 
 nsa = importlib.import_module("openbox-llm_b200")
+TOL = 2 * 2.0 ** -9
 pytestmark = pytest.mark.gpu
 
 
@@ -57,8 +58,13 @@ def test_against_64_bits(B, Hq, Hkv, T, D, window):
             s += torch.stack([(d * d).sum(), (y * y).sum()])
     for name, s in zip(("dq", "dk", "dv"), sums):
         e = (s[0] / s[1]).sqrt().item()
-        # a window of 1 has p = 1 and dS = 0 but for rounding: dq and dk have no scale of their own
-        assert e <= 8e-3 or (window == 1 and name != "dv"), (name, e)
+        assert e <= TOL or (window == 1 and name != "dv"), (name, e)
+    if window == 1:
+        # p = 1 and O = V: dP = delta, two fp32 sums of the same D products, each off by D 2^-23 of their absolute sum at most,
+        # in any order.  That is all there is in dS, and dq and dk are dS times a row of k and G rows of q.
+        G = Hq // Hkv
+        ds = 2 * D * 2.0 ** -23 * D ** -0.5 * (do.float() * v.float().repeat_interleave(G, 1)).abs().sum(-1).max().item() * 1.01
+        assert got[0].abs().max().item() <= ds * k.abs().max().item() and got[1].abs().max().item() <= G * ds * q.abs().max().item()
     assert all(torch.isfinite(x.float()).all() for x in got)
 
 
@@ -78,7 +84,11 @@ def test_gates_that_underflow():
     assert all(torch.isfinite(x.float()).all() for x in got)
     gate = torch.sigmoid(logits[..., 2].double())
     _, dk, dv = reference(q[:4], kv[4][:4], kv[5][:4], do[:4], 128, gate[:4])
-    assert rel(got[5][:4], dk) <= 8e-3 and rel(got[6][:4], dv) <= 8e-3
+    assert rel(got[5][:4], dk) <= TOL and rel(got[6][:4], dv) <= TOL
+    # dq of these rows is that of the other two branches: bit for bit the same beside other keys in the window
+    others = leaves[:5] + [torch.flip(x.detach(), [2]).requires_grad_(True) for x in leaves[5:7]] + leaves[7:]
+    dq = torch.autograd.grad(nsa.nsa_fused_forward(*others, idx, 64, 128), others[0], do)[0]
+    assert torch.equal(dq[:, :, ::3], got[0][:, :, ::3]) and not torch.equal(dq[:, :, 1::3], got[0][:, :, 1::3])
 
 
 def test_gradients_that_start_anywhere():
