@@ -472,21 +472,8 @@ tc_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     const uint32_t ds_row0 = smem_u32(sDs) + half * kSlabBytes + kr * 128;
     // Where K and V are finite, P = 0 masks dS = P * (dP - delta) as well, and rows past nq * G, zeros in Q and dO, may count
     // as attended (as others they would have these warps mask every element of every tile).  A K or V that is infinite
-    // or NaN spoils dS of rows that do not attend it, and rows that are not there.  The look at the tile hides behind
-    // the first S.
-    bool odd = false;
-    if (mbar_wait(bar_kv, 0, p.status, s_abort, 32)) {
-      __nv_bfloat162 z(0.f, 0.f);                    // x * 0: 0 or NaN
-#pragma unroll 8
-      for (int i = tid; i < 2 * L::kKVBytes / 16; i += 256) {        // (V lies behind K)
-        const uint4 u = reinterpret_cast<const uint4*>(sK)[i];
-        const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-        for (int e = 0; e < 4; ++e) z = __hfma2(reinterpret_cast<const __nv_bfloat162&>(w[e]), __nv_bfloat162(0.f, 0.f), z);
-      }
-      odd = (reinterpret_cast<const uint32_t&>(z) & 0x7fff7fffu) != 0u;
-    }
-    odd = group_or(3, 256, odd);
+    // or NaN spoils dS of rows that do not attend it, and rows that are not there.
+    const bool odd = group_or(3, 384, 0);
     if (odd) masked_row_tiles<D>(p, smem, tmem);
     for (int k = odd ? n_tiles : 0; k < n_tiles; ++k) {
       const int qi0 = k * p.nq, t0 = t_lo + qi0;
@@ -565,6 +552,21 @@ tc_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     const int row = quad * 32 + lane;
     const int slot = j % p.n_slots;
     const uint32_t lane_base = tmem + ((uint32_t)(quad * 32) << 16) + L::kColDQ;
+    // the dQ warps have nothing to do yet: they look at the tile's K and V for the compute warps, behind the first S (by the
+    // compute warps themselves: 8192 tokens of 16 / 2 heads of 128 123 us instead of 120; 119 without)
+    bool odd = false;
+    if (mbar_wait(bar_kv, 0, p.status, s_abort, 32)) {
+      __nv_bfloat162 z(0.f, 0.f);                    // x * 0: 0 or NaN
+#pragma unroll 8
+      for (int i = lt; i < 2 * L::kKVBytes / 16; i += 128) {        // (V lies behind K)
+        const uint4 u = reinterpret_cast<const uint4*>(sK)[i];
+        const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) z = __hfma2(reinterpret_cast<const __nv_bfloat162&>(w[e]), __nv_bfloat162(0.f, 0.f), z);
+      }
+      odd = (reinterpret_cast<const uint32_t&>(z) & 0x7fff7fffu) != 0u;
+    }
+    group_or(3, 384, odd);
     for (int k = 0; k < n_tiles; ++k) {
       uint8_t* stage = sOut;
       const bool ok = mbar_wait(acc_full, k & 1, p.status, s_abort, 128);
