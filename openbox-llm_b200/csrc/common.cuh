@@ -102,7 +102,9 @@ struct KernelScope {
 // from the same SMs.
 // Measured (us per call, one after the other -> chained): forward of the operator at T = 512 44.8 -> 39.5, at
 // T = 1024 53.1 -> 48.1, selection at T = 8192 forward and backward 362 -> 339 (350 with the backward's kernels
-// one after the other), three branches over given lists at T = 4096 94 -> 88.8 (alone in a graph, where the launches cost nothing, 80 -> 84).
+// one after the other), three branches over given lists at T = 4096 94 -> 88.8.
+// From a graph, where the launches cost nothing, over given lists: T = 4096 85 us before and now (80 with plain launches of the
+// present kernels), T = 5000 117 -> 106, 2 x 1000 33.5 -> 29.3, 2048 at heads of 128 59.7 -> 55.7.
 // Plain launches stay where an early CTA takes a place that another stream's kernel would fill: the block-outer
 // selection kernel (chained 98.6 where it is 89.3 plain) and, over given lists, the attention over pooled keys (T = 3000
 // 91 against 86.3), both beside the window's kernel.  With lists of the scorer the window is launched ahead of the
@@ -112,6 +114,7 @@ __device__ __forceinline__ void chain_go() { asm volatile("griddepcontrol.launch
 
 // What the kernel ahead writes is read by plain loads, which stay behind the wait: the read-only path (__ldg, a const
 // __restrict__ argument) takes its data not to change while the kernel is on the GPU, which includes the time before.
+// So do the scalar rows of sel_row.cuh, which run in chained kernels.
 __device__ __forceinline__ int32_t ld_plain(const int32_t* p) { int32_t v; asm volatile("ld.global.s32 %0, [%1];" : "=r"(v) : "l"(p)); return v; }
 __device__ __forceinline__ float ld_plain(const float* p) { float v; asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p)); return v; }
 __device__ __forceinline__ uint4 ld_plain(const uint4* p) {

@@ -20,10 +20,10 @@
 // tiles that its query attends, a K dQ of the rows that share one of its steps of 16 keys: 0 x inf in a product is NaN.
 //
 // What bounds it: at D = 128 the chain S -> p -> dP -> dS of one row tile, whose S and dP fill what TMEM dV and dK leave
-// (4.8 k cycles a row tile, the MMAs alone 2.7 k); at D = 64 the MMAs (4.2 k against 1.8 k by themselves: the warp that
+// (4.8 k cycles a row tile, the MMAs alone 2.7 k); at D = 64 the MMAs (4.2 k against 2.2 k by themselves, 33 of them: the warp that
 // issues them shares its scheduler with compute warps, and their operands share shared memory with dS and the tiles
-// going in and out).  8 x 32768 tokens, 16 heads of 128, window 512: 3.5 ms, 5.2 with tiles of 64 keys; 8 x 4096, 12 heads
-// of 64: 264 us, 428.
+// going in and out).  8 x 32768 tokens, 16 heads of 128, window 512: 3.6 ms, 5.2 with tiles of 64 keys; 8 x 4096, 12 heads
+// of 64: 267 us, 428.
 #include <type_traits>
 
 #include "tc_bwd_wide.cuh"

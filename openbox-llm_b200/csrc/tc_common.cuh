@@ -61,12 +61,13 @@ __device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
   return ok != 0;
 }
 
-// Bounded wait.  When the limit runs out the kernel raises the device status word, marks the
-// CTA as aborted and every later wait of the CTA returns at once, so the grid drains; other
-// CTAs notice the status word the next time one of their waits is slow.
-// Returns true when the phase completed, false when the wait was given up.  The abort flag is read at every 64th look
-// only: while the MMAs fetch operands from shared memory a load of the flag takes some 220 cycles (its bandwidth is
-// theirs first), a look at the barrier 30.
+// Bounded wait.  When the limit runs out the kernel raises the device status word and marks the
+// CTA as aborted; other CTAs notice the status word the next time one of their waits is slow.
+// Returns true when the phase completed, false when the wait was given up.  A wait of an aborted CTA whose phase is
+// complete returns true all the same, so that what is under way may still end; one
+// whose phase is not is given up at its 64th look, and with the first of these a role ends.  So the grid drains.
+// The flag is read at every 64th look only: while the MMAs fetch operands from shared memory a load of it takes
+// some 220 cycles (its bandwidth is theirs first), a look at the barrier 30.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* status,
                                           volatile int* s_abort, int code) {
   if (mbar_try_wait(bar, parity)) return true;
