@@ -942,9 +942,10 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
         for (int r = 0; r < kRounds; ++r) tq[r] = tq_of(k + 1, box_of(r));
       }
     }
-    if (*s_abort && pw == 0 && lane == 0) {
-      // give-up path: the loads still on their way into this CTA's shared memory land (bounded
-      // wait on the last phase of each stage) before the CTA ends
+    if (lane == 0) {
+      // The loads that this warp has sent land before it goes to the teardown barrier (bounded wait on the last phase of
+      // each stage), whether the CTA has given up, gives up later or not: none may be on its way when the CTA ends.
+      // A stage that not every warp has sent its boxes of, or the first has not armed, runs into the limit
       mbar_wait_drain(bar_kv, 0);
       for (int h = max(0, issued - 2 * kStages); h < issued; ++h)
         mbar_wait_drain((h & 1 ? q_full : do_full) + (h >> 1) % kStages, ((h >> 1) / kStages) & 1);

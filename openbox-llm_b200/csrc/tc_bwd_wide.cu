@@ -284,11 +284,9 @@ tc_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
           tma_load_3d(dst + s * kSlabBytes, is_q ? &tm_q : &tm_do, full + st, s * 64, head0, t_lo + k * p.nq);
         issued = k + 1;
       }
-      if (*s_abort) {
-        // give-up path: the loads still on their way land (bounded wait) before the CTA ends
-        if (is_q) mbar_wait_drain(bar_kv, 0);
-        for (int k = max(0, issued - kStages); k < issued; ++k) mbar_wait_drain(full + k % kStages, (k / kStages) & 1);
-      }
+      // the loads land (bounded wait) before the teardown barrier, whether the CTA has given up or gives up later
+      mbar_wait_drain(bar_kv, 0);
+      for (int k = max(0, issued - kStages); k < issued; ++k) mbar_wait_drain(full + k % kStages, (k / kStages) & 1);
     }
   } else if (warp == 13) {
     // ---- row statistics of every tile: lse for S, delta for dP, as the terms that one more step of 16 adds to the

@@ -89,7 +89,6 @@ tc_fwdpair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
   uint64_t* bar_drain = bars + 15;
   uint32_t* s_tmem = (uint32_t*)(bars + 16);
   volatile int* s_abort = (volatile int*)(s_tmem + 1);
-  volatile int* s_issued = (volatile int*)(s_tmem + 2);   // row tiles whose gather has been issued
   uint32_t* s_prow = (uint32_t*)(s_tmem + 4);             // [128] partial row of each tile row (ragged tile)
 
   if (!prefer_pairs(p.plan.hdr, p.nq_union, p.force)) return;
@@ -112,7 +111,6 @@ tc_fwdpair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
       bad = 1;
     }
     *s_abort = bad;
-    *s_issued = 0;
     mbar_init(bar_kv, 1);
     for (int s = 0; s < kPairQStages; ++s) { mbar_init(q_full + s, 1); mbar_init(q_empty + s, 1); }
     for (int s = 0; s < 2; ++s) {
@@ -165,13 +163,14 @@ tc_fwdpair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
       return (o < n_ops && qi < n_q) ? ldg_s32_now(p.plan.pairs + pair_base + qi) : p.T;
     };
     int tq0 = tq_of(0, o0), tq1 = tq_of(0, o1);
+    int issued = 0;                                  // row tiles whose boxes this warp has sent
     for (int k = 0; k < n_tiles; ++k) {
       const int st = k % kPairQStages;
       const bool ok = mbar_wait(q_empty + st, ((k / kPairQStages) + 1) & 1, p.status, s_abort, 512);
       const int tn0 = k + 1 < n_tiles ? tq_of(k + 1, o0) : p.T;          // next tile's positions, ahead
       const int tn1 = k + 1 < n_tiles ? tq_of(k + 1, o1) : p.T;
       if (!__all_sync(0xffffffffu, ok)) break;               // the whole warp leaves together
-      if (pw == 0 && lane == 0) { mbar_expect_tx(q_full + st, gather_bytes); *s_issued = k + 1; }
+      if (pw == 0 && lane == 0) mbar_expect_tx(q_full + st, gather_bytes);
       __syncwarp();
       uint8_t* dst = sQ + st * kQBytes;
 #pragma unroll
@@ -189,6 +188,13 @@ tc_fwdpair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
         }
       }
       tq0 = tn0; tq1 = tn1;
+      issued = k + 1;
+    }
+    if (lane == 0) {
+      // the loads land (bounded wait) before the teardown barrier, whether the CTA has given up or gives up later; a stage that not
+      // every warp has sent its boxes of runs into the limit
+      mbar_wait_drain(bar_kv, 0);
+      for (int k = max(0, issued - kPairQStages); k < issued; ++k) mbar_wait_drain(q_full + k % kPairQStages, (k / kPairQStages) & 1);
     }
   } else if (warp == 12 + kPairProducers) {
     // ---- MMA issuer ------------------------------------------------------------------------
@@ -367,15 +373,7 @@ tc_fwdpair_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
     if (et == 0) bulk_wait_all();
   }
 
-  // ---- teardown: every gather that was issued has landed, the tensor pipe is idle -----------------
-  __syncthreads();
-  if (*s_abort && tid == 0) {
-    const int issued = *s_issued;
-    for (int k = max(0, issued - kPairQStages); k < issued; ++k) {
-      // bounded: a gather that never lands was what made the CTA give up in the first place
-      mbar_wait_drain(q_full + k % kPairQStages, (k / kPairQStages) & 1);
-    }
-  }
+  // ---- teardown: every load that was sent has landed, the tensor pipe is idle -----------------
   tc_fence_before();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tmem, kTmemCols);

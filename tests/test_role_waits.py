@@ -24,6 +24,17 @@ def test_a_warp_that_issues_as_one_waits_as_one(name):
                 assert "__all_sync(" in line or "bar_kv" in line or "bar_drain" in line, line
 
 
+
+@pytest.mark.parametrize("name", ["tc_fwdpair_kernel.cu", "tc_bwd.cu", "tc_bwd_wide.cu"])
+def test_every_producer_waits_for_its_own_loads(name):
+    """No load is on its way into a CTA's shared memory when the CTA ends: each warp that sends some waits (bounded) until they
+    have landed, on its way to the teardown barrier, whoever gives up and whenever."""
+    roles = [part for part in re.split(r"\n\s*// ---- ", _source(name)) if part.startswith("producers")]
+    assert len(roles) == 1
+    assert "mbar_wait_drain(bar_kv, 0);" in roles[0] and roles[0].count("mbar_wait_drain(") == 2
+    assert not re.search(r"if \([^\n]*(s_abort|pw == 0)[^\n]*\{\n[^{}]*mbar_wait_drain", roles[0])
+
+
 READ_ONLY_PATH = r"__ldg\(|ldg_\w+_now\(|ld\.global\.nc|\bconst \w+\s*\* __restrict__"
 
 
