@@ -315,6 +315,9 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         auto ready = [&](uint64_t* bar, uint32_t parity, int code) -> bool {
           return __all_sync(0xffffffffu, mbar_wait(bar, parity, p.status, s_abort, code));
         };
+        auto both = [&](uint64_t* a, uint32_t pa, int ca, uint64_t* b, uint32_t pb, int cb) -> bool {    // one vote
+          return __all_sync(0xffffffffu, mbar_wait(a, pa, p.status, s_abort, ca) && mbar_wait(b, pb, p.status, s_abort, cb));
+        };
         auto issue_s = [&](int cc, bool last) {   // S = Q K^T of running key tile cc
           const int st = cc % kStages;
           const uint32_t qa = desc_lo_kmajor(smem_u32(sQ)), ka = desc_lo_kmajor(smem_u32(sK + st * L::kKVBytes));
@@ -331,7 +334,7 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         for (int w = w0; ok && w < w_end; w += gridDim.x) {
           const Tile x = tile_of(w);
           if (x.n_tiles == 0) continue;
-          ok = ready(bar_q, it & 1, 1) && ready(bar_k + c % kStages, (c / kStages) & 1, 2);
+          ok = both(bar_q, it & 1, 1, bar_k + c % kStages, (c / kStages) & 1, 2);
           // An S MMA overwrites the P of two key tiles back: that tile's PV has to be complete (MMAs of
           // different shapes and operand sources are not ordered by their issue).  Here every earlier
           // one is waited for; the threads that write the last row tile's output wait for it as well.
@@ -341,14 +344,15 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           issue_s(c, x.n_tiles == 1);
           for (int i = 0; i < x.n_tiles; ++i, ++c) {
             if (i + 1 < x.n_tiles) {
-              ok = ready(bar_k + (c + 1) % kStages, ((c + 1) / kStages) & 1, 2);
-              if (ok && i > 0) ok = ready(bar_o + ((c - 1) & 1), ((c - 1) >> 1) & 1, 0x2000);
+              uint64_t* k_next = bar_k + (c + 1) % kStages;
+              ok = i > 0 ? both(k_next, ((c + 1) / kStages) & 1, 2, bar_o + ((c - 1) & 1), ((c - 1) >> 1) & 1, 0x2000)
+                         : ready(k_next, ((c + 1) / kStages) & 1, 2);
               if (!ok) break;
               tc_fence_after();
               issue_s(c + 1, i + 2 == x.n_tiles);
             }
             const int st = c % kStages;
-            ok = ready(bar_p + (c & 1), (c >> 1) & 1, 0x2000) && ready(bar_v + st, (c / kStages) & 1, 16);
+            ok = both(bar_p + (c & 1), (c >> 1) & 1, 0x2000, bar_v + st, (c / kStages) & 1, 16);
             if (!ok) break;
             tc_fence_after();
             const uint32_t va = desc_lo_mnmajor(smem_u32(sV + st * L::kKVBytes), kKeys * 128);   // O (+)= P V
