@@ -11,7 +11,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(CSRC, "libnsa_b200.so")
 EXT = os.path.join(CSRC, "_nsa_torch.so")
-SOURCES = ["api.cu", "simt.cu", "simt_tile.cu", "aux.cu", "pool.cu", "sel_plan.cu", "tc.cu", "tc_bwd.cu", "tc_bwd_wide.cu", "tc_score.cu", "tc_fwdpair.cu", "tc_fwdpair_kernel.cu", "op.cu", "optim.cu"]
+SOURCES = ["api.cu", "simt.cu", "simt_tile.cu", "f32_tile.cu", "aux.cu", "pool.cu", "sel_plan.cu", "tc.cu", "tc_bwd.cu", "tc_bwd_wide.cu", "tc_score.cu", "tc_fwdpair.cu", "tc_fwdpair_kernel.cu", "op.cu", "optim.cu"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "-DNSA_B200",
               "-Xptxas", "-v"]

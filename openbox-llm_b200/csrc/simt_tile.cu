@@ -1,5 +1,5 @@
-// CUDA-core attention on tiles of 64 rows x 64 keys, fp32 arithmetic throughout: the fp32 path, and
-// bf16 shapes the tcgen05 kernels do not take (D of 16 / 32, one query head per kv head, other
+// CUDA-core attention on tiles of 64 rows x 64 keys, fp32 arithmetic throughout: the fp32 path (D of 64: f32_tile.cu, by the
+// same rules), and bf16 shapes the tcgen05 kernels do not take (D of 16 / 32, one query head per kv head, other
 // block sizes).  A row is one (query token, query head); the rows of a unit are numbered token-major
 // (row = t * G + head), so a tile's rows share their K / V tiles whatever the group size.
 //   window, compression   the tile walks the keys its rows can see, 64 at a time
@@ -9,22 +9,19 @@
 // patch of every product and reads its operands from shared memory as 16-byte vectors, 5 to 10 FFMAs
 // per word.  The row-per-warp kernels of simt.cu re-read K and V from L1 for every row and, in
 // backward, add every key's gradient by its own atomics; here one vector atomic per (row tile, key)
-// does, and window / compression / selection at B=1, T=2048, 8 heads of 64 in fp32 go from
+// does, and window / compression / selection at B=1, T=2048, 8 heads of 64 in fp32 went from
 // 1.6 / 3.8 ms (forward / backward, three branches) to 0.42 / 0.68 ms.
 // A row tile is one chain through its key tiles: where tiles are few a cluster of 2 or 4 CTAs shares
 // it, every CTA its key tiles, and adds up O (by its maximum) or dQ through distributed shared memory in
 // rank order; at that size selection goes from 299 / 453 us to 187 / 353.
 #include "cluster.cuh"
-#include "common.cuh"
+#include "simt_tile.cuh"
 
 namespace nsa {
 namespace {
 
-constexpr int kR = 64;           // rows per tile
-constexpr int kK = 64;           // keys per tile
 constexpr int kPad = 4;          // floats: 16-byte reads of 8 neighbouring rows cover all banks
 constexpr int kPLd = kK + kPad;
-constexpr int kMaxBlocks = 1024; // blocks a selection tile can tell apart
 const char* const kFwdNames[3] = {"simt_tile_fwd_win", "simt_tile_fwd_cmp", "simt_tile_fwd_slc"};
 const char* const kBwdNames[3] = {"simt_tile_bwd_win", "simt_tile_bwd_cmp", "simt_tile_bwd_slc"};
 
@@ -84,105 +81,6 @@ template <int C, typename T> __device__ __forceinline__ void store_cols(T* row, 
   for (int v = 0; v < C; ++v) store_val(row + col_of<C>(tx, v), f[v]);
 }
 
-// What a tile's rows attend: keys [first, first + n) of the unit, or the union of listed blocks.
-struct TileKeys {
-  int first, n;            // window / compression: first key and their number; selection: 0, keys of the union
-};
-
-struct SelList {           // selection only, in shared memory: as many blocks as the sequence has
-  unsigned long long* mask;   // queries of the tile that list a block
-  int* n_list;
-  int* repeats;               // not 0: some query lists a block more than once
-  uint16_t* list;             // the listed blocks, ascending
-};
-__host__ __device__ __forceinline__ int sel_blocks(const AttnArgs& a) { return (a.T + a.block_size - 1) / a.block_size; }
-__device__ __forceinline__ SelList sel_list(const AttnArgs& a, void* at) {
-  SelList s;
-  s.mask = (unsigned long long*)at;
-  s.n_list = (int*)(s.mask + (a.kind == 2 ? sel_blocks(a) : 0));
-  s.repeats = s.n_list + 1;
-  s.list = (uint16_t*)(s.n_list + 2);
-  return s;
-}
-
-// shared memory of one tile's key bookkeeping, double buffered: the next tile is fetched ahead
-struct KeyInfo {
-  int tok[2][kK];                        // token (or summary) of a key, -1: none
-  unsigned long long mask[2][kK];        // selection: queries that list its block
-};
-
-template <int kThreads>
-__device__ __forceinline__ TileKeys tile_keys(const AttnArgs& a, int bh, int t_first, int t_last, const SelList& sl) {
-  TileKeys k;
-  k.first = 0; k.n = 0;
-  if (a.kind == 0) {
-    k.first = max(0, t_first - a.window + 1);
-    k.n = max(0, min(t_last, a.Lk - 1) - k.first + 1);
-  } else if (a.kind == 1) {
-    k.n = cmp_visible(t_last, a.block_size, a.window, a.Lk);   // compression: window holds the stride
-  } else {
-    const int n_blk = (t_last + a.block_size) / a.block_size;   // blocks that start at or before t_last
-    for (int i = threadIdx.x; i < n_blk; i += kThreads) sl.mask[i] = 0ull;
-    if (threadIdx.x == 0) *sl.repeats = 0;
-    __syncthreads();
-    const int32_t* idx = a.block_idx + ((size_t)bh * a.T + t_first) * a.S;
-    const int n_e = (t_last - t_first + 1) * a.S;
-    for (int e = threadIdx.x; e < n_e; e += kThreads) {
-      const int ql = e / a.S;
-      const int blk = __ldg(idx + e);
-      if (blk >= 0 && (long long)blk * a.block_size <= t_first + ql &&
-          (atomicOr(&sl.mask[blk], 1ull << ql) >> ql & 1ull))
-        *sl.repeats = 1;
-    }
-    __syncthreads();
-    if (threadIdx.x < 32) {
-      int n = 0;
-      for (int b0 = 0; b0 < n_blk; b0 += 32) {
-        const int b = b0 + threadIdx.x;
-        const bool on = b < n_blk && sl.mask[b] != 0ull;
-        const unsigned m = __ballot_sync(0xffffffffu, on);
-        if (on) sl.list[n + __popc(m & ((1u << threadIdx.x) - 1u))] = (uint16_t)b;
-        n += __popc(m);
-      }
-      if (threadIdx.x == 0) *sl.n_list = n;
-    }
-    __syncthreads();
-    k.n = *sl.n_list * a.block_size;
-  }
-  return k;
-}
-
-// How often query t lists the block of token tok.  A block listed twice counts twice, as it does in the
-// row kernels, which go through the slots one by one.
-__device__ __forceinline__ int times_listed(const AttnArgs& a, int bh, int t, int tok) {
-  const int32_t* slot = a.block_idx + ((size_t)bh * a.T + t) * a.S;
-  const int blk = tok / a.block_size;
-  int n = 0;
-#pragma unroll 1
-  for (int s = 0; s < a.S; ++s) n += __ldg(slot + s) == blk;
-  return n;
-}
-
-// token and membership of key tile i's keys (threads 0..63)
-__device__ __forceinline__ void fill_keys(const AttnArgs& a, const TileKeys& tk, const SelList& sl, KeyInfo* ki, int buf, int i) {
-  if (threadIdx.x >= kK) return;
-  const int k = i * kK + threadIdx.x;
-  int tok = -1;
-  unsigned long long m = 0ull;
-  if (k < tk.n) {
-    if (a.kind == 2) {
-      const int b = sl.list[k / a.block_size];
-      tok = b * a.block_size + k % a.block_size;
-      m = sl.mask[b];
-      if (tok >= a.T) tok = -1;
-    } else {
-      tok = tk.first + k;
-    }
-  }
-  ki->tok[buf][threadIdx.x] = tok;
-  ki->mask[buf][threadIdx.x] = m;
-}
-
 // one K or V tile into shared memory [64][D + 4]; keys that do not exist read as zero
 template <typename T, int D, int kThreads>
 __device__ __forceinline__ void load_keys(float* dst, const T* __restrict__ base, const int* tok) {
@@ -206,14 +104,6 @@ __device__ __forceinline__ void load_keys(float* dst, const T* __restrict__ base
   }
 }
 
-// keys [lo, hi] a row of query t may see by position
-__device__ __forceinline__ void row_range(const AttnArgs& a, int t, int& lo, int& hi) {
-  lo = 0;
-  hi = min(t, a.Lk - 1);
-  if (a.kind == 0) lo = max(0, t - a.window + 1);
-  else if (a.kind == 1) hi = cmp_visible(t, a.block_size, a.window, a.Lk) - 1;
-}
-
 // Whether a value of the tile that this thread has put into shared memory is infinite or NaN; the loop is load_keys'.
 template <typename T, int D, int kThreads>
 __device__ __forceinline__ bool non_finite(const float* tile) {
@@ -229,13 +119,6 @@ __device__ __forceinline__ bool non_finite(const float* tile) {
   }
   return z != 0.f;
 }
-
-// What stands for a key that a row does not attend in the tile of P: the sign tells it from a probability of
-// zero.  As a factor it is a zero, as long as the other factor is finite; a tile that holds a value
-// that is not goes through loops that leave these keys out, so that such a value stays with the rows
-// (and keys) that it belongs to.
-constexpr float kMasked = -0.f;
-__device__ __forceinline__ bool attended(float p) { return __float_as_uint(p) != 0x80000000u; }
 
 template <int D> constexpr size_t fwd_floats() { return (size_t)3 * kR * (D + kPad) + (size_t)kR * kPLd; }
 template <int D> constexpr size_t bwd_floats() { return (size_t)4 * kR * (D + kPad) + (size_t)2 * kR * kPLd; }
@@ -711,14 +594,8 @@ simt_tile_bwd_kernel(const AttnArgs a, const int csize) {
     }
 }
 
-long long n_tiles(const AttnArgs& a) {
-  return ((long long)a.T * (a.Hq / a.Hkv) + kR - 1) / kR * a.B * a.Hkv;
-}
-
-size_t extra_smem(const AttnArgs& a) { return sizeof(KeyInfo) + 16 + (a.kind == 2 ? (size_t)sel_blocks(a) * 10 : 0); }
-
 // CTAs that share a row tile, each taking every csize-th key tile.  A row tile is one long chain; with few of them the
-// longest is what the call waits for.  The lines, in row tiles per SM (fp32, D = 64, 8 heads on 2; alone | 2 | 4 CTAs a
+// longest is what the call waits for.  The lines, in row tiles per SM (fp32, D = 64 on these kernels, 8 heads on 2; alone | 2 | 4 CTAs a
 // tile, us): selection at 0.86 forward 132 | 93 | 66, backward 232 | 180 | 125; at 1.7 310 | 189 | 182 and
 // 640 | 355 | 399; at 6.9 650 | 615 | 678 and 1507 | 1345 | 1499; at 21 1648 | 1691 | 2021 and 3935 | 3994 | 4467.
 // Window (chains of 9 key tiles) at 0.4 69 | 44 | 37 and 109 | 64 | 55; at 1.3 101 | 78 | 90 and 196 | 145 | 159; at 1.7
@@ -769,7 +646,9 @@ int launch_d(const AttnArgs& a, bool bwd, cudaStream_t st) {
   switch (a.D) {
     case 16: return launch<T, 16>(a, bwd, st);
     case 32: return launch<T, 32>(a, bwd, st);
-    case 64: return launch<T, 64>(a, bwd, st);
+    case 64:
+      if constexpr (sizeof(T) == 4) return f32_tile_launch(a, bwd, st);       // on the tensor cores
+      else return launch<T, 64>(a, bwd, st);
     case 128: return launch<T, 128>(a, bwd, st);
     default: set_error("head dim %d not in {16,32,64,128}", a.D); return NSA_ERR_UNSUPPORTED;
   }
