@@ -64,26 +64,6 @@ __host__ __device__ inline size_t fwd_smem_bytes(int D, int nb_sel, int nw, int 
 constexpr int kFwdThreads = 192;
 constexpr int kFwdSoftmax = 128;
 
-// Packed pairs of fp32: one instruction for two lanes' worth of the softmax arithmetic.
-__device__ __forceinline__ uint64_t pack_f32x2(float a, float b) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ void unpack_f32x2(uint64_t v, float& a, float& b) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-}
-__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-
 // One kernel for the three branches (kKind: 0 window, 1 compression, 2 selection).  192 threads in roles: warps 0-3 (thread = row
 // = TMEM lane) own the softmax, warp 4 sends the TMA loads, warp 5 issues the MMAs; two CTAs per SM,
 // each walking many row tiles (tile w, w + gridDim.x, ...), long rows first.

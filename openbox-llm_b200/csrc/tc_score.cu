@@ -295,42 +295,56 @@ __device__ __forceinline__ void sort_candidates(float (&v)[N], int (&j)[N]) {
 }
 
 // ------------------------------------------------------------------------------------------
-// The same for GQA groups of 4, 8 or 16 (padded) heads, without the shared-memory round trip:
-// the rows of a tile are ordered query-major (row = query * GP + head, one TMA box from the
-// (D, heads, T) view of q), so the GP heads of a query are GP neighbouring lanes of one warp.
-// They add their probabilities by a recursive-halving exchange (GP/2, ..., 1 lanes apart), after
-// which lane g holds the importance of the tile's blocks [g * 64/GP, (g+1) * 64/GP) and scans
-// exactly those for its top-16 list.  64 KB of shared memory: three CTAs per SM.
-// The first tile's candidates go into the empty lists by a sorting network: 8 x 4096 tokens, 12 heads of 64, where a
-// row tile has one tile of summaries, 110 -> 101 us.  A tile that every row of a warp sees whole needs no compare
-// and select per element: 64 heads x 65536 tokens 2.25 -> 2.15 ms, 8 x 32768 1.73 -> 1.63.
+// The same for GQA groups of 4, 8 or 16 (padded) heads, with the score tile turned round: summaries in the lanes of tensor
+// memory, rows (query-major: query * GP + head, one TMA box from the (D, heads, T) view of q) in its columns.  A thread has
+// one summary and adds the heads of a query up in registers, in the order (h, h + GP/2), ..., (h, h + 1); the sums go through
+// shared memory to the GP lanes of the query, lane g taking the tile's summaries [g * n / GP, (g + 1) * n / GP) into
+// its top-16 list.  A tile has 128 summaries, or, where 64 or 32 are left, two or four copies of those, so that all warps have
+// columns to do: warp w does n columns of its copy.
+// What bounds it: exponentials (1024 cycles of a full tile's 3.9 k at 64 heads) and the lists' bookkeeping, three CTAs of four warps an SM (four
+// at D = 64), and in short calls fetching instructions: insertions are loops, not unrolled.  Rows in the lanes, heads added by a
+// recursive-halving exchange of shuffles, took 240 instructions of a warp per 64 summaries; 64 heads of 128 x 65536 tokens 2.37 ->
+// 1.97 ms, 8 x 32768 tokens of 16 heads 2.0 -> 1.64, 8 x 4096 tokens of 12 heads of 64 109 -> 81 us.  The first tile's candidates go into
+// the empty lists by a sorting network (8 x 4096 tokens: 110 -> 101 us when it came).
 // ------------------------------------------------------------------------------------------
+constexpr int kImpLd = 144;              // floats of a query's row of sums: 128, and 4 more after every 32 (16-byte reads without conflicts)
+
+template <int D, int GP> struct ScoreLanes {
+  static constexpr int kSlabs = D / 64;
+  static constexpr int kQBytes = kRows * 128 * kSlabs, kKBytes = 128 * 128 * kSlabs;
+  static constexpr int kImpBytes = kRows / GP * kImpLd * 4;
+  static constexpr size_t kSmem = kQBytes + kKBytes + kImpBytes + 128 * 4 /*lse*/ + 64 /*barriers*/ + 1024;
+  static constexpr int kCtas = (int)(227 * 1024 / (kSmem + 1024)) > 4 ? 4 : (int)(227 * 1024 / (kSmem + 1024));
+};
+
 template <int D, int GP, bool kAligned>
-__global__ void __launch_bounds__(128, 3)
+__global__ void __launch_bounds__(128, ScoreLanes<D, GP>::kCtas)
 tc_score_lanes_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                       const ScoreArgs p) {
-  constexpr int kSlabs = D / 64;
-  constexpr int kQBytes = kRows * 128 * kSlabs, kKBytes = kKeys * 128 * kSlabs;
-  constexpr uint32_t kTmemCols = 64;
-  constexpr uint32_t kIdescQK = idesc_bf16(128, kKeys, 0, 0);
+  using L = ScoreLanes<D, GP>;
+  constexpr int kSlabs = L::kSlabs, kQBytes = L::kQBytes, kKBytes = L::kKBytes;
+  constexpr uint32_t kTmemCols = 128;
+  constexpr uint32_t kIdescKQ = idesc_bf16(128, 128, 0, 0);
   constexpr int NQ = kRows / GP;       // queries per tile
-  constexpr int PER = kKeys / GP;      // blocks of a tile each lane ends up owning
+  constexpr int PER = 128 / GP;        // summaries of a full tile that a lane takes
   constexpr int kList = 16;
 
   extern __shared__ uint8_t smem_raw[];
   chain_wait();
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   uint8_t* sQ = smem;
-  uint8_t* sK = sQ + kQBytes;                        // 2 stages
-  uint64_t* bars = (uint64_t*)(sK + 2 * kKBytes);
+  uint8_t* sK = sQ + kQBytes;
+  float* s_imp = (float*)(sK + kKBytes);             // [NQ][kImpLd]
+  float* s_lse = s_imp + NQ * kImpLd;                // [128], negative, log2 units
+  uint64_t* bars = (uint64_t*)(s_lse + 128);
   uint64_t* bar_q = bars + 0;
-  uint64_t* bar_k = bars + 1;   // [2]
-  uint64_t* bar_s = bars + 3;
-  uint64_t* bar_drain = bars + 4;   // an aborted CTA waits here for its last MMAs
-  uint32_t* s_tmem = (uint32_t*)(bars + 5);
+  uint64_t* bar_k = bars + 1;
+  uint64_t* bar_s = bars + 2;
+  uint64_t* bar_drain = bars + 3;   // an aborted CTA waits here for its last MMAs
+  uint32_t* s_tmem = (uint32_t*)(bars + 4);
   volatile int* s_abort = (volatile int*)(s_tmem + 1);
 
-  const int tid = threadIdx.x, warp = tid >> 5;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int qtile = p.n_qtiles - 1 - (int)blockIdx.x;
   const int bh = blockIdx.y;
   const int b = bh / p.Hkv, hkv = bh % p.Hkv;
@@ -343,7 +357,7 @@ tc_score_lanes_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   if (tid == 0) {
     *s_abort = (*(volatile int*)p.status != 0) ? 1 : 0;
     mbar_init(bar_q, 1);
-    mbar_init(bar_k + 0, 1); mbar_init(bar_k + 1, 1);
+    mbar_init(bar_k, 1);
     mbar_init(bar_s, 1);
     mbar_init(bar_drain, 1);
     fence_barrier_init();
@@ -352,12 +366,18 @@ tc_score_lanes_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   __syncthreads();
   if (*s_abort) return;
 
-  const int hi_last = cmp_visible(t_last, p.block_size, p.stride, p.n_blk) - 1;
-  int n_tiles = hi_last < 0 ? 0 : hi_last / kKeys + 1;
+  int n_sum = cmp_visible(t_last, p.block_size, p.stride, p.n_blk);      // summaries to go through
+  // (a block is a candidate from the summary before it on where they overlap: its own may be in the next tile)
+  if (!kAligned && n_sum > 0) n_sum += p.overlap;
   const bool forcing = p.n_init > 0 || p.n_local > 0;
-  // forced blocks are candidates whatever their importance: reach the tile whose lanes own the
-  // block that holds the last query
-  if (forcing) n_tiles = max(n_tiles, (p.r * (t_last / p.sel_block)) / kKeys + 1);
+  // forced blocks are candidates whatever their importance: as far as the block that holds the last query
+  if (forcing) n_sum = max(n_sum, p.r * (t_last / p.sel_block + 1));
+  const int n_tiles = (n_sum + 127) / 128;
+  // summaries in tile i: 128, or 64 or 32 (several copies) where that is what is left; whole blocks for each lane
+  auto size_of = [&](int i) -> int {
+    const int left = n_sum - 128 * i;
+    return left > 64 ? 128 : left > 32 || (!kAligned && p.r * GP > 32) ? 64 : 32;
+  };
 
   float lv[kList];
   int li[kList];
@@ -365,171 +385,213 @@ tc_score_lanes_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   for (int k = 0; k < kList; ++k) { lv[k] = -1.f; li[k] = -1; }
 
   if (n_tiles > 0) {
-    if (warp == 0) {
-      tmem_alloc(s_tmem, kTmemCols);
-      tmem_relinquish();
-    }
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const uint32_t tmem = *s_tmem;
-    chain_go();
-    bool aborted = false;
     int k_loaded = 0, k_seen = 0;   // thread 0: K tiles whose load was issued / whose arrival was seen
-    bool q_seen = false;
-    const uint32_t lane_base = tmem + ((uint32_t)(warp * 32) << 16);
-    const float lse2 = row_ok ? ld_plain(p.lse + (size_t)(b * p.Hq + hkv * p.G + g) * p.T + t) * kLog2e : 0.f;
-    const int n_vis = t < p.T ? cmp_visible(t, p.block_size, p.stride, p.n_blk) : 0;   // summaries query t sees
-    const int my_cur = t / p.sel_block;              // selection block that holds t
-    float carry = 0.f;                               // last summary of the previous tile (overlap)
-
     auto load_k = [&](int i) {
-      uint64_t* bar = bar_k + (i & 1);
-      mbar_expect_tx(bar, kKBytes);
+      const int groups = size_of(i) / 32;
+      mbar_expect_tx(bar_k, kKBytes);
 #pragma unroll
       for (int sl = 0; sl < kSlabs; ++sl)
-        tma_load_3d(sK + (i & 1) * kKBytes + sl * (kKeys * 128), &tm_k, bar, sl * 64, i * kKeys, bh);
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+          tma_load_3d(sK + sl * (128 * 128) + r * (32 * 128), &tm_k, bar_k, sl * 64, i * 128 + 32 * (r % groups), bh);
       k_loaded = i + 1;
     };
-    auto issue_s = [&](int i) {
-      const uint32_t qa = desc_lo_kmajor(smem_u32(sQ)), ka = desc_lo_kmajor(smem_u32(sK + (i & 1) * kKBytes));
-#pragma unroll
-      for (int kk = 0; kk < D / 16; ++kk) {
-        const uint32_t slab = kk >> 2, in = (kk & 3) * 32;
-        mma_ss(tmem, desc_at(qa, slab * (kRows * 128) + in), desc_at(ka, slab * (kKeys * 128) + in),
-               kIdescQK, kk > 0);
-      }
-      tc_commit(bar_s);
-    };
-    if (tid == 0) {
+    if (tid == 0) {                 // on their way while the rest is set up
       mbar_expect_tx(bar_q, kQBytes);
 #pragma unroll
       for (int sl = 0; sl < kSlabs; ++sl)     // box: 64 columns x GP heads x NQ tokens
         tma_load_3d(sQ + sl * (kRows * 128), &tm_q, bar_q, sl * 64, b * p.Hq + hkv * p.G, t0);
       load_k(0);
-      if (n_tiles > 1) load_k(1);
+    }
+    __syncwarp();
+    if (warp == 0) {
+      tmem_alloc(s_tmem, kTmemCols);
+      tmem_relinquish();
+    }
+    s_lse[tid] = row_ok ? ld_plain(p.lse + (size_t)(b * p.Hq + hkv * p.G + g) * p.T + t) * -kLog2e : 0.f;
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *s_tmem;
+    chain_go();
+    const uint64_t sc2 = pack_f32x2(p.scale_log2, p.scale_log2);
+    bool aborted = false, q_seen = false;
+    const uint32_t lane_base = tmem + ((uint32_t)(warp * 32) << 16);
+    const int n_vis = t < p.T ? cmp_visible(t, p.block_size, p.stride, p.n_blk) : 0;   // summaries query t sees
+    const int my_cur = t / p.sel_block;              // selection block that holds t
+    float carry = 0.f;                               // last summary of the previous tile (overlap)
+
+    auto insert = [&](float cv, int cj) {
+      if (cv > lv[kList - 1]) {                // beats the list's last entry (empty slots hold -1)
+#pragma unroll
+        for (int r = kList - 1; r >= 1; --r) {   // strict '>' keeps earlier (lower) indices ahead
+          const bool up = cv > lv[r - 1];
+          const bool here = cv > lv[r];
+          li[r] = up ? li[r - 1] : (here ? cj : li[r]);
+          lv[r] = up ? lv[r - 1] : (here ? cv : lv[r]);
+        }
+        if (cv > lv[0]) { lv[0] = cv; li[0] = cj; }
+      }
+    };
+    auto issue_s = [&]() {
+      const uint32_t qa = desc_lo_kmajor(smem_u32(sQ)), ka = desc_lo_kmajor(smem_u32(sK));
+#pragma unroll
+      for (int kk = 0; kk < D / 16; ++kk) {
+        const uint32_t at = (kk >> 2) * (128 * 128) + (kk & 3) * 32;
+        mma_ss(tmem, desc_at(ka, at), desc_at(qa, at), kIdescKQ, kk > 0);
+      }
+      tc_commit(bar_s);
+    };
+    if (tid == 0) {
       q_seen = mbar_wait(bar_q, 0, p.status, s_abort, 1);
       if (mbar_wait(bar_k, 0, p.status, s_abort, 2)) k_seen = 1;
       tc_fence_after();
-      if (!*s_abort) issue_s(0);
+      if (!*s_abort) issue_s();
     }
 
     for (int i = 0; i < n_tiles; ++i) {
-      const int key0 = i * kKeys;
-      mbar_wait(bar_s, i & 1, p.status, s_abort, 4);
+      const int key0 = i * 128, size = size_of(i);
+      const int per = size / GP;                     // of the tile's summaries, a lane's
+      const bool s_ok = mbar_wait(bar_s, i & 1, p.status, s_abort, 4);
       tc_fence_after();
       __syncwarp();
-      float v[64];
+      if (tid == 0 && s_ok && i + 1 < n_tiles) load_k(i + 1);          // the MMAs have read this tile's
       {
-        uint32_t r[64];
-        tmem_ld32(lane_base, r);
-        tmem_ld32(lane_base + 32, r + 32);
-        tmem_wait_ld();
-        tc_fence_before();
-        const int hi = row_ok ? min(kKeys - 1, n_vis - 1 - key0) : -1;
-        if (__all_sync(0xffffffffu, hi >= kKeys - 1)) {      // no compare and select per element
+        const int at = 32 * (warp % (size / 32)) + lane;               // this thread's summary in the tile
+        const int c0 = warp / (size / 32) * size;                      // and its columns
+        float* imp = s_imp + at + 4 * (at >> 5);
+#pragma unroll 1
+        for (int c = c0; c < c0 + size; c += 32) {
+          uint32_t r[32];
+          tmem_ld32(lane_base + c, r);
+          uint64_t e[16];                            // two columns each
+          tmem_wait_ld();
 #pragma unroll
-          for (int c = 0; c < 64; ++c) v[c] = ex2(__uint_as_float(r[c]) * p.scale_log2 - lse2);
-        } else {
+          for (int k = 0; k < 16; k += 2) {
+            const ulonglong2 l = *reinterpret_cast<const ulonglong2*>(s_lse + c + 2 * k);
 #pragma unroll
-          for (int c = 0; c < 64; ++c)
-            v[c] = (c <= hi) ? ex2(__uint_as_float(r[c]) * p.scale_log2 - lse2) : 0.f;
+            for (int x = 0; x < 2; ++x) {
+              float e0, e1;
+              unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(r[2 * (k + x)]), __uint_as_float(r[2 * (k + x) + 1])), sc2, x ? l.y : l.x), e0, e1);
+              e0 = ex2(e0);
+              e1 = ex2(e1);
+              // (padding: rows of the next group, or none)
+              const int h = 2 * (k + x) % GP;
+              if (h > GP / 2 && h >= p.G) e0 = 0.f;
+              if (h + 1 > GP / 2 && h + 1 >= p.G) e1 = 0.f;
+              e[k + x] = pack_f32x2(e0, e1);
+            }
+          }
+#pragma unroll
+          for (int q = 0; q < 32 / GP; ++q) {
+#pragma unroll
+            for (int o = GP / 4; o >= 1; o >>= 1)
+#pragma unroll
+              for (int h = 0; h < o; ++h) e[q * GP / 2 + h] = add_f32x2(e[q * GP / 2 + h], e[q * GP / 2 + h + o]);
+            float e0, e1;
+            unpack_f32x2(e[q * GP / 2], e0, e1);
+            imp[(c / GP + q) * kImpLd] = e0 + e1;
+          }
         }
+        tc_fence_before();
       }
-      // every thread has read S: the next MMA may overwrite it; one decision for the whole CTA:
+      // the sums are there, and S has been read: the next MMA may overwrite it; one decision for the whole CTA:
       // after a given-up wait nothing more is issued or written
       if (__syncthreads_or(*s_abort)) { aborted = true; break; }
-      if (tid == 0) {
-        if (i + 2 < n_tiles) load_k(i + 2);    // stage i & 1 was read by the MMA that just completed
-        if (i + 1 < n_tiles) {
-          tc_fence_after();
-          if (mbar_wait(bar_k + ((i + 1) & 1), ((i + 1) >> 1) & 1, p.status, s_abort, 2)) {
-            k_seen = i + 2;
-            issue_s(i + 1);
-          }
+      if (tid == 0 && i + 1 < n_tiles) {
+        tc_fence_after();
+        if (mbar_wait(bar_k, (i + 1) & 1, p.status, s_abort, 2)) {
+          k_seen = i + 2;
+          issue_s();
         }
       }
       __syncwarp();
-      // sum over the heads of the query: recursive halving, the lane with the bit set keeps the
-      // upper half of the columns
-      {
-        int width = 64;
-#pragma unroll
-        for (int o = GP / 2; o >= 1; o >>= 1) {
-          width >>= 1;
-          const bool upper = (g & o) != 0;
-#pragma unroll
-          for (int c = 0; c < 32; ++c) {
-            if (c < width) {
-              const float send = upper ? v[c] : v[c + width];
-              const float keep = upper ? v[c + width] : v[c];
-              v[c] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-            }
-          }
-        }
-      }
-      // lane g now holds the summaries key0 + g * PER + k in v[k].  A selection block is r
-      // consecutive summaries (plus, when the summaries overlap, the one before them); it is a
-      // candidate once its first summary is visible.
-      // kAligned: summaries and blocks coincide (r = 1, no overlap), all of it folds away
-      const int r_ = kAligned ? 1 : p.r, ov_ = kAligned ? 0 : p.overlap;
-      float prev = 0.f;
-      if (!kAligned) {
-        prev = __shfl_up_sync(0xffffffffu, v[PER - 1], 1);
-        if (g == 0) prev = carry;
-        carry = __shfl_sync(0xffffffffu, v[PER - 1], (threadIdx.x & 31 & ~(GP - 1)) + GP - 1);
-      }
+      // the query's sum at place k of the tile; what it does not see is zero
+      auto sum_at = [&](int k) -> float { return key0 + k < n_vis ? s_imp[ql * kImpLd + k + 4 * (k >> 5)] : 0.f; };
       float* out = (p.imp_out && t < p.T) ? p.imp_out + ((size_t)bh * p.T + t) * p.imp_cols : nullptr;
-      if (kAligned && i == 0 && !forcing) {
-        float sv[PER];
-        int sj[PER];
-#pragma unroll
-        for (int k = 0; k < PER; ++k) {
-          const int cj = g * PER + k;
-          const bool visible = cj < n_vis;
-          if (out && cj < p.imp_cols) out[cj] = visible ? v[k] : 0.f;
-          sv[k] = visible && v[k] >= 0.f ? v[k] : -1.f;      // (not what is NaN, which enters no list)
-          sj[k] = cj;
-        }
-        sort_candidates<PER>(sv, sj);
-#pragma unroll
-        for (int k = 0; k < PER; ++k) {
-          lv[k] = sv[k];
-          li[k] = sv[k] > -1.f ? sj[k] : -1;
-        }
-        continue;
-      }
       // A candidate below entry 16 / GP (counted from 1) of every one of the query's GP lists has
       // at least 16 entries ahead of it, so it cannot reach the merged top 16 and need not enter a
       // list; the bound only rises while the tile is scanned.
-      float tau = lv[kList / GP - 1];
+      auto bound = [&]() -> float {
+        float tau = lv[kList / GP - 1];
 #pragma unroll
-      for (int o = 1; o < GP; o <<= 1) tau = fminf(tau, __shfl_xor_sync(0xffffffffu, tau, o));
-      float accb = 0.f;
+        for (int o = 1; o < GP; o <<= 1) tau = fminf(tau, __shfl_xor_sync(0xffffffffu, tau, o));
+        return tau;
+      };
+      if (kAligned && !forcing) {
+        // summaries and blocks coincide: lane g's are key0 + g * per + k
+        float v[PER];
+        if (per >= 4) {
+          const int at = g * per;
+          const float* imp = s_imp + ql * kImpLd + at + 4 * (at >> 5);
 #pragma unroll
-      for (int k = 0; k < PER; ++k) {
-        if ((k & (r_ - 1)) == 0) accb = ov_ ? (k == 0 ? prev : v[k > 0 ? k - 1 : 0]) : 0.f;
-        accb += v[k];
-        if (((k + 1) & (r_ - 1)) != 0) continue;
-        const int cj = (key0 + g * PER + k) / r_;                  // block index
-        const bool visible = max(0, r_ * cj - ov_) < n_vis;        // first overlapping summary
-        if (out && cj < p.imp_cols) out[cj] = visible ? accb : 0.f;
-        float cv = visible ? accb : -1.f;
-        if (forcing && cj <= my_cur && t < p.T) {
-          if (cj < p.n_init) cv = kForcedInit - (float)cj;
-          else if (cj > my_cur - p.n_local) cv = kForcedLocal - (float)(my_cur - cj);
-        }
-        if (cv > lv[kList - 1] && cv >= tau) {   // beats the list's last entry (empty slots hold -1)
-#pragma unroll
-          for (int r = kList - 1; r >= 1; --r) {   // strict '>' keeps earlier (lower) indices ahead
-            const bool up = cv > lv[r - 1];
-            const bool here = cv > lv[r];
-            li[r] = up ? li[r - 1] : (here ? cj : li[r]);
-            lv[r] = up ? lv[r - 1] : (here ? cv : lv[r]);
+          for (int k = 0; k < PER; k += 4) {
+            if (k >= per) break;
+            const float4 x = *reinterpret_cast<const float4*>(imp + k);
+            v[k] = x.x; v[k + 1] = x.y; v[k + 2] = x.z; v[k + 3] = x.w;
           }
-          if (cv > lv[0]) { lv[0] = cv; li[0] = cj; }
+        } else {
+          v[0] = sum_at(g * per); v[1] = sum_at(g * per + 1);
         }
+        constexpr int kSort = 64 / GP;               // candidates of the first tile that are sorted into the empty lists
+        if (i == 0) {
+          float sv[kSort];
+          int sj[kSort];
+#pragma unroll
+          for (int k = 0; k < kSort; ++k) {
+            const int cj = g * per + k;
+            const bool visible = k < per && cj < n_vis;
+            sv[k] = visible && v[k] >= 0.f ? v[k] : -1.f;    // (not what is NaN, which enters no list)
+            sj[k] = cj;
+          }
+          sort_candidates<kSort>(sv, sj);
+#pragma unroll
+          for (int k = 0; k < kSort; ++k) {
+            lv[k] = sv[k];
+            li[k] = sv[k] > -1.f ? sj[k] : -1;
+          }
+        }
+        if (out)
+          for (int k = 0; k < per; ++k)
+            if (key0 + g * per + k < p.imp_cols) out[key0 + g * per + k] = sum_at(g * per + k);
+        if (i == 0 && per <= kSort) break;           // (the one tile there is)
+        // those that are left, a bit each: a lane's next one a round, for as many rounds as the lane with most of them needs
+        const float tau = bound();
+        uint32_t left = 0u;
+#pragma unroll
+        for (int k = 0; k < PER; ++k)
+          if (k < per && !(i == 0 && k < kSort) && key0 + g * per + k < n_vis && v[k] > lv[kList - 1] && v[k] >= tau) left |= 1u << k;
+        while (__any_sync(0xffffffffu, left != 0u)) {
+          if (left) {
+            const int at = g * per + __ffs(left) - 1;
+            left &= left - 1u;
+            insert(sum_at(at), key0 + at);
+          }
+          __syncwarp();
+        }
+      } else {
+        // A selection block is r consecutive summaries (plus, when the summaries overlap, the one before them); it is a
+        // candidate once its first summary is visible.
+        const int r_ = p.r, ov_ = p.overlap;
+        const float tau = bound();
+#pragma unroll 1
+        for (int k = g * per; k < (g + 1) * per; k += r_) {
+          float acc = !ov_ ? 0.f : k == 0 ? carry : sum_at(k - 1);
+#pragma unroll 1
+          for (int e = 0; e < r_; ++e) acc += sum_at(k + e);
+          const int cj = (key0 + k) / r_;                            // block index
+          const bool visible = max(0, r_ * cj - ov_) < n_vis;        // first overlapping summary
+          if (out && cj < p.imp_cols) out[cj] = visible ? acc : 0.f;
+          float cv = visible ? acc : -1.f;
+          if (forcing && cj <= my_cur && t < p.T) {
+            if (cj < p.n_init) cv = kForcedInit - (float)cj;
+            else if (cj > my_cur - p.n_local) cv = kForcedLocal - (float)(my_cur - cj);
+          }
+          if (cv >= tau) insert(cv, cj);
+        }
+        carry = sum_at(size - 1);
       }
+      if (i + 1 < n_tiles) __syncthreads();          // the next tile's sums may be written
     }
     if (!aborted) aborted = __syncthreads_or(*s_abort) != 0;
     if (aborted) {
@@ -538,7 +600,7 @@ tc_score_lanes_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       // goes back.
       if (tid == 0) {
         if (!q_seen) mbar_wait_drain(bar_q, 0);
-        for (int j = k_seen; j < k_loaded; ++j) mbar_wait_drain(bar_k + (j & 1), (j >> 1) & 1);
+        for (int j = k_seen; j < k_loaded; ++j) mbar_wait_drain(bar_k, j & 1);
         tc_commit(bar_drain);
         mbar_wait_drain(bar_drain, 0);
       }
@@ -573,12 +635,9 @@ tc_score_lanes_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   // importance columns no tile covered are zero
   if (p.imp_out && t < p.T) {
     float* out = p.imp_out + ((size_t)bh * p.T + t) * p.imp_cols;
-    for (int c = n_tiles * kKeys / (kAligned ? 1 : p.r) + g; c < p.imp_cols; c += GP) out[c] = 0.f;
+    const int seen = n_tiles > 0 ? (n_tiles - 1) * 128 + size_of(n_tiles - 1) : 0;
+    for (int c = seen / (kAligned ? 1 : p.r) + g; c < p.imp_cols; c += GP) out[c] = 0.f;
   }
-}
-
-__host__ inline size_t score_lanes_smem_bytes(int D) {
-  return (size_t)(kRows * 128 + 2 * kKeys * 128) * (D / 64) + 256 + 1024;
 }
 
 template <int D, int GP>
@@ -588,9 +647,9 @@ static int launch_score_lanes(const void* q, const void* k_cmp, const NsaDims& d
   p.n_qtiles = (d.T + p.nq - 1) / p.nq;
   CUtensorMap tm_q, tm_k;
   int rc = make_map_query_rows(&tm_q, q, d.D, d.T, d.B * d.Hq, GP, p.nq);
-  if (rc == NSA_OK) rc = make_map(&tm_k, k_cmp, d.D, n_blk, d.B * d.Hkv, kKeys, 1);
+  if (rc == NSA_OK) rc = make_map(&tm_k, k_cmp, d.D, n_blk, d.B * d.Hkv, 32, 1);
   if (rc != NSA_OK) return rc;
-  const size_t smem = score_lanes_smem_bytes(d.D);
+  const size_t smem = ScoreLanes<D, GP>::kSmem;
   KernelScope ks("tc_score_topn", st);
   if (p.r == 1 && p.overlap == 0) {
     NSA_CUDA_OK(func_smem((const void*)tc_score_lanes_kernel<D, GP, true>, smem));
