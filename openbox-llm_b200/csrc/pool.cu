@@ -3,9 +3,10 @@
 // (and mean pooling of fp32).  Every kernel takes the K and the V tensor of the branch in one
 // launch (blockIdx.y).  All of them are bound by the one pass over x (and dx); at 2 x 16 units of
 // 32768 x 128 the learned forward takes 0.11 ms (0.18 ms as two launches with their loads one
-// window row at a time) and its backward 0.22 ms (0.63 ms, which read x twice more and had the
-// projection gradient in a kernel of its own); at 4 units of 512 x 64 the forward takes 5 us
-// (2 x 14 us).
+// window row at a time) and its backward 0.18 ms (0.25 ms with the projection's gradient in scalar atomics; 0.63 ms when it read x
+// twice more and had that gradient in a kernel of its own); at 4 units of 512 x 64 the forward takes 5 us
+// (2 x 14 us).  In short calls the backward's end counts: D x D atomics of every CTA, and the last CTA's copy of their sums;
+// as vectors of four, and with the copy's loads all in flight, 2 x 1024 tokens of 4 heads of 128 in windows of 16 take 30 us, 63 before.
 #include "pool.cuh"
 
 namespace nsa {
@@ -51,9 +52,10 @@ __device__ __forceinline__ void pool_weights(const float* __restrict__ logits, f
 
 // Forward.  A CTA takes R consecutive summary rows: D/8 threads per token row with 16-byte loads,
 // 256/(D/8) token rows at a time, all loads of two summary rows in flight together; the
-// projection matrix travels into shared memory (cp.async, padded rows) meanwhile.  R = 8 where
+// projection matrix travels into shared memory (cp.async, padded rows) meanwhile.  R = 8, or 4, where
 // that still gives every SM a CTA, else 2: a short sequence has a few dozen rows in all, and the
-// latency of one CTA's chain is what counts.
+// latency of one CTA's chain is what counts.  512 rows of 128 in windows of 16: R = 8 14.5 us, 4 14.5, 2 18.8 (more CTAs than fit at once);
+// 552 rows of 64 in windows of 64: 14.6, 13.4, 16.7.
 template <int D, int R>
 struct PoolFwdSmem {
   static constexpr int kProjLd = D + 4;                 // float4 reads of 8 lanes cover all banks
@@ -214,6 +216,7 @@ pool_bwd_kernel(const PoolSides s, int T_, int len, int stride, int n_sum, int r
   constexpr int VL = D / 8, RG = kThreads / VL, R = PoolBwdSmem<D>::R;
   constexpr int kTile = D >= 64 ? D / 16 : D / 8;       // d_proj: each thread owns kTile x kTile entries
   constexpr int kSide = D / kTile;                      // of a kSide x kSide grid of threads
+  constexpr int kVec = kTile >= 4 ? 4 : 2;              // entries an atomic
   float* pj = sm;                 // [D][D]
   float* go = pj + D * D;         // [R][D] d_out
   float* dp = go + R * D;         // [R][D] d_pooled
@@ -375,7 +378,14 @@ pool_bwd_kernel(const PoolSides s, int T_, int len, int stride, int n_sum, int r
 #pragma unroll
     for (int a = 0; a < kTile; ++a)
 #pragma unroll
-      for (int c = 0; c < kTile; ++c) atomicAdd(acc_proj + (size_t)(to * kTile + a) * D + ti * kTile + c, pacc[a][c]);
+      for (int c = 0; c < kTile; c += kVec) {
+        float* at = acc_proj + (size_t)(to * kTile + a) * D + ti * kTile + c;
+        if constexpr (kVec == 4)
+          asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(at), "f"(pacc[a][c]), "f"(pacc[a][c + 1]), "f"(pacc[a][c + 2]),
+                       "f"(pacc[a][c + 3]) : "memory");
+        else
+          asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(at), "f"(pacc[a][c]), "f"(pacc[a][c + 1]) : "memory");
+      }
   }
   __syncthreads();
   for (int r = tid; r < len; r += kThreads) atomicAdd(acc_w + r, dw[r]);
@@ -402,7 +412,26 @@ pool_bwd_kernel(const PoolSides s, int T_, int len, int stride, int n_sum, int r
   for (int r = 0; r < len; ++r) dot = fmaf(dw[r], w[r], dot);
   for (int r = tid; r < len; r += kThreads) s.d_logits[side][r] = w[r] * (dw[r] - dot);
   for (int i = tid; i < len * D; i += kThreads) s.d_intra[side][i] = w[i / D] * sdps[i % D];
-  for (int i = tid; i < D * D; i += kThreads) s.d_proj[side][i] = __ldcg(acc_proj + i);
+  // (several vectors in flight: one at a time, this copy was half of a short call)
+  constexpr int kCopy = (D * D / 4 + kThreads - 1) / kThreads;
+  float4 out[kCopy];
+#pragma unroll
+  for (int k = 0; k < kCopy; ++k) {
+    const int i = tid + k * kThreads;
+    if (i < D * D / 4) out[k] = __ldcg(reinterpret_cast<const float4*>(acc_proj) + i);
+  }
+  const bool vec = (reinterpret_cast<uintptr_t>(s.d_proj[side]) & 15) == 0;
+#pragma unroll
+  for (int k = 0; k < kCopy; ++k) {
+    const int i = tid + k * kThreads;
+    if (i >= D * D / 4) continue;
+    float* dst = s.d_proj[side] + 4 * i;
+    if (vec) {
+      *reinterpret_cast<float4*>(dst) = out[k];
+    } else {
+      dst[0] = out[k].x; dst[1] = out[k].y; dst[2] = out[k].z; dst[3] = out[k].w;
+    }
+  }
 }
 
 // dx of overlapping windows (stride < len): token pos of (b, h) collects w[pos - j*stride] *
@@ -522,6 +551,7 @@ int launch_pool_fwd(const PoolSides& s, int T, int len, int stride, int n_sum, i
 template <int D>
 int launch_pool_fwd(const PoolSides& s, int T, int len, int stride, int n_sum, int rows, cudaStream_t st) {
   if ((long long)s.n * ((rows + 7) / 8) >= sm_count()) return launch_pool_fwd<D, 8>(s, T, len, stride, n_sum, rows, st);
+  if ((long long)s.n * ((rows + 3) / 4) >= sm_count()) return launch_pool_fwd<D, 4>(s, T, len, stride, n_sum, rows, st);
   return launch_pool_fwd<D, 2>(s, T, len, stride, n_sum, rows, st);
 }
 template <int D>
