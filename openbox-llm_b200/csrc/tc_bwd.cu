@@ -1708,7 +1708,11 @@ static BwdPlan plan_bwd(const AttnArgs& a) {
   const int item_rt = a.kind == 2 ? (max_rt < kSelChunkTiles ? max_rt : kSelChunkTiles) : max_rt;
   const long long base = (long long)units * pl.n_ktiles;
   pl.csize = 1;
-  while (a.kind != 1 && !a.dq_acc && !pl.wide && pl.csize < 8 && base * pl.csize * 2 <= sm_count() + 20 && item_rt >= 8 * pl.csize) pl.csize *= 2;
+  // Three-term row tiles take three times as long as others beside the same cost of a CTA, and early key tiles have most
+  // of them: up to two CTAs per SM.  128 key tiles of 13 row tiles (2 x 1024 tokens, 16 heads of 128, 8 blocks of 16 a list): alone 161 us, pairs 127,
+  // clusters of four 132.
+  const long long most = a.three_term ? 2LL * sm_count() : sm_count() + 20;
+  while (a.kind != 1 && !a.dq_acc && !pl.wide && pl.csize < 8 && base * pl.csize * 2 <= most && item_rt >= 8 * pl.csize) pl.csize *= 2;
   // compression: a few key tiles are attended by (almost) every query; they go in chunks of 48 row
   // tiles whose dK / dV meet in fp32 accumulators
   pl.n_splits = 1;
