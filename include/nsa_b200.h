@@ -190,6 +190,13 @@ int nsa_attention_fwd(const NsaAttentionDesc* desc, const NsaAttentionTensors* t
                       size_t workspace_bytes, void* stream);
 int nsa_attention_bwd(const NsaAttentionDesc* desc, const NsaAttentionTensors* t, const void* saved,
                       void* workspace, size_t workspace_bytes, void* stream);
+/* The same with the output and its gradient in [B, T, Hq, D], for a caller whose next GEMM takes tokens: `out` is
+ * written so; backward reads d_tokens and writes its rows in the order of the heads to t->d_out, which is scratch of
+ * the output's size.  bf16, D a power of two. */
+int nsa_attention_fwd_tokens(const NsaAttentionDesc* desc, const NsaAttentionTensors* t, void* saved, void* workspace,
+                             size_t workspace_bytes, void* stream);
+int nsa_attention_bwd_tokens(const NsaAttentionDesc* desc, const NsaAttentionTensors* t, const void* saved,
+                             void* workspace, size_t workspace_bytes, const void* d_tokens, void* stream);
 
 /* ---- block -> query CSR ---------------------------------------------------------------------
  * Replaces build_block_to_query_csr (nsa_fsa.py:14-64): pairs (query i, block j) with j >= 0

@@ -87,6 +87,8 @@ SIGNATURES = {
     "nsa_attention_sizes": (_i, [_ap, _sp, _sp, _sp]),
     "nsa_attention_fwd": (_i, [_ap, _vp, _vp, _vp, _sz, _vp]),
     "nsa_attention_bwd": (_i, [_ap, _vp, _vp, _vp, _sz, _vp]),
+    "nsa_attention_fwd_tokens": (_i, [_ap, _vp, _vp, _vp, _sz, _vp]),
+    "nsa_attention_bwd_tokens": (_i, [_ap, _vp, _vp, _vp, _sz, _vp, _vp]),
     "nsa_fused_projection_width": (_i, [_i, _i, _i]),
     "nsa_split_heads": (_i, [_vp] * 4 + [_i] * 6 + [_vp]),
     "nsa_merge_heads": (_i, [_vp] * 4 + [_i] * 6 + [_vp]),

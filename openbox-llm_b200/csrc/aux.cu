@@ -456,8 +456,7 @@ __global__ void gate_bwd_kernel(const T* __restrict__ oc, const T* __restrict__ 
 }
 
 // bf16 rows of D = 8 * VL elements (VL a power of two <= 32): VL threads per row, 16 bytes each
-__device__ __forceinline__ void load8(const __nv_bfloat16* p, float* f) {
-  const uint4 u = __ldg(reinterpret_cast<const uint4*>(p));
+__device__ __forceinline__ void unpack8(const uint4& u, float* f) {
   const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
 #pragma unroll
   for (int e = 0; e < 4; ++e) {
@@ -465,14 +464,25 @@ __device__ __forceinline__ void load8(const __nv_bfloat16* p, float* f) {
     f[2 * e] = t.x; f[2 * e + 1] = t.y;
   }
 }
+__device__ __forceinline__ void load8(const __nv_bfloat16* p, float* f) { unpack8(__ldg(reinterpret_cast<const uint4*>(p)), f); }
+
+// row (b, t, h) of a token-major tensor for row (b, h, t) of a head-major one (fewer than 2^32 rows)
+__device__ __forceinline__ size_t token_row(uint32_t row, uint32_t H, uint32_t T) {
+  const uint32_t bh = row / T, t = row - bh * T, b = bh / H;
+  return ((size_t)b * T + t) * H + (bh - b * H);
+}
 
 // (Where the merge may have blended, a grid of 16 CTAs per SM strides over the rows: a grid of a CTA for every 256
 // vectors took 148 us to come and go at 65536 tokens, 64 heads of 128.)
+// kTokens: `out` is [B, T, Hq, D], as the layer's last GEMM reads it, in place of a pass of its own over the output
+// (8 x 4096 tokens, 12 heads of 64: the layer's two such passes took 47 us of its 2560, this kernel 39 -> 45 and the
+// backward's 43 -> 47 with them; with one launch less the layer's forward on 256 tokens 92.4 -> 87.8).
+template <bool kTokens>
 __global__ void __launch_bounds__(256)
 gate_fwd_vec_kernel(const __nv_bfloat16* __restrict__ oc, const __nv_bfloat16* __restrict__ os,
                     const __nv_bfloat16* __restrict__ ow, const __nv_bfloat16* __restrict__ gate,
                     __nv_bfloat16* __restrict__ out, size_t rows, int VL, const SelPlanHeader* __restrict__ hdr, int nq_union,
-                    int force) {
+                    int force, uint32_t H, uint32_t T) {
   if (hdr != nullptr && tc::prefer_pairs(hdr, nq_union, force)) return;   // the merge of the selection has blended
   const size_t n = rows * VL, stride = (size_t)gridDim.x * blockDim.x;
   for (size_t gid = (size_t)blockIdx.x * blockDim.x + threadIdx.x; gid < n; gid += stride) {
@@ -488,18 +498,22 @@ gate_fwd_vec_kernel(const __nv_bfloat16* __restrict__ oc, const __nv_bfloat16* _
     for (int e = 0; e < 4; ++e)
       rs[e] = __floats2bfloat162_rn(g0 * a[2 * e] + g1 * b[2 * e] + g2 * c[2 * e],
                                     g0 * a[2 * e + 1] + g1 * b[2 * e + 1] + g2 * c[2 * e + 1]);
-    *reinterpret_cast<uint4*>(out + i) = r;
+    *reinterpret_cast<uint4*>(out + (kTokens ? token_row((uint32_t)row, H, T) * VL * 8 + i % (VL * 8) : i)) = r;
   }
 }
 
 // One 16-byte vector of each of the four tensors a thread; three lanes of a row finish a branch each.  Bound by the
 // pass: 4.5 GB in 704 us at 8 x 32768 tokens, 16 heads of 128 (847 with one lane for the three branches and
 // divisions for the row; more vectors a thread change nothing).
+// kTokens: d_out is [B, T, Hq, D], as the layer's GEMM leaves it; the rows in the order of the heads, which the branch
+// kernels fetch, are written on the way to d_heads.
+template <bool kTokens>
 __global__ void __launch_bounds__(256)
 gate_bwd_rows_vec_kernel(const __nv_bfloat16* __restrict__ oc, const __nv_bfloat16* __restrict__ os,
                          const __nv_bfloat16* __restrict__ ow, const __nv_bfloat16* __restrict__ gate,
                          const __nv_bfloat16* __restrict__ d_out, float* __restrict__ row_scale,
-                         float* __restrict__ row_dot, __nv_bfloat16* __restrict__ d_gate, size_t rows, int log_vl) {
+                         float* __restrict__ row_dot, __nv_bfloat16* __restrict__ d_gate, size_t rows, int log_vl,
+                         uint32_t H, uint32_t T, __nv_bfloat16* __restrict__ d_heads) {
   const int VL = 1 << log_vl;
   const size_t gid = (size_t)blockIdx.x * blockDim.x + threadIdx.x, row = gid >> log_vl;
   const bool live = row < rows;                   // the grid is padded to whole warps: no early return
@@ -507,7 +521,14 @@ gate_bwd_rows_vec_kernel(const __nv_bfloat16* __restrict__ oc, const __nv_bfloat
   if (live) {
     const size_t i = gid * 8;
     float g[8], a[8], b[8], c[8];
-    load8(d_out + i, g); load8(oc + i, a); load8(os + i, b); load8(ow + i, c);
+    if (kTokens) {
+      const uint4 u = __ldg(reinterpret_cast<const uint4*>(d_out + (token_row((uint32_t)row, H, T) << (log_vl + 3))) + (gid & (VL - 1)));
+      *reinterpret_cast<uint4*>(d_heads + i) = u;
+      unpack8(u, g);
+    } else {
+      load8(d_out + i, g);
+    }
+    load8(oc + i, a); load8(os + i, b); load8(ow + i, c);
 #pragma unroll
     for (int e = 0; e < 8; ++e) { a0 = fmaf(g[e], a[e], a0); a1 = fmaf(g[e], b[e], a1); a2 = fmaf(g[e], c[e], a2); }
   }
@@ -529,6 +550,9 @@ gate_bwd_rows_vec_kernel(const __nv_bfloat16* __restrict__ oc, const __nv_bfloat
 
 inline bool gate_vec_ok(int D, int dtype) {
   return dtype == NSA_DTYPE_BF16 && D >= 8 && D <= 256 && (D & (D - 1)) == 0;
+}
+inline bool token_major_ok(const NsaDims* d) {
+  return gate_vec_ok(d->D, d->dtype) && (size_t)d->B * d->Hq * d->T <= 0xffffffffu;
 }
 
 // out = a + b + c, fp32 accumulation, 8 elements per thread (bf16) or 4 (fp32)
@@ -961,18 +985,28 @@ extern "C" int nsa_gate_combine_bwd_rows(const void* o_cmp, const void* o_slc, c
                                          const void* gate_logits, const void* d_out, float* row_scale,
                                          float* row_dot, void* d_gate_logits, const NsaDims* dims,
                                          void* stream) {
+  return nsa::gate_bwd_rows(o_cmp, o_slc, o_win, gate_logits, d_out, row_scale, row_dot, d_gate_logits, dims, nullptr, stream);
+}
+
+int nsa::gate_bwd_rows(const void* o_cmp, const void* o_slc, const void* o_win, const void* gate_logits, const void* d_out,
+                       float* row_scale, float* row_dot, void* d_gate_logits, const NsaDims* dims, void* d_heads, void* stream) {
   NSA_CHECK_ARG(dims && row_scale && row_dot && d_gate_logits, "null argument");
   const size_t rows = (size_t)dims->B * dims->Hq * dims->T;
   if (rows == 0) return NSA_OK;
+  NSA_CHECK_ARG(!d_heads || token_major_ok(dims), "token-major rows take bf16 heads of 8 to 256 columns, a power of two");
   cudaStream_t st = (cudaStream_t)stream;
   KernelScope ks("gate_bwd_rows_kernel", st);
-  if (gate_vec_ok(dims->D, dims->dtype))
-  {
+  if (gate_vec_ok(dims->D, dims->dtype)) {
     int log_vl = 0;
     while ((8 << log_vl) < dims->D) ++log_vl;
-    gate_bwd_rows_vec_kernel<<<blocks_for(rows << log_vl, 256), 256, 0, st>>>(
-        (const __nv_bfloat16*)o_cmp, (const __nv_bfloat16*)o_slc, (const __nv_bfloat16*)o_win, (const __nv_bfloat16*)gate_logits,
-        (const __nv_bfloat16*)d_out, row_scale, row_dot, (__nv_bfloat16*)d_gate_logits, rows, log_vl);
+    auto go = [&](auto kernel) {
+      kernel<<<blocks_for(rows << log_vl, 256), 256, 0, st>>>(
+          (const __nv_bfloat16*)o_cmp, (const __nv_bfloat16*)o_slc, (const __nv_bfloat16*)o_win, (const __nv_bfloat16*)gate_logits,
+          (const __nv_bfloat16*)d_out, row_scale, row_dot, (__nv_bfloat16*)d_gate_logits, rows, log_vl, (uint32_t)dims->Hq,
+          (uint32_t)dims->T, (__nv_bfloat16*)d_heads);
+    };
+    if (d_heads) go(gate_bwd_rows_vec_kernel<true>);
+    else go(gate_bwd_rows_vec_kernel<false>);
   }
   else if (dims->dtype == NSA_DTYPE_BF16)
     gate_bwd_rows_kernel<<<blocks_for(rows, 8), 256, 0, st>>>((const __nv_bfloat16*)o_cmp, (const __nv_bfloat16*)o_slc, (const __nv_bfloat16*)o_win, (const __nv_bfloat16*)gate_logits, (const __nv_bfloat16*)d_out, row_scale, row_dot, (__nv_bfloat16*)d_gate_logits, rows, dims->D);
@@ -1204,19 +1238,29 @@ extern "C" int nsa_swap_heads_tokens(const void* src, void* dst, int B, int H, i
 extern "C" int nsa_gate_combine_fwd(const void* o_cmp, const void* o_slc, const void* o_win,
                                     const void* gate_logits, void* out, const NsaDims* dims,
                                     void* stream) {
-  return nsa::gate_fwd_unless_blended(o_cmp, o_slc, o_win, gate_logits, out, dims, nsa::SelChoice{}, stream);
+  return nsa::gate_fwd_unless_blended(o_cmp, o_slc, o_win, gate_logits, out, dims, nsa::SelChoice{}, false, stream);
 }
 
 int nsa::gate_fwd_unless_blended(const void* o_cmp, const void* o_slc, const void* o_win, const void* gate_logits, void* out,
-                                 const NsaDims* dims, const SelChoice& choice, void* stream) {
+                                 const NsaDims* dims, const SelChoice& choice, bool tokens, void* stream) {
   NSA_CHECK_ARG(dims, "null dims");
   const size_t rows = (size_t)dims->B * dims->Hq * dims->T;
   if (rows == 0) return NSA_OK;
+  NSA_CHECK_ARG(!tokens || token_major_ok(dims), "token-major rows take bf16 heads of 8 to 256 columns, a power of two");
   cudaStream_t st = (cudaStream_t)stream;
   unsigned grid = blocks_for(rows * (dims->D / 8), 256);
   if (choice.hdr) grid = std::min(grid, 16u * (unsigned)sm_count());
   if (gate_vec_ok(dims->D, dims->dtype))
-    { KernelScope ks("gate_fwd_kernel", st); gate_fwd_vec_kernel<<<grid, 256, 0, st>>>((const __nv_bfloat16*)o_cmp, (const __nv_bfloat16*)o_slc, (const __nv_bfloat16*)o_win, (const __nv_bfloat16*)gate_logits, (__nv_bfloat16*)out, rows, dims->D / 8, choice.hdr, choice.nq_union, choice.force); }
+  {
+    KernelScope ks("gate_fwd_kernel", st);
+    auto go = [&](auto kernel) {
+      kernel<<<grid, 256, 0, st>>>((const __nv_bfloat16*)o_cmp, (const __nv_bfloat16*)o_slc, (const __nv_bfloat16*)o_win,
+                                   (const __nv_bfloat16*)gate_logits, (__nv_bfloat16*)out, rows, dims->D / 8, choice.hdr,
+                                   choice.nq_union, choice.force, (uint32_t)dims->Hq, (uint32_t)dims->T);
+    };
+    if (tokens) go(gate_fwd_vec_kernel<true>);
+    else go(gate_fwd_vec_kernel<false>);
+  }
   else if (dims->dtype == NSA_DTYPE_BF16)
     { KernelScope ks("gate_fwd_kernel", st); gate_fwd_kernel<<<blocks_for(rows, 8), 256, 0, st>>>((const __nv_bfloat16*)o_cmp, (const __nv_bfloat16*)o_slc, (const __nv_bfloat16*)o_win, (const __nv_bfloat16*)gate_logits, (__nv_bfloat16*)out, rows, dims->D); }
   else

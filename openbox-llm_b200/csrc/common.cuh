@@ -159,6 +159,7 @@ struct AttnArgs {
   // where o_kept says so
   const void *g_cmp, *g_win, *g_logits;
   void *g_out, *o_kept;
+  bool g_tokens;          // g_out is [B, T, Hq, D]
   bool plan_kept;         // the plan outlives the dQ reduction: the backward need not copy its pair map
   // window backward without a dq of its own: who reads the partials knows that they may lie in tiles of 128 keys (a caller
   // who names neither the key count nor the options to nsa_dq_reduce3 gets them in tiles of 64)

@@ -264,8 +264,9 @@ extern "C" int nsa_attention_sizes(const NsaAttentionDesc* desc, size_t* saved_b
   return NSA_OK;
 }
 
-extern "C" int nsa_attention_fwd(const NsaAttentionDesc* d, const NsaAttentionTensors* t, void* saved,
-                                 void* workspace, size_t workspace_bytes, void* stream) {
+// tokens: `out` is [B, T, Hq, D]
+static int attention_fwd(const NsaAttentionDesc* d, const NsaAttentionTensors* t, void* saved, void* workspace,
+                         size_t workspace_bytes, bool tokens, void* stream) {
   NSA_CHECK_ARG(d && t, "null argument");
   OpPlan p;
   NSA_TRY(op_plan(d, &p));
@@ -303,6 +304,7 @@ extern "C" int nsa_attention_fwd(const NsaAttentionDesc* d, const NsaAttentionTe
       if (!fork.active()) {              // the other branches lie before this one: its merge can blend them
         a.g_cmp = o[0]; a.g_win = o[2]; a.g_logits = t->gate; a.g_out = t->out;
         a.o_kept = d->need_grad ? o[1] : nullptr;
+        a.g_tokens = tokens;
         choice = tc_sel_choice(a, plan);
       }
       return tc_sel_fwd(a, workspace, workspace_bytes, s);
@@ -349,12 +351,23 @@ extern "C" int nsa_attention_fwd(const NsaAttentionDesc* d, const NsaAttentionTe
     }
     NSA_TRY(fork.join(1));
   }
-  NSA_TRY(gate_fwd_unless_blended(o[0], o[1], o[2], t->gate, t->out, &m, choice, stream));
+  NSA_TRY(gate_fwd_unless_blended(o[0], o[1], o[2], t->gate, t->out, &m, choice, tokens, stream));
   return fork.join();                    // a plan that only the backward reads
 }
 
-extern "C" int nsa_attention_bwd(const NsaAttentionDesc* d, const NsaAttentionTensors* t, const void* saved,
-                                 void* workspace, size_t workspace_bytes, void* stream) {
+extern "C" int nsa_attention_fwd(const NsaAttentionDesc* d, const NsaAttentionTensors* t, void* saved, void* workspace,
+                                 size_t workspace_bytes, void* stream) {
+  return attention_fwd(d, t, saved, workspace, workspace_bytes, false, stream);
+}
+
+extern "C" int nsa_attention_fwd_tokens(const NsaAttentionDesc* d, const NsaAttentionTensors* t, void* saved, void* workspace,
+                                        size_t workspace_bytes, void* stream) {
+  return attention_fwd(d, t, saved, workspace, workspace_bytes, true, stream);
+}
+
+// d_tokens: d_out in [B, T, Hq, D], which this call writes to t->d_out in the order of the heads (null: it is there)
+static int attention_bwd(const NsaAttentionDesc* d, const NsaAttentionTensors* t, const void* saved, void* workspace,
+                         size_t workspace_bytes, const void* d_tokens, void* stream) {
   NSA_CHECK_ARG(d && t, "null argument");
   OpPlan p;
   NSA_TRY(op_plan(d, &p));
@@ -403,7 +416,8 @@ extern "C" int nsa_attention_bwd(const NsaAttentionDesc* d, const NsaAttentionTe
   if (p.acc_bytes) NSA_CUDA_OK(cudaMemsetAsync(w + p.acc, 0, p.acc_bytes, st));
   if (acc_mode) NSA_CUDA_OK(cudaMemsetAsync(dq_acc, 0, p.n_q * sizeof(float), st));
   // gate backward as per-row statistics; the branch kernels apply the gate factor themselves
-  NSA_TRY(nsa_gate_combine_bwd_rows(o[0], o[1], o[2], t->gate, t->d_out, rs[0], rd[0], t->d_gate, &m, stream));
+  NSA_TRY(gate_bwd_rows(o[0], o[1], o[2], t->gate, d_tokens ? d_tokens : t->d_out, rs[0], rd[0], t->d_gate, &m,
+                        d_tokens ? const_cast<void*>(t->d_out) : nullptr, stream));
   Fork fork(st, small_problem(d));
   NSA_TRY(fork.begin());
   cudaStream_t s_win = fork.stream(0), s_cmp = fork.stream(1);
@@ -472,4 +486,15 @@ extern "C" int nsa_attention_bwd(const NsaAttentionDesc* d, const NsaAttentionTe
     return tc_dq_reduce3(a, 0, 0, 0, p.S, d->block_size, 1, nullptr, ws[1], nullptr, pos, dq_acc, t->dq, st);
   return tc_dq_reduce3(a, p.n_cmp, d->cmp_len, d->cmp_stride, p.S, d->block_size, d->window,
                        p.n_cmp > 0 ? ws[0] : nullptr, ws[1], ws[2], pos, nullptr, t->dq, st);
+}
+
+extern "C" int nsa_attention_bwd(const NsaAttentionDesc* d, const NsaAttentionTensors* t, const void* saved, void* workspace,
+                                 size_t workspace_bytes, void* stream) {
+  return attention_bwd(d, t, saved, workspace, workspace_bytes, nullptr, stream);
+}
+
+extern "C" int nsa_attention_bwd_tokens(const NsaAttentionDesc* d, const NsaAttentionTensors* t, const void* saved,
+                                        void* workspace, size_t workspace_bytes, const void* d_tokens, void* stream) {
+  NSA_CHECK_ARG(d_tokens || !t || !t->d_out, "null tensor");
+  return attention_bwd(d, t, saved, workspace, workspace_bytes, d_tokens, stream);
 }

@@ -28,6 +28,7 @@ namespace tc {
 struct GateBlend {
   const __nv_bfloat16 *cmp, *win, *logits;
   __nv_bfloat16* out;
+  bool tokens;                             // out is [B, T, Hq, D]
 };
 template <int D, int H>
 __global__ void __launch_bounds__(256, 3)
@@ -125,7 +126,8 @@ sel_combine_kernel(const __nv_bfloat16* o_part, const float* ml,
                              gate[2] * __uint_as_float(xw[e] << 16),
                          gate[0] * __uint_as_float(xc[e] & 0xffff0000u) + gate[1] * __uint_as_float(xs[e] & 0xffff0000u) +
                              gate[2] * __uint_as_float(xw[e] & 0xffff0000u));
-      *reinterpret_cast<uint4*>(gb.out + orow * D + v * 8) = make_uint4(r[0], r[1], r[2], r[3]);
+      const size_t at = gb.tokens ? ((size_t)b * T + t) * Hq + hkv * G + g + h : orow;
+      *reinterpret_cast<uint4*>(gb.out + at * D + v * 8) = make_uint4(r[0], r[1], r[2], r[3]);
     }
     if (v == 0) lse[orow] = L[h] > 0.f ? (M[h] + log2f(L[h])) * kLn2 : kLseEmpty;
   }
@@ -230,7 +232,7 @@ int tc_sel_fwd(const AttnArgs& a, void* ws, size_t ws_bytes, cudaStream_t st) {
     NSA_CUDA_OK(launch_chained(kernel, cgrid, 256, 0, st, (const __nv_bfloat16*)(base + pl.off_part), (const float*)(base + pl.off_ml),
                                plan.pair_of_slot, plan.hdr, (__nv_bfloat16*)(a.g_out ? a.o_kept : a.o), a.lse,
                                GateBlend{(const __nv_bfloat16*)a.g_cmp, (const __nv_bfloat16*)a.g_win,
-                                         (const __nv_bfloat16*)a.g_logits, (__nv_bfloat16*)a.g_out},
+                                         (const __nv_bfloat16*)a.g_logits, (__nv_bfloat16*)a.g_out, a.g_tokens},
                                a.B, a.Hq, a.Hkv, a.T, G, a.S, nq_union, force));
     return NSA_OK;
   };

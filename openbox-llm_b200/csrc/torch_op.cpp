@@ -107,13 +107,14 @@ NsaAttentionTensors pointers(const Tensor* in, const Tensor* comp, const Tensor&
 }
 
 // out; `saved` keeps what backward reads.  Makes c.block_idx where the scorer writes it.
-Tensor op_forward(Call& c, bool need_grad, Tensor* saved) {
+// tokens: the shape of an output in token order ([B, T, Hq, D] elements)
+Tensor op_forward(Call& c, bool need_grad, Tensor* saved, at::IntArrayRef tokens = {}) {
   const Tensor& q = c.in[0];
   c.d.need_grad = need_grad;
   if (!c.d.given_lists) c.block_idx = fresh({c.d.dims.B, c.d.dims.Hkv, c.d.dims.T, c.d.n_sel}, at::kInt, q);
   size_t keep, fwd, bwd;
   check(nsa_attention_sizes(&c.d, &keep, &fwd, &bwd));
-  Tensor out = fresh_like(q);
+  Tensor out = tokens.empty() ? fresh_like(q) : fresh(tokens, q.scalar_type(), q);
   Tensor mem = bytes_like(keep + (need_grad ? 0 : fwd) + 1, q), ws;
   void* ws_ptr = (char*)mem.data_ptr() + keep;
   if (need_grad && fwd) {
@@ -122,14 +123,14 @@ Tensor op_forward(Call& c, bool need_grad, Tensor* saved) {
   }
   NsaAttentionTensors t = pointers(c.in, c.comp, c.block_idx, c.d.learned);
   t.out = out.data_ptr();
-  check(nsa_attention_fwd(&c.d, &t, mem.data_ptr(), ws_ptr, fwd, raw_stream(q)));
+  check((tokens.empty() ? nsa_attention_fwd : nsa_attention_fwd_tokens)(&c.d, &t, mem.data_ptr(), ws_ptr, fwd, raw_stream(q)));
   *saved = mem;
   return out;
 }
 
-// d_in: the eight gradients, allocated by the caller
+// d_in: the eight gradients, allocated by the caller.  d_tokens: the output's gradient in [B, T, Hq, D]; d_out is scratch then.
 void op_backward(const NsaAttentionDesc& d, const Tensor* in, const Tensor* comp, const Tensor& block_idx, const Tensor& saved,
-                 const Tensor& d_out, const Tensor* d_in, Tensor* d_comp) {
+                 const Tensor& d_out, const Tensor* d_in, Tensor* d_comp, const Tensor* d_tokens = nullptr) {
   size_t keep, fwd, bwd;
   check(nsa_attention_sizes(&d, &keep, &fwd, &bwd));
   NsaAttentionTensors t = pointers(in, comp, block_idx, d.learned);
@@ -141,7 +142,8 @@ void op_backward(const NsaAttentionDesc& d, const Tensor* in, const Tensor* comp
     t.d_comp[k] = d_comp[k].data_ptr<float>();
   }
   Tensor ws = bytes_like(bwd + 1, d_out);
-  check(nsa_attention_bwd(&d, &t, saved.data_ptr(), ws.data_ptr(), bwd, raw_stream(d_out)));
+  if (d_tokens) check(nsa_attention_bwd_tokens(&d, &t, saved.data_ptr(), ws.data_ptr(), bwd, d_tokens->data_ptr(), raw_stream(d_out)));
+  else check(nsa_attention_bwd(&d, &t, saved.data_ptr(), ws.data_ptr(), bwd, raw_stream(d_out)));
 }
 
 // A descriptor travels to the backward as a list of integers.
@@ -229,7 +231,7 @@ struct OpLearned : torch::autograd::Function<OpLearned> {
 // ---- the layer under bf16 autocast: projections, op and out_proj in one node ----------------------------
 // One launch casts x and the nine weights, laid out as the GEMMs read them; the gradients of x and the
 // weights leave their GEMMs in fp32, the K / V gradients of the six branches land in one buffer and the bias
-// row is summed over its own columns.  In place of torch's nodes and modules: 8 x 4096 tokens, 12 heads
+// row is summed over its own columns.  The op reads and writes the tokens of out_proj's GEMMs itself.  In place of torch's nodes and modules: 8 x 4096 tokens, 12 heads
 // of 64, forward + backward 3165 -> 2984 us; 256 tokens, forward, 271 -> 94.
 struct Layer {
   Call c;
@@ -270,9 +272,7 @@ struct LayerNode : torch::autograd::Function<LayerNode> {
     check(nsa_split_heads(y.data_ptr(), c.in[0].data_ptr(), kv.data_ptr(), c.in[7].data_ptr(), m.B, m.T, m.Hq, m.Hkv, m.D,
                           NSA_DTYPE_BF16, raw_stream(l.x)));
     Tensor saved;
-    Tensor o = op_forward(c, need_grad, &saved);
-    Tensor tokens = fresh({rows, hd}, at::kBFloat16, l.x);
-    check(nsa_swap_heads_tokens(o.data_ptr(), tokens.data_ptr(), m.B, m.Hq, m.T, m.D, NSA_DTYPE_BF16, 1, raw_stream(l.x)));
+    Tensor tokens = op_forward(c, need_grad, &saved, {rows, hd});
     Tensor out = at::mm(tokens, w_out.t()).view({l.B, l.T, l.dm});
     if (keep) {
       bool weights = false;
@@ -328,12 +328,11 @@ struct LayerNode : torch::autograd::Function<LayerNode> {
     if (ctx->needs_input_grad(10)) res[11] = at::mm(dy.t(), tokens, at::kFloat);
     if (!op_any) return res;
     Tensor d_tokens = at::mm(dy, w_out), d_out = fresh({m.B, m.Hq, m.T, m.D}, at::kBFloat16, kv);
-    check(nsa_swap_heads_tokens(d_tokens.data_ptr(), d_out.data_ptr(), m.B, m.Hq, m.T, m.D, NSA_DTYPE_BF16, 0, raw_stream(dy)));
     Tensor d_in[8], d_comp[6], d_kv = fresh_like(kv);
     d_in[0] = fresh_like(in[0]);
     d_in[7] = fresh_like(in[7]);
     for (int k = 0; k < 6; ++k) d_in[1 + k] = d_kv.select(0, k);
-    op_backward(d, in, kept.data() + 9, kept[3], kept[4], d_out, d_in, d_comp);
+    op_backward(d, in, kept.data() + 9, kept[3], kept[4], d_out, d_in, d_comp, &d_tokens);
     for (int k = 0; k < 6; ++k) res[12 + k] = d_comp[k];
     if (!rows_any) return res;
     Tensor d_rows = fresh({rows, width}, at::kBFloat16, kv);
