@@ -73,3 +73,25 @@ def test_token_rows_of_other_types_are_refused():
     t = L.OP_TENSORS(*[v.data_ptr() for v in x], *(None,) * 6, idx.data_ptr(), out.data_ptr())
     with pytest.raises(nsa.NsaError, match="token-major"):
         L.check(lib.nsa_attention_fwd_tokens(d, t, mem[0].data_ptr(), mem[1].data_ptr(), n[1].value, L.stream()))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", ["bf16", "f32"])
+@pytest.mark.parametrize("c", [(3, 3001, 12, 4, 64), (2, 33, 3, 1, 8), (1, 7, 8, 2, 128), (1, 4097, 64, 4, 64)], ids=str)
+def test_projection_rows(c, dtype):
+    """Rows of the fused projection <-> heads, every element, on both sides of the line between one token and eight a thread;
+    the padding behind the gates comes back as zeros."""
+    B, T, Hq, Hkv, D = c
+    L, lib = pkg()._lib, pkg().lib()
+    dt = torch.bfloat16 if dtype == "bf16" else torch.float32
+    code = L.DTYPE_BF16 if dtype == "bf16" else L.DTYPE_F32
+    W, n = lib.nsa_fused_projection_width(Hq, Hkv, D), (Hq + 6 * Hkv) * D
+    y = torch.randn(B, T, W, device="cuda").to(dt)
+    q, kv, gate = (torch.full(s, float("nan"), device="cuda", dtype=dt) for s in ((B, Hq, T, D), (6, B, Hkv, T, D), (B, Hq, T, 3)))
+    L.check(lib.nsa_split_heads(y.data_ptr(), q.data_ptr(), kv.data_ptr(), gate.data_ptr(), B, T, Hq, Hkv, D, code, L.stream()))
+    assert torch.equal(q, y[..., :Hq * D].view(B, T, Hq, D).transpose(1, 2))
+    assert torch.equal(kv, y[..., Hq * D:n].view(B, T, 6, Hkv, D).permute(2, 0, 3, 1, 4))
+    assert torch.equal(gate, y[..., n:n + 3 * Hq].view(B, T, Hq, 3).transpose(1, 2))
+    back = torch.full_like(y, float("nan"))
+    L.check(lib.nsa_merge_heads(q.data_ptr(), kv.data_ptr(), gate.data_ptr(), back.data_ptr(), B, T, Hq, Hkv, D, code, L.stream()))
+    assert torch.equal(back[..., :n + 3 * Hq], y[..., :n + 3 * Hq]) and not back[..., n + 3 * Hq:].any()
