@@ -507,16 +507,19 @@ gate_fwd_vec_kernel(const __nv_bfloat16* __restrict__ oc, const __nv_bfloat16* _
 // divisions for the row; more vectors a thread change nothing).
 // kTokens: d_out is [B, T, Hq, D], as the layer's GEMM leaves it; the rows in the order of the heads, which the branch
 // kernels fetch, are written on the way to d_heads.
+// `zeros`: what the pooling's backward, which follows in the op, adds to; a memset of its own cost a launch (5 us of host work,
+// what a pass over 1024 tokens is bound by).
 template <bool kTokens>
 __global__ void __launch_bounds__(256)
 gate_bwd_rows_vec_kernel(const __nv_bfloat16* __restrict__ oc, const __nv_bfloat16* __restrict__ os,
                          const __nv_bfloat16* __restrict__ ow, const __nv_bfloat16* __restrict__ gate,
                          const __nv_bfloat16* __restrict__ d_out, float* __restrict__ row_scale,
                          float* __restrict__ row_dot, __nv_bfloat16* __restrict__ d_gate, size_t rows, int log_vl,
-                         uint32_t H, uint32_t T, __nv_bfloat16* __restrict__ d_heads) {
+                         uint32_t H, uint32_t T, __nv_bfloat16* __restrict__ d_heads, float* __restrict__ zeros, size_t n_zeros) {
   const int VL = 1 << log_vl;
   const size_t gid = (size_t)blockIdx.x * blockDim.x + threadIdx.x, row = gid >> log_vl;
   const bool live = row < rows;                   // the grid is padded to whole warps: no early return
+  for (size_t z = gid; z < n_zeros; z += (size_t)gridDim.x * blockDim.x) zeros[z] = 0.f;
   float a0 = 0.f, a1 = 0.f, a2 = 0.f;
   if (live) {
     const size_t i = gid * 8;
@@ -985,25 +988,28 @@ extern "C" int nsa_gate_combine_bwd_rows(const void* o_cmp, const void* o_slc, c
                                          const void* gate_logits, const void* d_out, float* row_scale,
                                          float* row_dot, void* d_gate_logits, const NsaDims* dims,
                                          void* stream) {
-  return nsa::gate_bwd_rows(o_cmp, o_slc, o_win, gate_logits, d_out, row_scale, row_dot, d_gate_logits, dims, nullptr, stream);
+  return nsa::gate_bwd_rows(o_cmp, o_slc, o_win, gate_logits, d_out, row_scale, row_dot, d_gate_logits, dims, nullptr, nullptr, 0, stream);
 }
 
 int nsa::gate_bwd_rows(const void* o_cmp, const void* o_slc, const void* o_win, const void* gate_logits, const void* d_out,
-                       float* row_scale, float* row_dot, void* d_gate_logits, const NsaDims* dims, void* d_heads, void* stream) {
+                       float* row_scale, float* row_dot, void* d_gate_logits, const NsaDims* dims, void* d_heads, float* zeros,
+                       size_t n_zeros, void* stream) {
   NSA_CHECK_ARG(dims && row_scale && row_dot && d_gate_logits, "null argument");
   const size_t rows = (size_t)dims->B * dims->Hq * dims->T;
   if (rows == 0) return NSA_OK;
   NSA_CHECK_ARG(!d_heads || token_major_ok(dims), "token-major rows take bf16 heads of 8 to 256 columns, a power of two");
   cudaStream_t st = (cudaStream_t)stream;
+  const bool vec = gate_vec_ok(dims->D, dims->dtype);
+  if (n_zeros && !vec) NSA_CUDA_OK(cudaMemsetAsync(zeros, 0, n_zeros * sizeof(float), st));
   KernelScope ks("gate_bwd_rows_kernel", st);
-  if (gate_vec_ok(dims->D, dims->dtype)) {
+  if (vec) {
     int log_vl = 0;
     while ((8 << log_vl) < dims->D) ++log_vl;
     auto go = [&](auto kernel) {
       kernel<<<blocks_for(rows << log_vl, 256), 256, 0, st>>>(
           (const __nv_bfloat16*)o_cmp, (const __nv_bfloat16*)o_slc, (const __nv_bfloat16*)o_win, (const __nv_bfloat16*)gate_logits,
           (const __nv_bfloat16*)d_out, row_scale, row_dot, (__nv_bfloat16*)d_gate_logits, rows, log_vl, (uint32_t)dims->Hq,
-          (uint32_t)dims->T, (__nv_bfloat16*)d_heads);
+          (uint32_t)dims->T, (__nv_bfloat16*)d_heads, zeros, n_zeros);
     };
     if (d_heads) go(gate_bwd_rows_vec_kernel<true>);
     else go(gate_bwd_rows_vec_kernel<false>);

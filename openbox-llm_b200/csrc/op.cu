@@ -413,11 +413,10 @@ static int attention_bwd(const NsaAttentionDesc* d, const NsaAttentionTensors* t
     ws[k] = w + p.ws[k];
     dq[k] = p.fused ? nullptr : w + p.dq3 + k * p.n_q * p.es;
   }
-  if (p.acc_bytes) NSA_CUDA_OK(cudaMemsetAsync(w + p.acc, 0, p.acc_bytes, st));
   if (acc_mode) NSA_CUDA_OK(cudaMemsetAsync(dq_acc, 0, p.n_q * sizeof(float), st));
   // gate backward as per-row statistics; the branch kernels apply the gate factor themselves
   NSA_TRY(gate_bwd_rows(o[0], o[1], o[2], t->gate, d_tokens ? d_tokens : t->d_out, rs[0], rd[0], t->d_gate, &m,
-                        d_tokens ? const_cast<void*>(t->d_out) : nullptr, stream));
+                        d_tokens ? const_cast<void*>(t->d_out) : nullptr, (float*)(w + p.acc), p.acc_bytes / sizeof(float), stream));
   Fork fork(st, small_problem(d));
   NSA_TRY(fork.begin());
   cudaStream_t s_win = fork.stream(0), s_cmp = fork.stream(1);

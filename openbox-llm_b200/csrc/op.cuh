@@ -13,8 +13,10 @@ int topn_check(const NsaDims* dims, int n_cmp, int cmp_len, int cmp_stride, int 
 // nsa_gate_combine_fwd, unless the block-outer kernel has served the selection (a choice without header: always)
 int gate_fwd_unless_blended(const void* o_cmp, const void* o_slc, const void* o_win, const void* gate_logits, void* out,
                             const NsaDims* dims, const SelChoice& choice, bool tokens, void* stream);   // aux.cu
-// nsa_gate_combine_bwd_rows; with d_heads, d_out is token-major and its rows are written there in the order of the heads
+// nsa_gate_combine_bwd_rows; with d_heads, d_out is token-major and its rows are written there in the order of the heads;
+// n_zeros floats are zeroed
 int gate_bwd_rows(const void* o_cmp, const void* o_slc, const void* o_win, const void* gate_logits, const void* d_out,
-                  float* row_scale, float* row_dot, void* d_gate_logits, const NsaDims* dims, void* d_heads, void* stream);   // aux.cu
+                  float* row_scale, float* row_dot, void* d_gate_logits, const NsaDims* dims, void* d_heads, float* zeros, size_t n_zeros,
+                  void* stream);   // aux.cu
 bool profiling();     // every launch is bracketed by events on its stream: branches must not overlap
 }  // namespace nsa
