@@ -100,6 +100,15 @@ class Fork {
     for (int k = 0; k < 2; ++k) NSA_CUDA_OK(cudaStreamWaitEvent(side_->st[k], side_->begin, 0));
     return NSA_OK;
   }
+  // What side stream k holds so far is all that a later wait(k) has `main` wait for (no join of k between the two).
+  int mark(int k) {
+    if (side_) NSA_CUDA_OK(cudaEventRecord(side_->end[k], side_->st[k]));
+    return NSA_OK;
+  }
+  int wait(int k) {
+    if (side_) NSA_CUDA_OK(cudaStreamWaitEvent(main_, side_->end[k], 0));
+    return NSA_OK;
+  }
   int join(int which = 3) {                        // `main` waits for the side streams of the mask
     NSA_CUDA_OK(rejoin(open_ & which));
     return NSA_OK;
@@ -430,6 +439,7 @@ static int attention_bwd(const NsaAttentionDesc* d, const NsaAttentionTensors* t
     NSA_TRY(nsa_range_attn_bwd(t->q, k_cmp, v_cmp, o[0], lse[0], t->d_out, dq[0], dk_cmp, dv_cmp, &m, p.n_cmp,
                                NSA_MODE_COMPRESS_STRIDED, d->cmp_stride, d->cmp_len, rs[0], rd[0], ws[0], p.ws_bytes[0],
                                d->impl, s_cmp));
+  NSA_TRY(fork.mark(1));
   if (p.fast_pool) {
     PoolSides s = op_sides(d, t);
     s.d_out[0] = dk_cmp; s.d_out[1] = dv_cmp;
@@ -474,17 +484,24 @@ static int attention_bwd(const NsaAttentionDesc* d, const NsaAttentionTensors* t
   else
     NSA_TRY(window_bwd(t->q, t->kw, t->vw, o[2], lse[2], t->d_out, dq[2], t->dkw, t->dvw, &m, d->window, rs[2], rd[2],
                        ws[2], p.ws_bytes[2], d->impl, s_win));
-  NSA_TRY(fork.join());
-  if (!p.fused) return nsa_sum3(dq[0], dq[1], dq[2], t->dq, p.n_q, m.dtype, stream);
+  // the sum of dq needs the compression's attention, not the pooling behind it, which runs beside the sum
+  NSA_TRY(fork.join(1));
+  NSA_TRY(fork.wait(1));
+  if (!p.fused) {
+    NSA_TRY(nsa_sum3(dq[0], dq[1], dq[2], t->dq, p.n_q, m.dtype, stream));
+    return fork.join();
+  }
   // the three branches left their dQ partials in their workspaces (or two of them in the accumulator)
   AttnArgs a = base_args(&m, m.T);
   a.three_term = p.three_term;
   a.wide_dq = true;
   const int32_t* pos = sel_plan_pair_map(a, p.S, d->block_size, sv + p.plan);
   if (acc_mode)
-    return tc_dq_reduce3(a, 0, 0, 0, p.S, d->block_size, 1, nullptr, ws[1], nullptr, pos, dq_acc, t->dq, st);
-  return tc_dq_reduce3(a, p.n_cmp, d->cmp_len, d->cmp_stride, p.S, d->block_size, d->window,
-                       p.n_cmp > 0 ? ws[0] : nullptr, ws[1], ws[2], pos, nullptr, t->dq, st);
+    NSA_TRY(tc_dq_reduce3(a, 0, 0, 0, p.S, d->block_size, 1, nullptr, ws[1], nullptr, pos, dq_acc, t->dq, st));
+  else
+    NSA_TRY(tc_dq_reduce3(a, p.n_cmp, d->cmp_len, d->cmp_stride, p.S, d->block_size, d->window,
+                          p.n_cmp > 0 ? ws[0] : nullptr, ws[1], ws[2], pos, nullptr, t->dq, st));
+  return fork.join();
 }
 
 extern "C" int nsa_attention_bwd(const NsaAttentionDesc* d, const NsaAttentionTensors* t, const void* saved, void* workspace,
