@@ -1393,13 +1393,41 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
   if (warp == 0) tmem_dealloc(tmem, kTmemCols);
 }
 
+// Selection blocks whose row tiles were split over several work items collect dK / dV in the fp32 accumulators.  The rows of
+// those blocks are cleared before the backward kernel and turned into the bf16 outputs after it, a CTA to a key tile.
+// Where the call has a delta kernel its first CTAs clear them.  Bound by latency: 16 bytes a thread and access (8192 tokens, 16
+// heads of 64: the two kernels of scalar loops took 13.1 us, now 6.4 and 0.9 in the delta kernel; 8 x 32768 of 128 88 -> 55).
+struct SplitTiles {
+  const int32_t* offsets;                // null: no block is split
+  float *dk_acc, *dv_acc;
+  int n_ktiles, units, nq, Lk, D;
+  // elements of key tile `tile` (of all units) if it is split, else 0; base: its first element
+  __device__ __forceinline__ int elements(unsigned tile, size_t* base) const {
+    const int bh = (int)(tile / (unsigned)n_ktiles), j = (int)(tile % (unsigned)n_ktiles);
+    const int32_t* at = offsets + (size_t)bh * (n_ktiles + 1) + j;
+    const int n_rt = (ld_plain(at + 1) - ld_plain(at) + nq - 1) / nq;
+    *base = ((size_t)bh * Lk + (size_t)j * kKeys) * D;
+    return n_rt <= kSelChunkTiles ? 0 : min(kKeys, Lk - j * kKeys) * D;       // one work item: written directly
+  }
+  __device__ __forceinline__ void clear(unsigned tile) const {
+    size_t base;
+    const int n = elements(tile, &base);
+    const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int i = threadIdx.x * 4; i < n; i += blockDim.x * 4) {
+      *reinterpret_cast<float4*>(dk_acc + base + i) = z;
+      *reinterpret_cast<float4*>(dv_acc + base + i) = z;
+    }
+  }
+};
+
 // delta[b,h,t] = sum_d dO * O (fp32), D / 8 lanes to a row, one 16-byte vector of each: bound by the pass over both (16
 // heads x 8192 rows of 64: 6 us, 18 with a warp to a row).
 template <int D>
 __global__ void delta_kernel(const __nv_bfloat16* d_o, const __nv_bfloat16* o,
-                             float* delta, size_t rows, bool vec) {
+                             float* delta, size_t rows, bool vec, const SplitTiles split) {
   chain_wait();
   chain_go();
+  if (split.offsets && blockIdx.x < (unsigned)(split.n_ktiles * split.units)) split.clear(blockIdx.x);
   constexpr int kLanes = D / 8;
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x, row = i / kLanes;
   float s = 0.f;
@@ -1586,28 +1614,26 @@ static int reduce_launch(const Reduce3Args& r, int D, bool f32, const char* name
   return NSA_OK;
 }
 
-// Selection blocks whose row tiles were split over several work items collect dK / dV in the fp32
-// accumulators: this kernel clears the accumulator rows of those blocks before the backward
-// kernel (finalize = 0) and turns them into the bf16 outputs after it (finalize = 1).
-__global__ void sel_split_blocks_kernel(const int32_t* offsets, float* dk_acc,
-                                        float* dv_acc, __nv_bfloat16* dk,
-                                        __nv_bfloat16* dv, int n_ktiles, int nq, int Lk, int D,
-                                        int finalize) {
+__global__ void __launch_bounds__(256) sel_split_clear_kernel(const SplitTiles x) {
   chain_wait();
   chain_go();
-  const int j = blockIdx.x, bh = blockIdx.y;
-  const int n_q = offsets[(size_t)bh * (n_ktiles + 1) + j + 1] - offsets[(size_t)bh * (n_ktiles + 1) + j];
-  const int n_rt = (n_q + nq - 1) / nq;
-  if (n_rt <= kSelChunkTiles) return;                 // one work item: written directly
-  const int rows = min(kKeys, Lk - j * kKeys);
-  const size_t base = ((size_t)bh * Lk + (size_t)j * kKeys) * D;
-  for (int i = threadIdx.x; i < rows * D; i += blockDim.x) {
-    if (finalize) {
-      dk[base + i] = __float2bfloat16_rn(dk_acc[base + i]);
-      dv[base + i] = __float2bfloat16_rn(dv_acc[base + i]);
-    } else {
-      dk_acc[base + i] = 0.f;
-      dv_acc[base + i] = 0.f;
+  x.clear(blockIdx.x);
+}
+__global__ void __launch_bounds__(256) sel_split_finish_kernel(const SplitTiles x, __nv_bfloat16* dk, __nv_bfloat16* dv, bool vec) {
+  chain_wait();
+  chain_go();
+  size_t base;
+  const int n = x.elements(blockIdx.x, &base);
+#pragma unroll 4
+  for (int i = threadIdx.x * 4; i < n; i += 256 * 4) {
+    const float4 k = __ldcs(reinterpret_cast<const float4*>(x.dk_acc + base + i)), v = __ldcs(reinterpret_cast<const float4*>(x.dv_acc + base + i));
+    const uint2 uk = make_uint2(pack_bf16(k.x, k.y), pack_bf16(k.z, k.w)), uv = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
+    if (vec) {
+      *reinterpret_cast<uint2*>(dk + base + i) = uk;
+      *reinterpret_cast<uint2*>(dv + base + i) = uv;
+    } else {                                           // a caller's tensor may start anywhere
+      const __nv_bfloat16 *ek = reinterpret_cast<const __nv_bfloat16*>(&uk), *ev = reinterpret_cast<const __nv_bfloat16*>(&uv);
+      for (int e = 0; e < 4; ++e) { dk[base + i + e] = ek[e]; dv[base + i + e] = ev[e]; }
     }
   }
 }
@@ -1861,15 +1887,6 @@ int tc_attn_bwd(const AttnArgs& a, void* ws, size_t ws_bytes, cudaStream_t st) {
   if (pl.n_splits > 1 && !ordered)
     NSA_CUDA_OK(cudaMemsetAsync(base + pl.off_acc, 0, 2 * align_up(n_kv * sizeof(float), 256), st));
 
-  const size_t rows = (size_t)a.B * a.Hq * a.T;
-  if (!a.row_dot) {
-    KernelScope ks("delta_kernel", st);
-    const unsigned dgrid = (unsigned)((rows * (a.D / 8) + 255) / 256);
-    const auto *d_o = (const __nv_bfloat16*)a.d_o, *o = (const __nv_bfloat16*)a.o;
-    NSA_CUDA_OK(launch_chained(a.D == 128 ? delta_kernel<128> : delta_kernel<64>, dgrid, 256, 0, st, d_o, o,
-                               (float*)(base + pl.off_delta), rows, aligned16(d_o, o)));
-  }
-  NSA_LAUNCH_OK("delta_kernel");
   if (a.kind == 2) {
     const void* plan_mem = a.sel_plan;
     if (!plan_mem) {
@@ -1882,10 +1899,21 @@ int tc_attn_bwd(const AttnArgs& a, void* ws, size_t ws_bytes, cudaStream_t st) {
     }
     p.plan = sel_plan_at(plan_mem, pl.layout);
   }
-  if (pl.sel_split) {
-    KernelScope ks("sel_split_blocks_kernel", st);
-    NSA_CUDA_OK(launch_chained(sel_split_blocks_kernel, dim3(pl.n_ktiles, a.B * a.Hkv), 256, 0, st, p.plan.offsets, p.dk_acc, p.dv_acc,
-                               p.dk, p.dv, pl.n_ktiles, pl.nq, a.Lk, a.D, 0));
+  const SplitTiles split = {pl.sel_split ? p.plan.offsets : nullptr, p.dk_acc, p.dv_acc, pl.n_ktiles, a.B * a.Hkv, pl.nq, a.Lk, a.D};
+  const unsigned n_split = (unsigned)(pl.n_ktiles * a.B * a.Hkv);
+  const size_t rows = (size_t)a.B * a.Hq * a.T;
+  if (!a.row_dot) {
+    // (at least two CTAs for each key tile: its first ones clear the accumulators as well)
+    KernelScope ks("delta_kernel", st);
+    const unsigned dgrid = (unsigned)((rows * (a.D / 8) + 255) / 256);
+    const auto *d_o = (const __nv_bfloat16*)a.d_o, *o = (const __nv_bfloat16*)a.o;
+    NSA_CUDA_OK(launch_chained(a.D == 128 ? delta_kernel<128> : delta_kernel<64>, std::max(dgrid, split.offsets ? n_split : 0u), 256, 0,
+                               st, d_o, o, (float*)(base + pl.off_delta), rows, aligned16(d_o, o), split));
+    NSA_LAUNCH_OK("delta_kernel");
+  } else if (split.offsets) {
+    KernelScope ks("sel_split_clear_kernel", st);
+    NSA_CUDA_OK(launch_chained(sel_split_clear_kernel, n_split, 256, 0, st, split));
+    NSA_LAUNCH_OK("sel_split_clear_kernel");
   }
   int rc = NSA_OK;
   if (pl.wide) {
@@ -1902,10 +1930,10 @@ int tc_attn_bwd(const AttnArgs& a, void* ws, size_t ws_bytes, cudaStream_t st) {
   }
   if (rc != NSA_OK) return rc;
   if (pl.sel_split) {
-    KernelScope ks("sel_split_blocks_kernel", st);
-    NSA_CUDA_OK(launch_chained(sel_split_blocks_kernel, dim3(pl.n_ktiles, a.B * a.Hkv), 256, 0, st, p.plan.offsets, p.dk_acc, p.dv_acc,
-                               p.dk, p.dv, pl.n_ktiles, pl.nq, a.Lk, a.D, 1));
-    NSA_LAUNCH_OK("sel_split_blocks_kernel");
+    KernelScope ks("sel_split_finish_kernel", st);
+    NSA_CUDA_OK(launch_chained(sel_split_finish_kernel, n_split, 256, 0, st, split, p.dk, p.dv,
+                               (((uintptr_t)p.dk | (uintptr_t)p.dv) & 7) == 0));
+    NSA_LAUNCH_OK("sel_split_finish_kernel");
   }
   if (ordered) {
     KernelScope ks("cmp_chunks_kernel", st);
