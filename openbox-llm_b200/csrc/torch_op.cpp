@@ -97,10 +97,24 @@ bool comp_ok(const Call& c, at::Device dev) {
   return true;
 }
 
-NsaAttentionTensors pointers(const Tensor* in, const Tensor* comp, const Tensor& block_idx, bool learned) {
+// The eight inputs, or their gradients, by address.  Of the layer the keys and values of the branches are parts of one tensor: views of them
+// would cost a dispatch each (forward on 256 tokens, calls in a row, 99.8 -> 95.0 us).
+struct Eight {
+  void* p[8];
+  explicit Eight(const Tensor* t) {
+    for (int k = 0; k < 8; ++k) p[k] = t[k].data_ptr();
+  }
+  Eight(const Tensor& q, const Tensor& kv, const Tensor& gate) {
+    const size_t part = kv.nbytes() / 6;
+    p[0] = q.data_ptr();
+    for (int k = 0; k < 6; ++k) p[1 + k] = (char*)kv.data_ptr() + k * part;
+    p[7] = gate.data_ptr();
+  }
+};
+NsaAttentionTensors pointers(const Eight& in, const Tensor* comp, const Tensor& block_idx, bool learned) {
   NsaAttentionTensors t = {};
   const void** p[8] = {&t.q, &t.kc, &t.vc, &t.ks, &t.vs, &t.kw, &t.vw, &t.gate};
-  for (int k = 0; k < 8; ++k) *p[k] = in[k].data_ptr();
+  for (int k = 0; k < 8; ++k) *p[k] = in.p[k];
   for (int k = 0; k < 6 && learned; ++k) t.comp[k] = comp[k].data_ptr<float>();
   t.block_idx = block_idx.data_ptr<int32_t>();
   return t;
@@ -108,8 +122,7 @@ NsaAttentionTensors pointers(const Tensor* in, const Tensor* comp, const Tensor&
 
 // out; `saved` keeps what backward reads.  Makes c.block_idx where the scorer writes it.
 // tokens: the shape of an output in token order ([B, T, Hq, D] elements)
-Tensor op_forward(Call& c, bool need_grad, Tensor* saved, at::IntArrayRef tokens = {}) {
-  const Tensor& q = c.in[0];
+Tensor op_forward(Call& c, const Eight& in, const Tensor& q, bool need_grad, Tensor* saved, at::IntArrayRef tokens = {}) {
   c.d.need_grad = need_grad;
   if (!c.d.given_lists) c.block_idx = fresh({c.d.dims.B, c.d.dims.Hkv, c.d.dims.T, c.d.n_sel}, at::kInt, q);
   size_t keep, fwd, bwd;
@@ -121,7 +134,7 @@ Tensor op_forward(Call& c, bool need_grad, Tensor* saved, at::IntArrayRef tokens
     ws = bytes_like(fwd, q);
     ws_ptr = ws.data_ptr();
   }
-  NsaAttentionTensors t = pointers(c.in, c.comp, c.block_idx, c.d.learned);
+  NsaAttentionTensors t = pointers(in, c.comp, c.block_idx, c.d.learned);
   t.out = out.data_ptr();
   check((tokens.empty() ? nsa_attention_fwd : nsa_attention_fwd_tokens)(&c.d, &t, mem.data_ptr(), ws_ptr, fwd, raw_stream(q)));
   *saved = mem;
@@ -129,14 +142,14 @@ Tensor op_forward(Call& c, bool need_grad, Tensor* saved, at::IntArrayRef tokens
 }
 
 // d_in: the eight gradients, allocated by the caller.  d_tokens: the output's gradient in [B, T, Hq, D]; d_out is scratch then.
-void op_backward(const NsaAttentionDesc& d, const Tensor* in, const Tensor* comp, const Tensor& block_idx, const Tensor& saved,
-                 const Tensor& d_out, const Tensor* d_in, Tensor* d_comp, const Tensor* d_tokens = nullptr) {
+void op_backward(const NsaAttentionDesc& d, const Eight& in, const Tensor* comp, const Tensor& block_idx, const Tensor& saved,
+                 const Tensor& d_out, const Eight& d_in, Tensor* d_comp, const Tensor* d_tokens = nullptr) {
   size_t keep, fwd, bwd;
   check(nsa_attention_sizes(&d, &keep, &fwd, &bwd));
   NsaAttentionTensors t = pointers(in, comp, block_idx, d.learned);
   t.d_out = d_out.data_ptr();
   void** p[8] = {&t.dq, &t.dkc, &t.dvc, &t.dks, &t.dvs, &t.dkw, &t.dvw, &t.d_gate};
-  for (int k = 0; k < 8; ++k) *p[k] = d_in[k].data_ptr();
+  for (int k = 0; k < 8; ++k) *p[k] = d_in.p[k];
   for (int k = 0; k < 6 && d.learned; ++k) {
     d_comp[k] = fresh_like(comp[k]);
     t.d_comp[k] = d_comp[k].data_ptr<float>();
@@ -184,7 +197,7 @@ struct OpNode {
   template <typename... A>
   static Tensor run(AutogradContext* ctx, Call* c, const A&...) {
     Tensor saved;
-    Tensor out = op_forward(*c, true, &saved);
+    Tensor out = op_forward(*c, Eight(c->in), c->in[0], true, &saved);
     variable_list keep(c->in, c->in + 8);
     keep.push_back(c->block_idx);
     keep.push_back(saved);
@@ -206,7 +219,7 @@ struct OpNode {
     const Tensor d_out = aligned(g[0]);
     Tensor d_in[8], d_comp[6];
     for (int k = 0; k < 8; ++k) d_in[k] = fresh_like(kept[k]);
-    op_backward(d, kept.data(), kept.data() + 10, kept[8], kept[9], d_out, d_in, d_comp);
+    op_backward(d, Eight(kept.data()), kept.data() + 10, kept[8], kept[9], d_out, Eight(d_in), d_comp);
     for (int k = 0; k < 8; ++k) res[1 + k] = d_in[k];
     for (int k = 8; k < n; ++k) res[1 + k] = d_comp[k - 8];
     return res;
@@ -265,19 +278,18 @@ struct LayerNode : torch::autograd::Function<LayerNode> {
     check(nsa_cast_bf16_segments(s, n, raw_stream(l.x)));
     Tensor y = at::addmm(bias, xb, w.t());
     Call& c = l.c;
-    c.in[0] = fresh({m.B, m.Hq, m.T, m.D}, at::kBFloat16, l.x);
+    Tensor q = fresh({m.B, m.Hq, m.T, m.D}, at::kBFloat16, l.x);
     Tensor kv = fresh({6, m.B, m.Hkv, m.T, m.D}, at::kBFloat16, l.x);
-    c.in[7] = fresh({m.B, m.Hq, m.T, 3}, at::kBFloat16, l.x);
-    for (int k = 0; k < 6; ++k) c.in[1 + k] = kv.select(0, k);
-    check(nsa_split_heads(y.data_ptr(), c.in[0].data_ptr(), kv.data_ptr(), c.in[7].data_ptr(), m.B, m.T, m.Hq, m.Hkv, m.D,
+    Tensor gate = fresh({m.B, m.Hq, m.T, 3}, at::kBFloat16, l.x);
+    check(nsa_split_heads(y.data_ptr(), q.data_ptr(), kv.data_ptr(), gate.data_ptr(), m.B, m.T, m.Hq, m.Hkv, m.D,
                           NSA_DTYPE_BF16, raw_stream(l.x)));
     Tensor saved;
-    Tensor tokens = op_forward(c, need_grad, &saved, {rows, hd});
+    Tensor tokens = op_forward(c, Eight(q, kv, gate), q, need_grad, &saved, {rows, hd});
     Tensor out = at::mm(tokens, w_out.t()).view({l.B, l.T, l.dm});
     if (keep) {
       bool weights = false;
       for (const Tensor& t : l.w) weights |= t.requires_grad();
-      *keep = {c.in[0], kv, c.in[7], c.block_idx, saved, weights ? xb : Tensor(), l.x.requires_grad() ? w : Tensor(), w_out,
+      *keep = {q, kv, gate, c.block_idx, saved, weights ? xb : Tensor(), l.x.requires_grad() ? w : Tensor(), w_out,
                l.w_out.requires_grad() ? tokens : Tensor()};
       keep->insert(keep->end(), c.comp, c.comp + 6);
     }
@@ -318,25 +330,18 @@ struct LayerNode : torch::autograd::Function<LayerNode> {
     variable_list kept = ctx->get_saved_variables();
     for (Tensor& t : kept) t = aligned(t);
     const Tensor &kv = kept[1], &xb = kept[5], &w = kept[6], &w_out = kept[7], &tokens = kept[8];
-    Tensor in[8];
-    in[0] = kept[0];
-    in[7] = kept[2];
-    for (int k = 0; k < 6; ++k) in[1 + k] = kv.select(0, k);
     const int64_t rows = (int64_t)m.B * m.T, hd = (int64_t)m.Hq * m.D, dm = w_out.size(0);
     const int64_t width = nsa_fused_projection_width(m.Hq, m.Hkv, m.D);
     const Tensor dy = aligned(g[0].to(at::kBFloat16)).view({rows, dm});
     if (ctx->needs_input_grad(10)) res[11] = at::mm(dy.t(), tokens, at::kFloat);
     if (!op_any) return res;
     Tensor d_tokens = at::mm(dy, w_out), d_out = fresh({m.B, m.Hq, m.T, m.D}, at::kBFloat16, kv);
-    Tensor d_in[8], d_comp[6], d_kv = fresh_like(kv);
-    d_in[0] = fresh_like(in[0]);
-    d_in[7] = fresh_like(in[7]);
-    for (int k = 0; k < 6; ++k) d_in[1 + k] = d_kv.select(0, k);
-    op_backward(d, in, kept.data() + 9, kept[3], kept[4], d_out, d_in, d_comp, &d_tokens);
+    Tensor d_comp[6], d_q = fresh_like(kept[0]), d_kv = fresh_like(kv), d_gate = fresh_like(kept[2]);
+    op_backward(d, Eight(kept[0], kv, kept[2]), kept.data() + 9, kept[3], kept[4], d_out, Eight(d_q, d_kv, d_gate), d_comp, &d_tokens);
     for (int k = 0; k < 6; ++k) res[12 + k] = d_comp[k];
     if (!rows_any) return res;
     Tensor d_rows = fresh({rows, width}, at::kBFloat16, kv);
-    check(nsa_merge_heads(d_in[0].data_ptr(), d_kv.data_ptr(), d_in[7].data_ptr(), d_rows.data_ptr(), m.B, m.T, m.Hq, m.Hkv, m.D,
+    check(nsa_merge_heads(d_q.data_ptr(), d_kv.data_ptr(), d_gate.data_ptr(), d_rows.data_ptr(), m.B, m.T, m.Hq, m.Hkv, m.D,
                           NSA_DTYPE_BF16, raw_stream(dy)));
     if (ctx->needs_input_grad(0)) {
       Tensor dx = ctx->saved_data["x_bf16"].toBool() ? at::mm(d_rows, w) : at::mm(d_rows, w, at::kFloat);
@@ -413,7 +418,7 @@ PyObject* py_op(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (!need) {
       Tensor saved;
       at::NoGradGuard no_grad;
-      out = op_forward(c, false, &saved);
+      out = op_forward(c, Eight(c.in), c.in[0], false, &saved);
     } else if (learned) {
       out = OpLearned::apply(&c, c.in[0], c.in[1], c.in[2], c.in[3], c.in[4], c.in[5], c.in[6], c.in[7], c.comp[0], c.comp[1],
                              c.comp[2], c.comp[3], c.comp[4], c.comp[5]);
