@@ -11,7 +11,7 @@
 // What bounds them: mma.sync issues 1019 products a clock and SM, 170 of fp32, where FFMA does 128 at best and did
 // 58 here, with both operands from shared memory.  A tile takes 3.1 k cycles of them forward and 7.7 k backward, the operands' loads from
 // shared memory 2.9 k and 6 k, splits, masks and exponentials 2.6 k and 4 k issue slots; two CTAs of eight warps an SM overlap that to 6.1 k
-// and 12.6 k (tensor pipe active half of the time; CUDA-core tiles 9.3 k and 21 k).  Three branches of 2048 tokens, 8 heads of 64, forward and
+// and 12.6 k (tensor pipe active 46 to 49 % of the time forward, 61 to 62 % backward; CUDA-core tiles 9.3 k and 21 k).  Three branches of 2048 tokens, 8 heads of 64, forward and
 // backward: selection 188 + 351 -> 117 + 239 us, window 100 + 195 -> 66 + 134, the pass 850 -> 550.  Tried: four warps of 16 x 64 with 168
 // and 255 registers (forward 139, backward 225: the same work an SM, but a tile takes twice as long, which is what few
 // tiles wait for); K and V of the next tile brought into L1 ahead (3 % slower).
