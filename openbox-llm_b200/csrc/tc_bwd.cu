@@ -1065,6 +1065,10 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
     }
   } else if (warp < kB2Compute) {
     // ---- compute warps: S, dP -> P, dS, tile after tile -------------------------------------------
+    // Two columns an instruction in the arithmetic around the exponentials, the same bits: selection at D = 64, 8 x 4096 tokens of 12
+    // heads 528 -> 519 us, 3 x 3001 172 -> 168.5, 8192 of 16 182 -> 180.5.  Elsewhere it was slower: compression
+    // at D = 64 72 -> 74, selection at D = 128, which spills then, 8.6 -> 9.1 ms (8 x 32768 tokens).
+    constexpr bool kPacked = D == 64 && kGather;
     const int quad = warp & 3, half = warp >> 2;       // TMEM lane quadrant, key-column half
     const int row = quad * 32 + lane;
     const int ql = row / p.G, g = row % p.G;
@@ -1151,7 +1155,18 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
           pp[c2] = pack_bf16(p0, p1);
           pd[c2] = pack_bf16(d0, d1);
         };
-        if (__all_sync(0xffffffffu, all_cols)) {
+        if (kPacked && __all_sync(0xffffffffu, all_cols)) {
+          const uint64_t scale2 = pack_f32x2(p.scale_log2, p.scale_log2), neg_lse2 = pack_f32x2(-lse2, -lse2);
+          const uint64_t dscale2 = pack_f32x2(dscale, dscale), neg_ddelta2 = pack_f32x2(-ddelta, -ddelta);
+#pragma unroll
+          for (int c2 = 0; c2 < 16; ++c2) {
+            float x0, x1, y0, y1;
+            unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(rs[c2 * 2]), __uint_as_float(rs[c2 * 2 + 1])), scale2, neg_lse2), x0, x1);
+            unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(rp[c2 * 2]), __uint_as_float(rp[c2 * 2 + 1])), dscale2, neg_ddelta2), y0, y1);
+            const float p0 = ex2(x0), p1 = ex2(x1);
+            put(c2, p0, p1, p0 * y0, p1 * y1);
+          }
+        } else if (!kPacked && __all_sync(0xffffffffu, all_cols)) {
 #pragma unroll
           for (int c2 = 0; c2 < 16; ++c2) {
             const float p0 = ex2(fmaf(__uint_as_float(rs[c2 * 2]), p.scale_log2, -lse2));
