@@ -507,8 +507,8 @@ gate_fwd_vec_kernel(const __nv_bfloat16* __restrict__ oc, const __nv_bfloat16* _
 // divisions for the row; more vectors a thread change nothing).
 // kTokens: d_out is [B, T, Hq, D], as the layer's GEMM leaves it; the rows in the order of the heads, which the branch
 // kernels fetch, are written on the way to d_heads.
-// `zeros`: what the pooling's backward, which follows in the op, adds to; a memset of its own cost a launch (5 us of host work,
-// what a pass over 1024 tokens is bound by).
+// `zeros`: what the pooling's backward, which follows in the op, adds to, in place of a memset of its own ahead of this kernel: training on
+// 16-token blocks 282 -> 275 us, with overlapping summaries 199 -> 198, 1024 tokens 193 on both sides.
 template <bool kTokens>
 __global__ void __launch_bounds__(256)
 gate_bwd_rows_vec_kernel(const __nv_bfloat16* __restrict__ oc, const __nv_bfloat16* __restrict__ os,
