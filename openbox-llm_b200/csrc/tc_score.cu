@@ -306,13 +306,19 @@ __device__ __forceinline__ void sort_candidates(float (&v)[N], int (&j)[N]) {
 // recursive-halving exchange of shuffles, took 240 instructions of a warp per 64 summaries; 64 heads of 128 x 65536 tokens 2.37 ->
 // 1.97 ms, 8 x 32768 tokens of 16 heads 2.0 -> 1.64, 8 x 4096 tokens of 12 heads of 64 109 -> 81 us.  The first tile's candidates go into
 // the empty lists by a sorting network (8 x 4096 tokens: 110 -> 101 us when it came).
+// Groups of 4 at D = 128 hold 18 KB of sums beside 64 KB of Q and K: two CTAs an SM, which took longer than the shuffles from some 150 CTAs on.
+// There the sums lie over K, for a third CTA, and the next K is fetched after the lists, under the other CTAs' work (the shuffles | two
+// CTAs | this, us): 8192 tokens of 16 heads on 4 41 | 51 | 39, 16384 101 | 113 | 88, 65536 987 | 761 | 586; overlapping summaries every 16
+// tokens, 4096 29 | 38 | 28, 16384 184 | 254 | 173 (195 of it with divisions and five sums a block instead of shifts and four).
 // ------------------------------------------------------------------------------------------
 constexpr int kImpLd = 144;              // floats of a query's row of sums: 128, and 4 more after every 32 (16-byte reads without conflicts)
 
 template <int D, int GP> struct ScoreLanes {
   static constexpr int kSlabs = D / 64;
   static constexpr int kQBytes = kRows * 128 * kSlabs, kKBytes = 128 * 128 * kSlabs;
-  static constexpr int kImpBytes = kRows / GP * kImpLd * 4;
+  // Groups of 4 at D = 128: 18 KB of sums beside Q and K would leave two CTAs an SM; they take the place of K, and the next K waits.
+  static constexpr bool kOverK = D == 128 && GP == 4;
+  static constexpr int kImpBytes = kOverK ? 0 : kRows / GP * kImpLd * 4;
   static constexpr size_t kSmem = kQBytes + kKBytes + kImpBytes + 128 * 4 /*lse*/ + 64 /*barriers*/ + 1024;
   static constexpr int kCtas = (int)(227 * 1024 / (kSmem + 1024)) > 4 ? 4 : (int)(227 * 1024 / (kSmem + 1024));
 };
@@ -323,6 +329,7 @@ tc_score_lanes_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                       const ScoreArgs p) {
   using L = ScoreLanes<D, GP>;
   constexpr int kSlabs = L::kSlabs, kQBytes = L::kQBytes, kKBytes = L::kKBytes;
+  constexpr bool kOverK = L::kOverK;
   constexpr uint32_t kTmemCols = 128;
   constexpr uint32_t kIdescKQ = idesc_bf16(128, 128, 0, 0);
   constexpr int NQ = kRows / GP;       // queries per tile
@@ -334,8 +341,8 @@ tc_score_lanes_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   uint8_t* sQ = smem;
   uint8_t* sK = sQ + kQBytes;
-  float* s_imp = (float*)(sK + kKBytes);             // [NQ][kImpLd]
-  float* s_lse = s_imp + NQ * kImpLd;                // [128], negative, log2 units
+  float* s_imp = (float*)(kOverK ? sK : sK + kKBytes);              // [NQ][kImpLd]
+  float* s_lse = (float*)(sK + kKBytes + L::kImpBytes);            // [128], negative, log2 units
   uint64_t* bars = (uint64_t*)(s_lse + 128);
   uint64_t* bar_q = bars + 0;
   uint64_t* bar_k = bars + 1;
@@ -455,7 +462,7 @@ tc_score_lanes_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       const bool s_ok = mbar_wait(bar_s, i & 1, p.status, s_abort, 4);
       tc_fence_after();
       __syncwarp();
-      if (tid == 0 && s_ok && i + 1 < n_tiles) load_k(i + 1);          // the MMAs have read this tile's
+      if (!kOverK && tid == 0 && s_ok && i + 1 < n_tiles) load_k(i + 1);          // the MMAs have read this tile's
       {
         const int at = 32 * (warp % (size / 32)) + lane;               // this thread's summary in the tile
         const int c0 = warp / (size / 32) * size;                      // and its columns
@@ -498,13 +505,14 @@ tc_score_lanes_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       // the sums are there, and S has been read: the next MMA may overwrite it; one decision for the whole CTA:
       // after a given-up wait nothing more is issued or written
       if (__syncthreads_or(*s_abort)) { aborted = true; break; }
-      if (tid == 0 && i + 1 < n_tiles) {
+      auto next_s = [&]() {
         tc_fence_after();
         if (mbar_wait(bar_k, (i + 1) & 1, p.status, s_abort, 2)) {
           k_seen = i + 2;
           issue_s();
         }
-      }
+      };
+      if (!kOverK && tid == 0 && i + 1 < n_tiles) next_s();
       __syncwarp();
       // the query's sum at place k of the tile; what it does not see is zero
       auto sum_at = [&](int k) -> float { return key0 + k < n_vis ? s_imp[ql * kImpLd + k + 4 * (k >> 5)] : 0.f; };
@@ -572,14 +580,15 @@ tc_score_lanes_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       } else {
         // A selection block is r consecutive summaries (plus, when the summaries overlap, the one before them); it is a
         // candidate once its first summary is visible.
-        const int r_ = p.r, ov_ = p.overlap;
+        const int r_ = p.r, ov_ = p.overlap, log_r = 31 - __clz(p.r);       // (r: a power of two)
         const float tau = bound();
+        float last = !ov_ ? 0.f : g == 0 ? carry : sum_at(g * per - 1);     // the summary ahead, where blocks share one
 #pragma unroll 1
         for (int k = g * per; k < (g + 1) * per; k += r_) {
-          float acc = !ov_ ? 0.f : k == 0 ? carry : sum_at(k - 1);
+          float acc = ov_ ? last : 0.f;
 #pragma unroll 1
-          for (int e = 0; e < r_; ++e) acc += sum_at(k + e);
-          const int cj = (key0 + k) / r_;                            // block index
+          for (int e = 0; e < r_; ++e) acc += last = sum_at(k + e);
+          const int cj = (key0 + k) >> log_r;                        // block index
           const bool visible = max(0, r_ * cj - ov_) < n_vis;        // first overlapping summary
           if (out && cj < p.imp_cols) out[cj] = visible ? acc : 0.f;
           float cv = visible ? acc : -1.f;
@@ -591,7 +600,15 @@ tc_score_lanes_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         }
         carry = sum_at(size - 1);
       }
-      if (i + 1 < n_tiles) __syncthreads();          // the next tile's sums may be written
+      if (i + 1 < n_tiles) {
+        if (kOverK) fence_proxy_async();
+        __syncthreads();                             // the next tile's sums (or itself) may be written
+        if (kOverK && tid == 0) {
+          load_k(i + 1);
+          next_s();
+        }
+        if (kOverK) __syncwarp();
+      }
     }
     if (!aborted) aborted = __syncthreads_or(*s_abort) != 0;
     if (aborted) {

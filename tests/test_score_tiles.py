@@ -8,9 +8,9 @@ from tests.util import pkg
 pytestmark = pytest.mark.gpu
 
 
-# summaries: one, a tile of 32 and of 64 less, exactly and more than full, a second tile of every size
-@pytest.mark.parametrize("n_blk", [1, 31, 33, 64, 65, 96, 128, 129, 161, 200, 256])
-@pytest.mark.parametrize("Hq,Hkv,D", [(3, 1, 64), (8, 2, 64), (10, 2, 128), (16, 1, 128), (9, 1, 64)])
+# summaries: one, a tile of 32 and of 64 less, exactly and more than full, a second tile of every size, a third
+@pytest.mark.parametrize("n_blk", [1, 31, 33, 64, 65, 96, 128, 129, 161, 200, 256, 300])
+@pytest.mark.parametrize("Hq,Hkv,D", [(3, 1, 64), (8, 2, 64), (10, 2, 128), (16, 1, 128), (9, 1, 64), (8, 2, 128), (3, 1, 128)])
 def test_importances_and_lists(n_blk, Hq, Hkv, D):
     """Importances of all rows against 64 bits, and the lists against the canonical order of the kernel's own importances, bit for bit.  A
     score of a few units is good to 2^-20 (64 to 128 products, each rounded to 2^-24, and the tensor cores' truncation), the
@@ -34,20 +34,21 @@ def test_importances_and_lists(n_blk, Hq, Hkv, D):
     assert nsa.lib().nsa_device_status(None) == 0
 
 
+@pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("T", [544, 1040, 1056, 1072, 2064, 2080])
-def test_blocks_whose_first_summary_ends_a_tile(T):
+def test_blocks_whose_first_summary_ends_a_tile(T, D):
     """Summaries of 32 tokens every 16 under blocks of 64: a block is a candidate as soon as the summary before it, which reaches
     into it, is visible; that one may be the last of its tile."""
     nsa = pkg()
     g = torch.Generator(device="cuda").manual_seed(T)
     n = (T - 32) // 16 + 1
-    q = torch.randn(1, 8, T, 64, generator=g, device="cuda").bfloat16()
-    k = torch.randn(1, 2, n, 64, generator=g, device="cuda").bfloat16()
+    q = torch.randn(1, 8, T, D, generator=g, device="cuda").bfloat16()
+    k = torch.randn(1, 2, n, D, generator=g, device="cuda").bfloat16()
     _, lse = nsa.range_attn_forward(q, k, k, nsa.MODE_COMPRESS_STRIDED, 16, 32)
     idx, imp = nsa.topn_blocks(q, k, lse, 64, 16, return_importance=True, cmp_len=32, cmp_stride=16)
     t = torch.arange(T, device="cuda")
     sees = (t[:, None] - 31) // 16 >= torch.arange(n, device="cuda")
-    s = q.double() @ k.double().repeat_interleave(4, 1).transpose(-1, -2) * 64 ** -0.5
+    s = q.double() @ k.double().repeat_interleave(4, 1).transpose(-1, -2) * D ** -0.5
     p = (s - lse.double()[..., None]).exp().masked_fill(~sees, 0.0).view(1, 2, 4, T, n).sum(2)
     want, valid = O.block_importance(p.float().cpu(), T, 32, 16, 64)
     assert (imp.cpu() - want * valid).abs().max() <= 2.0 ** -17 * want.max()
