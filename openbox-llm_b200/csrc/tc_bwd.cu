@@ -1750,10 +1750,19 @@ static BwdPlan plan_bwd(const AttnArgs& a) {
   const long long base = (long long)units * pl.n_ktiles;
   pl.csize = 1;
   // Three-term row tiles take three times as long as others beside the same cost of a CTA, and early key tiles have most
-  // of them: up to two CTAs per SM.  128 key tiles of 13 row tiles (2 x 1024 tokens, 16 heads of 128, 8 blocks of 16 a list): alone 161 us, pairs 127,
-  // clusters of four 132.
-  const long long most = a.three_term ? 2LL * sm_count() : sm_count() + 20;
-  while (a.kind != 1 && !a.dq_acc && !pl.wide && pl.csize < 8 && base * pl.csize * 2 <= most && item_rt >= 8 * pl.csize) pl.csize *= 2;
+  // of them: up to two CTAs per SM, as long as a CTA keeps enough of them beside the one it shares its SM with: 8 (D = 64: 10) up to one and a half per SM,
+  // beyond that 12 (20).  Key tiles / row tiles of the longest (alone | pairs | fours | eights, us), D = 128: 128 / 8
+  // 62 | 68, 128 / 16 103 | 96, 128 / 32 152 | 125 | 130, 96 / 8 60 | 59, 96 / 48 203 | 111 | 111, 64 / 16 100 | 62 | 66, 64 / 32 152 | 84 | 77, 64 / 64
+  // 210 | 113 | 76 | 107, 32 / 32 148 | 84 | 51 | 58, 37 / 128 357 | 189 | 103 | 80; D = 64: 128 / 8 41 | 47, 128 / 16 66 | 68, 128 / 32 99 | 78, 96 / 8
+  // 39 | 41, 96 / 12 53 | 49, 88 / 11 48 | 43, 64 / 16 64 | 41 | 49, 64 / 32 74 | 44 | 45, 64 / 64 130 | 72 | 53 | 79, 32 / 32 94 | 54 | 35 | 45,
+  // 24 / 48 113 | 65 | 41 | 33, 37 / 128 269 | 144 | 80 | 62.
+  auto pays = [&](int csize) {
+    const long long ctas = base * csize * 2, sms = sm_count();
+    if (ctas <= sms + 20) return item_rt >= 8 * csize;
+    if (!a.three_term || ctas > 2 * sms) return false;
+    return item_rt >= (2 * ctas <= 3 * sms ? (a.D == 128 ? 8 : 10) : a.D == 128 ? 12 : 20) * csize;
+  };
+  while (a.kind != 1 && !a.dq_acc && !pl.wide && pl.csize < 8 && pays(pl.csize)) pl.csize *= 2;
   // compression: a few key tiles are attended by (almost) every query; they go in chunks of 48 row
   // tiles whose dK / dV meet in fp32 accumulators
   pl.n_splits = 1;

@@ -46,7 +46,8 @@ def _close(got, want, what):
 
 
 # one key tile and less; tiles and row tiles that end ragged; 2, 3, 4, 16 and 64 heads a group; few key tiles with many
-# rows (clusters); work items that are split (a block that every query lists, more than 128 row tiles)
+# rows (clusters); work items that are split (a block that every query lists, more than 128 row tiles); clusters of two, four and
+# eight on more CTAs than SMs, and key tiles with too few rows for them
 SHAPES = [dict(B=1, Hq=4, Hkv=2, D=64, T=17, block_size=16, S=1),
           dict(B=1, Hq=8, Hkv=2, D=128, T=64, block_size=16, S=3),
           dict(B=2, Hq=6, Hkv=2, D=64, T=129, block_size=32, S=2),
@@ -54,7 +55,11 @@ SHAPES = [dict(B=1, Hq=4, Hkv=2, D=64, T=17, block_size=16, S=1),
           dict(B=1, Hq=16, Hkv=1, D=128, T=833, block_size=32, S=5),
           dict(B=1, Hq=64, Hkv=1, D=64, T=321, block_size=16, S=40),
           dict(B=1, Hq=16, Hkv=1, D=64, T=1100, block_size=16, S=4),
-          dict(B=1, Hq=16, Hkv=1, D=128, T=1100, block_size=16, S=4)]
+          dict(B=1, Hq=16, Hkv=1, D=128, T=1100, block_size=16, S=4),
+          dict(B=2, Hq=16, Hkv=4, D=128, T=1030, block_size=16, S=3),
+          dict(B=1, Hq=8, Hkv=2, D=64, T=1543, block_size=16, S=3),
+          dict(B=1, Hq=4, Hkv=1, D=64, T=1600, block_size=32, S=3),
+          dict(B=8, Hq=16, Hkv=4, D=64, T=250, block_size=16, S=3)]
 
 
 @pytest.mark.parametrize("c", SHAPES, ids=cfg_id)
