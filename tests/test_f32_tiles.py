@@ -47,10 +47,11 @@ def _run(nsa, kind, q, k, v, do, idx, bs, W):
 
 
 # the last row tile with 1, 63 and all of its rows, key tiles of 1, 64 and 65 keys, one to eight heads on a kv head; clusters of four, two
-# and one (row tiles per SM: below 0.5, between, above 3)
+# and one (row tiles per SM: below 0.5, between, above 3); blocks that end within a key tile, and longer ones than it
 @pytest.mark.parametrize("B,Hq,Hkv,T,W,bs,S,repeat", [
     (1, 8, 2, 481, 2, 64, 8, False), (2, 3, 3, 575, 64, 16, 24, True), (1, 12, 4, 704, 65, 24, 20, True), (2, 8, 1, 1000, 133, 64, 16, False),
-    (1, 4, 4, 4097, 512, 64, 16, False), (6, 16, 2, 640, 200, 32, 12, True)])
+    (1, 4, 4, 4097, 512, 64, 16, False), (6, 16, 2, 640, 200, 32, 12, True), (2, 16, 1, 300, 70, 17, 9, True), (1, 8, 2, 705, 63, 40, 9, False),
+    (3, 6, 2, 901, 30, 100, 5, True)])
 def test_f32_tiles_are_fp32_arithmetic(B, Hq, Hkv, T, W, bs, S, repeat):
     """Against 64 bits, whole tensors.  A dot product of 64 terms is good to 2^-23 of its norm, and o and the gradients are chains of two to
     five such steps and of sums of up to 40 tiles, each rounded to 2^-24: 2^-20 of a tensor's norm (measured: up to 3.4e-7; 4.8e-7 with
