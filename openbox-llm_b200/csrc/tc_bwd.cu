@@ -1067,8 +1067,9 @@ tc_bwd2_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
     // ---- compute warps: S, dP -> P, dS, tile after tile -------------------------------------------
     // Two columns an instruction in the arithmetic around the exponentials, the same bits: selection at D = 64, 8 x 4096 tokens of 12
     // heads 528 -> 519 us, 3 x 3001 172 -> 168.5, 8192 of 16 182 -> 180.5.  Elsewhere it was slower: compression
-    // at D = 64 72 -> 74, selection at D = 128, which spills then, 8.6 -> 9.1 ms (8 x 32768 tokens).
-    constexpr bool kPacked = D == 64 && kGather;
+    // at D = 64 72 -> 74, selection at D = 128, which spills then, 8.6 -> 9.1 ms (8 x 32768 tokens), key tiles shared by a cluster
+    // (D = 64, 16 heads on 1, 5000 tokens 84 -> 88 us, 2048 49 -> 51; 64 on 4, 1000 tokens 78 -> 81).
+    constexpr bool kPacked = D == 64 && kGather && !kCluster;
     const int quad = warp & 3, half = warp >> 2;       // TMEM lane quadrant, key-column half
     const int row = quad * 32 + lane;
     const int ql = row / p.G, g = row % p.G;
