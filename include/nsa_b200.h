@@ -38,8 +38,10 @@ extern "C" {
 /* which kernel family serves a call */
 #define NSA_IMPL_AUTO 0   /* tcgen05 kernels when the shape allows, else the SIMT kernels; selection on blocks
                              of 16 or 32 tokens with P and dS in three bf16 terms (24 bits) and fp32 dQ
-                             partials, or, small calls among them, SIMT, whose arithmetic is fp32 throughout */
-#define NSA_IMPL_SIMT 1   /* CUDA-core kernels: any dtype, D in {16,32,64,128}, any G and block size */
+                             partials, or, small calls among them, SIMT, whose arithmetic is fp32 throughout;
+                             fp32 at D = 64 in tiles of 64 rows with every product as six products of bf16 terms
+                             on the tensor cores (24 bits; values below 2^-109 in size keep fewer) */
+#define NSA_IMPL_SIMT 1   /* CUDA-core kernels, products by FFMA: any dtype, D in {16,32,64,128}, any G and block size */
 #define NSA_IMPL_TC   2   /* tcgen05/TMEM kernels only; NSA_ERR_UNSUPPORTED if the shape does not fit */
 
 #define NSA_OK               0

@@ -317,6 +317,7 @@ static int range_attn_fwd(const void* q, const void* k, const void* v, void* o, 
     a.kind = NSA_MODE_COMPRESS;
   }
   a.chained = chained;
+  a.cuda_cores = impl == NSA_IMPL_SIMT;
   if (use_tc(dims, 64, impl, &rc) && Lk > 0) return tc_attn_fwd(a, (cudaStream_t)stream);
   if (rc != NSA_OK) return rc;
   return simt_attn_fwd(a, dims->dtype, (cudaStream_t)stream);
@@ -392,6 +393,7 @@ static int range_attn_bwd(const void* q, const void* k, const void* v, const voi
   a.row_scale = row_scale; a.row_dot = row_dot;
   a.dq_acc = dq_acc;
   a.wide_dq = wide_dq;
+  a.cuda_cores = impl == NSA_IMPL_SIMT;
   NSA_CHECK_ARG((row_scale == nullptr) == (row_dot == nullptr), "row_scale and row_dot go together");
   if (use_tc(dims, 64, impl, &rc)) {
     a.dk_acc = (float*)dk;   // tc path writes dk/dv itself; pass the outputs through
@@ -487,6 +489,7 @@ static int selection_fwd_impl(const void* q, const void* k, const void* v,
   a.q = q; a.k = k; a.v = v; a.o = o; a.lse = lse; a.block_idx = block_idx;
   a.kind = 2; a.S = S; a.block_size = block_size;
   a.sel_plan = plan;
+  a.cuda_cores = impl == NSA_IMPL_SIMT;
   a.three_term = use_three_term(dims, block_size, S, impl, false) && aligned16(q, k, v, o);
   if (a.three_term || (use_tc(dims, block_size, impl, &rc) && S > 0))
     return tc_sel_fwd(a, workspace, workspace_bytes, (cudaStream_t)stream);
@@ -570,6 +573,7 @@ static int selection_bwd_impl(const void* q, const void* k, const void* v,
   a.block_idx = block_idx; a.kind = 2; a.S = S; a.block_size = block_size;
   a.row_scale = row_scale; a.row_dot = row_dot;
   NSA_CHECK_ARG((row_scale == nullptr) == (row_dot == nullptr), "row_scale and row_dot go together");
+  a.cuda_cores = impl == NSA_IMPL_SIMT;
   a.three_term = dq && use_three_term(dims, block_size, S, impl, true) && aligned16(q, k, v, d_o, dq, dk, dv) &&
                (row_dot || aligned16(o));
   if (a.three_term || (use_tc(dims, block_size, impl, &rc) && S > 0)) {

@@ -164,6 +164,7 @@ struct AttnArgs {
   // window backward without a dq of its own: who reads the partials knows that they may lie in tiles of 128 keys (a caller
   // who names neither the key count nor the options to nsa_dq_reduce3 gets them in tiles of 64)
   bool wide_dq;
+  bool cuda_cores;   // fp32: FFMA throughout (NSA_IMPL_SIMT), where the call would take the bf16 terms of f32_tile.cu
   bool chained;      // tcgen05 compression forward: launched into the end of the pooling (launch_chained)
   int B, Hq, Hkv, T, Lk, D, S;
   int kind;          // 0 window, 1 compress, 2 selection

@@ -1,5 +1,5 @@
 // CUDA-core attention on tiles of 64 rows x 64 keys, fp32 arithmetic throughout: the fp32 path (D of 64: f32_tile.cu, by the
-// same rules), and bf16 shapes the tcgen05 kernels do not take (D of 16 / 32, one query head per kv head, other
+// same rules, unless the caller asks for the CUDA cores), and bf16 shapes the tcgen05 kernels do not take (D of 16 / 32, one query head per kv head, other
 // block sizes).  A row is one (query token, query head); the rows of a unit are numbered token-major
 // (row = t * G + head), so a tile's rows share their K / V tiles whatever the group size.
 //   window, compression   the tile walks the keys its rows can see, 64 at a time
@@ -595,7 +595,7 @@ simt_tile_bwd_kernel(const AttnArgs a, const int csize) {
 }
 
 // CTAs that share a row tile, each taking every csize-th key tile.  A row tile is one long chain; with few of them the
-// longest is what the call waits for.  The lines, in row tiles per SM (fp32, D = 64 on these kernels, 8 heads on 2; alone | 2 | 4 CTAs a
+// longest is what the call waits for.  The lines, in row tiles per SM (fp32, D = 64, 8 heads on 2; alone | 2 | 4 CTAs a
 // tile, us): selection at 0.86 forward 132 | 93 | 66, backward 232 | 180 | 125; at 1.7 310 | 189 | 182 and
 // 640 | 355 | 399; at 6.9 650 | 615 | 678 and 1507 | 1345 | 1499; at 21 1648 | 1691 | 2021 and 3935 | 3994 | 4467.
 // Window (chains of 9 key tiles) at 0.4 69 | 44 | 37 and 109 | 64 | 55; at 1.3 101 | 78 | 90 and 196 | 145 | 159; at 1.7
@@ -647,8 +647,8 @@ int launch_d(const AttnArgs& a, bool bwd, cudaStream_t st) {
     case 16: return launch<T, 16>(a, bwd, st);
     case 32: return launch<T, 32>(a, bwd, st);
     case 64:
-      if constexpr (sizeof(T) == 4) return f32_tile_launch(a, bwd, st);       // on the tensor cores
-      else return launch<T, 64>(a, bwd, st);
+      if (sizeof(T) == 4 && !a.cuda_cores) return f32_tile_launch(a, bwd, st);       // on the tensor cores
+      return launch<T, 64>(a, bwd, st);
     case 128: return launch<T, 128>(a, bwd, st);
     default: set_error("head dim %d not in {16,32,64,128}", a.D); return NSA_ERR_UNSUPPORTED;
   }

@@ -29,8 +29,9 @@ _dq_accumulator = False
 
 def set_impl(name: str):
     """Choose the kernel family: 'auto' (tcgen05 where the shape fits; selection on 16- and 32-token
-    blocks with the probabilities in three bf16 terms, 24 bits as on the CUDA cores), 'simt', or 'tc' (tcgen05, or an error; takes 16- and 32-token
-    blocks too, with bf16 probabilities as on 64-token blocks)."""
+    blocks with the probabilities in three bf16 terms, 24 bits as on the CUDA cores; fp32 heads of 64 with every product as six
+    products of bf16 terms on the tensor cores), 'simt' (the CUDA cores, products by FFMA), or 'tc' (tcgen05, or an error; takes 16- and
+    32-token blocks too, with bf16 probabilities as on 64-token blocks)."""
     global _impl
     assert name in L.IMPL
     _impl = name

@@ -102,3 +102,30 @@ def test_f32_values_that_cannot_be_split():
     for x, y in zip((o, dq, dk, dv), ref):
         assert (x.double() - y).norm() <= 2.0 ** -20 * y.norm()
     assert nsa.lib().nsa_device_status(None) == 0
+
+
+def test_simt_is_the_cuda_cores():
+    """Who asks for the CUDA cores gets FFMA tiles; by default fp32 heads of 64 go by bf16 terms.  Both to 2^-20 of the norm, as above."""
+    nsa = pkg()
+    L, lib = nsa._lib, nsa.lib()
+    g = torch.Generator(device="cuda").manual_seed(3)
+    T, bs = 700, 64
+    q, do = (torch.randn(1, 8, T, 64, generator=g, device="cuda") for _ in range(2))
+    k, v = (torch.randn(1, 2, T, 64, generator=g, device="cuda") for _ in range(2))
+    idx, keep = _lists(1, 2, T, bs, 6, False, g)
+    want = _dense(q, k, v, do, keep)
+    for impl, name in (("auto", "f32_tile"), ("simt", "simt_tile")):
+        nsa.set_impl(impl)
+        lib.nsa_profile_enable(1)
+        try:
+            got = _run(nsa, "selection", q, k, v, do, idx, bs, 0)
+            _run(nsa, "window", q, k, v, do, None, 0, 100)
+            _run(nsa, "compression", q, k[:, :, :T // bs].contiguous(), v[:, :, :T // bs].contiguous(), do, None, bs, 0)
+            torch.cuda.synchronize()
+            seen = {n for n in L.profile_summary() if "_fwd_" in n or "_bwd_" in n}
+        finally:
+            lib.nsa_profile_enable(0)
+            nsa.set_impl("auto")
+        assert seen == {f"{name}_{way}_{kind}" for way in ("fwd", "bwd") for kind in ("slc", "win", "cmp")}, seen
+        for x, y in zip(got, want):
+            assert (x.double() - y).norm() <= 2.0 ** -20 * y.norm()
