@@ -194,7 +194,8 @@ int nsa_attention_bwd(const NsaAttentionDesc* desc, const NsaAttentionTensors* t
                       void* workspace, size_t workspace_bytes, void* stream);
 /* The same with the output and its gradient in [B, T, Hq, D], for a caller whose next GEMM takes tokens: `out` is
  * written so; backward reads d_tokens and writes its rows in the order of the heads to t->d_out, which is scratch of
- * the output's size.  bf16, D a power of two. */
+ * the output's size.  bf16, D a power of two; anything else is refused before the first launch, as is (in the other
+ * order too, for bf16) an output or a gradient of it off a 16-byte boundary. */
 int nsa_attention_fwd_tokens(const NsaAttentionDesc* desc, const NsaAttentionTensors* t, void* saved, void* workspace,
                              size_t workspace_bytes, void* stream);
 int nsa_attention_bwd_tokens(const NsaAttentionDesc* desc, const NsaAttentionTensors* t, const void* saved,

@@ -554,9 +554,6 @@ gate_bwd_rows_vec_kernel(const __nv_bfloat16* __restrict__ oc, const __nv_bfloat
 inline bool gate_vec_ok(int D, int dtype) {
   return dtype == NSA_DTYPE_BF16 && D >= 8 && D <= 256 && (D & (D - 1)) == 0;
 }
-inline bool token_major_ok(const NsaDims* d) {
-  return gate_vec_ok(d->D, d->dtype) && (size_t)d->B * d->Hq * d->T <= 0xffffffffu;
-}
 
 // out = a + b + c, fp32 accumulation, 8 elements per thread (bf16) or 4 (fp32)
 __global__ void sum3_bf16_kernel(const uint4* __restrict__ a, const uint4* __restrict__ b,
@@ -622,6 +619,13 @@ inline bool pool_vec_ok(int D, int dtype, const void* a, const void* b) {
 inline unsigned blocks_for(size_t n, int per) { return (unsigned)((n + per - 1) / per); }
 
 }  // namespace
+int gate_args_ok(const NsaDims* d, const void* heads, const void* tokens) {
+  const bool vec = gate_vec_ok(d->D, d->dtype);
+  NSA_CHECK_ARG(!tokens || (vec && (size_t)d->B * d->Hq * d->T <= 0xffffffffu),
+                "token-major rows take bf16 heads of 8 to 256 columns, a power of two");
+  NSA_CHECK_ARG(!vec || (aligned16(heads) && aligned16(tokens)), "the output and its gradient have to start on a 16-byte boundary");
+  return NSA_OK;
+}
 }  // namespace nsa
 
 using namespace nsa;
@@ -997,7 +1001,6 @@ int nsa::gate_bwd_rows(const void* o_cmp, const void* o_slc, const void* o_win, 
   NSA_CHECK_ARG(dims && row_scale && row_dot && d_gate_logits, "null argument");
   const size_t rows = (size_t)dims->B * dims->Hq * dims->T;
   if (rows == 0) return NSA_OK;
-  NSA_CHECK_ARG(!d_heads || token_major_ok(dims), "token-major rows take bf16 heads of 8 to 256 columns, a power of two");
   cudaStream_t st = (cudaStream_t)stream;
   const bool vec = gate_vec_ok(dims->D, dims->dtype);
   if (n_zeros && !vec) NSA_CUDA_OK(cudaMemsetAsync(zeros, 0, n_zeros * sizeof(float), st));
@@ -1255,7 +1258,6 @@ int nsa::gate_fwd_unless_blended(const void* o_cmp, const void* o_slc, const voi
   NSA_CHECK_ARG(dims, "null dims");
   const size_t rows = (size_t)dims->B * dims->Hq * dims->T;
   if (rows == 0) return NSA_OK;
-  NSA_CHECK_ARG(!tokens || token_major_ok(dims), "token-major rows take bf16 heads of 8 to 256 columns, a power of two");
   cudaStream_t st = (cudaStream_t)stream;
   unsigned grid = blocks_for(rows * (dims->D / 8), 256);
   if (choice.hdr) grid = std::min(grid, 16u * (unsigned)sm_count());

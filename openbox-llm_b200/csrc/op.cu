@@ -283,6 +283,7 @@ static int attention_fwd(const NsaAttentionDesc* d, const NsaAttentionTensors* t
   if (p.rows == 0) return NSA_OK;
   NSA_CHECK_ARG(saved && t->q && t->kc && t->vc && t->ks && t->vs && t->kw && t->vw && t->gate && t->out &&
                 (p.S == 0 || t->block_idx), "null tensor");
+  NSA_TRY(gate_args_ok(&m, tokens ? nullptr : t->out, tokens ? t->out : nullptr));
   NSA_CHECK_ARG(p.fwd_ws == 0 || (workspace && workspace_bytes >= p.fwd_ws), "forward workspace too small: need %zu bytes", p.fwd_ws);
   if (d->learned)
     for (int k = 0; k < 6; ++k) NSA_CHECK_ARG(t->comp[k], "null compressor parameter");
@@ -392,6 +393,7 @@ static int attention_bwd(const NsaAttentionDesc* d, const NsaAttentionTensors* t
   }
   NSA_CHECK_ARG(saved && t->q && t->kc && t->vc && t->ks && t->vs && t->kw && t->vw && t->gate && t->d_out &&
                 (p.S == 0 || t->block_idx), "null tensor");
+  NSA_TRY(gate_args_ok(&m, t->d_out, d_tokens));
   NSA_CHECK_ARG(t->dq && t->dkc && t->dvc && t->dks && t->dvs && t->dkw && t->dvw && t->d_gate, "null gradient");
   NSA_CHECK_ARG(workspace && workspace_bytes >= p.bwd_ws, "backward workspace too small: need %zu bytes", p.bwd_ws);
   if (d->learned)

@@ -36,6 +36,30 @@ def test_bad_arguments_are_refused_before_any_launch(bad):
     assert _sizes(**bad) == -1
 
 
+@pytest.mark.parametrize("name,dtype,at,says", [
+    ("fwd_tokens", 1, {}, "token-major"), ("bwd_tokens", 1, {}, "token-major"), ("fwd_tokens", 0, dict(out=8), "16-byte"),
+    ("bwd_tokens", 0, dict(tokens=8), "16-byte"), ("bwd_tokens", 0, dict(d_out=2), "16-byte"), ("fwd", 0, dict(out=8), "16-byte"),
+    ("bwd", 0, dict(d_out=2), "16-byte")], ids=str)
+def test_outputs_the_gates_cannot_take_are_refused_before_any_launch(name, dtype, at, says):
+    """Tokens of another type than bf16, and a bf16 output, or its gradient, off a 16-byte boundary.  The addresses are no one's: the
+    refusal has to come from the host, ahead of every launch."""
+    L = importlib.import_module("openbox-llm_b200._lib")
+    if torch.cuda.is_available():
+        pytest.skip("for a machine without a GPU: what is not refused would be launched")
+    lib, far = L.lib(), 1 << 20
+    desc = L.NsaAttentionDesc(L.dims(1, 4, 2, 128, 64, dtype), 64, 1, 16, 0, 0, 64, 64, 0, 1, 1, 0, 0)
+    n = [ctypes.c_size_t() for _ in range(3)]
+    assert lib.nsa_attention_sizes(desc, *n) == 0
+    t = L.OP_TENSORS(*[far] * 8, *(None,) * 6, *[far] * 11)
+    t[15], t[16] = far + at.get("out", 0), far + at.get("d_out", 0)
+    before = lib.nsa_launch_count()
+    args = [desc, t, far, far, n[1 if "fwd" in name else 2].value]
+    if name == "bwd_tokens":
+        args.append(far + at.get("tokens", 0))
+    assert getattr(lib, "nsa_attention_" + name)(*args, None) == -1 and says in lib.nsa_last_error().decode()
+    assert lib.nsa_launch_count() == before
+
+
 def _inputs(B, Hq, Hkv, T, D, seed=4):
     g = torch.Generator(device="cuda").manual_seed(seed)
     mk = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()

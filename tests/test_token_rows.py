@@ -60,7 +60,7 @@ def test_token_rows(c, variant):
 
 @pytest.mark.gpu
 def test_token_rows_of_other_types_are_refused():
-    """fp32 has the order of the heads only."""
+    """fp32 has the order of the heads only; what is refused launches nothing."""
     nsa = pkg()
     L, lib = nsa._lib, nsa.lib()
     x = [torch.zeros(1, h, 64, w, device="cuda") for h, w in ((2, 64), *[(1, 64)] * 6, (2, 3))]
@@ -71,8 +71,10 @@ def test_token_rows_of_other_types_are_refused():
     mem = [torch.empty(v.value + 1, dtype=torch.uint8, device="cuda") for v in n]
     out = torch.empty_like(x[0])
     t = L.OP_TENSORS(*[v.data_ptr() for v in x], *(None,) * 6, idx.data_ptr(), out.data_ptr())
+    before = lib.nsa_launch_count()
     with pytest.raises(nsa.NsaError, match="token-major"):
         L.check(lib.nsa_attention_fwd_tokens(d, t, mem[0].data_ptr(), mem[1].data_ptr(), n[1].value, L.stream()))
+    assert lib.nsa_launch_count() == before
 
 
 @pytest.mark.gpu
