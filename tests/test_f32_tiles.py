@@ -104,6 +104,70 @@ def test_f32_values_that_cannot_be_split():
     assert nsa.lib().nsa_device_status(None) == 0
 
 
+def _attended(kind, B, Hkv, T, bs, S, W, repeat, g):
+    """How often each row attends each key, what _run takes for it, and the number of keys."""
+    t = torch.arange(T, device="cuda")
+    if kind == "selection":
+        idx, keep = _lists(B, Hkv, T, bs, S, repeat, g)
+        return keep, idx, T
+    if kind == "window":
+        return ((t[:, None] >= t) & (t[:, None] - t < W)).float().expand(B, Hkv, T, T), None, T
+    n = (T - bs) // W + 1                                  # summaries of bs tokens every W
+    return ((t[:, None] - bs + 1) // W >= torch.arange(n, device="cuda")).float().expand(B, Hkv, T, n), None, n
+
+
+# row tiles that clusters of four (up to half a row tile per SM; selection 0.87), of two (1.3; 3) and none share; lists that repeat blocks; blocks
+# of 24, 40 and 48 tokens; summaries of 16 tokens every W
+@pytest.mark.parametrize("kind,B,Hq,Hkv,T,bs,S,W,repeat", [
+    ("selection", 1, 8, 2, 700, 64, 6, 0, False), ("selection", 1, 4, 2, 1300, 24, 14, 0, True), ("selection", 3, 8, 2, 800, 48, 5, 0, True),
+    ("selection", 6, 8, 2, 700, 40, 5, 0, True), ("compression", 1, 4, 1, 500, 16, 0, 1, False), ("compression", 1, 8, 2, 900, 16, 0, 2, False),
+    ("compression", 2, 8, 2, 1000, 16, 0, 16, False), ("window", 1, 8, 2, 500, 0, 0, 480, False), ("window", 1, 8, 2, 700, 0, 0, 300, False),
+    ("window", 3, 8, 2, 700, 0, 0, 300, False)])
+def test_f32_values_that_cannot_be_split_in_every_branch(kind, B, Hq, Hkv, T, bs, S, W, repeat):
+    """The repairs by FFMA where a key tile is a union of listed blocks, counts blocks twice, or is shared out over a cluster: what is not
+    finite stays with the rows that attend it and their keys, huge values are exact to the same 2^-20."""
+    nsa = pkg()
+    g = torch.Generator(device="cuda").manual_seed(5)
+    n, idx, L = _attended(kind, B, Hkv, T, bs, S, W, repeat, g)
+    q, do = (torch.randn(B, Hq, T, 64, generator=g, device="cuda") for _ in range(2))
+    k, v = (torch.randn(B, Hkv, L, 64, generator=g, device="cuda") for _ in range(2))
+
+    def run(q, k, v, do):
+        if kind != "compression":
+            return _run(nsa, kind, q, k, v, do, idx, bs, W)
+        o, lse = nsa.range_attn_forward(q, k, v, nsa.MODE_COMPRESS_STRIDED, W, bs)
+        return o, *nsa.range_attn_backward(q, k, v, o, lse, do, nsa.MODE_COMPRESS_STRIDED, W, bs)
+
+    clean = run(q, k, v, do)
+    hit = lambda where, at: (n[..., at] > 0) if where in "kv" else (torch.arange(T, device="cuda") == at).expand(B, Hkv, T)
+    same = lambda a, b: torch.isfinite(a).all() and (a - b).norm() <= 2.0 ** -20 * b.norm()
+
+    def stays(got, where, at):
+        rows = hit(where, at)
+        keys = ((n > 0) & rows[..., None]).any(2)
+        far = (~rows).repeat_interleave(Hq // Hkv, 1), ~keys
+        for i, (x, y) in enumerate(zip(got, clean)):
+            assert same(x[far[i > 1]], y[far[i > 1]]), (where, at, i)
+
+    for at, where, bad in ((L // 3, "v", float("inf")), (L // 2, "k", float("nan")), (T - 70, "q", float("nan")), (T // 2 + 1, "do", float("-inf"))):
+        x = {"q": q, "k": k, "v": v, "do": do}
+        x[where] = x[where].clone()
+        x[where][:, :, at, 3] = bad
+        got = run(**x)
+        stays(got, where, at)
+        assert hit(where, at).any() and not torch.isfinite(got[0 if where == "v" else 1]).all(), where
+    for at, where, scale in ((L // 3, "v", 2.0 ** -100), (T // 2 + 1, "do", 1.0)):
+        x = {"q": q, "k": k, "v": v, "do": do * scale}
+        x[where] = x[where].clone()
+        x[where][:, :, at, 5] = 2.0 ** 100
+        got = run(**x)
+        for name, a, b in zip(("o", "dq", "dk", "dv"), got, _dense(*x.values(), n)):
+            assert (a.double() - b).norm() <= 2.0 ** -20 * b.norm(), (where, name)
+        if where == "do":
+            stays(got, where, at)
+    assert nsa.lib().nsa_device_status(None) == 0
+
+
 def test_simt_is_the_cuda_cores():
     """Who asks for the CUDA cores gets FFMA tiles; by default fp32 heads of 64 go by bf16 terms.  Both to 2^-20 of the norm, as above."""
     nsa = pkg()
