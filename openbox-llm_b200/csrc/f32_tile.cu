@@ -1,20 +1,25 @@
 // fp32 attention at D = 64 on the tensor cores: tiles of 64 rows x 64 keys as in simt_tile.cu, every product as six
 // products of bf16 terms.
 //
-// An fp32 value is the sum of three bf16 terms, each what the ones before it leave of it (24 bits in all).  Of the nine
+// An fp32 value is the sum of three bf16 terms, each what the ones before it leave of it (24 bits in all, down to values of 2^-109: below,
+// the last terms fall under bf16's smallest, and NSA_IMPL_SIMT keeps what these tiles drop).  Of the nine
 // products of two such sums the six largest are formed: what is left out is below 2^-26 of the product.  The tensor cores cut
 // the bits that fall out of a sum off, instead of rounding, so the five small products (2^-8 of the large one and less) have
-// an accumulator of their own, neither runs over more than 64 terms, and both are added up in fp32.  Measured over dot
+// an accumulator of their own, neither goes over more than 64 places of the contraction (320 products in the small one), and both are
+// added up in fp32.  Measured over dot
 // products of N(0, 1): 64 terms 0.7e-7 off the 64-bit value (a chain of 64 FFMAs 1.4e-7), 512 terms 0.9e-7 (4.1e-7), 2048
 // terms 1.3e-7 (8.0e-7); with one accumulator, small products first, 3.9e-7 at 64 terms.
 //
 // What bounds them: mma.sync issues 1019 products a clock and SM, 170 of fp32, where FFMA does 128 at best and did
 // 58 here, with both operands from shared memory.  A tile takes 3.1 k cycles of them forward and 7.7 k backward, the operands' loads from
 // shared memory 2.9 k and 6 k, splits, masks and exponentials 2.6 k and 4 k issue slots; two CTAs of eight warps an SM overlap that to 6.1 k
-// and 12.6 k (tensor pipe active 46 to 49 % of the time forward, 61 to 62 % backward; CUDA-core tiles 9.3 k and 21 k).  Three branches of 2048 tokens, 8 heads of 64, forward and
-// backward: selection 188 + 351 -> 117 + 239 us, window 100 + 195 -> 66 + 134, the pass 850 -> 550.  Tried: four warps of 16 x 64 with 168
+// and 12.6 k (selection and window: tensor pipe active 46 to 49 % of the time forward, 61 to 62 % backward; compression, one key tile a CTA,
+// 24 and 52 %; CUDA-core tiles 9.3 k and 21 k).  128 registers a thread, 140 bytes spilled forward and 72 backward.  Three branches of 2048 tokens, 8 heads of 64, forward and
+// backward: selection 188 + 351 -> 117 + 239 us, window 100 + 195 -> 66 + 134, the pass 850 -> 550.  Slower than the CUDA-core tiles, which fit three
+// CTAs an SM, is compression forward of one key tile on two to three row tiles per SM: 26.5 -> 29 us at 384 row tiles.  Tried: four warps of 16 x 64 with 168
 // and 255 registers (forward 139, backward 225: the same work an SM, but a tile takes twice as long, which is what few
-// tiles wait for); K and V of the next tile brought into L1 ahead (3 % slower).
+// tiles wait for); K and V of the next tile, or of the first, brought into L1 ahead (3 % slower, no change).  tcgen05.mma has three times this
+// rate; it is not tried: each 64 places its sums would come back from tensor memory for the adds in fp32, and P and dS go there in three terms.
 //
 // Values that the split cannot carry (infinite, NaN, or from 2^60 on, where its products could overflow) are zeros in the products,
 // eight neighbouring columns at a time, and noted by row and columns; what attends them is put right by FFMAs.  Rows that
@@ -110,24 +115,15 @@ __device__ __forceinline__ void mma(float* d, const uint32_t* a, const uint32_t*
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
-// Where a lane's 16 bytes of an operand lie in a term.  Row-major A (16 rows from m0, 16 columns from chunk c) and
-// what B is of a tile whose rows are its columns (16 of them from n0):
-__device__ __forceinline__ uint32_t at_a(int lane, int m0, int c) {
-  const int r = m0 + (lane & 15);
+// Where a lane's 16 bytes of an operand lie in a term.  A by rows (16 rows from r0, 16 columns from chunk c), or B of a tile whose
+// rows are the contraction, transposed as it is read:
+__device__ __forceinline__ uint32_t at_a(int lane, int r0, int c) {
+  const int r = r0 + (lane & 15);
   return r * 128 + (((c + (lane >> 4)) ^ (r & 7)) << 4);
 }
-__device__ __forceinline__ uint32_t at_b(int lane, int n0, int c) {
-  const int r = n0 + (lane & 7) + ((lane >> 4) << 3);
-  return r * 128 + (((c + ((lane >> 3) & 1)) ^ (r & 7)) << 4);
-}
-// B of a tile whose rows are the contraction (16 of them from k0, columns from chunk c), transposed as it is read, and A of such
-// a tile
-__device__ __forceinline__ uint32_t at_bt(int lane, int k0, int c) {
-  const int r = k0 + (lane & 15);
-  return r * 128 + (((c + (lane >> 4)) ^ (r & 7)) << 4);
-}
-__device__ __forceinline__ uint32_t at_at(int lane, int k0, int c) {
-  const int r = k0 + (lane & 7) + ((lane >> 4) << 3);
+// B of a tile whose rows are its columns (16 of them from r0), or A of one whose rows are the contraction:
+__device__ __forceinline__ uint32_t at_b(int lane, int r0, int c) {
+  const int r = r0 + (lane & 7) + ((lane >> 4) << 3);
   return r * 128 + (((c + ((lane >> 3) & 1)) ^ (r & 7)) << 4);
 }
 
@@ -204,7 +200,7 @@ struct RowKeys {
 // bookkeeping of key tile i: its keys (threads 0 .. 63), and what each row attends of it (64 .. 127), as two words of 32 keys
 __device__ __forceinline__ void fill_tile(const AttnArgs& a, const TileKeys& tk, const SelList& sl, KeyInfo* ki, uint32_t (*att)[2][kR],
                                           const RowKeys& rk, int buf, int i) {
-  fill_keys(a, tk, sl, ki, buf, i);
+  fill_keys<false>(a, tk, sl, ki, buf, i);
   const int r = (int)threadIdx.x - kK;
   if (r < 0 || r >= kR) return;
   const unsigned long long bits = rk.of_tile(a, tk, sl, i);
@@ -336,7 +332,7 @@ f32_tile_fwd_kernel(const AttnArgs a, const int csize) {
 #pragma unroll
                        for (int e = 0; e < 4; ++e) x[t][e] = p[kk][t][e];
                    },
-                   [&](int t, int kk, int j, uint32_t* y) { ldsm4t(sV + t * kTermBytes + at_bt(lane, 32 * half + 16 * kk, 4 * dh + j), y); });
+                   [&](int t, int kk, int j, uint32_t* y) { ldsm4t(sV + t * kTermBytes + at_a(lane, 32 * half + 16 * kk, 4 * dh + j), y); });
 #pragma unroll
         for (int j = 0; j < 4; ++j)
 #pragma unroll
@@ -576,20 +572,20 @@ f32_tile_bwd_kernel(const AttnArgs a, const int csize) {
     float acc[4][4];
     put(s);
     __syncthreads();
-    product<kR / 16>(acc, keys_a, [&](int t, int kk, int j, uint32_t* y) { ldsm4t(sDO + t * kTermBytes + at_bt(lane, 16 * kk, 4 * half + j), y); });
+    product<kR / 16>(acc, keys_a, [&](int t, int kk, int j, uint32_t* y) { ldsm4t(sDO + t * kTermBytes + at_a(lane, 16 * kk, 4 * half + j), y); });
     if (bad) add_bad_rows(acc, 3, d_o);
     add_rows(dvb, acc, tok[0], tok[1], 32 * half, t4);               // dV += P^T dO
     __syncthreads();
     put(ds);
     __syncthreads();
-    product<kR / 16>(acc, keys_a, [&](int t, int kk, int j, uint32_t* y) { ldsm4t(sQ + t * kTermBytes + at_bt(lane, 16 * kk, 4 * half + j), y); });
+    product<kR / 16>(acc, keys_a, [&](int t, int kk, int j, uint32_t* y) { ldsm4t(sQ + t * kTermBytes + at_a(lane, 16 * kk, 4 * half + j), y); });
     if (bad) add_bad_rows(acc, 2, q);
     add_rows(dkb, acc, tok[0], tok[1], 32 * half, t4);               // dK += dS^T Q (Q carries the scale)
     product<kK / 16>(acc, [&](int kk, uint32_t (*x)[4]) {
 #pragma unroll
-                       for (int t = 0; t < 3; ++t) ldsm4t(sV + t * kTermBytes + at_at(lane, 16 * kk, 2 * warp), x[t]);
+                       for (int t = 0; t < 3; ++t) ldsm4t(sV + t * kTermBytes + at_b(lane, 16 * kk, 2 * warp), x[t]);
                      },
-                     [&](int t, int kk, int j, uint32_t* y) { ldsm4t(sK + t * kTermBytes + at_bt(lane, 16 * kk, 4 * half + j), y); });
+                     [&](int t, int kk, int j, uint32_t* y) { ldsm4t(sK + t * kTermBytes + at_a(lane, 16 * kk, 4 * half + j), y); });
 #pragma unroll
     for (int j = 0; j < 4; ++j)
 #pragma unroll

@@ -55,7 +55,8 @@ __device__ __forceinline__ void pool_weights(const float* __restrict__ logits, f
 // projection matrix travels into shared memory (cp.async, padded rows) meanwhile.  R = 8, or 4, where
 // that still gives every SM a CTA, else 2: a short sequence has a few dozen rows in all, and the
 // latency of one CTA's chain is what counts.  512 rows of 128 in windows of 16: R = 8 14.5 us, 4 14.5, 2 18.8 (more CTAs than fit at once);
-// 552 rows of 64 in windows of 64: 14.6, 13.4, 16.7.
+// 552 rows of 64 in windows of 64: 14.6, 13.4, 16.7.  Over the range of R = 4 (K and V, R = 2 | 4), windows of 64: 296 rows of 64 10.5 | 10.3, 400
+// 12.5 | 11.5, 584 16.6 | 12.5; 296 rows of 128 13.0 | 12.5, 400 18.6 | 14.8, 584 20.7 | 16.7; windows of 16: 8.7 | 8.6 to 16.7 | 12.7.
 template <int D, int R>
 struct PoolFwdSmem {
   static constexpr int kProjLd = D + 4;                 // float4 reads of 8 lanes cover all banks

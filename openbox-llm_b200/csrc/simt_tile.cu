@@ -177,7 +177,7 @@ simt_tile_fwd_kernel(const AttnArgs a, const int csize) {
     for (int c = 0; c < C; ++c) o[i][c] = 0.f;
   }
   if (rank < n_kt) {
-    fill_keys(a, tk, sl, ki, 0, rank);
+    fill_keys<true>(a, tk, sl, ki, 0, rank);
     __syncthreads();
     load_keys<T, D, kFwdThreads>(sK, kbase, ki->tok[0]);
     cp_commit();
@@ -257,7 +257,7 @@ simt_tile_fwd_kernel(const AttnArgs a, const int csize) {
         }
       }
     }
-    if (more) fill_keys(a, tk, sl, ki, buf ^ 1, kt + csize);
+    if (more) fill_keys<true>(a, tk, sl, ki, buf ^ 1, kt + csize);
     __syncthreads();
     if (more) load_keys<T, D, kFwdThreads>(sK, kbase, ki->tok[buf ^ 1]);
     cp_commit();
@@ -380,7 +380,7 @@ simt_tile_bwd_kernel(const AttnArgs a, const int csize) {
   const T* vbase = reinterpret_cast<const T*>(a.v) + kvoff;
   float* dkb = a.dk_acc + kvoff;
   float* dvb = a.dv_acc + kvoff;
-  if (rank < n_kt) fill_keys(a, tk, sl, ki, 0, rank);
+  if (rank < n_kt) fill_keys<true>(a, tk, sl, ki, 0, rank);
   // Q (scaled), dO (times the gate of a gated branch), lse and delta; four threads per row
   bool rows_bad;                        // a value of Q or dO is infinite or NaN
   {
@@ -488,7 +488,7 @@ simt_tile_bwd_kernel(const AttnArgs a, const int csize) {
         if (n > 1) { sP[at] *= (float)n; sDS[at] *= (float)n; }
       }
     }
-    if (more) fill_keys(a, tk, sl, ki, buf ^ 1, kt + csize);
+    if (more) fill_keys<true>(a, tk, sl, ki, buf ^ 1, kt + csize);
     __syncthreads();
     if (more) load_keys<T, D, kBwdThreads>(sV, vbase, ki->tok[buf ^ 1]);
     // dQ += dS K

@@ -91,7 +91,8 @@ __device__ __forceinline__ int times_listed(const AttnArgs& a, int bh, int t, in
   return n;
 }
 
-// token and membership of key tile i's keys (threads 0..63)
+// token and, where asked for, membership of key tile i's keys (threads 0..63)
+template <bool kMask>
 __device__ __forceinline__ void fill_keys(const AttnArgs& a, const TileKeys& tk, const SelList& sl, KeyInfo* ki, int buf, int i) {
   if (threadIdx.x >= kK) return;
   const int k = i * kK + threadIdx.x;
@@ -101,14 +102,14 @@ __device__ __forceinline__ void fill_keys(const AttnArgs& a, const TileKeys& tk,
     if (a.kind == 2) {
       const int b = sl.list[k / a.block_size];
       tok = b * a.block_size + k % a.block_size;
-      m = sl.mask[b];
+      if (kMask) m = sl.mask[b];
       if (tok >= a.T) tok = -1;
     } else {
       tok = tk.first + k;
     }
   }
   ki->tok[buf][threadIdx.x] = tok;
-  ki->mask[buf][threadIdx.x] = m;
+  if (kMask) ki->mask[buf][threadIdx.x] = m;
 }
 
 // keys [lo, hi] a row of query t may see by position
