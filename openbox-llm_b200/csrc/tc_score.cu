@@ -310,6 +310,9 @@ __device__ __forceinline__ void sort_candidates(float (&v)[N], int (&j)[N]) {
 // There the sums lie over K, for a third CTA, and the next K is fetched after the lists, under the other CTAs' work (the shuffles | two
 // CTAs | this, us): 8192 tokens of 16 heads on 4 41 | 51 | 39, 16384 101 | 113 | 88, 65536 987 | 761 | 586; overlapping summaries every 16
 // tokens, 4096 29 | 38 | 28, 16384 184 | 254 | 173 (195 of it with divisions and five sums a block instead of shifts and four).
+// Forced blocks on the summaries' grid go into the lists by themselves, before the others (the shuffles | every candidate looked at one
+// by one for their sake | this, block 0 and two local ones, 32768 tokens): 12 heads of 64 on 4 317 | 367 | 181, 16 on 2 224 | 234 | 152, 12 of 128
+// on 4 332 | 544 | 223, 16 on 1 203 | 209 | 172; at 1024 tokens 14.6 to 15.9 | 14.6 | 12.8 to 14.6.
 // ------------------------------------------------------------------------------------------
 constexpr int kImpLd = 144;              // floats of a query's row of sums: 128, and 4 more after every 32 (16-byte reads without conflicts)
 
@@ -526,8 +529,11 @@ tc_score_lanes_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         for (int o = 1; o < GP; o <<= 1) tau = fminf(tau, __shfl_xor_sync(0xffffffffu, tau, o));
         return tau;
       };
-      if (kAligned && !forcing) {
-        // summaries and blocks coincide: lane g's are key0 + g * per + k
+      // Forced blocks, with values of more than any sum: the first n_init, and those from loc0 to the query's.
+      const int last_cur = forcing && t < p.T ? my_cur : -1, loc0 = max(p.n_init, my_cur - p.n_local + 1);
+      if (kAligned) {
+        // summaries and blocks coincide: lane g's are c0 + k, and the first n_cand of them candidates
+        const int c0 = key0 + g * per, n_cand = min(per, n_vis - c0);
         float v[PER];
         if (per >= 4) {
           const int at = g * per;
@@ -541,16 +547,18 @@ tc_score_lanes_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         } else {
           v[0] = sum_at(g * per); v[1] = sum_at(g * per + 1);
         }
+        const int c1 = c0 + per - 1, hi1 = min(min(c1, p.n_init - 1), last_cur), lo2 = max(c0, loc0), hi2 = min(c1, last_cur);
+        uint32_t by_force = 0u;                      // not candidates by their sums
+        if (c0 <= hi1) by_force |= (2u << (hi1 - c0)) - 1u;
+        if (lo2 <= hi2) by_force |= ((2u << (hi2 - lo2)) - 1u) << (lo2 - c0);
         constexpr int kSort = 64 / GP;               // candidates of the first tile that are sorted into the empty lists
         if (i == 0) {
           float sv[kSort];
           int sj[kSort];
 #pragma unroll
           for (int k = 0; k < kSort; ++k) {
-            const int cj = g * per + k;
-            const bool visible = k < per && cj < n_vis;
-            sv[k] = visible && v[k] >= 0.f ? v[k] : -1.f;    // (not what is NaN, which enters no list)
-            sj[k] = cj;
+            sv[k] = k < n_cand && !((by_force >> k) & 1u) && v[k] >= 0.f ? v[k] : -1.f;    // (not what is NaN, which enters no list)
+            sj[k] = c0 + k;
           }
           sort_candidates<kSort>(sv, sj);
 #pragma unroll
@@ -561,19 +569,27 @@ tc_score_lanes_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         }
         if (out)
           for (int k = 0; k < per; ++k)
-            if (key0 + g * per + k < p.imp_cols) out[key0 + g * per + k] = sum_at(g * per + k);
+            if (c0 + k < p.imp_cols) out[c0 + k] = sum_at(g * per + k);
+        if (by_force) {
+#pragma unroll 1
+          for (uint32_t f = by_force; f; f &= f - 1u) {
+            const int cj = c0 + __ffs(f) - 1;
+            insert(cj < p.n_init ? kForcedInit - (float)cj : kForcedLocal - (float)(my_cur - cj), cj);
+          }
+        }
         if (i == 0 && per <= kSort) break;           // (the one tile there is)
         // those that are left, a bit each: a lane's next one a round, for as many rounds as the lane with most of them needs
         const float tau = bound();
         uint32_t left = 0u;
 #pragma unroll
         for (int k = 0; k < PER; ++k)
-          if (k < per && !(i == 0 && k < kSort) && key0 + g * per + k < n_vis && v[k] > lv[kList - 1] && v[k] >= tau) left |= 1u << k;
+          if (k < n_cand && !(i == 0 && k < kSort) && v[k] > lv[kList - 1] && v[k] >= tau) left |= 1u << k;
+        left &= ~by_force;
         while (__any_sync(0xffffffffu, left != 0u)) {
           if (left) {
-            const int at = g * per + __ffs(left) - 1;
+            const int k = __ffs(left) - 1;
             left &= left - 1u;
-            insert(sum_at(at), key0 + at);
+            insert(sum_at(g * per + k), c0 + k);
           }
           __syncwarp();
         }
@@ -592,9 +608,9 @@ tc_score_lanes_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
           const bool visible = max(0, r_ * cj - ov_) < n_vis;        // first overlapping summary
           if (out && cj < p.imp_cols) out[cj] = visible ? acc : 0.f;
           float cv = visible ? acc : -1.f;
-          if (forcing && cj <= my_cur && t < p.T) {
+          if (cj <= last_cur) {
             if (cj < p.n_init) cv = kForcedInit - (float)cj;
-            else if (cj > my_cur - p.n_local) cv = kForcedLocal - (float)(my_cur - cj);
+            else if (cj >= loc0) cv = kForcedLocal - (float)(my_cur - cj);
           }
           if (cv >= tau) insert(cv, cj);
         }

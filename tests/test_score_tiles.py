@@ -34,6 +34,27 @@ def test_importances_and_lists(n_blk, Hq, Hkv, D):
     assert nsa.lib().nsa_device_status(None) == 0
 
 
+@pytest.mark.parametrize("n_init,n_local", [(1, 2), (0, 1), (3, 0), (7, 9)])
+@pytest.mark.parametrize("n_blk,Hq,Hkv,D", [(1, 4, 1, 64), (33, 16, 1, 64), (64, 6, 2, 128), (127, 8, 2, 64), (129, 8, 2, 128), (160, 10, 2, 64), (300, 3, 1, 64),
+                                            (300, 16, 1, 128)])
+def test_forced_blocks_on_the_summaries_grid(n_blk, Hq, Hkv, D, n_init, n_local):
+    """The first blocks and those up to the query's are listed whatever their importance (the last has no summary yet), the others
+    in the canonical order, bit for bit; forced blocks at the ends of tiles and lanes, and in a tile with no summary."""
+    nsa = pkg()
+    bs, S, B = 16, 16, 2
+    T = n_blk * bs + 5
+    g = torch.Generator(device="cuda").manual_seed(n_blk)
+    q = torch.randn(B, Hq, T, D, generator=g, device="cuda").bfloat16()
+    k = torch.randn(B, Hkv, n_blk, D, generator=g, device="cuda").bfloat16()
+    _, lse = nsa.range_attn_forward(q, k, k, nsa.MODE_COMPRESS, 0, bs)
+    _, imp = nsa.topn_blocks(q, k, lse, bs, S, return_importance=True)
+    idx = nsa.topn_blocks(q, k, lse, bs, S, n_init_blocks=n_init, n_local_blocks=n_local)
+    t = torch.arange(T)
+    valid = (t[:, None] + 1) // bs > torch.arange(n_blk)
+    assert (idx.cpu() == O.forced_topn(imp.cpu(), valid, S, T, bs, n_init, n_local)).all()
+    assert nsa.lib().nsa_device_status(None) == 0
+
+
 @pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("T", [544, 1040, 1056, 1072, 2064, 2080])
 def test_blocks_whose_first_summary_ends_a_tile(T, D):
