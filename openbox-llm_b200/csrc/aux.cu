@@ -1054,7 +1054,9 @@ namespace {
 // side follow one another: 59 us for 8 x 4096 rows of 2344 bf16, 87 with K = 1.
 // The gates' columns are threads of their own behind the others, one token each, lanes on neighbouring tokens: as the last
 // columns of every row they had a lane in nearly every block go through its tokens one after the other, and the block with it
-// (in the layer's pass split 68 -> 57 us, merge 57.5 -> 54; 4 or 16 tokens a thread and other cache hints change nothing).
+// (in the layer's pass split 68 -> 57 us, merge 57.5 -> 54; 4 or 16 tokens a thread and other cache hints change nothing).  Two
+// vectors of a token lie in neighbouring lanes, for whole 32-byte sectors: merge at 4 x 8192 tokens of 64 heads of 128, fp32, 452 us when the
+// gates were a row's last columns, 466 with a vector to a token, 457 so; 8 x 8192 of 16 heads 296, 300, 293; bf16 233, 238, 235 and 154, 153, 150.
 template <typename T, typename V, int K>   // V: the 16-byte vector of T
 __global__ void __launch_bounds__(256)
 split_heads_kernel(T* __restrict__ y, T* __restrict__ q, T* __restrict__ kv, T* __restrict__ gate, int B, int Tn, int Hq,
@@ -1091,8 +1093,10 @@ split_heads_kernel(T* __restrict__ y, T* __restrict__ q, T* __restrict__ kv, T* 
     for (int k = 0; k < K; ++k)
       if (k < n) *reinterpret_cast<V*>(to + k * to_ld) = v[k];
   } else {
-    const size_t rows = (size_t)B * Tn, at = (i - n_main) % rows;
-    const int c0 = (int)((i - n_main) / rows) * kPer, b = (int)(at / Tn), t = (int)(at % Tn);
+    const size_t rows = (size_t)B * Tn, x = i - n_main;
+    const int pair = (W - n_attn) / kPer % 2 == 0 ? 1 : 0;
+    const size_t at = (x >> pair) % rows;
+    const int c0 = (int)(((x >> pair) / rows << pair) + (x & pair)) * kPer, b = (int)(at / Tn), t = (int)(at % Tn);
     V* vec = reinterpret_cast<V*>(y + at * W + n_attn + c0);
     alignas(16) T tmp[kPer];
     if (to_heads) *reinterpret_cast<V*>(tmp) = *vec;
