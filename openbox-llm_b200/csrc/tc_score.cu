@@ -326,13 +326,17 @@ template <int D, int GP> struct ScoreLanes {
   static constexpr int kCtas = (int)(227 * 1024 / (kSmem + 1024)) > 4 ? 4 : (int)(227 * 1024 / (kSmem + 1024));
 };
 
-template <int D, int GP, bool kAligned>
+// kForm: kApart, summaries and blocks on grids of their own; kSame, the same grid; kPlain, that without forced blocks and
+// importances, whose code the others would fetch and step over (the op on 512 tokens, 16 heads on 4, replayed from a graph 36.3 us with it, 35.1
+// without; 131072 tokens, 24 heads on 4, the scorer 2401 and 2323).
+enum ScoreForm { kApart, kSame, kPlain };
+template <int D, int GP, ScoreForm kForm>
 __global__ void __launch_bounds__(128, ScoreLanes<D, GP>::kCtas)
 tc_score_lanes_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                       const ScoreArgs p) {
   using L = ScoreLanes<D, GP>;
   constexpr int kSlabs = L::kSlabs, kQBytes = L::kQBytes, kKBytes = L::kKBytes;
-  constexpr bool kOverK = L::kOverK;
+  constexpr bool kOverK = L::kOverK, kAligned = kForm != kApart;
   constexpr uint32_t kTmemCols = 128;
   constexpr uint32_t kIdescKQ = idesc_bf16(128, 128, 0, 0);
   constexpr int NQ = kRows / GP;       // queries per tile
@@ -379,7 +383,7 @@ tc_score_lanes_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   int n_sum = cmp_visible(t_last, p.block_size, p.stride, p.n_blk);      // summaries to go through
   // (a block is a candidate from the summary before it on where they overlap: its own may be in the next tile)
   if (!kAligned && n_sum > 0) n_sum += p.overlap;
-  const bool forcing = p.n_init > 0 || p.n_local > 0;
+  const bool forcing = kForm != kPlain && (p.n_init > 0 || p.n_local > 0);
   // forced blocks are candidates whatever their importance: as far as the block that holds the last query
   if (forcing) n_sum = max(n_sum, p.r * (t_last / p.sel_block + 1));
   const int n_tiles = (n_sum + 127) / 128;
@@ -549,8 +553,8 @@ tc_score_lanes_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         }
         const int c1 = c0 + per - 1, hi1 = min(min(c1, p.n_init - 1), last_cur), lo2 = max(c0, loc0), hi2 = min(c1, last_cur);
         uint32_t by_force = 0u;                      // not candidates by their sums
-        if (c0 <= hi1) by_force |= (2u << (hi1 - c0)) - 1u;
-        if (lo2 <= hi2) by_force |= ((2u << (hi2 - lo2)) - 1u) << (lo2 - c0);
+        if (kForm == kSame && c0 <= hi1) by_force |= (2u << (hi1 - c0)) - 1u;
+        if (kForm == kSame && lo2 <= hi2) by_force |= ((2u << (hi2 - lo2)) - 1u) << (lo2 - c0);
         constexpr int kSort = 64 / GP;               // candidates of the first tile that are sorted into the empty lists
         if (i == 0) {
           float sv[kSort];
@@ -569,7 +573,7 @@ tc_score_lanes_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         }
         // (Importances, where asked for: a warp's lanes write 32 columns of each of its queries.  A lane its own summaries: 16 heads of 64 on 4,
         // 32768 tokens 326 us with the call's other work, now 229; 16 of 128 on 4, 8192 tokens 45 -> 40.)
-        if (p.imp_out) {
+        if (kForm != kPlain && p.imp_out) {
           for (int k = lane; k < size; k += 32) {
             const float* imp = s_imp + warp * (32 / GP) * kImpLd + k + 4 * (k >> 5);
             float* row = p.imp_out + ((size_t)bh * p.T + t0 + warp * (32 / GP)) * p.imp_cols + key0 + k;
@@ -676,7 +680,7 @@ tc_score_lanes_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     if (g == 0 && t < p.T) p.block_idx[((size_t)bh * p.T + t) * p.n_sel + r] = bj;
   }
   // importance columns no tile covered are zero
-  if (p.imp_out && t < p.T) {
+  if (kForm != kPlain && p.imp_out && t < p.T) {
     float* out = p.imp_out + ((size_t)bh * p.T + t) * p.imp_cols;
     const int seen = n_tiles > 0 ? (n_tiles - 1) * 128 + size_of(n_tiles - 1) : 0;
     for (int c = seen / (kAligned ? 1 : p.r) + g; c < p.imp_cols; c += GP) out[c] = 0.f;
@@ -694,13 +698,10 @@ static int launch_score_lanes(const void* q, const void* k_cmp, const NsaDims& d
   if (rc != NSA_OK) return rc;
   const size_t smem = ScoreLanes<D, GP>::kSmem;
   KernelScope ks("tc_score_topn", st);
-  if (p.r == 1 && p.overlap == 0) {
-    NSA_CUDA_OK(func_smem((const void*)tc_score_lanes_kernel<D, GP, true>, smem));
-    NSA_CUDA_OK(launch_chained(tc_score_lanes_kernel<D, GP, true>, dim3(p.n_qtiles, d.B * d.Hkv), 128, smem, st, tm_q, tm_k, p));
-  } else {
-    NSA_CUDA_OK(func_smem((const void*)tc_score_lanes_kernel<D, GP, false>, smem));
-    NSA_CUDA_OK(launch_chained(tc_score_lanes_kernel<D, GP, false>, dim3(p.n_qtiles, d.B * d.Hkv), 128, smem, st, tm_q, tm_k, p));
-  }
+  const bool same = p.r == 1 && p.overlap == 0, plain = same && !p.imp_out && p.n_init <= 0 && p.n_local <= 0;
+  const auto kernel = plain ? tc_score_lanes_kernel<D, GP, kPlain> : same ? tc_score_lanes_kernel<D, GP, kSame> : tc_score_lanes_kernel<D, GP, kApart>;
+  NSA_CUDA_OK(func_smem((const void*)kernel, smem));
+  NSA_CUDA_OK(launch_chained(kernel, dim3(p.n_qtiles, d.B * d.Hkv), 128, smem, st, tm_q, tm_k, p));
   return NSA_OK;
 }
 
