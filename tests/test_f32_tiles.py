@@ -139,6 +139,8 @@ def test_f32_values_that_cannot_be_split_in_every_branch(kind, B, Hq, Hkv, T, bs
         return o, *nsa.range_attn_backward(q, k, v, o, lse, do, nsa.MODE_COMPRESS_STRIDED, W, bs)
 
     clean = run(q, k, v, do)
+    for name, a, b in zip(("o", "dq", "dk", "dv"), clean, _dense(q, k, v, do, n)):
+        assert (a.double() - b).norm() <= 2.0 ** -20 * b.norm(), name
     hit = lambda where, at: (n[..., at] > 0) if where in "kv" else (torch.arange(T, device="cuda") == at).expand(B, Hkv, T)
     same = lambda a, b: torch.isfinite(a).all() and (a - b).norm() <= 2.0 ** -20 * b.norm()
 
